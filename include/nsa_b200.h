@@ -104,6 +104,12 @@ typedef struct {
                             not fit the sizes is detected on the device (status 2, nothing computed).  Ignored
                             inside nsa_sel_bwd_args, which has an index field of its own                          */
   int64_t index_bytes;
+  int32_t* status;       /* optional: the device word the tensor-core kernels report through (they only OR into it: the
+                            caller clears it once and may share it between calls); NULL = the first word of the work
+                            buffer, cleared by the call                                                             */
+  void* index_out;       /* optional, forward only: build the index here (nsa_sel_index_bytes(args) bytes, 256-byte
+                            aligned) instead of at the head of the work buffer, for a caller that keeps it           */
+  int64_t index_out_bytes;
 } nsa_sel_fwd_args;
 
 int nsa_sel_fwd(const nsa_sel_fwd_args* args, void* stream);
@@ -136,6 +142,9 @@ typedef struct {
   nsa_tensor dq_out;     /* optional (ptr NULL = unused): dq in the dtype of q with these strides, see nsa_sel_bwd_stores_dq */
   const float* delta;    /* optional [B, q_heads, N] fp32: sum over d of out * dout for every row, for a caller that
                             has it already (the gated combine's backward forms it: gate * d gate); NULL = computed */
+  int32_t accumulate_kv; /* non-zero: dk and dv are added to as they are instead of zeroed first, for a caller that sums
+                            the gradients of several branches over the same keys                                */
+  int32_t reserved;
 } nsa_sel_bwd_args;
 
 int nsa_sel_bwd(const nsa_sel_bwd_args* args, void* stream);
@@ -232,6 +241,8 @@ typedef struct {
   int64_t workspace_bytes;
   void* pooled;          /* optional, instead of importance: see nsa_cmp_fwd_pools */
   int32_t pool;          /* block columns per selection block (selection_block_size / stride) */
+  int32_t reserved;
+  int32_t* status;       /* optional, as in nsa_sel_fwd_args                                  */
 } nsa_cmp_fwd_args;
 
 int nsa_cmp_fwd(const nsa_cmp_fwd_args* args, void* stream);
@@ -329,6 +340,7 @@ typedef struct {
   float scale;
   void* workspace;       /* nsa_swa_workspace_bytes(args, 0) bytes, may be NULL if that is 0 */
   int64_t workspace_bytes;
+  int32_t* status;       /* optional, as in nsa_sel_fwd_args                  */
 } nsa_swa_fwd_args;
 
 int nsa_swa_fwd(const nsa_swa_fwd_args* args, void* stream);
@@ -348,6 +360,8 @@ typedef struct {
   const void* index;     /* optional, see nsa_swa_index_bytes */
   int64_t index_bytes;
   const float* delta;    /* optional, as in nsa_sel_bwd_args */
+  int32_t accumulate_kv; /* as in nsa_sel_bwd_args */
+  int32_t reserved;
 } nsa_swa_bwd_args;
 
 int nsa_swa_bwd(const nsa_swa_bwd_args* args, void* stream);

@@ -29,12 +29,14 @@ class SelFwdArgs(C.Structure):
                 ('idx', vp), ('mask', vp), ('lse', vp),
                 ('batch', i32), ('q_heads', i32), ('kv_heads', i32), ('sel_heads', i32), ('seq', i32), ('dim_head', i32),
                 ('block', i32), ('nsel', i32), ('diag', i32), ('dtype', i32), ('impl', i32), ('scale', f32),
-                ('workspace', vp), ('workspace_bytes', i64), ('index', vp), ('index_bytes', i64)]
+                ('workspace', vp), ('workspace_bytes', i64), ('index', vp), ('index_bytes', i64), ('status', vp),
+                ('index_out', vp), ('index_out_bytes', i64)]
 
 
 class SelBwdArgs(C.Structure):
     _fields_ = [('fwd', SelFwdArgs), ('dout', Tensor4), ('dq', vp), ('dk', vp), ('dv', vp), ('slot_grads', vp),
-                ('index', vp), ('index_bytes', i64), ('dq_out', Tensor4), ('delta', vp)]
+                ('index', vp), ('index_bytes', i64), ('dq_out', Tensor4), ('delta', vp), ('accumulate_kv', i32),
+                ('reserved', i32)]
 
 
 class CmpFwdArgs(C.Structure):
@@ -42,7 +44,7 @@ class CmpFwdArgs(C.Structure):
                 ('batch', i32), ('q_heads', i32), ('kv_heads', i32), ('sel_heads', i32), ('seq', i32), ('dim_head', i32),
                 ('num_mem', i32), ('ncb', i32), ('stride', i32), ('causal', i32), ('dtype', i32), ('impl', i32),
                 ('scale', f32), ('sentinel', f32), ('workspace', vp), ('workspace_bytes', i64), ('pooled', vp),
-                ('pool', i32)]
+                ('pool', i32), ('reserved', i32), ('status', vp)]
 
 
 class CmpBwdArgs(C.Structure):
@@ -60,12 +62,12 @@ class SwaFwdArgs(C.Structure):
     _fields_ = [('q', Tensor4), ('k', Tensor4), ('v', Tensor4), ('out', Tensor4), ('lse', vp),
                 ('batch', i32), ('q_heads', i32), ('kv_heads', i32), ('seq', i32), ('dim_head', i32),
                 ('window', i32), ('causal', i32), ('dtype', i32), ('impl', i32), ('scale', f32),
-                ('workspace', vp), ('workspace_bytes', i64)]
+                ('workspace', vp), ('workspace_bytes', i64), ('status', vp)]
 
 
 class SwaBwdArgs(C.Structure):
     _fields_ = [('fwd', SwaFwdArgs), ('dout', Tensor4), ('dq', vp), ('dk', vp), ('dv', vp), ('dq_out', Tensor4),
-                ('index', vp), ('index_bytes', i64), ('delta', vp)]
+                ('index', vp), ('index_bytes', i64), ('delta', vp), ('accumulate_kv', i32), ('reserved', i32)]
 
 
 class CombineFwdArgs(C.Structure):
@@ -163,6 +165,24 @@ def load():
                            f'bytes, binding {C.sizeof(st)} bytes')
     _lib = lib
     return lib
+
+
+_host = None
+
+
+def host():
+    """The native host side of the operators (csrc/host), loaded once; it calls the library `load` returns."""
+    global _host
+    if _host is None:
+        load()
+        try:
+            from . import _nsa_host
+        except ImportError as e:
+            raise NsaError(f'the native host module does not load ({e}): build it with '
+                           '`python -m native_sparse_attention_pytorch_b200.build`') from e
+        _nsa_host.set_error_class(NsaError)
+        _host = _nsa_host
+    return _host
 
 
 def check(rc):

@@ -1,10 +1,12 @@
-"""Builds libnsa_b200.so (the C-ABI library) in-tree with nvcc for sm_100a.
+"""Builds libnsa_b200.so (the C-ABI library, nvcc for sm_100a) and _nsa_host.so (the native host side of the PyTorch
+operators, g++ against the installed PyTorch) in-tree.
 
     python -m native_sparse_attention_pytorch_b200.build [--force] [--verbose]
 """
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -13,37 +15,68 @@ LIB = os.path.join(HERE, 'libnsa_b200.so')
 SOURCES = ['nsa_abi.cu', 'nsa_simt_attend.cu', 'nsa_select.cu', 'nsa_combine.cu', 'nsa_rotary.cu', 'nsa_windows.cu', 'nsa_rmsnorm.cu', 'nsa_decode.cu', 'nsa_sm100_sel.cu']
 
 
-def _newest_source_mtime():
-    paths = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(ROOT, 'include', 'nsa_b200.h')]
-    return max(os.path.getmtime(p) for p in paths)
+HOST_LIB = os.path.join(HERE, '_nsa_host.so')
+HOST_SOURCES = ['module.cpp', 'selected.cpp']
 
 
-def build(force=False, verbose=False):
-    """Compile every kernel file for sm_100a and link the shared library."""
-    if not force and os.path.exists(LIB) and os.path.getmtime(LIB) >= _newest_source_mtime():
-        return LIB
-    nvcc = os.environ.get('NVCC', '/usr/local/cuda/bin/nvcc')
-    objdir = os.path.join(HERE, 'build')
-    os.makedirs(objdir, exist_ok=True)
-    flags = ['-gencode', 'arch=compute_100a,code=sm_100a', '-lineinfo', '-O3', '-std=c++17',
-             '-Xcompiler', '-fPIC', '-I', os.path.join(ROOT, 'include'), '-I', CSRC]
-    if verbose:
-        flags += ['-Xptxas', '-v']
-    procs = []
-    for src in SOURCES:
-        obj = os.path.join(objdir, src.replace('.cu', '.o'))
-        cmd = [nvcc, *flags, '-c', os.path.join(CSRC, src), '-o', obj]
-        procs.append((src, obj, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
-    objs = []
-    for src, obj, p in procs:
+def _newest(*dirs):
+    paths = [os.path.join(d, f) for d in dirs for f in os.listdir(d)] + [os.path.join(ROOT, 'include', 'nsa_b200.h')]
+    return max(os.path.getmtime(p) for p in paths if os.path.isfile(p))
+
+
+def _fresh(lib, *dirs):
+    return os.path.exists(lib) and os.path.getmtime(lib) >= _newest(*dirs)
+
+
+def _compile_all(jobs, verbose):
+    """jobs: (source name, object, command).  Runs them side by side and returns the objects."""
+    procs = [(src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)) for src, _, cmd in jobs]
+    failed = None
+    for src, p in procs:
         out, _ = p.communicate()
         if verbose or p.returncode != 0:
             sys.stderr.write(f'--- {src} ---\n{out}\n')
         if p.returncode != 0:
-            raise RuntimeError(f'nvcc failed on {src}')
-        objs.append(obj)
-    link = [nvcc, '-shared', '-o', LIB, *objs, '-cudart', 'static', '-gencode', 'arch=compute_100a,code=sm_100a']
-    subprocess.run(link, check=True)
+            failed = failed or src
+    if failed:
+        raise RuntimeError(f'compiling {failed} failed')
+    return [obj for _, obj, _ in jobs]
+
+
+def build(force=False, verbose=False):
+    """Compile every kernel file for sm_100a and link the two shared libraries."""
+    nvcc = os.environ.get('NVCC', '/usr/local/cuda/bin/nvcc')
+    objdir = os.path.join(HERE, 'build')
+    os.makedirs(objdir, exist_ok=True)
+    includes = ['-I', os.path.join(ROOT, 'include'), '-I', CSRC]
+    jobs, host_jobs = [], []
+    if force or not _fresh(LIB, CSRC):
+        flags = ['-gencode', 'arch=compute_100a,code=sm_100a', '-lineinfo', '-O3', '-std=c++17', '-Xcompiler', '-fPIC',
+                 *includes] + (['-Xptxas', '-v'] if verbose else [])
+        jobs = [(src, os.path.join(objdir, src.replace('.cu', '.o')),
+                 [nvcc, *flags, '-c', os.path.join(CSRC, src), '-o', os.path.join(objdir, src.replace('.cu', '.o'))])
+                for src in SOURCES]
+    if force or not _fresh(HOST_LIB, CSRC, os.path.join(CSRC, 'host')):
+        import torch
+        from torch.utils import cpp_extension
+        cuda = os.path.dirname(os.path.dirname(nvcc))
+        flags = ['-O2', '-std=c++17', '-fPIC', '-fvisibility=hidden', '-DTORCH_API_INCLUDE_EXTENSION_H',
+                 f'-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}', *includes,
+                 '-isystem', sysconfig.get_paths()['include'], '-isystem', os.path.join(cuda, 'include')]
+        for d in cpp_extension.include_paths():
+            flags += ['-isystem', d]
+        host_jobs = [(src, os.path.join(objdir, 'host_' + src.replace('.cpp', '.o')),
+                      ['g++', *flags, '-c', os.path.join(CSRC, 'host', src), '-o', os.path.join(objdir, 'host_' + src.replace('.cpp', '.o'))])
+                     for src in HOST_SOURCES]
+    objs = _compile_all(jobs + host_jobs, verbose)
+    if jobs:
+        subprocess.run([nvcc, '-shared', '-o', LIB, *objs[:len(jobs)], '-cudart', 'static',
+                        '-gencode', 'arch=compute_100a,code=sm_100a'], check=True)
+    if host_jobs:
+        import torch
+        torch_lib = os.path.join(os.path.dirname(torch.__file__), 'lib')
+        subprocess.run(['g++', '-shared', '-o', HOST_LIB, *objs[len(jobs):], '-L', HERE, '-lnsa_b200', '-L', torch_lib, '-ltorch', '-ltorch_cpu',
+                        '-ltorch_cuda', '-ltorch_python', '-lc10', '-lc10_cuda', '-Wl,-rpath,$ORIGIN'], check=True)
     return LIB
 
 

@@ -1,0 +1,75 @@
+// Shared pieces of the native host side: what stands between PyTorch tensors and the C ABI of libnsa_b200.so.
+//
+// The Python operators issue one call of this extension per direction.  Filling the argument structs, sizing and
+// allocating the buffers and issuing the launches from Python cost 100 to 150 us per operator and direction (ctypes
+// structs, stream look-ups, allocator calls through the dispatcher), several times what the GPU needs at ordinary
+// sizes; here it is a few microseconds plus the launches.
+#pragma once
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <optional>
+#include <stdexcept>
+#include <string>
+#include <vector>
+
+#include "nsa_b200.h"
+
+namespace nsa_host {
+
+using at::Tensor;
+using OptTensor = std::optional<Tensor>;
+
+// An NSA_ERR_* or CUDA error code with its message; reaches Python as the package's NsaError.
+struct Error : std::runtime_error {
+  explicit Error(const std::string& what) : std::runtime_error(what) {}
+};
+
+inline void check(int64_t rc) {
+  if (rc != 0) throw Error("libnsa_b200 returned " + std::to_string(rc) + ": " + nsa_last_error());
+}
+
+inline void require_cuda(const Tensor& t) {
+  if (t.defined() && !t.is_cuda())
+    throw Error("the NSA kernels run on CUDA tensors only; there is no CPU implementation in this package");
+}
+
+inline int dtype_code(const Tensor& t) {
+  if (t.scalar_type() == at::kFloat) return NSA_F32;
+  if (t.scalar_type() == at::kBFloat16) return NSA_BF16;
+  throw Error(std::string("unsupported dtype ") + c10::toString(t.scalar_type()) + ": the kernels take float32 or bfloat16");
+}
+
+// t itself if its last axis is contiguous and its rows are 16-byte aligned, else a contiguous copy
+inline Tensor rowwise(const Tensor& t) {
+  const int64_t per16 = 16 / t.element_size();
+  const auto st = t.strides();
+  bool ok = st.back() == 1 && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+  for (size_t i = 0; ok && i + 1 < st.size(); ++i) ok = st[i] % per16 == 0;
+  return ok ? t : t.contiguous();
+}
+
+inline nsa_tensor t4(const Tensor& t) { return {t.data_ptr(), t.stride(0), t.stride(1), t.stride(2)}; }
+inline nsa_tensor no_tensor() { return {nullptr, 0, 0, 0}; }
+
+template <typename T>
+T* ptr(const Tensor& t) { return t.defined() ? static_cast<T*>(t.data_ptr()) : nullptr; }
+
+inline Tensor empty(at::IntArrayRef sizes, const Tensor& like, at::ScalarType type) {
+  return at::empty(sizes, like.options().dtype(type));
+}
+inline Tensor bytes(int64_t n, const Tensor& like) { return at::empty({n}, like.options().dtype(at::kByte)); }
+
+inline void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+
+// Uninitialised tensor of t's shape and dtype whose dimensions lie in memory in the order t's do: a [b, h, n, d] view
+// of a [b, n, (h d)] projection output gives a [b, n, h, d] buffer seen as [b, h, n, d], so that the gradient of the
+// view that made t is a view again instead of a copy.
+Tensor empty_in_order_of(const Tensor& t);
+
+void bind_selected(pybind11::module_& m);
+
+}  // namespace nsa_host

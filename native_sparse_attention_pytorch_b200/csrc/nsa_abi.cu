@@ -68,6 +68,14 @@ static int zero_async(float* p, int64_t count, cudaStream_t stream) {
   return err == cudaSuccess ? NSA_OK : fail((int)err, cudaGetErrorString(err));
 }
 
+// dk and dv start from zero unless the caller adds to what they hold; one call where they lie back to back
+static int zero_kv(float* dk, float* dv, int64_t count, bool accumulate, cudaStream_t stream) {
+  if (accumulate) return NSA_OK;
+  if (dv == dk + count) return zero_async(dk, 2 * count, stream);
+  NSA_TRY(zero_async(dk, count, stream));
+  return zero_async(dv, count, stream);
+}
+
 // ---- selected-block branch ---------------------------------------------------
 
 static int fill_sel(AttnParams& P, const nsa_sel_fwd_args& a) {
@@ -180,6 +188,8 @@ int nsa_sel_fwd(const nsa_sel_fwd_args* a, void* stream) {
   NSA_TRY(fill_sel(P, *a));
   if (a->index != nullptr && (reinterpret_cast<uintptr_t>(a->index) & 15u))
     return fail(NSA_ERR_ALIGN, "index must be 16-byte aligned");
+  if (a->index_out != nullptr && (reinterpret_cast<uintptr_t>(a->index_out) & 255u))
+    return fail(NSA_ERR_ALIGN, "index_out must be 256-byte aligned");
   cudaStream_t st = (cudaStream_t)stream;
   if (a->impl != NSA_IMPL_SIMT) {
     const int rc = sm100_sel_fwd(*a, st);
@@ -251,8 +261,7 @@ int nsa_sel_bwd(const nsa_sel_bwd_args* a, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t d = a->fwd.dim_head, n = a->fwd.seq, b = a->fwd.batch;
   if (!dq_stored) NSA_TRY(zero_async(a->dq, b * a->fwd.q_heads * n * d, st));
-  NSA_TRY(zero_async(a->dk, b * a->fwd.kv_heads * n * d, st));
-  NSA_TRY(zero_async(a->dv, b * a->fwd.kv_heads * n * d, st));
+  NSA_TRY(zero_kv(a->dk, a->dv, b * a->fwd.kv_heads * n * d, a->accumulate_kv != 0, st));
   if (a->fwd.impl != NSA_IMPL_SIMT) {
     const int rc = sm100_sel_bwd(*a, st);
     if (rc != NSA_ERR_UNSUPPORTED || a->fwd.impl == NSA_IMPL_SM100) return rc;
@@ -331,8 +340,7 @@ int nsa_cmp_bwd(const nsa_cmp_bwd_args* a, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t d = a->fwd.dim_head, rows = a->fwd.num_mem + a->fwd.ncb, b = a->fwd.batch;
   if (!dq_stored) NSA_TRY(zero_async(a->dq, b * a->fwd.q_heads * a->fwd.seq * d, st));
-  NSA_TRY(zero_async(a->dck, b * a->fwd.kv_heads * rows * d, st));
-  NSA_TRY(zero_async(a->dcv, b * a->fwd.kv_heads * rows * d, st));
+  NSA_TRY(zero_kv(a->dck, a->dcv, b * a->fwd.kv_heads * rows * d, false, st));
   if (a->fwd.impl != NSA_IMPL_SIMT) {
     const int rc = sm100_cmp_bwd(*a, st);
     if (rc != NSA_ERR_UNSUPPORTED) return rc;
@@ -421,8 +429,7 @@ int nsa_swa_bwd(const nsa_swa_bwd_args* a, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t d = a->fwd.dim_head, n = a->fwd.seq, b = a->fwd.batch;
   if (!dq_stored) NSA_TRY(zero_async(a->dq, b * a->fwd.q_heads * n * d, st));
-  NSA_TRY(zero_async(a->dk, b * a->fwd.kv_heads * n * d, st));
-  NSA_TRY(zero_async(a->dv, b * a->fwd.kv_heads * n * d, st));
+  NSA_TRY(zero_kv(a->dk, a->dv, b * a->fwd.kv_heads * n * d, a->accumulate_kv != 0, st));
   if (a->fwd.impl != NSA_IMPL_SIMT) {
     const int rc = sm100_swa_bwd(*a, st);
     if (rc != NSA_ERR_UNSUPPORTED) return rc;

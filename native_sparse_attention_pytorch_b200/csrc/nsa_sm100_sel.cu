@@ -86,7 +86,8 @@ struct SelPlan {
   int nqb, nkb, ns, G, QT, nlists;
   int64_t entries_cap, items_cap;
   // byte offsets into the work buffer
-  int64_t off_status, off_num_items, off_counts, off_totals, off_list_base, off_items, off_entries;
+  int words;             // 32-bit words of slot bits per query
+  int64_t off_status, off_num_items, off_totals, off_list_base, off_cursors, off_bits, off_items, off_entries;
   int64_t off_partial, off_stats, off_delta;
   int64_t index_bytes;   // the leading part that holds the index (what the backward can take from the forward)
   int64_t total_bytes;
@@ -101,6 +102,8 @@ struct SelParams {
   const uint32_t* entries;
   const int4* items;
   const int* num_items;    // [0] items, [1] the tag the item kernel left
+  const uint32_t* bits;    // [B*Hkv*N][words]: the slots a query has (kModeSel)
+  int words;
   __nv_bfloat16* dq_lp;    // optional bf16 dq with its own batch / head / row strides (dq merge)
   int64_t dq_sb, dq_sh, dq_sn;
   uint32_t index_tag;
@@ -128,137 +131,159 @@ struct SelParams {
 // index that belongs to another problem, or a buffer nobody filled, must not steer any address.
 __device__ __forceinline__ int item_count(const SelParams& P) {
   if ((uint32_t)P.num_items[1] != P.index_tag) {
-    if (threadIdx.x == 0) atomicExch(P.status, 2);
+    if (threadIdx.x == 0) atomicOr(P.status, 2);
     return 0;
   }
   return P.num_items[0];
 }
 
 // ---- index pre-pass --------------------------------------------------------------
+//
+// Four short integer kernels, 28 us at batch 4, 8192 tokens, 16 slots (72 us as a [query block x key block] matrix of
+// counts with a scan over it): clear the list totals, count, lay the lists out, fill them.  A block owns 128 queries
+// of one (batch, KV head); it counts in shared memory and touches a list's total and cursor once, so the order of the
+// query blocks inside a list is whatever order the blocks arrive in.  Nothing downstream depends on it: every
+// (row, slot) partial is computed from its own row alone, and dk / dv are sums of fp32 reductions in any case.
+constexpr int kIndexQueries = 128;
 
-// counts[(bh*nqb + qb)*nkb + j] = entries that the queries of block qb contribute to list (bh, j)
+__global__ void __launch_bounds__(256) sel_clear_kernel(int* totals, int nlists) {
+  const int l = blockIdx.x * 256 + threadIdx.x;
+  if (l < nlists) totals[l] = 0;
+}
+
+// hist[blk] += 1 for every lane with `valid`; lanes of a warp that hit the same list are added together
+__device__ __forceinline__ void count_block(int* hist, bool valid, int blk, int lane) {
+  const unsigned vm = __ballot_sync(kFullMask, valid);
+  if (valid) {
+    const unsigned peers = __match_any_sync(vm, blk);
+    if (lane == __ffs(peers) - 1) atomicAdd(&hist[blk], __popc(peers));
+  }
+}
+
+// totals[list] += entries of this block's queries; bits[(bh*N + i)*words + w]: which of its slots query i has
 template <int MODE>
-__global__ void __launch_bounds__(kBlock) sel_hist_kernel(const BlockRule R, int* counts) {
+__global__ void __launch_bounds__(kIndexQueries) sel_count_kernel(const BlockRule R, int* totals, uint32_t* bits, int words) {
   extern __shared__ int hist[];
-  const int qb = blockIdx.x, nqb = gridDim.x, bh = blockIdx.y * gridDim.z + blockIdx.z;  // bh = b*Hkv + h
-  for (int j = threadIdx.x; j < R.nkb; j += kBlock) hist[j] = 0;
+  const int bh = blockIdx.y * gridDim.z + blockIdx.z;  // bh = b*Hkv + h
+  const int lane = threadIdx.x & 31;
+  for (int j = threadIdx.x; j < R.nkb; j += kIndexQueries) hist[j] = 0;
   __syncthreads();
-  const int i = qb * kBlock + threadIdx.x;
-  if (i < R.N) {
-    for (int s = 0; s < R.ns; ++s) {
-      int blk;
-      if (slot_block<MODE>(R, bh, i, s, &blk)) atomicAdd(&hist[blk], 1);
+  const int i = blockIdx.x * kIndexQueries + threadIdx.x;
+  for (int w = 0; w < words; ++w) {
+    uint32_t mine = 0;
+    const int s_end = min(R.ns, w * 32 + 32);
+#pragma unroll 4
+    for (int s = w * 32; s < s_end; ++s) {
+      int blk = 0;
+      const bool valid = i < R.N && slot_block<MODE>(R, bh, i, s, &blk);
+      mine |= valid ? 1u << (s & 31) : 0u;
+      count_block(hist, valid, blk, lane);
     }
+    if (i < R.N) bits[((int64_t)bh * R.N + i) * words + w] = mine;
   }
   __syncthreads();
-  int* row = counts + ((int64_t)bh * nqb + qb) * R.nkb;
-  for (int j = threadIdx.x; j < R.nkb; j += kBlock) row[j] = hist[j];
+  for (int j = threadIdx.x; j < R.nkb; j += kIndexQueries)
+    if (hist[j] > 0) atomicAdd(&totals[bh * R.nkb + j], hist[j]);
 }
 
-// per list: exclusive prefix over the contributing query blocks, and the list total.  A block handles 32
-// neighbouring lists (threadIdx.x, so that loads stay coalesced) with kScanSeg threads each (threadIdx.y): every
-// thread sums its segment of query blocks, the segments' sums are prefixed through shared memory, and a second pass
-// over the segment writes the prefixes.
-constexpr int kScanSeg = 8;
-__global__ void __launch_bounds__(32 * kScanSeg) sel_scan_kernel(int* counts, int* totals, int nlists, int nqb, int nkb) {
-  __shared__ int seg_sum[kScanSeg][32];
-  const int l = blockIdx.x * 32 + threadIdx.x, seg = threadIdx.y;
-  const bool live = l < nlists;
-  const int bh = live ? l / nkb : 0, j = live ? l - bh * nkb : 0;
-  const int per = (nqb + kScanSeg - 1) / kScanSeg;
-  const int q0 = min(nqb, seg * per), q1 = min(nqb, q0 + per);
-  int* base = counts + (int64_t)bh * nqb * nkb + j;
-  int sum = 0;
-  if (live)
-    for (int qb = q0; qb < q1; ++qb) sum += base[(int64_t)qb * nkb];
-  seg_sum[seg][threadIdx.x] = sum;
-  __syncthreads();
-  int running = 0;
-  for (int k = 0; k < seg; ++k) running += seg_sum[k][threadIdx.x];
-  if (live) {
-    for (int qb = q0; qb < q1; ++qb) {
-      int* c = base + (int64_t)qb * nkb;
-      const int v = *c;
-      *c = running;
-      running += v;
-    }
-    if (seg == kScanSeg - 1) totals[l] = running;
+// Exclusive prefix over the block's 1024 threads of two values at once; returns the totals.
+__device__ __forceinline__ int2 block_scan2(int2 v, int2* total, int2 (*warp_sums)[32]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int2 inc = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int a = __shfl_up_sync(kFullMask, inc.x, o), b = __shfl_up_sync(kFullMask, inc.y, o);
+    if (lane >= o) { inc.x += a; inc.y += b; }
   }
+  if (lane == 31) (*warp_sums)[warp] = inc;
+  __syncthreads();
+  if (warp == 0) {
+    int2 s = (*warp_sums)[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int a = __shfl_up_sync(kFullMask, s.x, o), b = __shfl_up_sync(kFullMask, s.y, o);
+      if (lane >= o) { s.x += a; s.y += b; }
+    }
+    (*warp_sums)[lane] = s;
+  }
+  __syncthreads();
+  const int2 before = warp > 0 ? (*warp_sums)[warp - 1] : make_int2(0, 0);
+  *total = (*warp_sums)[31];
+  __syncthreads();
+  return make_int2(before.x + inc.x - v.x, before.y + inc.y - v.y);
 }
 
-// list bases (padded to whole chunks) and the item table; one CTA of 1024 threads
-__global__ void __launch_bounds__(1024) sel_items_kernel(const int* totals, int* list_base, int4* items, int* num_items,
-                                                         int nlists, int QT, uint32_t tag) {
-  __shared__ int s_pad[1024], s_it[1024];
-  __shared__ int carry_pad, carry_it;
-  if (threadIdx.x == 0) carry_pad = carry_it = 0;
-  __syncthreads();
-  for (int t0 = 0; t0 < nlists; t0 += 1024) {
-    const int l = t0 + threadIdx.x;
-    const int cnt = l < nlists ? totals[l] : 0;
-    const int nch = (cnt + QT - 1) / QT;
-    const int nit = (nch + kChunksPerItem - 1) / kChunksPerItem;
-    s_pad[threadIdx.x] = nch * QT;
-    s_it[threadIdx.x] = nit;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-      int a = 0, b = 0;
-      if ((int)threadIdx.x >= o) { a = s_pad[threadIdx.x - o]; b = s_it[threadIdx.x - o]; }
-      __syncthreads();
-      s_pad[threadIdx.x] += a;
-      s_it[threadIdx.x] += b;
-      __syncthreads();
-    }
-    const int base = carry_pad + s_pad[threadIdx.x] - nch * QT;  // exclusive
-    const int ibase = carry_it + s_it[threadIdx.x] - nit;
-    if (l < nlists) {
-      list_base[l] = base;
-      for (int k = 0; k < nit; ++k) {
-        const int c0 = k * kChunksPerItem;
-        items[ibase + k] = make_int4(l, c0, min(kChunksPerItem, nch - c0), base + c0 * QT);
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x == 1023) { carry_pad += s_pad[1023]; carry_it += s_it[1023]; }
-    __syncthreads();
+// List bases (padded to whole chunks), the fill cursors and the item table; one CTA, every thread owns a run of lists.
+// A list is cut into items of at most kChunksPerItem chunks, fewer when the whole problem has few chunks: an item is
+// what one CTA walks serially, so a problem of a few hundred chunks in items of sixteen leaves most of the chip idle.
+// The line is kItemsTarget items (16 per SM): below it the K/V loads and the dK/dV flush of a short item still cost
+// less than the imbalance of long ones.
+constexpr int kItemsTarget = 148 * 16;
+__global__ void __launch_bounds__(1024) sel_items_kernel(const int* totals, int* list_base, int* cursors, int4* items,
+                                                         int* num_items, int nlists, int QT, uint32_t tag) {
+  __shared__ int2 warp_sums[32];
+  const int per = (nlists + 1023) / 1024;
+  const int l0 = min(nlists, (int)threadIdx.x * per), l1 = min(nlists, l0 + per);
+  int chunks = 0;
+  for (int l = l0; l < l1; ++l) chunks += (totals[l] + QT - 1) / QT;
+  int2 all;
+  block_scan2(make_int2(chunks, 0), &all, &warp_sums);
+  const int cpi = max(1, min(kChunksPerItem, all.x / kItemsTarget));
+  int nit = 0;
+  for (int l = l0; l < l1; ++l) nit += ((totals[l] + QT - 1) / QT + cpi - 1) / cpi;
+  int2 at = block_scan2(make_int2(chunks, nit), &all, &warp_sums);
+  int base = at.x * QT, ibase = at.y;
+  for (int l = l0; l < l1; ++l) {
+    const int nch = (totals[l] + QT - 1) / QT;
+    list_base[l] = base;
+    cursors[l] = base;
+    for (int c0 = 0; c0 < nch; c0 += cpi) items[ibase++] = make_int4(l, c0, min(cpi, nch - c0), base + c0 * QT);
+    base += nch * QT;
   }
   if (threadIdx.x == 0) {
-    num_items[0] = carry_it;
+    num_items[0] = all.y;
     num_items[1] = (int)tag;   // marks the index as built, and for which sizes
   }
 }
 
-// writes the entries (query | slot << 24) in a fixed order: by query block, then slot, then query
+// writes the entries (query | slot << 24) and pads every list to whole chunks
 template <int MODE>
-__global__ void __launch_bounds__(kBlock) sel_fill_kernel(const BlockRule R, const int* counts, const int* list_base,
-                                                          uint32_t* entries) {
+__global__ void __launch_bounds__(kIndexQueries) sel_fill_kernel(const BlockRule R, const int* totals, const int* list_base,
+                                                                 int* cursors, uint32_t* entries, int QT) {
   extern __shared__ int cursor[];
-  const int qb = blockIdx.x, nqb = gridDim.x, bh = blockIdx.y * gridDim.z + blockIdx.z;
-  const int* row = counts + ((int64_t)bh * nqb + qb) * R.nkb;
-  for (int j = threadIdx.x; j < R.nkb; j += kBlock) cursor[j] = list_base[bh * R.nkb + j] + row[j];
+  const int bh = blockIdx.y * gridDim.z + blockIdx.z;
+  const int lane = threadIdx.x & 31;
+  for (int j = threadIdx.x; j < R.nkb; j += kIndexQueries) cursor[j] = 0;
   __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int i = qb * kBlock + threadIdx.x;
+  const int i = blockIdx.x * kIndexQueries + threadIdx.x;
+#pragma unroll 4
   for (int s = 0; s < R.ns; ++s) {
     int blk = 0;
     const bool valid = i < R.N && slot_block<MODE>(R, bh, i, s, &blk);
-    for (int w = 0; w < 2; ++w) {
-      if (warp == w) {
-        const unsigned vm = __ballot_sync(kFullMask, valid);
-        if (valid) {
-          const unsigned peers = __match_any_sync(vm, blk);
-          const int rank = __popc(peers & ((1u << lane) - 1u));
-          const int leader = __ffs(peers) - 1;
-          int pos = 0;
-          if (lane == leader) {
-            pos = cursor[blk];
-            cursor[blk] = pos + __popc(peers);
-          }
-          pos = __shfl_sync(peers, pos, leader);
-          entries[pos + rank] = (uint32_t)i | ((uint32_t)s << 24);
-        }
-      }
-      __syncthreads();
+    count_block(cursor, valid, blk, lane);
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < R.nkb; j += kIndexQueries) {
+    const int mine = cursor[j];
+    if (mine > 0) cursor[j] = atomicAdd(&cursors[bh * R.nkb + j], mine);
+    if (blockIdx.x == 0) {
+      const int l = bh * R.nkb + j, end = list_base[l] + totals[l], stop = (end + QT - 1) / QT * QT;   // bases are multiples of QT
+      for (int p = end; p < stop; ++p) entries[p] = kInvalidEntry;
+    }
+  }
+  __syncthreads();
+#pragma unroll 4
+  for (int s = 0; s < R.ns; ++s) {
+    int blk = 0;
+    const bool valid = i < R.N && slot_block<MODE>(R, bh, i, s, &blk);
+    const unsigned vm = __ballot_sync(kFullMask, valid);
+    if (valid) {
+      const unsigned peers = __match_any_sync(vm, blk);
+      const int leader = __ffs(peers) - 1;
+      int pos = 0;
+      if (lane == leader) pos = atomicAdd(&cursor[blk], __popc(peers));
+      pos = __shfl_sync(peers, pos, leader) + __popc(peers & ((1u << lane) - 1u));
+      entries[pos] = (uint32_t)i | ((uint32_t)s << 24);
     }
   }
 }
@@ -593,13 +618,14 @@ sel_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tm, kCols);
-  if (tid == 0 && abort_flag) atomicExch(P.status, 1);
+  if (tid == 0 && abort_flag) atomicOr(P.status, 1);
 }
 
 // merges the partial results of every (batch, query head, query): one group of D/8 threads per row.
-// The statistics were cleared before the forward kernel ran, so a slot the query does not have reads (0, 0) and needs
-// no look-up in the index; its partial row was never written and is not read.  Loads are issued eight slots at a time
-// with nothing depending on them in between: the kernel is a stream over the partial buffer.
+// The index's slot bits (one word per 32 slots of a query, shared by its heads) say which slots the query has: the
+// partial rows and statistics of the others were never written and are not read, so neither needs clearing (clearing
+// the statistics took 22 us at 17.8 M slots).  Loads are issued eight slots at a time with nothing depending on them
+// in between: the kernel is a stream over the partial buffer.
 template <int D>
 __global__ void __launch_bounds__(256) sel_merge_kernel(const SelParams P) {
   constexpr int TPR = D / 8;
@@ -612,23 +638,25 @@ __global__ void __launch_bounds__(256) sel_merge_kernel(const SelParams P) {
   const int b = (int)(row / ((int64_t)P.N * P.Hq));
   const int ns = P.ns;
   const float2* st = P.stats + row * ns;
+  const uint32_t* bits = P.bits + ((int64_t)(b * P.Hkv + hq / P.G) * P.N + i) * P.words;
   const __nv_bfloat16* prow = P.partial + row * ns * D + part * 8;
   float M = -INFINITY;
-#pragma unroll 4
-  for (int s = 0; s < ns; ++s) {
-    const float2 ml = st[s];
-    if (ml.y > 0.f) M = fmaxf(M, ml.x);
+  for (int s0 = 0; s0 < ns; s0 += 8) {
+    const uint32_t has = bits[s0 >> 5] >> (s0 & 31);
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (has >> u & 1u) M = fmaxf(M, st[s0 + u].x);
   }
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   float L = 0.f;
   for (int s0 = 0; s0 < ns; s0 += 8) {
+    const uint32_t has = bits[s0 >> 5] >> (s0 & 31);
     float w[8];
     uint4 v[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
-      const bool in = s0 + u < ns;
-      const float2 ml = in ? st[s0 + u] : make_float2(0.f, 0.f);
-      const bool ok = ml.y > 0.f;
+      const bool ok = has >> u & 1u;
+      const float2 ml = ok ? st[s0 + u] : make_float2(0.f, 0.f);
       w[u] = ok ? ex2(ml.x - M) : 0.f;
       L = fmaf(w[u], ml.y, L);
       v[u] = ok ? *reinterpret_cast<const uint4*>(prow + (int64_t)(s0 + u) * D) : make_uint4(0u, 0u, 0u, 0u);
@@ -672,23 +700,25 @@ __global__ void __launch_bounds__(256) sel_merge_combine_kernel(const SelParams 
     const int64_t row = ((int64_t)b * P.Hq + hq) * P.N + i;
     const int ns = P.ns;
     const float2* st = P.stats + row * ns;
+    const uint32_t* bits = P.bits + ((int64_t)(b * P.Hkv + hq / P.G) * P.N + i) * P.words;
     const __nv_bfloat16* prow = P.partial + row * ns * D + part * 8;
     float M = -INFINITY;
-#pragma unroll 4
-    for (int s = 0; s < ns; ++s) {
-      const float2 ml = st[s];
-      if (ml.y > 0.f) M = fmaxf(M, ml.x);
+    for (int s0 = 0; s0 < ns; s0 += 8) {
+      const uint32_t has = bits[s0 >> 5] >> (s0 & 31);
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (has >> u & 1u) M = fmaxf(M, st[s0 + u].x);
     }
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     float Lsum = 0.f;
     for (int s0 = 0; s0 < ns; s0 += 8) {
+      const uint32_t has = bits[s0 >> 5] >> (s0 & 31);
       float w[8];
       uint4 v[8];
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
-        const bool in = s0 + u < ns;
-        const float2 ml = in ? st[s0 + u] : make_float2(0.f, 0.f);
-        const bool ok = ml.y > 0.f;
+        const bool ok = has >> u & 1u;
+        const float2 ml = ok ? st[s0 + u] : make_float2(0.f, 0.f);
         w[u] = ok ? ex2(ml.x - M) : 0.f;
         Lsum = fmaf(w[u], ml.y, Lsum);
         v[u] = ok ? *reinterpret_cast<const uint4*>(prow + (int64_t)(s0 + u) * D) : make_uint4(0u, 0u, 0u, 0u);
@@ -1107,7 +1137,7 @@ dense_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tm, kCols);
-  if (tid == 0 && abort_flag) atomicExch(P.status, 1);
+  if (tid == 0 && abort_flag) atomicOr(P.status, 1);
 }
 
 // ---- backward --------------------------------------------------------------------------
@@ -1339,7 +1369,7 @@ sel_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tm, kCols);
-  if (tid == 0 && abort_flag) atomicExch(P.status, 1);
+  if (tid == 0 && abort_flag) atomicOr(P.status, 1);
 }
 
 
@@ -1774,7 +1804,7 @@ sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tm, 512);
-  if (tid == 0 && abort_flag) atomicExch(P.status, 1);
+  if (tid == 0 && abort_flag) atomicOr(P.status, 1);
 }
 
 
@@ -1794,13 +1824,16 @@ __global__ void __launch_bounds__(256) sel_dq_merge_kernel(const SelParams P) {
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   const __nv_bfloat16* prow = P.partial + row * ns * D + part * 8;
   // eight slots at a time: first which of them the query has, then their loads together, then the sums
+  const uint32_t* bits = P.bits + ((int64_t)(b * P.Hkv + h) * P.N + i) * P.words;
   for (int s0 = 0; s0 < ns; s0 += 8) {
+    const uint32_t has = MODE == kModeSel ? bits[s0 >> 5] >> (s0 & 31) : 0u;
     bool ok[8];
     uint4 v[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       int blk_;
-      ok[u] = s0 + u < ns && slot_block<MODE>(P.rule, b * P.Hkv + h, i, s0 + u, &blk_);
+      ok[u] = MODE == kModeSel ? (has >> u & 1u) != 0
+                               : s0 + u < ns && slot_block<MODE>(P.rule, b * P.Hkv + h, i, s0 + u, &blk_);
     }
 #pragma unroll
     for (int u = 0; u < 8; ++u)
@@ -1873,8 +1906,11 @@ struct SelProblem {
   int64_t workspace_bytes;
   const CombineParams* fuse_combine;   // selected forward, optional: the merge also combines and stores (see
   const GatherTargets* fuse_targets;   // sel_merge_combine_kernel); `out` is then not written
-  const void* index;       // backward: the index part of the forward's work buffer, or NULL to rebuild it
+  const void* index;       // an index kept from an earlier call, or NULL to build it
   int64_t index_bytes;
+  void* index_out;         // optional: where to build it instead of the head of the work buffer
+  int64_t index_out_bytes;
+  int* status;             // optional: the word the kernels report through
   const float* delta;      // backward, optional: sum_d out * dout per row from the caller
   int B, Hq, Hkv, N, Nk, D;
   int nsel, diag, mode, window, stride, num_mem, ncb, round_bf16;
@@ -1924,23 +1960,25 @@ static SelPlan make_plan(const SelProblem& a, bool backward) {
   p.QT = kRows / p.G;
   p.nlists = a.B * a.Hkv * p.nkb;
   p.entries_cap = (int64_t)a.B * a.Hkv * (int64_t)a.N * p.ns + (int64_t)p.nlists * p.QT;
-  p.items_cap = p.entries_cap / p.QT / kChunksPerItem + p.nlists + 1;
+  p.items_cap = p.entries_cap / p.QT + p.nlists + 1;   // an item holds at least one chunk
+  p.words = (p.ns + 31) / 32;
   int64_t off = 0;
   p.off_status = off; off += 256;
   p.off_num_items = p.off_status + 128;
   if (!backward && dense_forward(a)) {   // only the status word is needed
-    p.off_counts = p.off_totals = p.off_list_base = p.off_items = p.off_entries = off;
+    p.off_totals = p.off_list_base = p.off_cursors = p.off_bits = p.off_items = p.off_entries = off;
     p.off_partial = p.off_stats = p.off_delta = off;
     p.index_bytes = 0;
     p.total_bytes = off;
     return p;
   }
-  p.off_counts = off; off = align_up(off + (int64_t)a.B * a.Hkv * p.nqb * p.nkb * 4, 256);
   p.off_totals = off; off = align_up(off + (int64_t)p.nlists * 4, 256);
   p.off_list_base = off; off = align_up(off + (int64_t)p.nlists * 4, 256);
+  p.off_cursors = off; off = align_up(off + (int64_t)p.nlists * 4, 256);
+  p.off_bits = off; off = align_up(off + (int64_t)a.B * a.Hkv * a.N * p.words * 4, 256);
   p.off_items = off; off = align_up(off + p.items_cap * 16, 256);
   p.off_entries = off; off = align_up(off + p.entries_cap * 4, 256);
-  p.index_bytes = off;   // status word, counts, list bases, items, entries: the same layout forward and backward
+  p.index_bytes = off;   // status word, totals, list bases, slot bits, items, entries: the same layout forward and backward
   const int64_t rows = (int64_t)a.B * a.Hq * a.N;
   p.off_partial = p.off_stats = p.off_delta = off;
   if (!backward) {
@@ -2009,33 +2047,54 @@ static uint32_t index_tag(const SelProblem& a, const SelPlan& p) {
   return h == 0 ? 1u : h;   // 0 is what a cleared buffer holds
 }
 
-static int build_index(const SelProblem& a, const SelPlan& p, uint8_t* ws, cudaStream_t st) {
-  int* counts = reinterpret_cast<int*>(ws + p.off_counts);
-  int* totals = reinterpret_cast<int*>(ws + p.off_totals);
-  int* list_base = reinterpret_cast<int*>(ws + p.off_list_base);
-  int4* items = reinterpret_cast<int4*>(ws + p.off_items);
-  int* num_items = reinterpret_cast<int*>(ws + p.off_num_items);
-  uint32_t* entries = reinterpret_cast<uint32_t*>(ws + p.off_entries);
-  CUDA_TRY(cudaMemsetAsync(ws + p.off_status, 0, 256, st));
-  CUDA_TRY(cudaMemsetAsync(entries, 0xff, (size_t)p.entries_cap * 4, st));
+static int build_index(const SelProblem& a, const SelPlan& p, uint8_t* ix, cudaStream_t st) {
+  int* totals = reinterpret_cast<int*>(ix + p.off_totals);
+  int* list_base = reinterpret_cast<int*>(ix + p.off_list_base);
+  int* cursors = reinterpret_cast<int*>(ix + p.off_cursors);
+  uint32_t* bits = reinterpret_cast<uint32_t*>(ix + p.off_bits);
+  int4* items = reinterpret_cast<int4*>(ix + p.off_items);
+  int* num_items = reinterpret_cast<int*>(ix + p.off_num_items);
+  uint32_t* entries = reinterpret_cast<uint32_t*>(ix + p.off_entries);
   const BlockRule R = make_rule(a, p);
-  const dim3 grid(p.nqb, a.B, a.Hkv);
-  const size_t hist_smem = (size_t)p.nkb * sizeof(int);
-  if (a.mode == kModeSel) sel_hist_kernel<kModeSel><<<grid, kBlock, hist_smem, st>>>(R, counts);
-  else if (a.mode == kModeSwa) sel_hist_kernel<kModeSwa><<<grid, kBlock, hist_smem, st>>>(R, counts);
-  else sel_hist_kernel<kModeCmp><<<grid, kBlock, hist_smem, st>>>(R, counts);
-  sel_scan_kernel<<<(p.nlists + 31) / 32, dim3(32, kScanSeg), 0, st>>>(counts, totals, p.nlists, p.nqb, p.nkb);
-  sel_items_kernel<<<1, 1024, 0, st>>>(totals, list_base, items, num_items, p.nlists, p.QT, index_tag(a, p));
-  if (a.mode == kModeSel) sel_fill_kernel<kModeSel><<<grid, kBlock, hist_smem, st>>>(R, counts, list_base, entries);
-  else if (a.mode == kModeSwa) sel_fill_kernel<kModeSwa><<<grid, kBlock, hist_smem, st>>>(R, counts, list_base, entries);
-  else sel_fill_kernel<kModeCmp><<<grid, kBlock, hist_smem, st>>>(R, counts, list_base, entries);
+  const dim3 grid((a.N + kIndexQueries - 1) / kIndexQueries, a.B, a.Hkv);
+  const size_t hist_smem = (size_t)p.nkb * sizeof(int);   // at most 32 KB
+  sel_clear_kernel<<<(p.nlists + 255) / 256, 256, 0, st>>>(totals, p.nlists);
+  if (a.mode == kModeSel) sel_count_kernel<kModeSel><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, bits, p.words);
+  else if (a.mode == kModeSwa) sel_count_kernel<kModeSwa><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, bits, p.words);
+  else sel_count_kernel<kModeCmp><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, bits, p.words);
+  sel_items_kernel<<<1, 1024, 0, st>>>(totals, list_base, cursors, items, num_items, p.nlists, p.QT, index_tag(a, p));
+  if (a.mode == kModeSel) sel_fill_kernel<kModeSel><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, list_base, cursors, entries, p.QT);
+  else if (a.mode == kModeSwa) sel_fill_kernel<kModeSwa><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, list_base, cursors, entries, p.QT);
+  else sel_fill_kernel<kModeCmp><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, list_base, cursors, entries, p.QT);
   CUDA_TRY(cudaGetLastError());
-  count_launches(4);   // histogram, scan, items, fill
+  count_launches(4);   // clear, count, items, fill
   return NSA_OK;
 }
 
-static void fill_params(SelParams& P, const SelProblem& a, const SelPlan& p, uint8_t* ws, const uint8_t* ix = nullptr) {
-  if (ix == nullptr) ix = ws;   // the index lives in the work buffer unless the caller kept the forward's
+// The word the kernels report through: the caller's accumulator, or the first word of the work buffer, cleared here.
+static int prepare_status(const SelProblem& a, const SelPlan& p, uint8_t* ws, cudaStream_t st) {
+  if (a.status == nullptr) CUDA_TRY(cudaMemsetAsync(ws + p.off_status, 0, 4, st));
+  return NSA_OK;
+}
+
+// Where the index is: the caller's (kept from an earlier call, or a buffer of its own to build it into), else the
+// leading part of the work buffer.
+static int prepare_index(const SelProblem& a, const SelPlan& p, uint8_t* ws, const uint8_t** ix, cudaStream_t st) {
+  if (a.index != nullptr) {
+    if (a.index_bytes != p.index_bytes) return fail(NSA_ERR_WORKSPACE, "index: not the size the matching *_index_bytes reports");
+    *ix = static_cast<const uint8_t*>(a.index);
+    return NSA_OK;
+  }
+  uint8_t* build = ws;
+  if (a.index_out != nullptr) {
+    if (a.index_out_bytes != p.index_bytes) return fail(NSA_ERR_WORKSPACE, "index_out: not the size the matching *_index_bytes reports");
+    build = static_cast<uint8_t*>(a.index_out);
+  }
+  *ix = build;
+  return build_index(a, p, build, st);
+}
+
+static void fill_params(SelParams& P, const SelProblem& a, const SelPlan& p, uint8_t* ws, const uint8_t* ix) {
   memset(&P, 0, sizeof(P));
   P.q = (const __nv_bfloat16*)a.q.ptr; P.q_sb = a.q.stride_b; P.q_sh = a.q.stride_h; P.q_sn = a.q.stride_n;
   P.out = (__nv_bfloat16*)a.out.ptr; P.o_sb = a.out.stride_b; P.o_sh = a.out.stride_h; P.o_sn = a.out.stride_n;
@@ -2044,7 +2103,9 @@ static void fill_params(SelParams& P, const SelProblem& a, const SelPlan& p, uin
   P.items = reinterpret_cast<const int4*>(ix + p.off_items);
   P.num_items = reinterpret_cast<const int*>(ix + p.off_num_items);
   P.index_tag = index_tag(a, p);
-  P.status = reinterpret_cast<int*>(ws + p.off_status);
+  P.bits = reinterpret_cast<const uint32_t*>(ix + p.off_bits);
+  P.words = p.words;
+  P.status = a.status != nullptr ? a.status : reinterpret_cast<int*>(ws + p.off_status);
   P.lse = a.lse;
   P.B = a.B; P.Hq = a.Hq; P.Hkv = a.Hkv; P.N = a.N; P.Nk = a.Nk; P.G = p.G; P.nsel = a.nsel; P.nfb = p.nkb;
   P.ns = p.ns;
@@ -2072,10 +2133,11 @@ static int run_fwd(const SelProblem& a, const SelPlan& p, uint8_t* ws, cudaStrea
   if (rc != NSA_OK) return rc;
   rc = make_kv_map(&tmV, a.v, a.B, a.Hkv, a.Nk, D);
   if (rc != NSA_OK) return rc;
+  rc = prepare_status(a, p, ws, st);
+  if (rc != NSA_OK) return rc;
   if (dense_forward(a)) {
-    CUDA_TRY(cudaMemsetAsync(ws + p.off_status, 0, 256, st));
     SelParams P;
-    fill_params(P, a, p, ws);
+    fill_params(P, a, p, ws, ws);
     const int QT = kRows / p.G;
     const int64_t tiles = (int64_t)a.B * a.Hkv * ((a.N + QT - 1) / QT);
     if (tiles > 0x7fffffffLL) return NSA_ERR_UNSUPPORTED;
@@ -2112,20 +2174,12 @@ static int run_fwd(const SelProblem& a, const SelPlan& p, uint8_t* ws, cudaStrea
     return NSA_OK;
   }
   const uint8_t* ix = nullptr;
-  if (a.index != nullptr) {   // the caller kept the index of an earlier forward over the same selection
-    if (a.index_bytes != p.index_bytes) return fail(NSA_ERR_WORKSPACE, "index: not the size nsa_sel_index_bytes reports");
-    ix = static_cast<const uint8_t*>(a.index);
-    CUDA_TRY(cudaMemsetAsync(ws + p.off_status, 0, 256, st));
-  } else {
-    rc = build_index(a, p, ws, st);
-    if (rc != NSA_OK) return rc;
-  }
+  rc = prepare_index(a, p, ws, &ix, st);
+  if (rc != NSA_OK) return rc;
   SelParams P;
   fill_params(P, a, p, ws, ix);
   P.partial = reinterpret_cast<__nv_bfloat16*>(ws + p.off_partial);
   P.stats = reinterpret_cast<float2*>(ws + p.off_stats);
-  // a slot that no list holds keeps (0, 0): the merge reads the statistics of every slot and skips those
-  CUDA_TRY(cudaMemsetAsync(P.stats, 0, (size_t)a.B * a.Hq * a.N * p.ns * sizeof(float2), st));
   constexpr int NC = D / 64;
   const int smem = 1024 + NC * (16384 + 8192 + 8192) + kRows * (D * 2 + 16);
   const int per_sm = D == 64 ? 4 : 2;
@@ -2151,15 +2205,11 @@ static int run_bwd(const SelProblem& a, const SelPlan& p, uint8_t* ws, cudaStrea
   if (rc != NSA_OK) return rc;
   rc = make_kv_map(&tmV, a.v, a.B, a.Hkv, a.Nk, D);
   if (rc != NSA_OK) return rc;
+  rc = prepare_status(a, p, ws, st);
+  if (rc != NSA_OK) return rc;
   const uint8_t* ix = nullptr;
-  if (a.index != nullptr) {
-    if (a.index_bytes != p.index_bytes) return fail(NSA_ERR_WORKSPACE, "index: not the size nsa_sel_index_bytes reports");
-    ix = static_cast<const uint8_t*>(a.index);
-    CUDA_TRY(cudaMemsetAsync(ws + p.off_status, 0, 256, st));
-  } else {
-    rc = build_index(a, p, ws, st);
-    if (rc != NSA_OK) return rc;
-  }
+  rc = prepare_index(a, p, ws, &ix, st);
+  if (rc != NSA_OK) return rc;
   SelParams P;
   fill_params(P, a, p, ws, ix);
   P.dout = (const __nv_bfloat16*)a.dout.ptr; P.do_sb = a.dout.stride_b; P.do_sh = a.dout.stride_h; P.do_sn = a.dout.stride_n;
@@ -2206,7 +2256,7 @@ static bool sel_problem(SelProblem& x, const nsa_sel_fwd_args& a) {
   x.q = a.q; x.k = a.k; x.v = a.v; x.out = a.out; x.idx = a.idx; x.mask = a.mask; x.lse = a.lse;
   x.workspace = a.workspace; x.workspace_bytes = a.workspace_bytes;
   x.B = a.batch; x.Hq = a.q_heads; x.Hkv = a.kv_heads; x.N = a.seq; x.Nk = a.seq; x.D = a.dim_head;
-  x.nsel = a.nsel; x.diag = a.diag; x.mode = kModeSel; x.scale = a.scale;
+  x.nsel = a.nsel; x.diag = a.diag; x.mode = kModeSel; x.scale = a.scale; x.status = a.status;
   return supported(x);
 }
 
@@ -2216,7 +2266,7 @@ static bool swa_problem(SelProblem& x, const nsa_swa_fwd_args& a) {
   x.q = a.q; x.k = a.k; x.v = a.v; x.out = a.out; x.lse = a.lse;
   x.workspace = a.workspace; x.workspace_bytes = a.workspace_bytes;
   x.B = a.batch; x.Hq = a.q_heads; x.Hkv = a.kv_heads; x.N = a.seq; x.Nk = a.seq; x.D = a.dim_head;
-  x.mode = kModeSwa; x.window = a.window; x.scale = a.scale;
+  x.mode = kModeSwa; x.window = a.window; x.scale = a.scale; x.status = a.status;
   return supported(x);
 }
 
@@ -2227,7 +2277,7 @@ static bool cmp_problem(SelProblem& x, const nsa_cmp_fwd_args& a) {
   x.workspace = a.workspace; x.workspace_bytes = a.workspace_bytes;
   x.B = a.batch; x.Hq = a.q_heads; x.Hkv = a.kv_heads; x.N = a.seq; x.Nk = a.num_mem + a.ncb; x.D = a.dim_head;
   x.mode = kModeCmp; x.stride = a.stride; x.num_mem = a.num_mem; x.ncb = a.ncb; x.round_bf16 = 1;
-  x.importance = a.importance; x.scale = a.scale;
+  x.importance = a.importance; x.scale = a.scale; x.status = a.status;
   x.pooled = static_cast<__nv_bfloat16*>(a.pooled); x.cpf = a.pool;
   return supported(x);
 }
@@ -2284,6 +2334,7 @@ int sm100_sel_fwd(const nsa_sel_fwd_args& a, cudaStream_t st) {
   SelProblem x;
   if (!sel_problem(x, a)) return NSA_ERR_UNSUPPORTED;
   x.index = a.index; x.index_bytes = a.index_bytes;
+  x.index_out = a.index_out; x.index_out_bytes = a.index_out_bytes;
   return problem_fwd(x, st);
 }
 int sm100_sel_fwd_combine(const nsa_sel_fwd_args& a, const CombineParams& c, const GatherTargets& t, cudaStream_t st) {
@@ -2291,6 +2342,7 @@ int sm100_sel_fwd_combine(const nsa_sel_fwd_args& a, const CombineParams& c, con
   if (!sel_problem(x, a)) return NSA_ERR_UNSUPPORTED;
   if (c.batch != x.B || c.q_heads != x.Hq || c.seq != x.N || c.d != x.D) return NSA_ERR_UNSUPPORTED;
   x.index = a.index; x.index_bytes = a.index_bytes;
+  x.index_out = a.index_out; x.index_out_bytes = a.index_out_bytes;
   x.fuse_combine = &c; x.fuse_targets = &t;
   return problem_fwd(x, st);
 }
@@ -2422,6 +2474,7 @@ static int static_scratch(unsigned char** out) {
 int sm100_sel_fwd_static(const nsa_sel_fwd_args& a, cudaStream_t st) {
   SelProblem x;
   if (!sel_problem(x, a)) return fail(NSA_ERR_UNSUPPORTED, "nsa_sel_fwd_static: shape outside the tensor-core family (bf16, block 64, dim_head 64/128, shared selection, own block included)");
+  x.status = nullptr;   // the area's own first word, see sm100_sel_static_status
   const SelPlan p = make_plan(x, false);
   if (p.total_bytes > kStaticScratchBytes) {
     static thread_local char msg[160];

@@ -28,13 +28,13 @@ def _sel_args(q, k, v, out, idx, mask, lse, block, diag, impl, scale):
     return L.SelFwdArgs(q=L.t4(q), k=L.t4(k), v=L.t4(v), out=L.t4(out), idx=L.ptr(idx), mask=L.ptr(mask),
                         lse=L.ptr(lse), batch=b, q_heads=hq, kv_heads=hkv, sel_heads=hs, seq=n, dim_head=d,
                         block=block, nsel=nsel, diag=diag, dtype=L.dtype_code(q), impl=impl, scale=scale,
-                        workspace=None, workspace_bytes=0)
+                        workspace=None, workspace_bytes=0, status=_status_word(q.device))
 
 
 # Device status of the tensor-core kernels.  Every such kernel reports through the first word of its work buffer:
 # 0 = fine, 1 = a bounded wait ran out (results invalid), 2 = it was handed an index built for another problem.  The
-# words are folded, in stream order, into one int32 per device (bitwise or), so nothing is lost however many kernels
-# run between two checks.  The autograd engine calls the backward functions from its own thread: one lock guards the
+# operators hand the kernels one int32 per device to OR into instead (`status`), so nothing is lost however many
+# kernels run between two checks, and nothing is launched to collect it.  The autograd engine calls the backward functions from its own thread: one lock guards the
 # tables below.
 _state_lock = threading.Lock()
 _status_acc = {}      # device index -> int32[1] device tensor
@@ -53,16 +53,26 @@ def _with_workspace(args, backward, device, sizer='nsa_sel_workspace_bytes'):
     return ws
 
 
+def _status_tensor(device):
+    """The device's accumulator.  The kernels OR into it directly (`status` in the argument structs)."""
+    key = device.index
+    acc = _status_acc.get(key)
+    if acc is None:
+        with _state_lock:
+            acc = _status_acc.get(key)
+            if acc is None:
+                acc = _status_acc[key] = torch.zeros(1, dtype=torch.int32, device=device)
+    return acc
+
+
+def _status_word(device):
+    return _status_tensor(device).data_ptr()
+
+
 def _keep_status(ws):
-    """Fold the status word of a work buffer into the device's accumulator (one tiny stream-ordered kernel)."""
-    if ws is None:
-        return
-    key = ws.device.index
-    with _state_lock:
-        acc = _status_acc.get(key)
-        if acc is None:
-            acc = _status_acc[key] = torch.zeros(1, dtype=torch.int32, device=ws.device)
-    acc.bitwise_or_(ws[:4].view(torch.int32))
+    """Fold the status word of a work buffer, for a call that reported there, into the device's accumulator."""
+    if ws is not None:
+        _status_tensor(ws.device).bitwise_or_(ws[:4].view(torch.int32))
 
 
 def _raise_for(code):
@@ -199,68 +209,36 @@ class SelectedAttention(Function):
 
     @staticmethod
     def forward(ctx, q, k, v, idx, mask, slot_scale, block, diag, impl, index_cache=None):
-        L.require_cuda(q, k, v, idx, mask)
-        lib = L.load()
-        q, k, v = L.rowwise(q), L.rowwise(k), L.rowwise(v)
-        if idx is not None:
-            idx = idx.to(torch.int64).contiguous()
-            mask = mask.to(torch.bool).contiguous().view(torch.uint8)
-        b, hq, n, d = q.shape
-        out = _empty_like_rows(q)
-        lse = torch.empty(b, hq, n, dtype=torch.float32, device=q.device)
-        scale = d ** -0.5
-        with torch.cuda.device(q.device):
-            args = _sel_args(q, k, v, out, idx, mask, lse, block, diag, impl, scale)
-            ws = _with_workspace(args, False, q.device)
-            # `index_cache`: a dict the caller owns while it calls several times with the SAME idx and mask (runs of
-            # query heads of one KV head); the first call of a shape leaves its index there, the later ones take it
+        L.require_cuda(q)
+        scale = q.shape[-1] ** -0.5
+        # `index_cache`: a dict the caller owns while it calls several times with the SAME idx and mask (runs of
+        # query heads of one KV head); the first call of a shape leaves its index there, the later ones take it
+        shared = None
+        if index_cache is not None:
             cache_key = (tuple(q.shape), tuple(k.shape), None if idx is None else tuple(idx.shape), block, diag, impl)
-            shared = index_cache.get(cache_key) if index_cache is not None else None
-            if shared is not None:
-                args.index, args.index_bytes = shared.data_ptr(), shared.numel()
-            L.check(lib.nsa_sel_fwd(C.byref(args), L.stream_of(q)))
-            # the index of which queries attend which key block: a few MB the backward need not rebuild
-            keep = ws is not None and ((REUSE_INDEX and any(ctx.needs_input_grad[:3])) or
-                                       (index_cache is not None and shared is None))
-            index_bytes = int(lib.nsa_sel_index_bytes(C.byref(args))) if keep else 0
-        ctx.index = shared if shared is not None else (ws[:index_bytes].clone() if index_bytes > 0 else None)
+            shared = index_cache.get(cache_key)
+        # the index of which queries attend which key block: a few MB the backward need not rebuild
+        keep = index_cache is not None or (REUSE_INDEX and any(ctx.needs_input_grad[:3]))
+        q, k, v, idx, mask, out, lse, ctx.index = L.host().sel_forward(
+            q, k, v, idx, mask, block, diag, impl, scale, _status_word(q.device), shared, keep)
         if index_cache is not None and shared is None and ctx.index is not None:
             index_cache[cache_key] = ctx.index
-        _keep_status(ws)
-        del ws
         ctx.save_for_backward(q, k, v, idx, mask, out, lse)
         ctx.cfg = (block, diag, impl, scale, None if slot_scale is None else slot_scale.dtype)
         ctx.mark_non_differentiable(lse)
+        ctx.set_materialize_grads(False)
         return out, lse
 
     @staticmethod
     def backward(ctx, dout, _dlse):
+        if dout is None:
+            return (None,) * 10
         q, k, v, idx, mask, out, lse = ctx.saved_tensors
         block, diag, impl, scale, slot_dtype = ctx.cfg
-        want_slot_grads = slot_dtype is not None
-        lib = L.load()
-        delta = _handed_over_delta(dout, lse.shape)
-        dout = L.rowwise(dout)
-        dk = torch.empty(k.shape, dtype=torch.float32, device=q.device)
-        dv = torch.empty(v.shape, dtype=torch.float32, device=q.device)
-        slot = torch.zeros(idx.shape, dtype=torch.float32, device=q.device) if want_slot_grads else None
-        with torch.cuda.device(q.device):
-            fwd = _sel_args(q, k, v, out, idx, mask, lse, block, diag, impl, scale)
-            ws = _with_workspace(fwd, True, q.device)
-            index = ctx.index
-
-            def make_args(direct):
-                dq, dq_out = _dq_buffers(lib, 'nsa_sel_bwd_stores_dq', fwd, q, need_fp32=not direct)
-                return L.SelBwdArgs(fwd=fwd, dout=L.t4(dout), dq=L.ptr(dq), dk=L.ptr(dk), dv=L.ptr(dv),
-                                    slot_grads=L.ptr(slot), index=L.ptr(index),
-                                    index_bytes=0 if index is None else index.numel(),
-                                    dq_out=L.t4(dq_out) if dq_out is not None else L.Tensor4(),
-                                    delta=L.ptr(delta)), dq, dq_out
-            dq = _call_bwd(lib.nsa_sel_bwd, make_args, q, L.stream_of(q))
-        _keep_status(ws)
-        del ws
-        return (dq, dk.to(k.dtype), dv.to(v.dtype), None, None,
-                None if slot is None else slot.to(slot_dtype), None, None, None, None)
+        dq, dk, dv, slots = L.host().sel_backward(
+            q, k, v, idx, mask, out, lse, dout, _handed_over_delta(dout, lse.shape), ctx.index, block, diag, impl, scale,
+            _status_word(q.device), slot_dtype is not None)
+        return dq, dk, dv, None, None, None if slots is None else slots.to(slot_dtype), None, None, None, None
 
 
 def native_sparse_attend(fq, fk, fv, block_size, selected_block_indices, fmask, sel_scale=None,
@@ -316,7 +294,7 @@ def _cmp_args(q, ck, cv, out, lse, imp, sel_heads, num_mem, stride, causal, impl
                         batch=b, q_heads=hq, kv_heads=ck.shape[1], sel_heads=sel_heads, seq=n, dim_head=d,
                         num_mem=num_mem, ncb=ck.shape[2] - num_mem, stride=stride, causal=int(causal),
                         dtype=L.dtype_code(q), impl=impl, scale=scale, sentinel=mask_sentinel(q.dtype), workspace=None,
-                        workspace_bytes=0)
+                        workspace_bytes=0, status=_status_word(q.device))
 
 
 class CompressedAttention(Function):
@@ -348,7 +326,6 @@ class CompressedAttention(Function):
                              pool if pooled is not None else 0)
             ws = _with_workspace(args, False, q.device, 'nsa_cmp_workspace_bytes')
             L.check(lib.nsa_cmp_fwd(C.byref(args), L.stream_of(q)))
-            _keep_status(ws)
             del ws
         ctx.save_for_backward(q, ck, cv, out, lse)
         ctx.cfg = (num_mem, stride, causal, sel_heads, impl, scale)
@@ -392,7 +369,6 @@ class CompressedAttention(Function):
                 dq = _call_bwd(lib.nsa_cmp_bwd, make_args, q, L.stream_of(q))
             if index is None:
                 _keep_index(key, ws, int(lib.nsa_cmp_index_bytes(C.byref(fwd))))
-            _keep_status(ws)
             del ws
         return dq, dck.to(ck.dtype), dcv.to(cv.dtype), None, None, None, None, None, None, None
 
@@ -552,7 +528,6 @@ def selected_attend_combine_gather(fq, fk, fv, block_size, idx, fmask, o_cmp, o_
         L.check(rc)
         if index_cache is not None and shared is None:
             index_cache[cache_key] = ws[:int(lib.nsa_sel_index_bytes(C.byref(args)))].clone()
-        _keep_status(ws)
     return True
 
 
@@ -564,7 +539,8 @@ def _swa_args(q, k, v, out, lse, window, causal, impl, scale):
     b, hq, n, d = q.shape
     return L.SwaFwdArgs(q=L.t4(q), k=L.t4(k), v=L.t4(v), out=L.t4(out), lse=L.ptr(lse), batch=b, q_heads=hq,
                         kv_heads=k.shape[1], seq=n, dim_head=d, window=window, causal=int(causal),
-                        dtype=L.dtype_code(q), impl=impl, scale=scale, workspace=None, workspace_bytes=0)
+                        dtype=L.dtype_code(q), impl=impl, scale=scale, workspace=None, workspace_bytes=0,
+                        status=_status_word(q.device))
 
 
 class SlidingAttention(Function):
@@ -581,7 +557,6 @@ class SlidingAttention(Function):
             args = _swa_args(q, k, v, out, lse, window, causal, impl, scale)
             ws = _with_workspace(args, False, q.device, 'nsa_swa_workspace_bytes')
             L.check(lib.nsa_swa_fwd(C.byref(args), L.stream_of(q)))
-            _keep_status(ws)
             del ws
         ctx.save_for_backward(q, k, v, out, lse)
         ctx.cfg = (window, causal, impl, scale)
@@ -611,7 +586,6 @@ class SlidingAttention(Function):
             dq = _call_bwd(lib.nsa_swa_bwd, make_args, q, L.stream_of(q))
             if index is None:
                 _keep_index(key, ws, int(lib.nsa_swa_index_bytes(C.byref(fwd))))
-            _keep_status(ws)
             del ws
         return dq, dk.to(k.dtype), dv.to(v.dtype), None, None, None
 

@@ -623,3 +623,15 @@ def test_selection_from_pooled_input_in_every_kernel_variant(cols, k):
     assert live.any() and torch.equal(idx0[live], idx1[live])
     # slots without a visible block: probability 0 in both; their column is the lowest zero column in both
     assert torch.equal(idx0, idx1)
+
+
+@pytest.mark.parametrize('case', [(1, 2, 1, 127, 64, 1), (2, 4, 2, 129, 64, 2), (1, 4, 1, 2600, 64, 35), (1, 8, 1, 1, 64, 1)])
+def test_index_at_the_edges_of_its_query_blocks_and_slot_words(case):
+    """The index counts and fills 128 queries per block and keeps 32 slots per word of slot bits: lengths around a
+    block, one query, and more slots than a word holds."""
+    b, hq, hkv, n, d, nsel = case
+    q, k, v, idx, mask, up = make_case(b, hq, hkv, n, d, nsel, seed=77)
+    fast = run_gpu(q, k, v, idx, mask, up, 'sm100')
+    slow = run_gpu(q, k, v, idx, mask, up, 'simt')
+    for f, s, w in zip(fast, slow, ('out', 'lse', 'dq', 'dk', 'dv')):
+        assert_close_bf16(f, s, w, roundings=2, rel_to_max=SUM_REL.get(w, 0.0))
