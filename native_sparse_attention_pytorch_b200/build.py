@@ -16,7 +16,7 @@ SOURCES = ['nsa_abi.cu', 'nsa_simt_attend.cu', 'nsa_select.cu', 'nsa_combine.cu'
 
 
 HOST_LIB = os.path.join(HERE, '_nsa_host.so')
-HOST_SOURCES = ['module.cpp', 'selected.cpp']
+HOST_SOURCES = ['module.cpp', 'selected.cpp', 'rooms.cpp', 'decode.cpp']
 
 
 def _newest(*dirs):

@@ -1,0 +1,153 @@
+// One decoding step: of the operator (the attention part) and of the whole layer.
+
+#include <algorithm>
+#include <cmath>
+#include <tuple>
+
+#include "nsa_kernels.h"
+#include "rooms.h"
+
+namespace nsa_host {
+
+static nsa_decode_args decode_args(const void* q, const void* qr, const Tensor& keys, const Tensor& vals, const Tensor& ck,
+                                   const Tensor& cv, const void* mem_k, const void* mem_v, int64_t num_mem, const void* gates,
+                                   void* out, int64_t heads, int64_t stride, int64_t block, int64_t nsel, int64_t window) {
+  nsa_decode_args a = {};
+  a.q = q; a.qr = qr; a.gates = gates; a.out = out; a.mem_k = mem_k; a.mem_v = mem_v;
+  a.keys = t4(keys); a.vals = t4(vals);
+  a.ncb = ck.size(2);
+  if (a.ncb > 0) { a.ck = t4(ck); a.cv = t4(cv); }
+  a.batch = keys.size(0); a.q_heads = heads; a.dim_head = keys.size(3); a.kv_heads = keys.size(1); a.cache_len = keys.size(2);
+  a.num_mem = num_mem; a.stride = stride; a.block = block; a.nsel = nsel; a.window = window;
+  a.dtype = dtype_code(keys); a.scale = 1.f / std::sqrt((float)keys.size(3));
+  return a;
+}
+
+// Attention part of a step on tensors the caller holds
+static Tensor decode_step(Tensor q, Tensor qr, Tensor keys, Tensor vals, Tensor ck, Tensor cv, Tensor mem_k, Tensor mem_v,
+                          Tensor gates, int64_t stride, int64_t block, int64_t nsel, int64_t window) {
+  for (const Tensor* t : {&q, &qr, &keys, &vals, &ck, &cv, &mem_k, &mem_v, &gates}) require_cuda(*t);
+  const c10::cuda::CUDAGuard guard(q.device());
+  const auto dt = q.scalar_type();
+  q = q.contiguous();
+  qr = qr.to(dt).contiguous();
+  gates = gates.to(dt).contiguous();
+  mem_k = mem_k.to(dt).contiguous();
+  mem_v = mem_v.to(dt).contiguous();
+  keys = rowwise(keys.to(dt));
+  vals = rowwise(vals.to(dt));
+  if (ck.size(2) > 0) {
+    ck = rowwise(ck.to(dt));
+    cv = rowwise(cv.to(dt));
+  }
+  Tensor out = at::empty({q.size(0), q.size(1) * q.size(2)}, q.options());
+  const nsa_decode_args a = decode_args(q.data_ptr(), qr.data_ptr(), keys, vals, ck, cv, mem_k.data_ptr(), mem_v.data_ptr(),
+                                        mem_k.size(1), gates.data_ptr(), out.data_ptr(), q.size(1), stride, block, nsel, window);
+  check(nsa_decode_step(&a, stream_of(q)));
+  return out;
+}
+
+// Rows of room behind a cache that has to move: an eighth of it, so that the copies of a long generation add up to a
+// small multiple of the final cache, within bounds that keep short caches and the largest ones sensible.
+static int64_t room_for(int64_t rows) { return std::min<int64_t>(std::max<int64_t>(rows / 8, 64), 2048); }
+
+// Token rows x [B, 1, dim] against the caches.  -> out, keys, vals, the window being filled (keys, values)
+static std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> layer_decode(
+    Tensor x, OptTensor norm_w, double eps, Tensor qkv_w, Tensor gate_w, Tensor gate_b, Tensor out_w, Tensor inv_freq,
+    Tensor mem_kv, Tensor past_k, Tensor past_v, Tensor ck, Tensor cv, Tensor run_k, Tensor run_v, int64_t heads,
+    int64_t stride, int64_t block, int64_t cbs, int64_t nsel, int64_t window) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  void* st = stream_of(x);
+  const int64_t B = x.size(0), dim = x.size(2), hkv = past_k.size(1), d = past_k.size(3), rows = 3 * heads;
+  const int dt = dtype_code(x);
+  x = rowwise(x);
+  ck = rowwise(ck);
+  cv = rowwise(cv);
+  GrownPair cache = Rooms::instance().extend(past_k, past_v, room_for(past_k.size(2)));
+  GrownPair run = Rooms::instance().extend(run_k, run_v, 4 * cbs);
+  // the qkv rows, the merged rows and the gates in one buffer of 16-byte aligned parts
+  auto up = [](int64_t n) { return (n + 7) / 8 * 8; };
+  const int64_t features = qkv_w.size(0), el = x.element_size();
+  const int64_t at_merged = up(B * features), at_gates = at_merged + up(B * heads * d);
+  Tensor work = at::empty({at_gates + B * rows}, x.options());
+  uint8_t* const w = static_cast<uint8_t*>(work.data_ptr());
+  void *qkv = w, *merged = w + at_merged * el, *gates = w + at_gates * el;
+  Tensor qkv_rows, gate_rows;
+  if (nsa::project_serves(B, dim, dt)) {
+    nsa::ProjectParams p = {};
+    p.x[0] = x.data_ptr(); p.x_sb = x.stride(0);
+    p.norm_w = norm_w.has_value() ? norm_w->data_ptr() : nullptr; p.eps = (float)eps;
+    p.w[0] = qkv_w.data_ptr(); p.gate_w = gate_w.data_ptr(); p.gate_b = gate_b.data_ptr();
+    p.y[0] = qkv; p.y_sb = features; p.gates = gates; p.rows = B; p.heads = p.sets = 1; p.dim = dim; p.features = features;
+    p.gates_n = rows;
+    check(nsa::launch_project(p, dt, (cudaStream_t)st));
+  } else {
+    const Tensor xn = norm_w.has_value() ? at::rms_norm(x, {dim}, norm_w, eps) : x;
+    qkv_rows = at::linear(xn, qkv_w);
+    gate_rows = at::sigmoid(at::linear(xn, gate_w, gate_b));
+    qkv = qkv_rows.data_ptr();
+    gates = gate_rows.data_ptr();
+  }
+  const uint8_t* mem = static_cast<const uint8_t*>(mem_kv.data_ptr());
+  const nsa_decode_args a = decode_args(nullptr, nullptr, cache.k, cache.v, ck, cv, mem, mem + mem_kv.numel() / 2 * el,
+                                        mem_kv.size(2), gates, merged, heads, stride, block, nsel, window);
+  nsa::DecodeParams p;
+  check(nsa::fill_decode(p, a));
+  p.qkv = qkv; p.inv_freq = ptr<float>(inv_freq);
+  p.new_keys = cache.k_buf; p.new_vals = cache.v_buf; p.c_sb = cache.k.stride(0); p.c_sh = cache.k.stride(1); p.row = cache.row;
+  p.run_k = run.k_buf; p.run_v = run.v_buf; p.r_sb = run.k.stride(0); p.r_sh = run.k.stride(1); p.run_row = run.row;
+  check(nsa::launch_decode(p, dt, (cudaStream_t)st));
+  Tensor out;
+  if (nsa::project_serves(B, heads * d, dt)) {
+    out = at::empty({B, 1, dim}, x.options());
+    nsa::ProjectParams o = {};
+    o.x[0] = merged; o.x_sb = heads * d; o.w[0] = out_w.data_ptr(); o.y[0] = out.data_ptr(); o.y_sb = dim;
+    o.rows = B; o.heads = o.sets = 1; o.dim = heads * d; o.features = dim;
+    check(nsa::launch_project(o, dt, (cudaStream_t)st));
+  } else {
+    out = at::linear(at::as_strided(work, {B, heads * d}, {heads * d, 1}, at_merged), out_w).unsqueeze(1);
+  }
+  return {out, cache.k, cache.v, run.k, run.v};
+}
+
+// The windows being filled (keys, values: [B, H, cbs, d]) have filled up: the two layers of either compress network, each
+// one launch for both, and the compressed row appended to ck / cv.  -> ck, cv, or nothing where these kernels do not serve.
+static std::optional<std::tuple<Tensor, Tensor>> compress_filled(Tensor run_k, Tensor run_v, Tensor pos_k, Tensor pos_v,
+                                                                 Tensor k1, Tensor kb1, Tensor k2, Tensor kb2, Tensor v1,
+                                                                 Tensor vb1, Tensor v2, Tensor vb2, Tensor ck, Tensor cv) {
+  const int64_t B = run_k.size(0), H = run_k.size(1), d = run_k.size(3), width = run_k.size(2) * d, hidden = k1.size(0);
+  const int dt = dtype_code(run_k);
+  if (!nsa::project_serves(B * H, width, dt) || !nsa::project_serves(B * H, hidden, dt) || run_k.stride(2) != d ||
+      run_k.strides() != run_v.strides() || run_k.stride(3) != 1 || run_v.stride(3) != 1)
+    return std::nullopt;
+  const c10::cuda::CUDAGuard guard(run_k.device());
+  cudaStream_t st = (cudaStream_t)stream_of(run_k);
+  GrownPair grown = Rooms::instance().extend(ck, cv, room_for(ck.size(2)));
+  Tensor h = at::empty({2, B * H, hidden}, run_k.options());
+  nsa::ProjectParams p = {};
+  p.x[0] = run_k.data_ptr(); p.x[1] = run_v.data_ptr(); p.x_sb = run_k.stride(0); p.x_sh = run_k.stride(1);
+  p.add[0] = pos_k.data_ptr(); p.add[1] = pos_v.data_ptr();
+  p.w[0] = k1.data_ptr(); p.w[1] = v1.data_ptr(); p.bias[0] = kb1.data_ptr(); p.bias[1] = vb1.data_ptr();
+  p.y[0] = h.data_ptr(); p.y[1] = static_cast<uint8_t*>(h.data_ptr()) + B * H * hidden * h.element_size();
+  p.y_sb = H * hidden; p.y_sh = hidden;
+  p.rows = B * H; p.heads = H; p.sets = 2; p.dim = width; p.features = hidden; p.relu = 1;
+  check(nsa::launch_project(p, dt, st));
+  nsa::ProjectParams o = {};
+  o.x[0] = p.y[0]; o.x[1] = p.y[1]; o.x_sb = p.y_sb; o.x_sh = p.y_sh;
+  o.w[0] = k2.data_ptr(); o.w[1] = v2.data_ptr(); o.bias[0] = kb2.data_ptr(); o.bias[1] = vb2.data_ptr();
+  const int64_t at = grown.row * d * run_k.element_size();
+  o.y[0] = static_cast<uint8_t*>(grown.k_buf) + at; o.y[1] = static_cast<uint8_t*>(grown.v_buf) + at;
+  o.y_sb = grown.k.stride(0); o.y_sh = grown.k.stride(1);
+  o.rows = B * H; o.heads = H; o.sets = 2; o.dim = hidden; o.features = d;
+  check(nsa::launch_project(o, dt, st));
+  return std::make_tuple(grown.k, grown.v);
+}
+
+void bind_decode(pybind11::module_& m) {
+  namespace py = pybind11;
+  m.def("decode_step", &decode_step, py::call_guard<py::gil_scoped_release>());
+  m.def("compress_filled", &compress_filled, py::call_guard<py::gil_scoped_release>());
+  m.def("layer_decode", &layer_decode, py::call_guard<py::gil_scoped_release>());
+}
+
+}  // namespace nsa_host

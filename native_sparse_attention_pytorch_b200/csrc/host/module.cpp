@@ -16,4 +16,5 @@ PYBIND11_MODULE(_nsa_host, m) {
     }
   });
   nsa_host::bind_selected(m);
+  nsa_host::bind_decode(m);
 }

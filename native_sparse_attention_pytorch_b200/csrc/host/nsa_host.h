@@ -71,5 +71,6 @@ inline void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream
 Tensor empty_in_order_of(const Tensor& t);
 
 void bind_selected(pybind11::module_& m);
+void bind_decode(pybind11::module_& m);
 
 }  // namespace nsa_host

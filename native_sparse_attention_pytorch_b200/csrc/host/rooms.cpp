@@ -1,0 +1,72 @@
+#include "rooms.h"
+
+#include <ATen/core/LegacyTypeDispatch.h>
+
+namespace nsa_host {
+
+Rooms& Rooms::instance() {
+  static Rooms* r = new Rooms;   // outlives the interpreter's tensors
+  return *r;
+}
+
+static Tensor rows_of(const Tensor& buf, int64_t first, int64_t rows) {
+  return at::as_strided(buf, {buf.size(0), buf.size(1), rows, buf.size(3)}, buf.strides(), first * buf.size(3));
+}
+
+GrownPair Rooms::fresh(const Tensor& like, int64_t batch, int64_t heads, int64_t rows, int64_t room, int64_t d) {
+  GrownPair g;
+  const Tensor k_buf = at::empty({batch, heads, rows + room, d}, like.options());
+  const Tensor v_buf = at::empty({batch, heads, rows + room, d}, like.options());
+  g.k = rows_of(k_buf, 0, rows);
+  g.v = rows_of(v_buf, 0, rows);
+  g.k_buf = k_buf.data_ptr();
+  g.v_buf = v_buf.data_ptr();
+  g.row = rows - 1;
+  std::lock_guard<std::mutex> lock(mutex_);
+  if (entries_.size() >= 256)      // forget the buffers that are gone
+    for (auto it = entries_.begin(); it != entries_.end();) it = it->second.k.expired() ? entries_.erase(it) : std::next(it);
+  const c10::StorageImpl* key = k_buf.storage().unsafeGetStorageImpl();
+  auto weak = [](const Tensor& t) {
+    return c10::weak_intrusive_ptr<c10::StorageImpl>(
+        c10::intrusive_ptr<c10::StorageImpl>::reclaim_copy(t.storage().unsafeGetStorageImpl()));
+  };
+  entries_.erase(key);             // the address of a storage that is gone may come back
+  entries_.emplace(key, Entry{weak(k_buf), weak(v_buf), rows});
+  return g;
+}
+
+GrownPair Rooms::extend(const Tensor& k, const Tensor& v, int64_t room) {
+  at::AutoDispatchBelowADInplaceOrView no_view_tracking;
+  const int64_t B = k.size(0), H = k.size(1), rows = k.size(2), d = k.size(3);
+  const c10::StorageImpl* ks = k.storage().unsafeGetStorageImpl();
+  const c10::StorageImpl* vs = v.storage().unsafeGetStorageImpl();
+  {
+    std::lock_guard<std::mutex> lock(mutex_);
+    auto it = entries_.find(ks);
+    if (it != entries_.end() && !it->second.k.expired() && it->second.v._unsafe_get_target() == vs && k.strides() == v.strides() &&
+        k.storage_offset() == v.storage_offset() && k.sizes() == v.sizes() && k.stride(3) == 1 && k.stride(2) == d &&
+        k.stride(0) == k.stride(1) * H && k.scalar_type() == v.scalar_type()) {
+      const int64_t capacity = k.stride(1) / d, first = k.storage_offset() / d, end = first + rows;
+      // the views of a continuation that was dropped are gone: nothing else is on these buffers
+      if (it->second.used > end && k.storage().use_count() == 1 && v.storage().use_count() == 1) it->second.used = end;
+      if (it->second.used == end && end < capacity && (int64_t)k.storage().nbytes() == B * H * capacity * d * k.element_size()) {
+        it->second.used = end + 1;
+        GrownPair g;
+        g.k_buf = k.storage().mutable_data();
+        g.v_buf = v.storage().mutable_data();
+        g.k = rows_of(k, first, rows + 1);
+        g.v = rows_of(v, first, rows + 1);
+        g.row = end;
+        return g;
+      }
+    }
+  }
+  GrownPair g = fresh(k, B, H, rows + 1, room, d);
+  if (rows > 0) {
+    rows_of(g.k, 0, rows).copy_(k);
+    rows_of(g.v, 0, rows).copy_(v);
+  }
+  return g;
+}
+
+}  // namespace nsa_host

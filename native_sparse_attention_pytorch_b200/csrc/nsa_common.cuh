@@ -7,6 +7,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "nsa_b200.h"
 
 namespace nsa {
@@ -92,6 +94,23 @@ __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFullMask, v, o);
   return v;
+}
+
+// Lets a kernel use all the dynamic shared memory its static part leaves, once per kernel and device (an attribute call
+// per launch is host time).  Always the same value, so threads that race here agree.
+constexpr int kMaxSharedBytes = 232448;
+template <auto Kernel>
+inline cudaError_t allow_shared_memory() {
+  static std::atomic<bool> done[64];
+  int dev = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err != cudaSuccess || (dev < 64 && done[dev].load(std::memory_order_acquire))) return err;
+  cudaFuncAttributes at;
+  err = cudaFuncGetAttributes(&at, Kernel);
+  if (err == cudaSuccess)
+    err = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSharedBytes - (int)at.sharedSizeBytes);
+  if (err == cudaSuccess && dev < 64) done[dev].store(true, std::memory_order_release);
+  return err;
 }
 
 }  // namespace nsa

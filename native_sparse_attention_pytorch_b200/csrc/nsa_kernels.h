@@ -108,6 +108,28 @@ struct DecodeParams {
   void* out;                     // [B, Hq * d]
   int batch, q_heads, kv_heads, d, T, ncb, num_mem, stride, block, nsel, window;
   float scale;
+  // instead of q and qr: the token rows of the qkv projection [B, (Hq + 2 Hkv) d]; the key (rotated) and the value are
+  // then appended at row `row` of the caches (which `keys` / `vals` look into) and, un-rotated, at row `run_row` of the
+  // window that is being filled
+  const void* qkv;
+  const float* inv_freq;         // [d / 2]
+  void *new_keys, *new_vals, *run_k, *run_v;
+  int64_t c_sb, c_sh, r_sb, r_sh;
+  int row, run_row;
+};
+
+// Projection of up to 16 rows (see nsa_decode.cu): y = f(x) w^T (+ bias) (ReLU), f = RMS norm, addition of `add`, or
+// nothing; for two independent sets at once where `sets` is 2 (keys and values).  Row t of x is at
+// x + (t / heads) x_sb + (t % heads) x_sh, of y likewise; `add` has one row per head.  Behind the rows of the first set:
+// gates = sigmoid(f(x) gate_w^T + gate_b).
+struct ProjectParams {
+  const void *x[2], *w[2], *bias[2], *add[2];   // w [features, dim], bias [features] or NULL, add [heads, dim] or NULL
+  void* y[2];
+  const void *norm_w, *gate_w, *gate_b;         // [dim] or NULL, [gates_n, dim], [gates_n]
+  void* gates;                                  // [rows, gates_n]
+  int64_t x_sb, x_sh, y_sb, y_sh;
+  int rows, heads, sets, dim, features, gates_n, relu;
+  float eps;
 };
 
 int fail(int code, const char* msg);
@@ -124,6 +146,9 @@ int launch_windows(const WindowParams& P, int dtype, bool backward, cudaStream_t
 int launch_rmsnorm(const NormParams& P, int dtype, bool backward, cudaStream_t stream);
 int launch_combine_gather(const CombineParams& P, const GatherTargets& Gt, int dtype, cudaStream_t stream);
 int launch_decode(const DecodeParams& P, int dtype, cudaStream_t stream);
+int fill_decode(DecodeParams& P, const nsa_decode_args& a);   // checks the arguments; q and qr may be NULL
+bool project_serves(int batch, int dim, int dtype);
+int launch_project(const ProjectParams& P, int dtype, cudaStream_t stream);
 
 // Tensor-core family for the selected-block branch.  Each returns
 // NSA_ERR_UNSUPPORTED (without touching the error message state of a later

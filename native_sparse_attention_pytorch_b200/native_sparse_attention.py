@@ -15,9 +15,21 @@ import torch.nn.functional as F
 from torch import nn
 from torch.nn import Module
 
+from . import _lib as L
 from . import ops
 from .norm import RMSNorm
-from .rotary import RotaryEmbedding
+from .rotary import RotaryEmbedding, inverse_frequencies
+
+_has_any_global_hook = nn.modules.module._has_any_global_hook
+_F32_EPS = torch.finfo(torch.float32).eps
+_PLAIN = (nn.Parameter, torch.Tensor)
+
+
+def _untouched(module, cls):
+    """`module` is exactly a `cls` that runs its own forward: no subclass, no hooks, no replaced forward."""
+    d = module.__dict__
+    return module.__class__ is cls and not (d['_forward_hooks'] or d['_forward_pre_hooks'] or d['_backward_hooks'] or
+                                            d['_backward_pre_hooks'] or 'forward' in d)
 
 
 class _Windows(Module):
@@ -68,7 +80,8 @@ class SparseAttention(Module):
         self.norm = RMSNorm(dim) if norm else nn.Identity()
         self.rotary_emb = RotaryEmbedding(dim_head)
         self.qkv_split = (dim_head * heads, dim_head * kv_heads, dim_head * kv_heads)
-        self.to_qkv = nn.Linear(dim, sum(self.qkv_split), bias=False)
+        self._qkv_rows = sum(self.qkv_split)
+        self.to_qkv = nn.Linear(dim, self._qkv_rows, bias=False)
 
         self.sliding_window_size = sliding_window_size
 
@@ -112,17 +125,109 @@ class SparseAttention(Module):
 
         self.combine_heads = nn.Linear(dim_head * heads, dim, bias=False)
 
+    def _native_weights(self, x):
+        """The parameters the native layer calls take, or None where the layer has to run module by module: a replaced
+        or hooked submodule, autocast, parameters of another type, dtype or device than the input."""
+        dtype, device, dim = x.dtype, x.device, x.shape[-1]
+        if (dtype is not torch.bfloat16 and dtype is not torch.float32) or x.dim() != 3 or torch.is_autocast_enabled('cuda') or \
+                _has_any_global_hook() or torch.compiler.is_compiling():
+            return None
+        m = self._modules
+        norm, gate, qkv, out = m['norm'], m['to_strategy_combine'], m['to_qkv'], m['combine_heads']
+        gate_linear = gate._modules.get('0')
+        norm_w, eps = None, 0.
+        if _untouched(norm, RMSNorm):
+            norm_w, eps = norm._parameters['weight'], norm.eps
+            if norm_w is None or tuple(norm_w.shape) != (dim,):
+                return None
+            eps = _F32_EPS if eps is None else eps
+        elif not _untouched(norm, nn.Identity):
+            return None
+        if not (_untouched(m['rotary_emb'], RotaryEmbedding) and _untouched(gate, nn.Sequential) and len(gate._modules) == 2 and
+                _untouched(gate._modules['1'], nn.Sigmoid) and _untouched(qkv, nn.Linear) and _untouched(out, nn.Linear) and
+                _untouched(gate_linear, nn.Linear)):
+            return None
+        if qkv._parameters['bias'] is not None or out._parameters['bias'] is not None:
+            return None
+        gate_w = gate_linear._parameters
+        w = (norm_w, qkv._parameters['weight'], gate_w['weight'], gate_w['bias'], out._parameters['weight'],
+             self._parameters['compress_mem_kv'])
+        for p in w:
+            if p is None:
+                if p is norm_w:
+                    continue
+                return None
+            if p.dtype is not dtype or p.device != device or not p.is_contiguous() or p.__class__ not in _PLAIN:
+                return None
+        if w[1].shape != (self._qkv_rows, dim) or w[2].shape != (3 * self.heads, dim) or dim % 8:
+            return None
+        return w, eps
+
     def _split_heads(self, t):
         b, n, _ = t.shape
         return t.view(b, n, -1, self.dim_head).transpose(1, 2)   # a view: the kernels take the strides
+
+    def _default_network(self, name, like):
+        """The parameters (two linear layers) of a compress network that is the default one, as built and of `like`'s
+        type, else None."""
+        net = self._modules[name]
+        m = list(net._modules.values()) if _untouched(net, nn.Sequential) else ()
+        if len(m) != 4 or not (_untouched(m[0], nn.Flatten) and (m[0].start_dim, m[0].end_dim) == (-2, -1) and
+                               _untouched(m[1], nn.Linear) and _untouched(m[2], nn.ReLU) and _untouched(m[3], nn.Linear)):
+            return None
+        w = (m[1]._parameters['weight'], m[1]._parameters['bias'], m[3]._parameters['weight'], m[3]._parameters['bias'])
+        for p in w:
+            if p is None or p.dtype is not like.dtype or p.device != like.device or not p.is_contiguous() or p.__class__ not in _PLAIN:
+                return None
+        width = self.compress_block_size * self.dim_head
+        return w if w[0].shape[1] == width and w[2].shape == (self.dim_head, w[0].shape[0]) else None
+
+    def _compress_filled(self, ck, cv, run_k, run_v, native=False):
+        """The window that was being filled is complete: compress it and keep its overlap with the next one (the step
+        before attended the blocks that existed before this token, as upstream's does)."""
+        grown = None
+        pk, pv = self.k_intrablock_positions, self.v_intrablock_positions
+        if native and pk.dtype is run_k.dtype and pv.dtype is run_k.dtype and pk.is_contiguous() and pv.is_contiguous():
+            k_net, v_net = self._default_network('k_compress', run_k), self._default_network('v_compress', run_k)
+            if k_net is not None and v_net is not None:
+                grown = L.host().compress_filled(run_k, run_v, pk, pv, *k_net, *v_net, ck, cv)
+        if grown is not None:
+            ck, cv = grown
+        else:
+            ck = torch.cat((ck, self.k_compress((run_k + pk)[:, :, None])), dim=-2)
+            cv = torch.cat((cv, self.v_compress((run_v + pv)[:, :, None])), dim=-2)
+        first = run_k.shape[-2] - (self.compress_block_size - self.compress_block_sliding_stride)
+        return ck, cv, run_k[..., first:, :], run_v[..., first:, :]
+
+    def _native_step(self, x, past_k, past_v, ck, cv, run_k, run_v):
+        """The step as three launches (norm with qkv and gate projections, attention with rotary and the append to the
+        caches, output projection) where nothing on it needs a gradient; None where it has to run module by module.  The returned caches are views of
+        buffers with some room behind them (csrc/host/rooms.h)."""
+        if torch.is_grad_enabled() and (x.requires_grad or past_k.requires_grad or past_v.requires_grad or
+                                        any(p.requires_grad for p in self.parameters())):
+            return None
+        d = self.dim_head
+        if x.shape[1] != 1 or d % 8 or d > 128 or self.num_selected_blocks > 32 or self.num_grouped_queries > 16:
+            return None
+        native = self._native_weights(x)
+        if native is None:
+            return None
+        for t in (past_k, past_v, ck, cv, run_k, run_v):
+            if t.dtype is not x.dtype or t.device != x.device or t.__class__ is not torch.Tensor:
+                return None
+        (norm_w, qkv_w, gate_w, gate_b, out_w, mem_kv), eps = native
+        return L.host().layer_decode(
+            x, norm_w, eps, qkv_w, gate_w, gate_b, out_w, inverse_frequencies(d, self.rotary_emb.theta, x.device), mem_kv,
+            past_k, past_v, ck, cv, run_k, run_v, self.heads, self.compress_block_sliding_stride, self.selection_block_size,
+            self.compress_block_size, self.num_selected_blocks, self.sliding_window_size)
 
     def forward_inference(self, inp, cache, return_cache=True):
         """One decoding step (upstream NSA:338-547): `inp` is the newest token [B, 1, dim], `cache` what the previous
         call returned: ((rotated keys, values), ((compressed keys, compressed values), (keys, values of the window
         that is being filled for the next compressed block, un-rotated))).  The attention part -- compressed branch,
         block selection, selected blocks plus the own block, sliding window, gated combine -- is one kernel launch
-        (`ops.decode_step`, all (batch, KV head) units in its grid); the projections, the rotary kernel and the
-        compress network of a window that has just filled up stay tensor operations.  It keeps upstream's behaviour,
+        (`ops.decode_step`, all (batch, KV head) units in its grid), and without gradients the whole step is three
+        launches (`_native_step`).  It keeps upstream's behaviour,
         including that the memory slots are attended only once a compressed block exists."""
         assert self.causal, 'inference only relevant for autoregressive'
         if not self.query_heads_share_selected_kv:
@@ -132,6 +237,14 @@ class SparseAttention(Module):
         b = inp.shape[0]
         h, d = self.heads, self.dim_head
         st, cbs, sel = self.compress_block_sliding_stride, self.compress_block_size, self.selection_block_size
+        native = self._native_step(inp, past_k, past_v, ck, cv, run_k, run_v)
+        if native is not None:
+            out, keys, vals, run_k, run_v = native
+            if not return_cache:
+                return out
+            if run_k.shape[-2] % cbs == 0:
+                ck, cv, run_k, run_v = self._compress_filled(ck, cv, run_k, run_v, native=True)
+            return out, ((keys, vals), ((ck, cv), (run_k, run_v)))
         pos = past_k.shape[-2]                       # position of the new token
         x = self.norm(inp)
         q, k, v = (self._split_heads(t).contiguous() for t in self.to_qkv(x).split(self.qkv_split, dim=-1))
@@ -145,13 +258,8 @@ class SparseAttention(Module):
                                  self.compress_mem_kv[1], gates, stride=st, block=sel,
                                  num_selected=self.num_selected_blocks, window=self.sliding_window_size)
 
-        # the window that was being filled is complete: compress it and keep its overlap with the next one (the step
-        # above attended the blocks that existed before this token, as upstream's does)
         if run_k.shape[-2] % cbs == 0:
-            ck = torch.cat((ck, self.k_compress((run_k + self.k_intrablock_positions)[:, :, None])), dim=-2)
-            cv = torch.cat((cv, self.v_compress((run_v + self.v_intrablock_positions)[:, :, None])), dim=-2)
-            keep = cbs - st
-            run_k, run_v = run_k[..., run_k.shape[-2] - keep:, :], run_v[..., run_v.shape[-2] - keep:, :]
+            ck, cv, run_k, run_v = self._compress_filled(ck, cv, run_k, run_v)
 
         out = self.combine_heads(merged.view(b, 1, h * d))
         if not return_cache:

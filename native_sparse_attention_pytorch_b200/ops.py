@@ -38,6 +38,7 @@ def _sel_args(q, k, v, out, idx, mask, lse, block, diag, impl, scale):
 # tables below.
 _state_lock = threading.Lock()
 _status_acc = {}      # device index -> int32[1] device tensor
+_status_fresh = {}    # device index -> a call has been handed the word since the last poll copied it
 _status_polls = {}    # device index -> (pinned int32[1], event) of the copy issued by the last poll
 
 
@@ -66,6 +67,7 @@ def _status_tensor(device):
 
 
 def _status_word(device):
+    _status_fresh[device.index] = True
     return _status_tensor(device).data_ptr()
 
 
@@ -73,6 +75,7 @@ def _keep_status(ws):
     """Fold the status word of a work buffer, for a call that reported there, into the device's accumulator."""
     if ws is not None:
         _status_tensor(ws.device).bitwise_or_(ws[:4].view(torch.int32))
+        _status_fresh[ws.device.index] = True
 
 
 def _raise_for(code):
@@ -105,14 +108,12 @@ def poll_device_status(device):
     key = torch.device(device).index
     if key is None:
         key = torch.cuda.current_device()
-    with _state_lock:
-        acc = _status_acc.get(key)
-        pending = _status_polls.get(key)
-    if acc is None:
-        return
+    acc, pending = _status_acc.get(key), _status_polls.get(key)
+    if acc is None or not (_status_fresh.get(key) or (pending is not None and pending[2])):
+        return                          # no such kernel since the last copy, and that copy has been read
     if pending is not None:
-        host, event = pending
-        if not event.query():
+        host, event, unread = pending
+        if unread and not event.query():
             return                      # the previous copy is still in flight: look again at the next call
         code = int(host.item())
         if code != 0:
@@ -120,12 +121,17 @@ def poll_device_status(device):
             with _state_lock:
                 _status_polls.pop(key, None)
             _raise_for(code)
+        if not _status_fresh.get(key):
+            with _state_lock:
+                _status_polls[key] = (host, event, False)
+            return
+    _status_fresh[key] = False
     host = pending[0] if pending is not None else torch.zeros(1, dtype=torch.int32).pin_memory()
     host.copy_(acc, non_blocking=True)
-    event = torch.cuda.Event()
+    event = pending[1] if pending is not None else torch.cuda.Event()
     event.record(torch.cuda.current_stream(acc.device))
     with _state_lock:
-        _status_polls[key] = (host, event)
+        _status_polls[key] = (host, event, True)
 
 
 def dim_order(t):
@@ -690,26 +696,7 @@ def decode_step(q, qr, keys, vals, ck, cv, mem_k, mem_v, gates, *, stride, block
     the token; keys, vals [B, Hkv, T, d]: rotated keys and values with the token appended; ck, cv [B, Hkv, ncb, d]:
     the blocks compressed so far (without memory slots, ncb may be 0); mem_k, mem_v [Hkv, M, d]; gates [B, Hq, 3]
     (compressed, selected, sliding).  Returns the merged row [B, Hq * d].  See nsa_decode_step in include/nsa_b200.h."""
-    L.require_cuda(q, qr, keys, vals, ck, cv, mem_k, mem_v, gates)
-    lib = L.load()
-    dt = q.dtype
-    q, qr, gates = q.contiguous(), qr.to(dt).contiguous(), gates.to(dt).contiguous()
-    mem_k, mem_v = mem_k.to(dt).contiguous(), mem_v.to(dt).contiguous()
-    keys, vals = L.rowwise(keys.to(dt)), L.rowwise(vals.to(dt))
-    b, hq, d = q.shape
-    ncb = ck.shape[2]
-    if ncb > 0:
-        ck, cv = L.rowwise(ck.to(dt)), L.rowwise(cv.to(dt))
-    out = torch.empty(b, hq * d, dtype=dt, device=q.device)
-    args = L.DecodeArgs(q=L.ptr(q), qr=L.ptr(qr), keys=L.t4(keys), vals=L.t4(vals),
-                        ck=L.t4(ck) if ncb > 0 else L.Tensor4(), cv=L.t4(cv) if ncb > 0 else L.Tensor4(),
-                        mem_k=L.ptr(mem_k), mem_v=L.ptr(mem_v), gates=L.ptr(gates), out=L.ptr(out), batch=b,
-                        q_heads=hq, kv_heads=keys.shape[1], dim_head=d, cache_len=keys.shape[2], ncb=ncb,
-                        num_mem=mem_k.shape[1], stride=stride, block=block, nsel=num_selected, window=window,
-                        dtype=L.dtype_code(q), scale=d ** -0.5, reserved=0)
-    with torch.cuda.device(q.device):
-        L.check(lib.nsa_decode_step(C.byref(args), L.stream_of(q)))
-    return out
+    return L.host().decode_step(q, qr, keys, vals, ck, cv, mem_k, mem_v, gates, stride, block, num_selected, window)
 
 
 # --------------------------------------------------------------------------

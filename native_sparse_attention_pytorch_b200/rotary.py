@@ -14,14 +14,19 @@ from torch.autograd import Function
 _INV_FREQ = {}
 
 
-def _tables(dim, theta, n, offset, device):
-    """cos / sin of the angles [n, dim/2], always in fp32: the inverse frequencies are rebuilt here instead of being
-    kept as a module buffer, which `module.bfloat16()` would round to 8 bits and so turn positions past a few hundred
-    into wrong angles."""
-    key = (dim, theta, str(device))
+def inverse_frequencies(dim, theta, device):
+    """theta^(-2m/dim), always fp32: kept here instead of as a module buffer, which `module.bfloat16()` would round to
+    8 bits and so turn positions past a few hundred into wrong angles."""
+    key = (dim, theta, device)
     inv_freq = _INV_FREQ.get(key)
     if inv_freq is None:   # computed on the host (as upstream's package does at construction), kept per device
         inv_freq = _INV_FREQ[key] = (theta ** (-torch.arange(0, dim, 2).float() / dim)).to(device)
+    return inv_freq
+
+
+def _tables(dim, theta, n, offset, device):
+    """cos / sin of the angles [n, dim/2] in fp32."""
+    inv_freq = inverse_frequencies(dim, theta, device)
     pos = torch.arange(n, device=device, dtype=torch.float32) + offset
     ang = pos[:, None] * inv_freq[None, :]
     return ang.cos().contiguous(), ang.sin().contiguous()

@@ -1,0 +1,85 @@
+"""The native decoding step (three launches, caches that grow in place) against the same layer run module by module:
+a forward hook on a submodule makes the layer take that path."""
+import pytest
+import torch
+
+import recipe
+from util import assert_close_bf16, assert_close_f32
+
+from native_sparse_attention_pytorch_b200 import SparseAttention
+
+pytestmark = pytest.mark.gpu
+DEV = 'cuda'
+
+
+def build(dtype, heads, kv_heads, d, dim=256, stride=16, nsel=4, window=100, norm=True):
+    layer = SparseAttention(dim=dim, dim_head=d, heads=heads, kv_heads=kv_heads, causal=True, sliding_window_size=window,
+                            compress_block_size=2 * stride, compress_block_sliding_stride=stride, selection_block_size=64,
+                            num_selected_blocks=nsel, norm=norm, use_triton_kernel=True)
+    recipe.fill_weights(layer, seed=3)
+    return layer.to(DEV).to(dtype).requires_grad_(False)
+
+
+def steps(layer, tokens, cache):
+    outs = []
+    for i in range(tokens.shape[1]):
+        out, cache = layer(tokens[:, i:i + 1], cache=cache, return_cache=True)
+        outs.append(out)
+    return torch.cat(outs, dim=1), cache
+
+
+def flat(cache):
+    (k, v), ((ck, cv), (rk, rv)) = cache
+    return k, v, ck, cv, rk, rv
+
+
+# batch (one token row to more than the projection kernels take), group size, head size, cache length: no compressed block
+# yet, one tile, several tiles per warp; a head size without a tensor form
+CASES = [(1, 4, 4, 64, 3, torch.bfloat16), (2, 8, 2, 64, 300, torch.bfloat16), (3, 16, 1, 128, 1100, torch.bfloat16),
+         (17, 4, 2, 64, 200, torch.bfloat16), (2, 6, 2, 40, 150, torch.bfloat16), (9, 8, 8, 64, 500, torch.bfloat16),
+         (2, 8, 4, 64, 130, torch.float32), (18, 2, 1, 128, 90, torch.float32)]
+
+
+@pytest.mark.parametrize('case', CASES)
+def test_native_steps_equal_the_module_by_module_steps(case):
+    b, hq, hkv, d, n, dtype = case
+    layer = build(dtype, hq, hkv, d)
+    x = recipe.randn((b, n, 256), 5).to(dtype).to(DEV)
+    tokens = recipe.randn((b, 20, 256), 6).to(dtype).to(DEV)
+    with torch.no_grad():
+        _, cache = layer(x, return_cache=True)
+        got, got_cache = steps(layer, tokens, cache)
+        hook = layer.combine_heads.register_forward_hook(lambda *_: None)
+        want, want_cache = steps(layer, tokens, cache)
+        hook.remove()
+    close = assert_close_f32 if dtype == torch.float32 else assert_close_bf16
+    close(got, want.float().cpu(), 'outputs')
+    for g, w, name in zip(flat(got_cache), flat(want_cache), ('keys', 'values', 'ck', 'cv', 'window k', 'window v')):
+        assert g.shape == w.shape and g.dtype == w.dtype, name
+        close(g, w.float().cpu(), name)
+
+
+def test_continuations_of_one_cache_do_not_disturb_each_other():
+    layer = build(torch.bfloat16, 8, 2, 64)
+    x = recipe.randn((2, 200, 256), 5).bfloat16().to(DEV)
+    a, b = (recipe.randn((2, 40, 256), s).bfloat16().to(DEV) for s in (6, 7))
+    with torch.no_grad():
+        _, cache = layer(x, return_cache=True)
+        base, mid = steps(layer, a[:, :5], cache)
+        out_a, cache_a = steps(layer, a[:, 5:], mid)               # grows in place
+        kept = [t.clone() for t in flat(cache_a)]
+        out_b, cache_b = steps(layer, b, mid)                      # another continuation while the first is alive
+        assert all(torch.equal(t, k) for t, k in zip(flat(cache_a), kept))
+        tail = cache_a[0][0][:, :, -1:]                            # a view outlives the cache it was taken from
+        tail_copy = tail.clone()
+        del cache_a, cache_b
+        again, _ = steps(layer, b, mid)
+        assert torch.equal(again, out_b) and torch.equal(tail, tail_copy)
+        del tail
+        again, _ = steps(layer, a[:, 5:], mid)                     # in place over the rows that were dropped
+        assert torch.equal(again, out_a)
+        # a cache from elsewhere, its rows cut off in front: positions count from its own first row
+        cut = ((mid[0][0][:, :, 64:], mid[0][1][:, :, 64:]), ((mid[1][0][0][:, :, 4:], mid[1][0][1][:, :, 4:]), mid[1][1]))
+        got, _ = steps(layer, b[:, :3], cut)
+        want, _ = steps(layer, b[:, :3], ((cut[0][0].clone(), cut[0][1].clone()), cut[1]))
+        assert torch.equal(got, want)
