@@ -118,8 +118,8 @@ int nsa_sel_fwd(const nsa_sel_fwd_args* args, void* stream);
  * Selected-block attention, backward.
  * Replaces NSA.backward -> native_sparse_attn_backward -> backward_preprocess_do_o_dot,
  * backward_kernel (TRI:1874-1925, 1646-1818, 696-756, 1427-1644).
- * dq [B,q_heads,N,d], dk, dv [B,kv_heads,N,d] are contiguous fp32 and are
- * zeroed by the call before accumulation (upstream returns fp32 too,
+ * dq [B,q_heads,N,d], dk, dv [B,kv_heads,N,d] are contiguous fp32; dk and dv
+ * are zeroed by the call before accumulation (upstream returns fp32 too,
  * TRI:1900-1902).  slot_grads, if not NULL, receives for every slot the
  * gradient of a multiplier of 1 on that slot's logits (TRI:1061-1080), fp32
  * [B, sel_heads, N, nsel].
@@ -282,6 +282,8 @@ typedef struct {
   const void* index;     /* optional, see nsa_cmp_index_bytes */
   int64_t index_bytes;
   const float* delta;    /* optional, as in nsa_sel_bwd_args */
+  int32_t accumulate_kv; /* as in nsa_sel_bwd_args, for dck and dcv */
+  int32_t reserved;
 } nsa_cmp_bwd_args;
 
 int nsa_cmp_bwd(const nsa_cmp_bwd_args* args, void* stream);

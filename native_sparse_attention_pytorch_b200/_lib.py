@@ -49,7 +49,7 @@ class CmpFwdArgs(C.Structure):
 
 class CmpBwdArgs(C.Structure):
     _fields_ = [('fwd', CmpFwdArgs), ('dout', Tensor4), ('dq', vp), ('dck', vp), ('dcv', vp), ('dq_out', Tensor4),
-                ('index', vp), ('index_bytes', i64), ('delta', vp)]
+                ('index', vp), ('index_bytes', i64), ('delta', vp), ('accumulate_kv', i32), ('reserved', i32)]
 
 
 class SelectArgs(C.Structure):

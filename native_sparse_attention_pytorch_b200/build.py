@@ -12,11 +12,11 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, 'csrc')
 LIB = os.path.join(HERE, 'libnsa_b200.so')
-SOURCES = ['nsa_abi.cu', 'nsa_simt_attend.cu', 'nsa_select.cu', 'nsa_combine.cu', 'nsa_rotary.cu', 'nsa_windows.cu', 'nsa_rmsnorm.cu', 'nsa_decode.cu', 'nsa_sm100_sel.cu']
+SOURCES = ['nsa_abi.cu', 'nsa_simt_attend.cu', 'nsa_select.cu', 'nsa_combine.cu', 'nsa_rotary.cu', 'nsa_windows.cu', 'nsa_rmsnorm.cu', 'nsa_decode.cu', 'nsa_layer.cu', 'nsa_sm100_sel.cu']
 
 
 HOST_LIB = os.path.join(HERE, '_nsa_host.so')
-HOST_SOURCES = ['module.cpp', 'selected.cpp', 'rooms.cpp', 'decode.cpp']
+HOST_SOURCES = ['module.cpp', 'status.cpp', 'selected.cpp', 'rooms.cpp', 'decode.cpp', 'layer.cpp']
 
 
 def _newest(*dirs):
@@ -75,8 +75,12 @@ def build(force=False, verbose=False):
     if host_jobs:
         import torch
         torch_lib = os.path.join(os.path.dirname(torch.__file__), 'lib')
+        # PyTorch's own copies of cuBLAS and the CUDA runtime, which its libraries have loaded by the time this one is
+        import glob
+        site = os.path.dirname(os.path.dirname(torch.__file__))
+        shared = [glob.glob(os.path.join(site, 'nvidia', *p))[0] for p in (('cublas', 'lib', 'libcublas.so.12'), ('cuda_runtime', 'lib', 'libcudart.so.12'))]
         subprocess.run(['g++', '-shared', '-o', HOST_LIB, *objs[len(jobs):], '-L', HERE, '-lnsa_b200', '-L', torch_lib, '-ltorch', '-ltorch_cpu',
-                        '-ltorch_cuda', '-ltorch_python', '-lc10', '-lc10_cuda', '-Wl,-rpath,$ORIGIN'], check=True)
+                        '-ltorch_cuda', '-ltorch_python', '-lc10', '-lc10_cuda', *shared, '-Wl,-rpath,$ORIGIN'], check=True)
     return LIB
 
 

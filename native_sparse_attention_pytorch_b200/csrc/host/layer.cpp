@@ -1,0 +1,575 @@
+// The whole layer natively: forward and backward of SparseAttention as one autograd node.
+//
+// Run module by module, a training step of the layer is nine autograd functions, some 140 launches and 3 ms of host
+// time whatever the size; most of the launches are small conversions, additions and copies between layouts.  Here the
+// layer is about 50 launches: the GEMMs (library), the attention kernels, and one pass for everything that happens
+// between two of them (nsa_layer.cu).
+
+#include <ATen/Context.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <cublas_v2.h>
+
+#include <cmath>
+#include <limits>
+
+#include "nsa_kernels.h"
+#include "rooms.h"
+
+namespace nsa_host {
+
+// Sizes and options of a layer call, from Python as one list of integers
+struct LayerConfig {
+  int64_t heads, kv_heads, d, window, cbs, stride, block, nsel, num_mem, causal, shared, diff_topk;
+};
+
+static LayerConfig config_of(const std::vector<int64_t>& c) {
+  return {c.at(0), c.at(1), c.at(2), c.at(3), c.at(4), c.at(5), c.at(6), c.at(7), c.at(8), c.at(9), c.at(10), c.at(11)};
+}
+
+// The parameters, in the order of the autograd function's arguments
+struct LayerWeights {
+  Tensor norm, qkv, gate, gate_b, out, mem, pos_k, pos_v, k1, kb1, k2, kb2, v1, vb1, v2, vb2;
+};
+static LayerWeights weights_of(const std::vector<OptTensor>& w) {
+  auto t = [&](size_t i) { return w.at(i).value_or(Tensor()); };
+  return {t(0), t(1), t(2), t(3), t(4), t(5), t(6), t(7), t(8), t(9), t(10), t(11), t(12), t(13), t(14), t(15)};
+}
+constexpr int kWeights = 16;
+
+// Row-major GEMMs, C [M, N] = (beta C +) op(A) op(B), on the library and with the settings at::mm uses, without the
+// tensor views and the dispatch around them (8 us of host time per product; a training step has 17).
+enum class Op { NT, NN, TN };   // A [M, K], B [N, K];  A [M, K], B [K, N];  A [K, M], B [K, N]
+static void gemm(Op op, at::ScalarType type, int64_t M, int64_t N, int64_t K, const void* A, const void* B, void* C, float beta = 0.f) {
+  const float alpha = 1.f;
+  const cublasOperation_t ta = op == Op::NT ? CUBLAS_OP_T : CUBLAS_OP_N, tb = op == Op::TN ? CUBLAS_OP_T : CUBLAS_OP_N;
+  const int lda = (int)(op == Op::NT ? K : N), ldb = (int)(op == Op::TN ? M : K);   // column-major: C^T = op(B)^T op(A)^T
+  const cublasHandle_t handle = at::cuda::getCurrentCUDABlasHandle();
+  const cublasStatus_t rc =
+      type == at::kFloat
+          ? cublasSgemm(handle, ta, tb, (int)N, (int)M, (int)K, &alpha, (const float*)B, lda, (const float*)A, ldb, &beta, (float*)C, (int)N)
+          : cublasGemmEx(handle, ta, tb, (int)N, (int)M, (int)K, &alpha, B, CUDA_R_16BF, lda, A, CUDA_R_16BF, ldb, &beta, C, CUDA_R_16BF,
+                         (int)N, CUBLAS_COMPUTE_32F, CUBLAS_GEMM_DEFAULT_TENSOR_OP);
+  if (rc != CUBLAS_STATUS_SUCCESS) throw Error("layer: a library GEMM failed");
+}
+// The settings above are PyTorch's defaults; where a program changed them its products go through at::mm.
+static bool default_blas(at::ScalarType type) {
+  auto& ctx = at::globalContext();
+  return ctx.blasPreferredBackend() == at::BlasBackend::Cublas &&
+         (type == at::kFloat || ctx.allowBF16ReductionCuBLAS() == at::CuBLASReductionOption::AllowReducedPrecisionWithSplitK);
+}
+static Tensor product(Op op, const Tensor& A, const Tensor& B) {
+  if (!default_blas(A.scalar_type())) return op == Op::NT ? at::mm(A, B.t()) : op == Op::NN ? at::mm(A, B) : at::mm(A.t(), B);
+  const int64_t M = A.size(op == Op::TN ? 1 : 0), K = A.size(op == Op::TN ? 0 : 1), N = B.size(op == Op::NT ? 0 : 1);
+  Tensor C = at::empty({M, N}, A.options());
+  gemm(op, A.scalar_type(), M, N, K, A.data_ptr(), B.data_ptr(), C.data_ptr());
+  return C;
+}
+
+// A [B, H, N, d] view without a tensor: pointer and strides in elements
+static nsa_tensor heads_view(void* p, int64_t sb, int64_t sh, int64_t sn) { return {p, sb, sh, sn}; }
+
+// One allocation cut into 256-byte aligned parts
+class Slab {
+ public:
+  int64_t add(int64_t bytes) {
+    const int64_t at = size_;
+    size_ += (bytes + 255) / 256 * 256;
+    return at;
+  }
+  void allocate(const Tensor& like) { buf_ = bytes(size_ > 0 ? size_ : 1, like); }
+  uint8_t* at(int64_t off) const { return static_cast<uint8_t*>(buf_.data_ptr()) + off; }
+  const Tensor& tensor() const { return buf_; }
+  Tensor view(int64_t off, at::IntArrayRef sizes, at::ScalarType type) const {
+    int64_t n = 1;
+    for (const int64_t s : sizes) n *= s;
+    const int64_t el = c10::elementSize(type);
+    return buf_.narrow(0, off, n * el).view(type).view(sizes);
+  }
+
+ private:
+  int64_t size_ = 0;
+  Tensor buf_;
+};
+
+// What both directions know about a call
+struct Layer {
+  LayerConfig c;
+  int64_t B, N, dim, G, ncb, F, el, k_sel, hs;
+  int dt;
+  at::ScalarType type;
+  float scale;
+  nsa::LayerShape shape;
+  int32_t* status;
+
+  Layer(const LayerConfig& cfg, const Tensor& x, int64_t status_word) : c(cfg) {
+    B = x.size(0); N = x.size(1); dim = x.size(2);
+    G = c.heads / c.kv_heads; ncb = N / c.stride; F = (c.heads + 2 * c.kv_heads) * c.d;
+    el = x.element_size(); dt = dtype_code(x); type = x.scalar_type();
+    hs = c.shared ? c.kv_heads : c.heads;
+    k_sel = std::min(std::min(c.nsel, ncb), ncb / (c.block / c.stride));
+    scale = (float)(1.0 / std::sqrt((double)c.d));
+    shape = {(int)B, (int)N, (int)c.heads, (int)c.kv_heads, (int)c.d, (int)ncb, (int)c.cbs, (int)c.stride, (int)c.num_mem};
+    status = reinterpret_cast<int32_t*>(status_word);
+  }
+
+  int64_t rows(int64_t heads) const { return B * heads * N; }
+  // contiguous [B, H, N, d]
+  nsa_tensor heads_of(void* p, int64_t H, int64_t n) const { return heads_view(p, H * n * c.d, n * c.d, c.d); }
+  // the queries (part 0), keys (1) or values (2) inside the qkv projection's output
+  nsa_tensor in_qkv(void* qkv, int part) const {
+    const int64_t first = part == 0 ? 0 : part == 1 ? c.heads : c.heads + c.kv_heads;
+    return heads_view(static_cast<uint8_t*>(qkv) + first * c.d * el, N * F, c.d, F);
+  }
+  float sentinel() const {   // (-finfo.max) // 10 in the tensor's type
+    if (dt == NSA_F32) return std::floor(-std::numeric_limits<float>::max() / 10.f);
+    return (float)c10::BFloat16((float)std::floor(-3.3895313892515355e38 / 10.0));
+  }
+
+  nsa_cmp_fwd_args cmp_args(void* qkv, void* ckv, void* out, float* lse) const {
+    nsa_cmp_fwd_args a = {};
+    const int64_t kv = c.num_mem + ncb;
+    a.q = in_qkv(qkv, 0);
+    a.ck = heads_of(ckv, c.kv_heads, kv);
+    a.cv = heads_of(static_cast<uint8_t*>(ckv) + B * c.kv_heads * kv * c.d * el, c.kv_heads, kv);
+    a.out = heads_of(out, c.heads, N);
+    a.lse = lse;
+    a.batch = B; a.q_heads = c.heads; a.kv_heads = c.kv_heads; a.sel_heads = k_sel > 0 ? hs : c.kv_heads;
+    a.seq = N; a.dim_head = c.d; a.num_mem = c.num_mem; a.ncb = ncb; a.stride = c.stride; a.causal = c.causal; a.dtype = dt;
+    a.scale = scale; a.sentinel = sentinel(); a.status = status;
+    return a;
+  }
+  nsa_sel_fwd_args sel_args(void* qr, const nsa_tensor& kr, const nsa_tensor& v, void* out, float* lse, const int64_t* idx,
+                            const uint8_t* mask) const {
+    nsa_sel_fwd_args a = {};
+    a.q = heads_of(qr, c.heads, N); a.k = kr; a.v = v; a.out = heads_of(out, c.heads, N);
+    a.idx = idx; a.mask = mask; a.lse = lse;
+    a.batch = B; a.q_heads = c.heads; a.kv_heads = c.kv_heads; a.sel_heads = k_sel > 0 ? hs : c.kv_heads;
+    a.seq = N; a.dim_head = c.d; a.block = c.block; a.nsel = k_sel; a.dtype = dt; a.scale = scale; a.status = status;
+    a.diag = k_sel > 0 ? (c.causal ? NSA_DIAG_CAUSAL : NSA_DIAG_NONE) : (c.causal ? NSA_DIAG_CAUSAL : NSA_DIAG_FULL);
+    return a;
+  }
+  nsa_swa_fwd_args swa_args(void* qr, const nsa_tensor& kr, const nsa_tensor& v, void* out, float* lse) const {
+    nsa_swa_fwd_args a = {};
+    a.q = heads_of(qr, c.heads, N); a.k = kr; a.v = v; a.out = heads_of(out, c.heads, N);
+    a.lse = lse;
+    a.batch = B; a.q_heads = c.heads; a.kv_heads = c.kv_heads; a.seq = N; a.dim_head = c.d;
+    a.window = c.window; a.causal = c.causal; a.dtype = dt; a.scale = scale; a.status = status;
+    return a;
+  }
+  nsa::CombineParams combine_params(void* o, const void* logits) const {
+    nsa::CombineParams p = {};
+    const int64_t part = rows(c.heads) * c.d * el;
+    for (int s = 0; s < 3; ++s) {
+      p.o[s] = static_cast<uint8_t*>(o) + s * part;
+      p.o_sb[s] = c.heads * N * c.d; p.o_sh[s] = N * c.d; p.o_sn[s] = c.d;
+    }
+    p.gates = logits; p.g_sb = N * 3 * c.heads; p.g_sh = 3; p.g_sn = 3 * c.heads;
+    p.logits = 1;
+    p.batch = B; p.q_heads = c.heads; p.seq = N; p.d = c.d;
+    return p;
+  }
+};
+
+// Scratch of one attention call
+template <typename Args, typename Size>
+static Tensor scratch(Args& a, Size size, int backward, const Tensor& like) {
+  const int64_t need = size(&a, backward);
+  if (need < 0) check(need);
+  Tensor ws;
+  if (need > 0) {
+    ws = bytes(need, like);
+    a.workspace = ws.data_ptr();
+    a.workspace_bytes = need;
+  }
+  return ws;
+}
+
+// -> out; cache (rotated keys, values, ck, cv, window keys, window values) where asked for; what the backward needs where asked for
+static std::vector<OptTensor> layer_forward(Tensor x, std::vector<OptTensor> weights, double eps, Tensor inv_freq,
+                                            std::vector<int64_t> cfg, int64_t status, bool save, bool want_cache) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  const LayerWeights w = weights_of(weights);
+  x = x.contiguous();
+  const Layer L(config_of(cfg), x, status);
+  const LayerConfig& c = L.c;
+  cudaStream_t st = (cudaStream_t)stream_of(x);
+  const int64_t B = L.B, N = L.N, BN = B * N, d = c.d, el = L.el, hkv = c.kv_heads;
+  const at::ScalarType type = L.type;
+
+  // norm
+  Tensor xn = x.view({BN, L.dim}), rstd;
+  if (w.norm.defined()) {
+    const Tensor x2 = xn;
+    if (L.dim * el / 16 <= 256) {
+      xn = at::empty({BN, L.dim}, x.options());
+      rstd = empty({BN}, x, at::kFloat);
+      nsa::NormParams p = {};
+      p.x = x2.data_ptr(); p.weight = w.norm.data_ptr(); p.y = xn.data_ptr(); p.rstd = ptr<float>(rstd);
+      p.rows = BN; p.x_stride = L.dim; p.dim = L.dim; p.eps = (float)eps;
+      check(nsa::launch_rmsnorm(p, L.dt, false, st));
+    } else {
+      xn = at::rms_norm(x2, {L.dim}, w.norm, eps);
+    }
+  }
+  const Tensor qkv = product(Op::NT, xn, w.qkv);
+  const Tensor logits = at::addmm(w.gate_b, xn, w.gate.t());
+
+  // kept for the backward (or until the end of this call): rotated q, compressed keys and values, branch outputs, ...
+  const int64_t q_bytes = L.rows(c.heads) * d * el, k_bytes = L.rows(hkv) * d * el, kv = c.num_mem + L.ncb;
+  Slab keep;
+  const int64_t at_qr = keep.add(q_bytes), at_kr = keep.add(k_bytes);
+  const int64_t at_win = keep.add(2 * B * hkv * L.ncb * c.cbs * d * el);
+  const int64_t at_ckv = keep.add(2 * B * hkv * kv * d * el);
+  const int64_t at_o = keep.add(3 * q_bytes), at_lse = keep.add(3 * L.rows(c.heads) * 4);
+  const int64_t picks = L.rows(L.hs) * L.k_sel;
+  const int64_t at_idx = keep.add(picks * 8), at_mask = keep.add(picks);
+  keep.allocate(x);
+  void* const qr = keep.at(at_qr);
+  float* const lse = reinterpret_cast<float*>(keep.at(at_lse));
+
+  nsa::LayerPrep prep = {};
+  prep.qkv = qkv.data_ptr(); prep.pos_k = w.pos_k.data_ptr(); prep.pos_v = w.pos_v.data_ptr(); prep.inv_freq = ptr<float>(inv_freq);
+  prep.qr = qr;
+  const int64_t win_half = B * hkv * L.ncb * c.cbs * d * el;
+  prep.kw = keep.at(at_win); prep.vw = keep.at(at_win + win_half);
+  nsa_tensor kr = L.heads_of(keep.at(at_kr), hkv, N), v = L.in_qkv(qkv.data_ptr(), 2);
+  GrownPair cache;
+  if (want_cache) {   // keys and values straight into buffers a following generation can append to
+    cache = Rooms::instance().fresh(x, B, hkv, N, std::min<int64_t>(std::max<int64_t>(N / 8, 64), 1024), d);
+    prep.kr = cache.k_buf; prep.v_out = cache.v_buf; prep.c_sb = cache.k.stride(0); prep.c_sh = cache.k.stride(1);
+    kr = t4(cache.k);
+    v = t4(cache.v);
+  } else {
+    prep.kr = kr.ptr; prep.c_sb = kr.stride_b; prep.c_sh = kr.stride_h;
+  }
+  check(nsa::launch_layer_prep(L.shape, prep, L.dt, st));
+
+  // compress networks: Linear, ReLU, Linear over each window
+  const int64_t wins = B * hkv * L.ncb, width = c.cbs * d;
+  const Tensor kw = keep.view(at_win, {wins, width}, type), vw = keep.view(at_win + win_half, {wins, width}, type);
+  const Tensor hk = at::_addmm_activation(w.kb1, kw, w.k1.t()), hv = at::_addmm_activation(w.vb1, vw, w.v1.t());
+  const Tensor ck = at::addmm(w.kb2, hk, w.k2.t()), cv = at::addmm(w.vb2, hv, w.v2.t());
+  void* const ckv = keep.at(at_ckv);
+  check(nsa::launch_join_mem(L.shape, w.mem.data_ptr(), ck.data_ptr(), cv.data_ptr(), ckv, L.dt, st));
+
+  // compressed branch; its logits rank the blocks
+  uint8_t* const o = keep.at(at_o);
+  int64_t* const idx = reinterpret_cast<int64_t*>(keep.at(at_idx));
+  uint8_t* const mask = keep.at(at_mask);
+  Tensor importance;
+  {
+    nsa_cmp_fwd_args a = L.cmp_args(qkv.data_ptr(), ckv, o, lse);
+    const int64_t cpf = c.block / c.stride;
+    bool pooled = false;
+    if (L.k_sel > 0) {
+      a.pool = cpf;
+      pooled = c.causal && !c.diff_topk && L.hs == hkv && nsa_cmp_fwd_pools(&a);
+      importance = pooled ? at::empty({B, L.hs, N, L.ncb / cpf}, x.options().dtype(at::kBFloat16))
+                          : at::empty({B, L.hs, N, L.ncb}, x.options().dtype(at::kFloat));
+      if (pooled) a.pooled = importance.data_ptr();
+      else { a.importance = ptr<float>(importance); a.pool = 0; }
+    }
+    const Tensor ws = scratch(a, nsa_cmp_workspace_bytes, 0, x);
+    check(nsa_cmp_fwd(&a, st));
+    if (L.k_sel > 0) {
+      nsa::SelectParams p = {};
+      p.imp = pooled ? nullptr : ptr<float>(importance);
+      p.pooled = pooled ? importance.data_ptr() : nullptr;
+      p.causal_limit = pooled;
+      p.idx = idx; p.mask = mask;
+      p.rows = B * L.hs; p.seq = N; p.cpf = pooled ? 1 : cpf; p.ncb = pooled ? L.ncb / cpf : L.ncb; p.cols = p.ncb / p.cpf;
+      p.k = L.k_sel; p.block = c.block; p.exclude_own = c.block != c.stride; p.round_bf16 = L.dt == NSA_BF16;
+      p.neg_max = L.dt == NSA_BF16 ? -3.3895313892515355e38f : -std::numeric_limits<float>::max();
+      check(nsa::launch_select(p, st));
+    }
+  }
+  // selected branch
+  Tensor index;
+  {
+    nsa_sel_fwd_args a = L.sel_args(qr, kr, v, o + q_bytes, lse + L.rows(c.heads), L.k_sel > 0 ? idx : nullptr, L.k_sel > 0 ? mask : nullptr);
+    const Tensor ws = scratch(a, nsa_sel_workspace_bytes, 0, x);
+    if (save && ws.defined()) {
+      index = bytes(nsa_sel_index_bytes(&a), x);
+      a.index_out = index.data_ptr();
+      a.index_out_bytes = index.numel();
+    }
+    check(nsa_sel_fwd(&a, st));
+  }
+  // sliding branch
+  {
+    nsa_swa_fwd_args a = L.swa_args(qr, kr, v, o + 2 * q_bytes, lse + 2 * L.rows(c.heads));
+    const Tensor ws = scratch(a, nsa_swa_workspace_bytes, 0, x);
+    check(nsa_swa_fwd(&a, st));
+  }
+  // gated combine and output projection
+  const Tensor merged = at::empty({BN, c.heads * d}, x.options());
+  {
+    const nsa::CombineParams p = L.combine_params(o, logits.data_ptr());
+    nsa::GatherTargets t = {};
+    t.outs[0] = merged.data_ptr(); t.num_outs = 1; t.total_features = c.heads * d;
+    check(nsa::launch_combine_gather(p, t, L.dt, st));
+  }
+  const Tensor out = product(Op::NT, merged, w.out).view({B, N, L.dim});
+
+  auto opt = [](const Tensor& t) { return t.defined() ? OptTensor(t) : OptTensor(); };
+  std::vector<OptTensor> result = {out};
+  if (want_cache) {
+    // the un-rotated rows of the window that is being filled (its overlap with the last complete one first, zero where
+    // that lies before the sequence)
+    const int64_t first = L.ncb * c.stride - (c.cbs - c.stride), len = N - first, pad = std::max<int64_t>(0, -first);
+    GrownPair run = Rooms::instance().fresh(x, B, hkv, len, 4 * c.cbs, d);
+    const Tensor all = qkv.view({B, N, c.heads + 2 * hkv, d}).permute({0, 2, 1, 3});
+    for (int s = 0; s < 2; ++s) {
+      const Tensor dst = s == 0 ? run.k : run.v;
+      if (pad > 0) dst.narrow(2, 0, pad).zero_();
+      dst.narrow(2, pad, len - pad).copy_(all.narrow(1, c.heads + s * hkv, hkv).narrow(2, std::max<int64_t>(0, first), len - pad));
+    }
+    result.insert(result.end(), {cache.k, cache.v, ck.view({B, hkv, L.ncb, d}), cv.view({B, hkv, L.ncb, d}), run.k, run.v});
+  }
+  if (save) {
+    result.insert(result.end(), {x, xn, opt(rstd), qkv, logits, keep.tensor(), hk, hv, opt(index), merged,
+                                 c.diff_topk ? opt(importance) : OptTensor()});
+  }
+  return result;
+}
+
+// Gradient through the differentiable top-k: d(value of a pick) back through gather, sink softmax, block mean and head
+// mean to the logits, as a matrix dlog [B, hs, N, ncb] (already times scale / heads averaged)
+static Tensor importance_gradient(const Layer& L, const Tensor& importance, const Tensor& idx, const Tensor& dvals) {
+  const int64_t B = L.B, N = L.N, cpf = L.c.block / L.c.stride, cols = L.ncb / cpf;
+  const bool own_excluded = cpf > 1;
+  Tensor s = importance, own;
+  if (cpf > 1) {
+    s = s.narrow(3, 0, cols * cpf).reshape({B, L.hs, N, cols, cpf}).mean(-1);
+    const auto opts = importance.options().dtype(at::kLong);
+    own = at::arange(N, opts).floor_divide(L.c.block).unsqueeze(1).eq(at::arange(cols, opts).unsqueeze(0));
+    s = s.masked_fill(own, -std::numeric_limits<float>::max());
+  }
+  const Tensor p = at::constant_pad_nd(s, {1, 0}, -1e3).softmax(-1).narrow(3, 1, cols);
+  const Tensor dp = at::zeros_like(p, at::MemoryFormat::Contiguous).scatter_add_(-1, idx, dvals);
+  Tensor ds = p * (dp - (p * dp).sum(-1, true));
+  if (own_excluded) {
+    ds = ds.masked_fill(own, 0.);
+    Tensor full = at::zeros_like(importance);
+    full.narrow(3, 0, cols * cpf).copy_((ds / (double)cpf).repeat_interleave(cpf, -1));
+    ds = full;
+  }
+  const int64_t per_sel = L.c.heads / L.hs;
+  ds = ds * (double)(L.scale / (float)per_sel);
+  if (L.c.causal) {
+    const auto opts = importance.options().dtype(at::kLong);
+    const Tensor visible = at::arange(L.ncb, opts).unsqueeze(0) < at::arange(N, opts).floor_divide(L.c.stride).unsqueeze(1);
+    ds = ds * visible;
+  }
+  return ds;
+}
+
+// -> gradients of x and of the parameters, in the order of the forward's arguments; `needs` says which are wanted
+static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor> weights, std::vector<OptTensor> saved,
+                                             double eps, Tensor inv_freq, std::vector<int64_t> cfg, int64_t status,
+                                             std::vector<bool> needs, OptTensor swa_index, OptTensor cmp_index) {
+  const LayerWeights w = weights_of(weights);
+  auto sv = [&](size_t i) { return saved.at(i).value_or(Tensor()); };
+  const Tensor x = sv(0), xn = sv(1), rstd = sv(2), qkv = sv(3), logits = sv(4), kept = sv(5), hk = sv(6), hv = sv(7), index = sv(8),
+               merged = sv(9), importance = sv(10);
+  const c10::cuda::CUDAGuard guard(x.device());
+  const Layer L(config_of(cfg), x, status);
+  const LayerConfig& c = L.c;
+  cudaStream_t st = (cudaStream_t)stream_of(x);
+  const int64_t B = L.B, N = L.N, BN = B * N, d = c.d, el = L.el, hkv = c.kv_heads, H = c.heads;
+  const at::ScalarType type = L.type;
+  const int64_t q_elems = L.rows(H) * d, k_elems = L.rows(hkv) * d, q_bytes = q_elems * el, kv = c.num_mem + L.ncb;
+  const int64_t c_elems = B * hkv * kv * d;
+  // the forward's slab, cut as there
+  Slab keep;
+  const int64_t at_qr = keep.add(q_bytes), at_kr = keep.add(k_elems * el);
+  const int64_t at_win = keep.add(2 * B * hkv * L.ncb * c.cbs * d * el);
+  const int64_t at_ckv = keep.add(2 * c_elems * el);
+  const int64_t at_o = keep.add(3 * q_bytes), at_lse = keep.add(3 * L.rows(H) * 4);
+  const int64_t picks = L.rows(L.hs) * L.k_sel;
+  const int64_t at_idx = keep.add(picks * 8), at_mask = keep.add(picks);
+  uint8_t* const kp = static_cast<uint8_t*>(kept.data_ptr());
+  float* const lse = reinterpret_cast<float*>(kp + at_lse);
+  auto kept_view = [&](int64_t off, at::IntArrayRef sizes, at::ScalarType t) {
+    int64_t n = 1;
+    for (const int64_t s : sizes) n *= s;
+    return kept.narrow(0, off, n * (int64_t)c10::elementSize(t)).view(t).view(sizes);
+  };
+
+  // fp32 accumulators, cleared together: dk, dv; dck, dcv; then the small gradients that end up in the layer's type
+  const int64_t pos = hkv * c.cbs * d, mems = hkv * c.num_mem * d, hid = w.k1.size(0);
+  auto even = [](int64_t n) { return (n + 7) / 8 * 8; };
+  const int64_t s_norm = 0, s_gate = s_norm + even(L.dim), s_mem = s_gate + even(3 * H), s_pos = s_mem + even(2 * mems),
+                s_b1 = s_pos + even(2 * pos), s_b2 = s_b1 + even(2 * hid), s_end = s_b2 + even(2 * d);
+  const int64_t a_small = even(2 * k_elems + 2 * c_elems);
+  Tensor acc = empty({a_small + s_end}, x, at::kFloat);
+  if (cudaMemsetAsync(acc.data_ptr(), 0, (a_small + s_end) * 4, st) != cudaSuccess) throw Error("clearing the gradient accumulators failed");
+  float* const dk = ptr<float>(acc);
+  float* const dck = dk + 2 * k_elems;
+  float* const small = dk + a_small;
+
+  // output projection and gated combine
+  dout = dout.reshape({BN, L.dim}).contiguous();
+  const Tensor d_merged = product(Op::NN, dout, w.out);
+  Slab tmp;
+  const int64_t t_do = tmp.add(3 * q_bytes), t_delta = tmp.add(3 * L.rows(H) * 4), t_dq = tmp.add(3 * q_elems * 4);
+  tmp.allocate(x);
+  const Tensor d_logits = at::empty({BN, 3 * H}, x.options());
+  {
+    nsa::CombineParams p = L.combine_params(kp + at_o, logits.data_ptr());
+    p.dout = d_merged.data_ptr();
+    for (int s = 0; s < 3; ++s) p.d_o[s] = tmp.at(t_do + s * q_bytes);
+    p.delta = reinterpret_cast<float*>(tmp.at(t_delta));
+    p.d_logits = d_logits.data_ptr();
+    check(nsa::launch_combine(p, L.dt, true, st));
+  }
+
+  // the three branches
+  nsa::QkvGrad qg = {};
+  const nsa_tensor kr = L.heads_of(kp + at_kr, hkv, N), v = L.in_qkv(qkv.data_ptr(), 2);
+  auto delta = [&](int s) { return reinterpret_cast<float*>(tmp.at(t_delta)) + s * L.rows(H); };
+  auto d_o = [&](int s) { return L.heads_of(tmp.at(t_do + s * q_bytes), H, N); };
+  // dq of branch s: rows in the layer's type where the kernels store them, else fp32; run(direct) issues the call
+  auto with_dq = [&](int s, bool stores, bool need_f32, nsa_tensor& dq_out, float*& dq, auto run) {
+    void* const at = tmp.at(t_dq + s * q_elems * 4);
+    int rc = NSA_ERR_UNSUPPORTED;
+    if (stores && !need_f32) {
+      dq_out = L.heads_of(at, H, N);
+      rc = run();
+      if (rc == 0) qg.dq[s] = at;
+    }
+    if (rc == NSA_ERR_UNSUPPORTED) {
+      dq_out = no_tensor();
+      dq = static_cast<float*>(at);
+      rc = run();
+      if (rc == 0) qg.dq_f32[s] = dq;
+    }
+    check(rc);
+  };
+  Tensor slots;
+  {
+    nsa_sel_bwd_args a = {};
+    a.fwd = L.sel_args(kp + at_qr, kr, v, kp + at_o + q_bytes, lse + L.rows(H),
+                       L.k_sel > 0 ? reinterpret_cast<int64_t*>(kp + at_idx) : nullptr, L.k_sel > 0 ? kp + at_mask : nullptr);
+    const Tensor ws = scratch(a.fwd, nsa_sel_workspace_bytes, 1, x);
+    a.dout = d_o(1); a.dk = dk; a.dv = dk + k_elems; a.accumulate_kv = 1; a.delta = delta(1);
+    if (index.defined()) { a.index = index.data_ptr(); a.index_bytes = index.numel(); }
+    if (c.diff_topk && L.k_sel > 0) {
+      slots = at::zeros({B, L.hs, N, L.k_sel}, x.options().dtype(at::kFloat));
+      a.slot_grads = ptr<float>(slots);
+    }
+    with_dq(1, nsa_sel_bwd_stores_dq(&a.fwd) == 1, false, a.dq_out, a.dq, [&] { return nsa_sel_bwd(&a, st); });
+  }
+  std::vector<OptTensor> built(2);
+  {
+    nsa_swa_bwd_args a = {};
+    a.fwd = L.swa_args(kp + at_qr, kr, v, kp + at_o + 2 * q_bytes, lse + 2 * L.rows(H));
+    const Tensor ws = scratch(a.fwd, nsa_swa_workspace_bytes, 1, x);
+    a.dout = d_o(2); a.dk = dk; a.dv = dk + k_elems; a.accumulate_kv = 1; a.delta = delta(2);
+    if (swa_index.has_value()) { a.index = swa_index->data_ptr(); a.index_bytes = swa_index->numel(); }
+    with_dq(2, nsa_swa_bwd_stores_dq(&a.fwd) == 1, false, a.dq_out, a.dq, [&] { return nsa_swa_bwd(&a, st); });
+    const int64_t n = swa_index.has_value() || !ws.defined() ? 0 : nsa_swa_index_bytes(&a.fwd);
+    if (n > 0) built[0] = ws.narrow(0, 0, n).clone();
+  }
+  const bool through_topk = slots.defined();
+  {
+    nsa_cmp_bwd_args a = {};
+    a.fwd = L.cmp_args(qkv.data_ptr(), kp + at_ckv, kp + at_o, lse);
+    const Tensor ws = scratch(a.fwd, nsa_cmp_workspace_bytes, 1, x);
+    a.dout = d_o(0); a.dck = dck; a.dcv = dck + c_elems; a.accumulate_kv = 1; a.delta = delta(0);
+    if (cmp_index.has_value()) { a.index = cmp_index->data_ptr(); a.index_bytes = cmp_index->numel(); }
+    with_dq(0, nsa_cmp_bwd_stores_dq(&a.fwd) == 1, through_topk, a.dq_out, a.dq, [&] { return nsa_cmp_bwd(&a, st); });
+    const int64_t n = cmp_index.has_value() || !ws.defined() ? 0 : nsa_cmp_index_bytes(&a.fwd);
+    if (n > 0) built[1] = ws.narrow(0, 0, n).clone();
+  }
+  if (through_topk) {
+    // every head of a selection head gets the same gradient of its logits: one product for all of them
+    const Tensor dlog = importance_gradient(L, importance, kept_view(at_idx, {B, L.hs, N, L.k_sel}, at::kLong), slots);
+    const int64_t per_sel = H / L.hs, sel_per_kv = L.hs / hkv;
+    const Tensor ckc = kept_view(at_ckv, {2, B, hkv, kv, d}, type).select(0, 0).narrow(2, c.num_mem, L.ncb).to(at::kFloat);   // [B, Hkv, ncb, d]
+    const Tensor dlog_kv = dlog.view({B, hkv, sel_per_kv * N, L.ncb});
+    const Tensor dq_add = at::matmul(dlog_kv, ckc).view({B, L.hs, 1, N, d});
+    tmp.view(t_dq, {B, L.hs, per_sel, N, d}, at::kFloat).add_(dq_add);
+    const Tensor q = qkv.view({B, N, c.heads + 2 * hkv, d}).narrow(2, 0, H).permute({0, 2, 1, 3}).to(at::kFloat);
+    const Tensor q_sum = q.reshape({B, L.hs, per_sel, N, d}).sum(2).view({B, hkv, sel_per_kv * N, d});
+    acc.narrow(0, 2 * k_elems, c_elems).view({B, hkv, kv, d}).narrow(2, c.num_mem, L.ncb).add_(at::matmul(dlog_kv.transpose(-1, -2), q_sum));
+  }
+
+  // compress networks
+  const int64_t wins = B * hkv * L.ncb, width = c.cbs * d;
+  const Tensor dc = at::empty({2, wins, d}, x.options());
+  check(nsa::launch_split_mem(L.shape, dck, dc.data_ptr(), small + s_mem, small + s_b2, L.dt, st));
+  const Tensor dck_rows = dc.select(0, 0), dcv_rows = dc.select(0, 1);
+  const Tensor dhk = product(Op::NN, dck_rows, w.k2), dhv = product(Op::NN, dcv_rows, w.v2);
+  {
+    nsa::ColumnSums p = {};
+    p.x[0] = dhk.data_ptr(); p.x[1] = dhv.data_ptr(); p.act[0] = hk.data_ptr(); p.act[1] = hv.data_ptr();
+    p.out[0] = small + s_b1; p.out[1] = small + s_b1 + hid;
+    p.rows = wins; p.cols = hid; p.sets = 2;
+    check(nsa::launch_column_sums(p, L.dt, st));
+  }
+  std::vector<OptTensor> g(1 + kWeights);
+  const Tensor kw = kept_view(at_win, {wins, width}, type), vw = kept_view(at_win + wins * width * el, {wins, width}, type);
+  if (needs[11]) g[11] = product(Op::TN, dck_rows, hk);
+  if (needs[15]) g[15] = product(Op::TN, dcv_rows, hv);
+  if (needs[9]) g[9] = product(Op::TN, dhk, kw);
+  if (needs[13]) g[13] = product(Op::TN, dhv, vw);
+  const Tensor dkw = product(Op::NN, dhk, w.k1), dvw = product(Op::NN, dhv, w.v1);
+  check(nsa::launch_pos_grad(L.shape, dkw.data_ptr(), dvw.data_ptr(), small + s_pos, L.dt, st));
+
+  // qkv, gates, norm
+  const Tensor d_qkv = at::empty({BN, L.F}, x.options());
+  qg.dk = dk; qg.dv = dk + k_elems; qg.dkw = dkw.data_ptr(); qg.dvw = dvw.data_ptr(); qg.inv_freq = ptr<float>(inv_freq); qg.out = d_qkv.data_ptr();
+  check(nsa::launch_qkv_grad(L.shape, qg, L.dt, st));
+  {
+    nsa::ColumnSums p = {};
+    p.x[0] = d_logits.data_ptr(); p.out[0] = small + s_gate; p.rows = BN; p.cols = 3 * H; p.sets = 1;
+    check(nsa::launch_column_sums(p, L.dt, st));
+  }
+  if (needs[5]) g[5] = product(Op::TN, dout, merged);
+  if (needs[2]) g[2] = product(Op::TN, d_qkv, xn);
+  if (needs[3]) g[3] = product(Op::TN, d_logits, xn);
+  if (needs[0] || needs[1]) {
+    Tensor dxn = product(Op::NN, d_qkv, w.qkv);
+    if (default_blas(type)) gemm(Op::NN, type, BN, L.dim, 3 * H, d_logits.data_ptr(), w.gate.data_ptr(), dxn.data_ptr(), 1.f);
+    else dxn.addmm_(d_logits, w.gate);
+    if (w.norm.defined()) {
+      const Tensor dx = at::empty({BN, L.dim}, x.options());
+      nsa::NormParams p = {};
+      p.x = x.data_ptr(); p.weight = w.norm.data_ptr(); p.rstd = ptr<float>(rstd); p.dy = dxn.data_ptr(); p.dx = dx.data_ptr();
+      p.dweight = small + s_norm; p.rows = BN; p.x_stride = L.dim; p.dim = L.dim; p.eps = (float)eps; p.accumulate = 1;
+      check(nsa::launch_rmsnorm(p, L.dt, true, st));
+      dxn = dx;
+    }
+    if (needs[0]) g[0] = dxn.view(x.sizes());
+  }
+  // the small gradients in the layer's type
+  Tensor rounded = acc.narrow(0, a_small, s_end);
+  if (type != at::kFloat) {
+    rounded = at::empty({s_end}, x.options());
+    check(nsa::launch_round(small, rounded.data_ptr(), s_end, st));
+  }
+  auto give = [&](int i, int64_t off, const Tensor& like) {
+    if (needs[i]) g[i] = rounded.narrow(0, off, like.numel()).view(like.sizes());
+  };
+  if (w.norm.defined()) give(1, s_norm, w.norm);
+  give(4, s_gate, w.gate_b);
+  give(6, s_mem, w.mem);
+  give(7, s_pos, w.pos_k);
+  give(8, s_pos + pos, w.pos_v);
+  give(10, s_b1, w.kb1);
+  give(14, s_b1 + hid, w.vb1);
+  give(12, s_b2, w.kb2);
+  give(16, s_b2 + d, w.vb2);
+  g.push_back(built[0]);
+  g.push_back(built[1]);
+  return g;
+}
+
+void bind_layer(pybind11::module_& m) {
+  namespace py = pybind11;
+  m.def("layer_forward", &layer_forward, py::call_guard<py::gil_scoped_release>());
+  m.def("layer_backward", &layer_backward, py::call_guard<py::gil_scoped_release>());
+}
+
+}  // namespace nsa_host

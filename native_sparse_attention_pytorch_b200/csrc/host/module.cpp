@@ -15,6 +15,8 @@ PYBIND11_MODULE(_nsa_host, m) {
       PyErr_SetString(g_error_class != nullptr ? g_error_class : PyExc_RuntimeError, e.what());
     }
   });
+  nsa_host::bind_status(m);
   nsa_host::bind_selected(m);
   nsa_host::bind_decode(m);
+  nsa_host::bind_layer(m);
 }

@@ -70,7 +70,9 @@ inline void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream
 // view that made t is a view again instead of a copy.
 Tensor empty_in_order_of(const Tensor& t);
 
+void bind_status(pybind11::module_& m);
 void bind_selected(pybind11::module_& m);
 void bind_decode(pybind11::module_& m);
+void bind_layer(pybind11::module_& m);
 
 }  // namespace nsa_host

@@ -14,6 +14,7 @@ static Tensor rows_of(const Tensor& buf, int64_t first, int64_t rows) {
 }
 
 GrownPair Rooms::fresh(const Tensor& like, int64_t batch, int64_t heads, int64_t rows, int64_t room, int64_t d) {
+  at::AutoDispatchBelowADInplaceOrView no_view_tracking;   // a tracked view keeps its base, and so a second user of the storage
   GrownPair g;
   const Tensor k_buf = at::empty({batch, heads, rows + room, d}, like.options());
   const Tensor v_buf = at::empty({batch, heads, rows + room, d}, like.options());

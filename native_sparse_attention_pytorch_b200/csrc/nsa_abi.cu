@@ -266,13 +266,11 @@ int nsa_sel_bwd(const nsa_sel_bwd_args* a, void* stream) {
     return fail(NSA_ERR_ALIGN, "index must be 16-byte aligned");
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t d = a->fwd.dim_head, n = a->fwd.seq, b = a->fwd.batch;
-  if (!dq_stored) NSA_TRY(zero_async(a->dq, b * a->fwd.q_heads * n * d, st));
   NSA_TRY(zero_kv(a->dk, a->dv, b * a->fwd.kv_heads * n * d, a->accumulate_kv != 0, st));
   if (a->fwd.impl != NSA_IMPL_SIMT) {
     const int rc = sm100_sel_bwd(*a, st);
     if (rc != NSA_ERR_UNSUPPORTED || a->fwd.impl == NSA_IMPL_SM100) return rc;
     if (a->dq == nullptr) return fail(NSA_ERR_UNSUPPORTED, "the tensor-core kernels could not take these tensors; pass an fp32 dq");
-    if (dq_stored) NSA_TRY(zero_async(a->dq, b * a->fwd.q_heads * n * d, st));
   }
   set_dout(P, a->dout);
   P.dq = a->dq; P.dk = a->dk; P.dv = a->dv; P.slot_grads = a->slot_grads;
@@ -345,14 +343,12 @@ int nsa_cmp_bwd(const nsa_cmp_bwd_args* a, void* stream) {
     return fail(NSA_ERR_ALIGN, "index must be 16-byte aligned");
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t d = a->fwd.dim_head, rows = a->fwd.num_mem + a->fwd.ncb, b = a->fwd.batch;
-  if (!dq_stored) NSA_TRY(zero_async(a->dq, b * a->fwd.q_heads * a->fwd.seq * d, st));
-  NSA_TRY(zero_kv(a->dck, a->dcv, b * a->fwd.kv_heads * rows * d, false, st));
+  NSA_TRY(zero_kv(a->dck, a->dcv, b * a->fwd.kv_heads * rows * d, a->accumulate_kv != 0, st));
   if (a->fwd.impl != NSA_IMPL_SIMT) {
     const int rc = sm100_cmp_bwd(*a, st);
     if (rc != NSA_ERR_UNSUPPORTED) return rc;
     if (a->fwd.impl == NSA_IMPL_SM100) return fail(NSA_ERR_UNSUPPORTED, "compressed branch: shape outside the tensor-core family");
     if (a->dq == nullptr) return fail(NSA_ERR_UNSUPPORTED, "the tensor-core kernels could not take these tensors; pass an fp32 dq");
-    if (dq_stored) NSA_TRY(zero_async(a->dq, b * a->fwd.q_heads * a->fwd.seq * d, st));
   }
   set_dout(P, a->dout);
   P.importance = nullptr;
@@ -374,7 +370,7 @@ int nsa_select(const nsa_select_args* a, void* stream) {
   if (a->pooled != nullptr && (a->importance != nullptr || a->cpf != 1 || a->input_is_prob))
     return fail(NSA_ERR_SHAPE, "pooled excludes importance and input_is_prob and needs cpf == 1");
   SelectParams P;
-  P.imp = a->importance; P.idx = a->idx; P.vals = a->vals;
+  P.imp = a->importance; P.idx = a->idx; P.vals = a->vals; P.mask = nullptr;
   P.pooled = a->pooled; P.causal_limit = (a->pooled != nullptr || a->causal_limit) ? 1 : 0;
   P.rows = a->rows; P.seq = a->seq; P.ncb = a->ncb; P.cpf = a->cpf; P.cols = cols; P.k = a->k;
   P.block = a->block; P.exclude_own = a->exclude_own; P.input_is_prob = a->input_is_prob;
@@ -434,14 +430,12 @@ int nsa_swa_bwd(const nsa_swa_bwd_args* a, void* stream) {
     return fail(NSA_ERR_ALIGN, "index must be 16-byte aligned");
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t d = a->fwd.dim_head, n = a->fwd.seq, b = a->fwd.batch;
-  if (!dq_stored) NSA_TRY(zero_async(a->dq, b * a->fwd.q_heads * n * d, st));
   NSA_TRY(zero_kv(a->dk, a->dv, b * a->fwd.kv_heads * n * d, a->accumulate_kv != 0, st));
   if (a->fwd.impl != NSA_IMPL_SIMT) {
     const int rc = sm100_swa_bwd(*a, st);
     if (rc != NSA_ERR_UNSUPPORTED) return rc;
     if (a->fwd.impl == NSA_IMPL_SM100) return fail(NSA_ERR_UNSUPPORTED, "sliding branch: shape outside the tensor-core family");
     if (a->dq == nullptr) return fail(NSA_ERR_UNSUPPORTED, "the tensor-core kernels could not take these tensors; pass an fp32 dq");
-    if (dq_stored) NSA_TRY(zero_async(a->dq, b * a->fwd.q_heads * n * d, st));
   }
   set_dout(P, a->dout);
   P.dq = a->dq; P.dk = a->dk; P.dv = a->dv;

@@ -6,6 +6,13 @@
 
 namespace nsa {
 
+// A gate from the tensor it is read from: the gate itself, or the logit whose sigmoid it is (rounded to T)
+template <typename T>
+__device__ __forceinline__ float gate_value(T raw, int logits) {
+  const float x = Elem<T>::to_float(raw);
+  return logits ? Elem<T>::to_float(Elem<T>::from_float(1.f / (1.f + expf(-x)))) : x;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) combine_fwd_kernel(const CombineParams P) {
   const int half = P.d / 2;
@@ -19,7 +26,7 @@ __global__ void __launch_bounds__(256) combine_fwd_kernel(const CombineParams P)
     float ax = 0.f, ay = 0.f;
 #pragma unroll
     for (int s = 0; s < 3; ++s) {
-      const float gs = Elem<T>::to_float(g[s]);
+      const float gs = gate_value<T>(g[s], P.logits);
       const float2 v = Elem<T>::load2((const T*)P.o[s] + b * P.o_sb[s] + h * P.o_sh[s] + (int64_t)n * P.o_sn[s] + c);
       ax = fmaf(gs, v.x, ax);
       ay = fmaf(gs, v.y, ay);
@@ -50,7 +57,7 @@ __global__ void __launch_bounds__(256) combine_gather_kernel(const CombineParams
     for (int x = 0; x < V; ++x) acc[x] = 0.f;
 #pragma unroll
     for (int s = 0; s < 3; ++s) {
-      const float gs = Elem<T>::to_float(g[s]);
+      const float gs = gate_value<T>(g[s], P.logits);
       const uint4 raw = *reinterpret_cast<const uint4*>((const T*)P.o[s] + b * P.o_sb[s] + h * P.o_sh[s] +
                                                        (int64_t)n * P.o_sn[s] + c);
       const T* v = reinterpret_cast<const T*>(&raw);
@@ -110,7 +117,7 @@ __global__ void __launch_bounds__(128) combine_bwd_kernel(const CombineParams P)
   const T* dout = (const T*)P.dout + (((int64_t)b * P.seq + n) * P.q_heads + h) * P.d;
   float gs[3], dg[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-  for (int s = 0; s < 3; ++s) gs[s] = Elem<T>::to_float(g[s]);
+  for (int s = 0; s < 3; ++s) gs[s] = gate_value<T>(g[s], P.logits);
   for (int c = 2 * lane; c < P.d; c += 64) {
     const float2 dy = Elem<T>::load2(dout + c);
 #pragma unroll
@@ -124,7 +131,8 @@ __global__ void __launch_bounds__(128) combine_bwd_kernel(const CombineParams P)
   for (int s = 0; s < 3; ++s) {
     const float t = warp_sum(dg[s]);
     if (lane == 0) {
-      P.d_gates[task * 3 + s] = t;
+      if (P.logits) ((T*)P.d_logits)[((int64_t)b * P.seq + n) * P.q_heads * 3 + h * 3 + s] = Elem<T>::from_float(t * gs[s] * (1.f - gs[s]));
+      else P.d_gates[task * 3 + s] = t;
       if (P.delta != nullptr) P.delta[s * ((int64_t)P.batch * P.q_heads * P.seq) + task] = gs[s] * t;
     }
   }
@@ -148,7 +156,7 @@ __global__ void __launch_bounds__(256) combine_bwd_vec_kernel(const CombineParam
     const T* dy = reinterpret_cast<const T*>(&draw);
 #pragma unroll
     for (int s = 0; s < 3; ++s) {
-      const float gs = Elem<T>::to_float(g[s]);
+      const float gs = gate_value<T>(g[s], P.logits);
       gate[s] = gs;
       const uint4 oraw = *reinterpret_cast<const uint4*>((const T*)P.o[s] + b * P.o_sb[s] + h * P.o_sh[s] +
                                                         (int64_t)n * P.o_sn[s] + c);
@@ -169,7 +177,13 @@ __global__ void __launch_bounds__(256) combine_bwd_vec_kernel(const CombineParam
 #pragma unroll
     for (int o = TPR / 2; o > 0; o >>= 1) dg[s] += __shfl_xor_sync(kFullMask, dg[s], o);
     if (live && part == 0) {
-      P.d_gates[task * 3 + s] = dg[s];
+      if (P.logits) {
+        const Coord4 at = split4(task, P.seq, P.q_heads, 1);
+        ((T*)P.d_logits)[((int64_t)at.i3 * P.seq + at.i0) * P.q_heads * 3 + at.i1 * 3 + s] =
+            Elem<T>::from_float(dg[s] * gate[s] * (1.f - gate[s]));
+      } else {
+        P.d_gates[task * 3 + s] = dg[s];
+      }
       if (P.delta != nullptr) P.delta[s * tasks + task] = gate[s] * dg[s];
     }
   }

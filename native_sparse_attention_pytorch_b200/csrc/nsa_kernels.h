@@ -43,6 +43,7 @@ struct SelectParams {
   int causal_limit;        // columns at and past i / block are not read: probability 0
   int64_t* idx;
   float* vals;
+  uint8_t* mask;           // optional: value above the threshold below which a slot is masked out
   int rows, seq, ncb, cpf, cols, k, block, exclude_own, input_is_prob, round_bf16;
   float neg_max;
 };
@@ -55,6 +56,8 @@ struct CombineParams {
   void* d_o[3];
   float* d_gates;
   float* delta;            // backward, optional: [3][batch * q_heads * seq] gate x d gate
+  void* d_logits;          // backward, with `logits`: [batch, seq, 3 q_heads] in the tensors' type, instead of d_gates
+  int logits;              // `gates` holds logits: the gate is their sigmoid, rounded as a tensor of it would be
   int batch, q_heads, seq, d;
 };
 
@@ -93,6 +96,7 @@ struct NormParams {
   float* dweight;     // [dim] fp32 (backward)
   int64_t rows, x_stride;
   int dim, weight_f32;
+  int accumulate;     // backward: dweight is added to as it is instead of zeroed first
   float eps;
 };
 
@@ -132,6 +136,33 @@ struct ProjectParams {
   float eps;
 };
 
+// The passes of a layer step between its GEMMs and its attention kernels (see nsa_layer.cu)
+struct LayerShape {
+  int batch, seq, heads, kv_heads, d, ncb, cbs, stride, num_mem;
+};
+struct LayerPrep {
+  const void *qkv, *pos_k, *pos_v;   // [B, N, (Hq + 2 Hkv) d], [Hkv, cbs, d] twice
+  const float* inv_freq;             // [d / 2]
+  void *qr, *kr, *v_out;             // [B, Hq, N, d]; [B, Hkv, N, d] with the strides below (v_out may be NULL)
+  int64_t c_sb, c_sh;
+  void *kw, *vw;                     // [B, Hkv, ncb, cbs, d]
+};
+struct ColumnSums {
+  void* x[2];                        // [rows, cols], masked in place where `act` is given
+  const void* act[2];
+  float* out[2];                     // added to
+  int64_t rows;
+  int cols, sets;                    // cols a multiple of 16 bytes
+};
+struct QkvGrad {
+  const void* dq[3];                 // compressed, selected, sliding: [B, Hq, N, d] in the layer's type ...
+  const float* dq_f32[3];            // ... or fp32
+  const float *dk, *dv;              // [B, Hkv, N, d]
+  const void *dkw, *dvw;             // [B, Hkv, ncb, cbs, d] or NULL
+  const float* inv_freq;
+  void* out;                         // [B, N, (Hq + 2 Hkv) d]
+};
+
 int fail(int code, const char* msg);
 
 // Every host function that launches kernels of this library reports how many it launched; nsa_launch_count() returns
@@ -145,6 +176,13 @@ int launch_rotary(const RotaryParams& P, int dtype, cudaStream_t stream);
 int launch_windows(const WindowParams& P, int dtype, bool backward, cudaStream_t stream);
 int launch_rmsnorm(const NormParams& P, int dtype, bool backward, cudaStream_t stream);
 int launch_combine_gather(const CombineParams& P, const GatherTargets& Gt, int dtype, cudaStream_t stream);
+int launch_layer_prep(const LayerShape& L, const LayerPrep& P, int dtype, cudaStream_t stream);
+int launch_join_mem(const LayerShape& L, const void* mem, const void* ck, const void* cv, void* out, int dtype, cudaStream_t stream);
+int launch_split_mem(const LayerShape& L, const float* grad, void* dc, float* dmem, float* dbias, int dtype, cudaStream_t stream);
+int launch_column_sums(const ColumnSums& P, int dtype, cudaStream_t stream);
+int launch_qkv_grad(const LayerShape& L, const QkvGrad& P, int dtype, cudaStream_t stream);
+int launch_pos_grad(const LayerShape& L, const void* dkw, const void* dvw, float* dpos, int dtype, cudaStream_t stream);
+int launch_round(const float* src, void* dst, int64_t n, cudaStream_t stream);
 int launch_decode(const DecodeParams& P, int dtype, cudaStream_t stream);
 int fill_decode(DecodeParams& P, const nsa_decode_args& a);   // checks the arguments; q and qr may be NULL
 bool project_serves(int batch, int dim, int dtype);

@@ -191,7 +191,7 @@ int launch_rmsnorm(const NormParams& P, int dtype, bool backward, cudaStream_t s
   // the backward adds one partial per block: a few blocks per SM bound the atomics, the forward is a plain stream
   const int64_t cap = backward ? 148 * 2 : 148 * 16;   // backward: the blocks one wave holds (two per SM)
   const unsigned grid = (unsigned)(blocks < cap ? blocks : cap);
-  if (backward) {
+  if (backward && !P.accumulate) {
     const cudaError_t zerr = cudaMemsetAsync(P.dweight, 0, (size_t)P.dim * sizeof(float), stream);
     if (zerr != cudaSuccess) return fail((int)zerr, cudaGetErrorString(zerr));
   }

@@ -10,6 +10,9 @@
 
 namespace nsa {
 
+// Slots at or below 1e-10 are masked out (upstream compares the values in their own type: the constant rounds with it)
+__device__ __forceinline__ float mask_threshold(const SelectParams& P) { return P.round_bf16 ? round_bf16(1e-10f) : 1e-10f; }
+
 __global__ void __launch_bounds__(128) select_kernel(const SelectParams P, int warps_per_block) {
   extern __shared__ float sbuf[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -84,7 +87,9 @@ __global__ void __launch_bounds__(128) select_kernel(const SelectParams P, int w
     }
     if (lane == 0) {
       P.idx[task * P.k + r] = best_i == INT_MAX ? 0 : best_i;
-      P.vals[task * P.k + r] = best_i == INT_MAX ? 0.f : best_v;
+      const float val = best_i == INT_MAX ? 0.f : best_v;
+      if (P.vals != nullptr) P.vals[task * P.k + r] = val;
+      if (P.mask != nullptr) P.mask[task * P.k + r] = val > mask_threshold(P);
     }
     prev_v = best_v;
     prev_i = best_i;
@@ -206,7 +211,8 @@ __device__ __forceinline__ void select_row(const SelectParams& P, int64_t task, 
     }
     if (lane < P.k) {
       P.idx[task * P.k + lane] = my_idx;
-      P.vals[task * P.k + lane] = my_val;
+      if (P.vals != nullptr) P.vals[task * P.k + lane] = my_val;
+      if (P.mask != nullptr) P.mask[task * P.k + lane] = my_val > mask_threshold(P);
     }
     return;
   }
@@ -237,7 +243,8 @@ __device__ __forceinline__ void select_row(const SelectParams& P, int64_t task, 
   }
   if (lane < P.k) {
     P.idx[task * P.k + lane] = my_idx;
-    P.vals[task * P.k + lane] = my_val;
+    if (P.vals != nullptr) P.vals[task * P.k + lane] = my_val;
+    if (P.mask != nullptr) P.mask[task * P.k + lane] = my_val > mask_threshold(P);
   }
 }
 

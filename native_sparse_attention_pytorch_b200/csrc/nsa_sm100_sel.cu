@@ -2236,6 +2236,7 @@ static int run_bwd(const SelProblem& a, const SelPlan& p, uint8_t* ws, cudaStrea
     count_launches(2 + own_delta);   // (delta,) backward kernel, dQ merge
     return NSA_OK;
   }
+  CUDA_TRY(cudaMemsetAsync(P.dq, 0, (size_t)a.B * a.Hq * a.N * D * sizeof(float), st));   // the kernel adds into dq
   constexpr int NC = D / 64;
   const int smem = 1024 + NC * (2 * 16384 + 2 * 8192) + kRows * (D * 4 + 16);
   const int per_sm = D == 64 ? 2 : 1;

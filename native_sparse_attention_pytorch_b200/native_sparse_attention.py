@@ -17,7 +17,7 @@ from torch.nn import Module
 
 from . import _lib as L
 from . import ops
-from .norm import RMSNorm
+from .norm import MAX_PIECES, RMSNorm
 from .rotary import RotaryEmbedding, inverse_frequencies
 
 _has_any_global_hook = nn.modules.module._has_any_global_hook
@@ -30,6 +30,42 @@ def _untouched(module, cls):
     d = module.__dict__
     return module.__class__ is cls and not (d['_forward_hooks'] or d['_forward_pre_hooks'] or d['_backward_hooks'] or
                                             d['_backward_pre_hooks'] or 'forward' in d)
+
+
+class _NativeLayer(torch.autograd.Function):
+    """The layer as one autograd node (csrc/host/layer.cpp): f(call, x, *weights), `call` = (eps, inverse frequencies,
+    configuration)."""
+
+    @staticmethod
+    def forward(ctx, call, x, *weights):
+        eps, inv_freq, cfg = call
+        out, *saved = L.host().layer_forward(x, weights, eps, inv_freq, cfg, ops._status_word(x.device), True, False)
+        ctx.save_for_backward(*weights, *saved)
+        ctx.call = call
+        return out
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, dout):
+        eps, inv_freq, cfg = ctx.call
+        weights, saved = ctx.saved_tensors[:_WEIGHTS], ctx.saved_tensors[_WEIGHTS:]
+        x = saved[0]
+        b, n, _ = x.shape
+        heads, kv_heads, d, window, _, stride, _, _, num_mem, causal, _, _ = cfg
+        # the index of the sliding and the compressed backward depends on the sizes only
+        q = (b, heads, n, d)
+        keys = (('swa', x.device.index, q, (b, kv_heads, n, d), window, bool(causal), L.IMPL_AUTO),
+                ('cmp', x.device.index, q, (b, kv_heads, num_mem + n // stride, d), num_mem, stride, bool(causal), L.IMPL_AUTO))
+        indices = [ops._cached_index(k) for k in keys]
+        *grads, swa_index, cmp_index = L.host().layer_backward(
+            dout, weights, saved, eps, inv_freq, cfg, ops._status_word(x.device), ctx.needs_input_grad[1:], *indices)
+        for key, built in zip(keys, (swa_index, cmp_index)):
+            if built is not None:
+                ops._keep_index(key, built, built.numel())
+        return (None, *grads)
+
+
+_WEIGHTS = 16
 
 
 class _Windows(Module):
@@ -162,6 +198,40 @@ class SparseAttention(Module):
         if w[1].shape != (self._qkv_rows, dim) or w[2].shape != (3 * self.heads, dim) or dim % 8:
             return None
         return w, eps
+
+    def _native_layer(self, x, return_cache):
+        """The whole forward natively, or None where the layer has to run module by module (a chosen kernel family, a
+        plug-in or hooked submodule, a sequence shorter than a compressed block, a cache that carries gradients)."""
+        if self.kernel_impl != 'auto' or not ops.HAND_OVER_DELTA or not ops.REUSE_INDEX:
+            return None
+        d, n = self.dim_head, x.shape[1]
+        if n < self.compress_block_sliding_stride or d % 8 or d > 256 or x.shape[0] == 0 or x.__class__ not in _PLAIN:
+            return None
+        native = self._native_weights(x)
+        if native is None:
+            return None
+        k_net, v_net = self._default_network('k_compress', x), self._default_network('v_compress', x)
+        pos = (self._parameters['k_intrablock_positions'], self._parameters['v_intrablock_positions'])
+        if k_net is None or v_net is None or k_net[0].shape != v_net[0].shape or k_net[0].shape[0] % 8:
+            return None
+        for p in pos:
+            if p.dtype is not x.dtype or p.device != x.device or not p.is_contiguous() or p.__class__ not in _PLAIN:
+                return None
+        w, eps = native
+        weights = (*w, *pos, *k_net, *v_net)
+        cfg = (self.heads, self.kv_heads, d, self.sliding_window_size, self.compress_block_size,
+               self.compress_block_sliding_stride, self.selection_block_size, self.num_selected_blocks,
+               self.num_mem_compress_kv, int(self.causal), int(self.query_heads_share_selected_kv), int(self.use_diff_topk))
+        inv_freq = inverse_frequencies(d, self.rotary_emb.theta, x.device)
+        if torch.is_grad_enabled() and (x.requires_grad or any([p.requires_grad for p in weights if p is not None])):
+            if return_cache or (w[0] is not None and x.shape[2] * x.element_size() > 16 * MAX_PIECES):
+                return None
+            return _NativeLayer.apply((eps, inv_freq, cfg), x, *weights)
+        out, *cache = L.host().layer_forward(x, weights, eps, inv_freq, cfg, ops._status_word(x.device), False, return_cache)
+        if not return_cache:
+            return out
+        keys, vals, ck, cv, run_k, run_v = cache
+        return out, ((keys, vals), ((ck, cv), (run_k, run_v)))
 
     def _split_heads(self, t):
         b, n, _ = t.shape
@@ -296,6 +366,11 @@ class SparseAttention(Module):
         if not inp.is_cuda:
             raise RuntimeError('SparseAttention (B200 kernels) needs CUDA tensors; there is no CPU path here')
         assert not (not self.causal and return_cache)
+
+        if not return_intermediates and forced_selection is None:
+            native = self._native_layer(inp, return_cache)
+            if native is not None:
+                return native
 
         b, n, _ = inp.shape
         h, hkv, d = self.heads, self.kv_heads, self.dim_head

@@ -39,7 +39,7 @@ def _sel_args(q, k, v, out, idx, mask, lse, block, diag, impl, scale):
 _state_lock = threading.Lock()
 _status_acc = {}      # device index -> int32[1] device tensor
 _status_fresh = {}    # device index -> a call has been handed the word since the last poll copied it
-_status_polls = {}    # device index -> (pinned int32[1], event) of the copy issued by the last poll
+_status_polls = {}    # device index -> [copy to the host issued by the last poll (csrc/host/status.cpp), not read yet]
 
 
 def _with_workspace(args, backward, device, sizer='nsa_sel_workspace_bytes'):
@@ -109,29 +109,25 @@ def poll_device_status(device):
     if key is None:
         key = torch.cuda.current_device()
     acc, pending = _status_acc.get(key), _status_polls.get(key)
-    if acc is None or not (_status_fresh.get(key) or (pending is not None and pending[2])):
+    fresh = _status_fresh.get(key)
+    if acc is None or not (fresh or (pending is not None and pending[1])):
         return                          # no such kernel since the last copy, and that copy has been read
-    if pending is not None:
-        host, event, unread = pending
-        if unread and not event.query():
-            return                      # the previous copy is still in flight: look again at the next call
-        code = int(host.item())
-        if code != 0:
-            acc.zero_()
-            with _state_lock:
-                _status_polls.pop(key, None)
-            _raise_for(code)
-        if not _status_fresh.get(key):
-            with _state_lock:
-                _status_polls[key] = (host, event, False)
-            return
-    _status_fresh[key] = False
-    host = pending[0] if pending is not None else torch.zeros(1, dtype=torch.int32).pin_memory()
-    host.copy_(acc, non_blocking=True)
-    event = pending[1] if pending is not None else torch.cuda.Event()
-    event.record(torch.cuda.current_stream(acc.device))
     with _state_lock:
-        _status_polls[key] = (host, event, True)
+        if pending is None:
+            pending = _status_polls[key] = [L.host().StatusCopy(), False]
+        copy, unread = pending
+        code = 0
+        if unread:
+            if not copy.landed():
+                return                  # the previous copy is still in flight: look again at the next call
+            code = copy.value()
+        pending[1] = bool(fresh) and code == 0
+        if pending[1]:
+            _status_fresh[key] = False
+            copy.start(acc)
+    if code != 0:
+        acc.zero_()
+        _raise_for(code)
 
 
 def dim_order(t):

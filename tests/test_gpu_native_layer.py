@@ -1,0 +1,82 @@
+"""The layer as one native call per direction against the same layer run module by module: a forward hook on a submodule
+makes the layer take that path."""
+import pytest
+import torch
+
+import recipe
+from util import assert_close_bf16, assert_close_f32
+
+from native_sparse_attention_pytorch_b200 import SparseAttention
+
+pytestmark = pytest.mark.gpu
+BF16, F32 = torch.bfloat16, torch.float32
+
+# (batch, length, heads, kv heads, head size, dtype, options): gates whose rows are not whole 16-byte pieces, lengths that
+# end inside a block, one block, a length below the overlap of the windows, head sizes without a tensor form, every option
+CASES = [
+    (2, 257, 4, 4, 64, BF16, {}),
+    (1, 1000, 8, 2, 64, BF16, dict(use_diff_topk=True)),
+    (3, 130, 16, 1, 128, BF16, dict(compress_block_size=16, selection_block_size=16)),
+    (1, 20, 4, 2, 64, BF16, dict(compress_block_size=64)),
+    (2, 96, 6, 2, 40, BF16, dict(norm=False)),
+    (1, 515, 4, 2, 64, BF16, dict(num_selected_blocks=0)),
+    (2, 200, 8, 4, 64, BF16, dict(query_heads_share_selected_kv=False, causal=False, use_diff_topk=True)),
+    (2, 140, 6, 3, 64, F32, dict(use_diff_topk=True)),
+    (1, 333, 2, 1, 128, F32, dict(causal=False, num_compressed_mem_kv=3)),
+    (2, 75, 4, 4, 40, F32, dict(query_heads_share_selected_kv=False, norm=False)),
+]
+
+
+def run(layer, x, dout):
+    x = x.clone().requires_grad_()
+    out = layer(x)
+    out.backward(dout)
+    grads = {n: p.grad for n, p in layer.named_parameters()}
+    for p in layer.parameters():
+        p.grad = None
+    return out, x.grad, grads
+
+
+@pytest.mark.parametrize('case', CASES)
+def test_native_layer_equals_the_module_by_module_layer(case):
+    b, n, heads, kv_heads, d, dtype, options = case
+    kw = dict(dim=256, dim_head=d, heads=heads, kv_heads=kv_heads, causal=True, sliding_window_size=70, compress_block_size=32,
+              compress_block_sliding_stride=16, selection_block_size=64, num_selected_blocks=3, use_triton_kernel=True)
+    layer = SparseAttention(**{**kw, **options})
+    recipe.fill_weights(layer, seed=3)
+    layer = layer.to('cuda').to(dtype)
+    layer.to_strategy_combine[0].bias.requires_grad_(False)
+    x, dout = (recipe.randn((b, n, 256), seed).to(dtype).to('cuda') for seed in (5, 6))
+
+    out, dx, grads = run(layer, x, dout)
+    assert 'NativeLayer' in out.grad_fn.name()
+    hook = layer.combine_heads.register_forward_hook(lambda *_: None)
+    want, want_dx, want_grads = run(layer, x, dout)
+    hook.remove()
+    assert 'NativeLayer' not in want.grad_fn.name()
+
+    def close(got, ref, what):
+        if dtype == F32:
+            assert_close_f32(got, ref, what)
+        else:   # the layer's gradients sum in fp32 what the modules add in bf16
+            assert_close_bf16(got, ref, what, roundings=2, rel_to_max=1e-2)
+    close(out, want, 'out')
+    close(dx, want_dx, 'd input')
+    assert grads.keys() == want_grads.keys()
+    for name, ref in want_grads.items():
+        # without selected blocks, or with hard picks, some parameters get no gradient or a zero one
+        if ref is None or grads[name] is None:
+            assert all(g is None or not g.any() for g in (ref, grads[name])), name
+        else:
+            assert grads[name].shape == ref.shape and grads[name].dtype == ref.dtype, name
+            close(grads[name], ref, name)
+
+    if layer.causal:
+        with torch.no_grad():
+            _, cache = layer(x, return_cache=True)
+            hook = layer.combine_heads.register_forward_hook(lambda *_: None)
+            _, ref = layer(x, return_cache=True)
+            hook.remove()
+        for got, want in zip((*cache[0], *cache[1][0], *cache[1][1]), (*ref[0], *ref[1][0], *ref[1][1])):
+            assert got.shape == want.shape and got.dtype == want.dtype
+            close(got, want, 'cache')
