@@ -377,30 +377,6 @@ __device__ __forceinline__ void store_row_bf16(uint32_t tile, int row, const flo
 }
 
 
-// Ships the 128 rows of a staging area (ROW_BYTES each, padded to `stride`) to scattered global rows.  Row r goes to
-// gbase + dst[r] * ROW_BYTES (skipped when dst[r] < 0); ROW_BYTES/16 neighbouring threads share a row, so every
-// store instruction writes whole 128-byte lines.  `t` is the thread's index among the 128 callers, which must have
-// synchronised after filling the staging area and dst[].  (One bulk copy per row would be simpler, but an SM issues
-// only about one bulk copy per 20 cycles, which made that the slowest step of a chunk.)
-template <int ROW_BYTES>
-__device__ __forceinline__ void store_rows_coalesced(uint32_t stage, uint32_t stride, const int* dst,
-                                                     uint8_t* gbase, int t) {
-  constexpr int TPR = ROW_BYTES / 16;
-  constexpr int RPP = kRows / TPR;
-  const int sub = t % TPR, r0 = t / TPR;
-  uint4 v[TPR];
-  int d[TPR];
-#pragma unroll
-  for (int k = 0; k < TPR; ++k) {
-    const int row = r0 + k * RPP;
-    d[k] = dst[row];
-    v[k] = lds_v4(stage + row * stride + sub * 16);
-  }
-#pragma unroll
-  for (int k = 0; k < TPR; ++k)
-    if (d[k] >= 0) *reinterpret_cast<uint4*>(gbase + (int64_t)d[k] * ROW_BYTES + sub * 16) = v[k];
-}
-
 // ---- forward -------------------------------------------------------------------------
 
 // Forward of the selected-block branch.  A CTA of 256 threads walks gather -> S -> softmax -> P V -> store chunk by
@@ -777,366 +753,454 @@ __global__ void __launch_bounds__(256) sel_merge_combine_kernel(const SelParams 
 // ---- forward of the dense causal branches, query-tile stationary ---------------------------------------------
 //
 // The compressed and the sliding-window branch attend a contiguous range of key blocks per query, the same range for
-// neighbouring queries.  For them the key-block-stationary form above pays for partial results it does not need: one
-// CTA here owns a tile of 128/G consecutive queries (128 rows with the G heads of the group), walks the key blocks
-// the tile can see and keeps the running maximum and sum of every row in registers and the output accumulator in
-// tensor memory, as a flash-attention forward does.  No index, no partial results, no merge.
-//   * Two threads share a row (32 of a block's 64 columns each; they exchange their maxima through shared memory),
-//     so a CTA has eight warps to hide latencies with.
-//   * S of block t+2 is issued as soon as P of block t has been handed to the PV MMA, so the tensor cores work on
-//     PV(t) and S(t+2) while the threads do the softmax of block t+1 (two S buffers in tensor memory, two K and two V
-//     buffers in shared memory, filled by TMA).
+// neighbouring queries.  For them the key-block-stationary form above pays for partial results it does not need: here a
+// tile of 128/G consecutive queries (128 rows with the G heads of the group) stays, the key blocks it can see pass by,
+// and the output accumulator stays in tensor memory, as in a flash-attention forward.  No index, no partial results.
+// One persistent CTA per SM with fixed roles:
+//   warps 0-7, 8-15 two streams: each has its own query tile (neighbours of one head), two S buffers and its own O in
+//                   tensor memory.  Two threads share a row (32 of a block's 64 columns each; they exchange maxima).
+//                   Softmax of block t: read S, importance, maximum, exponentials, P back over S's columns as bf16.
+//   warps 16, 17    issue the tcgen05.mma of a stream each: PV(t), then S(t+2) into the buffer that PV(t) has just read;
+//                   S of the next tile's first blocks follows the last PV without a gap.
+//   warp 18         TMA: K and V blocks through a ring shared by both streams, and the next Q tiles as soon as the last S
+//                   of the present ones is complete.
+// What bounds it: per 128 x 64 tile the exponentials take 512 cycles (16 per clock) and the tensor cores 512 at dim_head
+// 128; the roles reach about three times that (compressed branch with pooled importance 2000 cycles, sliding 1500), most
+// of it waits inside the softmax warps.  Sharing K / V matters: tile loads run at 29 bytes per clock and SM, 1100 cycles
+// for the 32 KB of a key block at dim_head 128.  One issuing warp per stream, because an issuing warp needs some 100
+// cycles per MMA next to the softmax warps: one for both streams took 15 % longer.
+// 65536 positions, 64 / 8 heads of 128: compressed 11.5 -> 7.6 ms, sliding (window 512) 2.6 -> 1.8 ms; 2 x 16384, 16 / 4
+// heads of 64: 419 -> 309 us and 290 -> 180 us (before: two CTAs per SM that walked the stages one after the other).
 //   * The accumulator is rescaled lazily: a row keeps its reference maximum until a block exceeds it by more than 2^8;
 //     only then is the O row read from tensor memory, scaled and written back (P stays below 2^8, exact in bf16's
 //     range, and the sum is fp32).
 //   * MODE compressed with IMP also writes the head-averaged logits of the visible columns (the importance), or with
 //     POOL their per-selection-block means: the head means of the last 128 compressed columns of every query wait in
-//     a ring in shared memory, and after every key block the threads average the selection blocks it completed.
+//     a ring in shared memory, and after every key block its two warps average the selection blocks it completed.
+namespace dense {
+constexpr int kStreams = 2, kSoftmaxWarps = 16, kThreads = (kSoftmaxWarps + kStreams + 1) * 32;
+constexpr int kRingCols = 192 + 16;          // POOL: columns per query, three key blocks' worth (rows padded against bank conflicts)
+constexpr uint32_t kImpTile = 32 * 64;       // per warp: the scaled logits of its half rows as bf16
+template <int D>
+struct Shape {
+  static constexpr int NC = D / 64;
+  static constexpr int kBufs = D == 64 ? 4 : 3;                                 // K and V blocks in flight
+  static constexpr uint32_t kTileQ = NC * 16384, kTileKV = NC * 8192;
+  static constexpr uint32_t kTiles = kStreams * kTileQ + 2 * kBufs * kTileKV;
+};
+__host__ __device__ constexpr uint32_t pool_bytes(int G) { return (uint32_t)(32 / G) * kRingCols * 2; }   // per pair of warps
+template <int D>
+constexpr uint32_t smem_bytes(int imp_heads, bool pool) {
+  return Shape<D>::kTiles + (imp_heads > 0 ? kSoftmaxWarps * kImpTile : 0) + (pool ? 8 * pool_bytes(imp_heads) : 0);
+}
+struct Bars {
+  uint64_t q_full[2], q_free[2];
+  uint64_t k_full[4], k_free[4], v_full[4], v_free[4];
+  // per S buffer: a stream may be two blocks ahead of its PV, and a waiter must know the phase before its own complete
+  uint64_t s_full[2][2], p_full[2][2], pv_done[2][2];
+  uint64_t drain[2];
+};
+// Byte offset of 16-byte piece c of row r in a warp's tile of 64-byte rows: no bank conflicts between the rows of eight
+// lanes that write, nor between the lanes of neighbouring queries (G rows each) that read.
+template <int G>
+__device__ __forceinline__ uint32_t imp_offset(int r, int c) {
+  return (uint32_t)((r * 64) ^ (((r / G) & 1) << 6)) + ((uint32_t)(c ^ ((r >> 1) & 3)) << 4);
+}
+// The sum of G values in the order of a butterfly over neighbouring lanes
+template <int G>
+__device__ __forceinline__ float tree_sum(const float* a) {
+  if constexpr (G == 1) return a[0];
+  else return tree_sum<G / 2>(a) + tree_sum<G / 2>(a + G / 2);
+}
+}  // namespace dense
+
 template <int D, int MODE, int GI, bool POOL = false>   // GI: 0 = no importance output, else the heads per KV head
-__global__ void __launch_bounds__(2 * kRows, 2)
-dense_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const SelParams P) {
-  constexpr int NC = D / 64;
-  constexpr uint32_t kTileQ = NC * 16384, kTileKV = NC * 8192;
-  constexpr uint32_t kStageStride = D * 2 + 16;
-  constexpr uint32_t kCols = 256;
-  constexpr int kThreads = 2 * kRows;   // two threads per row: each owns 32 of the 64 columns of a key block
-  // The dynamic segment is declared 1024-byte aligned (the swizzled tiles need it) and holds exactly the tiles: with
-  // dim_head 128 two CTAs then fill an SM's shared memory to the byte.
+__global__ void __launch_bounds__(dense::kThreads, 1)
+dense_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+                 const SelParams P, const int streams) {
+  using namespace dense;
+  using S = Shape<D>;
+  constexpr int NC = S::NC, kBufs = S::kBufs;
+  constexpr uint32_t kTileQ = S::kTileQ, kTileKV = S::kTileKV;
   extern __shared__ __align__(1024) uint8_t dense_smem[];
   __shared__ int abort_flag;
   __shared__ uint32_t tmem_slot;
-  __shared__ __align__(8) uint64_t bars[8];
+  __shared__ __align__(8) Bars bars;
+  __shared__ float xchg[2][kStreams][2][kRows];   // maxima (and, at the end, sums) of the two threads of a row
 
-  const uint32_t base = smem_u32(dense_smem);
-  const uint32_t sQ = base, sX = sQ + kTileQ, sK0 = sX + 16384, sV0 = sK0 + 2 * kTileKV;
-  // sX (16 KB): the two threads of a row exchange their partial maxima (and, at the end, sums) through it.  The Q tile
-  // and sX become the staging area of the output rows at the end, followed by the rows' destinations.
-  const uint32_t sStage = sQ;
-  int* const row_dst = reinterpret_cast<int*>(dense_smem + kRows * kStageStride);
-  float* const xchg = reinterpret_cast<float*>(dense_smem + kTileQ);   // [2 halves][kRows]
-  // POOL: the head means of the last 128 logit columns of every query of the tile, [QT][kRing] bf16 (rows padded so
-  // that neighbouring queries fall on different banks)
-  constexpr int kRing = 128 + 32;
-  __nv_bfloat16* const ring = reinterpret_cast<__nv_bfloat16*>(dense_smem + kTileQ + 1024);
-  // barriers: K buffers full (2), V buffers full (2), S buffers complete (2), PV complete, drain
-  const uint32_t bar0 = smem_u32(&bars[0]), bar_pv = bar0 + 48;
-  auto bar_k = [&](int t) { return bar0 + (uint32_t)(t & 1) * 8; };
-  auto bar_v = [&](int t) { return bar0 + 16 + (uint32_t)(t & 1) * 8; };
-  auto bar_s = [&](int t) { return bar0 + 32 + (uint32_t)(t & 1) * 8; };
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int half = tid >> 7, row = tid & (kRows - 1);
+  const uint32_t sQ0 = smem_u32(dense_smem), sK0 = sQ0 + kStreams * kTileQ, sV0 = sK0 + kBufs * kTileKV;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (tid == 0) {
     abort_flag = 0;
-    for (int i = 0; i < 8; ++i) mbar_init(smem_u32(&bars[i]), 1);
-    if (base & 1023u) abort_flag = 1;   // the tiles would be mis-swizzled: report instead of computing
+    if (sQ0 & 1023u) abort_flag = 1;   // the tiles would be mis-swizzled: report instead of computing
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(smem_u32(&bars.q_full[s]), 1);
+      mbar_init(smem_u32(&bars.q_free[s]), 1);
+      for (int i = 0; i < 2; ++i) {
+        mbar_init(smem_u32(&bars.s_full[s][i]), 1);
+        mbar_init(smem_u32(&bars.p_full[s][i]), 2 * kRows);
+        mbar_init(smem_u32(&bars.pv_done[s][i]), 1);
+      }
+    }
+    for (int i = 0; i < kBufs; ++i) {
+      mbar_init(smem_u32(&bars.k_full[i]), 1);
+      mbar_init(smem_u32(&bars.k_free[i]), streams);
+      mbar_init(smem_u32(&bars.v_full[i]), 1);
+      mbar_init(smem_u32(&bars.v_free[i]), streams);
+    }
+    mbar_init(smem_u32(&bars.drain[0]), 1);
+    mbar_init(smem_u32(&bars.drain[1]), 1);
     fence_mbar_init();
+    prefetch_tensormap(&tmQ);
     prefetch_tensormap(&tmK);
     prefetch_tensormap(&tmV);
   }
   __syncthreads();
   if (warp == 0) {
-    tmem_alloc(smem_u32(&tmem_slot), kCols);
+    tmem_alloc(smem_u32(&tmem_slot), 512);
     tmem_relinquish();
   }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tm = tmem_slot;
-  const uint32_t tm_lane = tm + ((uint32_t)((warp & 3) * 32) << 16);   // warps w and w + 4 share a lane quarter
-  const uint32_t tO = 128;
-  constexpr uint32_t idS = instr_desc_bf16(128, 64, false, false);
-  constexpr uint32_t idO = instr_desc_bf16(128, D, false, true);
+  const uint32_t tm = tmem_slot;                 // stream s: S buffers at 256 s and 256 s + 64, O at 256 s + 128
+  constexpr uint32_t tO = 128;
 
-  // the tile: heavy tiles (late queries) are launched first
+  // The n-th pair of tiles: late queries, which see the most blocks, first; heads side by side
   constexpr bool IMP = GI > 0;
-  const int G = IMP ? GI : P.G, QT = kRows / G, g_shift = 31 - __clz(G);
-  const int tiles_per_head = (P.N + QT - 1) / QT;
-  const int64_t tile = (int64_t)gridDim.x - 1 - blockIdx.x;
-  const int qt = (int)(tile % tiles_per_head), bh = (int)(tile / tiles_per_head), h = bh % P.Hkv, b = bh / P.Hkv;
-  const int i0 = qt * QT, i_last = min(i0 + QT - 1, P.N - 1);
-  const int q_local = row >> g_shift, g = row - (q_local << g_shift);
-  const int i = i0 + q_local;
-  const bool valid = i < P.N;
-  const int64_t hq = (int64_t)h * G + g;
-  int jb, je;
-  if (MODE == kModeCmp) {
-    jb = 0;
-    je = min(P.nfb, (P.rule.num_mem + i_last / P.rule.stride + kBlock - 1) / kBlock);
-  } else {
-    jb = max(0, i0 - P.rule.window) / kBlock;
-    je = i_last / kBlock + 1;
-  }
-  const int nb = je - jb;
-
-  // Q rows of the tile (zero rows past the end of the sequence) and the first K/V blocks
-  {
-    constexpr int CH = D / 8, RPP = kThreads / CH;
-    const int sub = tid % CH, r0 = tid / CH;
-    const __nv_bfloat16* qb = P.q + b * P.q_sb;
-#pragma unroll
-    for (int it = 0; it < kRows / RPP; ++it) {
-      const int rr = r0 + it * RPP;
-      const int qi = i0 + (rr >> g_shift), gg = rr & ((1 << g_shift) - 1);
-      const bool ok = qi < P.N;
-      cp_async16(sQ + (sub / 8) * (kRows * 128) + sw128_offset(rr, sub % 8),
-                 qb + (int64_t)((h << g_shift) + gg) * P.q_sh + (int64_t)(ok ? qi : 0) * P.q_sn + sub * 8, ok ? 16u : 0u);
-    }
-    cp_async_commit();
-  }
-  auto load_k = [&](int t) {   // thread 0: key block jb + t into K buffer t & 1
-    mbar_arrive_expect_tx(bar_k(t), kTileKV);
-#pragma unroll
-    for (int c = 0; c < NC; ++c) tma_load_4d(sK0 + (t & 1) * kTileKV + c * 8192, &tmK, bar_k(t), c * 64, (jb + t) * kBlock, h, b);
-  };
-  auto load_v = [&](int t) {
-    mbar_arrive_expect_tx(bar_v(t), kTileKV);
-#pragma unroll
-    for (int c = 0; c < NC; ++c) tma_load_4d(sV0 + (t & 1) * kTileKV + c * 8192, &tmV, bar_v(t), c * 64, (jb + t) * kBlock, h, b);
-  };
-  auto issue_s = [&](int t) {   // warp 0, converged: S(t) = Q K(t)^T into S buffer t & 1
-    mbar_wait_bounded(bar_k(t), (uint32_t)(t >> 1) & 1, &abort_flag);
-    __syncwarp();
-    tc_fence_after_sync();
-    const uint32_t sK = sK0 + (t & 1) * kTileKV;
-#pragma unroll
-    for (int k = 0; k < D / 16; ++k) {
-      const uint32_t ch = k / 4, in = (k % 4) * 32;
-      mma_bf16_elect(tm + (t & 1) * 64, smem_desc_sw128(sQ + ch * 16384 + in, 16), smem_desc_sw128(sK + ch * 8192 + in, 16),
-                     idS, k > 0);
-    }
-    mma_commit_elect(bar_s(t));
-  };
-  if (tid == 0) {
-    load_k(0);
-    load_v(0);
-    if (nb > 1) load_k(1);
-  }
-  cp_async_wait<0>();
-  fence_proxy_async_smem();
-  __syncthreads();
-  if (warp == 0) {
-    issue_s(0);
-    if (nb > 1) issue_s(1);
-  }
-
-  // POOL: selection blocks per key block, and the (batch, head) slice of the pooled output
-  const int cpf_shift = POOL ? 31 - __clz(P.cpf) : 0, kb_shift = 6 - cpf_shift;
-  const float inv_cpf = POOL ? 1.f / (float)P.cpf : 1.f;
-  __nv_bfloat16* const pooled_head = POOL ? P.pooled + ((int64_t)b * P.Hkv + h) * P.N * P.pool_cols : nullptr;
-
-  float m_ref = -INFINITY, l = 0.f;   // l: this thread's half of the row sum
-  for (int t = 0; t < nb; ++t) {
-    const int j = jb + t, sb = t & 1;
-    __syncwarp();
-    mbar_wait_warp(bar_s(t), (uint32_t)(t >> 1) & 1, &abort_flag);
-    tc_fence_after_sync();
-    if (tid == 0 && t + 2 < nb) load_k(t + 2);   // S(t) is complete: its K buffer is free
-    __syncwarp();
-    float s[32];
-    tmem_ld32(tm_lane + sb * 64 + half * 32, s);
-    tmem_ld_wait();
-    // visible columns of this block for this row, relative to this thread's half
-    int lo = 0, lim;
+  const int G = IMP ? GI : P.G, QT = kRows / G, g_shift = 31 - __clz(G), span = QT * streams;
+  const int spans = (P.N + span - 1) / span, heads = P.B * P.Hkv, total = spans * heads;
+  struct Tile { int i0, h, b, jb, nb; };
+  auto tile_at = [&](int n) {
+    Tile t;
+    const int back = n / heads, bh = n - back * heads;
+    t.b = bh / P.Hkv;
+    t.h = bh - t.b * P.Hkv;
+    t.i0 = (spans - 1 - back) * span;
+    const int i_last = min(t.i0 + span - 1, P.N - 1);
+    int je;
     if (MODE == kModeCmp) {
-      lim = min(kBlock - 1, P.rule.num_mem + i / P.rule.stride - 1 - j * kBlock);
+      t.jb = 0;
+      je = min(P.nfb, (P.rule.num_mem + i_last / P.rule.stride + kBlock - 1) / kBlock);
     } else {
-      lim = min(kBlock - 1, i - j * kBlock);
-      lo = max(0, i - P.rule.window - j * kBlock);
+      t.jb = max(0, t.i0 - P.rule.window) / kBlock;
+      je = i_last / kBlock + 1;
     }
-    if (!valid) lim = -1;
-    lim -= half * 32;
-    lo -= half * 32;
-    if constexpr (IMP) {
-      // the scaled logit of every visible block column, averaged over the G heads of the query (G neighbouring
-      // lanes), as the tensor of that dtype would hold it upstream: product, scaled logit and mean each rounded to
-      // bf16.  The G lanes reduce-scatter: every step a lane hands half of its columns to its partner and keeps the
-      // other half, so that it ends with 32/G fully summed columns, which it stores.
-      float v[32];
+    t.nb = je - t.jb;
+    return t;
+  };
+
+  if (warp < kSoftmaxWarps) {
+    // ------------------------------------------------------------------ softmax: two threads per row, 32 columns each
+    const int s = warp >> 3, half = (warp >> 2) & 1, row = (warp & 3) * 32 + lane;
+    const int q_local = row >> g_shift, g = row - (q_local << g_shift);
+    const uint32_t tm_lane = tm + s * 256 + ((uint32_t)((warp & 3) * 32) << 16);   // warps w and w + 4 share a lane quarter
+    const int pair = s * 4 + (warp & 3);
+    const uint32_t imp_tile = sQ0 + S::kTiles + warp * kImpTile;
+    __nv_bfloat16* const ring = reinterpret_cast<__nv_bfloat16*>(dense_smem + S::kTiles + kSoftmaxWarps * kImpTile + pair * pool_bytes(IMP ? GI : 1));
+    auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory"); };
+    const int cpf_shift = POOL ? 31 - __clz(P.cpf) : 0, kb_shift = 6 - cpf_shift;   // selection blocks per key block
+    const float inv_cpf = POOL ? 1.f / (float)P.cpf : 1.f;
+    uint32_t u = 0;
+    int slot = 0;                                // POOL: the ring's place for the present key block
+    for (int n = s < streams ? (int)blockIdx.x : total; n < total; n += gridDim.x) {
+      const Tile tile = tile_at(n);
+      const int i = tile.i0 + s * QT + q_local;
+      const bool valid = i < P.N;
+      // last and first visible key, relative to this thread's half of a block
+      const int lim_tile = (MODE == kModeCmp ? P.rule.num_mem + i / P.rule.stride - 1 : i) - half * 32;
+      const int lo_tile = i - P.rule.window - half * 32;
+      float m_ref = -INFINITY, l = 0.f;          // l: this thread's half of the row sum
+      for (int t = 0; t < tile.nb; ++t, ++u) {
+        const int j = tile.jb + t;
+        const uint32_t tS = tm_lane + (u & 1) * 64;
+        mbar_wait_warp(smem_u32(&bars.s_full[s][u & 1]), (u >> 1) & 1, &abort_flag);
+        tc_fence_after_sync();
+        float x0[32];
+        tmem_ld32(tS + half * 32, x0);
+        tmem_ld_wait();
+        const int lim = valid ? lim_tile - j * kBlock : -1;
+        const int lo = MODE == kModeCmp ? 0 : lo_tile - j * kBlock;
+        if constexpr (IMP) {
+          // the scaled logit of every visible block column, averaged over the G heads of the query (G neighbouring
+          // rows), as the tensor of that dtype would hold it upstream: product, scaled logit and mean each rounded to
+          // bf16.  The half rows of the warp go through shared memory; every lane then sums 32/G columns of its query
+          // over the heads (half the instructions of a reduce-scatter by shuffles).
+          constexpr int OWN = 32 / (IMP ? GI : 1);
+          constexpr float inv_g = 1.f / (float)(IMP ? GI : 1);
+          float mean[OWN];
 #pragma unroll
-      for (int x = 0; x < 32; ++x) v[x] = round_bf16(round_bf16(s[x]) * P.scale);
-      int first = 0;
+          for (int c = 0; c < 4; ++c) {
+            uint32_t w[4];
 #pragma unroll
-      for (int step = 0; step < 4; ++step) {
-        constexpr int kG = IMP ? GI : 1;
-        const int width = 16 >> step;
-        if ((1 << step) < kG) {
-          const bool upper = (g >> step) & 1;
+            for (int k = 0; k < 4; ++k) {
+              const uint32_t r = pack_bf16(x0[c * 8 + 2 * k], x0[c * 8 + 2 * k + 1]);   // (one value at a time would convert at a quarter of the rate)
+              w[k] = pack_bf16(__uint_as_float(r << 16) * P.scale, __uint_as_float(r & 0xffff0000u) * P.scale);
+            }
+            if constexpr (GI == 1) {
 #pragma unroll
-          for (int x = 0; x < 16; ++x) {
-            if (x < width) {
-              const float give = upper ? v[x] : v[x + width];
-              const float keep = upper ? v[x + width] : v[x];
-              v[x] = keep + __shfl_xor_sync(kFullMask, give, 1 << step);
+              for (int k = 0; k < 4; ++k) {
+                mean[c * 8 + 2 * k] = __uint_as_float(w[k] << 16);
+                mean[c * 8 + 2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u);
+              }
+            } else {
+              sts_v4(imp_tile + imp_offset<GI>(lane, c), make_uint4(w[0], w[1], w[2], w[3]));
             }
           }
-          first += upper ? width : 0;
+          const int group = lane & ((IMP ? GI : 1) - 1), first_row = lane - group, first = group * OWN;
+          if constexpr (GI > 1) {
+            __syncwarp();
+            constexpr int PIECE = OWN < 8 ? OWN : 8;          // columns per load
+#pragma unroll
+            for (int p = 0; p < OWN / PIECE; ++p) {
+              uint32_t w[GI][PIECE / 2];
+#pragma unroll
+              for (int k = 0; k < GI; ++k) {
+                const int col = first + p * PIECE;
+                const uint32_t at = imp_tile + imp_offset<GI>(first_row + k, col >> 3) + (col & 7) * 2;
+                if constexpr (PIECE == 8) {
+                  const uint4 v = lds_v4(at);
+                  w[k][0] = v.x; w[k][1] = v.y; w[k][2] = v.z; w[k][3] = v.w;
+                } else if constexpr (PIECE == 4) {
+                  const uint2 v = lds_v2(at);
+                  w[k][0] = v.x; w[k][1] = v.y;
+                } else {
+                  w[k][0] = lds_u32(at);
+                }
+              }
+#pragma unroll
+              for (int c = 0; c < PIECE; ++c) {
+                float a[GI];
+#pragma unroll
+                for (int k = 0; k < GI; ++k) a[k] = __uint_as_float(c & 1 ? w[k][c / 2] & 0xffff0000u : w[k][c / 2] << 16);
+                mean[p * PIECE + c] = tree_sum<GI>(a);
+              }
+            }
+          }
+          if constexpr (POOL) {
+            uint32_t* dst = reinterpret_cast<uint32_t*>(ring + (lane >> g_shift) * kRingCols + slot * kBlock + half * 32 + first);
+#pragma unroll
+            for (int x = 0; x < OWN / 2; ++x) dst[x] = pack_bf16(mean[2 * x] * inv_g, mean[2 * x + 1] * inv_g);
+          } else {
+            float* imp_row = P.importance + (((int64_t)tile.b * P.Hkv + tile.h) * P.N + (valid ? i : 0)) * P.ncb;
+            const int col0 = j * kBlock + half * 32 + first - P.rule.num_mem;
+#pragma unroll
+            for (int x = 0; x < OWN; ++x) {
+              const int col = col0 + x;
+              if (first + x <= lim && col >= 0 && col < P.ncb) imp_row[col] = round_bf16(mean[x] * inv_g);
+            }
+          }
         }
-      }
-      constexpr int owned = 32 / (IMP ? (GI > 16 ? 16 : GI) : 1);
-      float* imp_row = P.importance + (((int64_t)b * P.Hkv + h) * P.N + (valid ? i : 0)) * P.ncb;
-      constexpr float inv_g = 1.f / (float)(IMP ? GI : 1);
-      const int col0 = j * kBlock + half * 32 + first - P.rule.num_mem;
-      if constexpr (POOL) {
-        // this lane's `owned` neighbouring columns in one store (indexed by logit column, memory slots included)
-        uint32_t w[owned / 2];
+        // most blocks are fully visible to every row of the warp: the others are masked first
+        if (!__all_sync(kFullMask, lim >= 31 && lo <= 0)) {
 #pragma unroll
-        for (int x = 0; x < owned / 2; ++x) w[x] = pack_bf16(v[2 * x] * inv_g, v[2 * x + 1] * inv_g);
-        __nv_bfloat16* dst = ring + q_local * kRing + ((j & 1) * kBlock + half * 32 + first);
-        if constexpr (owned == 2) *reinterpret_cast<uint32_t*>(dst) = w[0];
-        else if constexpr (owned == 4) *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
-        else *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
-      } else {
-#pragma unroll
-        for (int x = 0; x < owned; ++x) {
-          const int col = col0 + x;
-          if (valid && first + x <= lim && col >= 0 && col < P.ncb) imp_row[col] = round_bf16(v[x] * inv_g);
+          for (int x = 0; x < 32; ++x)
+            if (x < lo || x > lim) x0[x] = -INFINITY;
         }
-      }
-    }
-    // most blocks are fully visible to every row of the warp: they take the loops without per-column tests
-    const bool all_full = __all_sync(kFullMask, lim >= 31 && lo <= 0);
-    float m = -INFINITY;
-    if (all_full) {
+        float mm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-      for (int x = 0; x < 32; ++x) m = fmaxf(m, s[x]);
-    } else {
-#pragma unroll
-      for (int x = 0; x < 32; ++x) m = ((MODE == kModeCmp || x >= lo) && x <= lim) ? fmaxf(m, s[x]) : m;
-    }
-    // the row maximum over both halves
-    xchg[half * kRows + row] = m;
-    __syncthreads();
-    m = fmaxf(m, xchg[(half ^ 1) * kRows + row]);
-    if constexpr (POOL) {
-      // the selection blocks whose last column this key block brought: mean of their cpf columns in the order and
-      // with the roundings of the selection kernel's own averaging; only blocks wholly before the query's own block
-      // are stored (all others have probability 0 in the selection, whatever their logits)
-      const int nm = P.rule.num_mem;
-      const int b_lo = t == 0 ? 0 : (j * kBlock - nm) >> cpf_shift;
-      const int b_hi = min(P.pool_cols, (j * kBlock + kBlock - nm) >> cpf_shift);
-      for (int e = tid; e < (QT << kb_shift); e += kThreads) {
-        const int pq = e >> kb_shift, bb = b_lo + (e & ((1 << kb_shift) - 1));
-        const int qi = i0 + pq;
-        if (bb < b_hi && qi < P.N && (bb + 1) * P.pool_block <= qi) {
-          const __nv_bfloat16* src = ring + pq * kRing;
-          const int c0 = (bb << cpf_shift) + nm;
-          float sum = 0.f;
-          for (int c = 0; c < (1 << cpf_shift); ++c) sum += __bfloat162float(src[(c0 + c) & 127]);
-          pooled_head[(int64_t)qi * P.pool_cols + bb] = __float2bfloat16_rn(sum * inv_cpf);   // cpf is a power of two
+        for (int x = 0; x < 32; ++x) mm[x & 3] = fmaxf(mm[x & 3], x0[x]);
+        float m = fmaxf(fmaxf(mm[0], mm[1]), fmaxf(mm[2], mm[3]));
+        // the row maximum over both halves; behind the barrier both have also read their S columns and written the ring
+        xchg[u & 1][s][half][row] = m;
+        pair_sync();
+        m = fmaxf(m, xchg[u & 1][s][half ^ 1][row]);
+        if constexpr (POOL) {
+          // the selection blocks whose last column this key block brought: mean of their cpf columns in the order and
+          // with the roundings of the selection kernel's own averaging; only blocks wholly before the query's own block
+          // are stored (all others have probability 0 in the selection, whatever their logits)
+          const int nm = P.rule.num_mem, before = slot == 0 ? 2 : slot - 1;
+          const int b_lo = t == 0 ? 0 : (j * kBlock - nm) >> cpf_shift;
+          const int b_hi = min(P.pool_cols, (j * kBlock + kBlock - nm) >> cpf_shift);
+          const int q0 = tile.i0 + s * QT + (((warp & 3) * 32) >> g_shift);
+          __nv_bfloat16* const pooled_head = P.pooled + ((int64_t)tile.b * P.Hkv + tile.h) * P.N * P.pool_cols;
+          for (int e = half * 32 + lane; e < ((32 / GI) << kb_shift); e += 64) {
+            const int pq = e >> kb_shift, bb = b_lo + (e & ((1 << kb_shift) - 1));
+            const int qi = q0 + pq;
+            if (bb < b_hi && qi < P.N && (bb + 1) * P.pool_block <= qi) {
+              const __nv_bfloat16* src = ring + pq * kRingCols;
+              const int c0 = (bb << cpf_shift) + nm - j * kBlock;   // negative: in the key block before
+              float sum = 0.f;
+              for (int c = 0; c < (1 << cpf_shift); ++c)
+                sum += __bfloat162float(src[c0 + c >= 0 ? slot * kBlock + c0 + c : (before + 1) * kBlock + c0 + c]);
+              pooled_head[(int64_t)qi * P.pool_cols + bb] = __float2bfloat16_rn(sum * inv_cpf);   // cpf is a power of two
+            }
+          }
+          slot = slot == 2 ? 0 : slot + 1;   // three places: the next block's may be written while a slow warp still reads
         }
-      }
-    }
-    const float m_blk2 = m * P.scale_log2;   // -inf when the row sees nothing of this block
-    bool need = false;
-    float alpha = 1.f;
-    if (m_ref == -INFINITY) {
-      m_ref = m_blk2;
-    } else if (m_blk2 > m_ref + 8.f) {
-      alpha = ex2(m_ref - m_blk2);
-      m_ref = m_blk2;
-      l *= alpha;
-      need = true;
-    }
-    if (t > 0 && __any_sync(kFullMask, need)) {
-      // some row of this warp outgrew its reference maximum: scale the accumulator rows (PV(t-1) must be complete);
-      // each half scales its half of the output columns
-      mbar_wait_warp(bar_pv, (uint32_t)(t - 1) & 1, &abort_flag);
-      tc_fence_after_sync();
+        const float m_blk2 = m * P.scale_log2;   // -inf: nothing visible
+        bool need = false;
+        float alpha = 1.f;
+        if (m_ref == -INFINITY) {
+          m_ref = m_blk2;
+        } else if (m_blk2 > m_ref + 8.f) {
+          alpha = ex2(m_ref - m_blk2);
+          m_ref = m_blk2;
+          l *= alpha;
+          need = true;
+        }
+        if (t > 0 && __any_sync(kFullMask, need)) {
+          // some row of this warp outgrew its reference maximum: scale the accumulator rows (PV(t-1) must be complete);
+          // each half scales its half of the output columns
+          mbar_wait_warp(smem_u32(&bars.pv_done[s][(u - 1) & 1]), ((u - 1) >> 1) & 1, &abort_flag);
+          tc_fence_after_sync();
 #pragma unroll 1
-      for (int c2 = 0; c2 < D / 32; ++c2) {
-        float o[16];
-        tmem_ld16(tm_lane + tO + half * (D / 2) + c2 * 16, o);
-        tmem_ld_wait();
+          for (int c = half * (D / 2); c < (half + 1) * (D / 2); c += 16) {
+            float o[16];
+            tmem_ld16(tm_lane + tO + c, o);
+            tmem_ld_wait();
 #pragma unroll
-        for (int x = 0; x < 16; ++x) o[x] *= alpha;
-        tmem_st16(tm_lane + tO + half * (D / 2) + c2 * 16, o);
-      }
-      tmem_st_wait();
-    }
-    if (all_full) {
+            for (int x = 0; x < 16; ++x) o[x] *= alpha;
+            tmem_st16(tm_lane + tO + c, o);
+          }
+          tmem_st_wait();
+        }
+        // a masked logit is -inf and gives 0; a row that has seen nothing yet must not compute -inf - -inf
+        const float off = m_ref == -INFINITY ? 0.f : -m_ref;
+        float ll[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int x = 0; x < 32; ++x) {
-        const float p = ex2(s[x] * P.scale_log2 - m_ref);
-        s[x] = p;
-        l += p;
+        for (int x = 0; x < 32; ++x) {
+          x0[x] = ex2(fmaf(x0[x], P.scale_log2, off));
+          ll[x & 3] += x0[x];
+        }
+        l += (ll[0] + ll[1]) + (ll[2] + ll[3]);
+        // P through tensor memory, over the first 32 columns of the row's S; S(t+2), which is issued after PV(t) by the
+        // same lane, overwrites them only after PV(t) has read them
+        tmem_st_bf16_row32(tS + half * 16, x0);
+        tmem_st_wait();
+        tc_fence_before_sync();
+        mbar_arrive(smem_u32(&bars.p_full[s][u & 1]));
       }
-    } else {
-#pragma unroll
-      for (int x = 0; x < 32; ++x) {
-        const float p = ((MODE == kModeCmp || x >= lo) && x <= lim) ? ex2(s[x] * P.scale_log2 - m_ref) : 0.f;
-        s[x] = p;
-        l += p;
-      }
-    }
-    if (t > 0) {   // PV(t-1) is complete: V buffer (t-1) & 1 is free
-      mbar_wait_warp(bar_pv, (uint32_t)(t - 1) & 1, &abort_flag);
+      // output row: O / l
+      xchg[u & 1][s][half][row] = l;
+      mbar_wait_warp(smem_u32(&bars.pv_done[s][(u - 1) & 1]), ((u - 1) >> 1) & 1, &abort_flag);
       tc_fence_after_sync();
+      pair_sync();
+      l += xchg[u & 1][s][half ^ 1][row];
+      const int64_t row_global = ((int64_t)tile.b * P.Hq + (int64_t)tile.h * G + g) * P.N + (valid ? i : 0);
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      // every thread stores its half of the row: four 16-byte pieces (two whole sectors) at a time, once per tile
+      __nv_bfloat16* const out_row = P.out + row_global * D + half * (D / 2);
+#pragma unroll 1
+      for (int c = 0; c < D / 2; c += 32) {
+        float o[32];
+        tmem_ld32(tm_lane + tO + half * (D / 2) + c, o);
+        tmem_ld_wait();
+        if (valid) {
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            uint4 v;
+            v.x = pack_bf16(o[x * 8 + 0] * inv, o[x * 8 + 1] * inv);
+            v.y = pack_bf16(o[x * 8 + 2] * inv, o[x * 8 + 3] * inv);
+            v.z = pack_bf16(o[x * 8 + 4] * inv, o[x * 8 + 5] * inv);
+            v.w = pack_bf16(o[x * 8 + 6] * inv, o[x * 8 + 7] * inv);
+            *reinterpret_cast<uint4*>(out_row + c + x * 8) = v;
+          }
+        }
+        __syncwarp();
+      }
+      if (half == 0 && valid) P.lse[row_global] = l > 0.f ? (m_ref + log2f(l)) * kLn2 : -INFINITY;
+      pair_sync();   // both have read the sums: the next tile's first block may write the same place
     }
-    if (tid == 0 && t + 1 < nb) load_v(t + 1);
-    // P through tensor memory, over the first 32 columns of S buffer sb (both threads of the row have read their S
-    // columns: the exchange of the maxima lies in between); S(t+2), which is issued after PV(t) by the same lane,
-    // overwrites them only after PV(t) has read them
-    tmem_st_bf16_row32(tm_lane + sb * 64 + half * 16, s);
-    tmem_st_wait();
-    tc_fence_before_sync();
-    __syncthreads();
-    if (warp == 0) {
-      mbar_wait_bounded(bar_v(t), (uint32_t)(t >> 1) & 1, &abort_flag);
+  } else if (warp < kSoftmaxWarps + kStreams) {
+    // ------------------------------------------------------------------ MMA issuer of a stream: the whole warp runs the
+    // loop, one elected lane issues
+    const int s = warp - kSoftmaxWarps;
+    constexpr uint32_t idS = instr_desc_bf16(128, 64, false, false);
+    constexpr uint32_t idO = instr_desc_bf16(128, D, false, true);
+    const uint32_t tStream = tm + s * 256;
+    const uint64_t dQ = smem_desc_sw128(sQ0 + s * kTileQ, 16);
+    // S is issued two key blocks ahead of PV, across tile boundaries: its own position in the work
+    int sn = s < streams ? (int)blockIdx.x : total, s_left = sn < total ? tile_at(sn).nb : 0;
+    bool s_first = true;
+    uint32_t su = 0, s_tiles = 0;
+    auto issue_s = [&]() {
+      const uint32_t buf = su % kBufs;
+      if (s_first) mbar_wait_bounded(smem_u32(&bars.q_full[s]), s_tiles & 1, &abort_flag);
+      mbar_wait_bounded(smem_u32(&bars.k_full[buf]), (su / kBufs) & 1, &abort_flag);
       __syncwarp();
       tc_fence_after_sync();
-      const uint32_t sV = sV0 + sb * kTileKV;
+      const uint64_t dK = smem_desc_sw128(sK0 + buf * kTileKV, 16);
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
-        mma_bf16_tmem_a_elect(tm + tO, tm + sb * 64 + k * 8, smem_desc_sw128(sV + k * 2048, 8192), idO, t > 0 || k > 0);
-      mma_commit_elect(bar_pv);
-      if (t + 2 < nb) issue_s(t + 2);
+      for (int k = 0; k < D / 16; ++k)
+        mma_bf16_elect(tStream + (su & 1) * 64, desc_advance(dQ, (k / 4) * 16384 + (k % 4) * 32),
+                       desc_advance(dK, (k / 4) * 8192 + (k % 4) * 32), idS, k > 0);
+      mma_commit_elect(smem_u32(&bars.s_full[s][su & 1]));
+      mma_commit_elect(smem_u32(&bars.k_free[buf]));
+      ++su;
+      s_first = --s_left == 0;
+      if (s_first) {
+        mma_commit_elect(smem_u32(&bars.q_free[s]));
+        sn += gridDim.x;
+        ++s_tiles;
+        s_left = sn < total ? tile_at(sn).nb : 0;
+      }
+    };
+    if (s_left > 0) issue_s();
+    if (s_left > 0) issue_s();
+    uint32_t u = 0;
+    for (int n = s < streams ? (int)blockIdx.x : total; n < total; n += gridDim.x) {
+      const int nb = tile_at(n).nb;
+      for (int t = 0; t < nb; ++t, ++u) {
+        const uint32_t buf = u % kBufs;
+        mbar_wait_bounded(smem_u32(&bars.v_full[buf]), (u / kBufs) & 1, &abort_flag);
+        mbar_wait_bounded(smem_u32(&bars.p_full[s][u & 1]), (u >> 1) & 1, &abort_flag);
+        __syncwarp();
+        tc_fence_after_sync();
+        const uint64_t dV = smem_desc_sw128(sV0 + buf * kTileKV, 8192);
+        const uint32_t tP = tStream + (u & 1) * 64;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) mma_bf16_tmem_a_elect(tStream + tO, tP + k * 8, desc_advance(dV, k * 2048), idO, t > 0 || k > 0);
+        mma_commit_elect(smem_u32(&bars.pv_done[s][u & 1]));
+        mma_commit_elect(smem_u32(&bars.v_free[buf]));
+        if (s_left > 0) issue_s();
+      }
+    }
+    // nothing of this CTA may still be running on the tensor cores when tensor memory is freed
+    mma_commit_elect(smem_u32(&bars.drain[s]));
+    mbar_wait_drain(smem_u32(&bars.drain[s]), 0);
+  } else {
+    // ------------------------------------------------------------------ TMA
+    if (lane == 0) {
+      uint32_t u = 0, tiles = 0;
+      for (int n = blockIdx.x; n < total; n += gridDim.x, ++tiles) {
+        const Tile tile = tile_at(n);
+        for (int t = 0; t < tile.nb; ++t, ++u) {
+          const uint32_t buf = u % kBufs, round = u / kBufs;
+          const int key = (tile.jb + t) * kBlock;
+          if (round >= 1) mbar_wait_bounded(smem_u32(&bars.k_free[buf]), (round - 1) & 1, &abort_flag);
+          mbar_arrive_expect_tx(smem_u32(&bars.k_full[buf]), kTileKV);
+#pragma unroll
+          for (int c = 0; c < NC; ++c) tma_load_4d(sK0 + buf * kTileKV + c * 8192, &tmK, smem_u32(&bars.k_full[buf]), c * 64, key, tile.h, tile.b);
+          if (t == 0) {
+            for (int s = 0; s < streams; ++s) {   // rows past the end of the sequence are zero
+              if (tiles >= 1) mbar_wait_bounded(smem_u32(&bars.q_free[s]), (tiles - 1) & 1, &abort_flag);
+              mbar_arrive_expect_tx(smem_u32(&bars.q_full[s]), kTileQ);
+#pragma unroll
+              for (int c = 0; c < NC; ++c)
+                tma_load_4d(sQ0 + s * kTileQ + c * 16384, &tmQ, smem_u32(&bars.q_full[s]), c * 64, tile.h * G, tile.i0 + s * QT, tile.b);
+            }
+          }
+          if (round >= 1) mbar_wait_bounded(smem_u32(&bars.v_free[buf]), (round - 1) & 1, &abort_flag);
+          mbar_arrive_expect_tx(smem_u32(&bars.v_full[buf]), kTileKV);
+#pragma unroll
+          for (int c = 0; c < NC; ++c) tma_load_4d(sV0 + buf * kTileKV + c * 8192, &tmV, smem_u32(&bars.v_full[buf]), c * 64, key, tile.h, tile.b);
+        }
+      }
+      // every request must have landed before the block may exit (also when it gave up)
+      for (uint32_t back = 1; back <= (uint32_t)kBufs && back <= u; ++back) {
+        const uint32_t w = u - back;
+        mbar_wait_drain(smem_u32(&bars.k_full[w % kBufs]), (w / kBufs) & 1);
+        mbar_wait_drain(smem_u32(&bars.v_full[w % kBufs]), (w / kBufs) & 1);
+      }
+      for (int s = 0; s < streams && tiles > 0; ++s) mbar_wait_drain(smem_u32(&bars.q_full[s]), (tiles - 1) & 1);
     }
   }
 
-  // output rows: O / l through the staging area, whole 128-byte lines per store instruction
-  __syncwarp();
-  if (nb > 0) {
-    mbar_wait_warp(bar_pv, (uint32_t)(nb - 1) & 1, &abort_flag);
-    tc_fence_after_sync();
-  }
-  __syncthreads();                       // nobody reads the maxima any more: the exchange area takes the sums
-  xchg[half * kRows + row] = l;
-  __syncthreads();
-  l += xchg[(half ^ 1) * kRows + row];
-  __syncthreads();                       // the sums are read: the staging area (which covers them) may be written
-  const float inv = l > 0.f ? 1.f / l : 0.f;
-  const int64_t row_global = ((int64_t)b * P.Hq + hq) * P.N + (valid ? i : 0);
-#pragma unroll
-  for (int c2 = 0; c2 < D / 64; ++c2) {
-    float tt[32];
-    tmem_ld32(tm_lane + tO + half * (D / 2) + c2 * 32, tt);
-    tmem_ld_wait();
-#pragma unroll
-    for (int x = 0; x < 4; ++x) {
-      uint4 v;
-      v.x = pack_bf16(tt[x * 8 + 0] * inv, tt[x * 8 + 1] * inv);
-      v.y = pack_bf16(tt[x * 8 + 2] * inv, tt[x * 8 + 3] * inv);
-      v.z = pack_bf16(tt[x * 8 + 4] * inv, tt[x * 8 + 5] * inv);
-      v.w = pack_bf16(tt[x * 8 + 6] * inv, tt[x * 8 + 7] * inv);
-      sts_v4(sStage + row * kStageStride + half * D + c2 * 64 + x * 16, v);
-    }
-  }
-  if (half == 0) row_dst[row] = valid && nb > 0 ? (int)row_global : -1;
-  __syncthreads();
-  if (half == 0) {
-    store_rows_coalesced<D * 2>(sStage, kStageStride, row_dst, reinterpret_cast<uint8_t*>(P.out), row);
-    if (valid) P.lse[row_global] = l > 0.f ? (m_ref + log2f(l)) * kLn2 : -INFINITY;
-  }
-
-  // nothing of this CTA may still be running on the tensor cores when tensor memory is freed
-  if (warp == 0) {
-    mma_commit_elect(smem_u32(&bars[7]));
-    mbar_wait_drain(smem_u32(&bars[7]), 0);
-  }
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tm, kCols);
+  if (warp == 0) tmem_dealloc(tm, 512);
   if (tid == 0 && abort_flag) atomicOr(P.status, 1);
 }
 
@@ -2023,6 +2087,22 @@ static int make_kv_map(CUtensorMap* map, const nsa_tensor& t, int B, int H, int 
   return NSA_OK;
 }
 
+// Tensor map over the queries of a [B, H, N, d] bf16 view; one box is [128 / G positions x G heads x 64 columns], whose
+// rows come in the order (position, head of the group).
+static int make_q_map(CUtensorMap* map, const nsa_tensor& t, int B, int H, int N, int d, int G) {
+  EncodeTiledFn enc = encode_fn();
+  if (enc == nullptr) return fail(NSA_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled is not available from this driver");
+  const int64_t sn = N > 1 ? t.stride_n : d, sh = H > 1 ? t.stride_h : sn * N, sb = B > 1 ? t.stride_b : (H > 1 ? sh * H : sn * N);
+  cuuint64_t dims[4] = {(cuuint64_t)d, (cuuint64_t)H, (cuuint64_t)N, (cuuint64_t)B};
+  cuuint64_t strides[3] = {(cuuint64_t)sh * 2, (cuuint64_t)sn * 2, (cuuint64_t)sb * 2};
+  cuuint32_t box[4] = {64, (cuuint32_t)G, (cuuint32_t)(kRows / G), 1}, es[4] = {1, 1, 1, 1};
+  const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, t.ptr, dims, strides, box, es,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return NSA_ERR_UNSUPPORTED;   // strides the tiled format cannot express
+  return NSA_OK;
+}
+
 #define CUDA_TRY(expr)                                                        \
   do {                                                                        \
     const cudaError_t e_ = (expr);                                            \
@@ -2141,25 +2221,23 @@ static int run_fwd(const SelProblem& a, const SelPlan& p, uint8_t* ws, cudaStrea
     const int QT = kRows / p.G;
     const int64_t tiles = (int64_t)a.B * a.Hkv * ((a.N + QT - 1) / QT);
     if (tiles > 0x7fffffffLL) return NSA_ERR_UNSUPPORTED;
-    const int smem = (D / 64) * 16384 + 16384 + 4 * (D / 64) * 8192;
-#define NSA_DENSE_LAUNCH(MODE, GI)                                                                                   \
+    CUtensorMap tmQ;
+    rc = make_q_map(&tmQ, a.q, a.B, a.Hq, a.N, D, p.G);
+    if (rc != NSA_OK) return rc;
+    // two streams per CTA (which share the K / V blocks) once there is a tile for every SM; below that a tile has its own SM
+    const int streams = tiles > num_sms() ? dense::kStreams : 1;
+    const int64_t work = (int64_t)a.B * a.Hkv * ((a.N + QT * streams - 1) / (QT * streams));
+    const unsigned grid = (unsigned)(work < num_sms() ? work : num_sms());
+#define NSA_DENSE_LAUNCH(MODE, GI, ...)                                                                                \
     do {                                                                                                              \
-      CUDA_TRY(cudaFuncSetAttribute(dense_fwd_kernel<D, MODE, GI>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); \
-      CUDA_TRY(cudaFuncSetAttribute(dense_fwd_kernel<D, MODE, GI>, cudaFuncAttributePreferredSharedMemoryCarveout,    \
-                                    cudaSharedmemCarveoutMaxShared));                                                 \
-      dense_fwd_kernel<D, MODE, GI><<<(unsigned)tiles, 2 * kRows, smem, st>>>(tmK, tmV, P);                               \
-    } while (0)
-#define NSA_DENSE_LAUNCH_POOL(GI)                                                                                     \
-    do {                                                                                                              \
-      CUDA_TRY(cudaFuncSetAttribute(dense_fwd_kernel<D, kModeCmp, GI, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); \
-      CUDA_TRY(cudaFuncSetAttribute(dense_fwd_kernel<D, kModeCmp, GI, true>, cudaFuncAttributePreferredSharedMemoryCarveout, \
-                                    cudaSharedmemCarveoutMaxShared));                                                 \
-      dense_fwd_kernel<D, kModeCmp, GI, true><<<(unsigned)tiles, 2 * kRows, smem, st>>>(tmK, tmV, P);                   \
+      const int smem = (int)dense::smem_bytes<D>(GI, P.pooled != nullptr);                                            \
+      CUDA_TRY(cudaFuncSetAttribute(dense_fwd_kernel<D, MODE, GI __VA_OPT__(,) __VA_ARGS__>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); \
+      dense_fwd_kernel<D, MODE, GI __VA_OPT__(,) __VA_ARGS__><<<grid, dense::kThreads, smem, st>>>(tmQ, tmK, tmV, P, streams); \
     } while (0)
     if (a.mode == kModeSwa) NSA_DENSE_LAUNCH(kModeSwa, 0);
-    else if (P.pooled != nullptr && p.G == 4) NSA_DENSE_LAUNCH_POOL(4);
-    else if (P.pooled != nullptr && p.G == 8) NSA_DENSE_LAUNCH_POOL(8);
-    else if (P.pooled != nullptr && p.G == 16) NSA_DENSE_LAUNCH_POOL(16);
+    else if (P.pooled != nullptr && p.G == 4) NSA_DENSE_LAUNCH(kModeCmp, 4, true);
+    else if (P.pooled != nullptr && p.G == 8) NSA_DENSE_LAUNCH(kModeCmp, 8, true);
+    else if (P.pooled != nullptr && p.G == 16) NSA_DENSE_LAUNCH(kModeCmp, 16, true);
     else if (P.pooled != nullptr) return NSA_ERR_UNSUPPORTED;
     else if (P.importance == nullptr) NSA_DENSE_LAUNCH(kModeCmp, 0);
     else if (p.G == 1) NSA_DENSE_LAUNCH(kModeCmp, 1);
@@ -2168,7 +2246,6 @@ static int run_fwd(const SelProblem& a, const SelPlan& p, uint8_t* ws, cudaStrea
     else if (p.G == 8) NSA_DENSE_LAUNCH(kModeCmp, 8);
     else NSA_DENSE_LAUNCH(kModeCmp, 16);
 #undef NSA_DENSE_LAUNCH
-#undef NSA_DENSE_LAUNCH_POOL
     CUDA_TRY(cudaGetLastError());
     count_launches(1);
     return NSA_OK;

@@ -6,7 +6,7 @@ import torch
 
 import recipe
 from oracle import nsa_oracle as O
-from util import SUM_REL, agreeing_queries, assert_bf16_no_worse_than_reference, assert_close_bf16, observe
+from util import SUM_REL, agreeing_queries, assert_bf16_no_worse_than_reference, assert_close_bf16, assert_close_f32, observe
 
 import native_sparse_attention_pytorch_b200 as nsa
 from native_sparse_attention_pytorch_b200 import ops
@@ -635,3 +635,25 @@ def test_index_at_the_edges_of_its_query_blocks_and_slot_words(case):
     slow = run_gpu(q, k, v, idx, mask, up, 'simt')
     for f, s, w in zip(fast, slow, ('out', 'lse', 'dq', 'dk', 'dv')):
         assert_close_bf16(f, s, w, roundings=2, rel_to_max=SUM_REL.get(w, 0.0))
+
+
+@pytest.mark.parametrize('case', [(1, 8, 1, 2368, 64), (1, 8, 1, 2369, 64), (3, 4, 4, 1669, 64), (2, 32, 2, 650, 128),
+                                  (1, 8, 4, 5000, 128), (1, 16, 4, 9, 64)])
+def test_dense_forward_at_the_edges_of_its_tiles_and_streams(case):
+    # one tile per SM (a stream per CTA) and one more (two streams, the last span half empty), several spans per CTA,
+    # every group size; against the generic kernels
+    b, hq, hkv, n, d = case
+    q, k, v = (recipe.randn((b, h, n, d), s).bfloat16().to(DEV) for h, s in ((hq, 1), (hkv, 2), (hkv, 3)))
+    for window in (70, 512):
+        out, lse = nsa.sliding_window_attend(q, k, v, window, True, impl='sm100', return_lse=True)
+        ref, ref_lse = nsa.sliding_window_attend(q, k, v, window, True, impl='simt', return_lse=True)
+        assert_close_bf16(out, ref, 'sliding', roundings=2)
+        assert_close_f32(lse, ref_lse, 'lse', tol=1e-3)
+    ck, cv = (recipe.randn((b, hkv, 1 + n // 8, d), s).bfloat16().to(DEV) for s in (4, 5))
+    out, imp = nsa.compressed_attend(q, ck, cv, 1, 8, True, impl='sm100')
+    ref, ref_imp = nsa.compressed_attend(q, ck, cv, 1, 8, True, impl='simt')
+    ops.check_device_status()
+    assert_close_bf16(out, ref, 'compressed', roundings=2)
+    seen = ref_imp > -1e30
+    assert torch.equal(seen, imp > -1e30)
+    assert_close_bf16(imp[seen], ref_imp[seen], 'importance', roundings=4)
