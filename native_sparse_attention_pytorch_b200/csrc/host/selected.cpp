@@ -94,6 +94,8 @@ static std::vector<OptTensor> sel_backward(Tensor q, Tensor k, Tensor v, OptTens
   a.dout = t4(dout);
   a.dk = ptr<float>(dkv);
   a.dv = a.dk + k.numel();
+  a.accumulate_kv = 1;
+  if (cudaMemsetAsync(a.dk, 0, 2 * k.numel() * sizeof(float), (cudaStream_t)stream_of(k)) != cudaSuccess) throw Error("clearing dk and dv failed");
   a.slot_grads = ptr<float>(slots);
   a.index = index.defined() ? index.data_ptr() : nullptr;
   a.index_bytes = index.defined() ? index.numel() : 0;

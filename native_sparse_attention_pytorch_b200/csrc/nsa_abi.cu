@@ -68,10 +68,9 @@ static int zero_async(float* p, int64_t count, cudaStream_t stream) {
   return err == cudaSuccess ? NSA_OK : fail((int)err, cudaGetErrorString(err));
 }
 
-// dk and dv start from zero unless the caller adds to what they hold; one call where they lie back to back
+// dk and dv start from zero unless the caller adds to what they hold
 static int zero_kv(float* dk, float* dv, int64_t count, bool accumulate, cudaStream_t stream) {
   if (accumulate) return NSA_OK;
-  if (dv == dk + count) return zero_async(dk, 2 * count, stream);
   NSA_TRY(zero_async(dk, count, stream));
   return zero_async(dv, count, stream);
 }

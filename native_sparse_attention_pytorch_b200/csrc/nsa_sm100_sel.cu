@@ -87,8 +87,9 @@ struct SelPlan {
   int64_t entries_cap, items_cap;
   // byte offsets into the work buffer
   int words;             // 32-bit words of slot bits per query
-  int64_t off_status, off_num_items, off_totals, off_list_base, off_cursors, off_bits, off_items, off_entries;
+  int64_t off_status, off_num_items, off_totals, off_list_base, off_list_item, off_cursors, off_bits, off_items, off_entries;
   int64_t off_partial, off_stats, off_delta;
+  int slices, pairs_per_slice;   // backward: launches over the (batch, KV head) pairs
   int64_t index_bytes;   // the leading part that holds the index (what the backward can take from the forward)
   int64_t total_bytes;
 };
@@ -102,6 +103,8 @@ struct SelParams {
   const uint32_t* entries;
   const int4* items;
   const int* num_items;    // [0] items, [1] the tag the item kernel left
+  const int* list_item;    // per list (and one more): its first item
+  int bh0, bh1;            // backward: the (batch, KV head) pairs of this launch, whose partial results share the buffer
   const uint32_t* bits;    // [B*Hkv*N][words]: the slots a query has (kModeSel)
   int words;
   __nv_bfloat16* dq_lp;    // optional bf16 dq with its own batch / head / row strides (dq merge)
@@ -219,7 +222,7 @@ __device__ __forceinline__ int2 block_scan2(int2 v, int2* total, int2 (*warp_sum
 // The line is kItemsTarget items (16 per SM): below it the K/V loads and the dK/dV flush of a short item still cost
 // less than the imbalance of long ones.
 constexpr int kItemsTarget = 148 * 16;
-__global__ void __launch_bounds__(1024) sel_items_kernel(const int* totals, int* list_base, int* cursors, int4* items,
+__global__ void __launch_bounds__(1024) sel_items_kernel(const int* totals, int* list_base, int* list_item, int* cursors, int4* items,
                                                          int* num_items, int nlists, int QT, uint32_t tag) {
   __shared__ int2 warp_sums[32];
   const int per = (nlists + 1023) / 1024;
@@ -236,11 +239,13 @@ __global__ void __launch_bounds__(1024) sel_items_kernel(const int* totals, int*
   for (int l = l0; l < l1; ++l) {
     const int nch = (totals[l] + QT - 1) / QT;
     list_base[l] = base;
+    list_item[l] = ibase;
     cursors[l] = base;
     for (int c0 = 0; c0 < nch; c0 += cpi) items[ibase++] = make_int4(l, c0, min(cpi, nch - c0), base + c0 * QT);
     base += nch * QT;
   }
   if (threadIdx.x == 0) {
+    list_item[nlists] = all.y;
     num_items[0] = all.y;
     num_items[1] = (int)tag;   // marks the index as built, and for which sizes
   }
@@ -314,68 +319,6 @@ __device__ __forceinline__ RowInfo decode_row(uint32_t e, int j, const BlockRule
   if (!r.valid) r.lim = -1;
   return r;
 }
-
-// All 128 threads copy the 128 rows of a chunk (D bf16 each) from global memory into swizzled [128 x 128 B]
-// tiles, one tile per 64 columns.  D/8 neighbouring threads share a row, so a warp reads whole 128-byte lines.
-// `base` points at batch element b; row r of the tile is query entries[r / G], head h*G + r % G.
-template <int D>
-__device__ __forceinline__ void gather_tile(uint32_t tile, const __nv_bfloat16* base, int64_t stride_h, int64_t stride_n,
-                                            const uint32_t* entries, int g_shift, int h, int tid) {
-  constexpr int CH = D / 8;         // 16-byte pieces per row
-  constexpr int RPP = kRows / CH;   // rows covered by one pass of the 128 threads
-  const int sub = tid % CH, r0 = tid / CH;
-  uint4 v[CH];
-#pragma unroll
-  for (int it = 0; it < CH; ++it) {
-    const int row = r0 + it * RPP;
-    const int ql = row >> g_shift, g = row - (ql << g_shift);
-    const uint32_t e = __ldg(entries + ql);
-    v[it] = make_uint4(0u, 0u, 0u, 0u);
-    if (e != kInvalidEntry)
-      v[it] = ldg_nc_v4(base + (int64_t)((h << g_shift) + g) * stride_h + (int64_t)(e & 0xffffffu) * stride_n + sub * 8);
-  }
-#pragma unroll
-  for (int it = 0; it < CH; ++it) {
-    const int row = r0 + it * RPP;
-    sts_v4(tile + (sub / 8) * (kRows * 128) + sw128_offset(row, sub % 8), v[it]);
-  }
-}
-
-// The same gather with 16-byte cp.async: returns at once, the rows land later (cp_async_wait).  Padding rows are
-// zero-filled.
-template <int D>
-__device__ __forceinline__ void gather_tile_async(uint32_t tile, const __nv_bfloat16* base, int64_t stride_h,
-                                                  int64_t stride_n, const uint32_t* entries, int g_shift, int h,
-                                                  int tid) {
-  constexpr int CH = D / 8;
-  constexpr int RPP = kRows / CH;
-  const int sub = tid % CH, r0 = tid / CH;
-  uint32_t ev[CH];
-#pragma unroll
-  for (int it = 0; it < CH; ++it) ev[it] = __ldg(entries + ((r0 + it * RPP) >> g_shift));
-#pragma unroll
-  for (int it = 0; it < CH; ++it) {
-    const int row = r0 + it * RPP;
-    const int g = row & ((1 << g_shift) - 1);
-    const bool valid = ev[it] != kInvalidEntry;
-    const int64_t i = valid ? (int64_t)(ev[it] & 0xffffffu) : 0;
-    cp_async16(tile + (sub / 8) * (kRows * 128) + sw128_offset(row, sub % 8),
-               base + (int64_t)((h << g_shift) + g) * stride_h + i * stride_n + sub * 8, valid ? 16u : 0u);
-  }
-}
-
-__device__ __forceinline__ void store_row_bf16(uint32_t tile, int row, const float (&x)[64]) {
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    uint4 v;
-    v.x = pack_bf16(x[c * 8 + 0], x[c * 8 + 1]);
-    v.y = pack_bf16(x[c * 8 + 2], x[c * 8 + 3]);
-    v.z = pack_bf16(x[c * 8 + 4], x[c * 8 + 5]);
-    v.w = pack_bf16(x[c * 8 + 6], x[c * 8 + 7]);
-    sts_v4(tile + sw128_offset(row, c), v);
-  }
-}
-
 
 // ---- forward -------------------------------------------------------------------------
 
@@ -1233,280 +1176,123 @@ __global__ void __launch_bounds__(256) sel_delta_kernel(const SelParams P, float
 }
 
 
-template <int D>
-__global__ void __launch_bounds__(kRows, D == 64 ? 2 : 1)
-sel_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const SelParams P) {
-  constexpr int NC = D / 64;
-  extern __shared__ uint8_t smem_raw[];
-  __shared__ int abort_flag;
-  __shared__ uint32_t tmem_slot;
-  __shared__ __align__(8) uint64_t bars[3];
-  const int nitems = item_count(P);
-  if ((int)blockIdx.x >= nitems) return;
-
-  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t sQ = base, sDO = sQ + NC * 16384, sK = sDO + NC * 16384, sV = sK + NC * 8192;
-  const uint32_t sP = sV + NC * 8192, sDS = sP + 16384;
-  // the P and dS tiles (plus a tail) double as the staging area of the dQ rows (one padded fp32 row per thread)
-  constexpr uint32_t kStageStride = D * 4 + 16;
-  const uint32_t sStage = sP;
-  const uint32_t bar_kv = smem_u32(&bars[0]), bar_1 = smem_u32(&bars[1]), bar_2 = smem_u32(&bars[2]);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  constexpr uint32_t kCols = D == 64 ? 256 : 512;
-  // tensor-memory columns: S and dP first; dQ overwrites them once they have been read
-  constexpr uint32_t tS = 0, tDP = 64, tDQ = 0, tDK = 128, tDV = 128 + D;
-
-  if (tid == 0) {
-    abort_flag = 0;
-    mbar_init(bar_kv, 1);
-    mbar_init(bar_1, 1);
-    mbar_init(bar_2, 1);
-    fence_mbar_init();
-    prefetch_tensormap(&tmK);
-    prefetch_tensormap(&tmV);
-  }
-  __syncthreads();
-  if (warp == 0) {
-    tmem_alloc(smem_u32(&tmem_slot), kCols);
-    tmem_relinquish();
-  }
-  tc_fence_before_sync();
-  __syncthreads();
-  tc_fence_after_sync();
-  const uint32_t tm = tmem_slot;
-  const uint32_t tm_lane = tm + ((uint32_t)(warp * 32) << 16);
-
-  const int G = P.G, QT = kRows / G, g_shift = 31 - __clz(G);
-  const int q_local = tid / G, g = tid - q_local * G;
-  uint32_t ph_kv = 0, ph_1 = 0, ph_2 = 0;
-  constexpr uint32_t idS = instr_desc_bf16(128, 64, false, false);    // S, dP : K-major A and B
-  constexpr uint32_t idDQ = instr_desc_bf16(128, D, false, true);     // dQ = dS K    : B MN-major
-  constexpr uint32_t idKV = instr_desc_bf16(64, D, true, true);       // dK, dV       : A and B MN-major
-
-  for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-    const int4 item = P.items[it];
-    const int list = item.x, j = list % P.nfb, bh = list / P.nfb, h = bh % P.Hkv, b = bh / P.Hkv;
-    if (tid == 0) {
-      mbar_arrive_expect_tx(bar_kv, 2 * NC * 8192);
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        tma_load_4d(sK + c * 8192, &tmK, bar_kv, c * 64, j * kBlock, h, b);
-        tma_load_4d(sV + c * 8192, &tmV, bar_kv, c * 64, j * kBlock, h, b);
-      }
-    }
-    for (int c = 0; c < item.z; ++c) {
-      const uint32_t* chunk_entries = P.entries + item.w + c * QT;
-      const uint32_t e = chunk_entries[q_local];
-      const RowInfo r = decode_row(e, j, P.rule);
-      const int64_t hq = (int64_t)h * G + g;
-      const int64_t row_global = ((int64_t)b * P.Hq + hq) * P.N + r.i;
-      gather_tile<D>(sQ, P.q + b * P.q_sb, P.q_sh, P.q_sn, chunk_entries, g_shift, h, tid);
-      gather_tile<D>(sDO, P.dout + b * P.do_sb, P.do_sh, P.do_sn, chunk_entries, g_shift, h, tid);
-      const float lse2 = r.valid ? P.lse[row_global] * kLog2e : 0.f;
-      const float delta = r.valid ? P.delta[row_global] : 0.f;
-      fence_proxy_async_smem();
-      bulk_wait_read();   // the previous chunk's dQ rows have left the staging area (= the P and dS tiles)
-      __syncthreads();
-      if (tid == 0) {
-        if (c == 0) mbar_wait_bounded(bar_kv, ph_kv, &abort_flag);
-        tc_fence_after_sync();
-        // (an MMA that accumulates into the previous one's tile waits for it, so independent chains are interleaved)
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t ch = k / 4, in = (k % 4) * 32;
-          mma_bf16(tm + tS, smem_desc_sw128(sQ + ch * 16384 + in, 16), smem_desc_sw128(sK + ch * 8192 + in, 16), idS,
-                   k > 0);
-          mma_bf16(tm + tDP, smem_desc_sw128(sDO + ch * 16384 + in, 16), smem_desc_sw128(sV + ch * 8192 + in, 16), idS,
-                   k > 0);
-        }
-        mma_commit(bar_1);
-      }
-      __syncwarp();
-      mbar_wait_bounded(bar_1, ph_1, &abort_flag);
-      ph_1 ^= 1;
-      tc_fence_after_sync();
-      __syncwarp();
-      float p[64], ds[64];
-      {
-        float t[32];
-        tmem_ld32(tm_lane + tS, t);
-        tmem_ld_wait();
-#pragma unroll
-        for (int x = 0; x < 32; ++x) p[x] = t[x];
-        tmem_ld32(tm_lane + tS + 32, t);
-        tmem_ld_wait();
-#pragma unroll
-        for (int x = 0; x < 32; ++x) p[32 + x] = t[x];
-        tmem_ld32(tm_lane + tDP, t);
-        tmem_ld_wait();
-#pragma unroll
-        for (int x = 0; x < 32; ++x) ds[x] = t[x];
-        tmem_ld32(tm_lane + tDP + 32, t);
-        tmem_ld_wait();
-#pragma unroll
-        for (int x = 0; x < 32; ++x) ds[32 + x] = t[x];
-      }
-      float slot_part = 0.f;
-#pragma unroll
-      for (int x = 0; x < 64; ++x) {
-        const float sx = p[x];
-        const float px = (x >= r.lo && x <= r.lim) ? ex2(sx * P.scale_log2 - lse2) : 0.f;
-        const float dsx = px * (ds[x] - delta);
-        slot_part = fmaf(dsx, sx * P.scale, slot_part);
-        p[x] = px;
-        ds[x] = dsx * P.scale;
-      }
-      store_row_bf16(sP, tid, p);
-      store_row_bf16(sDS, tid, ds);
-      if (P.slot_grads != nullptr) {
-        for (int o = G / 2; o > 0; o >>= 1) slot_part += __shfl_xor_sync(kFullMask, slot_part, o);
-        if (r.valid && g == 0 && r.slot < P.nsel)
-          P.slot_grads[(((int64_t)b * P.Hkv + h) * P.N + r.i) * P.nsel + r.slot] = slot_part;
-      }
-      fence_proxy_async_smem();
-      tc_fence_before_sync();
-      __syncthreads();
-      if (tid == 0) {
-        tc_fence_after_sync();
-        // dV += P^T dO, dK += dS^T Q over the 128 rows of the chunk (8 steps of 16 rows) and dQ_chunk = dS K over
-        // the 64 keys (4 steps of 16 keys), the three chains interleaved
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          mma_bf16(tm + tDV, smem_desc_sw128(sP + k * 2048, 16384), smem_desc_sw128(sDO + k * 2048, 16384), idKV,
-                   c > 0 || k > 0);
-          mma_bf16(tm + tDK, smem_desc_sw128(sDS + k * 2048, 16384), smem_desc_sw128(sQ + k * 2048, 16384), idKV,
-                   c > 0 || k > 0);
-          if (k < 4)
-            mma_bf16(tm + tDQ, smem_desc_sw128(sDS + k * 32, 16), smem_desc_sw128(sK + k * 2048, 8192), idDQ, k > 0);
-        }
-        mma_commit(bar_2);
-      }
-      __syncwarp();
-      mbar_wait_bounded(bar_2, ph_2, &abort_flag);
-      ph_2 ^= 1;
-      tc_fence_after_sync();
-      __syncwarp();
-#pragma unroll
-      for (int c2 = 0; c2 < D / 32; ++c2) {
-        float t[32];
-        tmem_ld32(tm_lane + tDQ + c2 * 32, t);
-        tmem_ld_wait();
-#pragma unroll
-        for (int x = 0; x < 8; ++x)
-          sts_v4f(sStage + tid * kStageStride + c2 * 128 + x * 16, t[x * 4], t[x * 4 + 1], t[x * 4 + 2], t[x * 4 + 3]);
-      }
-      // each thread adds its own dQ row into global memory with one bulk reduction
-      fence_proxy_async_smem();
-      if (r.valid) bulk_reduce_add_f32(P.dq + row_global * D, sStage + tid * kStageStride, D * 4);
-      bulk_commit();
-      tc_fence_before_sync();
-    }
-    // flush dK, dV of this item: accumulator rows 16w..16w+15 live in lanes 0..15 of warp w
-    {
-      const int key = j * kBlock + warp * 16 + lane;
-      const bool ok = lane < 16 && key < P.Nk;
-      float* dkp = P.dk + (((int64_t)b * P.Hkv + h) * P.Nk + key) * D;
-      float* dvp = P.dv + (((int64_t)b * P.Hkv + h) * P.Nk + key) * D;
-#pragma unroll
-      for (int c2 = 0; c2 < D / 32; ++c2) {
-        float t[32];
-        tmem_ld32(tm_lane + tDK + c2 * 32, t);
-        tmem_ld_wait();
-        if (ok) {
-#pragma unroll
-          for (int x = 0; x < 8; ++x) red_add_v4(dkp + c2 * 32 + x * 4, t[x * 4], t[x * 4 + 1], t[x * 4 + 2], t[x * 4 + 3]);
-        }
-        tmem_ld32(tm_lane + tDV + c2 * 32, t);
-        tmem_ld_wait();
-        if (ok) {
-#pragma unroll
-          for (int x = 0; x < 8; ++x) red_add_v4(dvp + c2 * 32 + x * 4, t[x * 4], t[x * 4 + 1], t[x * 4 + 2], t[x * 4 + 3]);
-        }
-      }
-      tc_fence_before_sync();
-    }
-    ph_kv ^= 1;
-    __syncthreads();
-  }
-
-  bulk_wait_read();
-  tc_fence_before_sync();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tm, kCols);
-  if (tid == 0 && abort_flag) atomicOr(P.status, 1);
-}
-
-
 // ---- backward, warp-specialised ---------------------------------------------------------------
 //
-// One CTA per SM, 13 warps with fixed roles, so that the gathers, the tensor-core work and the per-row
-// arithmetic of different chunks overlap instead of taking turns:
-//   warps 0-3, 4-7  two softmax groups; chunk n (counted per CTA) belongs to group n % 2.  A thread owns one row:
-//                   it reads S and dP from tensor memory, writes P and dS (bf16) for the second set of MMAs and
-//                   later stores its dQ row as a bf16 partial result (summed by sel_dq_merge_kernel).  Group t % 2
-//                   also flushes dK/dV of item t with fp32 reductions.
-//   warp 8          one thread issues every tcgen05.mma: S/dP of chunk n+1 before dQ/dV/dK of chunk n.
-//   warps 9-12      gather the Q and dO rows with 16-byte cp.async into a ring of kStages stages; a stage announces
-//                   itself (cp.async.mbarrier.arrive) when the copies have landed, the threads never wait for data.
-//   warp 13         one thread requests the K/V tiles of each item by TMA (double buffered).  It is a role of its
-//                   own because it waits for the consumer: a gathering thread that did so would hold back the
-//                   announcements the consumer is waiting for.
-// Tensor memory (512 columns): per softmax group S, dP and dQ (64 columns each), then dK and dV (64 each).  dQ has
-// columns of its own so that a group can go on to the S/dP of its next chunk and read dQ of the previous one out
-// afterwards, while the tensor cores are busy with the other group's chunk.
-// Every hand-over is an mbarrier; every wait is bounded.
+// One CTA per SM, 23 warps with fixed roles, so that the gathers, the tensor-core work and the per-row arithmetic of
+// different chunks overlap instead of taking turns:
+//   warps 0-7, 8-15  two softmax groups; chunk n (counted per CTA) belongs to group n % 2.  Two threads share a row (32
+//                    of the block's 64 columns each): they read S and dP from tensor memory, write P and dS (bf16) for
+//                    the second set of MMAs and then store the dQ row as a bf16 partial result (summed by
+//                    sel_dq_merge_kernel).  The group of an item's last chunk flushes its dK / dV with fp32 reductions.
+//   warp 16, 17      issue the tcgen05.mma: S / dP, which run a chunk ahead, and dV, dQ, dK.  Two of them, because an MMA
+//                    is accepted when the one before it starts: the waits and addresses in between leave the tensor
+//                    cores idle unless another warp issues meanwhile.
+//   warp 18          one thread requests the K / V tiles of each item by TMA.  It is a role of its own because it waits
+//                    for the consumer: a gathering thread that did so would hold back the announcements the consumer is
+//                    waiting for.
+//   warps 19-22      gather the Q and dO rows with 16-byte cp.async into a ring of stages; a stage announces itself
+//                    (cp.async.mbarrier.arrive) when the copies have landed, the threads never wait for data.
+// What bounds it: the chain of a group's chunk (wait for S, 2500 cycles of arithmetic, dV and dQ, 1500 of dQ read-out) with
+// two groups in flight; the gathers alone (32 KB per chunk at 18 bytes per clock and SM, the rate of scattered 128-byte
+// rows out of the L2) would take 1800 cycles per chunk, the MMAs 1100.  Batch 1, 3001 positions, 16 / 2 heads of 128: 253 us
+// -> 134 + 27 us for the dQ merge (before: a walk over chunks behind block-wide barriers, dq in fp32 reductions); batch 4,
+// 8192 positions, 32 / 4 heads of 64: 1.70 -> 1.75 ms; layer step with 2 x 16384, 16 / 4 heads of 64: 1.92 ms for its three
+// branches, as before.
+// Tensor memory (512 columns): S and dP of either group (64 columns each); dV and dK share D columns, dV in lanes 0-15 and
+// dK in lanes 16-31 of every quarter (a 64-row accumulator occupies half of the lanes); dQ: D columns, one buffer per
+// group at dim_head 64, one for both at 128.
+// Every hand-over is an mbarrier with one waiting role; every wait is bounded.
 namespace ws {
-constexpr int kStages = 3;
-constexpr uint32_t kMetaBytes = 3 * kRows * 4;   // per stage: entry, lse, delta of every row of the chunk
-constexpr uint32_t kPBytes = 32768;   // P and dS tiles
-constexpr uint32_t kDqRow = 64;       // staged half dQ row; its 16-byte pieces are swizzled with the row pair's index
-constexpr uint32_t kDqStage = 32 * kDqRow;   // per softmax warp
-constexpr int kThreads = 14 * 32;
-constexpr int kLoaderThreads = 128;
+constexpr int kSoftmaxWarps = 16, kThreads = 23 * 32;
+constexpr int kGroupThreads = 256, kLoaderThreads = 128;
+constexpr uint32_t kPBytes = 32768;         // P and dS tiles of a group
+
+template <int D>
+struct Shape {
+  static constexpr int NC = D / 64;
+  static constexpr int kStages = D == 64 ? 3 : 2;
+  static constexpr int kKv = D == 64 ? 2 : 1;              // K / V buffers
+  static constexpr int kDq = D == 64 ? 2 : 1;              // dQ buffers in tensor memory
+  static constexpr uint32_t kTileQ = NC * 16384, kStageBytes = 2 * kTileQ, kTileK = NC * 8192, kKvBytes = 2 * kTileK;
+  static constexpr uint32_t kMetaBytes = 2 * kRows * 4;    // per stage: lse, delta of every row of the chunk
+  static constexpr uint32_t kBytes = kStages * kStageBytes + 2 * kPBytes + kKv * kKvBytes + kStages * kMetaBytes;
+  static constexpr uint32_t tGroup = 128, tDP = 64, tAcc = 256, tDQ = tAcc + D;   // tensor-memory columns
+};
+constexpr uint32_t kLaneDK = 16u << 16;     // dK: lanes 16-31 of every quarter
+constexpr int kDqCols = 32;                 // dQ read-out: columns a warp stages at a time, in the P tile of its group
+constexpr uint32_t kDqRow = kDqCols * 2, kDqStage = 32 * kDqRow;
 
 struct Bars {
-  uint64_t q_full[kStages], q_free[kStages];
-  uint64_t s_full[2], p_full[2], mma2_done[2], dq_free[2];
+  uint64_t q_full[3], q_free[3];
+  uint64_t s_full[2], p_full[2], dq_done[2], tiles_free[2], dq_free;
   uint64_t kv_full[2], kv_free[2], acc_full[2], acc_free;
-  uint64_t drain;
+  uint64_t drain[2];
+};
+
+// The chunks of a CTA in order: chunk c of item `it` (the t-th of the CTA) is its n-th chunk.  The next item is requested
+// when the present one is entered.
+struct Cursor {
+  const int4* items;
+  int nitems, it, c, t, n;
+  int4 item, ahead;
+  __device__ __forceinline__ Cursor(const int4* items_, int nitems_, int first) : items(items_), nitems(nitems_), it(first), c(0), t(0), n(0) {
+    item = items[it];                      // a CTA without any item has returned
+    ahead = items[min(it + (int)gridDim.x, nitems - 1)];
+  }
+  __device__ __forceinline__ bool live() const { return it < nitems; }
+  __device__ __forceinline__ bool last() const { return c == item.z - 1; }
+  __device__ __forceinline__ bool next() {   // true: entered another item
+    ++n;
+    if (++c < item.z) return false;
+    c = 0;
+    ++t;
+    it += gridDim.x;
+    item = ahead;
+    ahead = items[min(it + (int)gridDim.x, nitems - 1)];
+    return true;
+  }
 };
 }  // namespace ws
 
+template <int D>
 __global__ void __launch_bounds__(ws::kThreads, 1)
 sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const SelParams P) {
   using namespace ws;
-  constexpr int D = 64;
-  extern __shared__ uint8_t smem_raw[];
+  using S = Shape<D>;
+  constexpr int NC = S::NC, kStages = S::kStages;
+  extern __shared__ __align__(1024) uint8_t ws_smem[];
   __shared__ int abort_flag;
   __shared__ uint32_t tmem_slot;
   __shared__ __align__(8) Bars bars;
-  const int nitems = item_count(P);
-  if ((int)blockIdx.x >= nitems) return;
+  if (item_count(P) == 0) return;
+  const int nitems = P.list_item[P.bh1 * P.nfb], first_item = P.list_item[P.bh0 * P.nfb] + (int)blockIdx.x;   // of the slice
+  if (first_item >= nitems) return;
 
-  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  // stage s: Q tile then dO tile (16 KB each); buffer b: P tile then dS tile; KV buffer: K tile then V tile (8 KB each)
-  const uint32_t sQ0 = base, sP0 = sQ0 + kStages * 32768, sKV0 = sP0 + 2 * kPBytes, sMeta0 = sKV0 + 2 * 16384,
-                 sDq0 = sMeta0 + kStages * kMetaBytes;
+  const uint32_t base = smem_u32(ws_smem);
+  // stage s: Q tiles then dO tiles; group g: P tile then dS tile; K / V buffer: K tiles then V tiles
+  const uint32_t sQ0 = base, sP0 = sQ0 + kStages * S::kStageBytes, sKV0 = sP0 + 2 * kPBytes, sMeta0 = sKV0 + S::kKv * S::kKvBytes;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (tid == 0) {
     abort_flag = 0;
-    for (int i = 0; i < kStages; ++i) {
+    if (base & 1023u) abort_flag = 1;   // the tiles would be mis-swizzled: report instead of computing
+    for (int i = 0; i < 3; ++i) {
       mbar_init(smem_u32(&bars.q_full[i]), kLoaderThreads);
       mbar_init(smem_u32(&bars.q_free[i]), 1);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&bars.s_full[i]), 1);
-      mbar_init(smem_u32(&bars.p_full[i]), kRows);
-      mbar_init(smem_u32(&bars.mma2_done[i]), 1);
-      mbar_init(smem_u32(&bars.dq_free[i]), kRows);
+      mbar_init(smem_u32(&bars.p_full[i]), kGroupThreads);
+      mbar_init(smem_u32(&bars.dq_done[i]), 1);
+      mbar_init(smem_u32(&bars.tiles_free[i]), 1);
       mbar_init(smem_u32(&bars.kv_full[i]), 1);
       mbar_init(smem_u32(&bars.kv_free[i]), 1);
+      mbar_init(smem_u32(&bars.acc_full[i]), 1);
     }
-    mbar_init(smem_u32(&bars.acc_full[0]), 1);
-    mbar_init(smem_u32(&bars.acc_full[1]), 1);
-    mbar_init(smem_u32(&bars.acc_free), kRows);
-    mbar_init(smem_u32(&bars.drain), 1);
+    mbar_init(smem_u32(&bars.dq_free), kGroupThreads);
+    mbar_init(smem_u32(&bars.acc_free), kGroupThreads);
+    mbar_init(smem_u32(&bars.drain[0]), 1);
+    mbar_init(smem_u32(&bars.drain[1]), 1);
     fence_mbar_init();
     prefetch_tensormap(&tmK);
     prefetch_tensormap(&tmV);
@@ -1522,344 +1308,308 @@ sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
   const uint32_t tm = tmem_slot;
   const int G = P.G, QT = kRows / G, g_shift = 31 - __clz(G);
 
-  if (warp < 8) {
+  if (warp < kSoftmaxWarps) {
     // ------------------------------------------------------------------ softmax groups
-    const int wg = warp >> 2, r_tid = tid & 127;
-    const uint32_t tm_lane = tm + ((uint32_t)((warp & 3) * 32) << 16);
-    const int q_local = r_tid >> g_shift, g = r_tid - (q_local << g_shift);
-    const uint32_t tS = wg * 192, tDP = tS + 64, tDQ = tS + 128;
+    const int wg = warp >> 3, half = (warp >> 2) & 1, row = (warp & 3) * 32 + lane;
+    const uint32_t tm_quarter = tm + ((uint32_t)((warp & 3) * 32) << 16);   // warps w and w + 4 share a lane quarter
+    const uint32_t tS = tm_quarter + wg * S::tGroup;
+    const int q_local = row >> g_shift, g = row - (q_local << g_shift);
     const uint32_t sP = sP0 + wg * kPBytes, sDS = sP + 16384;
-    // dQ row of the group's previous chunk, still to be read out of tensor memory: index of its (row, slot) partial
-    int prev_dst = -1;
-    bool have_prev = false;
-    uint32_t prev_use = 0;
-    const uint32_t sDq = sDq0 + warp * kDqStage;
-    // The dQ rows go out as the bf16 partial results of their (row, slot); sel_dq_merge_kernel sums them (plain stores
-    // run at memory speed, fp32 reductions into dq are limited by the L2 atomic units).  A thread that stored its own
-    // 128-byte row would make every store instruction touch 32 lines; the warp stages half rows in shared memory
-    // instead and stores them eight rows per instruction.
-    auto dq_out = [&]() {
-      mbar_wait_warp(smem_u32(&bars.mma2_done[wg]), prev_use & 1, &abort_flag);
+    const uint32_t sDq = sP + (warp & 3) * 4096 + half * kDqStage;   // in the warp's own rows of the P tile
+    // dQ of the chunk just handed over: the thread's half of the columns of its row, to the (row, slot) partial `dst_row`
+    // (plain stores run at memory speed, fp32 reductions into dq are limited by the L2 atomic units).  A thread that
+    // stored its own piece would make every store instruction touch 32 lines; the warp stages 32 columns at a time in
+    // the group's P tile, which the completed dV product no longer reads, and stores eight rows per instruction.
+    auto dq_out = [&](const int dst_row, const uint32_t use) {
+      mbar_wait_warp(smem_u32(&bars.dq_done[wg]), use & 1, &abort_flag);
       tc_fence_after_sync();
       __syncwarp();
       uint8_t* const pbase = reinterpret_cast<uint8_t*>(P.partial);
 #pragma unroll 1
-      for (int half = 0; half < 2; ++half) {
-        float tq[32];
-        tmem_ld32(tm_lane + tDQ + half * 32, tq);
-        tmem_ld_wait();
+      for (int piece = 0; piece < NC; ++piece) {
+        const int col = (half * NC + piece) * kDqCols;
+        {
+          float tq[kDqCols];
+          tmem_ld32(tm_quarter + S::tDQ + (S::kDq == 2 ? wg * D : 0) + col, tq);
+          tmem_ld_wait();
 #pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          uint4 v;
-          v.x = pack_bf16(tq[x * 8 + 0], tq[x * 8 + 1]); v.y = pack_bf16(tq[x * 8 + 2], tq[x * 8 + 3]);
-          v.z = pack_bf16(tq[x * 8 + 4], tq[x * 8 + 5]); v.w = pack_bf16(tq[x * 8 + 6], tq[x * 8 + 7]);
-          sts_v4(sDq + lane * kDqRow + ((x ^ ((lane >> 1) & 3)) << 4), v);   // conflict-free to write and to read
+          for (int x = 0; x < 4; ++x) {
+            uint4 v;
+            v.x = pack_bf16(tq[x * 8 + 0], tq[x * 8 + 1]); v.y = pack_bf16(tq[x * 8 + 2], tq[x * 8 + 3]);
+            v.z = pack_bf16(tq[x * 8 + 4], tq[x * 8 + 5]); v.w = pack_bf16(tq[x * 8 + 6], tq[x * 8 + 7]);
+            sts_v4(sDq + lane * kDqRow + ((x ^ ((lane >> 1) & 3)) << 4), v);   // conflict-free to write and to read
+          }
+        }
+        if (S::kDq == 1 && piece == NC - 1) {
+          tc_fence_before_sync();
+          mbar_arrive(smem_u32(&bars.dq_free));   // the other group's dQ may overwrite the columns
         }
         __syncwarp();
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const int rr = k * 8 + (lane >> 2);
-          const int dst = __shfl_sync(kFullMask, prev_dst, rr);
+          const int dst = __shfl_sync(kFullMask, dst_row, rr);
           const uint4 v = lds_v4(sDq + rr * kDqRow + (((lane & 3) ^ ((rr >> 1) & 3)) << 4));
-          if (dst >= 0)
-            *reinterpret_cast<uint4*>(pbase + (int64_t)dst * (D * 2) + half * 64 + (lane & 3) * 16) = v;
+          if (dst >= 0) *reinterpret_cast<uint4*>(pbase + (int64_t)dst * (D * 2) + col * 2 + (lane & 3) * 16) = v;
         }
         __syncwarp();
       }
-      tc_fence_before_sync();
-      mbar_arrive(smem_u32(&bars.dq_free[wg]));   // the dQ columns of this group may be overwritten
-      have_prev = false;
+      // the two warps that share these rows have read what they staged before either writes P again
+      asm volatile("bar.sync %0, 64;" ::"r"(1 + wg * 4 + (warp & 3)) : "memory");
     };
-    // one chunk of this group; the thread's entry and its row's statistics come from the stage's metadata, which
-    // the loaders fetched together with the rows
-    auto process_chunk = [&](const int4 item, const int n) {
-      {
-        const int list = item.x, j = list % P.nfb, bh = list / P.nfb, h = bh % P.Hkv, b = bh / P.Hkv;
-        const uint32_t use = (uint32_t)(n >> 1);   // how many chunks this group has had before
-        const uint32_t sMeta = sMeta0 + (n % kStages) * kMetaBytes + r_tid * 4;
-        mbar_wait_warp(smem_u32(&bars.s_full[wg]), use & 1, &abort_flag);
-        tc_fence_after_sync();
-        const uint32_t e = lds_u32(sMeta);
-        const float lse2 = __uint_as_float(lds_u32(sMeta + kRows * 4)) * kLog2e;
-        const float delta = __uint_as_float(lds_u32(sMeta + 2 * kRows * 4));
-        const RowInfo r = decode_row(e, j, P.rule);
-        const int64_t hq = (int64_t)h * G + g;
-        const int64_t row_global = ((int64_t)b * P.Hq + hq) * P.N + r.i;
-        float slot_part = 0.f;
-        const bool want_slot = P.slot_grads != nullptr;
-        // rows that see the whole block need no per-column test; only own-block (causal) and padding rows do
-        const bool all_full = __all_sync(kFullMask, r.lim == kBlock - 1 && r.lo == 0);
-        // 16 columns at a time in a rolled loop: the body stays small enough for the instruction cache, which four
-        // roles share
-        auto math16 = [&](float (&sv)[16], float (&dv)[16], const int q4) {
-          const int rem = r.lim - q4 * 16, rlo = r.lo - q4 * 16;   // columns rlo..rem of this group are visible
-          if (all_full) {
-#pragma unroll
-            for (int x = 0; x < 16; ++x) {
-              const float sx = sv[x];
-              const float px = ex2(sx * P.scale_log2 - lse2);
-              const float dsx = px * (dv[x] - delta);
-              if (want_slot) slot_part = fmaf(dsx, sx, slot_part);
-              sv[x] = px;
-              dv[x] = dsx;
-            }
-          } else {
-#pragma unroll
-            for (int x = 0; x < 16; ++x) {
-              const float sx = sv[x];
-              const float px = (x >= rlo && x <= rem) ? ex2(sx * P.scale_log2 - lse2) : 0.f;
-              const float dsx = px * (dv[x] - delta);
-              if (want_slot) slot_part = fmaf(dsx, sx, slot_part);
-              sv[x] = px;
-              dv[x] = dsx;
-            }
-          }
-#pragma unroll
-          for (int x = 0; x < 2; ++x) {
-            uint4 pv, dsv;
-            pv.x = pack_bf16(sv[x * 8 + 0], sv[x * 8 + 1]); pv.y = pack_bf16(sv[x * 8 + 2], sv[x * 8 + 3]);
-            pv.z = pack_bf16(sv[x * 8 + 4], sv[x * 8 + 5]); pv.w = pack_bf16(sv[x * 8 + 6], sv[x * 8 + 7]);
-            dsv.x = pack_bf16(dv[x * 8 + 0], dv[x * 8 + 1]); dsv.y = pack_bf16(dv[x * 8 + 2], dv[x * 8 + 3]);
-            dsv.z = pack_bf16(dv[x * 8 + 4], dv[x * 8 + 5]); dsv.w = pack_bf16(dv[x * 8 + 6], dv[x * 8 + 7]);
-            sts_v4(sP + sw128_offset(r_tid, q4 * 2 + x), pv);
-            sts_v4(sDS + sw128_offset(r_tid, q4 * 2 + x), dsv);
-          }
-        };
-        {
-          float sa[16], da[16], sb[16], db[16];
-          tmem_ld16(tm_lane + tS, sa);
-          tmem_ld16(tm_lane + tDP, da);
-          tmem_ld_wait();
+    uint32_t use = 0, flushes = 0;
+    int j = 0, h = 0, b = 0;
+    Cursor cur(P.items, nitems, first_item);
+    auto enter_item = [&]() {
+      const int list = cur.item.x, bh = list / P.nfb;
+      j = list - bh * P.nfb;
+      b = bh / P.Hkv;
+      h = bh - b * P.Hkv;
+    };
+    auto entry_of = [&]() { return cur.live() ? __ldg(P.entries + cur.item.w + cur.c * QT + q_local) : kInvalidEntry; };
+    if (wg == 1) cur.next();
+    enter_item();
+    uint32_t e_next = entry_of();
+    while (cur.live()) {
+      const uint32_t e = e_next;
+      const RowInfo r = decode_row(e, j, P.rule);
+      const int n = cur.n;
+      const uint32_t sMeta = sMeta0 + (n % kStages) * S::kMetaBytes + row * 4;
+      mbar_wait_warp(smem_u32(&bars.s_full[wg]), use & 1, &abort_flag);
+      tc_fence_after_sync();
+      const float lse2 = __uint_as_float(lds_u32(sMeta)) * kLog2e;
+      const float delta = __uint_as_float(lds_u32(sMeta + kRows * 4));
+      float slot_part = 0.f;
+      const bool want_slot = P.slot_grads != nullptr;
+      // rows that see the whole block need no per-column test; only own-block (causal) and padding rows do
+      const bool all_full = __all_sync(kFullMask, r.lim == kBlock - 1 && r.lo == 0);
 #pragma unroll 1
-          for (int q2 = 0; q2 < 2; ++q2) {
-            tmem_ld16(tm_lane + tS + q2 * 32 + 16, sb);
-            tmem_ld16(tm_lane + tDP + q2 * 32 + 16, db);
-            math16(sa, da, q2 * 2);
-            tmem_ld_wait();
-            if (q2 == 0) {
-              tmem_ld16(tm_lane + tS + 32, sa);
-              tmem_ld16(tm_lane + tDP + 32, da);
-            }
-            math16(sb, db, q2 * 2 + 1);
-            tmem_ld_wait();
+      for (int q = 0; q < 2; ++q) {         // 16 columns at a time: the body stays small enough for the instruction cache
+        const int col = half * 32 + q * 16;
+        float sv[16], dv[16];
+        tmem_ld16(tS + col, sv);
+        tmem_ld16(tS + S::tDP + col, dv);
+        tmem_ld_wait();
+        if (all_full) {
+#pragma unroll
+          for (int x = 0; x < 16; ++x) {
+            const float px = ex2(fmaf(sv[x], P.scale_log2, -lse2));
+            const float dsx = px * (dv[x] - delta);
+            if (want_slot) slot_part = fmaf(dsx, sv[x], slot_part);
+            sv[x] = px;
+            dv[x] = dsx;
+          }
+        } else {
+          const int rem = r.lim - col, rlo = r.lo - col;   // columns rlo..rem of this group are visible
+#pragma unroll
+          for (int x = 0; x < 16; ++x) {
+            const float px = (x >= rlo && x <= rem) ? ex2(fmaf(sv[x], P.scale_log2, -lse2)) : 0.f;
+            const float dsx = px * (dv[x] - delta);
+            if (want_slot) slot_part = fmaf(dsx, sv[x], slot_part);
+            sv[x] = px;
+            dv[x] = dsx;
           }
         }
-        fence_proxy_async_smem();
-        tc_fence_before_sync();
-        mbar_arrive(smem_u32(&bars.p_full[wg]));
-        if (P.slot_grads != nullptr) {
-          for (int o = G / 2; o > 0; o >>= 1) slot_part += __shfl_xor_sync(kFullMask, slot_part, o);
-          if (r.valid && g == 0 && r.slot < P.nsel)
-            P.slot_grads[(((int64_t)b * P.Hkv + h) * P.N + r.i) * P.nsel + r.slot] = slot_part * P.scale;
+        // dK of the group's previous chunk, the last product to read the tiles, is complete
+        if (q == 0 && use > 0) mbar_wait_warp(smem_u32(&bars.tiles_free[wg]), (use - 1) & 1, &abort_flag);
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          uint4 pv, dsv;
+          pv.x = pack_bf16(sv[x * 8 + 0], sv[x * 8 + 1]); pv.y = pack_bf16(sv[x * 8 + 2], sv[x * 8 + 3]);
+          pv.z = pack_bf16(sv[x * 8 + 4], sv[x * 8 + 5]); pv.w = pack_bf16(sv[x * 8 + 6], sv[x * 8 + 7]);
+          dsv.x = pack_bf16(dv[x * 8 + 0], dv[x * 8 + 1]); dsv.y = pack_bf16(dv[x * 8 + 2], dv[x * 8 + 3]);
+          dsv.z = pack_bf16(dv[x * 8 + 4], dv[x * 8 + 5]); dsv.w = pack_bf16(dv[x * 8 + 6], dv[x * 8 + 7]);
+          sts_v4(sP + sw128_offset(row, col / 8 + x), pv);
+          sts_v4(sDS + sw128_offset(row, col / 8 + x), dsv);
         }
-        // while the tensor cores work on this chunk's P and dS, read out dQ of the previous chunk of the group
-        if (have_prev) dq_out();
-        prev_dst = r.valid ? (int)(row_global * P.ns + r.slot) : -1;
-        prev_use = use;
-        have_prev = true;
       }
-    };
-    uint32_t flushes = 0;   // items this group has flushed
-    auto flush_item = [&](const int4 item, const int t) {
-      const int list = item.x, j = list % P.nfb, bh = list / P.nfb, h = bh % P.Hkv, b = bh / P.Hkv;
-      {
-        // flush dK/dV of this item: accumulator rows 16w..16w+15 live in lanes 0..15 of warp w of the group.
-        // "Accumulator complete" has one barrier per flushing group, counted by that group: with one barrier for both,
-        // a group that reached its wait before the other group's item was complete saw the phase before that one
-        // (same parity) as its own and flushed early.
+      fence_proxy_async_smem();
+      tc_fence_before_sync();
+      mbar_arrive(smem_u32(&bars.p_full[wg]));
+      const int64_t slice_row = ((int64_t)(b * P.Hkv + h - P.bh0) * G + g) * P.N + r.i;
+      const int dst = r.valid ? (int)(slice_row * P.ns + r.slot) : -1;
+      if (want_slot) {   // two threads of a row, in different warps: two additions to a cleared slot
+        for (int o = G / 2; o > 0; o >>= 1) slot_part += __shfl_xor_sync(kFullMask, slot_part, o);
+        if (r.valid && g == 0 && r.slot < P.nsel)
+          atomicAdd(P.slot_grads + (((int64_t)b * P.Hkv + h) * P.N + r.i) * P.nsel + r.slot, slot_part * P.scale);
+      }
+      // on to the group's next chunk: its entry travels under the read-out of dQ
+      const bool flush = cur.last();
+      const int key = j * kBlock + (warp & 3) * 16 + (lane & 15);
+      const int64_t key_row = ((int64_t)b * P.Hkv + h) * P.Nk + key;
+      bool entered = cur.next();
+      if (cur.live()) entered = cur.next() || entered;
+      if (entered && cur.live()) enter_item();
+      e_next = entry_of();
+      dq_out(dst, use);
+      ++use;
+      if (flush) {
+        // flush dK/dV of this item: keys 16w..16w+15 live in the lanes of quarter w, either half of the group takes half of
+        // the columns.  "Accumulator complete" has one barrier per flushing group, counted by
+        // that group: with one barrier for both, a group that reached its wait before the other group's item was complete
+        // saw the phase before that one (same parity) as its own and flushed early.
         mbar_wait_warp(smem_u32(&bars.acc_full[wg]), flushes & 1, &abort_flag);
         ++flushes;
         tc_fence_after_sync();
         __syncwarp();
-        const int key = j * kBlock + (warp & 3) * 16 + lane;
-        const bool ok = lane < 16 && key < P.Nk;
-        float* dkp = P.dk + (((int64_t)b * P.Hkv + h) * P.Nk + key) * D;
-        float* dvp = P.dv + (((int64_t)b * P.Hkv + h) * P.Nk + key) * D;
-        const uint32_t tDK = 384, tDV = 448;
-#pragma unroll
-        for (int c2 = 0; c2 < D / 32; ++c2) {
+        const float f = lane < 16 ? 1.f : P.scale;
+        float* const dstp = (lane < 16 ? P.dv : P.dk) + key_row * D + half * (D / 2);
+#pragma unroll 1
+        for (int c = 0; c < D / 2; c += 32) {
           float tk[32];
-          tmem_ld32(tm_lane + tDK + c2 * 32, tk);
+          tmem_ld32(tm_quarter + S::tAcc + half * (D / 2) + c, tk);
           tmem_ld_wait();
-          if (ok) {
+          if (key < P.Nk) {
 #pragma unroll
-            for (int x = 0; x < 8; ++x)
-              red_add_v4(dkp + c2 * 32 + x * 4, tk[x * 4] * P.scale, tk[x * 4 + 1] * P.scale, tk[x * 4 + 2] * P.scale, tk[x * 4 + 3] * P.scale);
-          }
-          tmem_ld32(tm_lane + tDV + c2 * 32, tk);
-          tmem_ld_wait();
-          if (ok) {
-#pragma unroll
-            for (int x = 0; x < 8; ++x) red_add_v4(dvp + c2 * 32 + x * 4, tk[x * 4], tk[x * 4 + 1], tk[x * 4 + 2], tk[x * 4 + 3]);
+            for (int x = 0; x < 8; ++x) red_add_v4(dstp + c + x * 4, tk[x * 4] * f, tk[x * 4 + 1] * f, tk[x * 4 + 2] * f, tk[x * 4 + 3] * f);
           }
         }
         tc_fence_before_sync();
         mbar_arrive(smem_u32(&bars.acc_free));
       }
-    };
-    // dK/dV of an item are flushed by the group that had the item's last chunk, as soon as the tensor cores are done
-    // with it: the next item's dV/dK MMAs wait for the accumulator
-    int n = 0, t = 0;
-    for (int it = blockIdx.x; it < nitems; it += gridDim.x, ++t) {
-      const int4 item = P.items[it];
-      for (int c = 0; c < item.z; ++c, ++n) {
-        if ((n & 1) != wg) continue;
-        process_chunk(item, n);
-        if (c == item.z - 1) flush_item(item, t);
-      }
     }
-    if (have_prev) dq_out();
-  } else if (warp == 8) {
-    // ------------------------------------------------------------------ MMA issuer: the whole warp runs the loop
-    // (so that its state lives in uniform registers), one elected lane issues
-    {
+  } else if (warp == kSoftmaxWarps) {
+    // ------------------------------------------------------------------ issuer of S and dP.  The whole warp runs the
+    // loop (so that its state lives in uniform registers), one elected lane issues.  The lbo field of a descriptor serves
+    // the tiles read MN-major (the distance to the next 64 columns); the others ignore it.  One descriptor per tile: every
+    // MMA then costs one 64-bit add to issue.
     constexpr uint32_t idS = instr_desc_bf16(128, 64, false, false);
-    constexpr uint32_t idDQ = instr_desc_bf16(128, D, false, true);
-    constexpr uint32_t idKV = instr_desc_bf16(64, D, true, true);
-    int n = 0, t = 0;
-    // state of the chunk whose second set of MMAs is still to be issued
-    bool pending = false;
-    int p_n = 0, p_t = 0, p_c = 0;
-    bool p_last = false;
-    auto issue_mma2 = [&](int pn, int pt, int pc, bool last) {
-      const int grp = pn & 1, stage = pn % kStages, kb = pt & 1;
-      const uint32_t sQ = sQ0 + stage * 32768, sDO = sQ + 16384;
-      const uint32_t sP = sP0 + grp * kPBytes, sDS = sP + 16384;
-      const uint32_t sK = sKV0 + kb * 16384;
-      mbar_wait_bounded(smem_u32(&bars.p_full[grp]), (uint32_t)(pn >> 1) & 1, &abort_flag);
-      // the accumulators are single: the first chunk of an item waits until the previous item has been flushed
-      if (pc == 0 && pt >= 1) mbar_wait_bounded(smem_u32(&bars.acc_free), (uint32_t)(pt - 1) & 1, &abort_flag);
+    int stage = 0, round = 0;
+    for (Cursor cur(P.items, nitems, first_item); cur.live(); cur.next()) {
+      const int grp = cur.n & 1, kb = S::kKv == 2 ? cur.t & 1 : 0;
+      const uint32_t sQ = sQ0 + stage * S::kStageBytes, sK = sKV0 + kb * S::kKvBytes, tS = tm + grp * S::tGroup;
+      const uint64_t dQt = smem_desc_sw128(sQ, 16384), dDOt = smem_desc_sw128(sQ + S::kTileQ, 16384);
+      const uint64_t dKt = smem_desc_sw128(sK, 8192), dVt = smem_desc_sw128(sK + S::kTileK, 8192);
+      // the group has read the S and dP before these
+      if (cur.n >= 2) mbar_wait_bounded(smem_u32(&bars.p_full[grp]), (uint32_t)((cur.n >> 1) - 1) & 1, &abort_flag);
+      mbar_wait_bounded(smem_u32(&bars.q_full[stage]), round & 1, &abort_flag);
+      if (cur.c == 0) mbar_wait_bounded(smem_u32(&bars.kv_full[kb]), (uint32_t)(S::kKv == 2 ? cur.t >> 1 : cur.t) & 1, &abort_flag);
       __syncwarp();
       tc_fence_after_sync();
-      const uint32_t tDK = 384, tDV = 448, tDQ = grp * 192 + 128;
-      // One descriptor per tile (the leading-offset field is unused for 64-wide tiles, so the same descriptor
-      // serves the K-major and the MN-major reading of a tile); every MMA then costs one 64-bit add to issue.
-      const uint64_t dQt = smem_desc_sw128(sQ, 16), dDOt = smem_desc_sw128(sDO, 16), dPt = smem_desc_sw128(sP, 16),
-                     dDSt = smem_desc_sw128(sDS, 16), dKt = smem_desc_sw128(sK, 16);
-      // dV and dK first: the group reads dQ of its previous chunk out right after it has handed P and dS over, and
-      // is done with it by the time these sixteen MMAs have been issued.
+#pragma unroll
+      for (int k = 0; k < D / 16; ++k) {
+        const uint32_t a = (k / 4) * 16384 + (k % 4) * 32, bb = (k / 4) * 8192 + (k % 4) * 32;
+        mma_bf16_elect(tS, desc_advance(dQt, a), desc_advance(dKt, bb), idS, k > 0);
+        mma_bf16_elect(tS + S::tDP, desc_advance(dDOt, a), desc_advance(dVt, bb), idS, k > 0);
+      }
+      mma_commit_elect(smem_u32(&bars.s_full[grp]));
+      if (++stage == kStages) { stage = 0; ++round; }
+    }
+    mma_commit_elect(smem_u32(&bars.drain[0]));
+    mbar_wait_drain(smem_u32(&bars.drain[0]), 0);
+  } else if (warp == kSoftmaxWarps + 1) {
+    // ------------------------------------------------------------------ issuer of dV, dQ and dK
+    constexpr uint32_t idDQ = instr_desc_bf16(128, D, false, true);
+    constexpr uint32_t idKV = instr_desc_bf16(64, D, true, true);
+    int stage = 0;
+    for (Cursor cur(P.items, nitems, first_item); cur.live(); cur.next()) {
+      const int grp = cur.n & 1, kb = S::kKv == 2 ? cur.t & 1 : 0;
+      const uint32_t sQ = sQ0 + stage * S::kStageBytes, sP = sP0 + grp * kPBytes;
+      const uint64_t dQt = smem_desc_sw128(sQ, 16384), dDOt = smem_desc_sw128(sQ + S::kTileQ, 16384);
+      const uint64_t dPt = smem_desc_sw128(sP, 16384), dDSt = smem_desc_sw128(sP + 16384, 16384);
+      const uint64_t dKt = smem_desc_sw128(sKV0 + kb * S::kKvBytes, 8192);
+      mbar_wait_bounded(smem_u32(&bars.p_full[grp]), (uint32_t)(cur.n >> 1) & 1, &abort_flag);
+      // the accumulators are single: the first chunk of an item waits until the previous item has been flushed
+      if (cur.c == 0 && cur.t >= 1) mbar_wait_bounded(smem_u32(&bars.acc_free), (uint32_t)(cur.t - 1) & 1, &abort_flag);
+      __syncwarp();
+      tc_fence_after_sync();
+      // dV += P^T dO over the 128 rows of the chunk, then dQ = dS K: the group waits for both (it stages its dQ rows in
+      // the P tile).  dQ's columns: the group (or, with one buffer, the other one) has read the dQ before it out.
 #pragma unroll
       for (int k = 0; k < 8; ++k)
-        mma_bf16_elect(tm + tDV, desc_advance(dPt, k * 2048), desc_advance(dDOt, k * 2048), idKV, pc > 0 || k > 0);
-#pragma unroll
-      for (int k = 0; k < 8; ++k)
-        mma_bf16_elect(tm + tDK, desc_advance(dDSt, k * 2048), desc_advance(dQt, k * 2048), idKV, pc > 0 || k > 0);
-      if (pn >= 2) {
-        mbar_wait_bounded(smem_u32(&bars.dq_free[grp]), (uint32_t)((pn >> 1) - 1) & 1, &abort_flag);
+        mma_bf16_elect(tm + S::tAcc, desc_advance(dPt, k * 2048), desc_advance(dDOt, k * 2048), idKV, cur.c > 0 || k > 0);
+      if (S::kDq == 1 && cur.n >= 1) {
+        mbar_wait_bounded(smem_u32(&bars.dq_free), (uint32_t)(cur.n - 1) & 1, &abort_flag);
         __syncwarp();
         tc_fence_after_sync();
       }
+      const uint32_t tDQ = tm + S::tDQ + (S::kDq == 2 ? grp * D : 0);
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
-        mma_bf16_elect(tm + tDQ, desc_advance(dDSt, k * 32), desc_advance(dKt, k * 2048), idDQ, k > 0);
-      mma_commit_elect(smem_u32(&bars.mma2_done[grp]));
+      for (int k = 0; k < 4; ++k) mma_bf16_elect(tDQ, desc_advance(dDSt, k * 32), desc_advance(dKt, k * 2048), idDQ, k > 0);
+      mma_commit_elect(smem_u32(&bars.dq_done[grp]));
+      // dK += dS^T Q
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        mma_bf16_elect(tm + S::tAcc + kLaneDK, desc_advance(dDSt, k * 2048), desc_advance(dQt, k * 2048), idKV, cur.c > 0 || k > 0);
+      mma_commit_elect(smem_u32(&bars.tiles_free[grp]));
       mma_commit_elect(smem_u32(&bars.q_free[stage]));
-      if (last) {
+      if (cur.last()) {
         mma_commit_elect(smem_u32(&bars.kv_free[kb]));
         mma_commit_elect(smem_u32(&bars.acc_full[grp]));   // the group of the item's last chunk flushes
       }
-    };
-    for (int it = blockIdx.x; it < nitems; it += gridDim.x, ++t) {
-      const int4 item = P.items[it];
-      const int kb = t & 1;
-      for (int c = 0; c < item.z; ++c, ++n) {
-        const int grp = n & 1, stage = n % kStages;
-        const uint32_t sQ = sQ0 + stage * 32768, sDO = sQ + 16384;
-        const uint32_t sK = sKV0 + kb * 16384, sV = sK + 8192;
-        mbar_wait_bounded(smem_u32(&bars.q_full[stage]), (uint32_t)(n / kStages) & 1, &abort_flag);
-        if (c == 0) mbar_wait_bounded(smem_u32(&bars.kv_full[kb]), (uint32_t)(t >> 1) & 1, &abort_flag);
-        __syncwarp();
-        tc_fence_after_sync();
-        {
-          // S and dP of the group are free: the group handed P and dS of its previous chunk over (waited for in
-          // issue_mma2 of that chunk, which ran before this point) only after reading them
-          const uint32_t tS = grp * 192, tDP = tS + 64;
-          const uint64_t dQt = smem_desc_sw128(sQ, 16), dDOt = smem_desc_sw128(sDO, 16), dKt = smem_desc_sw128(sK, 16),
-                         dVt = smem_desc_sw128(sV, 16);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            mma_bf16_elect(tm + tS, desc_advance(dQt, k * 32), desc_advance(dKt, k * 32), idS, k > 0);
-            mma_bf16_elect(tm + tDP, desc_advance(dDOt, k * 32), desc_advance(dVt, k * 32), idS, k > 0);
-          }
-          mma_commit_elect(smem_u32(&bars.s_full[grp]));
-        }
-        if (pending) issue_mma2(p_n, p_t, p_c, p_last);
-        pending = true;
-        p_n = n; p_t = t; p_c = c; p_last = (c == item.z - 1);
-      }
+      if (++stage == kStages) stage = 0;
     }
-    if (pending) issue_mma2(p_n, p_t, p_c, p_last);
     // nothing of this block may still be running on the tensor cores when tensor memory is freed
-    mma_commit_elect(smem_u32(&bars.drain));
-    mbar_wait_drain(smem_u32(&bars.drain), 0);
-    }
-  } else if (warp == 13) {
+    mma_commit_elect(smem_u32(&bars.drain[1]));
+    mbar_wait_drain(smem_u32(&bars.drain[1]), 0);
+  } else if (warp == kSoftmaxWarps + 2) {
     // ------------------------------------------------------------------ K/V tiles
     if (lane == 0) {
       int t = 0;
-      for (int it = blockIdx.x; it < nitems; it += gridDim.x, ++t) {
+      for (int it = first_item; it < nitems; it += gridDim.x, ++t) {
         const int4 item = P.items[it];
         const int list = item.x, j = list % P.nfb, bh = list / P.nfb, h = bh % P.Hkv, b = bh / P.Hkv;
-        const int kb = t & 1;
-        if (t >= 2) mbar_wait_bounded(smem_u32(&bars.kv_free[kb]), (uint32_t)((t >> 1) - 1) & 1, &abort_flag);
-        const uint32_t sK = sKV0 + kb * 16384, sV = sK + 8192;
+        const int kb = S::kKv == 2 ? t & 1 : 0, round = S::kKv == 2 ? t >> 1 : t;
+        if (round >= 1) mbar_wait_bounded(smem_u32(&bars.kv_free[kb]), (uint32_t)(round - 1) & 1, &abort_flag);
+        const uint32_t sK = sKV0 + kb * S::kKvBytes, sV = sK + S::kTileK;
         const uint32_t bar = smem_u32(&bars.kv_full[kb]);
-        mbar_arrive_expect_tx(bar, 2 * 8192);
-        tma_load_4d(sK, &tmK, bar, 0, j * kBlock, h, b);
-        tma_load_4d(sV, &tmV, bar, 0, j * kBlock, h, b);
+        mbar_arrive_expect_tx(bar, S::kKvBytes);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          tma_load_4d(sK + c * 8192, &tmK, bar, c * 64, j * kBlock, h, b);
+          tma_load_4d(sV + c * 8192, &tmV, bar, c * 64, j * kBlock, h, b);
+        }
       }
-      // the last two requests must have landed before the block may exit
-      for (int back = 1; back <= 2 && t - back >= 0; ++back) {
+      // the last requests must have landed before the block may exit
+      for (int back = 1; back <= S::kKv && t - back >= 0; ++back) {
         const int tt = t - back;
-        mbar_wait_drain(smem_u32(&bars.kv_full[tt & 1]), (uint32_t)(tt >> 1) & 1);
+        mbar_wait_drain(smem_u32(&bars.kv_full[S::kKv == 2 ? tt & 1 : 0]), (uint32_t)(S::kKv == 2 ? tt >> 1 : tt) & 1);
       }
     }
   } else {
     // ------------------------------------------------------------------ loaders
-    const int lt = tid - 9 * 32;           // 0..127
-    const int sub = lt & 7, r0 = lt >> 3;  // 16-byte piece of a row, first row (rows r0 + 16*k)
-    int n = 0, t = 0;
-    for (int it = blockIdx.x; it < nitems; it += gridDim.x, ++t) {
-      const int4 item = P.items[it];
-      const int list = item.x, bh = list / P.nfb, h = bh % P.Hkv, b = bh / P.Hkv;
-      const __nv_bfloat16* qb = P.q + b * P.q_sb;
-      const __nv_bfloat16* dob = P.dout + b * P.do_sb;
-      for (int c = 0; c < item.z; ++c, ++n) {
-        const int stage = n % kStages;
-        if (n >= kStages) mbar_wait_warp(smem_u32(&bars.q_free[stage]), (uint32_t)(n / kStages - 1) & 1, &abort_flag);
-        const uint32_t sQ = sQ0 + stage * 32768, sDO = sQ + 16384;
-        const uint32_t* chunk_entries = P.entries + item.w + c * QT;
+    constexpr int CH = D / 8, RPP = kLoaderThreads / CH, kPasses = kRows / RPP;   // pieces per row, rows per pass
+    const int lt = tid - (kSoftmaxWarps + 3) * 32;   // 0..127
+    const int sub = lt % CH, r0 = lt / CH;
+    for (Cursor cur(P.items, nitems, first_item); cur.live(); cur.next()) {
+      const int bh = cur.item.x / P.nfb, b = bh / P.Hkv, h = bh - b * P.Hkv;
+      const __nv_bfloat16* qb = P.q + b * P.q_sb + sub * 8;
+      const __nv_bfloat16* dob = P.dout + b * P.do_sb + sub * 8;
+      const int stage = cur.n % kStages;
+      if (cur.n >= kStages) mbar_wait_warp(smem_u32(&bars.q_free[stage]), (uint32_t)(cur.n / kStages - 1) & 1, &abort_flag);
+      const uint32_t sQ = sQ0 + stage * S::kStageBytes + (sub / 8) * 16384, sDO = sQ + S::kTileQ;
+      const uint32_t* chunk_entries = P.entries + cur.item.w + cur.c * QT;
+#pragma unroll
+      for (int k0 = 0; k0 < kPasses; k0 += 8) {
         // read the entries first: the copies below are compiler barriers, a load placed between them would be
-        // waited for eight times per chunk
+        // waited for eight times
         uint32_t ev[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) ev[k] = __ldg(chunk_entries + ((r0 + k * 16) >> g_shift));
+        for (int k = 0; k < 8; ++k) ev[k] = __ldg(chunk_entries + ((r0 + (k0 + k) * RPP) >> g_shift));
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-          const int row = r0 + k * 16;
+          const int row = r0 + (k0 + k) * RPP;
           const int g = row & ((1 << g_shift) - 1);
-          const uint32_t e = ev[k];
-          const bool valid = e != kInvalidEntry;
-          const int64_t i = valid ? (int64_t)(e & 0xffffffu) : 0;
+          const bool valid = ev[k] != kInvalidEntry;
+          const int64_t i = valid ? (int64_t)(ev[k] & 0xffffffu) : 0;
           const int64_t hq = (int64_t)((h << g_shift) + g);
-          const uint32_t off = sw128_offset(row, sub);
-          cp_async16(sQ + off, qb + hq * P.q_sh + i * P.q_sn + sub * 8, valid ? 16u : 0u);
-          cp_async16(sDO + off, dob + hq * P.do_sh + i * P.do_sn + sub * 8, valid ? 16u : 0u);
+          const uint32_t off = sw128_offset(row, sub % 8);
+          cp_async16(sQ + off, qb + hq * P.q_sh + i * P.q_sn, valid ? 16u : 0u);
+          cp_async16(sDO + off, dob + hq * P.do_sh + i * P.do_sn, valid ? 16u : 0u);
         }
-        {
-          // metadata of row lt: its entry and the statistics of its (query, head)
-          const uint32_t e = __ldg(chunk_entries + (lt >> g_shift));
-          const bool valid = e != kInvalidEntry;
-          const int64_t row = ((int64_t)b * P.Hq + (int64_t)((h << g_shift) + (lt & ((1 << g_shift) - 1)))) * P.N +
-                              (valid ? (int64_t)(e & 0xffffffu) : 0);
-          const uint32_t sMeta = sMeta0 + stage * kMetaBytes + lt * 4;
-          cp_async4(sMeta, chunk_entries + (lt >> g_shift), 4u);
-          cp_async4(sMeta + kRows * 4, P.lse + row, valid ? 4u : 0u);
-          cp_async4(sMeta + 2 * kRows * 4, P.delta + row, valid ? 4u : 0u);
-        }
-        // the stage announces itself when this thread's copies have landed; the thread moves on at once
-        cp_async_arrive_noinc(smem_u32(&bars.q_full[stage]));
       }
+      {
+        // the statistics of row lt
+        const uint32_t e = __ldg(chunk_entries + (lt >> g_shift));
+        const bool valid = e != kInvalidEntry;
+        const int64_t row = ((int64_t)b * P.Hq + (int64_t)((h << g_shift) + (lt & ((1 << g_shift) - 1)))) * P.N +
+                            (valid ? (int64_t)(e & 0xffffffu) : 0);
+        const uint32_t sMeta = sMeta0 + stage * S::kMetaBytes + lt * 4;
+        cp_async4(sMeta, P.lse + row, valid ? 4u : 0u);
+        cp_async4(sMeta + kRows * 4, P.delta + row, valid ? 4u : 0u);
+      }
+      // the stage announces itself when this thread's copies have landed; the thread moves on at once
+      cp_async_arrive_noinc(smem_u32(&bars.q_full[stage]));
     }
     cp_async_commit();
     cp_async_wait<0>();
@@ -1876,17 +1626,18 @@ sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 template <int D, int MODE>
 __global__ void __launch_bounds__(256) sel_dq_merge_kernel(const SelParams P) {
   constexpr int TPR = D / 8;
-  const int64_t row = ((int64_t)blockIdx.x * 256 + threadIdx.x) / TPR;
+  const int64_t part_row = ((int64_t)blockIdx.x * 256 + threadIdx.x) / TPR;   // row of the slice
   const int part = threadIdx.x % TPR;
-  const int64_t nrows = (int64_t)P.B * P.Hq * P.N;
-  if (row >= nrows) return;
+  const int64_t first = (int64_t)P.bh0 * P.G * P.N, nrows = (int64_t)(P.bh1 - P.bh0) * P.G * P.N;
+  if (part_row >= nrows) return;
+  const int64_t row = first + part_row;
   const int i = (int)(row % P.N);
   const int hq = (int)((row / P.N) % P.Hq);
   const int b = (int)(row / ((int64_t)P.N * P.Hq));
   const int h = hq / P.G;
   const int ns = P.ns;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  const __nv_bfloat16* prow = P.partial + row * ns * D + part * 8;
+  const __nv_bfloat16* prow = P.partial + part_row * ns * D + part * 8;
   // eight slots at a time: first which of them the query has, then their loads together, then the sums
   const uint32_t* bits = P.bits + ((int64_t)(b * P.Hkv + h) * P.N + i) * P.words;
   for (int s0 = 0; s0 < ns; s0 += 8) {
@@ -2015,6 +1766,8 @@ static bool dense_forward_serves(const SelProblem& a) {
   return a.out.stride_n == a.D && a.out.stride_h == (int64_t)a.N * a.D && a.out.stride_b == (int64_t)a.Hq * a.N * a.D;
 }
 
+constexpr int64_t kPartialBudget = 8ll << 30;
+
 static SelPlan make_plan(const SelProblem& a, bool backward) {
   SelPlan p;
   p.nqb = (a.N + kBlock - 1) / kBlock;
@@ -2030,7 +1783,7 @@ static SelPlan make_plan(const SelProblem& a, bool backward) {
   p.off_status = off; off += 256;
   p.off_num_items = p.off_status + 128;
   if (!backward && dense_forward(a)) {   // only the status word is needed
-    p.off_totals = p.off_list_base = p.off_cursors = p.off_bits = p.off_items = p.off_entries = off;
+    p.off_totals = p.off_list_base = p.off_list_item = p.off_cursors = p.off_bits = p.off_items = p.off_entries = off;
     p.off_partial = p.off_stats = p.off_delta = off;
     p.index_bytes = 0;
     p.total_bytes = off;
@@ -2038,6 +1791,7 @@ static SelPlan make_plan(const SelProblem& a, bool backward) {
   }
   p.off_totals = off; off = align_up(off + (int64_t)p.nlists * 4, 256);
   p.off_list_base = off; off = align_up(off + (int64_t)p.nlists * 4, 256);
+  p.off_list_item = off; off = align_up(off + (int64_t)(p.nlists + 1) * 4, 256);
   p.off_cursors = off; off = align_up(off + (int64_t)p.nlists * 4, 256);
   p.off_bits = off; off = align_up(off + (int64_t)a.B * a.Hkv * a.N * p.words * 4, 256);
   p.off_items = off; off = align_up(off + p.items_cap * 16, 256);
@@ -2045,12 +1799,21 @@ static SelPlan make_plan(const SelProblem& a, bool backward) {
   p.index_bytes = off;   // status word, totals, list bases, slot bits, items, entries: the same layout forward and backward
   const int64_t rows = (int64_t)a.B * a.Hq * a.N;
   p.off_partial = p.off_stats = p.off_delta = off;
+  p.slices = p.pairs_per_slice = 1;
   if (!backward) {
     p.off_partial = off; off = align_up(off + rows * p.ns * a.D * 2, 256);
     p.off_stats = off; off = align_up(off + rows * p.ns * 8, 256);
   } else {
+    // very long inputs (64 heads of 128 at 65536 positions: 70 GB for the compressed branch) run in slices of whole
+    // (batch, KV head) pairs that share a buffer of at most kPartialBudget, or of one pair
     p.off_delta = off; off = align_up(off + rows * 4, 256);
-    if (a.D == 64) { p.off_partial = off; off = align_up(off + rows * p.ns * a.D * 2, 256); }
+    const int pairs = a.B * a.Hkv;
+    const int64_t per_pair = (int64_t)p.G * a.N * p.ns * a.D * 2, most = kPartialBudget / per_pair;
+    const int per_slice = (int)(most < 1 ? 1 : most < pairs ? most : pairs);
+    p.slices = (pairs + per_slice - 1) / per_slice;
+    p.pairs_per_slice = (pairs + p.slices - 1) / p.slices;
+    p.slices = (pairs + p.pairs_per_slice - 1) / p.pairs_per_slice;
+    p.off_partial = off; off = align_up(off + p.pairs_per_slice * per_pair, 256);
   }
   p.total_bytes = off;
   return p;
@@ -2135,6 +1898,7 @@ static int build_index(const SelProblem& a, const SelPlan& p, uint8_t* ix, cudaS
   int4* items = reinterpret_cast<int4*>(ix + p.off_items);
   int* num_items = reinterpret_cast<int*>(ix + p.off_num_items);
   uint32_t* entries = reinterpret_cast<uint32_t*>(ix + p.off_entries);
+  int* list_item = reinterpret_cast<int*>(ix + p.off_list_item);
   const BlockRule R = make_rule(a, p);
   const dim3 grid((a.N + kIndexQueries - 1) / kIndexQueries, a.B, a.Hkv);
   const size_t hist_smem = (size_t)p.nkb * sizeof(int);   // at most 32 KB
@@ -2142,7 +1906,7 @@ static int build_index(const SelProblem& a, const SelPlan& p, uint8_t* ix, cudaS
   if (a.mode == kModeSel) sel_count_kernel<kModeSel><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, bits, p.words);
   else if (a.mode == kModeSwa) sel_count_kernel<kModeSwa><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, bits, p.words);
   else sel_count_kernel<kModeCmp><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, bits, p.words);
-  sel_items_kernel<<<1, 1024, 0, st>>>(totals, list_base, cursors, items, num_items, p.nlists, p.QT, index_tag(a, p));
+  sel_items_kernel<<<1, 1024, 0, st>>>(totals, list_base, list_item, cursors, items, num_items, p.nlists, p.QT, index_tag(a, p));
   if (a.mode == kModeSel) sel_fill_kernel<kModeSel><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, list_base, cursors, entries, p.QT);
   else if (a.mode == kModeSwa) sel_fill_kernel<kModeSwa><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, list_base, cursors, entries, p.QT);
   else sel_fill_kernel<kModeCmp><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, list_base, cursors, entries, p.QT);
@@ -2184,6 +1948,8 @@ static void fill_params(SelParams& P, const SelProblem& a, const SelPlan& p, uin
   P.num_items = reinterpret_cast<const int*>(ix + p.off_num_items);
   P.index_tag = index_tag(a, p);
   P.bits = reinterpret_cast<const uint32_t*>(ix + p.off_bits);
+  P.list_item = reinterpret_cast<const int*>(ix + p.off_list_item);
+  P.bh0 = 0; P.bh1 = a.B * a.Hkv;
   P.words = p.words;
   P.status = a.status != nullptr ? a.status : reinterpret_cast<int*>(ws + p.off_status);
   P.lse = a.lse;
@@ -2299,28 +2065,20 @@ static int run_bwd(const SelProblem& a, const SelPlan& p, uint8_t* ws, cudaStrea
   const int64_t threads = (int64_t)a.B * a.Hq * a.N * (D / 8);
   const int own_delta = a.delta == nullptr ? 1 : 0;   // the caller may hand the row sums over
   if (own_delta) sel_delta_kernel<D><<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(P, delta);
-  if (D == 64) {
-    const int smem = 1024 + ws::kStages * 32768 + 2 * ws::kPBytes + 2 * 16384 + ws::kStages * ws::kMetaBytes +
-                     8 * ws::kDqStage;
-    CUDA_TRY(cudaFuncSetAttribute(sel_bwd_ws_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    P.partial = reinterpret_cast<__nv_bfloat16*>(ws + p.off_partial);
-    sel_bwd_ws_kernel<<<num_sms(), ws::kThreads, smem, st>>>(tmK, tmV, P);
-    const unsigned mblocks = (unsigned)((threads + 255) / 256);
-    if (a.mode == kModeSel) sel_dq_merge_kernel<64, kModeSel><<<mblocks, 256, 0, st>>>(P);
-    else if (a.mode == kModeSwa) sel_dq_merge_kernel<64, kModeSwa><<<mblocks, 256, 0, st>>>(P);
-    else sel_dq_merge_kernel<64, kModeCmp><<<mblocks, 256, 0, st>>>(P);
-    CUDA_TRY(cudaGetLastError());
-    count_launches(2 + own_delta);   // (delta,) backward kernel, dQ merge
-    return NSA_OK;
+  if (a.slot_grads != nullptr) CUDA_TRY(cudaMemsetAsync(a.slot_grads, 0, (size_t)a.B * a.Hkv * a.N * a.nsel * sizeof(float), st));
+  CUDA_TRY(allow_shared_memory<sel_bwd_ws_kernel<D>>());
+  P.partial = reinterpret_cast<__nv_bfloat16*>(ws + p.off_partial);
+  for (int s = 0; s < p.slices; ++s) {
+    P.bh0 = s * p.pairs_per_slice;
+    P.bh1 = P.bh0 + p.pairs_per_slice < a.B * a.Hkv ? P.bh0 + p.pairs_per_slice : a.B * a.Hkv;
+    sel_bwd_ws_kernel<D><<<num_sms(), ws::kThreads, ws::Shape<D>::kBytes, st>>>(tmK, tmV, P);
+    const unsigned mblocks = (unsigned)(((int64_t)(P.bh1 - P.bh0) * p.G * a.N * (D / 8) + 255) / 256);
+    if (a.mode == kModeSel) sel_dq_merge_kernel<D, kModeSel><<<mblocks, 256, 0, st>>>(P);
+    else if (a.mode == kModeSwa) sel_dq_merge_kernel<D, kModeSwa><<<mblocks, 256, 0, st>>>(P);
+    else sel_dq_merge_kernel<D, kModeCmp><<<mblocks, 256, 0, st>>>(P);
   }
-  CUDA_TRY(cudaMemsetAsync(P.dq, 0, (size_t)a.B * a.Hq * a.N * D * sizeof(float), st));   // the kernel adds into dq
-  constexpr int NC = D / 64;
-  const int smem = 1024 + NC * (2 * 16384 + 2 * 8192) + kRows * (D * 4 + 16);
-  const int per_sm = D == 64 ? 2 : 1;
-  CUDA_TRY(cudaFuncSetAttribute(sel_bwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  sel_bwd_kernel<D><<<num_sms() * per_sm, kRows, smem, st>>>(tmK, tmV, P);
   CUDA_TRY(cudaGetLastError());
-  count_launches(1 + own_delta);   // (delta,) backward kernel
+  count_launches(2 * p.slices + own_delta);   // (delta,) backward kernel and dQ merge per slice
   return NSA_OK;
 }
 
@@ -2389,8 +2147,6 @@ static int problem_fwd(const SelProblem& x, cudaStream_t st) {
 }
 
 static int problem_bwd(const SelProblem& x, cudaStream_t st) {
-  // dq in the caller's dtype and strides: only the merge of the partials writes whole rows of dq
-  if (x.dq_out.ptr != nullptr && !(x.D == 64)) return NSA_ERR_UNSUPPORTED;
   const SelPlan p = make_plan(x, true);
   uint8_t* ws = nullptr;
   const int rc = check_ws(x, p, &ws);
@@ -2435,15 +2191,15 @@ int sm100_sel_bwd(const nsa_sel_bwd_args& b, cudaStream_t st) {
 // True when the backward of this problem stores every row of dq (partials + ordered merge) instead of adding into it.
 bool sm100_sel_bwd_overwrites_dq(const nsa_sel_fwd_args& a) {
   SelProblem x;
-  return sel_problem(x, a) && x.D == 64;
+  return sel_problem(x, a);
 }
 bool sm100_swa_bwd_overwrites_dq(const nsa_swa_fwd_args& a) {
   SelProblem x;
-  return swa_problem(x, a) && x.D == 64;
+  return swa_problem(x, a);
 }
 bool sm100_cmp_bwd_overwrites_dq(const nsa_cmp_fwd_args& a) {
   SelProblem x;
-  return cmp_problem(x, a) && x.D == 64;
+  return cmp_problem(x, a);
 }
 
 // The index of the sliding and the compressed backward depends on the sizes only: a caller may keep it across calls.

@@ -657,3 +657,21 @@ def test_dense_forward_at_the_edges_of_its_tiles_and_streams(case):
     seen = ref_imp > -1e30
     assert torch.equal(seen, imp > -1e30)
     assert_close_bf16(imp[seen], ref_imp[seen], 'importance', roundings=4)
+
+
+def test_backward_in_slices_equals_the_whole():
+    # partial results beyond the buffer's budget: the (batch, KV head) pairs run in slices.  Each half fits at once; dq
+    # must be the same to the bit, dk and dv are sums of fp32 reductions in any order
+    q, k, v, up = (torch.randn((1, h, 65536, 128), device=DEV).bfloat16() for h in (64, 4, 4, 64))
+
+    def grads(part, group):
+        qs, ks, vs = (t[:, part.start * m:part.stop * m].clone().requires_grad_() for t, m in ((q, group), (k, 1), (v, 1)))
+        out = nsa.sliding_window_attend(qs, ks, vs, 448, True, impl='sm100')
+        return torch.autograd.grad(out, (qs, ks, vs), up[:, part.start * group:part.stop * group])
+
+    whole = grads(slice(0, 4), 16)
+    halves = [grads(slice(p, p + 2), 16) for p in (0, 2)]
+    ops.check_device_status()
+    assert torch.equal(whole[0], torch.cat([h[0] for h in halves], dim=1))
+    for i in (1, 2):
+        assert_close_bf16(whole[i], torch.cat([h[i] for h in halves], dim=1), 'dk dv', roundings=2, rel_to_max=1e-3)
