@@ -8,9 +8,15 @@
 #include <ATen/Context.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <cublas_v2.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
 
 #include <cmath>
 #include <limits>
+#include <list>
+#include <mutex>
 
 #include "nsa_kernels.h"
 #include "rooms.h"
@@ -566,10 +572,129 @@ static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor>
   return g;
 }
 
+// The index of the sliding and of the compressed backward depends on the sizes only: kept for the last few shapes, per
+// stream (so that none is read by another stream than the one that built it).
+class IndexCache {
+ public:
+  using Key = std::vector<int64_t>;
+  static IndexCache& instance() {
+    static IndexCache* cache = new IndexCache;   // never destroyed: tensors must not outlive the CUDA context's teardown order
+    return *cache;
+  }
+  OptTensor find(const Key& key) {
+    const std::lock_guard<std::mutex> lock(mutex_);
+    for (const auto& e : entries_)
+      if (e.first == key) return e.second;
+    return {};
+  }
+  void keep(Key key, const Tensor& index) {
+    const std::lock_guard<std::mutex> lock(mutex_);
+    if (entries_.size() >= kMost) entries_.pop_front();
+    entries_.emplace_back(std::move(key), index);
+  }
+
+ private:
+  static constexpr size_t kMost = 16;
+  std::mutex mutex_;
+  std::list<std::pair<Key, Tensor>> entries_;
+};
+
+// The autograd node.  A Python function in its place cost 80 us per backward (the call from the engine's thread, saved
+// tensors and gradients crossing the language border one by one).
+struct NativeLayerBackward : torch::autograd::Node {
+  std::vector<torch::autograd::SavedVariable> weights, saved;
+  double eps = 0;
+  Tensor inv_freq;
+  std::vector<int64_t> cfg;
+  int64_t status = 0;
+
+  void release_variables() override {
+    for (auto& v : weights) v.reset_data();
+    for (auto& v : saved) v.reset_data();
+  }
+
+  torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
+    torch::autograd::variable_list out(1 + kWeights);
+    if (!grads[0].defined()) return out;
+    try {
+      const at::NoGradGuard no_grad;
+      auto unpack = [&](std::vector<torch::autograd::SavedVariable>& vs) {
+        std::vector<OptTensor> ts;
+        ts.reserve(vs.size());
+        for (auto& v : vs) {
+          Tensor t = v.unpack(getptr());
+          ts.emplace_back(t.defined() ? OptTensor(std::move(t)) : OptTensor());
+        }
+        return ts;
+      };
+      const std::vector<OptTensor> w = unpack(weights), sv = unpack(saved);
+      std::vector<bool> needs(1 + kWeights);
+      for (int i = 0; i < 1 + kWeights; ++i) needs[i] = task_should_compute_output(i);
+      const Tensor& x = *sv.at(0);
+      const LayerConfig c = config_of(cfg);
+      const IndexCache::Key base = {x.get_device(), reinterpret_cast<int64_t>(stream_of(x)), x.size(0), c.heads, c.kv_heads, x.size(1), c.d,
+                                    c.causal};
+      IndexCache::Key swa = base, cmp = base;
+      swa.insert(swa.end(), {0, c.window});
+      cmp.insert(cmp.end(), {1, c.num_mem, c.stride});
+      auto& cache = IndexCache::instance();
+      std::vector<OptTensor> g = layer_backward(grads[0], w, sv, eps, inv_freq, cfg, status, std::move(needs), cache.find(swa), cache.find(cmp));
+      for (int i = 0; i < 1 + kWeights; ++i)
+        if (g[i].has_value()) out[i] = std::move(*g[i]);
+      if (g[1 + kWeights].has_value()) cache.keep(std::move(swa), *g[1 + kWeights]);
+      if (g[2 + kWeights].has_value()) cache.keep(std::move(cmp), *g[2 + kWeights]);
+    } catch (const Error& e) {
+      raise_python_error(e.what());
+    }
+    if (at::GradMode::is_enabled()) {   // create_graph: the gradients are there, their own gradients are not
+      for (auto& t : out)
+        if (t.defined()) t.set_requires_grad(true);
+      torch::autograd::DelayedError fail("trying to differentiate twice the layer's native backward", (int64_t)out.size());
+      return fail.apply(std::move(out));
+    }
+    return out;
+  }
+
+ private:
+  [[noreturn]] static void raise_python_error(const char* what) {
+    const pybind11::gil_scoped_acquire gil;
+    PyErr_SetString(error_class(), what);
+    python_error err;
+    err.persist();
+    throw err;
+  }
+};
+
+static Tensor layer_apply(Tensor x, std::vector<OptTensor> weights, double eps, Tensor inv_freq, std::vector<int64_t> cfg, int64_t status) {
+  if (x._fw_grad(0).defined()) throw Error("the layer has no forward-mode derivative");
+  auto node = std::shared_ptr<NativeLayerBackward>(new NativeLayerBackward, torch::autograd::deleteNode);
+  torch::autograd::edge_list edges = {torch::autograd::impl::gradient_edge(x)};
+  node->weights.reserve(kWeights);
+  for (const auto& w : weights) {
+    edges.push_back(w.has_value() ? torch::autograd::impl::gradient_edge(*w) : torch::autograd::Edge());
+    node->weights.emplace_back(w.value_or(Tensor()), false);
+  }
+  node->set_next_edges(std::move(edges));
+  node->eps = eps;
+  node->inv_freq = inv_freq;
+  node->cfg = cfg;
+  node->status = status;
+  std::vector<OptTensor> r;
+  {
+    const at::NoGradGuard no_grad;
+    r = layer_forward(x, std::move(weights), eps, inv_freq, std::move(cfg), status, true, false);
+  }
+  node->saved.reserve(r.size() - 1);
+  for (size_t i = 1; i < r.size(); ++i) node->saved.emplace_back(i == 1 && r[i]->is_same(x) ? x : r[i].value_or(Tensor()), false);
+  Tensor out = *r[0];
+  torch::autograd::set_history(out, node);
+  return out;
+}
+
 void bind_layer(pybind11::module_& m) {
   namespace py = pybind11;
   m.def("layer_forward", &layer_forward, py::call_guard<py::gil_scoped_release>());
-  m.def("layer_backward", &layer_backward, py::call_guard<py::gil_scoped_release>());
+  m.def("layer_apply", &layer_apply, py::call_guard<py::gil_scoped_release>());
 }
 
 }  // namespace nsa_host

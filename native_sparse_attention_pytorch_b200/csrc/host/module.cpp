@@ -6,13 +6,15 @@ namespace py = pybind11;
 
 static PyObject* g_error_class = nullptr;   // the package's NsaError, handed over once at load time
 
+PyObject* nsa_host::error_class() { return g_error_class != nullptr ? g_error_class : PyExc_RuntimeError; }
+
 PYBIND11_MODULE(_nsa_host, m) {
   m.def("set_error_class", [](py::object cls) { g_error_class = cls.release().ptr(); });
   py::register_exception_translator([](std::exception_ptr p) {
     try {
       if (p) std::rethrow_exception(p);
     } catch (const nsa_host::Error& e) {
-      PyErr_SetString(g_error_class != nullptr ? g_error_class : PyExc_RuntimeError, e.what());
+      PyErr_SetString(nsa_host::error_class(), e.what());
     }
   });
   nsa_host::bind_status(m);

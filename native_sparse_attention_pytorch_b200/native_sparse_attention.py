@@ -32,42 +32,6 @@ def _untouched(module, cls):
                                             d['_backward_pre_hooks'] or 'forward' in d)
 
 
-class _NativeLayer(torch.autograd.Function):
-    """The layer as one autograd node (csrc/host/layer.cpp): f(call, x, *weights), `call` = (eps, inverse frequencies,
-    configuration)."""
-
-    @staticmethod
-    def forward(ctx, call, x, *weights):
-        eps, inv_freq, cfg = call
-        out, *saved = L.host().layer_forward(x, weights, eps, inv_freq, cfg, ops._status_word(x.device), True, False)
-        ctx.save_for_backward(*weights, *saved)
-        ctx.call = call
-        return out
-
-    @staticmethod
-    @torch.autograd.function.once_differentiable
-    def backward(ctx, dout):
-        eps, inv_freq, cfg = ctx.call
-        weights, saved = ctx.saved_tensors[:_WEIGHTS], ctx.saved_tensors[_WEIGHTS:]
-        x = saved[0]
-        b, n, _ = x.shape
-        heads, kv_heads, d, window, _, stride, _, _, num_mem, causal, _, _ = cfg
-        # the index of the sliding and the compressed backward depends on the sizes only
-        q = (b, heads, n, d)
-        keys = (('swa', x.device.index, q, (b, kv_heads, n, d), window, bool(causal), L.IMPL_AUTO),
-                ('cmp', x.device.index, q, (b, kv_heads, num_mem + n // stride, d), num_mem, stride, bool(causal), L.IMPL_AUTO))
-        indices = [ops._cached_index(k) for k in keys]
-        *grads, swa_index, cmp_index = L.host().layer_backward(
-            dout, weights, saved, eps, inv_freq, cfg, ops._status_word(x.device), ctx.needs_input_grad[1:], *indices)
-        for key, built in zip(keys, (swa_index, cmp_index)):
-            if built is not None:
-                ops._keep_index(key, built, built.numel())
-        return (None, *grads)
-
-
-_WEIGHTS = 16
-
-
 class _Windows(Module):
     """[B,H,N,d] -> [B,H,ncb,cbs,d]: window w holds tokens (w+1)*stride-cbs .. (w+1)*stride-1,
     zero where that is negative (same result as upstream's pad + unfold, NSA:270-275)."""
@@ -226,7 +190,7 @@ class SparseAttention(Module):
         if torch.is_grad_enabled() and (x.requires_grad or any([p.requires_grad for p in weights if p is not None])):
             if return_cache or (w[0] is not None and x.shape[2] * x.element_size() > 16 * MAX_PIECES):
                 return None
-            return _NativeLayer.apply((eps, inv_freq, cfg), x, *weights)
+            return L.host().layer_apply(x, weights, eps, inv_freq, cfg, ops._status_word(x.device))
         out, *cache = L.host().layer_forward(x, weights, eps, inv_freq, cfg, ops._status_word(x.device), False, return_cache)
         if not return_cache:
             return out
