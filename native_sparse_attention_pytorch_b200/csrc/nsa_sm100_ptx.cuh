@@ -295,6 +295,16 @@ __device__ __forceinline__ uint4 lds_v4(uint32_t addr) {
   return v;
 }
 
+// Bulk (TMA) copy from this CTA's shared memory to global memory; size is a multiple of 16 bytes and both addresses are
+// 16-byte aligned.  Whoever wrote the shared memory must have run fence_proxy_async_smem() first.
+__device__ __forceinline__ void bulk_store(void* gdst, uint32_t ssrc, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gdst), "r"(ssrc), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// Waits until the bulk copies of this thread no longer read shared memory, or until they are complete.
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 // Byte offset of 16-byte chunk `chunk` (0..7) of row `row` inside a swizzled [rows x 128 B] tile.
 __device__ __forceinline__ uint32_t sw128_offset(int row, int chunk) {
   return static_cast<uint32_t>(row * 128 + ((chunk ^ (row & 7)) << 4));

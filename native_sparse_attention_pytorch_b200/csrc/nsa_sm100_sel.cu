@@ -87,7 +87,7 @@ struct SelPlan {
   int64_t entries_cap, items_cap;
   // byte offsets into the work buffer
   int words;             // 32-bit words of slot bits per query
-  int64_t off_status, off_num_items, off_totals, off_list_base, off_list_item, off_cursors, off_bits, off_items, off_entries;
+  int64_t off_status, off_num_items, off_totals, off_list_base, off_list_item, off_cursors, off_bits, off_items, off_entries, off_positions;
   int64_t off_partial, off_stats, off_delta;
   int slices, pairs_per_slice;   // backward: launches over the (batch, KV head) pairs
   int64_t index_bytes;   // the leading part that holds the index (what the backward can take from the forward)
@@ -104,6 +104,7 @@ struct SelParams {
   const int4* items;
   const int* num_items;    // [0] items, [1] the tag the item kernel left
   const int* list_item;    // per list (and one more): its first item
+  const int* positions;    // kModeSel: [B*Hkv*N][ns], the entry of every (query, slot)
   int bh0, bh1;            // backward: the (batch, KV head) pairs of this launch, whose partial results share the buffer
   const uint32_t* bits;    // [B*Hkv*N][words]: the slots a query has (kModeSel)
   int words;
@@ -130,10 +131,20 @@ struct SelParams {
   int cpf, pool_cols, pool_block;
 };
 
+// The partial results of the forward lie chunk by chunk, as they leave shared memory: row r of chunk c at (128 c + r) * 2 D
+// bytes, its 16-byte pieces exchanged by r & 7.  A chunk is then one bulk store, which leaves the load / store units to
+// the gathers; the merge finds the row of (query, slot) through `positions` (row = entry * G + head of the group) and
+// reads the G heads side by side.
+template <int D>
+__device__ __forceinline__ const uint4* partial_piece(const __nv_bfloat16* partial, int64_t row, int part) {
+  return reinterpret_cast<const uint4*>(partial) + row * (D / 8) + (part ^ (int)(row & 7));
+}
+
 // Number of items of the index, or 0 (and status 2) when the index was not built for these sizes: a caller-kept
 // index that belongs to another problem, or a buffer nobody filled, must not steer any address.
+__device__ __forceinline__ bool foreign_index(const SelParams& P) { return (uint32_t)P.num_items[1] != P.index_tag; }
 __device__ __forceinline__ int item_count(const SelParams& P) {
-  if ((uint32_t)P.num_items[1] != P.index_tag) {
+  if (foreign_index(P)) {
     if (threadIdx.x == 0) atomicOr(P.status, 2);
     return 0;
   }
@@ -251,10 +262,10 @@ __global__ void __launch_bounds__(1024) sel_items_kernel(const int* totals, int*
   }
 }
 
-// writes the entries (query | slot << 24) and pads every list to whole chunks
+// writes the entries (query | slot << 24) and, for the forward, where each one is, and pads every list to whole chunks
 template <int MODE>
 __global__ void __launch_bounds__(kIndexQueries) sel_fill_kernel(const BlockRule R, const int* totals, const int* list_base,
-                                                                 int* cursors, uint32_t* entries, int QT) {
+                                                                 int* cursors, uint32_t* entries, int* positions, int QT) {
   extern __shared__ int cursor[];
   const int bh = blockIdx.y * gridDim.z + blockIdx.z;
   const int lane = threadIdx.x & 31;
@@ -289,6 +300,7 @@ __global__ void __launch_bounds__(kIndexQueries) sel_fill_kernel(const BlockRule
       if (lane == leader) pos = atomicAdd(&cursor[blk], __popc(peers));
       pos = __shfl_sync(peers, pos, leader) + __popc(peers & ((1u << lane) - 1u));
       entries[pos] = (uint32_t)i | ((uint32_t)s << 24);
+      if (MODE == kModeSel) positions[((int64_t)bh * R.N + i) * R.ns + s] = pos;
     }
   }
 }
@@ -324,10 +336,12 @@ __device__ __forceinline__ RowInfo decode_row(uint32_t e, int j, const BlockRule
 
 // Forward of the selected-block branch.  A CTA of 256 threads walks gather -> S -> softmax -> P V -> store chunk by
 // chunk; several CTAs share an SM (4 at dim_head 64) and fill each other's waits.  Two threads share a row (32 of the
-// block's 64 columns each; they exchange maximum and sum through shared memory), which halves the serial work per
-// thread and, above all, doubles the number of warps that issue the gather: a warp gets only about 1.3 bytes per
-// clock of scattered 128-byte rows out of the L2 however many copies it has in flight (measured: 5.5 B/clk per SM
-// with 4 warps copying, 17 with 16, 26 with 32), and the gather of the Q rows is what bounds this kernel.
+// block's 64 columns each; they exchange maximum and sum through shared memory), which halves the serial work per thread.
+// What bounds it: the gather of the Q rows, 18 bytes per clock and SM out of the L2 (900 cycles for the 16 KB of a chunk
+// at dim_head 64, measured with nothing else running, whatever the number of copying warps; as TMA boxes or gathers 1900
+// and more), plus 440 for the bulk store of the partial rows; the chunk takes 1900.  With the partial rows stored row by
+// row through the load / store units it took 2200: batch 4, 8192 positions, 32 / 4 heads of 64 1.10 -> 0.96 ms, 65536
+// positions, 64 / 8 heads of 128 9.1 -> 7.4 ms.
 template <int D>
 __device__ __forceinline__ void gather_tile_async2(uint32_t tile, const __nv_bfloat16* base, int64_t stride_h,
                                                    int64_t stride_n, const uint32_t* entries, int g_shift, int h,
@@ -357,14 +371,12 @@ sel_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
   __shared__ int abort_flag;
   __shared__ uint32_t tmem_slot;
   __shared__ __align__(8) uint64_t bars[3];
-  __shared__ int row_dst[kRows];
   __shared__ float xmax[2][kRows], xsum[2][kRows];
   const int nitems = item_count(P);
   if ((int)blockIdx.x >= nitems) return;
 
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t sQ = base, sK = sQ + NC * 16384, sV = sK + NC * 8192, sStage = sV + NC * 8192;
-  constexpr uint32_t kStageStride = D * 2 + 16;   // one padded partial-output row per row of the chunk
   const uint32_t bar_kv = smem_u32(&bars[0]), bar_s = smem_u32(&bars[1]), bar_o = smem_u32(&bars[2]);
   const int tid = threadIdx.x, warp = tid >> 5;
   const int half = tid >> 7, row = tid & (kRows - 1);   // this thread: columns 32*half .. 32*half+31 of row `row`
@@ -392,7 +404,7 @@ sel_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
   const uint32_t tS = 0, tO = 64;
 
   const int G = P.G, QT = kRows / G, g_shift = 31 - __clz(G);
-  const int q_local = row >> g_shift, g = row - (q_local << g_shift);
+  const int q_local = row >> g_shift;
   uint32_t ph_kv = 0, ph_s = 0, ph_o = 0;
   constexpr uint32_t idS = instr_desc_bf16(128, 64, false, false);
   constexpr uint32_t idO = instr_desc_bf16(128, D, false, true);
@@ -457,6 +469,7 @@ sel_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
       }
       float m = fmaxf(fmaxf(mm[0], mm[1]), fmaxf(mm[2], mm[3]));
       xmax[half][row] = m;
+      if (tid == 0) bulk_wait_read();   // the staging tile's last store has left shared memory (written again behind the barriers)
       __syncthreads();
       m = fmaxf(m, xmax[half ^ 1][row]);
       const float m2 = r.valid ? m * P.scale_log2 : 0.f;
@@ -489,9 +502,7 @@ sel_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
         mma_commit_elect(bar_o);
       }
       const float l = xsum[0][row] + xsum[1][row];
-      const int64_t hq = (int64_t)h * G + g;
-      const int64_t row_global = ((int64_t)b * P.Hq + hq) * P.N + r.i;
-      const int64_t pslot = r.valid ? row_global * P.ns + r.slot : 0;
+      const int64_t chunk = item.w / QT + c;
       __syncwarp();
       mbar_wait_warp(bar_o, ph_o, &abort_flag);
       ph_o ^= 1;
@@ -510,86 +521,114 @@ sel_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
           v.y = pack_bf16(t[x * 8 + 2], t[x * 8 + 3]);
           v.z = pack_bf16(t[x * 8 + 4], t[x * 8 + 5]);
           v.w = pack_bf16(t[x * 8 + 6], t[x * 8 + 7]);
-          sts_v4(sStage + row * kStageStride + half * D + c2 * 64 + x * 16, v);
+          const int piece = half * (D / 16) + c2 * 4 + x;   // 16-byte piece of the row
+          sts_v4(sStage + row * (D * 2) + ((piece ^ (row & 7)) << 4), v);
         }
       }
-      if (half == 0) row_dst[row] = r.valid ? (int)pslot : -1;
+      if (half == 0) P.stats[chunk * kRows + row] = make_float2(m2, l);
+      fence_proxy_async_smem();
       tc_fence_before_sync();
       __syncthreads();
-      {   // whole 128-byte lines per store instruction: D/8 neighbouring threads share a row
-        constexpr int TPR = D / 8, RPP = 2 * kRows / TPR;
-        const int sub = tid % TPR, r0 = tid / TPR;
-        uint8_t* const pbase = reinterpret_cast<uint8_t*>(P.partial);
-#pragma unroll
-        for (int k = 0; k < kRows / RPP; ++k) {
-          const int rr = r0 + k * RPP;
-          const int dst = row_dst[rr];
-          const uint4 v = lds_v4(sStage + rr * kStageStride + sub * 16);
-          if (dst >= 0) *reinterpret_cast<uint4*>(pbase + (int64_t)dst * (D * 2) + sub * 16) = v;
-        }
+      if (tid == 0) {
+        bulk_store(reinterpret_cast<uint8_t*>(P.partial) + chunk * (NC * 16384), sStage, NC * 16384);
+        bulk_commit();
       }
-      if (half == 0 && r.valid) P.stats[pslot] = make_float2(m2, l);
     }
     ph_kv ^= 1;
     __syncthreads();   // every thread is done with this item's tiles before the next TMA overwrites them
   }
 
+  if (tid == 0) bulk_wait_all();
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tm, kCols);
   if (tid == 0 && abort_flag) atomicOr(P.status, 1);
 }
 
-// merges the partial results of every (batch, query head, query): one group of D/8 threads per row.
-// The index's slot bits (one word per 32 slots of a query, shared by its heads) say which slots the query has: the
-// partial rows and statistics of the others were never written and are not read, so neither needs clearing (clearing
-// the statistics took 22 us at 17.8 M slots).  Loads are issued eight slots at a time with nothing depending on them
-// in between: the kernel is a stream over the partial buffer.
+// Merges the partial results of head g of the group (batch, KV head) bh at query i: acc[8] of a thread's 16-byte piece
+// (unnormalised), the reference maximum and the sum.  The D/8 threads of a row (neighbouring lanes) share the work on the
+// slots: each looks up the position and the statistics of every D/8-th one, and hands them on by shuffles; the rows' loads
+// are issued eight at a time with nothing depending on them in between, the kernel is a stream over the partial buffer.
+// The index's slot bits (one word per 32 slots of a query, shared by its heads) say which slots the query has.
 template <int D>
-__global__ void __launch_bounds__(256) sel_merge_kernel(const SelParams P) {
-  constexpr int TPR = D / 8;
-  const int64_t row = ((int64_t)blockIdx.x * 256 + threadIdx.x) / TPR;
-  const int part = threadIdx.x % TPR;
-  const int64_t nrows = (int64_t)P.B * P.Hq * P.N;
-  if (row >= nrows) return;
-  const int i = (int)(row % P.N);
-  const int hq = (int)((row / P.N) % P.Hq);
-  const int b = (int)(row / ((int64_t)P.N * P.Hq));
+__device__ __forceinline__ void merge_row(const SelParams& P, int bh, int i, int g, int part, float (&acc)[8], float* M_out, float* L_out) {
+  constexpr int TPR = D / 8, PER = 32 / TPR;
+  const unsigned mask = (TPR == 8 ? 0xffu : 0xffffu) << (threadIdx.x & 31 & ~(TPR - 1));
   const int ns = P.ns;
-  const float2* st = P.stats + row * ns;
-  const uint32_t* bits = P.bits + ((int64_t)(b * P.Hkv + hq / P.G) * P.N + i) * P.words;
-  const __nv_bfloat16* prow = P.partial + row * ns * D + part * 8;
-  float M = -INFINITY;
-  for (int s0 = 0; s0 < ns; s0 += 8) {
-    const uint32_t has = bits[s0 >> 5] >> (s0 & 31);
+  const int64_t query = (int64_t)bh * P.N + i;
+  const uint32_t* bits = P.bits + query * P.words;
+  const int* positions = P.positions + query * ns;
+  float M = -INFINITY, L = 0.f;
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
-      if (has >> u & 1u) M = fmaxf(M, st[s0 + u].x);
-  }
-  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  float L = 0.f;
-  for (int s0 = 0; s0 < ns; s0 += 8) {
-    const uint32_t has = bits[s0 >> 5] >> (s0 & 31);
-    float w[8];
-    uint4 v[8];
+  for (int x = 0; x < 8; ++x) acc[x] = 0.f;
+  for (int s0 = 0; s0 < ns; s0 += 32) {
+    const uint32_t has = bits[s0 >> 5] >> part;
+    int pos[PER];
+    float w[PER], lsum = 0.f, m = -INFINITY;
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const bool ok = has >> u & 1u;
-      const float2 ml = ok ? st[s0 + u] : make_float2(0.f, 0.f);
-      w[u] = ok ? ex2(ml.x - M) : 0.f;
-      L = fmaf(w[u], ml.y, L);
-      v[u] = ok ? *reinterpret_cast<const uint4*>(prow + (int64_t)(s0 + u) * D) : make_uint4(0u, 0u, 0u, 0u);
+    for (int k = 0; k < PER; ++k) pos[k] = has >> (k * TPR) & 1u ? positions[s0 + k * TPR + part] : -1;
+    float2 st[PER];
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+      st[k] = pos[k] >= 0 ? P.stats[(int64_t)pos[k] * P.G + g] : make_float2(-INFINITY, 0.f);
+      m = fmaxf(m, st[k].x);
     }
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const uint32_t q[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+    for (int o = TPR / 2; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(mask, m, o));
+    if (m == -INFINITY) continue;          // (the same for all threads of the row)
+    const float top = fmaxf(M, m), keep = ex2(M - top);
 #pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        acc[2 * x] = fmaf(w[u], __uint_as_float(q[x] << 16), acc[2 * x]);
-        acc[2 * x + 1] = fmaf(w[u], __uint_as_float(q[x] & 0xffff0000u), acc[2 * x + 1]);
+    for (int k = 0; k < PER; ++k) {
+      w[k] = ex2(st[k].x - top);
+      lsum = fmaf(w[k], st[k].y, lsum);
+    }
+#pragma unroll
+    for (int o = TPR / 2; o > 0; o >>= 1) lsum += __shfl_xor_sync(mask, lsum, o);
+    L = fmaf(L, keep, lsum);
+    M = top;
+#pragma unroll
+    for (int x = 0; x < 8; ++x) acc[x] *= keep;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+#pragma unroll
+      for (int u0 = 0; u0 < TPR; u0 += 8) {
+        if (s0 + k * TPR + u0 >= ns) break;
+        uint4 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int p = __shfl_sync(mask, pos[k], u0 + u, TPR);
+          v[u] = p >= 0 ? *partial_piece<D>(P.partial, (int64_t)p * P.G + g, part) : make_uint4(0u, 0u, 0u, 0u);
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const float wu = __shfl_sync(mask, w[k], u0 + u, TPR);
+          const uint32_t q[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            acc[2 * x] = fmaf(wu, __uint_as_float(q[x] << 16), acc[2 * x]);
+            acc[2 * x + 1] = fmaf(wu, __uint_as_float(q[x] & 0xffff0000u), acc[2 * x + 1]);
+          }
+        }
       }
     }
   }
+  *M_out = M;
+  *L_out = L;
+}
+
+// One group of D/8 threads per row; the heads of a group, whose partial rows are neighbours, next to each other.  Four
+// blocks per SM (64 registers): 17 slots of 1 M rows of 64 take 520 us = 0.73 of the copy bandwidth; left to the compiler
+// (78 registers, three blocks) 600 us, at 40 registers the loads no longer stay in flight together, 583 us.
+template <int D>
+__global__ void __launch_bounds__(256, 4) sel_merge_kernel(const SelParams P) {
+  constexpr int TPR = D / 8;
+  const int64_t t = ((int64_t)blockIdx.x * 256 + threadIdx.x) / TPR;
+  const int part = threadIdx.x % TPR;
+  if (t >= (int64_t)P.B * P.Hq * P.N || foreign_index(P)) return;
+  const int g = (int)(t % P.G), i = (int)((t / P.G) % P.N), bh = (int)(t / ((int64_t)P.G * P.N));
+  const int b = bh / P.Hkv, hq = (bh - b * P.Hkv) * P.G + g;
+  float acc[8], M, L;
+  merge_row<D>(P, bh, i, g, part, acc, &M, &L);
   const float inv = L > 0.f ? 1.f / L : 0.f;
   uint4 o;
   o.x = pack_bf16(acc[0] * inv, acc[1] * inv);
@@ -597,7 +636,7 @@ __global__ void __launch_bounds__(256) sel_merge_kernel(const SelParams P) {
   o.z = pack_bf16(acc[4] * inv, acc[5] * inv);
   o.w = pack_bf16(acc[6] * inv, acc[7] * inv);
   *reinterpret_cast<uint4*>(P.out + b * P.o_sb + (int64_t)hq * P.o_sh + (int64_t)i * P.o_sn + part * 8) = o;
-  if (part == 0) P.lse[row] = L > 0.f ? (M + log2f(L)) * kLn2 : -INFINITY;
+  if (part == 0) P.lse[((int64_t)b * P.Hq + hq) * P.N + i] = L > 0.f ? (M + log2f(L)) * kLn2 : -INFINITY;
 }
 
 // The merge of the selected branch that also does the gated combine and the head merge (and, with several
@@ -607,51 +646,18 @@ __global__ void __launch_bounds__(256) sel_merge_kernel(const SelParams P) {
 // branch's own output tensor is not written.  Thread groups walk the rows position-major (b, i, head), so that the
 // heads of one position land next to each other in the destinations' [B, N, features] rows.
 template <int D, bool MC>
-__global__ void __launch_bounds__(256) sel_merge_combine_kernel(const SelParams P, const CombineParams Cp, const GatherTargets Gt) {
+__global__ void __launch_bounds__(256, 4) sel_merge_combine_kernel(const SelParams P, const CombineParams Cp, const GatherTargets Gt) {
   constexpr int TPR = D / 8;
   const int64_t t = ((int64_t)blockIdx.x * 256 + threadIdx.x) / TPR;
   const int part = threadIdx.x % TPR;
   const int64_t nrows = (int64_t)P.B * P.Hq * P.N;
-  if (t < nrows) {
+  if (t < nrows && !foreign_index(P)) {
     const int hq = (int)(t % P.Hq);
     const int i = (int)((t / P.Hq) % P.N);
     const int b = (int)(t / ((int64_t)P.N * P.Hq));
     const int64_t row = ((int64_t)b * P.Hq + hq) * P.N + i;
-    const int ns = P.ns;
-    const float2* st = P.stats + row * ns;
-    const uint32_t* bits = P.bits + ((int64_t)(b * P.Hkv + hq / P.G) * P.N + i) * P.words;
-    const __nv_bfloat16* prow = P.partial + row * ns * D + part * 8;
-    float M = -INFINITY;
-    for (int s0 = 0; s0 < ns; s0 += 8) {
-      const uint32_t has = bits[s0 >> 5] >> (s0 & 31);
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-        if (has >> u & 1u) M = fmaxf(M, st[s0 + u].x);
-    }
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    float Lsum = 0.f;
-    for (int s0 = 0; s0 < ns; s0 += 8) {
-      const uint32_t has = bits[s0 >> 5] >> (s0 & 31);
-      float w[8];
-      uint4 v[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const bool ok = has >> u & 1u;
-        const float2 ml = ok ? st[s0 + u] : make_float2(0.f, 0.f);
-        w[u] = ok ? ex2(ml.x - M) : 0.f;
-        Lsum = fmaf(w[u], ml.y, Lsum);
-        v[u] = ok ? *reinterpret_cast<const uint4*>(prow + (int64_t)(s0 + u) * D) : make_uint4(0u, 0u, 0u, 0u);
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const uint32_t q[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
-#pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          acc[2 * x] = fmaf(w[u], __uint_as_float(q[x] << 16), acc[2 * x]);
-          acc[2 * x + 1] = fmaf(w[u], __uint_as_float(q[x] & 0xffff0000u), acc[2 * x + 1]);
-        }
-      }
-    }
+    float acc[8], M, Lsum;
+    merge_row<D>(P, b * P.Hkv + hq / P.G, i, hq % P.G, part, acc, &M, &Lsum);
     const float inv = Lsum > 0.f ? 1.f / Lsum : 0.f;
     if (part == 0 && P.lse != nullptr) P.lse[row] = Lsum > 0.f ? (M + log2f(Lsum)) * kLn2 : -INFINITY;
     // combine: gates in the order compressed, selected, sliding
@@ -1783,7 +1789,7 @@ static SelPlan make_plan(const SelProblem& a, bool backward) {
   p.off_status = off; off += 256;
   p.off_num_items = p.off_status + 128;
   if (!backward && dense_forward(a)) {   // only the status word is needed
-    p.off_totals = p.off_list_base = p.off_list_item = p.off_cursors = p.off_bits = p.off_items = p.off_entries = off;
+    p.off_totals = p.off_list_base = p.off_list_item = p.off_cursors = p.off_bits = p.off_items = p.off_entries = p.off_positions = off;
     p.off_partial = p.off_stats = p.off_delta = off;
     p.index_bytes = 0;
     p.total_bytes = off;
@@ -1796,13 +1802,15 @@ static SelPlan make_plan(const SelProblem& a, bool backward) {
   p.off_bits = off; off = align_up(off + (int64_t)a.B * a.Hkv * a.N * p.words * 4, 256);
   p.off_items = off; off = align_up(off + p.items_cap * 16, 256);
   p.off_entries = off; off = align_up(off + p.entries_cap * 4, 256);
-  p.index_bytes = off;   // status word, totals, list bases, slot bits, items, entries: the same layout forward and backward
+  p.off_positions = off;
+  if (a.mode == kModeSel) off = align_up(off + (int64_t)a.B * a.Hkv * a.N * p.ns * 4, 256);
+  p.index_bytes = off;   // status word to positions: the same layout forward and backward
   const int64_t rows = (int64_t)a.B * a.Hq * a.N;
   p.off_partial = p.off_stats = p.off_delta = off;
   p.slices = p.pairs_per_slice = 1;
   if (!backward) {
-    p.off_partial = off; off = align_up(off + rows * p.ns * a.D * 2, 256);
-    p.off_stats = off; off = align_up(off + rows * p.ns * 8, 256);
+    p.off_partial = off; off = align_up(off + p.entries_cap * p.G * a.D * 2, 256);
+    p.off_stats = off; off = align_up(off + p.entries_cap * p.G * 8, 256);
   } else {
     // very long inputs (64 heads of 128 at 65536 positions: 70 GB for the compressed branch) run in slices of whole
     // (batch, KV head) pairs that share a buffer of at most kPartialBudget, or of one pair
@@ -1899,6 +1907,7 @@ static int build_index(const SelProblem& a, const SelPlan& p, uint8_t* ix, cudaS
   int* num_items = reinterpret_cast<int*>(ix + p.off_num_items);
   uint32_t* entries = reinterpret_cast<uint32_t*>(ix + p.off_entries);
   int* list_item = reinterpret_cast<int*>(ix + p.off_list_item);
+  int* positions = reinterpret_cast<int*>(ix + p.off_positions);
   const BlockRule R = make_rule(a, p);
   const dim3 grid((a.N + kIndexQueries - 1) / kIndexQueries, a.B, a.Hkv);
   const size_t hist_smem = (size_t)p.nkb * sizeof(int);   // at most 32 KB
@@ -1907,9 +1916,9 @@ static int build_index(const SelProblem& a, const SelPlan& p, uint8_t* ix, cudaS
   else if (a.mode == kModeSwa) sel_count_kernel<kModeSwa><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, bits, p.words);
   else sel_count_kernel<kModeCmp><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, bits, p.words);
   sel_items_kernel<<<1, 1024, 0, st>>>(totals, list_base, list_item, cursors, items, num_items, p.nlists, p.QT, index_tag(a, p));
-  if (a.mode == kModeSel) sel_fill_kernel<kModeSel><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, list_base, cursors, entries, p.QT);
-  else if (a.mode == kModeSwa) sel_fill_kernel<kModeSwa><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, list_base, cursors, entries, p.QT);
-  else sel_fill_kernel<kModeCmp><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, list_base, cursors, entries, p.QT);
+  if (a.mode == kModeSel) sel_fill_kernel<kModeSel><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, list_base, cursors, entries, positions, p.QT);
+  else if (a.mode == kModeSwa) sel_fill_kernel<kModeSwa><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, list_base, cursors, entries, positions, p.QT);
+  else sel_fill_kernel<kModeCmp><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, list_base, cursors, entries, positions, p.QT);
   CUDA_TRY(cudaGetLastError());
   count_launches(4);   // clear, count, items, fill
   return NSA_OK;
@@ -1949,6 +1958,7 @@ static void fill_params(SelParams& P, const SelProblem& a, const SelPlan& p, uin
   P.index_tag = index_tag(a, p);
   P.bits = reinterpret_cast<const uint32_t*>(ix + p.off_bits);
   P.list_item = reinterpret_cast<const int*>(ix + p.off_list_item);
+  P.positions = reinterpret_cast<const int*>(ix + p.off_positions);
   P.bh0 = 0; P.bh1 = a.B * a.Hkv;
   P.words = p.words;
   P.status = a.status != nullptr ? a.status : reinterpret_cast<int*>(ws + p.off_status);
@@ -2024,7 +2034,7 @@ static int run_fwd(const SelProblem& a, const SelPlan& p, uint8_t* ws, cudaStrea
   P.partial = reinterpret_cast<__nv_bfloat16*>(ws + p.off_partial);
   P.stats = reinterpret_cast<float2*>(ws + p.off_stats);
   constexpr int NC = D / 64;
-  const int smem = 1024 + NC * (16384 + 8192 + 8192) + kRows * (D * 2 + 16);
+  const int smem = 1024 + NC * (16384 + 8192 + 8192 + 16384);
   const int per_sm = D == 64 ? 4 : 2;
   CUDA_TRY(cudaFuncSetAttribute(sel_fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   sel_fwd_kernel<D><<<num_sms() * per_sm, 2 * kRows, smem, st>>>(tmK, tmV, P);
@@ -2282,7 +2292,7 @@ int sm100_cmp_bwd(const nsa_cmp_bwd_args& b, cudaStream_t st) {
 // memory pool is closed to extensions, an embedder that forbids cudaMalloc after start-up).  For
 // them the forward pass can run on a fixed scratch area that is part of the library image.  Every
 // device that loads the library reserves kStaticScratchBytes for it until the process ends.
-constexpr int64_t kStaticScratchBytes = 32ll << 20;
+constexpr int64_t kStaticScratchBytes = 96ll << 20;   // (32 MB of partial rows and, at most, twice that of padding to whole chunks)
 static __device__ __align__(256) unsigned char g_sel_scratch[kStaticScratchBytes];
 
 // Filled on first use per device without a lock: every thread that races here stores the same address.
