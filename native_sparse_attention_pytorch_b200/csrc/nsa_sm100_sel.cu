@@ -17,7 +17,7 @@
 //   backward: S = Q K^T and dP = dO V^T -> P = exp(S - lse), dS = P (dP - delta)
 //             -> dV += P^T dO and dK += dS^T Q stay in tensor memory across the
 //             chunks of the item (flushed once with fp32 reductions), and
-//             dQ_chunk = dS K goes out as a bf16 partial per (row, slot) that a
+//             dQ_chunk = dS K goes out as a partial per (row, slot) that a
 //             last kernel sums into dq.
 //
 // All operand tiles are [rows x 64 columns] bf16 with 128-byte rows and the
@@ -1188,7 +1188,7 @@ __global__ void __launch_bounds__(256) sel_delta_kernel(const SelParams P, float
 // different chunks overlap instead of taking turns:
 //   warps 0-7, 8-15  two softmax groups; chunk n (counted per CTA) belongs to group n % 2.  Two threads share a row (32
 //                    of the block's 64 columns each): they read S and dP from tensor memory, write P and dS (bf16) for
-//                    the second set of MMAs and then store the dQ row as a bf16 partial result (summed by
+//                    the second set of MMAs and then store the dQ row as a partial result (summed by
 //                    sel_dq_merge_kernel).  The group of an item's last chunk flushes its dK / dV with fp32 reductions.
 //   warp 16, 17      issue the tcgen05.mma: S / dP, which run a chunk ahead, and dV, dQ, dK.  Two of them, because an MMA
 //                    is accepted when the one before it starts: the waits and addresses in between leave the tensor
@@ -1225,8 +1225,10 @@ struct Shape {
   static constexpr uint32_t tGroup = 128, tDP = 64, tAcc = 256, tDQ = tAcc + D;   // tensor-memory columns
 };
 constexpr uint32_t kLaneDK = 16u << 16;     // dK: lanes 16-31 of every quarter
-constexpr int kDqCols = 32;                 // dQ read-out: columns a warp stages at a time, in the P tile of its group
-constexpr uint32_t kDqRow = kDqCols * 2, kDqStage = 32 * kDqRow;
+// dQ partials: bf16 at dim_head 64; fp32 at 128, where dq has always been summed from fp32 terms
+template <int D>
+constexpr int kDqElem = D == 64 ? 2 : 4;
+constexpr uint32_t kDqRow = 64, kDqStage = 32 * kDqRow;   // read-out: bytes of a row that a warp stages at a time, in the P tile
 
 struct Bars {
   uint64_t q_full[3], q_free[3];
@@ -1331,22 +1333,28 @@ sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
       tc_fence_after_sync();
       __syncwarp();
       uint8_t* const pbase = reinterpret_cast<uint8_t*>(P.partial);
+      constexpr int kCols = (int)kDqRow / kDqElem<D>, kPieces = D / 2 / kCols;   // columns per piece, pieces per half row
 #pragma unroll 1
-      for (int piece = 0; piece < NC; ++piece) {
-        const int col = (half * NC + piece) * kDqCols;
+      for (int piece = 0; piece < kPieces; ++piece) {
+        const int col = (half * kPieces + piece) * kCols;
         {
-          float tq[kDqCols];
-          tmem_ld32(tm_quarter + S::tDQ + (S::kDq == 2 ? wg * D : 0) + col, tq);
+          float tq[kCols];
+          if constexpr (kCols == 32) tmem_ld32(tm_quarter + S::tDQ + (S::kDq == 2 ? wg * D : 0) + col, tq);
+          else tmem_ld16(tm_quarter + S::tDQ + (S::kDq == 2 ? wg * D : 0) + col, tq);
           tmem_ld_wait();
 #pragma unroll
           for (int x = 0; x < 4; ++x) {
             uint4 v;
-            v.x = pack_bf16(tq[x * 8 + 0], tq[x * 8 + 1]); v.y = pack_bf16(tq[x * 8 + 2], tq[x * 8 + 3]);
-            v.z = pack_bf16(tq[x * 8 + 4], tq[x * 8 + 5]); v.w = pack_bf16(tq[x * 8 + 6], tq[x * 8 + 7]);
+            if constexpr (kCols == 32) {
+              v.x = pack_bf16(tq[x * 8 + 0], tq[x * 8 + 1]); v.y = pack_bf16(tq[x * 8 + 2], tq[x * 8 + 3]);
+              v.z = pack_bf16(tq[x * 8 + 4], tq[x * 8 + 5]); v.w = pack_bf16(tq[x * 8 + 6], tq[x * 8 + 7]);
+            } else {
+              v = make_uint4(__float_as_uint(tq[x * 4]), __float_as_uint(tq[x * 4 + 1]), __float_as_uint(tq[x * 4 + 2]), __float_as_uint(tq[x * 4 + 3]));
+            }
             sts_v4(sDq + lane * kDqRow + ((x ^ ((lane >> 1) & 3)) << 4), v);   // conflict-free to write and to read
           }
         }
-        if (S::kDq == 1 && piece == NC - 1) {
+        if (S::kDq == 1 && piece == kPieces - 1) {
           tc_fence_before_sync();
           mbar_arrive(smem_u32(&bars.dq_free));   // the other group's dQ may overwrite the columns
         }
@@ -1356,7 +1364,7 @@ sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
           const int rr = k * 8 + (lane >> 2);
           const int dst = __shfl_sync(kFullMask, dst_row, rr);
           const uint4 v = lds_v4(sDq + rr * kDqRow + (((lane & 3) ^ ((rr >> 1) & 3)) << 4));
-          if (dst >= 0) *reinterpret_cast<uint4*>(pbase + (int64_t)dst * (D * 2) + col * 2 + (lane & 3) * 16) = v;
+          if (dst >= 0) *reinterpret_cast<uint4*>(pbase + ((int64_t)dst * D + col) * kDqElem<D> + (lane & 3) * 16) = v;
         }
         __syncwarp();
       }
@@ -1628,7 +1636,7 @@ sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 }
 
 
-// sums the bf16 dQ partials of every (batch, query head, query) into the fp32 dq row: D/8 threads per row
+// sums the dQ partials of every (batch, query head, query) into the fp32 dq row: D/8 threads per row
 template <int D, int MODE>
 __global__ void __launch_bounds__(256) sel_dq_merge_kernel(const SelParams P) {
   constexpr int TPR = D / 8;
@@ -1643,31 +1651,40 @@ __global__ void __launch_bounds__(256) sel_dq_merge_kernel(const SelParams P) {
   const int h = hq / P.G;
   const int ns = P.ns;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  const __nv_bfloat16* prow = P.partial + part_row * ns * D + part * 8;
-  // eight slots at a time: first which of them the query has, then their loads together, then the sums
+  constexpr int BYTES = ws::kDqElem<D>, BATCH = BYTES == 2 ? 8 : 4, QUADS = BYTES / 2;
+  const uint8_t* prow = reinterpret_cast<const uint8_t*>(P.partial) + (part_row * ns * D + part * 8) * BYTES;
+  // some slots at a time: first which of them the query has, then their loads together, then the sums
   const uint32_t* bits = P.bits + ((int64_t)(b * P.Hkv + h) * P.N + i) * P.words;
-  for (int s0 = 0; s0 < ns; s0 += 8) {
+  for (int s0 = 0; s0 < ns; s0 += BATCH) {
     const uint32_t has = MODE == kModeSel ? bits[s0 >> 5] >> (s0 & 31) : 0u;
-    bool ok[8];
-    uint4 v[8];
+    bool ok[BATCH];
+    uint4 v[BATCH][QUADS];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
+    for (int u = 0; u < BATCH; ++u) {
       int blk_;
       ok[u] = MODE == kModeSel ? (has >> u & 1u) != 0
                                : s0 + u < ns && slot_block<MODE>(P.rule, b * P.Hkv + h, i, s0 + u, &blk_);
     }
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
-      v[u] = ok[u] ? *reinterpret_cast<const uint4*>(prow + (int64_t)(s0 + u) * D) : make_uint4(0u, 0u, 0u, 0u);
+    for (int u = 0; u < BATCH; ++u)
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const uint32_t q[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+      for (int w = 0; w < QUADS; ++w)
+        v[u][w] = ok[u] ? reinterpret_cast<const uint4*>(prow + (int64_t)(s0 + u) * (D * BYTES))[w] : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        acc[2 * x] += __uint_as_float(q[x] << 16);
-        acc[2 * x + 1] += __uint_as_float(q[x] & 0xffff0000u);
+    for (int u = 0; u < BATCH; ++u)
+#pragma unroll
+      for (int w = 0; w < QUADS; ++w) {
+        const uint32_t q[4] = {v[u][w].x, v[u][w].y, v[u][w].z, v[u][w].w};
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          if constexpr (BYTES == 2) {
+            acc[2 * x] += __uint_as_float(q[x] << 16);
+            acc[2 * x + 1] += __uint_as_float(q[x] & 0xffff0000u);
+          } else {
+            acc[4 * w + x] += __uint_as_float(q[x]);
+          }
+        }
       }
-    }
   }
   // the partials hold dS K without the logit scale
   if (P.dq_lp != nullptr) {   // the caller asked for dq in the dtype and row layout of q
@@ -1816,7 +1833,7 @@ static SelPlan make_plan(const SelProblem& a, bool backward) {
     // (batch, KV head) pairs that share a buffer of at most kPartialBudget, or of one pair
     p.off_delta = off; off = align_up(off + rows * 4, 256);
     const int pairs = a.B * a.Hkv;
-    const int64_t per_pair = (int64_t)p.G * a.N * p.ns * a.D * 2, most = kPartialBudget / per_pair;
+    const int64_t per_pair = (int64_t)p.G * a.N * p.ns * a.D * (a.D == 64 ? 2 : 4), most = kPartialBudget / per_pair;
     const int per_slice = (int)(most < 1 ? 1 : most < pairs ? most : pairs);
     p.slices = (pairs + per_slice - 1) / per_slice;
     p.pairs_per_slice = (pairs + p.slices - 1) / p.slices;
