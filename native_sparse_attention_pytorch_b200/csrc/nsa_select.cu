@@ -109,62 +109,150 @@ __device__ __forceinline__ float from_ordered_bits(unsigned k) {
   return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
+// The k picks of a row of many columns without ordering all of it, for probabilities that are rounded to bf16.  The k-th
+// largest of the 32 lanes' maxima bounds the k-th largest logit from below, so the picks are among the entries above it;
+// rounding can put an entry level with one whose logit is less than 2^-7 higher (the column then decides), which the margin
+// covers.  Some 30 to 50 entries of a row pass: only they are divided by the sum and ranked.  Returns false, having
+// written nothing, where the bound does not hold or help (fewer than k lanes with entries, probabilities so small that
+// the spacing of bf16 is no longer relative, or a crowd of equal logits).
+// A row of 1024 columns took 2000 instructions with every entry divided, sorted and drawn one by one; 8 heads of 65536
+// rows 3.2 ms, now 1.3 ms (with the loads of a row side by side).
+constexpr int kCandidates = 96;
+template <int CPL>
+__device__ __forceinline__ bool select_from_the_top(const SelectParams& P, int64_t task, int lane, const float (&v)[CPL], unsigned alive,
+                                                    float lane_max, float mx, float z, float* cand_v, unsigned* cand) {
+  const unsigned head = alive != 0 ? ordered_bits(lane_max) >> 16 : 0u;
+  unsigned bound = 0;
+#pragma unroll
+  for (int bit = 15; bit >= 0; --bit) {
+    const unsigned trial = bound | (1u << bit);
+    if (__popc(__ballot_sync(kFullMask, head >= trial)) >= P.k) bound = trial;
+  }
+  const float floor_v = from_ordered_bits(bound << 16);
+  if (bound == 0u || !(expf(floor_v - mx) / z > 1e-30f)) return false;
+  const float from = floor_v - 0.016f;
+  int n = 0;
+#pragma unroll
+  for (int t = 0; t < CPL; ++t) {
+    const bool in = (alive >> t & 1) && v[t] >= from;
+    const unsigned who = __ballot_sync(kFullMask, in);
+    const int at = n + __popc(who & ((1u << lane) - 1u));
+    if (in && at < kCandidates) {
+      cand_v[at] = v[t];
+      cand[at] = (unsigned)(lane + 32 * t);
+    }
+    n += __popc(who);
+  }
+  if (n > kCandidates || n < P.k) return false;   // (fewer: lanes whose maximum is the sink)
+  __syncwarp();
+  // value and column in one word: the probability's 16 significant bits, then the lower column first
+  unsigned key[kCandidates / 32];
+#pragma unroll
+  for (int q = 0; q < kCandidates / 32; ++q) {
+    key[q] = 0u;
+    const int c = lane + 32 * q;
+    if (c < n) key[q] = (ordered_bits(round_bf16(expf(cand_v[c] - mx) / z)) & 0xffff0000u) | (1023u - cand[c]);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < kCandidates / 32; ++q) cand[lane + 32 * q] = key[q];
+  __syncwarp();
+  int rank[kCandidates / 32] = {};
+  for (int e = 0; e < n; e += 4) {           // (the places behind the n-th hold 0)
+    const uint4 o = *reinterpret_cast<const uint4*>(cand + e);
+#pragma unroll
+    for (int q = 0; q < kCandidates / 32; ++q)
+      rank[q] += (o.x > key[q]) + (o.y > key[q]) + (o.z > key[q]) + (o.w > key[q]);
+  }
+#pragma unroll
+  for (int q = 0; q < kCandidates / 32; ++q) {
+    if (key[q] != 0u && rank[q] < P.k) {
+      const int64_t at = task * P.k + rank[q];
+      const float val = from_ordered_bits((key[q] & 0xffff0000u) | ((key[q] & 0x80000000u) ? 0u : 0xffffu));
+      P.idx[at] = (int64_t)(1023u - (key[q] & 1023u));
+      if (P.vals != nullptr) P.vals[at] = val;
+      if (P.mask != nullptr) P.mask[at] = val > mask_threshold(P);
+    }
+  }
+  return true;
+}
+
 // `limit`: columns at and past it are not read, they hold probability 0 (causal_limit); `need`: columns that can
 // appear among the k picks (all of them, or with a limit the first limit + k: zeros are picked in column order).
 template <int CPL>
-__device__ __forceinline__ void select_row(const SelectParams& P, int64_t task, int i, int lane, int limit, int need) {
+__device__ __forceinline__ void select_row(const SelectParams& P, int64_t task, int i, int lane, int limit, int need, float* cand_v,
+                                           unsigned* cand) {
   const float* src = P.imp + task * P.ncb;
   const __nv_bfloat16* psrc = static_cast<const __nv_bfloat16*>(P.pooled) + task * P.ncb;
   const bool vec4 = P.cpf == 4 && (P.ncb & 3) == 0 && (reinterpret_cast<uintptr_t>(P.imp) & 15u) == 0;
   float v[CPL];
+  // The loads of a row stand together and without branches (columns past the limit read the last one before it): in
+  // branches of their own each waited for the one before, 25000 cycles per row of 1024 columns
+  const int last = max(limit, 1) - 1;
+  if (P.pooled != nullptr) {
+    __nv_bfloat16 raw[CPL];
+#pragma unroll
+    for (int t = 0; t < CPL; ++t) raw[t] = psrc[min(lane + 32 * t, last)];
+#pragma unroll
+    for (int t = 0; t < CPL; ++t) v[t] = __bfloat162float(raw[t]);
+  } else if (P.cpf == 1) {
+#pragma unroll
+    for (int t = 0; t < CPL; ++t) v[t] = src[min(lane + 32 * t, last)];
+  } else {
+    const float cpf = (float)P.cpf;
+    if (vec4) {
+#pragma unroll
+      for (int t0 = 0; t0 < CPL; t0 += 4) {
+        float4 q[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (t0 + u < CPL) q[u] = *reinterpret_cast<const float4*>(src + min(lane + 32 * (t0 + u), last) * 4);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (t0 + u < CPL) v[t0 + u] = (((0.f + q[u].x) + q[u].y) + q[u].z + q[u].w) / cpf;
+      }
+    } else {
+#pragma unroll
+      for (int t = 0; t < CPL; ++t) {
+        const float* at = src + min(lane + 32 * t, last) * P.cpf;
+        float sum = 0.f;
+        for (int c = 0; c < P.cpf; ++c) sum += at[c];
+        v[t] = sum / cpf;
+      }
+    }
+    if (P.round_bf16) {
+#pragma unroll
+      for (int t = 0; t < CPL; ++t) v[t] = round_bf16(v[t]);
+    }
+  }
   unsigned alive = 0;
+  const int own = !P.input_is_prob && P.exclude_own ? i / P.block : -1;
 #pragma unroll
   for (int t = 0; t < CPL; ++t) {
     const int j = lane + 32 * t;
-    v[t] = 0.f;
-    if (j < need) {
-      alive |= 1u << t;
-      float x;
-      if (j >= limit) {
-        x = P.neg_max;
-      } else if (P.pooled != nullptr) {
-        x = __bfloat162float(psrc[j]);
-      } else if (P.cpf == 1) {
-        x = src[j];
-      } else {
-        float sum = 0.f;
-        if (vec4) {
-          const float4 q = *reinterpret_cast<const float4*>(src + j * 4);
-          sum = ((sum + q.x) + q.y) + q.z + q.w;
-        } else {
-          for (int c = 0; c < P.cpf; ++c) sum += src[j * P.cpf + c];
-        }
-        x = sum / (float)P.cpf;
-        if (P.round_bf16) x = round_bf16(x);
-      }
-      if (!P.input_is_prob && P.exclude_own && j == i / P.block) x = P.neg_max;
-      v[t] = x;
-    }
+    if (j >= limit || j == own) v[t] = P.neg_max;
+    if (j < need) alive |= 1u << t;
+    else v[t] = 0.f;
   }
   if (!P.input_is_prob) {
     float mx = -1000.f;  // the sink logit
 #pragma unroll
     for (int t = 0; t < CPL; ++t)
       if (alive >> t & 1) mx = fmaxf(mx, v[t]);
+    const float lane_max = mx;
     mx = warp_max(mx);
     float part = 0.f;
 #pragma unroll
-    for (int t = 0; t < CPL; ++t) {
-      if (alive >> t & 1) {
-        v[t] = expf(v[t] - mx);
-        part += v[t];
-      }
-    }
+    for (int t = 0; t < CPL; ++t)
+      if (alive >> t & 1) part += expf(v[t] - mx);
     const float z = warp_sum(part) + expf(-1000.f - mx);
+    if constexpr (CPL >= 4) {   // (rows of up to 64 columns: ordering two entries per lane is less work than the search)
+      if (P.round_bf16 && select_from_the_top(P, task, lane, v, alive, lane_max, mx, z, cand_v, cand)) return;
+    }
 #pragma unroll
     for (int t = 0; t < CPL; ++t) {
       if (alive >> t & 1) {
-        float p = v[t] / z;
+        float p = expf(v[t] - mx) / z;
         if (P.round_bf16) p = round_bf16(p);
         v[t] = p;
       }
@@ -252,18 +340,20 @@ __device__ __forceinline__ void select_row(const SelectParams& P, int64_t task, 
 // limit the early queries of a sequence need few).
 template <int CPLMAX>
 __global__ void __launch_bounds__(128) select_reg_kernel(const SelectParams P) {
+  __shared__ float cand_v[4][kCandidates];
+  __shared__ __align__(16) unsigned cand[4][kCandidates];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t task = (int64_t)blockIdx.x * 4 + warp;
   if (task >= (int64_t)P.rows * P.seq) return;
   const int i = (int)(task % P.seq);
   const int limit = P.causal_limit ? min(P.cols, i / P.block) : P.cols;
   const int need = P.causal_limit ? min(P.cols, limit + P.k) : P.cols;
-  if (CPLMAX > 1 && need <= 32) select_row<1>(P, task, i, lane, limit, need);
-  else if (CPLMAX > 2 && need <= 64) select_row<2>(P, task, i, lane, limit, need);
-  else if (CPLMAX > 4 && need <= 128) select_row<4>(P, task, i, lane, limit, need);
-  else if (CPLMAX > 8 && need <= 256) select_row<8>(P, task, i, lane, limit, need);
-  else if (CPLMAX > 16 && need <= 512) select_row<16>(P, task, i, lane, limit, need);
-  else select_row<CPLMAX>(P, task, i, lane, limit, need);
+  if (CPLMAX > 1 && need <= 32) select_row<1>(P, task, i, lane, limit, need, cand_v[warp], cand[warp]);
+  else if (CPLMAX > 2 && need <= 64) select_row<2>(P, task, i, lane, limit, need, cand_v[warp], cand[warp]);
+  else if (CPLMAX > 4 && need <= 128) select_row<4>(P, task, i, lane, limit, need, cand_v[warp], cand[warp]);
+  else if (CPLMAX > 8 && need <= 256) select_row<8>(P, task, i, lane, limit, need, cand_v[warp], cand[warp]);
+  else if (CPLMAX > 16 && need <= 512) select_row<16>(P, task, i, lane, limit, need, cand_v[warp], cand[warp]);
+  else select_row<CPLMAX>(P, task, i, lane, limit, need, cand_v[warp], cand[warp]);
 }
 
 int launch_select(const SelectParams& P, cudaStream_t stream) {

@@ -444,3 +444,25 @@ def test_compress_windows_match_pad_unfold_add(dtype, block, stride):
     close(out, ref, 'windows')
     close(dx, gx, 'd x')
     assert_close_bf16(dp, gp, 'd positions', rel_to_max=5e-3) if dtype == torch.bfloat16 else close(dp, gp, 'd positions')
+
+
+@pytest.mark.parametrize('cols,k', [(96, 4), (129, 16), (512, 32), (1000, 16), (1024, 3)])
+def test_selection_of_crowded_and_lopsided_rows(cols, k):
+    # rows the search from the top has to leave to the full ordering (equal logits, one logit far above the rest, fewer
+    # lanes with entries than picks) next to ordinary ones, as probabilities rounded to bf16: the picks of the fp32 oracle
+    n = 64
+    imp = recipe.randn((1, 2, n, cols), 5).bfloat16().float()
+    imp[0, 0, 0:8] = 0.25                                   # all equal
+    imp[0, 0, 8:16, 7] = 120.                               # everything else has probability 0
+    imp[0, 0, 16:24] *= 0.01                                # many columns level after rounding
+    imp[0, 0, 24:32, ::2] = -300.
+    imp = imp.to(DEV)
+    vals, idx = nsa.select_blocks(imp, 16, 16, k, dtype=torch.bfloat16)
+    p = torch.cat((torch.full_like(imp[..., :1], -1000.), imp), dim=-1).softmax(dim=-1)[..., 1:].bfloat16().float()
+    got = p.gather(-1, idx)
+    want = p.sort(dim=-1, descending=True, stable=True)
+    # the device's exponential may round a probability to its neighbour: the picked probabilities agree to that
+    assert ((got - want.values[..., :k]).abs() <= 2.0 ** -7 * want.values[..., :k]).all()
+    assert torch.equal(vals.float(), vals.float().sort(dim=-1, descending=True).values)
+    assert (idx.sort(dim=-1).values.diff(dim=-1) > 0).all()
+    assert torch.equal(idx[0, 0, :16], want.indices[0, 0, :16, :k])
