@@ -289,8 +289,16 @@ static std::vector<OptTensor> layer_forward(Tensor x, std::vector<OptTensor> wei
       check(nsa::launch_select(p, st));
     }
   }
-  // selected branch
+  // sliding branch
+  {
+    nsa_swa_fwd_args a = L.swa_args(qr, kr, v, o + 2 * q_bytes, lse + 2 * L.rows(c.heads));
+    const Tensor ws = scratch(a, nsa_swa_workspace_bytes, 0, x);
+    check(nsa_swa_fwd(&a, st));
+  }
+  // selected branch and gated combine: one pass over the partial results where the kernels can (then the branch's own
+  // output is stored for the backward only), else one after the other
   Tensor index;
+  const Tensor merged = at::empty({BN, c.heads * d}, x.options());
   {
     nsa_sel_fwd_args a = L.sel_args(qr, kr, v, o + q_bytes, lse + L.rows(c.heads), L.k_sel > 0 ? idx : nullptr, L.k_sel > 0 ? mask : nullptr);
     const Tensor ws = scratch(a, nsa_sel_workspace_bytes, 0, x);
@@ -299,22 +307,19 @@ static std::vector<OptTensor> layer_forward(Tensor x, std::vector<OptTensor> wei
       a.index_out = index.data_ptr();
       a.index_out_bytes = index.numel();
     }
-    check(nsa_sel_fwd(&a, st));
-  }
-  // sliding branch
-  {
-    nsa_swa_fwd_args a = L.swa_args(qr, kr, v, o + 2 * q_bytes, lse + 2 * L.rows(c.heads));
-    const Tensor ws = scratch(a, nsa_swa_workspace_bytes, 0, x);
-    check(nsa_swa_fwd(&a, st));
-  }
-  // gated combine and output projection
-  const Tensor merged = at::empty({BN, c.heads * d}, x.options());
-  {
     const nsa::CombineParams p = L.combine_params(o, logits.data_ptr());
     nsa::GatherTargets t = {};
     t.outs[0] = merged.data_ptr(); t.num_outs = 1; t.total_features = c.heads * d;
-    check(nsa::launch_combine_gather(p, t, L.dt, st));
+    nsa_sel_fwd_args fused = a;
+    if (!save) fused.out = no_tensor();
+    int rc = ws.defined() ? nsa::sm100_sel_fwd_combine(fused, p, t, st) : NSA_ERR_UNSUPPORTED;
+    if (rc == NSA_ERR_UNSUPPORTED) {
+      check(nsa_sel_fwd(&a, st));
+      rc = nsa::launch_combine_gather(p, t, L.dt, st);
+    }
+    check(rc);
   }
+  // output projection
   const Tensor out = product(Op::NT, merged, w.out).view({B, N, L.dim});
 
   auto opt = [](const Tensor& t) { return t.defined() ? OptTensor(t) : OptTensor(); };

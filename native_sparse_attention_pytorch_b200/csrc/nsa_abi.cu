@@ -533,6 +533,7 @@ int nsa_sel_fwd_combine_gather(const nsa_sel_fwd_args* s, const nsa_combine_gath
   GatherTargets Gt;
   NSA_TRY(fill_gather(P, Gt, *c, 1));
   P.o[1] = nullptr;
+  sel.out.ptr = nullptr;   // not written by this entry point
   const int rc = sm100_sel_fwd_combine(sel, P, Gt, (cudaStream_t)stream);
   if (rc == NSA_ERR_UNSUPPORTED) return fail(NSA_ERR_UNSUPPORTED, "selected branch: shape outside the tensor-core family");
   return rc;

@@ -6,13 +6,6 @@
 
 namespace nsa {
 
-// A gate from the tensor it is read from: the gate itself, or the logit whose sigmoid it is (rounded to T)
-template <typename T>
-__device__ __forceinline__ float gate_value(T raw, int logits) {
-  const float x = Elem<T>::to_float(raw);
-  return logits ? Elem<T>::to_float(Elem<T>::from_float(1.f / (1.f + expf(-x)))) : x;
-}
-
 template <typename T>
 __global__ void __launch_bounds__(256) combine_fwd_kernel(const CombineParams P) {
   const int half = P.d / 2;

@@ -65,6 +65,13 @@ __device__ __forceinline__ float round_bf16(float v) {
   return __bfloat162float(__float2bfloat16_rn(v));
 }
 
+// A gate from the tensor it is read from: the gate itself, or the logit whose sigmoid it is (rounded to T)
+template <typename T>
+__device__ __forceinline__ float gate_value(T raw, int logits) {
+  const float x = Elem<T>::to_float(raw);
+  return logits ? Elem<T>::to_float(Elem<T>::from_float(1.f / (1.f + expf(-x)))) : x;
+}
+
 // Split a flat index over [d3][d2][d1][d0] (d0 fastest) into its four coordinates; with 32-bit arithmetic whenever
 // the index fits (64-bit divisions cost several times more instructions, and these kernels are otherwise a few
 // loads and stores per thread).

@@ -643,8 +643,8 @@ __global__ void __launch_bounds__(256, 4) sel_merge_kernel(const SelParams P) {
 // destinations, the all-gather of the head-sharded layout): the merged selected row is rounded to bf16 as the tensor
 // between the two kernels would be, combined with the compressed and the sliding row exactly as combine_gather_kernel
 // does (the same three fused multiply-adds in the same order), and stored into every destination.  The selected
-// branch's own output tensor is not written.  Thread groups walk the rows position-major (b, i, head), so that the
-// heads of one position land next to each other in the destinations' [B, N, features] rows.
+// branch's own output tensor is written where the caller wants it.  Thread groups walk the rows position-major
+// (b, i, head), so that the heads of one position land next to each other in the destinations' [B, N, features] rows.
 template <int D, bool MC>
 __global__ void __launch_bounds__(256, 4) sel_merge_combine_kernel(const SelParams P, const CombineParams Cp, const GatherTargets Gt) {
   constexpr int TPR = D / 8;
@@ -662,17 +662,17 @@ __global__ void __launch_bounds__(256, 4) sel_merge_combine_kernel(const SelPara
     if (part == 0 && P.lse != nullptr) P.lse[row] = Lsum > 0.f ? (M + log2f(Lsum)) * kLn2 : -INFINITY;
     // combine: gates in the order compressed, selected, sliding
     const __nv_bfloat16* g = (const __nv_bfloat16*)Cp.gates + b * Cp.g_sb + hq * Cp.g_sh + (int64_t)i * Cp.g_sn;
-    const float g0 = __bfloat162float(g[0]), g1 = __bfloat162float(g[1]), g2 = __bfloat162float(g[2]);
+    const float g0 = gate_value(g[0], Cp.logits), g1 = gate_value(g[1], Cp.logits), g2 = gate_value(g[2], Cp.logits);
     const uint4 rc = *reinterpret_cast<const uint4*>((const __nv_bfloat16*)Cp.o[0] + b * Cp.o_sb[0] + hq * Cp.o_sh[0] +
                                                      (int64_t)i * Cp.o_sn[0] + part * 8);
     const uint4 rw = *reinterpret_cast<const uint4*>((const __nv_bfloat16*)Cp.o[2] + b * Cp.o_sb[2] + hq * Cp.o_sh[2] +
                                                      (int64_t)i * Cp.o_sn[2] + part * 8);
     const uint32_t qc[4] = {rc.x, rc.y, rc.z, rc.w}, qw[4] = {rw.x, rw.y, rw.z, rw.w};
-    uint32_t packed[4];
+    uint32_t packed[4], sel[4];
 #pragma unroll
     for (int x = 0; x < 4; ++x) {
-      // the selected row as its bf16 tensor would hold it
-      const uint32_t os = pack_bf16(acc[2 * x] * inv, acc[2 * x + 1] * inv);
+      // the selected row as its bf16 tensor holds it
+      const uint32_t os = sel[x] = pack_bf16(acc[2 * x] * inv, acc[2 * x + 1] * inv);
       float lo = fmaf(g0, __uint_as_float(qc[x] << 16), 0.f);
       float hi = fmaf(g0, __uint_as_float(qc[x] & 0xffff0000u), 0.f);
       lo = fmaf(g1, __uint_as_float(os << 16), lo);
@@ -681,6 +681,8 @@ __global__ void __launch_bounds__(256, 4) sel_merge_combine_kernel(const SelPara
       hi = fmaf(g2, __uint_as_float(qw[x] & 0xffff0000u), hi);
       packed[x] = pack_bf16(lo, hi);
     }
+    if (P.out != nullptr)
+      *reinterpret_cast<uint4*>(P.out + b * P.o_sb + (int64_t)hq * P.o_sh + (int64_t)i * P.o_sn + part * 8) = make_uint4(sel[0], sel[1], sel[2], sel[3]);
     const int64_t at = ((int64_t)b * P.N + i) * Gt.total_features + Gt.feature_offset + (int64_t)hq * D + part * 8;
     if (MC) {
       asm volatile("multimem.st.weak.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"((__nv_bfloat16*)Gt.outs[0] + at),
@@ -1743,7 +1745,7 @@ struct SelProblem {
   void* workspace;
   int64_t workspace_bytes;
   const CombineParams* fuse_combine;   // selected forward, optional: the merge also combines and stores (see
-  const GatherTargets* fuse_targets;   // sel_merge_combine_kernel); `out` is then not written
+  const GatherTargets* fuse_targets;   // sel_merge_combine_kernel); `out` may then be missing
   const void* index;       // an index kept from an earlier call, or NULL to build it
   int64_t index_bytes;
   void* index_out;         // optional: where to build it instead of the head of the work buffer
