@@ -499,7 +499,7 @@ def kernel_rows(breakdown, w, mask, f_fwd, f_bwd, tensor_peak):
     part = slots * (d * 2)                                            # bf16 partial rows
     rows_bytes = b * hq * n * d * 2
     work = {   # kernel name prefix -> (bound, algorithmic FLOPs or bytes per launch)
-        'sel_fwd_kernel': ('tensor', f_fwd), 'sel_bwd_ws_kernel': ('tensor', f_bwd), 'sel_bwd_kernel': ('tensor', f_bwd),
+        'sel_fwd_kernel': ('tensor', f_fwd), 'sel_bwd_ws_kernel': ('tensor', f_bwd),
         'sel_merge_kernel': ('hbm', part + slots * 8 + rows_bytes), 'sel_dq_merge_kernel': ('hbm', part + rows_bytes),
         'sel_delta_kernel': ('hbm', 2 * rows_bytes + b * hq * n * 4),
         'attend_fwd_kernel': ('tensor', f_fwd), 'attend_bwd_kernel': ('tensor', f_bwd),
