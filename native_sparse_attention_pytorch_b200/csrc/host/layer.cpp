@@ -8,7 +8,6 @@
 #include <ATen/Context.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <cublas_v2.h>
-#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/functions/basic_ops.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
@@ -658,15 +657,6 @@ struct NativeLayerBackward : torch::autograd::Node {
       return fail.apply(std::move(out));
     }
     return out;
-  }
-
- private:
-  [[noreturn]] static void raise_python_error(const char* what) {
-    const pybind11::gil_scoped_acquire gil;
-    PyErr_SetString(error_class(), what);
-    python_error err;
-    err.persist();
-    throw err;
   }
 };
 

@@ -28,7 +28,7 @@ struct Error : std::runtime_error {
   explicit Error(const std::string& what) : std::runtime_error(what) {}
 };
 
-PyObject* error_class();   // NsaError (module.cpp); the caller holds the GIL
+[[noreturn]] void raise_python_error(const char* what);   // as the package's NsaError, from a thread of the autograd engine
 
 inline void check(int64_t rc) {
   if (rc != 0) throw Error("libnsa_b200 returned " + std::to_string(rc) + ": " + nsa_last_error());

@@ -1,6 +1,13 @@
-// Selected-block attention: the bodies of the autograd function's two directions.
+// Selected-block attention: the bodies of the two directions, and the autograd node around them.
+
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/python_cpp_function.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/autograd/saved_variable.h>
 
 #include <algorithm>
+#include <cmath>
 #include <numeric>
 
 #include "nsa_host.h"
@@ -119,8 +126,118 @@ static std::vector<OptTensor> sel_backward(Tensor q, Tensor k, Tensor v, OptTens
   return {dq, dkv.select(0, 0), dkv.select(0, 1), want_slots ? OptTensor(slots) : OptTensor()};
 }
 
+// The autograd node of native_sparse_attend: 137 -> 110 us for forward and backward of 1 x 1024 positions against the same
+// calls behind a Python function.
+struct NativeSelectedBackward : torch::autograd::Node {
+  torch::autograd::SavedVariable q, k, v, idx, mask, out, lse;
+  Tensor index;            // which queries attend which key block, as the forward built it; `grad_fn.index` in Python
+  int64_t block = 0, diag = 0, impl = 0, status = 0;
+  double scale = 0;
+  std::optional<at::ScalarType> slot_type;
+
+  void release_variables() override {
+    for (auto* t : {&q, &k, &v, &idx, &mask, &out, &lse}) t->reset_data();
+    index = Tensor();
+  }
+
+  // The row sums sum_d out * dout that the gated combine's backward attaches to the branch gradient it returns
+  static OptTensor handed_over_delta(const Tensor& dout, const Tensor& lse) {
+    if (dout.unsafeGetTensorImpl()->pyobj_slot()->load_pyobj() == nullptr) return {};   // never seen by Python
+    const pybind11::gil_scoped_acquire gil;
+    const pybind11::object t = pybind11::reinterpret_steal<pybind11::object>(THPVariable_Wrap(dout));
+    const pybind11::object d = pybind11::getattr(t, "_nsa_delta", pybind11::none());
+    if (d.is_none()) return {};
+    Tensor delta = THPVariable_Unpack(d.ptr());
+    if (delta.sizes() != lse.sizes() || delta.scalar_type() != at::kFloat || !delta.is_contiguous() || delta.device() != dout.device()) return {};
+    return delta;
+  }
+
+  torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
+    torch::autograd::variable_list g(4);
+    if (!grads[0].defined()) return g;
+    try {
+      const at::NoGradGuard no_grad;
+      auto opt = [&](const torch::autograd::SavedVariable& s) {
+        Tensor t = s.unpack(getptr());
+        return t.defined() ? OptTensor(std::move(t)) : OptTensor();
+      };
+      const Tensor l = lse.unpack(getptr());
+      std::vector<OptTensor> r = sel_backward(q.unpack(getptr()), k.unpack(getptr()), v.unpack(getptr()), opt(idx), opt(mask), out.unpack(getptr()), l,
+                                              grads[0], handed_over_delta(grads[0], l), index.defined() ? OptTensor(index) : OptTensor(), block,
+                                              diag, impl, scale, status, slot_type.has_value());
+      for (int i = 0; i < 3; ++i) g[i] = std::move(*r[i]);
+      if (r[3].has_value()) g[3] = r[3]->to(*slot_type);
+    } catch (const Error& e) {
+      raise_python_error(e.what());
+    }
+    if (at::GradMode::is_enabled()) {   // create_graph: the gradients are there, their own gradients are not
+      for (auto& t : g)
+        if (t.defined()) t.set_requires_grad(true);
+      torch::autograd::DelayedError fail("trying to differentiate twice the native backward of selected-block attention", 4);
+      return fail.apply(std::move(g));
+    }
+    return g;
+  }
+};
+
+// -> out, lse
+static std::vector<Tensor> sel_attend(Tensor q, Tensor k, Tensor v, OptTensor idx, OptTensor mask, OptTensor slot_scale, int64_t block,
+                                      int64_t diag, int64_t impl, int64_t status, bool reuse_index) {
+  const double scale = 1.0 / std::sqrt((double)q.size(3));
+  const bool slots = slot_scale.has_value() && slot_scale->requires_grad();
+  const bool direct = q.requires_grad() || k.requires_grad() || v.requires_grad();
+  const bool wanted = at::GradMode::is_enabled() && (direct || slots);
+  std::vector<OptTensor> r;
+  {
+    const at::NoGradGuard no_grad;
+    r = sel_forward(q, k, v, std::move(idx), std::move(mask), block, diag, impl, scale, status, {}, wanted && direct && reuse_index);
+  }
+  Tensor out = *r[5], lse = *r[6];
+  if (!wanted) return {out, lse};
+  using torch::autograd::SavedVariable;
+  auto node = std::shared_ptr<NativeSelectedBackward>(new NativeSelectedBackward, torch::autograd::deleteNode);
+  torch::autograd::edge_list edges = {torch::autograd::impl::gradient_edge(q), torch::autograd::impl::gradient_edge(k),
+                                      torch::autograd::impl::gradient_edge(v),
+                                      slot_scale.has_value() ? torch::autograd::impl::gradient_edge(*slot_scale) : torch::autograd::Edge()};
+  node->set_next_edges(std::move(edges));
+  auto saved = [&](int i) { return r[i].value_or(Tensor()); };
+  node->q = SavedVariable(saved(0), false); node->k = SavedVariable(saved(1), false); node->v = SavedVariable(saved(2), false);
+  node->idx = SavedVariable(saved(3), false); node->mask = SavedVariable(saved(4), false); node->lse = SavedVariable(lse, false);
+  node->index = saved(7);
+  node->block = block; node->diag = diag; node->impl = impl; node->status = status; node->scale = scale;
+  if (slot_scale.has_value()) node->slot_type = slot_scale->scalar_type();
+  torch::autograd::set_history(out, node);
+  node->out = SavedVariable(out, true);
+  return {out, lse};
+}
+
+static PyObject* node_index(PyObject* self, void*) {
+  const auto* node = dynamic_cast<NativeSelectedBackward*>(reinterpret_cast<torch::autograd::THPCppFunction*>(self)->cdata.get());
+  if (node == nullptr || !node->index.defined()) Py_RETURN_NONE;
+  return THPVariable_Wrap(node->index);
+}
+
+static void register_node() {
+  namespace ta = torch::autograd;
+  using namespace torch::autograd;   // the property table's names
+  static PyTypeObject type;
+  static PyGetSetDef properties[] = {THP_FUNCTION_DEFAULT_PROPERTIES,
+                                     {(char*)"index", node_index, nullptr, nullptr, nullptr},
+                                     {nullptr, nullptr, nullptr, nullptr, nullptr}};
+  static PyMethodDef methods[] = {{"_register_hook_dict", ta::THPCppFunction_register_hook_dict, METH_O, nullptr},
+                                  {"register_hook", ta::THPCppFunction_register_hook, METH_O, nullptr},
+                                  {"register_prehook", ta::THPCppFunction_register_prehook, METH_O, nullptr},
+                                  {"name", ta::THPCppFunction_name, METH_NOARGS, nullptr},
+                                  {"_sequence_nr", ta::THPCppFunction_sequence_nr, METH_NOARGS, nullptr},
+                                  {nullptr, nullptr, 0, nullptr}};
+  ta::_initFunctionPyTypeObject(type, "NativeSelectedBackward", properties, methods);
+  ta::registerCppFunction(typeid(NativeSelectedBackward), &type);
+}
+
 void bind_selected(pybind11::module_& m) {
   namespace py = pybind11;
+  register_node();
+  m.def("sel_attend", &sel_attend, py::call_guard<py::gil_scoped_release>());
   m.def("sel_forward", &sel_forward, py::call_guard<py::gil_scoped_release>());
   m.def("sel_backward", &sel_backward, py::call_guard<py::gil_scoped_release>());
 }

@@ -266,8 +266,13 @@ def native_sparse_attend(fq, fk, fv, block_size, selected_block_indices, fmask, 
     assert q_heads % kv_heads == 0
     assert sel_heads in (q_heads, kv_heads)
     diag = L.DIAG_CAUSAL if include_block_causal else L.DIAG_NONE
-    out, lse = SelectedAttention.apply(fq, fk, fv, selected_block_indices, fmask, sel_scale, block_size, diag,
-                                       L.IMPL_BY_NAME[impl], index_cache)
+    if index_cache is None:
+        L.require_cuda(fq)
+        out, lse = L.host().sel_attend(fq, fk, fv, selected_block_indices, fmask, sel_scale, block_size, diag,
+                                       L.IMPL_BY_NAME[impl], _status_word(fq.device), REUSE_INDEX)
+    else:
+        out, lse = SelectedAttention.apply(fq, fk, fv, selected_block_indices, fmask, sel_scale, block_size, diag,
+                                           L.IMPL_BY_NAME[impl], index_cache)
     if return_sliding_window_out:
         sliding_out, sliding_lse = SlidingAttention.apply(fq, fk, fv, block_size, True, L.IMPL_BY_NAME[impl])
         out, lse = (out, sliding_out), (lse, sliding_lse)
