@@ -230,11 +230,13 @@ __device__ __forceinline__ int2 block_scan2(int2 v, int2* total, int2 (*warp_sum
 // List bases (padded to whole chunks), the fill cursors and the item table; one CTA, every thread owns a run of lists.
 // A list is cut into items of at most kChunksPerItem chunks, fewer when the whole problem has few chunks: an item is
 // what one CTA walks serially, so a problem of a few hundred chunks in items of sixteen leaves most of the chip idle.
-// The line is kItemsTarget items (16 per SM): below it the K/V loads and the dK/dV flush of a short item still cost
-// less than the imbalance of long ones.
-constexpr int kItemsTarget = 148 * 16;
+// The line is 16 items per SM at dim_head 64 and 8 at 128, where an item's K/V loads and dK/dV flush cost twice as much
+// and the forward has two CTAs per SM instead of four.  Below it these costs outweigh the imbalance of long items: 3001
+// positions, 16 / 2 heads of 128, backward + forward 198 us with 16, 160 with 8, 158 with 5, 173 with 3; 3 x 4997, 8 / 4 heads
+// of 64 545 us with 16, 614 with 8.
+static int items_target(int D) { return 148 * (D == 64 ? 16 : 8); }
 __global__ void __launch_bounds__(1024) sel_items_kernel(const int* totals, int* list_base, int* list_item, int* cursors, int4* items,
-                                                         int* num_items, int nlists, int QT, uint32_t tag) {
+                                                         int* num_items, int nlists, int QT, int target, uint32_t tag) {
   __shared__ int2 warp_sums[32];
   const int per = (nlists + 1023) / 1024;
   const int l0 = min(nlists, (int)threadIdx.x * per), l1 = min(nlists, l0 + per);
@@ -242,7 +244,7 @@ __global__ void __launch_bounds__(1024) sel_items_kernel(const int* totals, int*
   for (int l = l0; l < l1; ++l) chunks += (totals[l] + QT - 1) / QT;
   int2 all;
   block_scan2(make_int2(chunks, 0), &all, &warp_sums);
-  const int cpi = max(1, min(kChunksPerItem, all.x / kItemsTarget));
+  const int cpi = max(1, min(kChunksPerItem, all.x / target));
   int nit = 0;
   for (int l = l0; l < l1; ++l) nit += ((totals[l] + QT - 1) / QT + cpi - 1) / cpi;
   int2 at = block_scan2(make_int2(chunks, nit), &all, &warp_sums);
@@ -1934,7 +1936,7 @@ static int build_index(const SelProblem& a, const SelPlan& p, uint8_t* ix, cudaS
   if (a.mode == kModeSel) sel_count_kernel<kModeSel><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, bits, p.words);
   else if (a.mode == kModeSwa) sel_count_kernel<kModeSwa><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, bits, p.words);
   else sel_count_kernel<kModeCmp><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, bits, p.words);
-  sel_items_kernel<<<1, 1024, 0, st>>>(totals, list_base, list_item, cursors, items, num_items, p.nlists, p.QT, index_tag(a, p));
+  sel_items_kernel<<<1, 1024, 0, st>>>(totals, list_base, list_item, cursors, items, num_items, p.nlists, p.QT, items_target(a.D), index_tag(a, p));
   if (a.mode == kModeSel) sel_fill_kernel<kModeSel><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, list_base, cursors, entries, positions, p.QT);
   else if (a.mode == kModeSwa) sel_fill_kernel<kModeSwa><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, list_base, cursors, entries, positions, p.QT);
   else sel_fill_kernel<kModeCmp><<<grid, kIndexQueries, hist_smem, st>>>(R, totals, list_base, cursors, entries, positions, p.QT);
