@@ -82,7 +82,8 @@ PREFILL_WORKLOADS = {
 
 
 # dram__bytes_read.sum + dram__bytes_write.sum per launch, from single-launch ncu captures of this command
-# (`ncu --set full -k regex:<kernel> -c 1 python bench.py --steps 2 --warmup 3 --no-cpu-baseline`) at this build.
+# (`ncu --set full -k regex:<kernel> -c 1 python bench.py --steps 2 --warmup 3 --no-cpu-baseline`), taken
+# while the partial rows still left row by row; their amount is the same.
 NCU_DRAM_BYTES = {
     'sel_bwd_ws_kernel': 701.6e6 + 2195.7e6,
     'sel_fwd_kernel': 902.5e6 + 2425.9e6,
