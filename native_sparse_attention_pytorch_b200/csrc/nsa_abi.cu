@@ -20,7 +20,6 @@ int fail(int code, const char* msg) {
 static std::atomic<long long> g_launches{0};
 void count_launches(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
-static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // A [B,H,N,d] view is usable when rows start on 16-byte boundaries.
 static int check_tensor(const nsa_tensor& t, int dtype, const char* name) {

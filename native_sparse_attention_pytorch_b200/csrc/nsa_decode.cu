@@ -949,6 +949,9 @@ int launch_project(const ProjectParams& P, int dtype, cudaStream_t stream) {
   const int smem = project_smem(P.rows, P.dim, dtype);
   if (P.rows == 0) return NSA_OK;
   if (smem == 0) return fail(NSA_ERR_UNSUPPORTED, "projection of token rows: too many or too long");
+  const int V = dtype == NSA_F32 ? 4 : 8;   // (only the first `sets` of the pairs are given; the others are NULL)
+  if (!aligned16(P.x[0], P.x[1], P.w[0], P.w[1], P.add[0], P.add[1], P.norm_w, P.gate_w) || P.x_sb % V || P.x_sh % V)
+    return fail(NSA_ERR_ALIGN, "projection of token rows: rows and weights must start on 16-byte boundaries");
   if (dtype == NSA_F32) {
     const int pairs = (P.features + 1) / 2 + (P.gates_n + 1) / 2, blocks = min((pairs + kProjWarps - 1) / kProjWarps, 148 * 4);
     if (P.rows <= 1) return launch_project_with<project_f32_kernel<1>>(P, blocks, smem, stream);

@@ -10,6 +10,10 @@ namespace nsa {
 
 enum { BR_SEL = 0, BR_CMP = 1, BR_SWA = 2 };
 
+// Every pointer (NULL included) on a 16-byte boundary, as the kernels' vector accesses need it
+template <typename... P>
+inline bool aligned16(const P*... p) { return ((reinterpret_cast<uintptr_t>(p) | ...) & 15u) == 0; }
+
 // Parameters of the generic attention kernels (all three branches).
 struct AttnParams {
   const void *q, *k, *v, *dout;

@@ -108,6 +108,8 @@ __global__ void __launch_bounds__(256) layer_prep_kernel(const LayerShape L, con
 
 int launch_layer_prep(const LayerShape& L, const LayerPrep& P, int dtype, cudaStream_t stream) {
   const int V = dtype == NSA_F32 ? 4 : 8;
+  if (!aligned16(P.qkv, P.pos_k, P.pos_v, P.qr, P.kr, P.v_out, P.kw, P.vw) || P.c_sb % V || P.c_sh % V || L.d % V)
+    return fail(NSA_ERR_ALIGN, "layer: qkv rows, positions and outputs must start on 16-byte boundaries");
   const int64_t rot = (int64_t)L.batch * ((L.seq + kTileN - 1) / kTileN);
   const int64_t win = (2 * (int64_t)L.batch * L.kv_heads * L.ncb * L.cbs * (L.d / V) + 255) / 256;
   if (rot > 0x3fffffff) return fail(NSA_ERR_SHAPE, "layer: too many positions for one launch");
@@ -140,6 +142,7 @@ __global__ void __launch_bounds__(256) join_mem_kernel(const LayerShape L, const
 
 int launch_join_mem(const LayerShape& L, const void* mem, const void* ck, const void* cv, void* out, int dtype, cudaStream_t stream) {
   const int V = dtype == NSA_F32 ? 4 : 8;
+  if (!aligned16(mem, ck, cv, out) || L.d % V) return fail(NSA_ERR_ALIGN, "layer: memory slots and compressed rows must start on 16-byte boundaries");
   const int64_t blocks = (2 * (int64_t)L.batch * L.kv_heads * (L.num_mem + L.ncb) * (L.d / V) + 255) / 256;
   if (blocks == 0) return NSA_OK;
   const unsigned grid = (unsigned)(blocks < 148 * 8 ? blocks : 148 * 8);

@@ -187,6 +187,9 @@ int launch_rmsnorm(const NormParams& P, int dtype, bool backward, cudaStream_t s
     }
     return NSA_OK;
   }
+  const int V = dtype == NSA_F32 ? 4 : 8;
+  if (!aligned16(P.x, P.weight, P.y, P.dy, P.dx) || P.x_stride % V)
+    return fail(NSA_ERR_ALIGN, "RMS norm: the rows and the weight must start on 16-byte boundaries");
   const int64_t blocks = (P.rows + 7) / 8;
   // the backward adds one partial per block: a few blocks per SM bound the atomics, the forward is a plain stream
   const int64_t cap = backward ? 148 * 2 : 148 * 16;   // backward: the blocks one wave holds (two per SM)

@@ -25,6 +25,13 @@ _F32_EPS = torch.finfo(torch.float32).eps
 _PLAIN = (nn.Parameter, torch.Tensor)
 
 
+def _takes(p, like):
+    """The native kernels can read parameter `p` next to activations `like`: same type and device, dense, and on the
+    16-byte boundary their loads need (a view into a flat buffer of many parameters often is not)."""
+    return p.dtype is like.dtype and p.device == like.device and p.is_contiguous() and p.__class__ in _PLAIN and \
+        not p.data_ptr() & 15
+
+
 def _untouched(module, cls):
     """`module` is exactly a `cls` that runs its own forward: no subclass, no hooks, no replaced forward."""
     d = module.__dict__
@@ -127,10 +134,11 @@ class SparseAttention(Module):
 
     def _native_weights(self, x):
         """The parameters the native layer calls take, or None where the layer has to run module by module: a replaced
-        or hooked submodule, autocast, parameters of another type, dtype or device than the input."""
-        dtype, device, dim = x.dtype, x.device, x.shape[-1]
+        or hooked submodule, autocast, parameters of another type, dtype or device than the input, an input or
+        parameters off the 16-byte boundaries the kernels load from."""
+        dtype, dim = x.dtype, x.shape[-1]
         if (dtype is not torch.bfloat16 and dtype is not torch.float32) or x.dim() != 3 or torch.is_autocast_enabled('cuda') or \
-                _has_any_global_hook() or torch.compiler.is_compiling():
+                _has_any_global_hook() or torch.compiler.is_compiling() or x.data_ptr() & 15:
             return None
         m = self._modules
         norm, gate, qkv, out = m['norm'], m['to_strategy_combine'], m['to_qkv'], m['combine_heads']
@@ -157,11 +165,25 @@ class SparseAttention(Module):
                 if p is norm_w:
                     continue
                 return None
-            if p.dtype is not dtype or p.device != device or not p.is_contiguous() or p.__class__ not in _PLAIN:
+            if not _takes(p, x):
                 return None
         if w[1].shape != (self._qkv_rows, dim) or w[2].shape != (3 * self.heads, dim) or dim % 8:
             return None
         return w, eps
+
+    def _native_parameters(self, x):
+        """All parameters of a native layer call, in its order, and the norm's epsilon; or None as `_native_weights`."""
+        native = self._native_weights(x)
+        if native is None:
+            return None
+        k_net, v_net = self._default_network('k_compress', x), self._default_network('v_compress', x)
+        pos = (self._parameters['k_intrablock_positions'], self._parameters['v_intrablock_positions'])
+        if k_net is None or v_net is None or k_net[0].shape != v_net[0].shape or k_net[0].shape[0] % 8:
+            return None
+        if not (_takes(pos[0], x) and _takes(pos[1], x)):
+            return None
+        w, eps = native
+        return (*w, *pos, *k_net, *v_net), eps
 
     def _native_layer(self, x, return_cache):
         """The whole forward natively, or None where the layer has to run module by module (a chosen kernel family, a
@@ -171,24 +193,16 @@ class SparseAttention(Module):
         d, n = self.dim_head, x.shape[1]
         if n < self.compress_block_sliding_stride or d % 8 or d > 256 or x.shape[0] == 0 or x.__class__ not in _PLAIN:
             return None
-        native = self._native_weights(x)
+        native = self._native_parameters(x)
         if native is None:
             return None
-        k_net, v_net = self._default_network('k_compress', x), self._default_network('v_compress', x)
-        pos = (self._parameters['k_intrablock_positions'], self._parameters['v_intrablock_positions'])
-        if k_net is None or v_net is None or k_net[0].shape != v_net[0].shape or k_net[0].shape[0] % 8:
-            return None
-        for p in pos:
-            if p.dtype is not x.dtype or p.device != x.device or not p.is_contiguous() or p.__class__ not in _PLAIN:
-                return None
-        w, eps = native
-        weights = (*w, *pos, *k_net, *v_net)
+        weights, eps = native
         cfg = (self.heads, self.kv_heads, d, self.sliding_window_size, self.compress_block_size,
                self.compress_block_sliding_stride, self.selection_block_size, self.num_selected_blocks,
                self.num_mem_compress_kv, int(self.causal), int(self.query_heads_share_selected_kv), int(self.use_diff_topk))
         inv_freq = inverse_frequencies(d, self.rotary_emb.theta, x.device)
         if torch.is_grad_enabled() and (x.requires_grad or any([p.requires_grad for p in weights if p is not None])):
-            if return_cache or (w[0] is not None and x.shape[2] * x.element_size() > 16 * MAX_PIECES):
+            if return_cache or (weights[0] is not None and x.shape[2] * x.element_size() > 16 * MAX_PIECES):
                 return None
             return L.host().layer_apply(x, weights, eps, inv_freq, cfg, ops._status_word(x.device))
         out, *cache = L.host().layer_forward(x, weights, eps, inv_freq, cfg, ops._status_word(x.device), False, return_cache)
@@ -211,7 +225,7 @@ class SparseAttention(Module):
             return None
         w = (m[1]._parameters['weight'], m[1]._parameters['bias'], m[3]._parameters['weight'], m[3]._parameters['bias'])
         for p in w:
-            if p is None or p.dtype is not like.dtype or p.device != like.device or not p.is_contiguous() or p.__class__ not in _PLAIN:
+            if p is None or not _takes(p, like):
                 return None
         width = self.compress_block_size * self.dim_head
         return w if w[0].shape[1] == width and w[2].shape == (self.dim_head, w[0].shape[0]) else None
@@ -221,7 +235,7 @@ class SparseAttention(Module):
         before attended the blocks that existed before this token, as upstream's does)."""
         grown = None
         pk, pv = self.k_intrablock_positions, self.v_intrablock_positions
-        if native and pk.dtype is run_k.dtype and pv.dtype is run_k.dtype and pk.is_contiguous() and pv.is_contiguous():
+        if native and _takes(pk, run_k) and _takes(pv, run_k):
             k_net, v_net = self._default_network('k_compress', run_k), self._default_network('v_compress', run_k)
             if k_net is not None and v_net is not None:
                 grown = L.host().compress_filled(run_k, run_v, pk, pv, *k_net, *v_net, ck, cv)

@@ -83,3 +83,25 @@ def test_continuations_of_one_cache_do_not_disturb_each_other():
         got, _ = steps(layer, b[:, :3], cut)
         want, _ = steps(layer, b[:, :3], ((cut[0][0].clone(), cut[0][1].clone()), cut[1]))
         assert torch.equal(got, want)
+
+
+def test_step_refuses_weights_off_the_16_byte_boundary():
+    """Below the layer's own check: the native call reports NSA_ERR_ALIGN instead of loading from such addresses."""
+    from native_sparse_attention_pytorch_b200 import _lib as L
+    from native_sparse_attention_pytorch_b200.rotary import inverse_frequencies
+    layer = build(torch.bfloat16, 8, 2, 64)
+    x = recipe.randn((2, 200, 256), 5).bfloat16().to(DEV)
+    with torch.no_grad():
+        _, cache = layer(x, return_cache=True)
+    (w, eps) = layer._native_weights(x[:, :1])
+
+    def step(norm, qkv, gate, gate_b, out, mem):
+        return L.host().layer_decode(x[:, :1], norm, eps, qkv, gate, gate_b, out, inverse_frequencies(64, 10000., x.device), mem,
+                                     *flat(cache), 8, 16, 64, 32, 4, 100)
+    want = step(*w)[0]
+    for i in (0, 1, 2, 4, 5):
+        buf = torch.empty(w[i].numel() + 4, dtype=w[i].dtype, device=DEV)
+        moved = buf[4:].view(w[i].shape).copy_(w[i])
+        with pytest.raises(L.NsaError, match='16-byte'):
+            step(*w[:i], moved, *w[i + 1:])
+    assert torch.equal(step(*w)[0], want)

@@ -80,3 +80,33 @@ def test_native_layer_equals_the_module_by_module_layer(case):
         for got, want in zip((*cache[0], *cache[1][0], *cache[1][1]), (*ref[0], *ref[1][0], *ref[1][1])):
             assert got.shape == want.shape and got.dtype == want.dtype
             close(got, want, 'cache')
+
+
+def test_parameters_packed_into_one_buffer_take_the_module_path():
+    """Four heads in bf16: the gate bias is 24 bytes long, so the projections packed behind it start at 8 mod 16 and the
+    layer has to take the path whose operators read such weights."""
+    layer = SparseAttention(dim=256, dim_head=64, heads=4, kv_heads=2, causal=True, sliding_window_size=70, compress_block_size=32,
+                            compress_block_sliding_stride=16, selection_block_size=64, num_selected_blocks=3, use_triton_kernel=True)
+    recipe.fill_weights(layer, seed=3)
+    layer = layer.to('cuda').to(BF16)
+    x, dout, token = (recipe.randn((2, n, 256), seed).to(BF16).to('cuda') for n, seed in ((257, 5), (257, 6), (1, 7)))
+
+    def everything():
+        out, dx, grads = run(layer, x, dout)
+        with torch.no_grad():
+            _, cache = layer(x, return_cache=True)
+            step = layer(token, cache=cache)
+        return [out, dx, step, *grads.values()]
+    hook = layer.combine_heads.register_forward_hook(lambda *_: None)
+    want = everything()
+    hook.remove()
+    flat, at = torch.cat([p.detach().reshape(-1) for p in layer.parameters()]), 0
+    for name, p in list(layer.named_parameters()):
+        owner, _, leaf = name.rpartition('.')
+        layer.get_submodule(owner)._parameters[leaf] = torch.nn.Parameter(flat[at:at + p.numel()].view(p.shape))
+        at += p.numel()
+    assert any(p.data_ptr() % 16 for p in layer.parameters()) and layer.norm.weight.data_ptr() % 16 == 0
+    for got, ref in zip(everything(), want):
+        assert (got is None) == (ref is None)
+        if ref is not None:
+            assert_close_bf16(got, ref, 'packed parameters')

@@ -1,0 +1,60 @@
+"""What the layer checks on the host before it hands raw pointers to the native calls.  No GPU: the checks look at
+tensors, the calls behind them are never reached."""
+import pytest
+import torch
+
+from native_sparse_attention_pytorch_b200 import SparseAttention
+from native_sparse_attention_pytorch_b200 import _lib as L
+
+BF16, F32 = torch.bfloat16, torch.float32
+DIM, HEADS, KV_HEADS, D, CBS = 64, 4, 2, 64, 16
+
+
+def build(dtype=BF16, **options):
+    kw = dict(dim=DIM, dim_head=D, heads=HEADS, kv_heads=KV_HEADS, causal=True, sliding_window_size=32, compress_block_size=CBS,
+              compress_block_sliding_stride=8, selection_block_size=16, num_selected_blocks=2, use_triton_kernel=True)
+    return SparseAttention(**{**kw, **options}).to(dtype)
+
+
+def off_by(t, elements):
+    """A dense copy of t that starts `elements` elements behind a 16-byte boundary."""
+    buf = torch.empty(t.numel() + 16, dtype=t.dtype)
+    lead = (-buf.data_ptr() % 16) // t.element_size()
+    view = buf[lead + elements:lead + elements + t.numel()].view(t.shape)
+    view.copy_(t)
+    assert view.is_contiguous() and view.data_ptr() % 16 == elements * t.element_size() % 16
+    return view
+
+
+@pytest.mark.parametrize('dtype', [BF16, F32])
+def test_parameters_off_the_16_byte_boundary_take_the_module_path(dtype):
+    """A parameter that is a view into a flat buffer may start anywhere; the native kernels load 16 bytes at a time."""
+    layer, x = build(dtype), torch.zeros(2, 32, DIM, dtype=dtype)
+    assert layer._native_parameters(x) is not None
+    for name, p in list(layer.named_parameters()):
+        owner = layer.get_submodule(name.rpartition('.')[0])
+        owner._parameters[name.rpartition('.')[2]] = torch.nn.Parameter(off_by(p.detach(), 2))
+        assert layer._native_parameters(x) is None, name
+        owner._parameters[name.rpartition('.')[2]] = torch.nn.Parameter(off_by(p.detach(), 16 // p.element_size()))
+        assert layer._native_parameters(x) is not None, name
+
+
+@pytest.mark.parametrize('dtype', [BF16, F32])
+def test_parameters_packed_into_one_buffer(dtype):
+    """Four heads in bf16: the gate bias is 24 bytes, so what is packed behind it starts at 8 mod 16."""
+    layer, x = build(dtype), torch.zeros(1, 32, DIM, dtype=dtype)
+    flat = torch.cat([p.detach().reshape(-1) for p in layer.parameters()])
+    at, aligned = 0, True
+    for name, p in list(layer.named_parameters()):
+        view = flat[at:at + p.numel()].view(p.shape)
+        aligned = aligned and view.data_ptr() % 16 == 0
+        layer.get_submodule(name.rpartition('.')[0])._parameters[name.rpartition('.')[2]] = torch.nn.Parameter(view)
+        at += p.numel()
+    assert (layer._native_parameters(x) is not None) == aligned
+    assert aligned == (dtype == F32)
+
+
+def test_an_input_at_an_odd_offset_takes_the_module_path():
+    layer, x = build(), torch.zeros(1, 32, DIM, dtype=BF16)
+    assert layer._native_weights(x) is not None
+    assert layer._native_weights(off_by(x, 1)) is None
