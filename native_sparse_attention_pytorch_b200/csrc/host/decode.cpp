@@ -23,10 +23,28 @@ static nsa_decode_args decode_args(const void* q, const void* qr, const Tensor& 
   return a;
 }
 
+// The kernels take batch, heads and row length from one tensor and address the others with them
+static void require_shape(bool ok, const char* what) {
+  if (!ok) throw Error(std::string("decode step: ") + what);
+}
+static bool is_cache(const Tensor& k, const Tensor& v, int64_t batch, int64_t heads, int64_t d) {
+  return k.dim() == 4 && k.size(0) == batch && k.size(1) == heads && k.size(3) == d && v.sizes() == k.sizes();
+}
+static void check_compressed(const Tensor& ck, const Tensor& cv, int64_t batch, int64_t heads, int64_t d) {
+  require_shape(is_cache(ck, cv, batch, heads, d), "compressed keys and values must both be [batch, kv_heads, blocks, dim_head] of the cache they belong to");
+}
+
 // Attention part of a step on tensors the caller holds
 static Tensor decode_step(Tensor q, Tensor qr, Tensor keys, Tensor vals, Tensor ck, Tensor cv, Tensor mem_k, Tensor mem_v,
                           Tensor gates, int64_t stride, int64_t block, int64_t nsel, int64_t window) {
   for (const Tensor* t : {&q, &qr, &keys, &vals, &ck, &cv, &mem_k, &mem_v, &gates}) require_cuda(*t);
+  require_shape(q.dim() == 3 && qr.sizes() == q.sizes(), "q and qr must both be [batch, q_heads, dim_head]");
+  require_shape(keys.dim() == 4 && is_cache(keys, vals, q.size(0), keys.size(1), q.size(2)),
+                "keys and values must both be [batch, kv_heads, rows, dim_head] with the batch and dim_head of q");
+  check_compressed(ck, cv, q.size(0), keys.size(1), q.size(2));
+  require_shape(mem_k.dim() == 3 && mem_k.size(0) == keys.size(1) && mem_k.size(2) == q.size(2) && mem_v.sizes() == mem_k.sizes(),
+                "memory keys and values must both be [kv_heads, slots, dim_head]");
+  require_shape(gates.numel() == q.size(0) * q.size(1) * 3, "gates must be [batch, q_heads, 3]");
   const c10::cuda::CUDAGuard guard(q.device());
   const auto dt = q.scalar_type();
   q = q.contiguous();
@@ -56,9 +74,19 @@ static std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> layer_decode(
     Tensor x, OptTensor norm_w, double eps, Tensor qkv_w, Tensor gate_w, Tensor gate_b, Tensor out_w, Tensor inv_freq,
     Tensor mem_kv, Tensor past_k, Tensor past_v, Tensor ck, Tensor cv, Tensor run_k, Tensor run_v, int64_t heads,
     int64_t stride, int64_t block, int64_t cbs, int64_t nsel, int64_t window) {
+  require_shape(x.dim() == 3 && x.size(1) == 1, "the input must be [batch, 1, dim]");
+  require_shape(mem_kv.dim() == 4 && mem_kv.size(0) == 2, "memory slots must be [2, kv_heads, slots, dim_head]");
+  const int64_t B = x.size(0), dim = x.size(2), hkv = mem_kv.size(1), d = mem_kv.size(3), rows = 3 * heads;
+  require_shape(qkv_w.dim() == 2 && qkv_w.size(0) == (heads + 2 * hkv) * d && qkv_w.size(1) == dim && gate_w.dim() == 2 &&
+                    gate_w.size(0) == rows && gate_w.size(1) == dim && gate_b.numel() == rows && out_w.dim() == 2 &&
+                    out_w.size(0) == dim && out_w.size(1) == heads * d && (!norm_w.has_value() || norm_w->numel() == dim) &&
+                    inv_freq.numel() == d / 2,
+                "the weights are not those of a layer with these heads");
+  require_shape(is_cache(past_k, past_v, B, hkv, d), "cached keys and values must both be [batch, kv_heads, rows, dim_head] with the batch of the input");
+  check_compressed(ck, cv, B, hkv, d);
+  require_shape(is_cache(run_k, run_v, B, hkv, d), "the window being filled must be [batch, kv_heads, rows, dim_head], keys and values alike");
   const c10::cuda::CUDAGuard guard(x.device());
   void* st = stream_of(x);
-  const int64_t B = x.size(0), dim = x.size(2), hkv = past_k.size(1), d = past_k.size(3), rows = 3 * heads;
   const int dt = dtype_code(x);
   x = rowwise(x);
   ck = rowwise(ck);
@@ -116,6 +144,7 @@ static std::optional<std::tuple<Tensor, Tensor>> compress_filled(Tensor run_k, T
                                                                  Tensor k1, Tensor kb1, Tensor k2, Tensor kb2, Tensor v1,
                                                                  Tensor vb1, Tensor v2, Tensor vb2, Tensor ck, Tensor cv) {
   const int64_t B = run_k.size(0), H = run_k.size(1), d = run_k.size(3), width = run_k.size(2) * d, hidden = k1.size(0);
+  check_compressed(ck, cv, B, H, d);
   const int dt = dtype_code(run_k);
   if (!nsa::project_serves(B * H, width, dt) || !nsa::project_serves(B * H, hidden, dt) || run_k.stride(2) != d ||
       run_k.strides() != run_v.strides() || run_k.stride(3) != 1 || run_v.stride(3) != 1)

@@ -58,3 +58,29 @@ def test_an_input_at_an_odd_offset_takes_the_module_path():
     layer, x = build(), torch.zeros(1, 32, DIM, dtype=BF16)
     assert layer._native_weights(x) is not None
     assert layer._native_weights(off_by(x, 1)) is None
+
+
+def decode_arguments(layer, **changes):
+    b, t, ncb, r = 2, 20, 2, 5
+    cache = dict(past_k=(b, KV_HEADS, t, D), past_v=(b, KV_HEADS, t, D), ck=(b, KV_HEADS, ncb, D), cv=(b, KV_HEADS, ncb, D),
+                 run_k=(b, KV_HEADS, r, D), run_v=(b, KV_HEADS, r, D))
+    x = torch.zeros(changes.pop('x', (b, 1, DIM)), dtype=BF16)
+    (norm, qkv, gate, gate_b, out, mem), eps = layer._native_weights(x)
+    w = dict(qkv=qkv, gate=gate, gate_b=gate_b, out=out, mem=mem)
+    for name, shape in changes.items():
+        (cache if name in cache else w)[name] = shape if name in cache else torch.zeros(shape, dtype=BF16)
+    return (x, norm, eps, w['qkv'], w['gate'], w['gate_b'], w['out'], torch.zeros(D // 2), w['mem'],
+            *(torch.zeros(s, dtype=BF16) for s in cache.values()), HEADS, 8, 16, CBS, 2, 32)
+
+
+@pytest.mark.parametrize('changes', [
+    dict(x=(3, 1, DIM)), dict(x=(1, 1, DIM)), dict(x=(2, 2, DIM)),
+    dict(past_k=(3, KV_HEADS, 20, D)), dict(past_v=(2, KV_HEADS, 19, D)), dict(past_k=(2, HEADS, 20, D)), dict(past_v=(2, KV_HEADS, 20, 32)),
+    dict(ck=(1, KV_HEADS, 2, D)), dict(cv=(2, KV_HEADS, 1, D)), dict(cv=(2, 1, 2, D)), dict(ck=(2, KV_HEADS, 2, 32)),
+    dict(run_k=(1, KV_HEADS, 5, D)), dict(run_v=(2, KV_HEADS, 4, D)), dict(run_v=(2, 1, 5, D)), dict(run_k=(2, KV_HEADS, D)),
+    dict(out=(DIM, 2 * HEADS * D)), dict(out=(2 * DIM, HEADS * D)), dict(mem=(2, 1, 1, D)), dict(gate_b=(3,))],
+    ids=lambda c: '-'.join(f'{k}{list(v)}' for k, v in c.items()))
+def test_a_step_refuses_caches_of_another_shape(changes):
+    """Batch, heads and row length are taken from one tensor and address all others, so each has to agree."""
+    with pytest.raises(L.NsaError, match='decode step'):
+        L.host().layer_decode(*decode_arguments(build(), **changes))
