@@ -374,10 +374,11 @@ static Tensor importance_gradient(const Layer& L, const Tensor& importance, cons
   return ds;
 }
 
-// -> gradients of x and of the parameters, in the order of the forward's arguments; `needs` says which are wanted
+// -> gradients of x and of the parameters, in the order of the forward's arguments; `needs` says which are wanted.  With
+// `keep_built` the indexes of the sliding and the compressed backward that had to be built here follow.
 static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor> weights, std::vector<OptTensor> saved,
                                              double eps, Tensor inv_freq, std::vector<int64_t> cfg, int64_t status,
-                                             std::vector<bool> needs, OptTensor swa_index, OptTensor cmp_index) {
+                                             std::vector<bool> needs, OptTensor swa_index, OptTensor cmp_index, bool keep_built) {
   const LayerWeights w = weights_of(weights);
   auto sv = [&](size_t i) { return saved.at(i).value_or(Tensor()); };
   const Tensor x = sv(0), xn = sv(1), rstd = sv(2), qkv = sv(3), logits = sv(4), kept = sv(5), hk = sv(6), hv = sv(7), index = sv(8),
@@ -478,7 +479,7 @@ static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor>
     a.dout = d_o(2); a.dk = dk; a.dv = dk + k_elems; a.accumulate_kv = 1; a.delta = delta(2);
     if (swa_index.has_value()) { a.index = swa_index->data_ptr(); a.index_bytes = swa_index->numel(); }
     with_dq(2, nsa_swa_bwd_stores_dq(&a.fwd) == 1, false, a.dq_out, a.dq, [&] { return nsa_swa_bwd(&a, st); });
-    const int64_t n = swa_index.has_value() || !ws.defined() ? 0 : nsa_swa_index_bytes(&a.fwd);
+    const int64_t n = !keep_built || swa_index.has_value() || !ws.defined() ? 0 : nsa_swa_index_bytes(&a.fwd);
     if (n > 0) built[0] = ws.narrow(0, 0, n).clone();
   }
   const bool through_topk = slots.defined();
@@ -489,7 +490,7 @@ static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor>
     a.dout = d_o(0); a.dck = dck; a.dcv = dck + c_elems; a.accumulate_kv = 1; a.delta = delta(0);
     if (cmp_index.has_value()) { a.index = cmp_index->data_ptr(); a.index_bytes = cmp_index->numel(); }
     with_dq(0, nsa_cmp_bwd_stores_dq(&a.fwd) == 1, through_topk, a.dq_out, a.dq, [&] { return nsa_cmp_bwd(&a, st); });
-    const int64_t n = cmp_index.has_value() || !ws.defined() ? 0 : nsa_cmp_index_bytes(&a.fwd);
+    const int64_t n = !keep_built || cmp_index.has_value() || !ws.defined() ? 0 : nsa_cmp_index_bytes(&a.fwd);
     if (n > 0) built[1] = ws.narrow(0, 0, n).clone();
   }
   if (through_topk) {
@@ -577,7 +578,9 @@ static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor>
 }
 
 // The index of the sliding and of the compressed backward depends on the sizes only: kept for the last few shapes, per
-// stream (so that none is read by another stream than the one that built it).
+// stream (so that none is read by another stream than the one that built it).  Not while the stream is being captured:
+// what a graph builds exists only once it is replayed, and what it was handed would have to live as long as the graph.  A
+// captured step builds its indexes itself, in the graph's own memory.
 class IndexCache {
  public:
   using Key = std::vector<int64_t>;
@@ -642,7 +645,11 @@ struct NativeLayerBackward : torch::autograd::Node {
       swa.insert(swa.end(), {0, c.window});
       cmp.insert(cmp.end(), {1, c.num_mem, c.stride});
       auto& cache = IndexCache::instance();
-      std::vector<OptTensor> g = layer_backward(grads[0], w, sv, eps, inv_freq, cfg, status, std::move(needs), cache.find(swa), cache.find(cmp));
+      cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+      if (cudaStreamIsCapturing((cudaStream_t)stream_of(x), &capture) != cudaSuccess) throw Error("layer: the state of the stream cannot be read");
+      const bool eager = capture == cudaStreamCaptureStatusNone;
+      std::vector<OptTensor> g = layer_backward(grads[0], w, sv, eps, inv_freq, cfg, status, std::move(needs), eager ? cache.find(swa) : OptTensor(),
+                                                eager ? cache.find(cmp) : OptTensor(), eager);
       for (int i = 0; i < 1 + kWeights; ++i)
         if (g[i].has_value()) out[i] = std::move(*g[i]);
       if (g[1 + kWeights].has_value()) cache.keep(std::move(swa), *g[1 + kWeights]);

@@ -179,20 +179,22 @@ def _call_bwd(fn, make_args, q, stream):
 
 
 # The index the sliding and the compressed backward walk depends on the sizes only: built once per shape and device
-# (by the first backward call, inside its work buffer), then handed to later calls.  A few MB per entry.
+# (by the first backward call, inside its work buffer), then handed to later calls.  A few MB per entry.  Not while the
+# stream is being captured: what a graph builds exists only once it is replayed, and what it was handed would have to
+# live as long as the graph does.
 _shape_index = {}
 _SHAPE_INDEX_ENTRIES = 8
 
 
 def _cached_index(key):
-    if not REUSE_INDEX:
+    if not REUSE_INDEX or torch.cuda.is_current_stream_capturing():
         return None
     with _state_lock:
         return _shape_index.get(key)
 
 
 def _keep_index(key, ws, nbytes):
-    if not (REUSE_INDEX and ws is not None and nbytes > 0):
+    if not (REUSE_INDEX and ws is not None and nbytes > 0) or torch.cuda.is_current_stream_capturing():
         return
     with _state_lock:
         if key in _shape_index:

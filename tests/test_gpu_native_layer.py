@@ -110,3 +110,58 @@ def test_parameters_packed_into_one_buffer_take_the_module_path():
         assert (got is None) == (ref is None)
         if ref is not None:
             assert_close_bf16(got, ref, 'packed parameters')
+
+
+@pytest.mark.parametrize('how', ['native', 'module by module'])
+def test_graphs_and_eager_steps_of_one_shape_do_not_share_an_index(how):
+    """Two graphs of one shape, recorded on a stream that never ran this shape before; an eager step on that stream before
+    either graph was replayed; then replays after so many other shapes that every index kept for eager steps is gone."""
+    from native_sparse_attention_pytorch_b200 import ops
+    layer = SparseAttention(dim=256, dim_head=64, heads=8, kv_heads=2, causal=True, sliding_window_size=128, compress_block_size=32,
+                            compress_block_sliding_stride=16, selection_block_size=64, num_selected_blocks=4, use_triton_kernel=True)
+    recipe.fill_weights(layer, seed=7)
+    layer = layer.to('cuda').to(BF16)
+    if how != 'native':
+        layer.combine_heads.register_forward_hook(lambda *_: None)
+    params = list(layer.parameters())
+
+    def step(x, dout):
+        out = layer(x)
+        return [g for g in torch.autograd.grad(out, [x, *params], dout) if g is not None]
+
+    def inputs(n, seed):
+        x, dout = (recipe.randn((1, n, 256), seed + i).to(BF16).to('cuda') for i in range(2))
+        return x.requires_grad_(), dout
+
+    def same(got, want):
+        torch.cuda.synchronize()
+        ops.check_device_status()
+        for g, w in zip(got, want):
+            assert_close_bf16(g, w, 'gradient', roundings=2, rel_to_max=1e-2)
+
+    warm, other = torch.cuda.Stream(), torch.cuda.Stream()
+    warm.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(warm):
+        x, dout = inputs(700, 11)
+        want = step(x, dout)
+        step(x, dout)
+    torch.cuda.synchronize()
+    graphs = []
+    with torch.cuda.stream(other):
+        for _ in range(2):
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=other):
+                got = step(x, dout)
+            graphs.append((graph, got))
+        same(step(x, dout), want)
+        for graph, got in reversed(graphs):
+            graph.replay()
+            same(got, want)
+        for i in range(20):
+            step(*inputs(200 + 10 * i, 31))
+        for graph, got in graphs:
+            for g in got:
+                g.zero_()
+            graph.replay()
+            same(got, want)
+    del graphs, graph, got
