@@ -13,8 +13,21 @@ static Tensor rows_of(const Tensor& buf, int64_t first, int64_t rows) {
   return at::as_strided(buf, {buf.size(0), buf.size(1), rows, buf.size(3)}, buf.strides(), first * buf.size(3));
 }
 
+Rooms::Owner Rooms::current_owner(const Tensor& t) {
+  Owner o;
+  o.stream = stream_of(t);
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamGetCaptureInfo((cudaStream_t)o.stream, &status, &o.capture) != cudaSuccess) {
+    cudaGetLastError();
+    return o;
+  }
+  if (status == cudaStreamCaptureStatusNone) o.capture = 0;
+  o.known = true;
+  return o;
+}
+
 GrownPair Rooms::fresh(const Tensor& like, int64_t batch, int64_t heads, int64_t rows, int64_t room, int64_t d) {
-  at::AutoDispatchBelowADInplaceOrView no_view_tracking;   // a tracked view keeps its base, and so a second user of the storage
+  at::AutoDispatchBelowADInplaceOrView no_view_tracking;   // a tracked view would keep its base
   GrownPair g;
   const Tensor k_buf = at::empty({batch, heads, rows + room, d}, like.options());
   const Tensor v_buf = at::empty({batch, heads, rows + room, d}, like.options());
@@ -32,7 +45,7 @@ GrownPair Rooms::fresh(const Tensor& like, int64_t batch, int64_t heads, int64_t
         c10::intrusive_ptr<c10::StorageImpl>::reclaim_copy(t.storage().unsafeGetStorageImpl()));
   };
   entries_.erase(key);             // the address of a storage that is gone may come back
-  entries_.emplace(key, Entry{weak(k_buf), weak(v_buf), rows});
+  entries_.emplace(key, Entry{weak(k_buf), weak(v_buf), rows, current_owner(like)});
   return g;
 }
 
@@ -48,9 +61,8 @@ GrownPair Rooms::extend(const Tensor& k, const Tensor& v, int64_t room) {
         k.storage_offset() == v.storage_offset() && k.sizes() == v.sizes() && k.stride(3) == 1 && k.stride(2) == d &&
         k.stride(0) == k.stride(1) * H && k.scalar_type() == v.scalar_type()) {
       const int64_t capacity = k.stride(1) / d, first = k.storage_offset() / d, end = first + rows;
-      // the views of a continuation that was dropped are gone: nothing else is on these buffers
-      if (it->second.used > end && k.storage().use_count() == 1 && v.storage().use_count() == 1) it->second.used = end;
-      if (it->second.used == end && end < capacity && (int64_t)k.storage().nbytes() == B * H * capacity * d * k.element_size()) {
+      if (it->second.used == end && end < capacity && it->second.owner == current_owner(k) &&
+          (int64_t)k.storage().nbytes() == B * H * capacity * d * k.element_size()) {
         it->second.used = end + 1;
         GrownPair g;
         g.k_buf = k.storage().mutable_data();

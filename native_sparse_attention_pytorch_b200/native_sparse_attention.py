@@ -275,7 +275,9 @@ class SparseAttention(Module):
         that is being filled for the next compressed block, un-rotated))).  The attention part -- compressed branch,
         block selection, selected blocks plus the own block, sliding window, gated combine -- is one kernel launch
         (`ops.decode_step`, all (batch, KV head) units in its grid), and without gradients the whole step is three
-        launches (`_native_step`).  It keeps upstream's behaviour,
+        launches (`_native_step`) and the returned caches share memory with the ones they continue, where those are the
+        newest of their buffer and of the same stream (csrc/host/rooms.h): editing one in place changes the rows the
+        others have in common with it; clone a cache that is to be edited.  It keeps upstream's behaviour,
         including that the memory slots are attended only once a compressed block exists."""
         assert self.causal, 'inference only relevant for autoregressive'
         if not self.query_heads_share_selected_kv:

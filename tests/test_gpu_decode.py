@@ -76,7 +76,7 @@ def test_continuations_of_one_cache_do_not_disturb_each_other():
         again, _ = steps(layer, b, mid)
         assert torch.equal(again, out_b) and torch.equal(tail, tail_copy)
         del tail
-        again, _ = steps(layer, a[:, 5:], mid)                     # in place over the rows that were dropped
+        again, _ = steps(layer, a[:, 5:], mid)                     # and once more when the others are gone
         assert torch.equal(again, out_a)
         # a cache from elsewhere, its rows cut off in front: positions count from its own first row
         cut = ((mid[0][0][:, :, 64:], mid[0][1][:, :, 64:]), ((mid[1][0][0][:, :, 4:], mid[1][0][1][:, :, 4:]), mid[1][1]))
@@ -105,3 +105,61 @@ def test_step_refuses_weights_off_the_16_byte_boundary():
         with pytest.raises(L.NsaError, match='16-byte'):
             step(*w[:i], moved, *w[i + 1:])
     assert torch.equal(step(*w)[0], want)
+
+
+def storages(cache):
+    return [t.untyped_storage().data_ptr() for t in (*cache[0], *cache[1][1])]     # the tensors a step appends to
+
+
+def test_a_row_is_appended_in_place_only_where_nobody_ever_was():
+    layer = build(torch.bfloat16, 8, 2, 64)
+    x = recipe.randn((2, 203, 256), 5).bfloat16().to(DEV)
+    a, b = (recipe.randn((2, 6, 256), s).bfloat16().to(DEV) for s in (6, 7))
+    with torch.no_grad():
+        _, mid = layer(x, return_cache=True)
+        out_a, first = steps(layer, a, mid)
+        assert storages(first) == storages(mid)                    # the prefill's buffers, their only continuation so far
+        del first
+        out_b, second = steps(layer, b, mid)                       # the rows behind `mid` were given out once
+        assert not set(storages(second)) & set(storages(mid))
+        # a continuation on another stream gets tensors of that stream
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            out_c, third = steps(layer, a, second)
+            assert not set(storages(third)) & set(storages(second))
+            more, fourth = steps(layer, a, third)
+            assert storages(fourth) == storages(third)             # and goes on in place there
+        torch.cuda.current_stream().wait_stream(side)
+        want, _ = steps(layer, a, tuple(tuple(t.clone() for t in pair) if isinstance(pair[0], torch.Tensor) else
+                                        tuple(tuple(t.clone() for t in p) for p in pair) for pair in second))
+        assert torch.equal(out_c, want)
+
+
+def test_a_recorded_step_leaves_the_caches_of_eager_steps_alone():
+    layer = build(torch.bfloat16, 8, 2, 64)
+    x = recipe.randn((2, 203, 256), 5).bfloat16().to(DEV)
+    a, b = (recipe.randn((2, 4, 256), s).bfloat16().to(DEV) for s in (6, 7))
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.no_grad(), torch.cuda.stream(stream):
+        _, mid = layer(x, return_cache=True)
+        want, _ = steps(layer, a, tuple((t[0], t[1]) for t in mid))
+        _, mid = layer(x, return_cache=True)                       # buffers nothing has been appended to
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            out, recorded = steps(layer, a, mid)
+            assert not set(storages(recorded)) & set(storages(mid))
+        eager_out, eager = steps(layer, b, mid)
+        kept = [t.clone() for t in flat(eager)]
+        for _ in range(2):
+            graph.replay()
+            assert torch.equal(out, want)
+        assert all(torch.equal(t, k) for t, k in zip(flat(eager), kept))
+        after, grown = steps(layer, b, recorded)                   # an eager continuation of what the graph returned
+        assert not set(storages(grown)) & set(storages(recorded))
+        kept = [t.clone() for t in flat(grown)]
+        graph.replay()
+        assert all(torch.equal(t, k) for t, k in zip(flat(grown), kept))
+        torch.cuda.synchronize()
+    del recorded, out, graph
