@@ -407,17 +407,22 @@ static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor>
     return kept.narrow(0, off, n * (int64_t)c10::elementSize(t)).view(t).view(sizes);
   };
 
-  // fp32 accumulators, cleared together: dk, dv; dck, dcv; then the small gradients that end up in the layer's type
+  // fp32 accumulators, cleared together: dk, dv; dck, dcv; then the small gradients that end up in the layer's type.  An
+  // fp32 layer returns the small ones as they are: there they have memory of their own, a gradient that a program keeps
+  // must not keep the scratch of dk and dv with it.
   const int64_t pos = hkv * c.cbs * d, mems = hkv * c.num_mem * d, hid = w.k1.size(0);
   auto even = [](int64_t n) { return (n + 7) / 8 * 8; };
   const int64_t s_norm = 0, s_gate = s_norm + even(L.dim), s_mem = s_gate + even(3 * H), s_pos = s_mem + even(2 * mems),
                 s_b1 = s_pos + even(2 * pos), s_b2 = s_b1 + even(2 * hid), s_end = s_b2 + even(2 * d);
   const int64_t a_small = even(2 * k_elems + 2 * c_elems);
-  Tensor acc = empty({a_small + s_end}, x, at::kFloat);
-  if (cudaMemsetAsync(acc.data_ptr(), 0, (a_small + s_end) * 4, st) != cudaSuccess) throw Error("clearing the gradient accumulators failed");
+  const bool apart = type == at::kFloat;
+  Tensor acc = empty({apart ? a_small : a_small + s_end}, x, at::kFloat);
+  Tensor rounded = apart ? empty({s_end}, x, at::kFloat) : Tensor();
   float* const dk = ptr<float>(acc);
   float* const dck = dk + 2 * k_elems;
-  float* const small = dk + a_small;
+  float* const small = apart ? ptr<float>(rounded) : dk + a_small;
+  if (cudaMemsetAsync(dk, 0, acc.numel() * 4, st) != cudaSuccess || (apart && cudaMemsetAsync(small, 0, s_end * 4, st) != cudaSuccess))
+    throw Error("clearing the gradient accumulators failed");
 
   // output projection and gated combine
   dout = dout.reshape({BN, L.dim}).contiguous();
@@ -555,8 +560,7 @@ static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor>
     if (needs[0]) g[0] = dxn.view(x.sizes());
   }
   // the small gradients in the layer's type
-  Tensor rounded = acc.narrow(0, a_small, s_end);
-  if (type != at::kFloat) {
+  if (!apart) {
     rounded = at::empty({s_end}, x.options());
     check(nsa::launch_round(small, rounded.data_ptr(), s_end, st));
   }

@@ -165,3 +165,18 @@ def test_graphs_and_eager_steps_of_one_shape_do_not_share_an_index(how):
             graph.replay()
             same(got, want)
     del graphs, graph, got
+
+
+@pytest.mark.parametrize('dtype', [BF16, F32])
+def test_kept_gradients_do_not_keep_the_scratch_of_the_backward(dtype):
+    layer = SparseAttention(dim=256, dim_head=64, heads=4, kv_heads=2, causal=True, sliding_window_size=70, compress_block_size=32,
+                            compress_block_sliding_stride=16, selection_block_size=64, num_selected_blocks=3, use_triton_kernel=True)
+    recipe.fill_weights(layer, seed=3)
+    layer = layer.to('cuda').to(dtype)
+    sizes = []
+    for n in (64, 2048):
+        x, dout = (recipe.randn((2, n, 256), seed).to(dtype).to('cuda') for seed in (5, 6))
+        out, dx, grads = run(layer, x, dout)
+        assert 'NativeLayer' in out.grad_fn.name()
+        sizes.append({name: g.untyped_storage().nbytes() for name, g in grads.items()})
+    assert sizes[0] == sizes[1]
