@@ -672,7 +672,6 @@ struct NativeLayerBackward : torch::autograd::Node {
 };
 
 static Tensor layer_apply(Tensor x, std::vector<OptTensor> weights, double eps, Tensor inv_freq, std::vector<int64_t> cfg, int64_t status) {
-  if (x._fw_grad(0).defined()) throw Error("the layer has no forward-mode derivative");
   auto node = std::shared_ptr<NativeLayerBackward>(new NativeLayerBackward, torch::autograd::deleteNode);
   torch::autograd::edge_list edges = {torch::autograd::impl::gradient_edge(x)};
   node->weights.reserve(kWeights);

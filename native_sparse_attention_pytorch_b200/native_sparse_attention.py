@@ -13,6 +13,7 @@ from copy import deepcopy
 import torch
 import torch.nn.functional as F
 from torch import nn
+from torch.autograd import forward_ad
 from torch.nn import Module
 
 from . import _lib as L
@@ -134,11 +135,12 @@ class SparseAttention(Module):
 
     def _native_weights(self, x):
         """The parameters the native layer calls take, or None where the layer has to run module by module: a replaced
-        or hooked submodule, autocast, parameters of another type, dtype or device than the input, an input or
+        or hooked submodule, autocast, forward-mode differentiation (the modules refuse it), parameters of another type, dtype or device than the input, an input or
         parameters off the 16-byte boundaries the kernels load from."""
         dtype, dim = x.dtype, x.shape[-1]
         if (dtype is not torch.bfloat16 and dtype is not torch.float32) or x.dim() != 3 or torch.is_autocast_enabled('cuda') or \
-                _has_any_global_hook() or torch.compiler.is_compiling() or x.data_ptr() & 15:
+                _has_any_global_hook() or torch.compiler.is_compiling() or forward_ad._current_level >= 0 or \
+                x.data_ptr() & 15:
             return None
         m = self._modules
         norm, gate, qkv, out = m['norm'], m['to_strategy_combine'], m['to_qkv'], m['combine_heads']

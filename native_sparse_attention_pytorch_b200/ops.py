@@ -6,7 +6,7 @@ import ctypes as C
 import threading
 
 import torch
-from torch.autograd import Function
+from torch.autograd import Function, forward_ad
 
 from . import _lib as L
 
@@ -268,7 +268,7 @@ def native_sparse_attend(fq, fk, fv, block_size, selected_block_indices, fmask, 
     assert q_heads % kv_heads == 0
     assert sel_heads in (q_heads, kv_heads)
     diag = L.DIAG_CAUSAL if include_block_causal else L.DIAG_NONE
-    if index_cache is None:
+    if index_cache is None and forward_ad._current_level < 0:   # (the Function refuses tensors that carry a tangent)
         L.require_cuda(fq)
         out, lse = L.host().sel_attend(fq, fk, fv, selected_block_indices, fmask, sel_scale, block_size, diag,
                                        L.IMPL_BY_NAME[impl], _status_word(fq.device), REUSE_INDEX)

@@ -180,3 +180,25 @@ def test_kept_gradients_do_not_keep_the_scratch_of_the_backward(dtype):
         assert 'NativeLayer' in out.grad_fn.name()
         sizes.append({name: g.untyped_storage().nbytes() for name, g in grads.items()})
     assert sizes[0] == sizes[1]
+
+
+def test_a_tangent_is_refused_and_not_dropped():
+    from native_sparse_attention_pytorch_b200 import native_sparse_attend
+    layer = SparseAttention(dim=256, dim_head=64, heads=4, kv_heads=2, causal=True, sliding_window_size=70, compress_block_size=32,
+                            compress_block_sliding_stride=16, selection_block_size=64, num_selected_blocks=3, use_triton_kernel=True).to('cuda')
+    x, t = (recipe.randn((1, 130, 256), seed).to('cuda') for seed in (5, 6))
+    q, dq = (recipe.randn((1, 4, 130, 64), seed).to('cuda') for seed in (7, 8))
+    k = recipe.randn((1, 2, 130, 64), 9).to('cuda')
+    idx, mask = torch.zeros(1, 2, 130, 1, dtype=torch.int64, device='cuda'), torch.zeros(1, 2, 130, 1, dtype=torch.bool, device='cuda')
+    fwd = torch.autograd.forward_ad
+    with fwd.dual_level():
+        for grad in (True, False):
+            with torch.set_grad_enabled(grad):
+                with pytest.raises(RuntimeError, match='jvp'):
+                    layer(fwd.make_dual(x, t))
+                with pytest.raises(RuntimeError, match='jvp'):
+                    native_sparse_attend(fwd.make_dual(q, dq), k, k, 64, idx, mask)
+        weight = layer.to_qkv.weight.detach()
+        with pytest.raises(RuntimeError, match='jvp'):
+            torch.func.functional_call(layer, {'to_qkv.weight': fwd.make_dual(weight, weight)}, (x,))
+        assert native_sparse_attend(q, k, k, 64, idx, mask).shape == q.shape

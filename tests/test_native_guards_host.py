@@ -84,3 +84,12 @@ def test_a_step_refuses_caches_of_another_shape(changes):
     """Batch, heads and row length are taken from one tensor and address all others, so each has to agree."""
     with pytest.raises(L.NsaError, match='decode step'):
         L.host().layer_decode(*decode_arguments(build(), **changes))
+
+
+def test_forward_mode_differentiation_takes_the_module_path():
+    """The native calls have no tangents to give; the modules' operators say so."""
+    layer, x = build(), torch.zeros(2, 32, DIM, dtype=BF16)
+    assert layer._native_weights(x) is not None
+    with torch.autograd.forward_ad.dual_level():
+        assert layer._native_weights(x) is None
+    assert layer._native_weights(x) is not None
