@@ -88,8 +88,7 @@ class SparseAttention(Module):
         self.norm = RMSNorm(dim) if norm else nn.Identity()
         self.rotary_emb = RotaryEmbedding(dim_head)
         self.qkv_split = (dim_head * heads, dim_head * kv_heads, dim_head * kv_heads)
-        self._qkv_rows = sum(self.qkv_split)
-        self.to_qkv = nn.Linear(dim, self._qkv_rows, bias=False)
+        self.to_qkv = nn.Linear(dim, sum(self.qkv_split), bias=False)
 
         self.sliding_window_size = sliding_window_size
 
@@ -135,7 +134,8 @@ class SparseAttention(Module):
 
     def _native_weights(self, x):
         """The parameters the native layer calls take, or None where the layer has to run module by module: a replaced
-        or hooked submodule, autocast, forward-mode differentiation (the modules refuse it), parameters of another type, dtype or device than the input, an input or
+        or hooked submodule, a parameter that is not one any more (a wrapper put a plain tensor in its place) or has
+        another shape, autocast, forward-mode differentiation (the modules refuse it), parameters of another type, dtype or device than the input, an input or
         parameters off the 16-byte boundaries the kernels load from."""
         dtype, dim = x.dtype, x.shape[-1]
         if (dtype is not torch.bfloat16 and dtype is not torch.float32) or x.dim() != 3 or torch.is_autocast_enabled('cuda') or \
@@ -147,7 +147,7 @@ class SparseAttention(Module):
         gate_linear = gate._modules.get('0')
         norm_w, eps = None, 0.
         if _untouched(norm, RMSNorm):
-            norm_w, eps = norm._parameters['weight'], norm.eps
+            norm_w, eps = norm._parameters.get('weight'), norm.eps
             if norm_w is None or tuple(norm_w.shape) != (dim,):
                 return None
             eps = _F32_EPS if eps is None else eps
@@ -157,11 +157,10 @@ class SparseAttention(Module):
                 _untouched(gate._modules['1'], nn.Sigmoid) and _untouched(qkv, nn.Linear) and _untouched(out, nn.Linear) and
                 _untouched(gate_linear, nn.Linear)):
             return None
-        if qkv._parameters['bias'] is not None or out._parameters['bias'] is not None:
+        if qkv.bias is not None or out.bias is not None:
             return None
-        gate_w = gate_linear._parameters
-        w = (norm_w, qkv._parameters['weight'], gate_w['weight'], gate_w['bias'], out._parameters['weight'],
-             self._parameters['compress_mem_kv'])
+        w = (norm_w, qkv._parameters.get('weight'), gate_linear._parameters.get('weight'), gate_linear._parameters.get('bias'),
+             out._parameters.get('weight'), self._parameters.get('compress_mem_kv'))
         for p in w:
             if p is None:
                 if p is norm_w:
@@ -169,7 +168,9 @@ class SparseAttention(Module):
                 return None
             if not _takes(p, x):
                 return None
-        if w[1].shape != (self._qkv_rows, dim) or w[2].shape != (3 * self.heads, dim) or dim % 8:
+        h, d = self.heads, self.dim_head
+        if w[1].shape != (sum(self.qkv_split), dim) or w[2].shape != (3 * h, dim) or w[3].shape != (3 * h,) or \
+                w[4].shape != (dim, h * d) or w[5].shape != (2, self.kv_heads, self.num_mem_compress_kv, d) or dim % 8:
             return None
         return w, eps
 
@@ -179,11 +180,12 @@ class SparseAttention(Module):
         if native is None:
             return None
         k_net, v_net = self._default_network('k_compress', x), self._default_network('v_compress', x)
-        pos = (self._parameters['k_intrablock_positions'], self._parameters['v_intrablock_positions'])
+        pos = (self._parameters.get('k_intrablock_positions'), self._parameters.get('v_intrablock_positions'))
         if k_net is None or v_net is None or k_net[0].shape != v_net[0].shape or k_net[0].shape[0] % 8:
             return None
-        if not (_takes(pos[0], x) and _takes(pos[1], x)):
-            return None
+        for p in pos:
+            if p is None or not _takes(p, x) or p.shape != (self.kv_heads, self.compress_block_size, self.dim_head):
+                return None
         w, eps = native
         return (*w, *pos, *k_net, *v_net), eps
 
@@ -225,12 +227,14 @@ class SparseAttention(Module):
         if len(m) != 4 or not (_untouched(m[0], nn.Flatten) and (m[0].start_dim, m[0].end_dim) == (-2, -1) and
                                _untouched(m[1], nn.Linear) and _untouched(m[2], nn.ReLU) and _untouched(m[3], nn.Linear)):
             return None
-        w = (m[1]._parameters['weight'], m[1]._parameters['bias'], m[3]._parameters['weight'], m[3]._parameters['bias'])
+        w = (m[1]._parameters.get('weight'), m[1]._parameters.get('bias'), m[3]._parameters.get('weight'), m[3]._parameters.get('bias'))
         for p in w:
             if p is None or not _takes(p, like):
                 return None
         width = self.compress_block_size * self.dim_head
-        return w if w[0].shape[1] == width and w[2].shape == (self.dim_head, w[0].shape[0]) else None
+        hidden = w[0].shape[0]
+        return w if w[0].shape == (hidden, width) and w[1].shape == (hidden,) and w[2].shape == (self.dim_head, hidden) and \
+            w[3].shape == (self.dim_head,) else None
 
     def _compress_filled(self, ck, cv, run_k, run_v, native=False):
         """The window that was being filled is complete: compress it and keep its overlap with the next one (the step

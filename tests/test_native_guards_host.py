@@ -93,3 +93,38 @@ def test_forward_mode_differentiation_takes_the_module_path():
     with torch.autograd.forward_ad.dual_level():
         assert layer._native_weights(x) is None
     assert layer._native_weights(x) is not None
+
+
+def test_parameters_that_became_plain_tensors_take_the_module_path():
+    """A wrapper that shards parameters may delete them from their modules and put views of its own buffer there."""
+    x = torch.zeros(2, 32, DIM, dtype=BF16)
+    for name, _ in build().named_parameters():
+        layer = build()
+        owner, _, leaf = name.rpartition('.')
+        owner = layer.get_submodule(owner)
+        value = getattr(owner, leaf).detach().clone()
+        delattr(owner, leaf)
+        setattr(owner, leaf, value)
+        assert layer._native_parameters(x) is None, name
+
+
+@pytest.mark.parametrize('name, module', [
+    ('combine_heads', torch.nn.Linear(HEADS * D, 2 * DIM, bias=False)), ('combine_heads', torch.nn.Linear(HEADS * D, DIM)),
+    ('to_qkv', torch.nn.Linear(DIM, (HEADS + 2 * KV_HEADS) * D)), ('to_strategy_combine.0', torch.nn.Linear(DIM, 3 * HEADS, bias=False)),
+    ('k_compress.3', torch.nn.Linear(CBS * D, D, bias=False)), ('v_compress.1', torch.nn.Linear(CBS * D, 2 * CBS * D))])
+def test_replaced_submodules_take_the_module_path(name, module):
+    layer, x = build(), torch.zeros(2, 32, DIM, dtype=BF16)
+    owner, _, leaf = name.rpartition('.')
+    setattr(layer.get_submodule(owner), leaf, module.to(BF16))
+    assert layer._native_parameters(x) is None
+
+
+def test_a_layer_pickled_before_it_had_native_calls_still_runs():
+    layer, x = build(), torch.zeros(2, 32, DIM, dtype=BF16)
+    before = {'heads', 'kv_heads', 'dim_head', 'num_grouped_queries', 'scale', 'causal', 'kernel_impl', 'qkv_split', 'sliding_window_size',
+              'compress_block_size', 'compress_block_sliding_stride', 'num_mem_compress_kv', 'use_diff_topk', 'query_heads_share_selected_kv',
+              'selection_block_size', 'num_selected_blocks', 'use_triton_kernel', 'training'}
+    for name in [n for n in layer.__dict__ if not n.startswith(('_parameters', '_modules', '_buffers', '_backward', '_forward', '_is_full',
+                                                                '_non_persistent', '_state_dict', '_load_state')) and n not in before]:
+        del layer.__dict__[name]
+    assert layer._native_parameters(x) is not None
