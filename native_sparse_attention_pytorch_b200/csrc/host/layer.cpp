@@ -407,14 +407,14 @@ static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor>
     return kept.narrow(0, off, n * (int64_t)c10::elementSize(t)).view(t).view(sizes);
   };
 
-  // fp32 accumulators, cleared together: dk, dv; dck, dcv; then the small gradients that end up in the layer's type.  An
+  // fp32 accumulators, cleared together: dk, dv; dck, dcv; (counters); then the small gradients that end up in the layer's type.  An
   // fp32 layer returns the small ones as they are: there they have memory of their own, a gradient that a program keeps
   // must not keep the scratch of dk and dv with it.
   const int64_t pos = hkv * c.cbs * d, mems = hkv * c.num_mem * d, hid = w.k1.size(0);
   auto even = [](int64_t n) { return (n + 7) / 8 * 8; };
   const int64_t s_norm = 0, s_gate = s_norm + even(L.dim), s_mem = s_gate + even(3 * H), s_pos = s_mem + even(2 * mems),
                 s_b1 = s_pos + even(2 * pos), s_b2 = s_b1 + even(2 * hid), s_end = s_b2 + even(2 * d);
-  const int64_t a_small = even(2 * k_elems + 2 * c_elems);
+  const int64_t a_counters = 2 * k_elems + 2 * c_elems, a_small = even(a_counters + nsa::gate_sums_counters((int)(3 * H)));
   const bool apart = type == at::kFloat;
   Tensor acc = empty({apart ? a_small : a_small + s_end}, x, at::kFloat);
   Tensor rounded = apart ? empty({s_end}, x, at::kFloat) : Tensor();
@@ -429,6 +429,7 @@ static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor>
   const Tensor d_merged = product(Op::NN, dout, w.out);
   Slab tmp;
   const int64_t t_do = tmp.add(3 * q_bytes), t_delta = tmp.add(3 * L.rows(H) * 4), t_dq = tmp.add(3 * q_elems * 4);
+  const int64_t t_gates = tmp.add(nsa::gate_sums_partial((int)(3 * H)) * 4);
   tmp.allocate(x);
   const Tensor d_logits = at::empty({BN, 3 * H}, x.options());
   {
@@ -522,7 +523,7 @@ static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor>
     p.x[0] = dhk.data_ptr(); p.x[1] = dhv.data_ptr(); p.act[0] = hk.data_ptr(); p.act[1] = hv.data_ptr();
     p.out[0] = small + s_b1; p.out[1] = small + s_b1 + hid;
     p.rows = wins; p.cols = hid; p.sets = 2;
-    check(nsa::launch_column_sums(p, L.dt, st));
+    check(nsa::launch_relu_sums(p, L.dt, st));
   }
   std::vector<OptTensor> g(1 + kWeights);
   const Tensor kw = kept_view(at_win, {wins, width}, type), vw = kept_view(at_win + wins * width * el, {wins, width}, type);
@@ -537,11 +538,8 @@ static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor>
   const Tensor d_qkv = at::empty({BN, L.F}, x.options());
   qg.dk = dk; qg.dv = dk + k_elems; qg.dkw = dkw.data_ptr(); qg.dvw = dvw.data_ptr(); qg.inv_freq = ptr<float>(inv_freq); qg.out = d_qkv.data_ptr();
   check(nsa::launch_qkv_grad(L.shape, qg, L.dt, st));
-  {
-    nsa::ColumnSums p = {};
-    p.x[0] = d_logits.data_ptr(); p.out[0] = small + s_gate; p.rows = BN; p.cols = 3 * H; p.sets = 1;
-    check(nsa::launch_column_sums(p, L.dt, st));
-  }
+  check(nsa::launch_gate_sums(d_logits.data_ptr(), small + s_gate, BN, (int)(3 * H), reinterpret_cast<float*>(tmp.at(t_gates)),
+                              reinterpret_cast<unsigned*>(dk + a_counters), L.dt, st));
   if (needs[5]) g[5] = product(Op::TN, dout, merged);
   if (needs[2]) g[2] = product(Op::TN, d_qkv, xn);
   if (needs[3]) g[3] = product(Op::TN, d_logits, xn);

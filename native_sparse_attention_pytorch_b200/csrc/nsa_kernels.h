@@ -152,7 +152,7 @@ struct LayerPrep {
   void *kw, *vw;                     // [B, Hkv, ncb, cbs, d]
 };
 struct ColumnSums {
-  void* x[2];                        // [rows, cols], masked in place where `act` is given
+  void* x[2];                        // [rows, cols], masked in place
   const void* act[2];
   float* out[2];                     // added to
   int64_t rows;
@@ -183,7 +183,10 @@ int launch_combine_gather(const CombineParams& P, const GatherTargets& Gt, int d
 int launch_layer_prep(const LayerShape& L, const LayerPrep& P, int dtype, cudaStream_t stream);
 int launch_join_mem(const LayerShape& L, const void* mem, const void* ck, const void* cv, void* out, int dtype, cudaStream_t stream);
 int launch_split_mem(const LayerShape& L, const float* grad, void* dc, float* dmem, float* dbias, int dtype, cudaStream_t stream);
-int launch_column_sums(const ColumnSums& P, int dtype, cudaStream_t stream);
+int launch_relu_sums(const ColumnSums& P, int dtype, cudaStream_t stream);
+int64_t gate_sums_partial(int cols);    // floats
+int gate_sums_counters(int cols);       // zero before the call
+int launch_gate_sums(const void* x, float* out, int64_t rows, int cols, float* partial, unsigned* arrived, int dtype, cudaStream_t stream);
 int launch_qkv_grad(const LayerShape& L, const QkvGrad& P, int dtype, cudaStream_t stream);
 int launch_pos_grad(const LayerShape& L, const void* dkw, const void* dvw, float* dpos, int dtype, cudaStream_t stream);
 int launch_round(const float* src, void* dst, int64_t n, cudaStream_t stream);

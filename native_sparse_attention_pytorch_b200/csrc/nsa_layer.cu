@@ -194,10 +194,12 @@ int launch_split_mem(const LayerShape& L, const float* grad, void* dc, float* dm
   return err == cudaSuccess ? NSA_OK : fail((int)err, cudaGetErrorString(err));
 }
 
-// ---- column sums (bias gradients), optionally behind the ReLU whose output is `act`: x = act > 0 ? x : 0 in place.
-// A block owns 32 sixteen-byte columns and a slice of the rows; sets side by side in blockIdx.z.
-template <typename T, bool RELU>
-__global__ void __launch_bounds__(256) column_sums_kernel(const ColumnSums P) {
+// ---- column sums (the bias of the first compress layer) behind the ReLU whose output is `act`: x = act > 0 ? x : 0 in
+// place.  A block owns 32 sixteen-byte columns and a slice of the rows; sets side by side in blockIdx.z.  The slices meet in
+// float atomics, as those of split_mem_kernel and pos_grad_kernel do: the last bits of these sums differ from run to run,
+// like those of dk and dv behind them (fp32 reductions of the attention kernels).
+template <typename T>
+__global__ void __launch_bounds__(256) relu_sums_kernel(const ColumnSums P) {
   constexpr int V = Vec<T>::V;
   __shared__ float fold[8][32 * V];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, set = blockIdx.z;
@@ -210,17 +212,15 @@ __global__ void __launch_bounds__(256) column_sums_kernel(const ColumnSums P) {
     const int64_t step = (int64_t)gridDim.y * 8;
     int64_t r = (int64_t)blockIdx.y * 8 + warp;
     for (; r < P.rows; r += step) {
-      Vec<T> v;
+      Vec<T> v, a;
       v.load(x + r * P.cols + col);
-      if (RELU) {
-        Vec<T> a;
-        a.load(act + r * P.cols + col);
+      a.load(act + r * P.cols + col);
 #pragma unroll
-        for (int i = 0; i < V; ++i) v.x[i] = a.x[i] > 0.f ? v.x[i] : 0.f;
-        v.store(x + r * P.cols + col);
+      for (int i = 0; i < V; ++i) {
+        v.x[i] = a.x[i] > 0.f ? v.x[i] : 0.f;
+        sum.x[i] += v.x[i];
       }
-#pragma unroll
-      for (int i = 0; i < V; ++i) sum.x[i] += v.x[i];
+      v.store(x + r * P.cols + col);
     }
   }
 #pragma unroll
@@ -237,44 +237,96 @@ __global__ void __launch_bounds__(256) column_sums_kernel(const ColumnSums P) {
   }
 }
 
-// The same for matrices whose rows are not whole 16-byte pieces (the gates of a few heads): a thread owns one column.
-template <typename T>
-__global__ void __launch_bounds__(256) narrow_sums_kernel(const ColumnSums P) {
-  const int width = min(256, P.cols - (int)blockIdx.x * 256), lane_rows = 256 / width;
-  const int c = blockIdx.x * 256 + threadIdx.x % width, r0 = threadIdx.x / width;
-  if (r0 >= lane_rows) return;
-  const T* x = (const T*)P.x[blockIdx.z];
-  float sum = 0.f;
-#pragma unroll 4
-  for (int64_t r = (int64_t)blockIdx.y * lane_rows + r0; r < P.rows; r += (int64_t)gridDim.y * lane_rows) sum += Elem<T>::to_float(x[r * P.cols + c]);
-  atomicAdd(P.out[blockIdx.z] + c, sum);
-}
-
-int launch_column_sums(const ColumnSums& P, int dtype, cudaStream_t stream) {
+int launch_relu_sums(const ColumnSums& P, int dtype, cudaStream_t stream) {
   if (P.rows == 0 || P.cols == 0) return NSA_OK;
   const int V = dtype == NSA_F32 ? 4 : 8;
+  if (P.cols % V) return fail(NSA_ERR_ALIGN, "column sums behind a ReLU need rows of whole 16-byte pieces");
   const int gx = (P.cols / V + 31) / 32;
   int64_t gy = 148 * 4 / ((int64_t)gx * P.sets) + 1;              // about four blocks per SM: every block ends in atomics
   const int64_t most = (P.rows + 15) / 16;
   gy = gy < most ? gy : most;
   const dim3 grid((unsigned)gx, (unsigned)(gy < 65535 ? gy : 65535), (unsigned)P.sets);
-  const bool relu = P.act[0] != nullptr;
-  if (P.cols % V) {
-    if (relu) return fail(NSA_ERR_ALIGN, "column sums behind a ReLU need rows of whole 16-byte pieces");
-    const int64_t slices = (P.rows * P.cols + 2047) / 2048;
-    const dim3 ngrid((unsigned)((P.cols + 255) / 256), (unsigned)(slices < 148 * 2 ? slices : 148 * 2), (unsigned)P.sets);
-    if (dtype == NSA_F32) narrow_sums_kernel<float><<<ngrid, 256, 0, stream>>>(P);
-    else narrow_sums_kernel<__nv_bfloat16><<<ngrid, 256, 0, stream>>>(P);
-    count_launches(1);
-    const cudaError_t nerr = cudaGetLastError();
-    return nerr == cudaSuccess ? NSA_OK : fail((int)nerr, cudaGetErrorString(nerr));
+  if (dtype == NSA_F32) relu_sums_kernel<float><<<grid, 256, 0, stream>>>(P);
+  else relu_sums_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(P);
+  count_launches(1);
+  const cudaError_t err = cudaGetLastError();
+  return err == cudaSuccess ? NSA_OK : fail((int)err, cudaGetErrorString(err));
+}
+
+// ---- column sums of the gates' gradient (their bias), in a fixed order: nothing before them depends on the order of
+// atomics, so their bits repeat from run to run, and must not be lost here.  A block sums a slice of the rows of up to 256
+// columns, VEC at a time per thread (one where a row is not whole 16-byte pieces), and leaves its part in `partial`; the
+// block that arrives last adds the slices up in their order.  Up to 64 slices: the last block reads them all.
+// `arrived`: one counter per 256 columns, zero.
+constexpr int kGateSlices = 64;
+template <typename T, int VEC>
+__global__ void __launch_bounds__(256) gate_sums_kernel(const T* x, float* out, int64_t rows, int cols, float* partial, unsigned* arrived) {
+  __shared__ float fold[256 * VEC];
+  __shared__ bool last;
+  const int c0 = blockIdx.x * 256, width = min(256, cols - c0), units = width / VEC;
+  const int tid = threadIdx.x, u = tid % units, r0 = tid / units, step = 256 / units;
+  float sum[VEC];
+#pragma unroll
+  for (int i = 0; i < VEC; ++i) sum[i] = 0.f;
+  if (r0 < step) {
+    const int64_t per = (rows + gridDim.y - 1) / gridDim.y, end = min(rows, (blockIdx.y + 1) * per);
+#pragma unroll 4
+    for (int64_t r = blockIdx.y * per + r0; r < end; r += step) {
+      const T* at = x + r * cols + c0 + u * VEC;
+      if constexpr (VEC == 1) {
+        sum[0] += Elem<T>::to_float(*at);
+      } else {
+        float v[VEC];
+        Elem<T>::load_vec(at, v);
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) sum[i] += v[i];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) fold[r0 * width + u * VEC + i] = sum[i];
   }
+  __syncthreads();
+  if (tid < width) {
+    float s = 0.f;
+    for (int k = 0; k < step; ++k) s += fold[k * width + tid];
+    partial[(int64_t)blockIdx.y * cols + c0 + tid] = s;
+  }
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) last = atomicAdd(arrived + blockIdx.x, 1u) == gridDim.y - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const int groups = 256 / width, c = tid % width, g = tid / width;
+  float s = 0.f;
+  if (g < groups) {
+#pragma unroll 8
+    for (int y = g; y < (int)gridDim.y; y += groups) s += __ldcg(partial + (int64_t)y * cols + c0 + c);
+    fold[g * width + c] = s;
+  }
+  __syncthreads();
+  if (tid < width) {
+    s = 0.f;
+    for (int k = 0; k < groups; ++k) s += fold[k * width + tid];
+    out[c0 + tid] = s;
+  }
+}
+
+int64_t gate_sums_partial(int cols) { return (int64_t)kGateSlices * cols; }
+int gate_sums_counters(int cols) { return (cols + 255) / 256; }
+
+int launch_gate_sums(const void* x, float* out, int64_t rows, int cols, float* partial, unsigned* arrived, int dtype, cudaStream_t stream) {
+  if (rows == 0 || cols == 0) return NSA_OK;
+  const int V = dtype == NSA_F32 ? 4 : 8;
+  const int64_t slices = (rows * cols + 2047) / 2048;
+  const dim3 grid((unsigned)gate_sums_counters(cols), (unsigned)(slices < kGateSlices ? slices : kGateSlices));
+  const bool vec = cols % V == 0 && aligned16(x);
   if (dtype == NSA_F32) {
-    if (relu) column_sums_kernel<float, true><<<grid, 256, 0, stream>>>(P);
-    else column_sums_kernel<float, false><<<grid, 256, 0, stream>>>(P);
+    if (vec) gate_sums_kernel<float, 4><<<grid, 256, 0, stream>>>((const float*)x, out, rows, cols, partial, arrived);
+    else gate_sums_kernel<float, 1><<<grid, 256, 0, stream>>>((const float*)x, out, rows, cols, partial, arrived);
   } else {
-    if (relu) column_sums_kernel<__nv_bfloat16, true><<<grid, 256, 0, stream>>>(P);
-    else column_sums_kernel<__nv_bfloat16, false><<<grid, 256, 0, stream>>>(P);
+    if (vec) gate_sums_kernel<__nv_bfloat16, 8><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)x, out, rows, cols, partial, arrived);
+    else gate_sums_kernel<__nv_bfloat16, 1><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)x, out, rows, cols, partial, arrived);
   }
   count_launches(1);
   const cudaError_t err = cudaGetLastError();

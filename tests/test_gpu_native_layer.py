@@ -202,3 +202,25 @@ def test_a_tangent_is_refused_and_not_dropped():
         with pytest.raises(RuntimeError, match='jvp'):
             torch.func.functional_call(layer, {'to_qkv.weight': fwd.make_dual(weight, weight)}, (x,))
         assert native_sparse_attend(q, k, k, 64, idx, mask).shape == q.shape
+
+
+# one slice and many, one and several groups of 256 columns, rows of whole 16-byte pieces and not
+@pytest.mark.parametrize('b, n, heads, d, dtype', [(1, 40, 2, 64, F32), (2, 4096, 8, 64, F32), (5, 700, 6, 40, F32), (2, 2000, 96, 8, BF16)])
+def test_the_gradient_of_the_gate_bias_repeats_to_the_bit(b, n, heads, d, dtype):
+    """Nothing in front of it depends on the order of atomics."""
+    layer = SparseAttention(dim=256, dim_head=d, heads=heads, kv_heads=heads // 2, causal=True, sliding_window_size=70, compress_block_size=32,
+                            compress_block_sliding_stride=16, selection_block_size=64, num_selected_blocks=3, use_triton_kernel=True)
+    recipe.fill_weights(layer, seed=3)
+    layer = layer.to('cuda').to(dtype)
+    x, dout = (recipe.randn((b, n, 256), seed).to(dtype).to('cuda') for seed in (5, 6))
+    out, _, grads = run(layer, x, dout)
+    assert 'NativeLayer' in out.grad_fn.name()
+    hook = layer.combine_heads.register_forward_hook(lambda *_: None)
+    _, _, want = run(layer, x, dout)
+    hook.remove()
+    for name in ('to_strategy_combine.0.bias', 'k_compress.1.bias'):
+        if dtype == F32:
+            assert_close_f32(grads[name], want[name], name)
+    for _ in range(4):
+        _, _, again = run(layer, x, dout)
+        assert torch.equal(again['to_strategy_combine.0.bias'], grads['to_strategy_combine.0.bias'])
