@@ -140,10 +140,16 @@ static std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> layer_decode(
 
 // The windows being filled (keys, values: [B, H, cbs, d]) have filled up: the two layers of either compress network, each
 // one launch for both, and the compressed row appended to ck / cv.  -> ck, cv, or nothing where these kernels do not serve.
-static std::optional<std::tuple<Tensor, Tensor>> compress_filled(Tensor run_k, Tensor run_v, Tensor pos_k, Tensor pos_v,
+static std::optional<std::tuple<Tensor, Tensor>> compress_filled(Tensor run_k, Tensor run_v, OptTensor pos_k, OptTensor pos_v,
                                                                  Tensor k1, Tensor kb1, Tensor k2, Tensor kb2, Tensor v1,
                                                                  Tensor vb1, Tensor v2, Tensor vb2, Tensor ck, Tensor cv) {
   const int64_t B = run_k.size(0), H = run_k.size(1), d = run_k.size(3), width = run_k.size(2) * d, hidden = k1.size(0);
+  for (const OptTensor& p : {pos_k, pos_v})
+    if (!fits(p, run_k, {H, run_k.size(2), d})) return std::nullopt;
+  for (const auto& net : {std::make_tuple(k1, kb1, k2, kb2), std::make_tuple(v1, vb1, v2, vb2)})
+    if (!fits(std::get<0>(net), run_k, {hidden, width}) || !fits(std::get<1>(net), run_k, {hidden}) || !fits(std::get<2>(net), run_k, {d, hidden}) ||
+        !fits(std::get<3>(net), run_k, {d}))
+      return std::nullopt;
   check_compressed(ck, cv, B, H, d);
   const int dt = dtype_code(run_k);
   if (!nsa::project_serves(B * H, width, dt) || !nsa::project_serves(B * H, hidden, dt) || run_k.stride(2) != d ||
@@ -155,7 +161,7 @@ static std::optional<std::tuple<Tensor, Tensor>> compress_filled(Tensor run_k, T
   Tensor h = at::empty({2, B * H, hidden}, run_k.options());
   nsa::ProjectParams p = {};
   p.x[0] = run_k.data_ptr(); p.x[1] = run_v.data_ptr(); p.x_sb = run_k.stride(0); p.x_sh = run_k.stride(1);
-  p.add[0] = pos_k.data_ptr(); p.add[1] = pos_v.data_ptr();
+  p.add[0] = pos_k->data_ptr(); p.add[1] = pos_v->data_ptr();
   p.w[0] = k1.data_ptr(); p.w[1] = v1.data_ptr(); p.bias[0] = kb1.data_ptr(); p.bias[1] = vb1.data_ptr();
   p.y[0] = h.data_ptr(); p.y[1] = static_cast<uint8_t*>(h.data_ptr()) + B * H * hidden * h.element_size();
   p.y_sb = H * hidden; p.y_sh = hidden;

@@ -41,6 +41,24 @@ static LayerWeights weights_of(const std::vector<OptTensor>& w) {
 }
 constexpr int kWeights = 16;
 
+// Can the native calls take this input and these parameters (all, or the first six for a decoding step)?
+static bool layer_takes(const Tensor& x, const std::vector<OptTensor>& w, int64_t heads, int64_t kv_heads, int64_t d, int64_t cbs, int64_t num_mem) {
+  if (x.dim() != 3 || !x.has_storage() || reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 || x.size(2) % 8) return false;
+  const int64_t dim = x.size(2);
+  if (w.at(0).has_value() && !fits(w[0], x, {dim})) return false;
+  if (!fits(w.at(1), x, {(heads + 2 * kv_heads) * d, dim}) || !fits(w.at(2), x, {3 * heads, dim}) || !fits(w.at(3), x, {3 * heads}) ||
+      !fits(w.at(4), x, {dim, heads * d}) || !fits(w.at(5), x, {2, kv_heads, num_mem, d}))
+    return false;
+  if (w.size() == 6) return true;
+  if (!w.at(8).has_value() || w[8]->dim() != 2) return false;
+  const int64_t hidden = w[8]->size(0);
+  for (int s = 0; s < 2; ++s)
+    if (!fits(w.at(6 + s), x, {kv_heads, cbs, d}) || !fits(w.at(8 + 4 * s), x, {hidden, cbs * d}) || !fits(w.at(9 + 4 * s), x, {hidden}) ||
+        !fits(w.at(10 + 4 * s), x, {d, hidden}) || !fits(w.at(11 + 4 * s), x, {d}))
+      return false;
+  return hidden % 8 == 0;
+}
+
 // Row-major GEMMs, C [M, N] = (beta C +) op(A) op(B), on the library and with the settings at::mm uses, without the
 // tensor views and the dispatch around them (8 us of host time per product; a training step has 17).
 enum class Op { NT, NN, TN };   // A [M, K], B [N, K];  A [M, K], B [K, N];  A [K, M], B [K, N]
@@ -696,6 +714,7 @@ static Tensor layer_apply(Tensor x, std::vector<OptTensor> weights, double eps, 
 
 void bind_layer(pybind11::module_& m) {
   namespace py = pybind11;
+  m.def("layer_takes", &layer_takes);
   m.def("layer_forward", &layer_forward, py::call_guard<py::gil_scoped_release>());
   m.def("layer_apply", &layer_apply, py::call_guard<py::gil_scoped_release>());
 }

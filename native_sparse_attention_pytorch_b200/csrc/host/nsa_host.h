@@ -54,6 +54,13 @@ inline Tensor rowwise(const Tensor& t) {
   return ok ? t : t.contiguous();
 }
 
+// A parameter the kernels can read as it is next to activations x: of these sizes, of x's type and device, dense, and on the
+// 16-byte boundary their loads need (a view into a flat buffer of many parameters often is not)
+inline bool fits(const OptTensor& t, const Tensor& x, at::IntArrayRef sizes) {
+  return t.has_value() && t->defined() && t->has_storage() && t->scalar_type() == x.scalar_type() && t->device() == x.device() &&
+         t->sizes() == sizes && t->is_contiguous() && reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0;
+}
+
 inline nsa_tensor t4(const Tensor& t) { return {t.data_ptr(), t.stride(0), t.stride(1), t.stride(2)}; }
 inline nsa_tensor no_tensor() { return {nullptr, 0, 0, 0}; }
 

@@ -26,11 +26,12 @@ _F32_EPS = torch.finfo(torch.float32).eps
 _PLAIN = (nn.Parameter, torch.Tensor)
 
 
-def _takes(p, like):
-    """The native kernels can read parameter `p` next to activations `like`: same type and device, dense, and on the
-    16-byte boundary their loads need (a view into a flat buffer of many parameters often is not)."""
-    return p.dtype is like.dtype and p.device == like.device and p.is_contiguous() and p.__class__ in _PLAIN and \
-        not p.data_ptr() & 15
+def _plain(*params):
+    """All are tensors of the ordinary classes (a parameter that is missing is not)."""
+    for p in params:
+        if p.__class__ not in _PLAIN:
+            return False
+    return True
 
 
 def _untouched(module, cls):
@@ -134,13 +135,11 @@ class SparseAttention(Module):
 
     def _native_weights(self, x):
         """The parameters the native layer calls take, or None where the layer has to run module by module: a replaced
-        or hooked submodule, a parameter that is not one any more (a wrapper put a plain tensor in its place) or has
-        another shape, autocast, forward-mode differentiation (the modules refuse it), parameters of another type, dtype or device than the input, an input or
-        parameters off the 16-byte boundaries the kernels load from."""
-        dtype, dim = x.dtype, x.shape[-1]
-        if (dtype is not torch.bfloat16 and dtype is not torch.float32) or x.dim() != 3 or torch.is_autocast_enabled('cuda') or \
-                _has_any_global_hook() or torch.compiler.is_compiling() or forward_ad._current_level >= 0 or \
-                x.data_ptr() & 15:
+        or hooked submodule, a parameter that is not one any more (a wrapper put a plain tensor in its place), autocast,
+        forward-mode differentiation (the modules refuse it).  Whether the calls can take them as they are is for
+        `layer_takes` to say."""
+        if (x.dtype is not torch.bfloat16 and x.dtype is not torch.float32) or torch.is_autocast_enabled('cuda') or \
+                _has_any_global_hook() or torch.compiler.is_compiling() or forward_ad._current_level >= 0:
             return None
         m = self._modules
         norm, gate, qkv, out = m['norm'], m['to_strategy_combine'], m['to_qkv'], m['combine_heads']
@@ -148,7 +147,7 @@ class SparseAttention(Module):
         norm_w, eps = None, 0.
         if _untouched(norm, RMSNorm):
             norm_w, eps = norm._parameters.get('weight'), norm.eps
-            if norm_w is None or tuple(norm_w.shape) != (dim,):
+            if not _plain(norm_w):
                 return None
             eps = _F32_EPS if eps is None else eps
         elif not _untouched(norm, nn.Identity):
@@ -159,35 +158,23 @@ class SparseAttention(Module):
             return None
         if qkv.bias is not None or out.bias is not None:
             return None
-        w = (norm_w, qkv._parameters.get('weight'), gate_linear._parameters.get('weight'), gate_linear._parameters.get('bias'),
+        w = (qkv._parameters.get('weight'), gate_linear._parameters.get('weight'), gate_linear._parameters.get('bias'),
              out._parameters.get('weight'), self._parameters.get('compress_mem_kv'))
-        for p in w:
-            if p is None:
-                if p is norm_w:
-                    continue
-                return None
-            if not _takes(p, x):
-                return None
-        h, d = self.heads, self.dim_head
-        if w[1].shape != (sum(self.qkv_split), dim) or w[2].shape != (3 * h, dim) or w[3].shape != (3 * h,) or \
-                w[4].shape != (dim, h * d) or w[5].shape != (2, self.kv_heads, self.num_mem_compress_kv, d) or dim % 8:
-            return None
-        return w, eps
+        return ((norm_w, *w), eps) if _plain(*w) else None
+
+    def _layer_takes(self, x, weights):
+        return L.host().layer_takes(x, weights, self.heads, self.kv_heads, self.dim_head, self.compress_block_size, self.num_mem_compress_kv)
 
     def _native_parameters(self, x):
-        """All parameters of a native layer call, in its order, and the norm's epsilon; or None as `_native_weights`."""
-        native = self._native_weights(x)
-        if native is None:
-            return None
-        k_net, v_net = self._default_network('k_compress', x), self._default_network('v_compress', x)
+        """All parameters of a native layer call, in its order, and the norm's epsilon; or None where the layer has to run
+        module by module (`_native_weights`, another compress network, or an input or parameters that do not fit: of another
+        type, device or shape, or off the 16-byte boundaries the kernels load from)."""
+        native, k_net, v_net = self._native_weights(x), self._default_network('k_compress'), self._default_network('v_compress')
         pos = (self._parameters.get('k_intrablock_positions'), self._parameters.get('v_intrablock_positions'))
-        if k_net is None or v_net is None or k_net[0].shape != v_net[0].shape or k_net[0].shape[0] % 8:
+        if native is None or k_net is None or v_net is None or not _plain(*pos):
             return None
-        for p in pos:
-            if p is None or not _takes(p, x) or p.shape != (self.kv_heads, self.compress_block_size, self.dim_head):
-                return None
-        w, eps = native
-        return (*w, *pos, *k_net, *v_net), eps
+        weights = (*native[0], *pos, *k_net, *v_net)
+        return (weights, native[1]) if self._layer_takes(x, weights) else None
 
     def _native_layer(self, x, return_cache):
         """The whole forward natively, or None where the layer has to run module by module (a chosen kernel family, a
@@ -219,31 +206,24 @@ class SparseAttention(Module):
         b, n, _ = t.shape
         return t.view(b, n, -1, self.dim_head).transpose(1, 2)   # a view: the kernels take the strides
 
-    def _default_network(self, name, like):
-        """The parameters (two linear layers) of a compress network that is the default one, as built and of `like`'s
-        type, else None."""
+    def _default_network(self, name):
+        """The parameters (two linear layers) of a compress network that is the default one, as built, else None."""
         net = self._modules[name]
         m = list(net._modules.values()) if _untouched(net, nn.Sequential) else ()
         if len(m) != 4 or not (_untouched(m[0], nn.Flatten) and (m[0].start_dim, m[0].end_dim) == (-2, -1) and
                                _untouched(m[1], nn.Linear) and _untouched(m[2], nn.ReLU) and _untouched(m[3], nn.Linear)):
             return None
         w = (m[1]._parameters.get('weight'), m[1]._parameters.get('bias'), m[3]._parameters.get('weight'), m[3]._parameters.get('bias'))
-        for p in w:
-            if p is None or not _takes(p, like):
-                return None
-        width = self.compress_block_size * self.dim_head
-        hidden = w[0].shape[0]
-        return w if w[0].shape == (hidden, width) and w[1].shape == (hidden,) and w[2].shape == (self.dim_head, hidden) and \
-            w[3].shape == (self.dim_head,) else None
+        return w if _plain(*w) else None
 
     def _compress_filled(self, ck, cv, run_k, run_v, native=False):
         """The window that was being filled is complete: compress it and keep its overlap with the next one (the step
         before attended the blocks that existed before this token, as upstream's does)."""
         grown = None
         pk, pv = self.k_intrablock_positions, self.v_intrablock_positions
-        if native and _takes(pk, run_k) and _takes(pv, run_k):
-            k_net, v_net = self._default_network('k_compress', run_k), self._default_network('v_compress', run_k)
-            if k_net is not None and v_net is not None:
+        if native:
+            k_net, v_net = self._default_network('k_compress'), self._default_network('v_compress')
+            if k_net is not None and v_net is not None and _plain(pk, pv):
                 grown = L.host().compress_filled(run_k, run_v, pk, pv, *k_net, *v_net, ck, cv)
         if grown is not None:
             ck, cv = grown
@@ -264,7 +244,7 @@ class SparseAttention(Module):
         if x.shape[1] != 1 or d % 8 or d > 128 or self.num_selected_blocks > 32 or self.num_grouped_queries > 16:
             return None
         native = self._native_weights(x)
-        if native is None:
+        if native is None or not self._layer_takes(x, native[0]):
             return None
         for t in (past_k, past_v, ck, cv, run_k, run_v):
             if t.dtype is not x.dtype or t.device != x.device or t.__class__ is not torch.Tensor:

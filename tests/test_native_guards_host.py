@@ -56,8 +56,8 @@ def test_parameters_packed_into_one_buffer(dtype):
 
 def test_an_input_at_an_odd_offset_takes_the_module_path():
     layer, x = build(), torch.zeros(1, 32, DIM, dtype=BF16)
-    assert layer._native_weights(x) is not None
-    assert layer._native_weights(off_by(x, 1)) is None
+    assert layer._native_parameters(x) is not None
+    assert layer._native_parameters(off_by(x, 1)) is None
 
 
 def decode_arguments(layer, **changes):
@@ -113,10 +113,13 @@ def test_parameters_that_became_plain_tensors_take_the_module_path():
     ('to_qkv', torch.nn.Linear(DIM, (HEADS + 2 * KV_HEADS) * D)), ('to_strategy_combine.0', torch.nn.Linear(DIM, 3 * HEADS, bias=False)),
     ('k_compress.3', torch.nn.Linear(CBS * D, D, bias=False)), ('v_compress.1', torch.nn.Linear(CBS * D, 2 * CBS * D))])
 def test_replaced_submodules_take_the_module_path(name, module):
-    layer, x = build(), torch.zeros(2, 32, DIM, dtype=BF16)
-    owner, _, leaf = name.rpartition('.')
-    setattr(layer.get_submodule(owner), leaf, module.to(BF16))
-    assert layer._native_parameters(x) is None
+    x = torch.zeros(2, 32, DIM, dtype=BF16)
+    for norm in (True, False):
+        layer = build(norm=norm)
+        assert layer._native_parameters(x) is not None
+        owner, _, leaf = name.rpartition('.')
+        setattr(layer.get_submodule(owner), leaf, module.to(BF16))
+        assert layer._native_parameters(x) is None
 
 
 def test_a_layer_pickled_before_it_had_native_calls_still_runs():
