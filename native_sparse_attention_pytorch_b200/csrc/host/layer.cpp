@@ -179,11 +179,10 @@ struct Layer {
     a.window = c.window; a.causal = c.causal; a.dtype = dt; a.scale = scale; a.status = status;
     return a;
   }
-  nsa::CombineParams combine_params(void* o, const void* logits) const {
+  nsa::CombineParams combine_params(void* const (&outs)[3], const void* logits) const {
     nsa::CombineParams p = {};
-    const int64_t part = rows(c.heads) * c.d * el;
     for (int s = 0; s < 3; ++s) {
-      p.o[s] = static_cast<uint8_t*>(o) + s * part;
+      p.o[s] = outs[s];
       p.o_sb[s] = c.heads * N * c.d; p.o_sh[s] = N * c.d; p.o_sn[s] = c.d;
     }
     p.gates = logits; p.g_sb = N * 3 * c.heads; p.g_sh = 3; p.g_sn = 3 * c.heads;
@@ -236,6 +235,7 @@ static std::vector<OptTensor> layer_forward(Tensor x, std::vector<OptTensor> wei
   }
   const Tensor qkv = product(Op::NT, xn, w.qkv);
   const Tensor logits = at::addmm(w.gate_b, xn, w.gate.t());
+  if (!save) xn = Tensor();   // here and below: what nobody needs any more makes room for the partial results
 
   // kept for the backward (or until the end of this call): rotated q, compressed keys and values, branch outputs, ...
   const int64_t q_bytes = L.rows(c.heads) * d * el, k_bytes = L.rows(hkv) * d * el, kv = c.num_mem + L.ncb;
@@ -243,10 +243,14 @@ static std::vector<OptTensor> layer_forward(Tensor x, std::vector<OptTensor> wei
   const int64_t at_qr = keep.add(q_bytes), at_kr = keep.add(k_bytes);
   const int64_t at_win = keep.add(2 * B * hkv * L.ncb * c.cbs * d * el);
   const int64_t at_ckv = keep.add(2 * B * hkv * kv * d * el);
-  const int64_t at_o = keep.add(3 * q_bytes), at_lse = keep.add(3 * L.rows(c.heads) * 4);
+  const int64_t at_o = keep.add((save ? 3 : 2) * q_bytes), at_lse = keep.add(3 * L.rows(c.heads) * 4);
   const int64_t picks = L.rows(L.hs) * L.k_sel;
   const int64_t at_idx = keep.add(picks * 8), at_mask = keep.add(picks);
   keep.allocate(x);
+  // branch outputs: compressed, selected, sliding; without a backward the selected one is only needed where the merge does
+  // not do the combine
+  uint8_t* const o = keep.at(at_o);
+  void* outs[3] = {o, save ? o + q_bytes : nullptr, o + (save ? 2 : 1) * q_bytes};
   void* const qr = keep.at(at_qr);
   float* const lse = reinterpret_cast<float*>(keep.at(at_lse));
 
@@ -270,18 +274,18 @@ static std::vector<OptTensor> layer_forward(Tensor x, std::vector<OptTensor> wei
   // compress networks: Linear, ReLU, Linear over each window
   const int64_t wins = B * hkv * L.ncb, width = c.cbs * d;
   const Tensor kw = keep.view(at_win, {wins, width}, type), vw = keep.view(at_win + win_half, {wins, width}, type);
-  const Tensor hk = at::_addmm_activation(w.kb1, kw, w.k1.t()), hv = at::_addmm_activation(w.vb1, vw, w.v1.t());
+  Tensor hk = at::_addmm_activation(w.kb1, kw, w.k1.t()), hv = at::_addmm_activation(w.vb1, vw, w.v1.t());
   const Tensor ck = at::addmm(w.kb2, hk, w.k2.t()), cv = at::addmm(w.vb2, hv, w.v2.t());
+  if (!save) hk = hv = Tensor();
   void* const ckv = keep.at(at_ckv);
   check(nsa::launch_join_mem(L.shape, w.mem.data_ptr(), ck.data_ptr(), cv.data_ptr(), ckv, L.dt, st));
 
   // compressed branch; its logits rank the blocks
-  uint8_t* const o = keep.at(at_o);
   int64_t* const idx = reinterpret_cast<int64_t*>(keep.at(at_idx));
   uint8_t* const mask = keep.at(at_mask);
   Tensor importance;
   {
-    nsa_cmp_fwd_args a = L.cmp_args(qkv.data_ptr(), ckv, o, lse);
+    nsa_cmp_fwd_args a = L.cmp_args(qkv.data_ptr(), ckv, outs[0], lse);
     const int64_t cpf = c.block / c.stride;
     bool pooled = false;
     if (L.k_sel > 0) {
@@ -305,10 +309,11 @@ static std::vector<OptTensor> layer_forward(Tensor x, std::vector<OptTensor> wei
       p.neg_max = L.dt == NSA_BF16 ? -3.3895313892515355e38f : -std::numeric_limits<float>::max();
       check(nsa::launch_select(p, st));
     }
+    if (!c.diff_topk) importance = Tensor();
   }
   // sliding branch
   {
-    nsa_swa_fwd_args a = L.swa_args(qr, kr, v, o + 2 * q_bytes, lse + 2 * L.rows(c.heads));
+    nsa_swa_fwd_args a = L.swa_args(qr, kr, v, outs[2], lse + 2 * L.rows(c.heads));
     const Tensor ws = scratch(a, nsa_swa_workspace_bytes, 0, x);
     check(nsa_swa_fwd(&a, st));
   }
@@ -317,20 +322,26 @@ static std::vector<OptTensor> layer_forward(Tensor x, std::vector<OptTensor> wei
   Tensor index;
   const Tensor merged = at::empty({BN, c.heads * d}, x.options());
   {
-    nsa_sel_fwd_args a = L.sel_args(qr, kr, v, o + q_bytes, lse + L.rows(c.heads), L.k_sel > 0 ? idx : nullptr, L.k_sel > 0 ? mask : nullptr);
+    nsa_sel_fwd_args a = L.sel_args(qr, kr, v, outs[1], lse + L.rows(c.heads), L.k_sel > 0 ? idx : nullptr, L.k_sel > 0 ? mask : nullptr);
     const Tensor ws = scratch(a, nsa_sel_workspace_bytes, 0, x);
     if (save && ws.defined()) {
       index = bytes(nsa_sel_index_bytes(&a), x);
       a.index_out = index.data_ptr();
       a.index_out_bytes = index.numel();
     }
-    const nsa::CombineParams p = L.combine_params(o, logits.data_ptr());
+    nsa::CombineParams p = L.combine_params(outs, logits.data_ptr());
     nsa::GatherTargets t = {};
     t.outs[0] = merged.data_ptr(); t.num_outs = 1; t.total_features = c.heads * d;
     nsa_sel_fwd_args fused = a;
     if (!save) fused.out = no_tensor();
     int rc = ws.defined() ? nsa::sm100_sel_fwd_combine(fused, p, t, st) : NSA_ERR_UNSUPPORTED;
+    Tensor selected;
     if (rc == NSA_ERR_UNSUPPORTED) {
+      if (!save) {
+        selected = bytes(q_bytes, x);
+        a.out.ptr = selected.data_ptr();
+        p.o[1] = a.out.ptr;
+      }
       check(nsa_sel_fwd(&a, st));
       rc = nsa::launch_combine_gather(p, t, L.dt, st);
     }
@@ -444,42 +455,49 @@ static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor>
 
   // output projection and gated combine
   dout = dout.reshape({BN, L.dim}).contiguous();
-  const Tensor d_merged = product(Op::NN, dout, w.out);
+  // (what a later step does not need is given back as soon as it has been used: the partial results of the branches are
+  // larger than all of it together)
+  Tensor d_merged = product(Op::NN, dout, w.out);
   Slab tmp;
-  const int64_t t_do = tmp.add(3 * q_bytes), t_delta = tmp.add(3 * L.rows(H) * 4), t_dq = tmp.add(3 * q_elems * 4);
-  const int64_t t_gates = tmp.add(nsa::gate_sums_partial((int)(3 * H)) * 4);
+  const int64_t t_delta = tmp.add(3 * L.rows(H) * 4), t_gates = tmp.add(nsa::gate_sums_partial((int)(3 * H)) * 4);
   tmp.allocate(x);
+  Tensor d_outs[3], dqs[3];
+  for (Tensor& t : d_outs) t = bytes(q_bytes, x);
   const Tensor d_logits = at::empty({BN, 3 * H}, x.options());
   {
-    nsa::CombineParams p = L.combine_params(kp + at_o, logits.data_ptr());
+    void* const outs[3] = {kp + at_o, kp + at_o + q_bytes, kp + at_o + 2 * q_bytes};
+    nsa::CombineParams p = L.combine_params(outs, logits.data_ptr());
     p.dout = d_merged.data_ptr();
-    for (int s = 0; s < 3; ++s) p.d_o[s] = tmp.at(t_do + s * q_bytes);
+    for (int s = 0; s < 3; ++s) p.d_o[s] = d_outs[s].data_ptr();
     p.delta = reinterpret_cast<float*>(tmp.at(t_delta));
     p.d_logits = d_logits.data_ptr();
     check(nsa::launch_combine(p, L.dt, true, st));
+    d_merged = Tensor();
   }
 
   // the three branches
   nsa::QkvGrad qg = {};
   const nsa_tensor kr = L.heads_of(kp + at_kr, hkv, N), v = L.in_qkv(qkv.data_ptr(), 2);
   auto delta = [&](int s) { return reinterpret_cast<float*>(tmp.at(t_delta)) + s * L.rows(H); };
-  auto d_o = [&](int s) { return L.heads_of(tmp.at(t_do + s * q_bytes), H, N); };
+  auto d_o = [&](int s) { return L.heads_of(d_outs[s].data_ptr(), H, N); };
   // dq of branch s: rows in the layer's type where the kernels store them, else fp32; run(direct) issues the call
   auto with_dq = [&](int s, bool stores, bool need_f32, nsa_tensor& dq_out, float*& dq, auto run) {
-    void* const at = tmp.at(t_dq + s * q_elems * 4);
     int rc = NSA_ERR_UNSUPPORTED;
     if (stores && !need_f32) {
-      dq_out = L.heads_of(at, H, N);
+      dqs[s] = bytes(q_bytes, x);
+      dq_out = L.heads_of(dqs[s].data_ptr(), H, N);
       rc = run();
-      if (rc == 0) qg.dq[s] = at;
+      if (rc == 0) qg.dq[s] = dqs[s].data_ptr();
     }
     if (rc == NSA_ERR_UNSUPPORTED) {
+      dqs[s] = bytes(q_elems * 4, x);
       dq_out = no_tensor();
-      dq = static_cast<float*>(at);
+      dq = ptr<float>(dqs[s]);
       rc = run();
       if (rc == 0) qg.dq_f32[s] = dq;
     }
     check(rc);
+    d_outs[s] = Tensor();
   };
   Tensor slots;
   {
@@ -524,7 +542,7 @@ static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor>
     const Tensor ckc = kept_view(at_ckv, {2, B, hkv, kv, d}, type).select(0, 0).narrow(2, c.num_mem, L.ncb).to(at::kFloat);   // [B, Hkv, ncb, d]
     const Tensor dlog_kv = dlog.view({B, hkv, sel_per_kv * N, L.ncb});
     const Tensor dq_add = at::matmul(dlog_kv, ckc).view({B, L.hs, 1, N, d});
-    tmp.view(t_dq, {B, L.hs, per_sel, N, d}, at::kFloat).add_(dq_add);
+    dqs[0].view(at::kFloat).view({B, L.hs, per_sel, N, d}).add_(dq_add);
     const Tensor q = qkv.view({B, N, c.heads + 2 * hkv, d}).narrow(2, 0, H).permute({0, 2, 1, 3}).to(at::kFloat);
     const Tensor q_sum = q.reshape({B, L.hs, per_sel, N, d}).sum(2).view({B, hkv, sel_per_kv * N, d});
     acc.narrow(0, 2 * k_elems, c_elems).view({B, hkv, kv, d}).narrow(2, c.num_mem, L.ncb).add_(at::matmul(dlog_kv.transpose(-1, -2), q_sum));
@@ -535,7 +553,7 @@ static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor>
   const Tensor dc = at::empty({2, wins, d}, x.options());
   check(nsa::launch_split_mem(L.shape, dck, dc.data_ptr(), small + s_mem, small + s_b2, L.dt, st));
   const Tensor dck_rows = dc.select(0, 0), dcv_rows = dc.select(0, 1);
-  const Tensor dhk = product(Op::NN, dck_rows, w.k2), dhv = product(Op::NN, dcv_rows, w.v2);
+  Tensor dhk = product(Op::NN, dck_rows, w.k2), dhv = product(Op::NN, dcv_rows, w.v2);
   {
     nsa::ColumnSums p = {};
     p.x[0] = dhk.data_ptr(); p.x[1] = dhv.data_ptr(); p.act[0] = hk.data_ptr(); p.act[1] = hv.data_ptr();
@@ -549,13 +567,16 @@ static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor>
   if (needs[15]) g[15] = product(Op::TN, dcv_rows, hv);
   if (needs[9]) g[9] = product(Op::TN, dhk, kw);
   if (needs[13]) g[13] = product(Op::TN, dhv, vw);
-  const Tensor dkw = product(Op::NN, dhk, w.k1), dvw = product(Op::NN, dhv, w.v1);
+  Tensor dkw = product(Op::NN, dhk, w.k1), dvw = product(Op::NN, dhv, w.v1);
+  dhk = dhv = Tensor();
   check(nsa::launch_pos_grad(L.shape, dkw.data_ptr(), dvw.data_ptr(), small + s_pos, L.dt, st));
 
   // qkv, gates, norm
   const Tensor d_qkv = at::empty({BN, L.F}, x.options());
   qg.dk = dk; qg.dv = dk + k_elems; qg.dkw = dkw.data_ptr(); qg.dvw = dvw.data_ptr(); qg.inv_freq = ptr<float>(inv_freq); qg.out = d_qkv.data_ptr();
   check(nsa::launch_qkv_grad(L.shape, qg, L.dt, st));
+  for (Tensor& t : dqs) t = Tensor();
+  dkw = dvw = Tensor();
   check(nsa::launch_gate_sums(d_logits.data_ptr(), small + s_gate, BN, (int)(3 * H), reinterpret_cast<float*>(tmp.at(t_gates)),
                               reinterpret_cast<unsigned*>(dk + a_counters), L.dt, st));
   if (needs[5]) g[5] = product(Op::TN, dout, merged);

@@ -224,3 +224,35 @@ def test_the_gradient_of_the_gate_bias_repeats_to_the_bit(b, n, heads, d, dtype)
     for _ in range(4):
         _, _, again = run(layer, x, dout)
         assert torch.equal(again['to_strategy_combine.0.bias'], grads['to_strategy_combine.0.bias'])
+
+
+@pytest.mark.parametrize('options', [{}, dict(dim_head=128, heads=8)])
+def test_the_native_layer_needs_no_more_memory_than_the_modules(options):
+    kw = dict(dim=512, dim_head=64, heads=16, kv_heads=4, causal=True, sliding_window_size=128, compress_block_size=32,
+              compress_block_sliding_stride=16, selection_block_size=64, num_selected_blocks=8, use_triton_kernel=True)
+    layer = SparseAttention(**{**kw, **options})
+    recipe.fill_weights(layer, seed=3)
+    layer, n = layer.to('cuda').to(BF16), 4096
+    x, dout = (recipe.randn((2, n, 512), seed).to(BF16).to('cuda') for seed in (5, 6))
+
+    def peaks():
+        def peak(call):
+            call()
+            torch.cuda.synchronize()
+            before = torch.cuda.memory_allocated()
+            torch.cuda.reset_peak_memory_stats()
+            call()
+            return torch.cuda.max_memory_allocated() - before
+
+        def prefill():
+            with torch.no_grad():
+                layer(x, return_cache=True)
+        return peak(lambda: run(layer, x, dout)), peak(prefill)
+    native = peaks()
+    hook = layer.combine_heads.register_forward_hook(lambda *_: None)
+    modules = peaks()
+    hook.remove()
+    # the caches of the native prefill have room for 64 to 1024 more rows
+    rows = 4 * 2 * layer.kv_heads * (n // 8 + 64) * layer.dim_head * x.element_size()
+    # the backward gives up what the forward saved at its end, where the modules release theirs one by one
+    assert native[0] <= 1.03 * modules[0] and native[1] <= 1.03 * modules[1] + rows, (native, modules)
