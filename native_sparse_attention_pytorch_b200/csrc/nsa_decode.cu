@@ -55,8 +55,8 @@ __device__ __forceinline__ void st_cluster(uint32_t addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
 
-// A tile of up to kTile consecutive keys: where its rows are
-constexpr int kTile = 16;
+// A tile of up to kTile consecutive keys (kLongTile in the form for very long caches): where its rows are
+constexpr int kTile = 16, kLongTile = 4;
 template <typename T>
 struct KeyTile {
   const T *k, *v;
@@ -64,9 +64,9 @@ struct KeyTile {
   int cnt;
 };
 
-// Requests the key and value rows of a tile into a staging buffer (kTile rows of each, padded by 16 bytes so that
+// Requests the key and value rows of a tile into a staging buffer (ROWS rows of each, padded by 16 bytes so that
 // neighbouring rows fall on different banks); one commit group.  Missing rows are zeroed: they take part in products.
-template <typename T>
+template <typename T, int ROWS>
 __device__ __forceinline__ void stage_tile(uint32_t buf, const KeyTile<T>& t, int d, int lane) {
   const int row_bytes = d * (int)sizeof(T), padded = row_bytes + 16;
   const int pieces = row_bytes / 16;
@@ -74,13 +74,13 @@ __device__ __forceinline__ void stage_tile(uint32_t buf, const KeyTile<T>& t, in
   const int lpr = pieces >= 32 ? 32 : pieces >= 16 ? 16 : pieces >= 8 ? 8 : pieces >= 4 ? 4 : pieces >= 2 ? 2 : 1;
   const int sub = lane & (lpr - 1);
 #pragma unroll 1
-  for (int r = lane / lpr; r < kTile; r += 32 / lpr) {
+  for (int r = lane / lpr; r < ROWS; r += 32 / lpr) {
     const bool ok = r < t.cnt;
     const T *kr = t.k + (ok ? r * t.k_sn : 0), *vr = t.v + (ok ? r * t.v_sn : 0);
     const uint32_t dst = buf + r * padded;
     for (int c = sub; c < pieces; c += lpr) {
       ptx::cp_async16(dst + c * 16, kr + c * (16 / (int)sizeof(T)), ok ? 16u : 0u);
-      ptx::cp_async16(dst + kTile * padded + c * 16, vr + c * (16 / (int)sizeof(T)), ok ? 16u : 0u);
+      ptx::cp_async16(dst + ROWS * padded + c * 16, vr + c * (16 / (int)sizeof(T)), ok ? 16u : 0u);
     }
   }
   ptx::cp_async_commit();
@@ -88,9 +88,9 @@ __device__ __forceinline__ void stage_tile(uint32_t buf, const KeyTile<T>& t, in
 
 // The state of a branch in one warp, on CUDA cores (fp32 inputs, and head sizes the tensor form below does not have).
 // Two lanes share a key for the dot products; for the values a lane owns feature pairs.
-template <typename T, int GT>
+template <typename T, int GT, int ROWS = kTile>
 struct ScalarState {
-  static constexpr int kHeads = GT;
+  static constexpr int kHeads = GT, kRows = ROWS;
   float m[GT], l[GT], acc[GT][2][2];
 
   __device__ __forceinline__ void start(const T*, int, int) {
@@ -112,7 +112,7 @@ struct ScalarState {
     float logit[GT];
 #pragma unroll
     for (int g = 0; g < GT; ++g) logit[g] = 0.f;
-    const T* key = reinterpret_cast<const T*>(buf + (lane / 2) * padded);
+    const T* key = reinterpret_cast<const T*>(buf + min(lane / 2, ROWS - 1) * padded);
 #pragma unroll 1
     for (int c = (lane & 1) * V; c < d; c += 2 * V) {
       float kv[V];
@@ -145,7 +145,7 @@ struct ScalarState {
       acc[g][1][0] *= alpha; acc[g][1][1] *= alpha;
     }
     const bool in0 = 2 * lane < d, in1 = 64 + 2 * lane < d;
-    const uint8_t* vrow = buf + kTile * padded + 2 * lane * (int)sizeof(T);
+    const uint8_t* vrow = buf + ROWS * padded + 2 * lane * (int)sizeof(T);
 #pragma unroll 2
     for (int k = 0; k < cnt; ++k) {
       const T* row = reinterpret_cast<const T*>(vrow + k * padded);
@@ -206,7 +206,7 @@ __device__ __forceinline__ uint32_t transpose_8x8(uint32_t v) {
 template <int D, int GT>
 struct TensorState {
   using T = __nv_bfloat16;
-  static constexpr int kHeads = GT;
+  static constexpr int kHeads = GT, kRows = kTile;
   static constexpr int NT = (GT + 7) / 8;        // groups of eight heads
   // lane l holds heads 8 n + 2 (l % 4) + {0, 1}; accumulator rows are the features 16 t + l / 4 (+ 8)
   float m[NT][2], l[NT][2], o[NT][D / 16][4];
@@ -417,13 +417,13 @@ struct DecodeLayout {
   int stage, q, area, recv, ml, imp, prob, total;
   int shift;      // a CTA finishes 2^shift features of every head of the group
 };
-__host__ __device__ inline DecodeLayout decode_layout(int el, int GT, int d, int W, int S, int ncb, int cols) {
+__host__ __device__ inline DecodeLayout decode_layout(int el, int GT, int rows, int d, int W, int S, int ncb, int cols) {
   DecodeLayout L;
   auto up = [](int x) { return (x + 15) / 16 * 16; };
   L.shift = 0;
   while ((S << L.shift) < d) ++L.shift;
-  L.stage = 0;                                               // [W][2 buffers][keys, values][kTile] rows
-  L.q = L.stage + W * 4 * kTile * (d * el + 16);             // [un-rotated, rotated][GT] rows of d + 8
+  L.stage = 0;                                               // [W][2 buffers][keys, values][tile] rows
+  L.q = L.stage + W * 4 * rows * (d * el + 16);              // [un-rotated, rotated][GT] rows of d + 8
   L.area = L.q + up(2 * GT * (d + 8) * el);                  // parked warp states [W][GT][d + 2]
   L.recv = L.area + up(W * GT * (d + 2) * 4);                // [S][3 branches][GT][2^shift]: every CTA's part of this CTA's features
   L.ml = L.recv + up(((S * 3 * GT) << L.shift) * 4);         // [S][3][GT][2]: every CTA's maxima and sums
@@ -435,7 +435,7 @@ __host__ __device__ inline DecodeLayout decode_layout(int el, int GT, int d, int
 
 template <typename T, typename State>
 __global__ void __launch_bounds__(DecodeShape<T>::kWarps * 32, 1) decode_kernel(const DecodeParams P, int S) {
-  constexpr int GT = State::kHeads;
+  constexpr int GT = State::kHeads, ROWS = State::kRows;
   const int kThreads = blockDim.x, W = kThreads / 32;
   extern __shared__ __align__(16) uint8_t decode_smem[];
   __shared__ int sel_idx[32];
@@ -449,8 +449,8 @@ __global__ void __launch_bounds__(DecodeShape<T>::kWarps * 32, 1) decode_kernel(
   const int G = P.q_heads / P.kv_heads, d = P.d;
   const int cpf = P.block / P.stride;
   const int cols = P.stride != P.block ? P.ncb / cpf : P.ncb;
-  const DecodeLayout L = decode_layout((int)sizeof(T), GT, d, W, S, P.ncb, cols);
-  const int buf_bytes = 2 * kTile * (d * (int)sizeof(T) + 16);
+  const DecodeLayout L = decode_layout((int)sizeof(T), GT, ROWS, d, W, S, P.ncb, cols);
+  const int buf_bytes = 2 * ROWS * (d * (int)sizeof(T) + 16);
   uint8_t* const stage = decode_smem + L.stage + warp * 2 * buf_bytes;
   T* const q_s = reinterpret_cast<T*>(decode_smem + L.q);
   float* const area = reinterpret_cast<float*>(decode_smem + L.area);
@@ -461,43 +461,43 @@ __global__ void __launch_bounds__(DecodeShape<T>::kWarps * 32, 1) decode_kernel(
   const T* kb = (const T*)P.keys + b * P.k_sb + (int64_t)kvh * P.k_sh;
   const T* vb = (const T*)P.vals + b * P.v_sb + (int64_t)kvh * P.v_sh;
   const int pos = P.T - 1;
-  const int mem_tiles = P.ncb > 0 ? (P.num_mem + kTile - 1) / kTile : 0;
+  const int mem_tiles = P.ncb > 0 ? (P.num_mem + ROWS - 1) / ROWS : 0;
   const int win0 = max(0, pos - P.window), own0 = pos / P.block * P.block;
-  const int per_block = (P.block + kTile - 1) / kTile;
+  const int per_block = (P.block + ROWS - 1) / ROWS;
   auto tiles_of = [&](int phase) {
-    if (phase == 0) return mem_tiles + (P.ncb + kTile - 1) / kTile;
-    if (phase == 1) return (pos + 1 - win0 + kTile - 1) / kTile;
-    return sel_count * per_block + (pos + 1 - own0 + kTile - 1) / kTile;
+    if (phase == 0) return mem_tiles + (P.ncb + ROWS - 1) / ROWS;
+    if (phase == 1) return (pos + 1 - win0 + ROWS - 1) / ROWS;
+    return sel_count * per_block + (pos + 1 - own0 + ROWS - 1) / ROWS;
   };
   auto locate = [&](int phase, int t) {
     if (phase == 0) {
       if (t < mem_tiles) {
-        const int64_t at = ((int64_t)kvh * P.num_mem + t * kTile) * d;
-        return KeyTile<T>{(const T*)P.mem_k + at, (const T*)P.mem_v + at, d, d, min(kTile, P.num_mem - t * kTile)};
+        const int64_t at = ((int64_t)kvh * P.num_mem + t * ROWS) * d;
+        return KeyTile<T>{(const T*)P.mem_k + at, (const T*)P.mem_v + at, d, d, min(ROWS, P.num_mem - t * ROWS)};
       }
-      const int t0 = (t - mem_tiles) * kTile;
+      const int t0 = (t - mem_tiles) * ROWS;
       return KeyTile<T>{(const T*)P.ck + b * P.ck_sb + (int64_t)kvh * P.ck_sh + t0 * P.ck_sn,
                         (const T*)P.cv + b * P.cv_sb + (int64_t)kvh * P.cv_sh + t0 * P.cv_sn, P.ck_sn, P.cv_sn,
-                        min(kTile, P.ncb - t0)};
+                        min(ROWS, P.ncb - t0)};
     }
-    int t0 = win0 + t * kTile, end = pos + 1;
+    int t0 = win0 + t * ROWS, end = pos + 1;
     if (phase == 2) {
       const int chosen = sel_count * per_block;
       if (t < chosen) {
         const int s = t / per_block;
-        t0 = sel_idx[s] * P.block + (t - s * per_block) * kTile;
+        t0 = sel_idx[s] * P.block + (t - s * per_block) * ROWS;
         end = min((sel_idx[s] + 1) * P.block, P.T);
       } else {
-        t0 = own0 + (t - chosen) * kTile;
+        t0 = own0 + (t - chosen) * ROWS;
       }
     }
-    return KeyTile<T>{kb + t0 * P.k_sn, vb + t0 * P.v_sn, P.k_sn, P.v_sn, min(kTile, end - t0)};
+    return KeyTile<T>{kb + t0 * P.k_sn, vb + t0 * P.v_sn, P.k_sn, P.v_sn, min(ROWS, end - t0)};
   };
   // The warps of the cluster take a branch's tiles in turn; warp 0 of every CTA sits the window out and ranks
   auto first_of = [&](int phase) { return phase == 1 ? (warp == 0 ? 0x3fffffff : (warp - 1) * S + rank) : warp * S + rank; };
 
   if (tid == 0) sel_count = 0;
-  if (first_of(0) < tiles_of(0)) stage_tile<T>(ptx::smem_u32(stage), locate(0, first_of(0)), d, lane);
+  if (first_of(0) < tiles_of(0)) stage_tile<T, ROWS>(ptx::smem_u32(stage), locate(0, first_of(0)), d, lane);
   for (int e = tid; e < 3 * G; e += kThreads)
     gate_s[e] = Elem<T>::to_float(((const T*)P.gates)[((int64_t)b * P.q_heads + kvh * G) * 3 + e]);
   {
@@ -574,7 +574,7 @@ __global__ void __launch_bounds__(DecodeShape<T>::kWarps * 32, 1) decode_kernel(
 #pragma unroll 1
     for (int t = first_of(phase); t < total; t += step) {
       if (t + step < total) {
-        stage_tile<T>(ptx::smem_u32(stage) + (which ^ 1) * buf_bytes, locate(phase, t + step), d, lane);
+        stage_tile<T, ROWS>(ptx::smem_u32(stage) + (which ^ 1) * buf_bytes, locate(phase, t + step), d, lane);
         ptx::cp_async_wait<1>();
       } else {
         ptx::cp_async_wait<0>();
@@ -584,7 +584,7 @@ __global__ void __launch_bounds__(DecodeShape<T>::kWarps * 32, 1) decode_kernel(
       const bool want = phase == 0 && t >= mem_tiles;
       if (cnt > 0)
         state.tile(stage + which * buf_bytes, rows, cnt, d, P.scale, lane, G, want, [&](int key, float mean) {
-          const uint32_t dst = ptx::smem_u32(imp_s + (t - mem_tiles) * kTile + key);
+          const uint32_t dst = ptx::smem_u32(imp_s + (t - mem_tiles) * ROWS + key);
           for (int r = 0; r < S; ++r) st_cluster(map_rank(dst, r), mean);
         });
       __syncwarp();
@@ -594,11 +594,11 @@ __global__ void __launch_bounds__(DecodeShape<T>::kWarps * 32, 1) decode_kernel(
     if (phase == 0) {
       cluster_arrive();       // this warp's logits are on their way to everybody
       // the first tile of the window travels under the fold
-      if (first_of(1) < tiles_of(1)) stage_tile<T>(ptx::smem_u32(stage), locate(1, first_of(1)), d, lane);
+      if (first_of(1) < tiles_of(1)) stage_tile<T, ROWS>(ptx::smem_u32(stage), locate(1, first_of(1)), d, lane);
     }
     state.park(area + (size_t)warp * GT * (d + 2), d, lane);
     __syncthreads();
-    if (phase == 1 && first_of(2) < tiles_of(2)) stage_tile<T>(ptx::smem_u32(stage), locate(2, first_of(2)), d, lane);
+    if (phase == 1 && first_of(2) < tiles_of(2)) stage_tile<T, ROWS>(ptx::smem_u32(stage), locate(2, first_of(2)), d, lane);
     // Fold the warps' states and send every element to the CTA that finishes it: kThreads / GT threads per head
     {
       const int branch = phase == 0 ? 0 : 3 - phase;          // in the order of the gates: compressed, selected, sliding
@@ -668,27 +668,37 @@ __global__ void __launch_bounds__(DecodeShape<T>::kWarps * 32, 1) decode_kernel(
   }
 }
 
+// CTAs per (batch, KV head) and warps per CTA; no warps where the logits of all compressed blocks do not fit
 template <typename T, typename State>
-static int launch_decode_state(const DecodeParams& P, cudaStream_t stream) {
-  constexpr int GT = State::kHeads;
+static void decode_split(const DecodeParams& P, int* S_out, int* W_out, int* smem) {
+  constexpr int ROWS = State::kRows;
+  constexpr int kMost = 224 * 1024;            // beside the kernel's static part
   const int cpf = P.block / P.stride;
   const int cols = P.stride != P.block ? P.ncb / cpf : P.ncb;
-  // CTAs per (batch, KV head): enough warps for one tile of the longest branch each, as long as the grid fits one wave
+  // enough warps for one tile of the longest branch each, as long as the grid fits one wave
   const int units = P.batch * P.kv_heads;
   const int keys = max(P.ncb, max(P.window + 1, (min(P.nsel, cols) + 1) * P.block));
   int W = DecodeShape<T>::kWarps, S = 1;
-  const int tiles = (min(keys, P.T) + kTile - 1) / kTile;
+  const int tiles = (min(keys, P.T) + ROWS - 1) / ROWS;
   while (S < kMaxCluster && S * W < tiles && units * S * 2 <= 148) S *= 2;
-  auto bytes = [&](int warps) { return decode_layout((int)sizeof(T), GT, P.d, warps, S, P.ncb, cols).total; };
-  constexpr int kMost = 220 * 1024;
-  while (W > 2 && bytes(W) > kMost) W /= 2;    // very long caches: the logits take the room of staging areas
-  const int smem = bytes(W);
-  if (smem > kMost || P.ncb > (1 << 24)) return fail(NSA_ERR_UNSUPPORTED, "decode step: too many compressed blocks for one CTA's shared memory");
+  auto bytes = [&](int warps) { return (int64_t)decode_layout((int)sizeof(T), State::kHeads, ROWS, P.d, warps, S, P.ncb, cols).total; };
+  while (W > 2 && bytes(W) > kMost) W /= 2;    // long caches: the logits take the room of staging areas
+  *S_out = S;
+  *W_out = P.ncb <= (1 << 24) && bytes(W) <= kMost ? W : 0;
+  *smem = (int)bytes(W);
+}
+
+// NSA_ERR_UNSUPPORTED (without a message) where the compressed logits do not fit beside this form's staging areas
+template <typename T, typename State>
+static int launch_decode_state(const DecodeParams& P, cudaStream_t stream) {
+  int S, W, smem;
+  decode_split<T, State>(P, &S, &W, &smem);
+  if (W == 0) return NSA_ERR_UNSUPPORTED;
   auto kern = decode_kernel<T, State>;
   cudaError_t err = allow_shared_memory<decode_kernel<T, State>>();
   if (err != cudaSuccess) return fail((int)err, cudaGetErrorString(err));
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(units * S));
+  cfg.gridDim = dim3((unsigned)(P.batch * P.kv_heads * S));
   cfg.blockDim = dim3(W * 32);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
@@ -704,20 +714,27 @@ static int launch_decode_state(const DecodeParams& P, cudaStream_t stream) {
   return NSA_OK;
 }
 
-// bf16 with head sizes of 64 and 128 runs on the tensor instructions, everything else on the CUDA cores
+// bf16 with head sizes of 64 and 128 runs on the tensor instructions, everything else on the CUDA cores.  Every CTA holds
+// the logits of all compressed blocks; where they leave no room for staging areas of 16 rows (from 300 000 cached tokens on,
+// by type, group and head size), tiles of 4 rows on the CUDA cores take their place: slower per tile, but the step is served
+// up to 230 KB of logits.
 template <typename T, int GT>
 static int launch_decode_gt(const DecodeParams& P, cudaStream_t stream) {
-  if constexpr (sizeof(T) == 2 && GT >= 8) {
-    if (P.d == 64) return launch_decode_state<T, TensorState<64, GT>>(P, stream);
-    if (P.d == 128) return launch_decode_state<T, TensorState<128, GT>>(P, stream);
+  int rc = NSA_ERR_UNSUPPORTED;
+  if constexpr (sizeof(T) == 2) {   // the tensor form works on eight heads in any case
+    if (P.d == 64) rc = launch_decode_state<T, TensorState<64, GT < 8 ? 8 : GT>>(P, stream);
+    else if (P.d == 128) rc = launch_decode_state<T, TensorState<128, GT < 8 ? 8 : GT>>(P, stream);
+    else rc = launch_decode_state<T, ScalarState<T, GT>>(P, stream);
+  } else {
+    rc = launch_decode_state<T, ScalarState<T, GT>>(P, stream);
   }
-  return launch_decode_state<T, ScalarState<T, GT>>(P, stream);
+  if (rc == NSA_ERR_UNSUPPORTED) rc = launch_decode_state<T, ScalarState<T, GT, kLongTile>>(P, stream);
+  return rc == NSA_ERR_UNSUPPORTED ? fail(rc, "decode step: too many compressed blocks for one CTA's shared memory") : rc;
 }
 
 template <typename T>
 static int launch_decode_t(const DecodeParams& P, cudaStream_t stream) {
   const int G = P.q_heads / P.kv_heads;
-  if (sizeof(T) == 2 && (P.d == 64 || P.d == 128) && G <= 8) return launch_decode_gt<T, 8>(P, stream);   // eight columns per step in any case
   if (G == 1) return launch_decode_gt<T, 1>(P, stream);
   if (G == 2) return launch_decode_gt<T, 2>(P, stream);
   if (G <= 4) return launch_decode_gt<T, 4>(P, stream);

@@ -163,3 +163,37 @@ def test_a_recorded_step_leaves_the_caches_of_eager_steps_alone():
         assert all(torch.equal(t, k) for t, k in zip(flat(grown), kept))
         torch.cuda.synchronize()
     del recorded, out, graph
+
+
+# caches whose compressed logits nearly fill a CTA's shared memory, by type, group and head size: just below what the step
+# has always served.  (heads, kv heads, head size, dtype, stride, block, compressed blocks, own rows behind the last one)
+@pytest.mark.parametrize('case', [(1, 1, 64, torch.bfloat16, 1, 1, 25100, 3), (2, 1, 128, torch.bfloat16, 1, 2, 31800, 2),
+                                  (8, 1, 128, torch.float32, 1, 1, 18800, 1), (16, 1, 128, torch.float32, 1, 1, 12150, 5),
+                                  (3, 1, 40, torch.float32, 1, 4, 39220, 7)])
+def test_step_on_caches_as_long_as_shared_memory_allows(case):
+    from native_sparse_attention_pytorch_b200 import ops
+    hq, hkv, d, dtype, stride, block, ncb, rest = case
+    t, nsel, window, g = ncb * stride + rest, 5, 37, hq // hkv
+    gen = torch.Generator(DEV).manual_seed(ncb)
+
+    def randn(*shape):
+        return torch.randn(shape, device=DEV, generator=gen).to(dtype)
+    q, qr, keys, vals = randn(1, hq, d), randn(1, hq, d), randn(1, hkv, t, d), randn(1, hkv, t, d)
+    ck, cv, mem, gates = randn(1, hkv, ncb, d), randn(1, hkv, ncb, d), randn(2, hkv, 1, d), torch.rand(1, hq, 3, device=DEV, generator=gen).to(dtype)
+    got = ops.decode_step(q, qr, keys, vals, ck, cv, mem[0], mem[1], gates, stride=stride, block=block, num_selected=nsel, window=window)
+
+    f = lambda x: x.double().squeeze(0)
+    def attend(query, k, v):
+        sim = query @ k.transpose(-1, -2) * d ** -0.5
+        return sim.softmax(-1) @ v, sim
+    k, v, c = f(keys)[0], f(vals)[0], block // stride
+    o_cmp, sim = attend(f(q), torch.cat((mem[0, 0].double(), f(ck)[0])), torch.cat((mem[1, 0].double(), f(cv)[0])))
+    logits = sim[:, 1:].mean(0)[:ncb // c * c].view(-1, c).mean(1)
+    picks = torch.cat((torch.tensor([-1e3], device=DEV, dtype=torch.double), logits)).softmax(0)[1:].topk(nsel)
+    assert picks.values[-1] > 1e-10
+    rows = [torch.arange(i * block, (i + 1) * block, device=DEV) for i in picks.indices.tolist()] + [torch.arange((t - 1) // block * block, t, device=DEV)]
+    o_sel, _ = attend(f(qr), k[torch.cat(rows)], v[torch.cat(rows)])
+    o_swa, _ = attend(f(qr), k[-window - 1:], v[-window - 1:])
+    gate = f(gates)
+    want = (gate[:, 0:1] * o_cmp + gate[:, 1:2] * o_sel + gate[:, 2:3] * o_swa).reshape(1, -1)
+    (assert_close_f32 if dtype == torch.float32 else assert_close_bf16)(got, want.float().cpu(), 'merged row')
