@@ -3,6 +3,7 @@ operators, g++ against the installed PyTorch) in-tree.
 
     python -m native_sparse_attention_pytorch_b200.build [--force] [--verbose]
 """
+import glob
 import os
 import subprocess
 import sys
@@ -26,6 +27,33 @@ def _newest(*dirs):
 
 def _fresh(lib, *dirs):
     return os.path.exists(lib) and os.path.getmtime(lib) >= _newest(*dirs)
+
+
+HOST_STAMP = os.path.join(HERE, 'build', 'host_built_for.txt')
+
+
+def _built_for():
+    """What _nsa_host.so depends on besides its sources: it does not load into another PyTorch or Python."""
+    import torch
+    return f'PyTorch {torch.__version__} at {os.path.dirname(torch.__file__)}, {sysconfig.get_config_var("SOABI")}\n'
+
+
+def _host_fresh():
+    if not (_fresh(HOST_LIB, CSRC, os.path.join(CSRC, 'host')) and os.path.exists(HOST_STAMP)):
+        return False
+    with open(HOST_STAMP) as f:
+        return f.read() == _built_for()
+
+
+def _cuda_library(name, package, site, toolkit):
+    """The shared library PyTorch itself uses: from NVIDIA's wheels beside it, or from the toolkit it was built with."""
+    places = [os.path.join(site, 'nvidia', package, 'lib'), os.path.join(site, 'nvidia', 'cu*', 'lib'), os.path.join(toolkit, 'lib64'),
+              os.path.join(toolkit, 'targets', '*', 'lib')]
+    for place in places:
+        found = sorted(glob.glob(os.path.join(place, name + '.so.[0-9]*'))) or glob.glob(os.path.join(place, name + '.so'))
+        if found:
+            return min(found, key=len)     # libcublas.so.12 rather than libcublas.so.12.8.4.1
+    raise RuntimeError(f'{name}.so was found in none of {places}: _nsa_host.so links against the one PyTorch uses')
 
 
 def _compile_all(jobs, verbose):
@@ -56,7 +84,7 @@ def build(force=False, verbose=False):
         jobs = [(src, os.path.join(objdir, src.replace('.cu', '.o')),
                  [nvcc, *flags, '-c', os.path.join(CSRC, src), '-o', os.path.join(objdir, src.replace('.cu', '.o'))])
                 for src in SOURCES]
-    if force or not _fresh(HOST_LIB, CSRC, os.path.join(CSRC, 'host')):
+    if force or not _host_fresh():
         import torch
         from torch.utils import cpp_extension
         cuda = os.path.dirname(os.path.dirname(nvcc))
@@ -76,11 +104,12 @@ def build(force=False, verbose=False):
         import torch
         torch_lib = os.path.join(os.path.dirname(torch.__file__), 'lib')
         # PyTorch's own copies of cuBLAS and the CUDA runtime, which its libraries have loaded by the time this one is
-        import glob
-        site = os.path.dirname(os.path.dirname(torch.__file__))
-        shared = [glob.glob(os.path.join(site, 'nvidia', *p))[0] for p in (('cublas', 'lib', 'libcublas.so.12'), ('cuda_runtime', 'lib', 'libcudart.so.12'))]
+        site, toolkit = os.path.dirname(os.path.dirname(torch.__file__)), os.path.dirname(os.path.dirname(nvcc))
+        shared = [_cuda_library('libcublas', 'cublas', site, toolkit), _cuda_library('libcudart', 'cuda_runtime', site, toolkit)]
         subprocess.run(['g++', '-shared', '-o', HOST_LIB, *objs[len(jobs):], '-L', HERE, '-lnsa_b200', '-L', torch_lib, '-ltorch', '-ltorch_cpu',
                         '-ltorch_cuda', '-ltorch_python', '-lc10', '-lc10_cuda', *shared, '-Wl,-rpath,$ORIGIN'], check=True)
+        with open(HOST_STAMP, 'w') as f:
+            f.write(_built_for())
     return LIB
 
 

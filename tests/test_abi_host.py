@@ -138,3 +138,30 @@ def test_decode_and_diff_topk_are_part_of_the_module_interface():
     assert attn.use_diff_topk
     with pytest.raises(RuntimeError):                         # still no CPU path, also with a cache
         attn(torch.randn(1, 1, 64), cache=((torch.zeros(1, 4, 0, 16),) * 2, ((torch.zeros(1, 4, 0, 16),) * 2,) * 2))
+
+
+def test_the_build_finds_the_cuda_libraries_pytorch_uses(tmp_path):
+    """In NVIDIA's wheels beside PyTorch, else in the toolkit; a message that names the places where there is neither."""
+    from native_sparse_attention_pytorch_b200 import build
+    site, toolkit = tmp_path / 'site', tmp_path / 'cuda'
+    with pytest.raises(RuntimeError, match='libcublas.so was found in none of'):
+        build._cuda_library('libcublas', 'cublas', str(site), str(toolkit))
+    for place, names in ((toolkit / 'lib64', ['libcublas.so', 'libcublas.so.12', 'libcublas.so.12.9.1']),
+                         (site / 'nvidia' / 'cublas' / 'lib', ['libcublas.so.12', 'libcublasLt.so.12'])):
+        place.mkdir(parents=True)
+        for name in names:
+            (place / name).touch()
+        assert build._cuda_library('libcublas', 'cublas', str(site), str(toolkit)) == str(place / 'libcublas.so.12')
+
+
+def test_the_build_knows_when_the_host_module_belongs_to_another_pytorch(tmp_path, monkeypatch):
+    from native_sparse_attention_pytorch_b200 import build
+    lib, stamp = tmp_path / '_nsa_host.so', tmp_path / 'built_for.txt'
+    monkeypatch.setattr(build, 'HOST_LIB', str(lib))
+    monkeypatch.setattr(build, 'HOST_STAMP', str(stamp))
+    lib.touch()
+    assert not build._host_fresh()
+    stamp.write_text(build._built_for())
+    assert build._host_fresh()
+    monkeypatch.setattr(torch, '__version__', '0.0.1')
+    assert not build._host_fresh()
