@@ -8,28 +8,42 @@ namespace nsa_host {
 
 class StatusCopy {
  public:
-  StatusCopy() {
-    if (cudaHostAlloc(reinterpret_cast<void**>(&word_), sizeof(int32_t), cudaHostAllocDefault) != cudaSuccess ||
+  // `word` [1]: the device's status word; the event belongs to its device, whichever is current
+  explicit StatusCopy(const Tensor& word) : device_(word.device()) {
+    require_cuda(word);
+    const c10::cuda::CUDAGuard guard(device_);
+    if (cudaHostAlloc(reinterpret_cast<void**>(&word_), sizeof(int32_t), cudaHostAllocPortable) != cudaSuccess ||
         cudaEventCreateWithFlags(&event_, cudaEventDisableTiming) != cudaSuccess)
       throw Error("status poll: no pinned word or event");
     *word_ = 0;
   }
   ~StatusCopy() {
-    cudaEventSynchronize(event_);
-    cudaEventDestroy(event_);
-    cudaFreeHost(word_);
+    if (event_ != nullptr) {
+      cudaEventSynchronize(event_);
+      cudaEventDestroy(event_);
+    }
+    if (word_ != nullptr) cudaFreeHost(word_);
   }
   StatusCopy(const StatusCopy&) = delete;
   void start(const Tensor& word) {
+    const c10::cuda::CUDAGuard guard(device_);
     const cudaStream_t st = (cudaStream_t)stream_of(word);
     if (cudaMemcpyAsync(word_, word.data_ptr(), sizeof(int32_t), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaEventRecord(event_, st) != cudaSuccess)
       throw Error("status poll: the copy could not be issued");
   }
-  bool landed() const { return cudaEventQuery(event_) == cudaSuccess; }
+  // An error of the device is not "still in flight": it is reported here
+  bool landed() const {
+    const cudaError_t rc = cudaEventQuery(event_);
+    if (rc == cudaSuccess) return true;
+    cudaGetLastError();   // "not ready" must not be taken for the failure of a later launch
+    if (rc != cudaErrorNotReady) throw Error(std::string("status poll: ") + cudaGetErrorString(rc));
+    return false;
+  }
   int32_t value() const { return *word_; }
 
  private:
+  c10::Device device_;
   int32_t* word_ = nullptr;
   cudaEvent_t event_ = nullptr;
 };
@@ -37,7 +51,7 @@ class StatusCopy {
 void bind_status(pybind11::module_& m) {
   namespace py = pybind11;
   py::class_<StatusCopy>(m, "StatusCopy")
-      .def(py::init<>())
+      .def(py::init<const Tensor&>())
       .def("start", &StatusCopy::start)
       .def("landed", &StatusCopy::landed)
       .def("value", &StatusCopy::value);

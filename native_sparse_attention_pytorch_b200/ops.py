@@ -114,7 +114,7 @@ def poll_device_status(device):
         return                          # no such kernel since the last copy, and that copy has been read
     with _state_lock:
         if pending is None:
-            pending = _status_polls[key] = [L.host().StatusCopy(), False]
+            pending = _status_polls[key] = [L.host().StatusCopy(acc), False]
         copy, unread = pending
         code = 0
         if unread:

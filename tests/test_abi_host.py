@@ -165,3 +165,8 @@ def test_the_build_knows_when_the_host_module_belongs_to_another_pytorch(tmp_pat
     assert build._host_fresh()
     monkeypatch.setattr(torch, '__version__', '0.0.1')
     assert not build._host_fresh()
+
+
+def test_a_status_copy_wants_a_word_on_a_gpu():
+    with pytest.raises(L.NsaError, match='CUDA tensors only'):
+        L.host().StatusCopy(torch.zeros(1, dtype=torch.int32))
