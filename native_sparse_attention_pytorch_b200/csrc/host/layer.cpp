@@ -691,6 +691,7 @@ struct NativeLayerBackward : torch::autograd::Node {
       const bool eager = capture == cudaStreamCaptureStatusNone;
       std::vector<OptTensor> g = layer_backward(grads[0], w, sv, eps, inv_freq, cfg, status, std::move(needs), eager ? cache.find(swa) : OptTensor(),
                                                 eager ? cache.find(cmp) : OptTensor(), eager);
+      note_backward(x);
       for (int i = 0; i < 1 + kWeights; ++i)
         if (g[i].has_value()) out[i] = std::move(*g[i]);
       if (g[1 + kWeights].has_value()) cache.keep(std::move(swa), *g[1 + kWeights]);

@@ -79,6 +79,10 @@ inline void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream
 // view that made t is a view again instead of a copy.
 Tensor empty_in_order_of(const Tensor& t);
 
+// A native backward has launched kernels that report through the device's status word: the next poll has to copy it (the
+// operators' Python side notes its own calls)
+void note_backward(const Tensor& t);
+
 void bind_status(pybind11::module_& m);
 void bind_selected(pybind11::module_& m);
 void bind_decode(pybind11::module_& m);

@@ -165,6 +165,7 @@ struct NativeSelectedBackward : torch::autograd::Node {
       std::vector<OptTensor> r = sel_backward(q.unpack(getptr()), k.unpack(getptr()), v.unpack(getptr()), opt(idx), opt(mask), out.unpack(getptr()), l,
                                               grads[0], handed_over_delta(grads[0], l), index.defined() ? OptTensor(index) : OptTensor(), block,
                                               diag, impl, scale, status, slot_type.has_value());
+      note_backward(l);
       for (int i = 0; i < 3; ++i) g[i] = std::move(*r[i]);
       if (r[3].has_value()) g[3] = r[3]->to(*slot_type);
     } catch (const Error& e) {

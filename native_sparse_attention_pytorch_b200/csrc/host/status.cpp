@@ -2,9 +2,15 @@
 
 #include <cuda_runtime_api.h>
 
+#include <atomic>
+
 #include "nsa_host.h"
 
 namespace nsa_host {
+
+static std::atomic<bool> g_backward_ran[C10_COMPILE_TIME_MAX_GPUS];
+
+void note_backward(const Tensor& t) { g_backward_ran[t.get_device()].store(true, std::memory_order_release); }
 
 class StatusCopy {
  public:
@@ -50,6 +56,11 @@ class StatusCopy {
 
 void bind_status(pybind11::module_& m) {
   namespace py = pybind11;
+  // Has a native backward launched kernels since `clear` was last asked for?
+  m.def("backward_ran", [](int64_t device, bool clear) {
+    auto& ran = g_backward_ran[device];
+    return clear ? ran.exchange(false, std::memory_order_acq_rel) : ran.load(std::memory_order_acquire);
+  });
   py::class_<StatusCopy>(m, "StatusCopy")
       .def(py::init<const Tensor&>())
       .def("start", &StatusCopy::start)

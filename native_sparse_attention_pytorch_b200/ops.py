@@ -109,8 +109,10 @@ def poll_device_status(device):
     if key is None:
         key = torch.cuda.current_device()
     acc, pending = _status_acc.get(key), _status_polls.get(key)
-    fresh = _status_fresh.get(key)
-    if acc is None or not (fresh or (pending is not None and pending[1])):
+    if acc is None:
+        return
+    fresh = _status_fresh.get(key) or L.host().backward_ran(key, False)
+    if not (fresh or (pending is not None and pending[1])):
         return                          # no such kernel since the last copy, and that copy has been read
     with _state_lock:
         if pending is None:
@@ -124,6 +126,7 @@ def poll_device_status(device):
         pending[1] = bool(fresh) and code == 0
         if pending[1]:
             _status_fresh[key] = False
+            L.host().backward_ran(key, True)
             copy.start(acc)
     if code != 0:
         acc.zero_()

@@ -675,3 +675,31 @@ def test_backward_in_slices_equals_the_whole():
     assert torch.equal(whole[0], torch.cat([h[0] for h in halves], dim=1))
     for i in (1, 2):
         assert_close_bf16(whole[i], torch.cat([h[i] for h in halves], dim=1), 'dk dv', roundings=2, rel_to_max=1e-3)
+
+
+@pytest.mark.parametrize('what', ['operator', 'layer'])
+def test_a_poll_sees_what_a_native_backward_reports(what):
+    """Also when the last poll was between the forward and the backward and no forward of these kernels follows."""
+    from native_sparse_attention_pytorch_b200 import SparseAttention, native_sparse_attend, ops
+    if what == 'operator':
+        q, k, v, idx, mask, up = make_case(1, 8, 2, 300, 64, 3, seed=3)
+        q, k, v, up = (t.bfloat16().to(DEV) for t in (q, k, v, up))
+        x = q.requires_grad_()
+        out = native_sparse_attend(x, k, v, 64, idx.to(DEV), mask.to(DEV))
+    else:
+        layer = SparseAttention(dim=128, dim_head=64, heads=4, kv_heads=2, causal=True, sliding_window_size=64, compress_block_size=32,
+                                compress_block_sliding_stride=16, selection_block_size=64, num_selected_blocks=2,
+                                use_triton_kernel=True).to(DEV).bfloat16()
+        x = torch.randn(1, 200, 128, device=DEV, dtype=torch.bfloat16, requires_grad=True)
+        out = layer(x)
+        up = torch.randn_like(out)
+    for _ in range(3):
+        torch.cuda.synchronize()
+        ops.poll_device_status(DEV)                         # nothing is left to read
+    out.backward(up)
+    ops._status_tensor(out.device).fill_(1)                 # as a kernel of the backward that gave up would
+    ops.poll_device_status(DEV)
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match='bounded wait'):
+        ops.poll_device_status(DEV)
+    ops.check_device_status()
