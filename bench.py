@@ -81,16 +81,6 @@ PREFILL_WORKLOADS = {
 }
 
 
-# dram__bytes_read.sum + dram__bytes_write.sum per launch, from single-launch ncu captures of this command
-# (`ncu --set full -k regex:<kernel> -c 1 python bench.py --steps 2 --warmup 3 --no-cpu-baseline`), taken
-# while the partial rows still left row by row; their amount is the same.
-NCU_DRAM_BYTES = {
-    'sel_bwd_ws_kernel': 701.6e6 + 2195.7e6,
-    'sel_fwd_kernel': 902.5e6 + 2425.9e6,
-    'sel_merge_kernel': 2417.0e6,      # dram__bytes.sum.per_second x gpu__time_duration of a sections-only capture
-    'sel_dq_merge_kernel': 2312.0e6,
-    'sel_delta_kernel': 276.0e6,
-}
 # the other workloads whose numbers ride on the default line: (name, timed steps)
 EXTRA_WORKLOADS = (('layer_fwd_bwd_b2_n16384_dim1024_h16kv4_d64', 5), ('prefill_b1_n65536_h64kv8_d128', 3),
                    ('lm_step_b8_n8192_dim512_depth8', 3))
@@ -463,8 +453,6 @@ def main():
             'gpu_launches': launches,
             'clocks': clocks,
         }
-        top = max(line['roofline']['kernels'] or [{'dram_bytes': None, 'ms': 0}], key=lambda r: r['ms'])
-        line['roofline']['traffic'] = top.get('dram_bytes')
         if args.rows and world == 1:
             del q, k, v, idx, mask, do
             line['rows'] = measure_rows(dev, flush)
@@ -515,8 +503,7 @@ def kernel_rows(breakdown, w, mask, f_fwd, f_bwd, tensor_peak):
             rate = amount / (us / 1e6)
             row.update(bound=bound, work=amount, achieved=rate / (1e12 if bound == 'tensor' else 1e9),
                        unit='TFLOP/s' if bound == 'tensor' else 'GB/s',
-                       frac=rate / ((tensor_peak * 1e12) if bound == 'tensor' else (hbm * 1e9)),
-                       dram_bytes=NCU_DRAM_BYTES.get(key))
+                       frac=rate / ((tensor_peak * 1e12) if bound == 'tensor' else (hbm * 1e9)))
         out.append(row)
     total = sum(r['ms'] * r['launches_per_step'] for r in out)
     for r in out:

@@ -154,8 +154,8 @@ int nsa_sel_bwd(const nsa_sel_bwd_args* args, void* stream);
 int64_t nsa_sel_index_bytes(const nsa_sel_fwd_args* args);
 
 /* 1 when the backward of this problem stores every row of dq in one ordered
- * pass (the tensor-core family at dim_head 64) instead of adding into it, 0
- * otherwise, negative = NSA_ERR_*.  Where it is 1 the caller may set
+ * pass in the dtype of q (the tensor-core family), 0 otherwise, negative =
+ * NSA_ERR_*.  Where it is 1 the caller may set
  * `dq_out` (rows of dim_head contiguous elements in the dtype of q, 16-byte
  * aligned, any batch / head / row strides -- for instance the layout of q
  * itself) and pass dq = NULL: dq is then written there, already rounded, and
@@ -270,8 +270,8 @@ int nsa_cmp_fwd_pools(const nsa_cmp_fwd_args* args);
 int64_t nsa_cmp_workspace_bytes(const nsa_cmp_fwd_args* args, int backward);
 
 /* Backward of the compressed branch (autograd of NSA:621-639 in upstream).
- * dq [B,q_heads,N,d], dck, dcv [B,kv_heads,num_mem+ncb,d] contiguous fp32,
- * zeroed by the call.  The importance output carries no gradient. */
+ * dq [B,q_heads,N,d], dck, dcv [B,kv_heads,num_mem+ncb,d] contiguous fp32;
+ * dck and dcv are zeroed by the call before accumulation.  The importance output carries no gradient. */
 typedef struct {
   nsa_cmp_fwd_args fwd;
   nsa_tensor dout;
@@ -355,8 +355,8 @@ int64_t nsa_swa_workspace_bytes(const nsa_swa_fwd_args* args, int backward);
 typedef struct {
   nsa_swa_fwd_args fwd;
   nsa_tensor dout;
-  float* dq;             /* contiguous fp32, zeroed by the call               */
-  float* dk;
+  float* dq;             /* contiguous fp32, written                          */
+  float* dk;             /* contiguous fp32, as in nsa_sel_bwd_args           */
   float* dv;
   nsa_tensor dq_out;     /* optional, as in nsa_sel_bwd_args */
   const void* index;     /* optional, see nsa_swa_index_bytes */

@@ -172,7 +172,7 @@ int64_t nsa_sel_workspace_bytes(const nsa_sel_fwd_args* a, int backward) {
   return need;
 }
 
-// dq_out: rows of dim_head elements in the dtype of q; only the tensor-core family at dim_head 64 writes it
+// dq_out: rows of dim_head elements in the dtype of q; only the tensor-core family writes it
 static int check_dq_out(const nsa_tensor& t, int dtype, bool served) {
   if (t.ptr == nullptr) return NSA_OK;
   if (!served) return fail(NSA_ERR_UNSUPPORTED, "dq_out: this problem's backward does not store dq in one pass (see *_bwd_stores_dq)");
@@ -256,7 +256,7 @@ int nsa_sel_bwd(const nsa_sel_bwd_args* a, void* stream) {
   AttnParams P;
   NSA_TRY(fill_sel(P, a->fwd));
   NSA_TRY(check_tensor(a->dout, a->fwd.dtype, "dout"));
-  // dk and dv are accumulated into; dq too, unless the kernels that will run store every row of it
+  // dk and dv are accumulated into; every kernel stores dq, and the tensor-core ones can do so in q's type (dq_out)
   const bool dq_stored = a->fwd.impl != NSA_IMPL_SIMT && sm100_sel_bwd_overwrites_dq(a->fwd);
   NSA_TRY(check_dq_out(a->dq_out, a->fwd.dtype, dq_stored));
   if ((!a->dq && !a->dq_out.ptr) || !a->dk || !a->dv) return fail(NSA_ERR_NULL, "dq/dk/dv: NULL pointer");

@@ -753,9 +753,9 @@ int launch_decode(const DecodeParams& P, int dtype, cudaStream_t stream) {
 // y = norm(x) W^T for up to 16 token rows x, and behind the rows of W the gates: sigmoid(norm(x) Wg^T + bg); also the two
 // layers of the compress networks when a window has filled up, keys and values side by side.
 // Bound: the weights, read once.  bf16: a CTA owns 16 rows of W and requests all of them with cp.async before it
-// normalises the token rows, then one warp walks K with m16n8k16 products in the order the library's GEMM does (the
-// results are the same bits, so nothing downstream, the block selection included, depends on which of the two ran).
-// fp32: a warp owns a pair of rows and uses CUDA cores.
+// normalises the token rows, then one warp walks K upwards with m16n8k16 products, fp32 accumulators.
+// fp32: a warp owns a pair of rows and uses CUDA cores.  Beside a library GEMM, which serves more than 16 rows, the results
+// agree as two orders of the same fp32 sum do.
 
 constexpr int kProjWarps = 8;
 constexpr int kProjRows = 16;

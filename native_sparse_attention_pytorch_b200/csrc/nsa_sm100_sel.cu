@@ -231,9 +231,14 @@ __device__ __forceinline__ int2 block_scan2(int2 v, int2* total, int2 (*warp_sum
 // A list is cut into items of at most kChunksPerItem chunks, fewer when the whole problem has few chunks: an item is
 // what one CTA walks serially, so a problem of a few hundred chunks in items of sixteen leaves most of the chip idle.
 // The line is 16 items per SM at dim_head 64 and 8 at 128, where an item's K/V loads and dK/dV flush cost twice as much
-// and the forward has two CTAs per SM instead of four.  Below it these costs outweigh the imbalance of long items: 3001
-// positions, 16 / 2 heads of 128, backward + forward 198 us with 16, 160 with 8, 158 with 5, 173 with 3; 3 x 4997, 8 / 4 heads
-// of 64 545 us with 16, 614 with 8.
+// and the forward has two CTAs per SM instead of four; below it these costs outweigh the imbalance of long items.  All
+// kernels of the selected branch, forward + backward, in us with 4 / 8 / 16 / 32 items per SM:
+//   64:  1 x 3001, 16 / 4 heads 145 147 160 160; 4 x 2048, 8 / 4 307 285 288 311; 2 x 4096, 16 / 2 537 521 505 528;
+//        1 x 8192, 32 / 4 1024 1023 994 989; 4 x 8192, 32 / 4 the same within 0.2 % (3763)
+//   128: 1 x 3001, 16 / 2 273 268 308 308; 4 x 2048, 8 / 4 558 519 514 589; 2 x 4096, 16 / 2 1061 1024 981 1020;
+//        2 x 8192, 16 / 4 1371 1370 1278 1281; 1 x 8192, 32 / 4 2093 2093 2035 2024
+// so either line is right for some sizes and costs others: 8 at 128 keeps the short ones from losing 15 %, where 16 would
+// give the longer ones 3 to 7 %.
 static int items_target(int D) { return 148 * (D == 64 ? 16 : 8); }
 __global__ void __launch_bounds__(1024) sel_items_kernel(const int* totals, int* list_base, int* list_item, int* cursors, int4* items,
                                                          int* num_items, int nlists, int QT, int target, uint32_t tag) {

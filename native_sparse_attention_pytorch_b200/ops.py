@@ -31,11 +31,11 @@ def _sel_args(q, k, v, out, idx, mask, lse, block, diag, impl, scale):
                         workspace=None, workspace_bytes=0, status=_status_word(q.device))
 
 
-# Device status of the tensor-core kernels.  Every such kernel reports through the first word of its work buffer:
-# 0 = fine, 1 = a bounded wait ran out (results invalid), 2 = it was handed an index built for another problem.  The
-# operators hand the kernels one int32 per device to OR into instead (`status`), so nothing is lost however many
-# kernels run between two checks, and nothing is launched to collect it.  The autograd engine calls the backward functions from its own thread: one lock guards the
-# tables below.
+# Device status of the tensor-core kernels: 0 = fine, 1 = a bounded wait ran out (results invalid), 2 = handed an index built
+# for another problem.  A kernel reports through the first word of its work buffer unless it is given a word to OR into
+# (`status` in the argument structs); the operators hand them one int32 per device, so nothing is lost however many kernels
+# run between two checks, and nothing is launched to collect it.  The autograd engine calls the backward functions from its
+# own thread: one lock guards the tables below.
 _state_lock = threading.Lock()
 _status_acc = {}      # device index -> int32[1] device tensor
 _status_fresh = {}    # device index -> a call has been handed the word since the last poll copied it
