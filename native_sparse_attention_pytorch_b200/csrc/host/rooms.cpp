@@ -1,5 +1,7 @@
 #include "rooms.h"
 
+#include "nsa_kernels.h"
+
 #include <ATen/core/LegacyTypeDispatch.h>
 
 namespace nsa_host {
@@ -49,6 +51,26 @@ GrownPair Rooms::fresh(const Tensor& like, int64_t batch, int64_t heads, int64_t
   return g;
 }
 
+// The rows of k and v to the front of the buffers of g.  Caches whose heads are runs of whole 16-byte pieces at one distance
+// from each other (all that come from here) go in one launch.
+static void copy_rows(const GrownPair& g, const Tensor& k, const Tensor& v) {
+  const int64_t B = k.size(0), H = k.size(1), rows = k.size(2), d = k.size(3), el = k.element_size();
+  if (B * H * rows == 0) return;
+  auto whole = [&](const void* p, int64_t step) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && step * el % 16 == 0; };
+  const bool runs = k.strides() == v.strides() && k.stride(3) == 1 && (rows == 1 || k.stride(2) == d) && (B == 1 || k.stride(0) == k.stride(1) * H) &&
+                    d * el % 16 == 0 && whole(k.data_ptr(), k.stride(1)) && whole(v.data_ptr(), k.stride(1)) && k.scalar_type() == g.k.scalar_type() &&
+                    v.scalar_type() == g.k.scalar_type();
+  if (!runs) {
+    rows_of(g.k, 0, rows).copy_(k);
+    rows_of(g.v, 0, rows).copy_(v);
+    return;
+  }
+  nsa::CacheCopy c = {};
+  c.src[0] = k.data_ptr(); c.src[1] = v.data_ptr(); c.dst[0] = g.k_buf; c.dst[1] = g.v_buf;
+  c.src_step = k.stride(1) * el / 16; c.dst_step = g.k.stride(1) * el / 16; c.pieces = rows * d * el / 16; c.heads = (int)(B * H);
+  check(nsa::launch_cache_copy(c, (cudaStream_t)stream_of(k)));
+}
+
 GrownPair Rooms::extend(const Tensor& k, const Tensor& v, int64_t room) {
   at::AutoDispatchBelowADInplaceOrView no_view_tracking;
   const int64_t B = k.size(0), H = k.size(1), rows = k.size(2), d = k.size(3);
@@ -75,10 +97,7 @@ GrownPair Rooms::extend(const Tensor& k, const Tensor& v, int64_t room) {
     }
   }
   GrownPair g = fresh(k, B, H, rows + 1, room, d);
-  if (rows > 0) {
-    rows_of(g.k, 0, rows).copy_(k);
-    rows_of(g.v, 0, rows).copy_(v);
-  }
+  copy_rows(g, k, v);
   return g;
 }
 

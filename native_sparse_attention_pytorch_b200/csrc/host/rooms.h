@@ -7,8 +7,8 @@
 // copied into a new buffer: a second continuation of one cache, also when the first one has been dropped (kernels of other
 // streams may still read its rows, which the allocator knows and this table does not); a continuation on another stream
 // (whose tensors have to be that stream's own); a cache from elsewhere; no room left.  A step that is recorded into a CUDA
-// graph appends only to buffers of the same recording: a replay writes the same rows again.  What the copy costs where
-// one prompt is continued again and again: 4 x 32768 cached rows of 2 heads of 128, 115 us per continuation.
+// graph appends only to buffers of the same recording: a replay writes the same rows again.  The copy is one
+// launch (cache_copy_kernel).
 #pragma once
 
 #include <mutex>

@@ -748,6 +748,39 @@ int launch_decode(const DecodeParams& P, int dtype, cudaStream_t stream) {
   return dtype == NSA_F32 ? launch_decode_t<float>(P, stream) : launch_decode_t<__nv_bfloat16>(P, stream);
 }
 
+// ---- a cache that cannot grow where it is ------------------------------------------------------------------------
+//
+// Keys and values in one launch, 16 bytes per access and four of them in flight per thread.  Bound: HBM.  As two tensor
+// copies (strided, 2 bytes per access) the 134 MB of 4 x 32768 rows of 2 heads of 128 made a pass of 8 steps 568 us, so 453,
+// what it takes without any copy; 16 steps at 300 rows 505 -> 479.
+__global__ void __launch_bounds__(256) cache_copy_kernel(const CacheCopy P) {
+  const int which = blockIdx.z;
+  for (int head = blockIdx.y; head < P.heads; head += gridDim.y) {
+    const uint4* src = static_cast<const uint4*>(P.src[which]) + head * P.src_step;
+    uint4* dst = static_cast<uint4*>(P.dst[which]) + head * P.dst_step;
+    for (int64_t i = (int64_t)blockIdx.x * 1024 + threadIdx.x; i < P.pieces; i += (int64_t)gridDim.x * 1024) {
+      uint4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (i + u * 256 < P.pieces) v[u] = src[i + u * 256];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (i + u * 256 < P.pieces) dst[i + u * 256] = v[u];
+    }
+  }
+}
+
+int launch_cache_copy(const CacheCopy& P, cudaStream_t stream) {
+  if (P.pieces == 0 || P.heads == 0) return NSA_OK;
+  if (!aligned16(P.src[0], P.src[1], P.dst[0], P.dst[1])) return fail(NSA_ERR_ALIGN, "cache copy: rows must start on 16-byte boundaries");
+  const int64_t chunks = (P.pieces + 1023) / 1024, most = 148 * 16 / (2 * (int64_t)P.heads) + 1;   // about 16 blocks per SM in all
+  const dim3 grid((unsigned)(chunks < most ? chunks : most), (unsigned)(P.heads < 65535 ? P.heads : 65535), 2);
+  cache_copy_kernel<<<grid, 256, 0, stream>>>(P);
+  count_launches(1);
+  const cudaError_t err = cudaGetLastError();
+  return err == cudaSuccess ? NSA_OK : fail((int)err, cudaGetErrorString(err));
+}
+
 // ---- the projections of a step ---------------------------------------------------------------------------------
 //
 // y = norm(x) W^T for up to 16 token rows x, and behind the rows of W the gates: sigmoid(norm(x) Wg^T + bg); also the two

@@ -140,6 +140,15 @@ struct ProjectParams {
   float eps;
 };
 
+// The rows of a key and a value cache into larger ones: per head one contiguous run of `pieces` sixteen-byte pieces, the heads
+// `src_step` / `dst_step` pieces apart
+struct CacheCopy {
+  const void* src[2];
+  void* dst[2];
+  int64_t src_step, dst_step, pieces;
+  int heads;
+};
+
 // The passes of a layer step between its GEMMs and its attention kernels (see nsa_layer.cu)
 struct LayerShape {
   int batch, seq, heads, kv_heads, d, ncb, cbs, stride, num_mem;
@@ -192,6 +201,7 @@ int launch_pos_grad(const LayerShape& L, const void* dkw, const void* dvw, float
 int launch_round(const float* src, void* dst, int64_t n, cudaStream_t stream);
 int launch_decode(const DecodeParams& P, int dtype, cudaStream_t stream);
 int fill_decode(DecodeParams& P, const nsa_decode_args& a);   // checks the arguments; q and qr may be NULL
+int launch_cache_copy(const CacheCopy& P, cudaStream_t stream);
 bool project_serves(int batch, int dim, int dtype);
 int launch_project(const ProjectParams& P, int dtype, cudaStream_t stream);
 

@@ -197,3 +197,27 @@ def test_step_on_caches_as_long_as_shared_memory_allows(case):
     gate = f(gates)
     want = (gate[:, 0:1] * o_cmp + gate[:, 1:2] * o_sel + gate[:, 2:3] * o_swa).reshape(1, -1)
     (assert_close_f32 if dtype == torch.float32 else assert_close_bf16)(got, want.float().cpu(), 'merged row')
+
+
+# (batch, heads, rows, head size, dtype): one piece per row and many, runs of less and more than a block's share, one head and
+# many; then views whose heads are not runs, or not on 16-byte boundaries
+@pytest.mark.parametrize('case', [(1, 1, 1, 8, torch.bfloat16), (2, 3, 5, 40, torch.float32), (1, 1, 255, 64, torch.bfloat16), (3, 2, 129, 64, torch.bfloat16),
+                                  (1, 2, 70000, 128, torch.bfloat16), (64, 8, 33, 64, torch.float32)])
+@pytest.mark.parametrize('form', ['dense', 'front cut', 'batch part', 'positions first', 'odd offset'])
+def test_a_cache_that_cannot_grow_in_place_is_copied_whole(case, form):
+    b, h, rows, d, dtype = case
+    layer = build(dtype, 2 * h, h, d, dim=64)
+    gen = torch.Generator(DEV).manual_seed(rows)
+
+    def cache(n):
+        shape = {'dense': (b, h, n, d), 'front cut': (b, h, n + 2, d), 'batch part': (b + 1, h, n, d), 'positions first': (b, n, h, d)}.get(form)
+        if form == 'odd offset':
+            return torch.randn(b * h * n * d + 1, device=DEV, generator=gen).to(dtype)[1:].view(b, h, n, d)
+        t = torch.randn(shape, device=DEV, generator=gen).to(dtype)
+        return {'dense': t, 'front cut': t[:, :, 2:], 'batch part': t[1:], 'positions first': t.transpose(1, 2)}[form]
+    k, v, run_k, run_v = cache(rows), cache(rows), cache(7), cache(7)
+    empty = torch.zeros(b, h, 0, d, device=DEV, dtype=dtype)
+    with torch.no_grad():
+        _, got = layer(torch.randn(b, 1, 64, device=DEV, generator=gen).to(dtype), cache=((k, v), ((empty, empty), (run_k, run_v))), return_cache=True)
+    for old, new in ((k, got[0][0]), (v, got[0][1]), (run_k, got[1][1][0]), (run_v, got[1][1][1])):
+        assert new.shape[2] == old.shape[2] + 1 and torch.equal(new[:, :, :-1], old)
