@@ -12,6 +12,7 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
 
+#include <climits>
 #include <cmath>
 #include <limits>
 #include <list>
@@ -87,6 +88,87 @@ static Tensor product(Op op, const Tensor& A, const Tensor& B) {
   gemm(op, A.scalar_type(), M, N, K, A.data_ptr(), B.data_ptr(), C.data_ptr());
   return C;
 }
+
+// Products that do not depend on one another: in one launch of nsa_gemm.cu, or one library GEMM each.
+//   fp32: in one launch, unless the program allows TF32 (which the library's kernels then use) or changed the settings above.
+//   bf16: while the K steps of the tiles come to at most kStepsPerSM per SM.  Beyond that the library's larger tiles, which
+//   read the operands a quarter as often, win on the GPU: the last products of a layer's backward, own kernel against library,
+//   with 4 steps per SM (1024 rows, dim 256) 16 us against 21, with 7 (512 rows, dim 512) 23 against 17, with 29 (2048 rows)
+//   47 against 24; on the host the launch is 4 us, a library product 12 to 17.
+class Products {
+ public:
+  struct Product {
+    Op op;
+    Tensor A, B, C;         // matrices; C dense
+    Tensor A2, B2;          // a second product that is added, or undefined
+    Tensor act;             // own kernel only: zero where this is not positive,
+    float* sums = nullptr;  // and the column sums of the result are added here
+  };
+  Products(at::ScalarType type, int32_t* status) : type_(type), status_(status) { items_.reserve(nsa::GemmGroup::kMost); }
+  Product& add(Op op, const Tensor& A, const Tensor& B, const Tensor& C) {
+    items_.push_back({op, A, B, C});
+    return items_.back();
+  }
+  // False: by the library, which leaves `act` and `sums` to the caller
+  bool run(cudaStream_t stream) const {
+    nsa::GemmGroup g;
+    const bool own = grouped(g);
+    if (own) check(nsa::launch_gemm(g, code(), stream));
+    else
+      for (const Product& p : items_) library(p);
+    return own;
+  }
+  // The products as one launch; false where the library serves better, or has to
+  bool grouped(nsa::GemmGroup& g) const {
+    g = {};
+    g.status = status_;
+    int64_t steps = 0, most = 0;
+    for (const Product& p : items_) {
+      nsa::GemmTask& t = g.task[g.tasks++];
+      t.op = p.op == Op::NT ? nsa::kGemmNT : p.op == Op::NN ? nsa::kGemmNN : nsa::kGemmTN;
+      t.m = (int)p.C.size(0); t.n = (int)p.C.size(1);
+      int64_t deep = 0;
+      auto part = [&](int i, const Tensor& A, const Tensor& B) {
+        const int64_t K = depth(p, A);
+        t.a[i] = A.data_ptr(); t.lda[i] = A.size(1);
+        t.b[i] = B.data_ptr(); t.ldb[i] = B.size(1);
+        t.k[i] = (int)K;
+        deep += (K + 63) / 64;
+        most = std::max({most, K, A.size(1), B.size(1)});
+      };
+      part(0, p.A, p.B);
+      if (p.A2.defined()) part(1, p.A2, p.B2);
+      t.act = ptr<void>(p.act); t.sums = p.sums; t.c = p.C.data_ptr();
+      steps += (p.C.size(0) + 127) / 128 * ((p.C.size(1) + 63) / 64) * deep;
+      most = std::max({most, p.C.size(0), p.C.size(1)});
+    }
+    if (most >= INT_MAX || !default_blas(type_) || !nsa::gemm_serves(g, code())) return false;
+    return type_ == at::kFloat ? !at::globalContext().allowTF32CuBLAS() : steps <= 148 * kStepsPerSM;
+  }
+
+ private:
+  static constexpr int64_t kStepsPerSM = 5;
+  std::vector<Product> items_;
+  at::ScalarType type_;
+  int32_t* status_;
+
+  int code() const { return type_ == at::kFloat ? NSA_F32 : NSA_BF16; }
+  static int64_t depth(const Product& p, const Tensor& A) { return A.size(p.op == Op::TN ? 0 : 1); }
+  void library(const Product& p) const {
+    const Tensor a = p.op == Op::TN ? p.A.t() : p.A, b = p.op == Op::NT ? p.B.t() : p.B;
+    Tensor c = p.C;
+    auto issue = [&](const Tensor& A, const Tensor& B, float beta) {
+      gemm(p.op, type_, c.size(0), c.size(1), depth(p, A), A.data_ptr(), B.data_ptr(), c.data_ptr(), beta);
+    };
+    if (default_blas(type_)) {
+      issue(p.A, p.B, 0.f);
+      if (p.A2.defined()) issue(p.A2, p.B2, 1.f);
+    } else {
+      at::mm_out(c, a, b);
+      if (p.A2.defined()) c.addmm_(p.op == Op::TN ? p.A2.t() : p.A2, p.op == Op::NT ? p.B2.t() : p.B2);
+    }
+  }
+};
 
 // A [B, H, N, d] view without a tensor: pointer and strides in elements
 static nsa_tensor heads_view(void* p, int64_t sb, int64_t sh, int64_t sn) { return {p, sb, sh, sn}; }
@@ -233,6 +315,8 @@ static std::vector<OptTensor> layer_forward(Tensor x, std::vector<OptTensor> wei
       xn = at::rms_norm(x2, {L.dim}, w.norm, eps);
     }
   }
+  // The products in front of the ReLU and the selection stay with the library, as in the layer run module by module: a value
+  // that rounds the other way there switches a hidden unit or a block, and the two forms of the layer have to agree.
   const Tensor qkv = product(Op::NT, xn, w.qkv);
   const Tensor logits = at::addmm(w.gate_b, xn, w.gate.t());
   if (!save) xn = Tensor();   // here and below: what nobody needs any more makes room for the partial results
@@ -348,7 +432,12 @@ static std::vector<OptTensor> layer_forward(Tensor x, std::vector<OptTensor> wei
     check(rc);
   }
   // output projection
-  const Tensor out = product(Op::NT, merged, w.out).view({B, N, L.dim});
+  const Tensor out = at::empty({B, N, L.dim}, x.options());
+  {
+    Products p(type, L.status);
+    p.add(Op::NT, merged, w.out, out.view({BN, L.dim}));
+    p.run(st);
+  }
 
   auto opt = [](const Tensor& t) { return t.defined() ? OptTensor(t) : OptTensor(); };
   std::vector<OptTensor> result = {out};
@@ -457,7 +546,17 @@ static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor>
   dout = dout.reshape({BN, L.dim}).contiguous();
   // (what a later step does not need is given back as soon as it has been used: the partial results of the branches are
   // larger than all of it together)
-  Tensor d_merged = product(Op::NN, dout, w.out);
+  std::vector<OptTensor> g(1 + kWeights);
+  Tensor d_merged = at::empty({BN, c.heads * d}, x.options());
+  {
+    Products p(type, L.status);
+    p.add(Op::NN, dout, w.out, d_merged);
+    if (needs[5]) {
+      g[5] = at::empty({L.dim, c.heads * d}, x.options());
+      p.add(Op::TN, dout, merged, *g[5]);
+    }
+    p.run(st);
+  }
   Slab tmp;
   const int64_t t_delta = tmp.add(3 * L.rows(H) * 4), t_gates = tmp.add(nsa::gate_sums_partial((int)(3 * H)) * 4);
   tmp.allocate(x);
@@ -553,21 +652,41 @@ static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor>
   const Tensor dc = at::empty({2, wins, d}, x.options());
   check(nsa::launch_split_mem(L.shape, dck, dc.data_ptr(), small + s_mem, small + s_b2, L.dt, st));
   const Tensor dck_rows = dc.select(0, 0), dcv_rows = dc.select(0, 1);
-  Tensor dhk = product(Op::NN, dck_rows, w.k2), dhv = product(Op::NN, dcv_rows, w.v2);
+  Tensor dhk = at::empty({wins, hid}, x.options()), dhv = at::empty({wins, hid}, x.options());
+  auto weight_grad = [&](Products& p, int i, const Tensor& dy, const Tensor& in) {   // of a weight [features of dy, features of in]
+    if (!needs[i]) return;
+    g[i] = at::empty({dy.size(1), in.size(1)}, x.options());
+    p.add(Op::TN, dy, in, *g[i]);
+  };
   {
-    nsa::ColumnSums p = {};
-    p.x[0] = dhk.data_ptr(); p.x[1] = dhv.data_ptr(); p.act[0] = hk.data_ptr(); p.act[1] = hv.data_ptr();
-    p.out[0] = small + s_b1; p.out[1] = small + s_b1 + hid;
-    p.rows = wins; p.cols = hid; p.sets = 2;
-    check(nsa::launch_relu_sums(p, L.dt, st));
+    Products p(type, L.status);
+    auto hidden_grad = [&](const Tensor& dy, const Tensor& weight, const Tensor& act, const Tensor& dh, float* sums) {
+      auto& q = p.add(Op::NN, dy, weight, dh);
+      q.act = act;
+      q.sums = sums;
+    };
+    hidden_grad(dck_rows, w.k2, hk, dhk, small + s_b1);
+    hidden_grad(dcv_rows, w.v2, hv, dhv, small + s_b1 + hid);
+    weight_grad(p, 11, dck_rows, hk);
+    weight_grad(p, 15, dcv_rows, hv);
+    if (!p.run(st)) {
+      nsa::ColumnSums r = {};
+      r.x[0] = dhk.data_ptr(); r.x[1] = dhv.data_ptr(); r.act[0] = hk.data_ptr(); r.act[1] = hv.data_ptr();
+      r.out[0] = small + s_b1; r.out[1] = small + s_b1 + hid;
+      r.rows = wins; r.cols = hid; r.sets = 2;
+      check(nsa::launch_relu_sums(r, L.dt, st));
+    }
   }
-  std::vector<OptTensor> g(1 + kWeights);
   const Tensor kw = kept_view(at_win, {wins, width}, type), vw = kept_view(at_win + wins * width * el, {wins, width}, type);
-  if (needs[11]) g[11] = product(Op::TN, dck_rows, hk);
-  if (needs[15]) g[15] = product(Op::TN, dcv_rows, hv);
-  if (needs[9]) g[9] = product(Op::TN, dhk, kw);
-  if (needs[13]) g[13] = product(Op::TN, dhv, vw);
-  Tensor dkw = product(Op::NN, dhk, w.k1), dvw = product(Op::NN, dhv, w.v1);
+  Tensor dkw = at::empty({wins, width}, x.options()), dvw = at::empty({wins, width}, x.options());
+  {
+    Products p(type, L.status);
+    weight_grad(p, 9, dhk, kw);
+    weight_grad(p, 13, dhv, vw);
+    p.add(Op::NN, dhk, w.k1, dkw);
+    p.add(Op::NN, dhv, w.v1, dvw);
+    p.run(st);
+  }
   dhk = dhv = Tensor();
   check(nsa::launch_pos_grad(L.shape, dkw.data_ptr(), dvw.data_ptr(), small + s_pos, L.dt, st));
 
@@ -579,13 +698,23 @@ static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor>
   dkw = dvw = Tensor();
   check(nsa::launch_gate_sums(d_logits.data_ptr(), small + s_gate, BN, (int)(3 * H), reinterpret_cast<float*>(tmp.at(t_gates)),
                               reinterpret_cast<unsigned*>(dk + a_counters), L.dt, st));
-  if (needs[5]) g[5] = product(Op::TN, dout, merged);
-  if (needs[2]) g[2] = product(Op::TN, d_qkv, xn);
-  if (needs[3]) g[3] = product(Op::TN, d_logits, xn);
+  Tensor dxn;
+  {
+    Products p(type, L.status);
+    weight_grad(p, 2, d_qkv, xn);
+    // (in bf16 the library splits this sum over the rows and adds its parts in bf16; the modules' gradient, which this one is
+    // compared with, is off by that)
+    if (type == at::kFloat) weight_grad(p, 3, d_logits, xn);
+    else if (needs[3]) g[3] = product(Op::TN, d_logits, xn);
+    if (needs[0] || needs[1]) {
+      dxn = at::empty({BN, L.dim}, x.options());
+      auto& q = p.add(Op::NN, d_qkv, w.qkv, dxn);
+      q.A2 = d_logits;
+      q.B2 = w.gate;
+    }
+    p.run(st);
+  }
   if (needs[0] || needs[1]) {
-    Tensor dxn = product(Op::NN, d_qkv, w.qkv);
-    if (default_blas(type)) gemm(Op::NN, type, BN, L.dim, 3 * H, d_logits.data_ptr(), w.gate.data_ptr(), dxn.data_ptr(), 1.f);
-    else dxn.addmm_(d_logits, w.gate);
     if (w.norm.defined()) {
       const Tensor dx = at::empty({BN, L.dim}, x.options());
       nsa::NormParams p = {};
@@ -734,8 +863,46 @@ static Tensor layer_apply(Tensor x, std::vector<OptTensor> weights, double eps, 
   return out;
 }
 
+// One launch of the grouped products on dense matrices, for tests: (op, A, B, act, A2, B2) each -> C and, with
+// act, the column sums of C; cols and split as in GemmGroup
+static std::vector<Tensor> products_together(
+    std::vector<std::tuple<int64_t, Tensor, Tensor, OptTensor, OptTensor, OptTensor>> tasks, int64_t status, int cols, int split) {
+  std::vector<Tensor> result;
+  if (tasks.empty() || tasks.size() > (size_t)nsa::GemmGroup::kMost) throw Error("products: one to four of them");
+  const Tensor& like = std::get<1>(tasks[0]);
+  require_cuda(like);
+  const c10::cuda::CUDAGuard guard(like.device());
+  Products p(like.scalar_type(), reinterpret_cast<int32_t*>(status));
+  for (const auto& [op_code, A, B, act, A2, B2] : tasks) {
+    const Op op = op_code == 0 ? Op::NT : op_code == 1 ? Op::NN : Op::TN;
+    auto rows = [&](const Tensor& a) { return a.size(op == Op::TN ? 1 : 0); };
+    auto cols = [&](const Tensor& b) { return b.size(op == Op::NT ? 0 : 1); };
+    auto deep = [&](const Tensor& a, const Tensor& b) {
+      return a.dim() == 2 && b.dim() == 2 && a.is_contiguous() && b.is_contiguous() && a.scalar_type() == like.scalar_type() &&
+             b.scalar_type() == like.scalar_type() && a.device() == like.device() && b.device() == like.device() &&
+             a.size(op == Op::TN ? 0 : 1) == b.size(op == Op::NT ? 1 : 0) && a.numel() < INT_MAX && b.numel() < INT_MAX;
+    };
+    if (!deep(A, B) || A2.has_value() != B2.has_value() || (A2.has_value() && (!deep(*A2, *B2) || rows(*A2) != rows(A) || cols(*B2) != cols(B))) ||
+        (act.has_value() && !fits(act, like, {rows(A), cols(B)})))
+      throw Error("products: matrices that do not go together");
+    const Tensor C = at::empty({rows(A), cols(B)}, like.options()), sums = at::zeros({cols(B)}, like.options().dtype(at::kFloat));
+    auto& q = p.add(op, A, B, C);
+    q.act = act.value_or(Tensor());
+    q.A2 = A2.value_or(Tensor()); q.B2 = B2.value_or(Tensor());
+    if (act.has_value()) q.sums = ptr<float>(sums);
+    result.insert(result.end(), {C, sums});
+  }
+  nsa::GemmGroup g;
+  p.grouped(g);
+  g.cols = cols;
+  g.split = split;
+  check(nsa::launch_gemm(g, dtype_code(like), (cudaStream_t)stream_of(like)));
+  return result;
+}
+
 void bind_layer(pybind11::module_& m) {
   namespace py = pybind11;
+  m.def("products_together", &products_together, py::call_guard<py::gil_scoped_release>());
   m.def("layer_takes", &layer_takes);
   m.def("layer_forward", &layer_forward, py::call_guard<py::gil_scoped_release>());
   m.def("layer_apply", &layer_apply, py::call_guard<py::gil_scoped_release>());

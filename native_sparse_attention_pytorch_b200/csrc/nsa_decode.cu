@@ -38,22 +38,11 @@ __device__ __forceinline__ void store_vec(T* dst, const float* x) {
   for (int e = 0; e < Elem<T>::kVec; e += 2) Elem<T>::store2(dst + e, x[e], x[e + 1]);
 }
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-// The address of this CTA's shared-memory location in CTA `rank` of the cluster
-__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void st_cluster(uint32_t addr, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
-}
+using ptx::cluster_arrive;
+using ptx::cluster_rank;
+using ptx::cluster_wait;
+using ptx::map_rank;
+using ptx::st_cluster;
 
 // A tile of up to kTile consecutive keys (kLongTile in the form for very long caches): where its rows are
 constexpr int kTile = 16, kLongTile = 4;

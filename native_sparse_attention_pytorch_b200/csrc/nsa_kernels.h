@@ -176,6 +176,29 @@ struct QkvGrad {
   void* out;                         // [B, N, (Hq + 2 Hkv) d]
 };
 
+
+// Matrix products that share a launch: C [m, n] = the sum over the two parts of op(A) op(B), row-major, dense rows of C.
+// NT: A [m, k], B [n, k];  NN: A [m, k], B [k, n];  TN: A [k, m], B [k, n].  Behind the sum: zero where act [m, n] is not
+// positive; the column sums of what is stored are added to `sums`.
+enum { kGemmNT = 0, kGemmNN = 1, kGemmTN = 2 };
+struct GemmTask {
+  const void *a[2], *b[2];
+  int64_t lda[2], ldb[2];
+  int k[2];                          // k[1] = 0: one part
+  const void* act;
+  float* sums;
+  void* c;
+  int m, n, op;
+  int first_cta, split, c_vec;       // filled in by launch_gemm
+};
+struct GemmGroup {
+  static constexpr int kMost = 4;
+  GemmTask task[kMost];
+  int* status;
+  int tasks;
+  int cols, split;                   // 0, or the columns of a tile (fp32: 64, 128) and the CTAs that share one (1, 2, 4, 8)
+};
+
 int fail(int code, const char* msg);
 
 // Every host function that launches kernels of this library reports how many it launched; nsa_launch_count() returns
@@ -198,6 +221,8 @@ int gate_sums_counters(int cols);       // zero before the call
 int launch_gate_sums(const void* x, float* out, int64_t rows, int cols, float* partial, unsigned* arrived, int dtype, cudaStream_t stream);
 int launch_qkv_grad(const LayerShape& L, const QkvGrad& P, int dtype, cudaStream_t stream);
 int launch_pos_grad(const LayerShape& L, const void* dkw, const void* dvw, float* dpos, int dtype, cudaStream_t stream);
+bool gemm_serves(const GemmGroup& G, int dtype);   // fp32: sums of up to 35840 products (70 steps of 64 on each of 8 CTAs)
+int launch_gemm(GemmGroup& G, int dtype, cudaStream_t stream);
 int launch_round(const float* src, void* dst, int64_t n, cudaStream_t stream);
 int launch_decode(const DecodeParams& P, int dtype, cudaStream_t stream);
 int fill_decode(DecodeParams& P, const nsa_decode_args& a);   // checks the arguments; q and qr may be NULL
