@@ -461,37 +461,6 @@ static std::vector<OptTensor> layer_forward(Tensor x, std::vector<OptTensor> wei
   return result;
 }
 
-// Gradient through the differentiable top-k: d(value of a pick) back through gather, sink softmax, block mean and head
-// mean to the logits, as a matrix dlog [B, hs, N, ncb] (already times scale / heads averaged)
-static Tensor importance_gradient(const Layer& L, const Tensor& importance, const Tensor& idx, const Tensor& dvals) {
-  const int64_t B = L.B, N = L.N, cpf = L.c.block / L.c.stride, cols = L.ncb / cpf;
-  const bool own_excluded = cpf > 1;
-  Tensor s = importance, own;
-  if (cpf > 1) {
-    s = s.narrow(3, 0, cols * cpf).reshape({B, L.hs, N, cols, cpf}).mean(-1);
-    const auto opts = importance.options().dtype(at::kLong);
-    own = at::arange(N, opts).floor_divide(L.c.block).unsqueeze(1).eq(at::arange(cols, opts).unsqueeze(0));
-    s = s.masked_fill(own, -std::numeric_limits<float>::max());
-  }
-  const Tensor p = at::constant_pad_nd(s, {1, 0}, -1e3).softmax(-1).narrow(3, 1, cols);
-  const Tensor dp = at::zeros_like(p, at::MemoryFormat::Contiguous).scatter_add_(-1, idx, dvals);
-  Tensor ds = p * (dp - (p * dp).sum(-1, true));
-  if (own_excluded) {
-    ds = ds.masked_fill(own, 0.);
-    Tensor full = at::zeros_like(importance);
-    full.narrow(3, 0, cols * cpf).copy_((ds / (double)cpf).repeat_interleave(cpf, -1));
-    ds = full;
-  }
-  const int64_t per_sel = L.c.heads / L.hs;
-  ds = ds * (double)(L.scale / (float)per_sel);
-  if (L.c.causal) {
-    const auto opts = importance.options().dtype(at::kLong);
-    const Tensor visible = at::arange(L.ncb, opts).unsqueeze(0) < at::arange(N, opts).floor_divide(L.c.stride).unsqueeze(1);
-    ds = ds * visible;
-  }
-  return ds;
-}
-
 // -> gradients of x and of the parameters, in the order of the forward's arguments; `needs` says which are wanted.  With
 // `keep_built` the indexes of the sliding and the compressed backward that had to be built here follow.
 static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor> weights, std::vector<OptTensor> saved,
@@ -635,16 +604,14 @@ static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor>
     if (n > 0) built[1] = ws.narrow(0, 0, n).clone();
   }
   if (through_topk) {
-    // every head of a selection head gets the same gradient of its logits: one product for all of them
-    const Tensor dlog = importance_gradient(L, importance, kept_view(at_idx, {B, L.hs, N, L.k_sel}, at::kLong), slots);
-    const int64_t per_sel = H / L.hs, sel_per_kv = L.hs / hkv;
-    const Tensor ckc = kept_view(at_ckv, {2, B, hkv, kv, d}, type).select(0, 0).narrow(2, c.num_mem, L.ncb).to(at::kFloat);   // [B, Hkv, ncb, d]
-    const Tensor dlog_kv = dlog.view({B, hkv, sel_per_kv * N, L.ncb});
-    const Tensor dq_add = at::matmul(dlog_kv, ckc).view({B, L.hs, 1, N, d});
-    dqs[0].view(at::kFloat).view({B, L.hs, per_sel, N, d}).add_(dq_add);
-    const Tensor q = qkv.view({B, N, c.heads + 2 * hkv, d}).narrow(2, 0, H).permute({0, 2, 1, 3}).to(at::kFloat);
-    const Tensor q_sum = q.reshape({B, L.hs, per_sel, N, d}).sum(2).view({B, hkv, sel_per_kv * N, d});
-    acc.narrow(0, 2 * k_elems, c_elems).view({B, hkv, kv, d}).narrow(2, c.num_mem, L.ncb).add_(at::matmul(dlog_kv.transpose(-1, -2), q_sum));
+    const Tensor dlog = at::empty({B, L.hs, N, L.ncb}, importance.options());
+    nsa::TopkGrad t = {};
+    t.importance = ptr<float>(importance); t.idx = reinterpret_cast<const int64_t*>(kp + at_idx); t.dvals = ptr<float>(slots); t.dlog = ptr<float>(dlog);
+    t.qkv = qkv.data_ptr(); t.ck = kp + at_ckv; t.dq = ptr<float>(dqs[0]); t.dck = dck;
+    t.batch = B; t.seq = N; t.heads = H; t.kv_heads = hkv; t.sel_heads = L.hs; t.d = d; t.ncb = L.ncb; t.num_mem = c.num_mem;
+    t.cpf = c.block / c.stride; t.k = L.k_sel; t.block = c.block; t.stride = c.stride; t.causal = c.causal;
+    t.scale = L.scale / (float)(H / L.hs);
+    check(nsa::launch_topk_grad(t, L.dt, st));
   }
 
   // compress networks

@@ -10,7 +10,8 @@
 // tensor cores reach with six products.
 //
 // A CTA computes a tile of 128 x BN.  Eight (fp32: sixteen) warps bring the operands in K steps of 64 into a ring of stages: bf16 by
-// cp.async, fp32 through registers (the next step's loads stand before the split of the present one).  Another warp issues
+// cp.async, fp32 through registers (the next step's loads stand before the split of the present one; 16-byte pieces, whole
+// memory rows per warp: with 32 bytes per thread every load took twice the wavefronts, 3744 x 2048 x 2048 520 -> 473 us).  Another warp issues
 // the products.  What bounds it: operands out of the L2, 24 (fp32 48 to 64) KB per step and tile.
 // Accuracy in fp32: tensor cores do not round their sums to nearest, so long sums lose bits in one direction.  The leading
 // products of a slice of K therefore have an accumulator of their own, the five small ones another, and the epilogue adds
@@ -43,116 +44,118 @@ struct Shape {
   static constexpr uint32_t kCols = sizeof(T) == 4 ? 512 : BN;
 };
 
-// Eight consecutive elements of an operand, in memory order; `count` of them exist
-template <typename T>
-struct Piece;
-template <>
-struct Piece<float> {
-  float x[8];
-  __device__ __forceinline__ void load(const float* p, int count, int vec) {
-    if (vec == 16 && count >= 8) {
-      const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
-      x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
-      x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] = i < count ? __ldg(p + i) : 0.f;
-    }
-  }
-};
-
-// x = h + m + l, each term rounded to bf16; the remainders are exact.  False where h is not finite (the terms would give
-// NaN for an infinite product, or for a value that rounds to infinity).
-__device__ __forceinline__ bool split3(const float (&x)[8], uint32_t (&h)[4], uint32_t (&m)[4], uint32_t (&l)[4]) {
-  bool finite = true;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    float a = x[2 * i], b = x[2 * i + 1];
-    finite = finite && fabsf(a) < 3.38e38f && fabsf(b) < 3.38e38f;
-    h[i] = pack_bf16(a, b);
-    a -= __uint_as_float(h[i] << 16);
-    b -= __uint_as_float(h[i] & 0xffff0000u);
-    m[i] = pack_bf16(a, b);
-    a -= __uint_as_float(m[i] << 16);
-    b -= __uint_as_float(m[i] & 0xffff0000u);
-    l[i] = pack_bf16(a, b);
-  }
-  return finite;
+// x = h + m + l, each term rounded to bf16; the remainders are exact.  Where h is not finite (x is not, or rounds to infinity)
+// the last term is NaN, and stays in `odd`: the terms would give NaN for an infinite product.
+__device__ __forceinline__ void split3(const float4& x, uint2& h, uint2& m, uint2& l, __nv_bfloat162& odd) {
+  auto pair = [&](float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+    hi = pack_bf16(a, b);
+    a -= __uint_as_float(hi << 16);
+    b -= __uint_as_float(hi & 0xffff0000u);
+    mid = pack_bf16(a, b);
+    a -= __uint_as_float(mid << 16);
+    b -= __uint_as_float(mid & 0xffff0000u);
+    lo = pack_bf16(a, b);
+    odd = __hfma2(*reinterpret_cast<const __nv_bfloat162*>(&lo), __floats2bfloat162_rn(0.f, 0.f), odd);
+  };
+  pair(x.x, x.y, h.x, m.x, l.x);
+  pair(x.z, x.w, h.y, m.y, l.y);
 }
 
-// Where the pieces of an operand tile lie: ROWS values of the M / N index, 64 of K.  K-major: memory rows are the M / N
-// index, pieces run along K; else memory rows are K and pieces run along M / N (64 of them per swizzled block).
+// An operand from a tile's first row / column on.  K-major: memory rows are the M / N index; else memory rows are K.
 struct Operand {
   const void* p;
   int64_t ld;
-  int rows, k;        // extents that exist, from the tile's first row / column on
+  int rows, k;        // extents that exist
   bool mn;            // M / N index contiguous in memory
   int vec;            // bytes that one access may move: 16, 4 or an element
 };
-template <int ROWS>
-__device__ __forceinline__ void locate(const Operand& o, int e, int k0, int64_t& at, int& count, uint32_t& off) {
-  if (o.mn) {
-    const int kr = e / (ROWS / 8), c = e % (ROWS / 8);
-    at = (int64_t)(k0 + kr) * o.ld + c * 8;
-    count = k0 + kr < o.k ? o.rows - c * 8 : 0;
-    off = (c / 8) * 8192 + sw128_offset(kr, c % 8);
-  } else {
-    const int r = e / 8, c = e % 8;
-    at = (int64_t)r * o.ld + k0 + c * 8;
-    count = r < o.rows ? o.k - k0 - c * 8 : 0;
-    off = sw128_offset(r, c);
+// The 16-byte pieces of an operand tile (ROWS x 64 of K) that a thread brings: memory rows `pass` apart, so that one address
+// and one place in shared memory serve all of them.
+template <typename T, int ROWS, int LOADERS>
+struct Places {
+  static constexpr int V = 16 / (int)sizeof(T), N = ROWS * kBK / (V * LOADERS);
+  const T* p;
+  int64_t step, hop;  // elements to the next K step and to the next piece
+  int row, left, pass, rows;   // K-major: memory row, K values from the piece on; else K row, values of the M / N index from the piece on
+  uint32_t off;
+  bool mn;
+  int vec;
+  __device__ __forceinline__ Places(const Operand& o, int k0, int tid) : mn(o.mn), vec(o.vec) {
+    const int per = (mn ? ROWS : kBK) / V, r = tid / per, c = tid % per * V;
+    pass = LOADERS / per;
+    hop = pass * o.ld;
+    if (mn) {
+      p = static_cast<const T*>(o.p) + (int64_t)(k0 + r) * o.ld + c;
+      step = kBK * o.ld;
+      row = k0 + r; rows = o.k; left = o.rows - c;
+    } else {
+      p = static_cast<const T*>(o.p) + (int64_t)r * o.ld + k0 + c;
+      step = kBK;
+      row = r; rows = o.rows; left = o.k - k0 - c;
+    }
+    off = (uint32_t)(c / 64) * 8192 + sw128_offset(r, c % 64 * 2 / sizeof(uint4)) + (c * 2) % 16;
   }
-}
+  __device__ __forceinline__ void next() {
+    p += step;
+    if (mn) row += kBK;
+    else left -= kBK;
+  }
+  __device__ __forceinline__ int count(int i) const { return row + i * pass < rows ? left : 0; }   // (may be negative, or above V)
+  __device__ __forceinline__ uint32_t place(int i) const { return off + i * pass * 128; }
+};
 
-template <int ROWS, int LOADERS>
-__device__ __forceinline__ void fetch(const Operand& o, int k0, int tid, Piece<float> (&v)[ROWS * 8 / LOADERS]) {
+template <int ROWS, int LOADERS, int N>
+__device__ __forceinline__ void fetch(const Places<float, ROWS, LOADERS>& at, float4 (&v)[N]) {
+  static_assert(N == Places<float, ROWS, LOADERS>::N, "");
 #pragma unroll
-  for (int i = 0; i < ROWS * 8 / LOADERS; ++i) {
-    int64_t at;
-    int count;
-    uint32_t off;
-    locate<ROWS>(o, tid + i * LOADERS, k0, at, count, off);
-    v[i].load(static_cast<const float*>(o.p) + at, count, o.vec);
+  for (int i = 0; i < N; ++i) {
+    const float* p = at.p + i * at.hop;
+    const int count = at.count(i);
+    if (at.vec == 16 && count >= 4) {
+      v[i] = __ldg(reinterpret_cast<const float4*>(p));
+    } else {
+      v[i].x = count > 0 ? __ldg(p) : 0.f;
+      v[i].y = count > 1 ? __ldg(p + 1) : 0.f;
+      v[i].z = count > 2 ? __ldg(p + 2) : 0.f;
+      v[i].w = count > 3 ? __ldg(p + 3) : 0.f;
+    }
+  }
+}
+__device__ __forceinline__ void sts_v2(uint32_t addr, uint2 v) {
+  asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(v.x), "r"(v.y) : "memory");
+}
+template <int ROWS, int LOADERS, int N>
+__device__ __forceinline__ void put(const Places<float, ROWS, LOADERS>& at, uint32_t tile, const float4 (&v)[N], __nv_bfloat162& odd) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    uint2 h, m, l;
+    split3(v[i], h, m, l, odd);
+    const uint32_t dst = tile + at.place(i);
+    sts_v2(dst, h);
+    sts_v2(dst + ROWS * 128, m);
+    sts_v2(dst + 2 * ROWS * 128, l);
   }
 }
 template <int ROWS, int LOADERS>
-__device__ __forceinline__ bool put(const Operand& o, uint32_t tile, int tid, const Piece<float> (&v)[ROWS * 8 / LOADERS]) {
-  bool finite = true;
+__device__ __forceinline__ void copy(const Places<__nv_bfloat16, ROWS, LOADERS>& at, uint32_t tile) {
 #pragma unroll
-  for (int i = 0; i < ROWS * 8 / LOADERS; ++i) {
-    int64_t at;
-    int count;
-    uint32_t off, h[4], m[4], l[4];
-    locate<ROWS>(o, tid + i * LOADERS, 0, at, count, off);
-    finite = split3(v[i].x, h, m, l) && finite;
-    sts_v4(tile + off, make_uint4(h[0], h[1], h[2], h[3]));
-    sts_v4(tile + ROWS * 128 + off, make_uint4(m[0], m[1], m[2], m[3]));
-    sts_v4(tile + 2 * ROWS * 128 + off, make_uint4(l[0], l[1], l[2], l[3]));
-  }
-  return finite;
-}
-template <int ROWS, int LOADERS>
-__device__ __forceinline__ void copy(const Operand& o, uint32_t tile, int k0, int tid) {
-#pragma unroll
-  for (int i = 0; i < ROWS * 8 / LOADERS; ++i) {
-    int64_t at;
-    int count;
-    uint32_t off;
-    locate<ROWS>(o, tid + i * LOADERS, k0, at, count, off);
-    const uint16_t* src = static_cast<const uint16_t*>(o.p) + at;
+  for (int i = 0; i < Places<__nv_bfloat16, ROWS, LOADERS>::N; ++i) {
+    const uint16_t* src = reinterpret_cast<const uint16_t*>(at.p + i * at.hop);
+    const int count = at.count(i);
+    const uint32_t dst = tile + at.place(i);
     if (count <= 0) {
-      sts_v4(tile + off, make_uint4(0u, 0u, 0u, 0u));
-    } else if (o.vec == 16 && count >= 8) {
-      cp_async16(tile + off, src, 16u);
-    } else if (o.vec >= 4 && count % 2 == 0) {
+      sts_v4(dst, make_uint4(0u, 0u, 0u, 0u));
+    } else if (at.vec == 16 && count >= 8) {
+      cp_async16(dst, src, 16u);
+    } else if (at.vec >= 4 && count % 2 == 0) {
 #pragma unroll
-      for (int x = 0; x < 4; ++x) cp_async4(tile + off + x * 4, 2 * x < count ? src + 2 * x : src, 2 * x < count ? 4u : 0u);
+      for (int x = 0; x < 4; ++x) cp_async4(dst + x * 4, 2 * x < count ? src + 2 * x : src, 2 * x < count ? 4u : 0u);
     } else {
       uint32_t w[4];
 #pragma unroll
       for (int x = 0; x < 4; ++x)
         w[x] = (2 * x < count ? (uint32_t)__ldg(src + 2 * x) : 0u) | (2 * x + 1 < count ? (uint32_t)__ldg(src + 2 * x + 1) << 16 : 0u);
-      sts_v4(tile + off, make_uint4(w[0], w[1], w[2], w[3]));
+      sts_v4(dst, make_uint4(w[0], w[1], w[2], w[3]));
     }
   }
 }
@@ -226,26 +229,29 @@ __global__ void __launch_bounds__((gemm::Shape<T, BN>::kThreads), sizeof(T) == 4
       return Operand{p, ld, (int)((second ? task.n : task.m) - from), task.k[seg], mn, odd % 16 == 0 ? 16 : odd % 4 == 0 ? 4 : 2};
     };
     int seg = first < steps0 ? 0 : 1, k0 = (seg == 0 ? first : first - steps0) * kBK;    // of the step that is requested next
-    Operand A = operand(false, seg), B = operand(true, seg);
+    Places<T, kBM, kLoaders> A(operand(false, seg), k0, tid);
+    Places<T, BN, kLoaders> B(operand(true, seg), k0, tid);
     auto advance = [&]() {
       k0 += kBK;
       if (k0 >= task.k[seg] && seg == 0 && task.k[1] > 0) {
         seg = 1;
         k0 = 0;
-        A = operand(false, 1);
-        B = operand(true, 1);
+        A = Places<T, kBM, kLoaders>(operand(false, 1), 0, tid);
+        B = Places<T, BN, kLoaders>(operand(true, 1), 0, tid);
+      } else {
+        A.next();
+        B.next();
       }
     };
     auto wait_free = [&](int step) {
       if (step >= kStages) mbar_wait_warp(smem_u32(&bars.empty[step % kStages]), (uint32_t)(step / kStages - 1) & 1, &abort_flag);
     };
     if constexpr (F32) {
-      bool finite = true;
-      Piece<float> a[2][kBM * 8 / kLoaders], b[2][BN * 8 / kLoaders];
-      const Operand shape_a = A, shape_b = B;   // the places in shared memory depend on the layout only
+      __nv_bfloat162 odd = __floats2bfloat162_rn(0.f, 0.f);
+      float4 a[2][decltype(A)::N], b[2][decltype(B)::N];
       if (steps > 0) {
-        fetch<kBM, kLoaders>(A, k0, tid, a[0]);
-        fetch<BN, kLoaders>(B, k0, tid, b[0]);
+        fetch(A, a[0]);
+        fetch(B, b[0]);
       }
       for (int step0 = 0; step0 < steps; step0 += 2) {
 #pragma unroll
@@ -254,27 +260,27 @@ __global__ void __launch_bounds__((gemm::Shape<T, BN>::kThreads), sizeof(T) == 4
           if (step < steps) {
             if (step + 1 < steps) {
               advance();
-              fetch<kBM, kLoaders>(A, k0, tid, a[u ^ 1]);
-              fetch<BN, kLoaders>(B, k0, tid, b[u ^ 1]);
+              fetch(A, a[u ^ 1]);
+              fetch(B, b[u ^ 1]);
             }
             wait_free(step);
-            const uint32_t at = base + (step % kStages) * S::kStage;
-            finite = put<kBM, kLoaders>(shape_a, at, tid, a[u]) && finite;
-            finite = put<BN, kLoaders>(shape_b, at + 3 * S::kPlaneA, tid, b[u]) && finite;
+            const uint32_t at = base + (step % kStages) * S::kStage;   // (the places depend on the layout only, not on the part)
+            put(A, at, a[u], odd);
+            put(B, at + 3 * S::kPlaneA, b[u], odd);
             fence_proxy_async_smem();
             mbar_arrive(smem_u32(&bars.full[step % kStages]));
           }
         }
       }
-      if (!finite) odd_input = 1;
+      if (__hisnan(odd.x) || __hisnan(odd.y)) odd_input = 1;
     } else {
       constexpr int kAhead = kStages - 1;
       for (int step = 0; step < steps + kAhead; ++step) {
         if (step < steps) {
           wait_free(step);
           const uint32_t at = base + (step % kStages) * S::kStage;
-          copy<kBM, kLoaders>(A, at, k0, tid);
-          copy<BN, kLoaders>(B, at + S::kPlaneA, k0, tid);
+          copy(A, at);
+          copy(B, at + S::kPlaneA);
           advance();
         }
         cp_async_commit();
@@ -469,36 +475,44 @@ static int64_t tiles_of(const GemmTask& t, int cols) { return (int64_t)((t.m + g
 // 1.1e-6).  Longer sums are split over the CTAs of a cluster.
 static int most_steps(int cols) { return cols == 64 ? 70 : 32; }
 
-// How a group is cut: columns of a tile, CTAs per cluster, and the K steps from which on a task's tiles are shared by a cluster
+// How a group of products is cut: columns of a tile, CTAs per cluster, and the K steps from which on a task's tiles are shared by a cluster
 struct GemmCut {
   int cols, split, from;
   int of(const GemmTask& t) const { return t.sums == nullptr && steps_of(t) >= from ? split : 1; }
 };
+// The cut with the shortest estimate (against the best of all cuts, measured for 22 groups of 62 to 15000 rows: within 10 % for all but two,
+// which take 1.2 times as long): the K steps of the longest CTA, or the steps per SM, whichever is more; a step with 128
+// columns costs 1.6 of one with 64, and CTAs that share a tile meet for the price of some two steps.
 static GemmCut gemm_cut(const GemmGroup& G, int dtype) {
-  int64_t wide = 0, longest = 0;
-  for (int t = 0; t < G.tasks; ++t) {
-    wide += tiles_of(G.task[t], 128);
-    if (steps_of(G.task[t]) > longest) longest = steps_of(G.task[t]);
+  const bool f32 = dtype == NSA_F32;
+  GemmCut best = {64, 1, 1 << 30};
+  double least = -1.;
+  for (int cols = 64; cols <= (f32 ? 128 : 64); cols *= 2) {
+    if (G.cols != 0 && f32 && cols != G.cols) continue;
+    for (int split = 1; split <= gemm::kMaxSplit; split *= 2) {
+      if (G.split != 0 && split != G.split) continue;
+      // from which length on tasks are shared: all that leave a CTA two steps, or the long ones only
+      for (int from = 2 * split; from <= 1024; from *= 2) {
+        const GemmCut cut = {cols, split, from};
+        int64_t total = 0, longest = 0;
+        bool fits = true;
+        for (int t = 0; t < G.tasks; ++t) {
+          const int64_t per = (steps_of(G.task[t]) + cut.of(G.task[t]) - 1) / cut.of(G.task[t]);
+          longest = per > longest && tiles_of(G.task[t], cols) > 0 ? per : longest;
+          total += tiles_of(G.task[t], cols) * (steps_of(G.task[t]) + (cut.of(G.task[t]) > 1 ? 2 * split : 0));
+          fits = fits && (!f32 || per <= most_steps(cols));
+        }
+        const double per_sm = (double)total / 148., estimate = (per_sm > longest ? per_sm : longest + .5 * per_sm) * (cols == 64 ? 1. : 1.6) + (split > 1 ? 2. : 0.);
+        if (G.split == 0 && !fits) continue;
+        if (least < 0. || estimate < least) {
+          least = estimate;
+          best = cut;
+        }
+        if (split == 1) break;
+      }
+    }
   }
-  // 128 columns halve what the rows cost, as long as such tiles still fill the chip: 2 x [1024 x 1024 x 1024] 45 us, with 64
-  // columns 55; but 2048 x 512 x 1024 and its weight gradients, 100 wide tiles, 55 with 64 columns, 82 with 128
-  GemmCut cut = {dtype == NSA_F32 && wide >= 128 && longest <= (int64_t)most_steps(128) * gemm::kMaxSplit ? 128 : 64, 1, 1 << 30};
-  if (G.cols != 0) cut.cols = dtype == NSA_F32 ? G.cols : 64;
-  if (dtype == NSA_F32) {   // what the accumulators need
-    cut.from = most_steps(cut.cols) + 1;
-    while (cut.split < gemm::kMaxSplit && longest > (int64_t)most_steps(cut.cols) * cut.split) cut.split *= 2;
-  }
-  // and while the chip has room for it and every CTA keeps two steps (62 x 1536 x 512 24 -> 19 us, 62 rows of the backward's
-  // last products 48 -> 28)
-  for (int s = cut.split * 2; s <= gemm::kMaxSplit && longest >= 2 * s; s *= 2) {
-    const GemmCut more = {cut.cols, s, 2 * s};
-    int64_t ctas = 0;
-    for (int t = 0; t < G.tasks; ++t) ctas += tiles_of(G.task[t], cut.cols) * more.of(G.task[t]);
-    if (ctas > 148) break;
-    cut = more;
-  }
-  if (G.split != 0) cut = {cut.cols, G.split, 2 * G.split};
-  return cut;
+  return best;
 }
 
 template <typename T, int BN>

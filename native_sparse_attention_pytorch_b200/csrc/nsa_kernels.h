@@ -176,6 +176,17 @@ struct QkvGrad {
   void* out;                         // [B, N, (Hq + 2 Hkv) d]
 };
 
+// Gradient through the differentiable top-k (see nsa_topk_grad.cu)
+struct TopkGrad {
+  const float* importance;           // [B, Hs, N, ncb], as the forward left it
+  const int64_t* idx;                // [B, Hs, N, k]
+  const float* dvals;                // [B, Hs, N, k]
+  float* dlog;                       // [B, Hs, N, ncb], scratch
+  const void *qkv, *ck;              // [B, N, (Hq + 2 Hkv) d]; [B, Hkv, num_mem + ncb, d]
+  float *dq, *dck;                   // [B, Hq, N, d], [B, Hkv, num_mem + ncb, d]: added to
+  int batch, seq, heads, kv_heads, sel_heads, d, ncb, num_mem, cpf, k, block, stride, causal;
+  float scale;                       // of the logits, over the heads that share a selection
+};
 
 // Matrix products that share a launch: C [m, n] = the sum over the two parts of op(A) op(B), row-major, dense rows of C.
 // NT: A [m, k], B [n, k];  NN: A [m, k], B [k, n];  TN: A [k, m], B [k, n].  Behind the sum: zero where act [m, n] is not
@@ -223,6 +234,7 @@ int launch_qkv_grad(const LayerShape& L, const QkvGrad& P, int dtype, cudaStream
 int launch_pos_grad(const LayerShape& L, const void* dkw, const void* dvw, float* dpos, int dtype, cudaStream_t stream);
 bool gemm_serves(const GemmGroup& G, int dtype);   // fp32: sums of up to 35840 products (70 steps of 64 on each of 8 CTAs)
 int launch_gemm(GemmGroup& G, int dtype, cudaStream_t stream);
+int launch_topk_grad(const TopkGrad& P, int dtype, cudaStream_t stream);
 int launch_round(const float* src, void* dst, int64_t n, cudaStream_t stream);
 int launch_decode(const DecodeParams& P, int dtype, cudaStream_t stream);
 int fill_decode(DecodeParams& P, const nsa_decode_args& a);   // checks the arguments; q and qr may be NULL
