@@ -11,6 +11,7 @@
 #include <numeric>
 
 #include "nsa_host.h"
+#include "nsa_kernels.h"
 
 namespace nsa_host {
 
@@ -95,33 +96,35 @@ static std::vector<OptTensor> sel_backward(Tensor q, Tensor k, Tensor v, OptTens
     a.fwd.workspace = ws.data_ptr();
     a.fwd.workspace_bytes = need;
   }
-  // dk and dv side by side: one clearing, one conversion
+  // dk and dv side by side: one clearing, one conversion; in the tensor-core family both are part of other launches
   Tensor dkv = empty({2, k.size(0), k.size(1), k.size(2), k.size(3)}, k, at::kFloat);
   Tensor slots = want_slots ? at::zeros(idx.sizes(), q.options().dtype(at::kFloat)) : Tensor();
   a.dout = t4(dout);
   a.dk = ptr<float>(dkv);
   a.dv = a.dk + k.numel();
   a.accumulate_kv = 1;
-  if (cudaMemsetAsync(a.dk, 0, 2 * k.numel() * sizeof(float), (cudaStream_t)stream_of(k)) != cudaSuccess) throw Error("clearing dk and dv failed");
   a.slot_grads = ptr<float>(slots);
   a.index = index.defined() ? index.data_ptr() : nullptr;
   a.index_bytes = index.defined() ? index.numel() : 0;
   a.delta = delta.has_value() ? ptr<float>(*delta) : nullptr;
   Tensor dq;
-  int rc = NSA_ERR_UNSUPPORTED;
   if (q.scalar_type() == at::kBFloat16 && nsa_sel_bwd_stores_dq(&a.fwd) == 1) {
     dq = empty_in_order_of(q);
     a.dq_out = t4(dq);
-    rc = nsa_sel_bwd(&a, stream_of(q));
+    Tensor rounded = at::empty(dkv.sizes(), k.options());
+    const int rc = nsa::sel_bwd_rounded(a, rounded.data_ptr(), (cudaStream_t)stream_of(q));
+    if (rc != NSA_ERR_UNSUPPORTED) {
+      check(rc);
+      return {dq, rounded.select(0, 0), rounded.select(0, 1), want_slots ? OptTensor(slots) : OptTensor()};
+    }
   }
-  if (rc == NSA_ERR_UNSUPPORTED) {   // no direct dq, or the tensor-core kernels declined these tensors: fp32 dq
-    Tensor dq32 = empty(q.sizes(), q, at::kFloat);
-    a.dq_out = no_tensor();
-    a.dq = ptr<float>(dq32);
-    rc = nsa_sel_bwd(&a, stream_of(q));
-    if (rc == 0) dq = dq32.to(q.scalar_type());
-  }
-  check(rc);
+  // the generic kernels, or tensors the tensor-core ones declined: fp32 dq
+  if (cudaMemsetAsync(a.dk, 0, 2 * k.numel() * sizeof(float), (cudaStream_t)stream_of(k)) != cudaSuccess) throw Error("clearing dk and dv failed");
+  Tensor dq32 = empty(q.sizes(), q, at::kFloat);
+  a.dq_out = no_tensor();
+  a.dq = ptr<float>(dq32);
+  check(nsa_sel_bwd(&a, stream_of(q)));
+  dq = dq32.to(q.scalar_type());
   dkv = dkv.to(k.scalar_type());
   return {dq, dkv.select(0, 0), dkv.select(0, 1), want_slots ? OptTensor(slots) : OptTensor()};
 }

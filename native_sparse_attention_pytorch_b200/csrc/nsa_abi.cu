@@ -266,7 +266,7 @@ int nsa_sel_bwd(const nsa_sel_bwd_args* a, void* stream) {
   const int64_t d = a->fwd.dim_head, n = a->fwd.seq, b = a->fwd.batch;
   NSA_TRY(zero_kv(a->dk, a->dv, b * a->fwd.kv_heads * n * d, a->accumulate_kv != 0, st));
   if (a->fwd.impl != NSA_IMPL_SIMT) {
-    const int rc = sm100_sel_bwd(*a, st);
+    const int rc = sm100_sel_bwd(*a, nullptr, st);
     if (rc != NSA_ERR_UNSUPPORTED || a->fwd.impl == NSA_IMPL_SM100) return rc;
     if (a->dq == nullptr) return fail(NSA_ERR_UNSUPPORTED, "the tensor-core kernels could not take these tensors; pass an fp32 dq");
   }
@@ -674,3 +674,19 @@ int nsa_rmsnorm_bwd(const nsa_rmsnorm_bwd_args* a, void* stream) {
 }
 
 }  // extern "C"
+
+namespace nsa {
+
+int sel_bwd_rounded(const nsa_sel_bwd_args& a, void* dkv_out, cudaStream_t stream) {
+  if (a.fwd.impl == NSA_IMPL_SIMT || !sm100_sel_bwd_overwrites_dq(a.fwd)) return NSA_ERR_UNSUPPORTED;
+  AttnParams P;
+  NSA_TRY(fill_sel(P, a.fwd));
+  NSA_TRY(check_tensor(a.dout, a.fwd.dtype, "dout"));
+  NSA_TRY(check_dq_out(a.dq_out, a.fwd.dtype, true));
+  if (!a.dq_out.ptr || !a.dk || !a.dv || dkv_out == nullptr) return fail(NSA_ERR_NULL, "dq/dk/dv: NULL pointer");
+  if (a.dv != a.dk + (int64_t)a.fwd.batch * a.fwd.kv_heads * a.fwd.seq * a.fwd.dim_head) return fail(NSA_ERR_SHAPE, "dk and dv must lie one behind the other");
+  if (!aligned16(a.index, a.dk, dkv_out)) return fail(NSA_ERR_ALIGN, "index, dk and dv must be 16-byte aligned");
+  return sm100_sel_bwd(a, dkv_out, stream);
+}
+
+}  // namespace nsa

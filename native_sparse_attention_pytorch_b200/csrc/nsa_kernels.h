@@ -250,7 +250,10 @@ int64_t sm100_sel_index_bytes(const nsa_sel_fwd_args& a);
 int64_t sm100_swa_index_bytes(const nsa_swa_fwd_args& a);
 int64_t sm100_cmp_index_bytes(const nsa_cmp_fwd_args& a);
 int sm100_sel_fwd(const nsa_sel_fwd_args& a, cudaStream_t stream);
-int sm100_sel_bwd(const nsa_sel_bwd_args& a, cudaStream_t stream);
+// with dkv_out: dk and dv lie one behind the other, are cleared first and rounded into it (bf16) at the end
+int sm100_sel_bwd(const nsa_sel_bwd_args& a, void* dkv_out, cudaStream_t stream);
+// nsa_sel_bwd of the tensor-core family with dq_out and, in place of cleared dk and dv, dkv_out
+int sel_bwd_rounded(const nsa_sel_bwd_args& a, void* dkv_out, cudaStream_t stream);
 int sm100_sel_fwd_static(const nsa_sel_fwd_args& a, cudaStream_t stream);
 int64_t sm100_swa_workspace_bytes(const nsa_swa_fwd_args& a, bool backward);
 int sm100_swa_fwd(const nsa_swa_fwd_args& a, cudaStream_t stream);

@@ -110,6 +110,7 @@ struct SelParams {
   int words;
   __nv_bfloat16* dq_lp;    // optional bf16 dq with its own batch / head / row strides (dq merge)
   int64_t dq_sb, dq_sh, dq_sn;
+  __nv_bfloat16* dkv_lp;   // optional: where the dq merge rounds dk and dv (which lie one behind the other) to
   uint32_t index_tag;
   __nv_bfloat16* partial;
   float2* stats;
@@ -1164,10 +1165,17 @@ dense_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
 // ---- backward --------------------------------------------------------------------------
 
-// delta[row] = sum_c out[row][c] * dout[row][c]; D/8 threads per row
+// delta[row] = sum_c out[row][c] * dout[row][c]; D/8 threads per row.  The blocks behind those of the rows clear dk and dv
+// (`clear` 16-byte pieces from P.dk on).
 template <int D>
-__global__ void __launch_bounds__(256) sel_delta_kernel(const SelParams P, float* delta) {
+__global__ void __launch_bounds__(256) sel_delta_kernel(const SelParams P, float* delta, unsigned row_blocks, int64_t clear) {
   constexpr int TPR = D / 8;
+  if (blockIdx.x >= row_blocks) {
+    const int64_t step = (int64_t)(gridDim.x - row_blocks) * 256;
+    for (int64_t e = (int64_t)(blockIdx.x - row_blocks) * 256 + threadIdx.x; e < clear; e += step)
+      reinterpret_cast<float4*>(P.dk)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+    return;
+  }
   const int64_t row = ((int64_t)blockIdx.x * 256 + threadIdx.x) / TPR;
   const int part = threadIdx.x % TPR;
   const int64_t nrows = (int64_t)P.B * P.Hq * P.N;
@@ -1645,10 +1653,19 @@ sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 }
 
 
-// sums the dQ partials of every (batch, query head, query) into the fp32 dq row: D/8 threads per row
+// sums the dQ partials of every (batch, query head, query) into the fp32 dq row: D/8 threads per row.  The blocks behind
+// those of the rows round dk and dv, which the kernel before has completed, to bf16 (`round` pieces of 8 from P.dk on).
 template <int D, int MODE>
-__global__ void __launch_bounds__(256) sel_dq_merge_kernel(const SelParams P) {
+__global__ void __launch_bounds__(256) sel_dq_merge_kernel(const SelParams P, unsigned row_blocks, int64_t round) {
   constexpr int TPR = D / 8;
+  if (blockIdx.x >= row_blocks) {
+    const int64_t step = (int64_t)(gridDim.x - row_blocks) * 256;
+    for (int64_t e = (int64_t)(blockIdx.x - row_blocks) * 256 + threadIdx.x; e < round; e += step) {
+      const float4 a = reinterpret_cast<const float4*>(P.dk)[2 * e], c = reinterpret_cast<const float4*>(P.dk)[2 * e + 1];
+      reinterpret_cast<uint4*>(P.dkv_lp)[e] = make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(c.x, c.y), pack_bf16(c.z, c.w));
+    }
+    return;
+  }
   const int64_t part_row = ((int64_t)blockIdx.x * 256 + threadIdx.x) / TPR;   // row of the slice
   const int part = threadIdx.x % TPR;
   const int64_t first = (int64_t)P.bh0 * P.G * P.N, nrows = (int64_t)(P.bh1 - P.bh0) * P.G * P.N;
@@ -1746,6 +1763,7 @@ struct SelProblem {
   float* lse;
   float *dq, *dk, *dv, *slot_grads;
   nsa_tensor dq_out;       // backward, optional: dq in the dtype and strides the caller chose
+  void* dkv_out;           // backward, optional: dk and dv (one behind the other) in bf16; dk and dv are then cleared here
   float* importance;
   __nv_bfloat16* pooled;   // compressed forward, instead of importance: per-selection-block means, see SelParams
   int cpf;
@@ -2100,7 +2118,12 @@ static int run_bwd(const SelProblem& a, const SelPlan& p, uint8_t* ws, cudaStrea
   }
   const int64_t threads = (int64_t)a.B * a.Hq * a.N * (D / 8);
   const int own_delta = a.delta == nullptr ? 1 : 0;   // the caller may hand the row sums over
-  if (own_delta) sel_delta_kernel<D><<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(P, delta);
+  // dk and dv together, as 16-byte pieces: cleared beside the row sums, rounded beside the last merge
+  const int64_t kv_pieces = a.dkv_out != nullptr ? (int64_t)a.B * a.Hkv * a.Nk * D / 2 : 0;
+  const unsigned kv_blocks = (unsigned)((kv_pieces + 255) / 256 < 148 * 4 ? (kv_pieces + 255) / 256 : 148 * 4), row_blocks = (unsigned)((threads + 255) / 256);
+  P.dkv_lp = static_cast<__nv_bfloat16*>(a.dkv_out);
+  if (own_delta) sel_delta_kernel<D><<<row_blocks + kv_blocks, 256, 0, st>>>(P, delta, row_blocks, kv_pieces);
+  else if (kv_pieces > 0) CUDA_TRY(cudaMemsetAsync(a.dk, 0, (size_t)kv_pieces * 16, st));
   if (a.slot_grads != nullptr) CUDA_TRY(cudaMemsetAsync(a.slot_grads, 0, (size_t)a.B * a.Hkv * a.N * a.nsel * sizeof(float), st));
   CUDA_TRY(allow_shared_memory<sel_bwd_ws_kernel<D>>());
   P.partial = reinterpret_cast<__nv_bfloat16*>(ws + p.off_partial);
@@ -2109,9 +2132,12 @@ static int run_bwd(const SelProblem& a, const SelPlan& p, uint8_t* ws, cudaStrea
     P.bh1 = P.bh0 + p.pairs_per_slice < a.B * a.Hkv ? P.bh0 + p.pairs_per_slice : a.B * a.Hkv;
     sel_bwd_ws_kernel<D><<<num_sms(), ws::kThreads, ws::Shape<D>::kBytes, st>>>(tmK, tmV, P);
     const unsigned mblocks = (unsigned)(((int64_t)(P.bh1 - P.bh0) * p.G * a.N * (D / 8) + 255) / 256);
-    if (a.mode == kModeSel) sel_dq_merge_kernel<D, kModeSel><<<mblocks, 256, 0, st>>>(P);
-    else if (a.mode == kModeSwa) sel_dq_merge_kernel<D, kModeSwa><<<mblocks, 256, 0, st>>>(P);
-    else sel_dq_merge_kernel<D, kModeCmp><<<mblocks, 256, 0, st>>>(P);
+    const bool last = s == p.slices - 1;
+    const unsigned grid = mblocks + (last ? (kv_blocks + 1) / 2 : 0);
+    const int64_t round = last ? kv_pieces / 2 : 0;
+    if (a.mode == kModeSel) sel_dq_merge_kernel<D, kModeSel><<<grid, 256, 0, st>>>(P, mblocks, round);
+    else if (a.mode == kModeSwa) sel_dq_merge_kernel<D, kModeSwa><<<grid, 256, 0, st>>>(P, mblocks, round);
+    else sel_dq_merge_kernel<D, kModeCmp><<<grid, 256, 0, st>>>(P, mblocks, round);
   }
   CUDA_TRY(cudaGetLastError());
   count_launches(2 * p.slices + own_delta);   // (delta,) backward kernel and dQ merge per slice
@@ -2216,9 +2242,10 @@ int sm100_sel_fwd_combine(const nsa_sel_fwd_args& a, const CombineParams& c, con
   x.fuse_combine = &c; x.fuse_targets = &t;
   return problem_fwd(x, st);
 }
-int sm100_sel_bwd(const nsa_sel_bwd_args& b, cudaStream_t st) {
+int sm100_sel_bwd(const nsa_sel_bwd_args& b, void* dkv_out, cudaStream_t st) {
   SelProblem x;
   if (!sel_problem(x, b.fwd)) return NSA_ERR_UNSUPPORTED;
+  x.dkv_out = dkv_out;
   x.dout = b.dout; x.dq = b.dq; x.dk = b.dk; x.dv = b.dv; x.slot_grads = b.slot_grads;
   x.index = b.index; x.index_bytes = b.index_bytes; x.dq_out = b.dq_out; x.delta = b.delta;
   return problem_bwd(x, st);
