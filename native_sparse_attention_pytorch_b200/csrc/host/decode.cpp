@@ -101,13 +101,14 @@ static std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> layer_decode(
   uint8_t* const w = static_cast<uint8_t*>(work.data_ptr());
   void *qkv = w, *merged = w + at_merged * el, *gates = w + at_gates * el;
   Tensor qkv_rows, gate_rows;
-  if (nsa::project_serves(B, dim, dt)) {
+  const bool projected = nsa::project_serves(B, dim, dt);
+  if (projected) {
     nsa::ProjectParams p = {};
     p.x[0] = x.data_ptr(); p.x_sb = x.stride(0);
     p.norm_w = norm_w.has_value() ? norm_w->data_ptr() : nullptr; p.eps = (float)eps;
     p.w[0] = qkv_w.data_ptr(); p.gate_w = gate_w.data_ptr(); p.gate_b = gate_b.data_ptr();
     p.y[0] = qkv; p.y_sb = features; p.gates = gates; p.rows = B; p.heads = p.sets = 1; p.dim = dim; p.features = features;
-    p.gates_n = rows;
+    p.gates_n = rows; p.chained = 1;
     check(nsa::launch_project(p, dt, (cudaStream_t)st));
   } else {
     const Tensor xn = norm_w.has_value() ? at::rms_norm(x, {dim}, norm_w, eps) : x;
@@ -124,13 +125,14 @@ static std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> layer_decode(
   p.qkv = qkv; p.inv_freq = ptr<float>(inv_freq);
   p.new_keys = cache.k_buf; p.new_vals = cache.v_buf; p.c_sb = cache.k.stride(0); p.c_sh = cache.k.stride(1); p.row = cache.row;
   p.run_k = run.k_buf; p.run_v = run.v_buf; p.r_sb = run.k.stride(0); p.r_sh = run.k.stride(1); p.run_row = run.row;
+  p.chained = projected;
   check(nsa::launch_decode(p, dt, (cudaStream_t)st));
   Tensor out;
   if (nsa::project_serves(B, heads * d, dt)) {
     out = at::empty({B, 1, dim}, x.options());
     nsa::ProjectParams o = {};
     o.x[0] = merged; o.x_sb = heads * d; o.w[0] = out_w.data_ptr(); o.y[0] = out.data_ptr(); o.y_sb = dim;
-    o.rows = B; o.heads = o.sets = 1; o.dim = heads * d; o.features = dim;
+    o.rows = B; o.heads = o.sets = 1; o.dim = heads * d; o.features = dim; o.chained = 2;
     check(nsa::launch_project(o, dt, (cudaStream_t)st));
   } else {
     out = at::linear(at::as_strided(work, {B, heads * d}, {heads * d, 1}, at_merged), out_w).unsqueeze(1);

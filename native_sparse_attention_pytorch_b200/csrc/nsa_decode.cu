@@ -10,8 +10,8 @@
 // spread over the cluster a warp has one or two tiles of 16 keys per branch.  Inside a branch the warps of the cluster
 // take tiles in turn, keep an online softmax each and fold through shared memory; the CTAs' results meet at the end
 // through distributed shared memory.  The compressed logits are stored into every CTA of the cluster as they are
-// computed, so each of them ranks the blocks itself (warp 0, while the other warps run the sliding window, which does
-// not depend on it): one cluster barrier instead of two.
+// computed, so each of them selects the blocks itself, behind the sliding window, which does not depend on them: one cluster
+// barrier instead of two.
 //   * Key and value rows are staged by cp.async (whole 128-byte lines) into two buffers per warp, the first tile of a
 //     branch before the previous branch is folded; two lanes share a key for the dot products.
 //
@@ -43,6 +43,7 @@ using ptx::cluster_rank;
 using ptx::cluster_wait;
 using ptx::map_rank;
 using ptx::st_cluster;
+using ptx::st_cluster_v2;
 
 // A tile of up to kTile consecutive keys (kLongTile in the form for very long caches): where its rows are
 constexpr int kTile = 16, kLongTile = 4;
@@ -150,16 +151,16 @@ struct ScalarState {
       }
     }
   }
-  // to shared memory: [g][2 + d]: maximum (base-2 logarithm), sum, unnormalised row
+  // to shared memory: [g][d + 2]: unnormalised row, maximum (base-2 logarithm), sum
   __device__ __forceinline__ void park(float* dst, int d, int lane) const {
 #pragma unroll
     for (int g = 0; g < GT; ++g) {
       float* row = dst + g * (d + 2);
-      if (lane == 0) { row[0] = m[g] * kLog2e; row[1] = l[g]; }
+      if (lane == 0) { row[d] = m[g] * kLog2e; row[d + 1] = l[g]; }
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         const int dim = 64 * c + 2 * lane;
-        if (dim < d) { row[2 + dim] = acc[g][c][0]; row[3 + dim] = acc[g][c][1]; }
+        if (dim < d) { row[dim] = acc[g][c][0]; row[dim + 1] = acc[g][c][1]; }
       }
     }
   }
@@ -297,11 +298,11 @@ struct TensorState {
         const int g = 8 * n + 2 * (lane & 3) + e;
         if (g < GT) {
           float* row = dst + g * (D + 2);
-          if (lane < 4) { row[0] = m[n][e]; row[1] = sum; }
+          if (lane < 4) { row[D] = m[n][e]; row[D + 1] = sum; }
 #pragma unroll
           for (int t = 0; t < D / 16; ++t) {
-            row[2 + 16 * t + lane / 4] = o[n][t][e];
-            row[2 + 16 * t + 8 + lane / 4] = o[n][t][2 + e];
+            row[16 * t + lane / 4] = o[n][t][e];
+            row[16 * t + 8 + lane / 4] = o[n][t][2 + e];
           }
         }
       }
@@ -311,94 +312,76 @@ struct TensorState {
 // Logit of block column j: mean over its compressed blocks
 __device__ __forceinline__ float block_logit(const DecodeParams& P, const float* imp_s, int j, int cpf) {
   if (P.stride == P.block) return imp_s[j];
-  float sum = 0.f;
   if (cpf == 4) {
     const float4 q = *reinterpret_cast<const float4*>(imp_s + 4 * j);
-    sum = ((q.x + q.y) + q.z) + q.w;
-  } else {
-    for (int c = 0; c < cpf; ++c) sum += imp_s[j * cpf + c];
+    return (((q.x + q.y) + q.z) + q.w) * 0.25f;
   }
+  float sum = 0.f;
+  for (int c = 0; c < cpf; ++c) sum += imp_s[j * cpf + c];
   return sum / (float)cpf;
 }
 
-// Mean over the compressed blocks of a selection block, softmax with the sink, the k largest probabilities (ties to the
-// lower column); one warp, CPL columns per lane in registers (CPL = 0: any number, in shared memory).  The picks are a
-// set here -- attention does not care in which order the blocks come -- so instead of k rounds of "largest remaining"
-// (12.5 k cycles for 16 of 512, the longest step of the kernel) the k-th largest value is found by bisection on the
-// values' bit patterns, which order as the values do because probabilities are not negative.
-template <int CPL>
-__device__ __forceinline__ int rank_blocks(const DecodeParams& P, const float* imp_s, float* prob_s, int cols, int cpf,
-                                           int k_sel, int* sel_idx, int lane) {
-  constexpr int R = CPL > 0 ? CPL : 1;
-  float v[R];
-  const int per_lane = CPL > 0 ? CPL : (cols + 31) / 32;
-  auto get = [&](int t) { return CPL > 0 ? v[CPL > 0 ? t : 0] : lane + 32 * t < cols ? prob_s[lane + 32 * t] : 0.f; };
-  auto put = [&](int t, float x) {
-    if (CPL > 0) v[CPL > 0 ? t : 0] = x;
-    else if (lane + 32 * t < cols) prob_s[lane + 32 * t] = x;
+// The `want` largest of `cols` probabilities (ties to the lower column); one warp.  The picks are a set: attention does not
+// care in which order the blocks come.  The want-th largest of the 32 lanes' maxima bounds them from below, the columns that
+// reach it (20 to 30 of 512) are ranked against each other; where they are more than kCandidates, the want-th largest value is
+// found by bisection on the values' bit patterns, which order as the values do because probabilities are not negative.
+constexpr int kCandidates = 64;
+__device__ __forceinline__ void pick_blocks(const float* prob_s, int cols, int want, float* cand_p, int* cand_col, int* sel_idx, int lane) {
+  float top = 0.f;
+  for (int j = lane; j < cols; j += 32) top = fmaxf(top, prob_s[j]);
+  int r = 0;
+#pragma unroll
+  for (int o = 0; o < 32; ++o) {
+    const float other = __shfl_sync(kFullMask, top, o);
+    r += other > top || (other == top && o < lane) ? 1 : 0;
+  }
+  const float bound = __shfl_sync(kFullMask, top, __ffs(__ballot_sync(kFullMask, r == want - 1)) - 1);
+  int n = 0;
+  for (int j0 = 0; j0 < cols; j0 += 32) {
+    const float p = j0 + lane < cols ? prob_s[j0 + lane] : -1.f;
+    const unsigned in = __ballot_sync(kFullMask, p >= bound);
+    const int at = n + __popc(in & ((1u << lane) - 1u));
+    if (p >= bound && at < kCandidates) {
+      cand_p[at] = p;
+      cand_col[at] = j0 + lane;
+    }
+    n += __popc(in);
+  }
+  __syncwarp();
+  if (n <= kCandidates) {                       // in the order of their columns
+    for (int c = lane; c < n; c += 32) {
+      const float p = cand_p[c];
+      int rank = 0;
+      for (int o = 0; o < n; ++o) rank += cand_p[o] > p || (cand_p[o] == p && o < c) ? 1 : 0;
+      if (rank < want) sel_idx[rank] = cand_col[c];
+    }
+    return;
+  }
+  auto key_of = [&](int j) { return j < cols ? __float_as_uint(prob_s[j]) : 0u; };
+  auto count_from = [&](unsigned from) {
+    unsigned c = 0u;
+    for (int j = lane; j < cols; j += 32) c += key_of(j) >= from ? 1u : 0u;
+    return (int)__reduce_add_sync(kFullMask, c);
   };
-  float mx = -1000.f;   // the sink logit
-#pragma unroll
-  for (int t = 0; t < per_lane; ++t) {
-    const int j = lane + 32 * t;
-    const float x = j < cols ? block_logit(P, imp_s, j, cpf) : -INFINITY;
-    put(t, x);
-    mx = fmaxf(mx, x);
-  }
-  mx = warp_max(mx);
-  float part = 0.f;
-#pragma unroll
-  for (int t = 0; t < per_lane; ++t) {
-    const float e = lane + 32 * t < cols ? expf(get(t) - mx) : 0.f;
-    put(t, e);
-    part += e;
-  }
-  const float z = warp_sum(part) + expf(-1000.f - mx);
-  unsigned top = 0u;
-  int live = 0;         // columns above the threshold below which upstream masks a slot out
-#pragma unroll
-  for (int t = 0; t < per_lane; ++t) {
-    const float p = get(t) / z;
-    put(t, p);
-    top = max(top, __float_as_uint(p));
-    live += p > 1e-10f ? 1 : 0;
-  }
-  live = (int)__reduce_add_sync(kFullMask, (unsigned)live);
-  const int want = min(k_sel, live);
-  if (want == 0) return 0;
   // the largest `cut` with at least `want` columns at or above it
-  unsigned lo = __float_as_uint(1e-10f), hi = __reduce_max_sync(kFullMask, top) + 1u;   // count(lo + 1) >= want > count(hi)
-  auto count_from = [&](unsigned cut) {
-    unsigned n = 0u;
-#pragma unroll
-    for (int t = 0; t < per_lane; ++t) n += __float_as_uint(get(t)) >= cut ? 1u : 0u;
-    return (int)__reduce_add_sync(kFullMask, n);
-  };
-  unsigned cut = lo + 1u;
+  unsigned cut = __float_as_uint(bound), hi = __reduce_max_sync(kFullMask, __float_as_uint(top)) + 1u;
 #pragma unroll 1
   while (hi - cut > 1u) {
     const unsigned mid = cut + (hi - cut) / 2u;
-    const int n = count_from(mid);
-    if (n >= want) cut = mid;
+    if (count_from(mid) >= want) cut = mid;
     else hi = mid;
-    if (n == want) break;
   }
   // everything above the cut, and of the columns at it the lowest
-  int above = count_from(cut + 1u);
-  const bool exact = count_from(cut) == want;
-  int at_cut = exact ? cols : want - above;     // how many columns equal to the cut are taken
-  int count = 0;
-#pragma unroll
-  for (int t = 0; t < per_lane; ++t) {
-    const unsigned key = __float_as_uint(get(t));
+  int at_cut = want - count_from(cut + 1u), count = 0;
+  for (int j0 = 0; j0 < cols; j0 += 32) {
+    const unsigned key = key_of(j0 + lane);
     const unsigned eq = __ballot_sync(kFullMask, key == cut);
     const bool take = key > cut || (key == cut && __popc(eq & ((1u << lane) - 1u)) < at_cut);
     at_cut -= min(at_cut, __popc(eq));
     const unsigned picked = __ballot_sync(kFullMask, take);
-    if (take) sel_idx[count + __popc(picked & ((1u << lane) - 1u))] = lane + 32 * t;
+    if (take) sel_idx[count + __popc(picked & ((1u << lane) - 1u))] = j0 + lane;
     count += __popc(picked);
   }
-  return count;
 }
 
 // What a CTA needs in shared memory, in bytes from the start of the dynamic segment (the same in all of a cluster)
@@ -422,6 +405,9 @@ __host__ __device__ inline DecodeLayout decode_layout(int el, int GT, int rows, 
   return L;
 }
 
+// `P.chained`: the kernel before it in the stream is the projection it reads the qkv rows and gates from, whose CTAs let this one
+// start once everything before the projection is complete.  What does not come from the projection (caches, angles) is then
+// fetched while it runs.
 template <typename T, typename State>
 __global__ void __launch_bounds__(DecodeShape<T>::kWarps * 32, 1) decode_kernel(const DecodeParams P, int S) {
   constexpr int GT = State::kHeads, ROWS = State::kRows;
@@ -430,7 +416,8 @@ __global__ void __launch_bounds__(DecodeShape<T>::kWarps * 32, 1) decode_kernel(
   __shared__ int sel_idx[32];
   __shared__ int sel_count;
   __shared__ float weight[3][GT][kMaxCluster];
-  __shared__ float gate_s[3 * GT], turn_s[2][64];
+  __shared__ float gate_s[3 * GT], turn_s[2][64], fold_s[2][DecodeShape<T>::kWarps];
+  __shared__ int live_s[DecodeShape<T>::kWarps];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rank = (int)cluster_rank();
   const int unit = blockIdx.x / S;
@@ -482,11 +469,20 @@ __global__ void __launch_bounds__(DecodeShape<T>::kWarps * 32, 1) decode_kernel(
     }
     return KeyTile<T>{kb + t0 * P.k_sn, vb + t0 * P.v_sn, P.k_sn, P.v_sn, min(ROWS, end - t0)};
   };
-  // The warps of the cluster take a branch's tiles in turn; warp 0 of every CTA sits the window out and ranks
-  auto first_of = [&](int phase) { return phase == 1 ? (warp == 0 ? 0x3fffffff : (warp - 1) * S + rank) : warp * S + rank; };
+  // The warps of the cluster take a branch's tiles in turn
+  const int first = warp * S + rank;
 
+  ptx::grid_allow_next();
   if (tid == 0) sel_count = 0;
-  if (first_of(0) < tiles_of(0)) stage_tile<T, ROWS>(ptx::smem_u32(stage), locate(0, first_of(0)), d, lane);
+  if (first < tiles_of(0)) stage_tile<T, ROWS>(ptx::smem_u32(stage), locate(0, first), d, lane);
+  if (P.qkv != nullptr)
+    for (int e = tid; e < d / 2; e += kThreads) {
+      const float ang = (float)pos * P.inv_freq[e];
+      turn_s[0][e] = cosf(ang);
+      turn_s[1][e] = sinf(ang);
+    }
+  __syncthreads();
+  ptx::grid_wait();
   for (int e = tid; e < 3 * G; e += kThreads)
     gate_s[e] = Elem<T>::to_float(((const T*)P.gates)[((int64_t)b * P.q_heads + kvh * G) * 3 + e]);
   {
@@ -494,12 +490,6 @@ __global__ void __launch_bounds__(DecodeShape<T>::kWarps * 32, 1) decode_kernel(
     const int pieces = d / V;
     if (P.qkv != nullptr) {
       // straight from the qkv projection: rotate the queries, and (one CTA) the new key, append key and value
-      for (int e = tid; e < d / 2; e += kThreads) {
-        const float ang = (float)pos * P.inv_freq[e];
-        turn_s[0][e] = cosf(ang);
-        turn_s[1][e] = sinf(ang);
-      }
-      __syncthreads();
       const int features = (P.q_heads + 2 * P.kv_heads) * d;
       const T* row = (const T*)P.qkv + (int64_t)b * features;
       for (int e = tid; e < (GT + (rank == 0 ? 2 : 0)) * pieces; e += kThreads) {
@@ -538,6 +528,7 @@ __global__ void __launch_bounds__(DecodeShape<T>::kWarps * 32, 1) decode_kernel(
       }
     }
   }
+  __syncwarp();
   cluster_arrive();     // nobody writes into another CTA's shared memory before that CTA runs, or reads the new cache
   __syncthreads();      // row before it is written
   cluster_wait();
@@ -547,21 +538,11 @@ __global__ void __launch_bounds__(DecodeShape<T>::kWarps * 32, 1) decode_kernel(
   for (int phase = 0; phase < 3; ++phase) {
     const T* rows = q_s + (phase == 0 ? 0 : GT * (d + 8));
     state.start(rows, d, lane);
-    if (phase == 1 && warp == 0) {
-      // selection, on the logits of the whole cluster
-      cluster_wait();
-      float* const prob_s = reinterpret_cast<float*>(decode_smem + L.prob);
-      const int k_sel = min(min(P.nsel, cols), 32);
-      const int n = cols <= 128   ? rank_blocks<4>(P, imp_s, prob_s, cols, cpf, k_sel, sel_idx, lane)
-                    : cols <= 512 ? rank_blocks<16>(P, imp_s, prob_s, cols, cpf, k_sel, sel_idx, lane)
-                                  : rank_blocks<0>(P, imp_s, prob_s, cols, cpf, k_sel, sel_idx, lane);
-      if (lane == 0) sel_count = n;
-    }
     // two staging buffers: the next tile travels under this one's work
-    const int total = tiles_of(phase), step = (phase == 1 ? W - 1 : W) * S;
+    const int total = tiles_of(phase), step = W * S;
     int which = 0;
 #pragma unroll 1
-    for (int t = first_of(phase); t < total; t += step) {
+    for (int t = first; t < total; t += step) {
       if (t + step < total) {
         stage_tile<T, ROWS>(ptx::smem_u32(stage) + (which ^ 1) * buf_bytes, locate(phase, t + step), d, lane);
         ptx::cp_async_wait<1>();
@@ -579,16 +560,60 @@ __global__ void __launch_bounds__(DecodeShape<T>::kWarps * 32, 1) decode_kernel(
       __syncwarp();
       which ^= 1;
     }
-    if (phase == 1 && warp != 0) cluster_wait();
     if (phase == 0) {
       cluster_arrive();       // this warp's logits are on their way to everybody
       // the first tile of the window travels under the fold
-      if (first_of(1) < tiles_of(1)) stage_tile<T, ROWS>(ptx::smem_u32(stage), locate(1, first_of(1)), d, lane);
+      if (first < tiles_of(1)) stage_tile<T, ROWS>(ptx::smem_u32(stage), locate(1, first), d, lane);
     }
     state.park(area + (size_t)warp * GT * (d + 2), d, lane);
+    if (phase == 1) {
+      // Selection, by every CTA for itself on the logits of the whole cluster: softmax with the sink over the block columns, all
+      // threads; then one warp picks.  (One warp for all of it took 11.7 k of the kernel's 46 k cycles at 512 columns.)
+      __syncwarp();
+      cluster_wait();
+      float* const prob_s = reinterpret_cast<float*>(decode_smem + L.prob);
+      float mx = -1000.f;     // the sink logit
+      for (int j = tid; j < cols; j += kThreads) {
+        const float x = block_logit(P, imp_s, j, cpf);
+        prob_s[j] = x;
+        mx = fmaxf(mx, x);
+      }
+      mx = warp_max(mx);
+      if (lane == 0) fold_s[0][warp] = mx;
+      __syncthreads();
+      for (int w = 0; w < W; ++w) mx = fmaxf(mx, fold_s[0][w]);
+      float part = 0.f;
+      for (int j = tid; j < cols; j += kThreads) {
+        const float e = expf(prob_s[j] - mx);
+        prob_s[j] = e;
+        part += e;
+      }
+      part = warp_sum(part);
+      if (lane == 0) fold_s[1][warp] = part;
+      __syncthreads();
+      float z = expf(-1000.f - mx);
+      for (int w = 0; w < W; ++w) z += fold_s[1][w];
+      unsigned live = 0u;     // columns above the threshold below which upstream masks a slot out
+      for (int j = tid; j < cols; j += kThreads) {
+        const float p = prob_s[j] / z;
+        prob_s[j] = p;
+        live += p > 1e-10f ? 1u : 0u;
+      }
+      live = __reduce_add_sync(kFullMask, live);
+      if (lane == 0) live_s[warp] = (int)live;
+      __syncthreads();
+      if (warp == 0) {
+        int want = 0;
+        for (int w = 0; w < W; ++w) want += live_s[w];
+        want = min(want, min(min(P.nsel, cols), 32));
+        if (want > 0) pick_blocks(prob_s, cols, want, turn_s[0], reinterpret_cast<int*>(turn_s[1]), sel_idx, lane);
+        if (lane == 0) sel_count = want;
+      }
+    }
     __syncthreads();
-    if (phase == 1 && first_of(2) < tiles_of(2)) stage_tile<T, ROWS>(ptx::smem_u32(stage), locate(2, first_of(2)), d, lane);
-    // Fold the warps' states and send every element to the CTA that finishes it: kThreads / GT threads per head
+    if (phase == 1 && first < tiles_of(2)) stage_tile<T, ROWS>(ptx::smem_u32(stage), locate(2, first), d, lane);
+    // Fold the warps' states and send every element to the CTA that finishes it: kThreads / GT threads per head, two
+    // neighbouring features each
     {
       const int branch = phase == 0 ? 0 : 3 - phase;          // in the order of the gates: compressed, selected, sliding
       const int per = kThreads / GT, g = tid / per, c0 = tid - g * per;
@@ -597,28 +622,35 @@ __global__ void __launch_bounds__(DecodeShape<T>::kWarps * 32, 1) decode_kernel(
       float f[8], M = -INFINITY, sum = 0.f;
 #pragma unroll
       for (int w = 0; w < 8; ++w) {
-        f[w] = w < W ? src[w * next] : -INFINITY;
+        f[w] = w < W ? src[w * next + d] : -INFINITY;
         M = fmaxf(M, f[w]);
       }
 #pragma unroll
       for (int w = 0; w < 8; ++w) {
         f[w] = f[w] == -INFINITY ? 0.f : exp2f(f[w] - M);
-        if (w < W) sum = fmaf(f[w], src[w * next + 1], sum);
+        if (w < W) sum = fmaf(f[w], src[w * next + d + 1], sum);
       }
       const uint32_t ml = ptx::smem_u32(decode_smem + L.ml) + (uint32_t)(((rank * 3 + branch) * GT + g) * 2) * 4u;
-      for (int r = c0; r < S; r += per) {
-        st_cluster(map_rank(ml, r), M);
-        st_cluster(map_rank(ml + 4, r), sum);
-      }
+      for (int r = c0; r < S; r += per) st_cluster_v2(map_rank(ml, r), M, sum);
       const uint32_t recv = ptx::smem_u32(decode_smem + L.recv) + ((uint32_t)((rank * 3 + branch) * GT + g) << (L.shift + 2));
-#pragma unroll 1
-      for (int c = c0; c < d; c += per) {
-        float o = 0.f;
+#pragma unroll 2
+      for (int c = 2 * c0; c < d; c += 2 * per) {
+        float2 o = make_float2(0.f, 0.f);
 #pragma unroll
         for (int w = 0; w < 8; ++w)
-          if (w < W) o = fmaf(f[w], src[w * next + 2 + c], o);
+          if (w < W) {
+            const float2 x = *reinterpret_cast<const float2*>(src + w * next + c);
+            o.x = fmaf(f[w], x.x, o.x);
+            o.y = fmaf(f[w], x.y, o.y);
+          }
         const int owner = c >> L.shift;
-        st_cluster(map_rank(recv + (uint32_t)(c - (owner << L.shift)) * 4u, owner), o);
+        const uint32_t dst = recv + (uint32_t)(c - (owner << L.shift)) * 4u;
+        if (L.shift > 0) {
+          st_cluster_v2(map_rank(dst, owner), o.x, o.y);
+        } else {              // a CTA finishes one feature
+          st_cluster(map_rank(dst, owner), o.x);
+          st_cluster(map_rank(dst, owner + 1), o.y);
+        }
       }
     }
     __syncthreads();
@@ -691,12 +723,14 @@ static int launch_decode_state(const DecodeParams& P, cudaStream_t stream) {
   cfg.blockDim = dim3(W * 32);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = (unsigned)S;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = P.chained ? 2 : 1;
   err = cudaLaunchKernelEx(&cfg, kern, P, S);
   if (err != cudaSuccess) return fail((int)err, cudaGetErrorString(err));
   count_launches(1);
@@ -775,7 +809,10 @@ int launch_cache_copy(const CacheCopy& P, cudaStream_t stream) {
 // y = norm(x) W^T for up to 16 token rows x, and behind the rows of W the gates: sigmoid(norm(x) Wg^T + bg); also the two
 // layers of the compress networks when a window has filled up, keys and values side by side.
 // Bound: the weights, read once.  bf16: a CTA owns 16 rows of W and requests all of them with cp.async before it
-// normalises the token rows, then one warp walks K upwards with m16n8k16 products, fp32 accumulators.
+// normalises the token rows, then its warps share K (m16n8k16 products, fp32 accumulators) and add their parts in order.
+// `chained` 1: the first kernel of a step, which may be scheduled before the kernel in front of it has ended but does nothing
+// until then; 2: the last one, behind the attention, which fetches its weights meanwhile (nothing in the step writes them, and
+// what came before the step was complete before the attention could start).
 // fp32: a warp owns a pair of rows and uses CUDA cores.  Beside a library GEMM, which serves more than 16 rows, the results
 // agree as two orders of the same fp32 sum do.
 
@@ -845,6 +882,8 @@ __device__ __forceinline__ void emit(const ProjectParams& P, bool gates, int t, 
 template <int NT>   // groups of eight tokens
 __global__ void __launch_bounds__(kProjWarps * 32) project_bf16_kernel(const ProjectParams P) {
   using T = __nv_bfloat16;
+  if (P.chained != 2) ptx::grid_wait();
+  ptx::grid_allow_next();
   extern __shared__ __align__(16) uint8_t proj_smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int stride = P.dim + 8;                    // elements; 16 bytes of padding keep ldmatrix free of conflicts
@@ -865,17 +904,18 @@ __global__ void __launch_bounds__(kProjWarps * 32) project_bf16_kernel(const Pro
     }
   }
   ptx::cp_async_commit();
+  if (P.chained == 2) ptx::grid_wait();
   load_rows<T>(P, x_s, stride, 8 * NT, warp, kProjWarps, lane);
   ptx::cp_async_wait<0>();
   __syncthreads();
-  if (warp != 0) return;
   float acc[NT][4];
 #pragma unroll
   for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
   const uint32_t a_at = ptx::smem_u32(w_s + (lane & 15) * stride + (lane >> 4) * 8);
   const T* const b_at = x_s + (lane / 4) * stride + 2 * (lane & 3);
-#pragma unroll 8
-  for (int k = 0; k < P.dim; k += 16) {
+  const int k_end = P.dim / 16 * (warp + 1) / kProjWarps * 16;
+#pragma unroll 4
+  for (int k = P.dim / 16 * warp / kProjWarps * 16; k < k_end; k += 16) {
     uint32_t a[4];
     ldmatrix4<false>(a, a_at + k * 2);
 #pragma unroll
@@ -884,13 +924,21 @@ __global__ void __launch_bounds__(kProjWarps * 32) project_bf16_kernel(const Pro
       mma_16816(acc[n], a, *reinterpret_cast<const uint32_t*>(src), *reinterpret_cast<const uint32_t*>(src + 8));
     }
   }
+  // the warps' parts of the sum, in their order
+  __syncthreads();                                 // (over the weights)
+  float* const part = reinterpret_cast<float*>(proj_smem);
 #pragma unroll
   for (int n = 0; n < NT; ++n)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int f = f0 + lane / 4 + (e / 2) * 8, t = 8 * n + 2 * (lane & 3) + (e & 1);
-      if (f < end && t < P.rows) emit<T>(P, gates, t, f, acc[n][e]);
-    }
+    for (int e = 0; e < 4; ++e) part[(warp * NT * 4 + n * 4 + e) * 32 + lane] = acc[n][e];
+  __syncthreads();
+  if (tid >= NT * 128) return;
+  const int n = tid / 128, e = tid / 32 % 4;
+  float v = 0.f;
+#pragma unroll
+  for (int w = 0; w < kProjWarps; ++w) v += part[w * NT * 128 + tid];
+  const int f = f0 + lane / 4 + (e / 2) * 8, t = 8 * n + 2 * (lane & 3) + (e & 1);
+  if (f < end && t < P.rows) emit<T>(P, gates, t, f, v);
 }
 
 // fp32: the weights come from the L2 or from memory, so a lane requests four 16-byte pieces of either row at a time, the
@@ -919,10 +967,13 @@ __global__ void __launch_bounds__(kProjWarps * 32) project_f32_kernel(const Proj
     }
   };
   const int first = blockIdx.x * kProjWarps + warp;
+  if (P.chained != 2) ptx::grid_wait();
+  ptx::grid_allow_next();
   if (first < pairs) {
     aim(first);
     fetch(0);
   }
+  if (P.chained == 2) ptx::grid_wait();
   load_rows<float>(P, x_s, P.dim, BT, warp, kProjWarps, lane);
   __syncthreads();
   for (int p = first; p < pairs; p += gridDim.x * kProjWarps) {
@@ -966,8 +1017,10 @@ __global__ void __launch_bounds__(kProjWarps * 32) project_f32_kernel(const Proj
 // weight row often enough), or rows that do not fit.
 static int project_smem(int batch, int dim, int dtype) {
   if (batch > 16 || dim % 16) return 0;
-  const int64_t need = dtype == NSA_F32 ? (int64_t)(batch <= 1 ? 1 : batch <= 4 ? 4 : 16) * dim * 4
-                                        : (int64_t)(kProjRows + (batch <= 8 ? 8 : 16)) * (dim + 8) * 2;
+  const int tokens = batch <= 8 ? 8 : 16;
+  const int64_t parts = kProjWarps * kProjRows * tokens * 4;      // bf16: the warps' sums, over the weights
+  const int64_t rows = (int64_t)(kProjRows + tokens) * (dim + 8) * 2;
+  const int64_t need = dtype == NSA_F32 ? (int64_t)(batch <= 1 ? 1 : batch <= 4 ? 4 : 16) * dim * 4 : rows > parts ? rows : parts;
   return need <= 220 * 1024 ? (int)need : 0;
 }
 
@@ -977,9 +1030,18 @@ template <auto Kernel>
 static int launch_project_with(const ProjectParams& P, int blocks, int smem, cudaStream_t stream) {
   cudaError_t err = allow_shared_memory<Kernel>();
   if (err == cudaSuccess) {
-    Kernel<<<dim3((unsigned)blocks, (unsigned)P.sets), kProjWarps * 32, smem, stream>>>(P);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks, (unsigned)P.sets);
+    cfg.blockDim = dim3(kProjWarps * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = P.chained ? 1 : 0;
+    err = cudaLaunchKernelEx(&cfg, Kernel, P);
     count_launches(1);
-    err = cudaGetLastError();
   }
   return err == cudaSuccess ? NSA_OK : fail((int)err, cudaGetErrorString(err));
 }

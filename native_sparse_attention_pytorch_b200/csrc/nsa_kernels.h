@@ -124,6 +124,7 @@ struct DecodeParams {
   void *new_keys, *new_vals, *run_k, *run_v;
   int64_t c_sb, c_sh, r_sb, r_sh;
   int row, run_row;
+  int chained;                   // the kernel launched before is the projection that writes qkv and gates (launch_project)
 };
 
 // Projection of up to 16 rows (see nsa_decode.cu): y = f(x) w^T (+ bias) (ReLU), f = RMS norm, addition of `add`, or
@@ -137,6 +138,7 @@ struct ProjectParams {
   void* gates;                                  // [rows, gates_n]
   int64_t x_sb, x_sh, y_sb, y_sh;
   int rows, heads, sets, dim, features, gates_n, relu;
+  int chained;                                  // 1: first, 2: last kernel of a step, see nsa_decode.cu; else 0
   float eps;
 };
 
