@@ -140,6 +140,23 @@ static std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> layer_decode(
   return {out, cache.k, cache.v, run.k, run.v};
 }
 
+// The same for a layer that has not looked at its tensors yet: nothing where the step has to run module by module (another
+// input than one token, parameters or caches of another type or device, off the 16-byte boundary).  `weights` as in
+// layer_takes; cfg: heads, stride, block, cbs, nsel, window.  Asked one by one from Python, these questions were a fifth of a
+// step's host time.
+static std::optional<std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor>> layer_step(
+    const Tensor& x, const std::vector<OptTensor>& w, double eps, const Tensor& inv_freq, const Tensor& past_k, const Tensor& past_v,
+    const Tensor& ck, const Tensor& cv, const Tensor& run_k, const Tensor& run_v, const std::vector<int64_t>& cfg) {
+  const int64_t heads = cfg.at(0), stride = cfg.at(1), block = cfg.at(2), cbs = cfg.at(3), nsel = cfg.at(4), window = cfg.at(5);
+  if (x.dim() != 3 || x.size(1) != 1 || !w.at(5).has_value() || w[5]->dim() != 4) return std::nullopt;
+  const Tensor& mem = *w[5];
+  if (!layer_takes(x, w, heads, mem.size(1), mem.size(3), cbs, mem.size(2))) return std::nullopt;
+  for (const Tensor* t : {&past_k, &past_v, &ck, &cv, &run_k, &run_v})
+    if (t->scalar_type() != x.scalar_type() || t->device() != x.device()) return std::nullopt;
+  return layer_decode(x, w[0], eps, *w[1], *w[2], *w[3], *w[4], inv_freq, mem, past_k, past_v, ck, cv, run_k, run_v, heads, stride, block, cbs,
+                      nsel, window);
+}
+
 // The windows being filled (keys, values: [B, H, cbs, d]) have filled up: the two layers of either compress network, each
 // one launch for both, and the compressed row appended to ck / cv.  -> ck, cv, or nothing where these kernels do not serve.
 static std::optional<std::tuple<Tensor, Tensor>> compress_filled(Tensor run_k, Tensor run_v, OptTensor pos_k, OptTensor pos_v,
@@ -184,6 +201,7 @@ void bind_decode(pybind11::module_& m) {
   namespace py = pybind11;
   m.def("decode_step", &decode_step, py::call_guard<py::gil_scoped_release>());
   m.def("compress_filled", &compress_filled, py::call_guard<py::gil_scoped_release>());
+  m.def("layer_step", &layer_step, py::call_guard<py::gil_scoped_release>());
   m.def("layer_decode", &layer_decode, py::call_guard<py::gil_scoped_release>());
 }
 

@@ -42,8 +42,7 @@ static LayerWeights weights_of(const std::vector<OptTensor>& w) {
 }
 constexpr int kWeights = 16;
 
-// Can the native calls take this input and these parameters (all, or the first six for a decoding step)?
-static bool layer_takes(const Tensor& x, const std::vector<OptTensor>& w, int64_t heads, int64_t kv_heads, int64_t d, int64_t cbs, int64_t num_mem) {
+bool layer_takes(const Tensor& x, const std::vector<OptTensor>& w, int64_t heads, int64_t kv_heads, int64_t d, int64_t cbs, int64_t num_mem) {
   if (x.dim() != 3 || !x.has_storage() || reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 || x.size(2) % 8) return false;
   const int64_t dim = x.size(2);
   if (w.at(0).has_value() && !fits(w[0], x, {dim})) return false;

@@ -61,6 +61,9 @@ inline bool fits(const OptTensor& t, const Tensor& x, at::IntArrayRef sizes) {
          t->sizes() == sizes && t->is_contiguous() && reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0;
 }
 
+// Can the native layer calls take this input and these parameters (all, or the first six for a decoding step)?
+bool layer_takes(const Tensor& x, const std::vector<OptTensor>& w, int64_t heads, int64_t kv_heads, int64_t d, int64_t cbs, int64_t num_mem);
+
 inline nsa_tensor t4(const Tensor& t) { return {t.data_ptr(), t.stride(0), t.stride(1), t.stride(2)}; }
 inline nsa_tensor no_tensor() { return {nullptr, 0, 0, 0}; }
 

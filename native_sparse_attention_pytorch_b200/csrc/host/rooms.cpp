@@ -4,6 +4,8 @@
 
 #include <ATen/core/LegacyTypeDispatch.h>
 
+#include <array>
+
 namespace nsa_host {
 
 Rooms& Rooms::instance() {
@@ -11,8 +13,12 @@ Rooms& Rooms::instance() {
   return *r;
 }
 
+// (what as_strided makes of it below autograd, without the dispatch: four of them are made per step)
 static Tensor rows_of(const Tensor& buf, int64_t first, int64_t rows) {
-  return at::as_strided(buf, {buf.size(0), buf.size(1), rows, buf.size(3)}, buf.strides(), first * buf.size(3));
+  Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::TensorImpl::VIEW, c10::Storage(buf.storage()), buf.key_set(), buf.dtype());
+  t.unsafeGetTensorImpl()->set_sizes_and_strides(std::array<int64_t, 4>{buf.size(0), buf.size(1), rows, buf.size(3)}, buf.strides(),
+                                                 first * buf.size(3));
+  return t;
 }
 
 Rooms::Owner Rooms::current_owner(const Tensor& t) {

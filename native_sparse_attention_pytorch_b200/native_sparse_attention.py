@@ -241,19 +241,18 @@ class SparseAttention(Module):
                                         any(p.requires_grad for p in self.parameters())):
             return None
         d = self.dim_head
-        if x.shape[1] != 1 or d % 8 or d > 128 or self.num_selected_blocks > 32 or self.num_grouped_queries > 16:
+        if d % 8 or d > 128 or self.num_selected_blocks > 32 or self.num_grouped_queries > 16:
             return None
         native = self._native_weights(x)
-        if native is None or not self._layer_takes(x, native[0]):
+        if native is None:
             return None
         for t in (past_k, past_v, ck, cv, run_k, run_v):
-            if t.dtype is not x.dtype or t.device != x.device or t.__class__ is not torch.Tensor:
+            if t.__class__ is not torch.Tensor:
                 return None
-        (norm_w, qkv_w, gate_w, gate_b, out_w, mem_kv), eps = native
-        return L.host().layer_decode(
-            x, norm_w, eps, qkv_w, gate_w, gate_b, out_w, inverse_frequencies(d, self.rotary_emb.theta, x.device), mem_kv,
-            past_k, past_v, ck, cv, run_k, run_v, self.heads, self.compress_block_sliding_stride, self.selection_block_size,
-            self.compress_block_size, self.num_selected_blocks, self.sliding_window_size)
+        return L.host().layer_step(
+            x, native[0], native[1], inverse_frequencies(d, self.rotary_emb.theta, x.device), past_k, past_v, ck, cv, run_k, run_v,
+            (self.heads, self.compress_block_sliding_stride, self.selection_block_size, self.compress_block_size, self.num_selected_blocks,
+             self.sliding_window_size))
 
     def forward_inference(self, inp, cache, return_cache=True):
         """One decoding step (upstream NSA:338-547): `inp` is the newest token [B, 1, dim], `cache` what the previous

@@ -103,17 +103,18 @@ def poll_device_status(device):
     """The same check without a synchronisation, one call late: looks at the status copy the previous poll started
     (if it has landed) and starts the next one.  `SparseAttention.forward` calls this, so a training loop learns of
     an invalid step at its next forward without any host wait on the hot path."""
-    if torch.cuda.is_current_stream_capturing():
-        return                          # a CUDA graph is being recorded: nothing here may touch the host
-    key = torch.device(device).index
+    key = device.index if device.__class__ is torch.device else torch.device(device).index
     if key is None:
         key = torch.cuda.current_device()
-    acc, pending = _status_acc.get(key), _status_polls.get(key)
+    acc = _status_acc.get(key)
     if acc is None:
         return
+    pending = _status_polls.get(key)
     fresh = _status_fresh.get(key) or L.host().backward_ran(key, False)
     if not (fresh or (pending is not None and pending[1])):
         return                          # no such kernel since the last copy, and that copy has been read
+    if torch.cuda.is_current_stream_capturing():
+        return                          # a CUDA graph is being recorded: nothing here may touch the host
     with _state_lock:
         if pending is None:
             pending = _status_polls[key] = [L.host().StatusCopy(acc), False]
