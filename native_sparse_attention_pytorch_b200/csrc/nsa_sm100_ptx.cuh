@@ -58,15 +58,11 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
   }
 }
 
-// The same for a whole warp: one lane polls, the others sleep at the warp barrier and then observe the completed
-// phase themselves (one probe), so that 32 lanes do not poll side by side.
+// The same for a whole warp, which asks as one.
 __device__ __forceinline__ void mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                                long long limit = kWaitLimitCycles) {
-  if ((threadIdx.x & 31) == 0) mbar_wait_bounded(bar, parity, abort_flag, limit);
+  mbar_wait_bounded(bar, parity, abort_flag, limit);
   __syncwarp();
-  while (!mbar_try_wait(bar, parity)) {
-    if (*abort_flag) break;
-  }
 }
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
