@@ -1279,7 +1279,7 @@ struct Cursor {
 };
 }  // namespace ws
 
-template <int D>
+template <int D, bool SLOTS>   // SLOTS: the gradients of the slot scales are wanted
 __global__ void __launch_bounds__(ws::kThreads, 1)
 sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const SelParams P) {
   using namespace ws;
@@ -1345,8 +1345,7 @@ sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     // (plain stores run at memory speed, fp32 reductions into dq are limited by the L2 atomic units).  A thread that
     // stored its own piece would make every store instruction touch 32 lines; the warp stages 32 columns at a time in
     // the group's P tile, which the completed dV product no longer reads, and stores eight rows per instruction.
-    auto dq_out = [&](const int dst_row, const uint32_t use) {
-      mbar_wait_warp(smem_u32(&bars.dq_done[wg]), use & 1, &abort_flag);
+    auto dq_out = [&](const int dst_row) {
       tc_fence_after_sync();
       __syncwarp();
       uint8_t* const pbase = reinterpret_cast<uint8_t*>(P.partial);
@@ -1388,91 +1387,100 @@ sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
       // the two warps that share these rows have read what they staged before either writes P again
       asm volatile("bar.sync %0, 64;" ::"r"(1 + wg * 4 + (warp & 3)) : "memory");
     };
+    // The chunks of the group: every second one of the CTA.  Chunk c of `item`; the next item is requested when this one is entered.
     uint32_t use = 0, flushes = 0;
-    int j = 0, h = 0, b = 0;
-    Cursor cur(P.items, nitems, first_item);
-    auto enter_item = [&]() {
-      const int list = cur.item.x, bh = list / P.nfb;
-      j = list - bh * P.nfb;
-      b = bh / P.Hkv;
-      h = bh - b * P.Hkv;
+    int it = first_item, c = wg, stage = wg % kStages, j = 0, key_row0 = 0, dst0 = 0;
+    int4 item = P.items[it], ahead = P.items[min(it + (int)gridDim.x, nitems - 1)];
+    auto settle = [&](bool entered) {       // onto the item that holds chunk c
+      while (it < nitems && c >= item.z) {
+        c -= item.z;
+        it += gridDim.x;
+        item = ahead;
+        ahead = P.items[min(it + (int)gridDim.x, nitems - 1)];
+        entered = true;
+      }
+      if (!entered || it >= nitems) return;
+      const int bh = item.x / P.nfb;
+      j = item.x - bh * P.nfb;
+      key_row0 = bh * P.Nk;                 // 32 bits hold every row id (see `supported`)
+      dst0 = ((bh - P.bh0) * G + g) * P.N * P.ns;
     };
-    auto entry_of = [&]() { return cur.live() ? __ldg(P.entries + cur.item.w + cur.c * QT + q_local) : kInvalidEntry; };
-    if (wg == 1) cur.next();
-    enter_item();
+    auto entry_of = [&]() { return it < nitems ? __ldg(P.entries + item.w + c * QT + q_local) : kInvalidEntry; };
+    settle(true);
     uint32_t e_next = entry_of();
-    while (cur.live()) {
-      const uint32_t e = e_next;
-      const RowInfo r = decode_row(e, j, P.rule);
-      const int n = cur.n;
-      const uint32_t sMeta = sMeta0 + (n % kStages) * S::kMetaBytes + row * 4;
+    int dst_prev = -1;
+    while (it < nitems) {
+      const RowInfo r = decode_row(e_next, j, P.rule);
+      const uint32_t sMeta = sMeta0 + stage * S::kMetaBytes + row * 4;
       mbar_wait_warp(smem_u32(&bars.s_full[wg]), use & 1, &abort_flag);
       tc_fence_after_sync();
       const float lse2 = __uint_as_float(lds_u32(sMeta)) * kLog2e;
       const float delta = __uint_as_float(lds_u32(sMeta + kRows * 4));
       float slot_part = 0.f;
-      const bool want_slot = P.slot_grads != nullptr;
       // rows that see the whole block need no per-column test; only own-block (causal) and padding rows do
       const bool all_full = __all_sync(kFullMask, r.lim == kBlock - 1 && r.lo == 0);
+      const uint64_t scale2 = pack2(P.scale_log2, P.scale_log2), lse2n = pack2(-lse2, -lse2), delta2n = pack2(-delta, -delta);
 #pragma unroll 1
       for (int q = 0; q < 2; ++q) {         // 16 columns at a time: the body stays small enough for the instruction cache
         const int col = half * 32 + q * 16;
-        float sv[16], dv[16];
-        tmem_ld16(tS + col, sv);
-        tmem_ld16(tS + S::tDP + col, dv);
-        tmem_ld_wait();
-        if (all_full) {
-#pragma unroll
-          for (int x = 0; x < 16; ++x) {
-            const float px = ex2(fmaf(sv[x], P.scale_log2, -lse2));
-            const float dsx = px * (dv[x] - delta);
-            if (want_slot) slot_part = fmaf(dsx, sv[x], slot_part);
-            sv[x] = px;
-            dv[x] = dsx;
-          }
-        } else {
+        uint32_t pw[8], dsw[8];             // P and dS as bf16
+        {
+          float sv[16], dv[16];
+          tmem_ld16(tS + col, sv);
+          tmem_ld16(tS + S::tDP + col, dv);
+          tmem_ld_wait();
           const int rem = r.lim - col, rlo = r.lo - col;   // columns rlo..rem of this group are visible
 #pragma unroll
-          for (int x = 0; x < 16; ++x) {
-            const float px = (x >= rlo && x <= rem) ? ex2(fmaf(sv[x], P.scale_log2, -lse2)) : 0.f;
-            const float dsx = px * (dv[x] - delta);
-            if (want_slot) slot_part = fmaf(dsx, sv[x], slot_part);
-            sv[x] = px;
-            dv[x] = dsx;
+          for (int x = 0; x < 8; ++x) {
+            float p0, p1, d0, d1;
+            unpack2(fma2(pack2(sv[2 * x], sv[2 * x + 1]), scale2, lse2n), p0, p1);
+            p0 = ex2(p0);
+            p1 = ex2(p1);
+            if (!all_full) {
+              p0 = 2 * x >= rlo && 2 * x <= rem ? p0 : 0.f;
+              p1 = 2 * x + 1 >= rlo && 2 * x + 1 <= rem ? p1 : 0.f;
+            }
+            unpack2(mul2(pack2(p0, p1), add2(pack2(dv[2 * x], dv[2 * x + 1]), delta2n)), d0, d1);
+            if constexpr (SLOTS) slot_part = fmaf(d1, sv[2 * x + 1], fmaf(d0, sv[2 * x], slot_part));
+            pw[x] = pack_bf16(p0, p1);
+            dsw[x] = pack_bf16(d0, d1);
           }
         }
         // dK of the group's previous chunk, the last product to read the tiles, is complete
         if (q == 0 && use > 0) mbar_wait_warp(smem_u32(&bars.tiles_free[wg]), (use - 1) & 1, &abort_flag);
 #pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          uint4 pv, dsv;
-          pv.x = pack_bf16(sv[x * 8 + 0], sv[x * 8 + 1]); pv.y = pack_bf16(sv[x * 8 + 2], sv[x * 8 + 3]);
-          pv.z = pack_bf16(sv[x * 8 + 4], sv[x * 8 + 5]); pv.w = pack_bf16(sv[x * 8 + 6], sv[x * 8 + 7]);
-          dsv.x = pack_bf16(dv[x * 8 + 0], dv[x * 8 + 1]); dsv.y = pack_bf16(dv[x * 8 + 2], dv[x * 8 + 3]);
-          dsv.z = pack_bf16(dv[x * 8 + 4], dv[x * 8 + 5]); dsv.w = pack_bf16(dv[x * 8 + 6], dv[x * 8 + 7]);
-          sts_v4(sP + sw128_offset(row, col / 8 + x), pv);
-          sts_v4(sDS + sw128_offset(row, col / 8 + x), dsv);
+        for (int x = 0; x < 2; ++x)
+          sts_v4(sDS + sw128_offset(row, col / 8 + x), make_uint4(dsw[4 * x], dsw[4 * x + 1], dsw[4 * x + 2], dsw[4 * x + 3]));
+        // with a dQ buffer for either group that chunk's rows leave here: its products have run under the arithmetic above
+        if constexpr (S::kDq == 2) {
+          if (q == 0 && use > 0) dq_out(dst_prev);
         }
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+          sts_v4(sP + sw128_offset(row, col / 8 + x), make_uint4(pw[4 * x], pw[4 * x + 1], pw[4 * x + 2], pw[4 * x + 3]));
       }
       fence_proxy_async_smem();
       tc_fence_before_sync();
       mbar_arrive(smem_u32(&bars.p_full[wg]));
-      const int64_t slice_row = ((int64_t)(b * P.Hkv + h - P.bh0) * G + g) * P.N + r.i;
-      const int dst = r.valid ? (int)(slice_row * P.ns + r.slot) : -1;
-      if (want_slot) {   // two threads of a row, in different warps: two additions to a cleared slot
+      dst_prev = r.valid ? dst0 + r.i * P.ns + r.slot : -1;
+      if constexpr (SLOTS) {   // two threads of a row, in different warps: two additions to a cleared slot
         for (int o = G / 2; o > 0; o >>= 1) slot_part += __shfl_xor_sync(kFullMask, slot_part, o);
-        if (r.valid && g == 0 && r.slot < P.nsel)
-          atomicAdd(P.slot_grads + (((int64_t)b * P.Hkv + h) * P.N + r.i) * P.nsel + r.slot, slot_part * P.scale);
+        const int bh = item.x / P.nfb;
+        if (r.valid && g == 0 && r.slot < P.nsel) atomicAdd(P.slot_grads + ((int64_t)bh * P.N + r.i) * P.nsel + r.slot, slot_part * P.scale);
       }
-      // on to the group's next chunk: its entry travels under the read-out of dQ
-      const bool flush = cur.last();
+      // on to the group's next chunk: its entry travels under what is left of this one
+      const bool flush = c == item.z - 1;
       const int key = j * kBlock + (warp & 3) * 16 + (lane & 15);
-      const int64_t key_row = ((int64_t)b * P.Hkv + h) * P.Nk + key;
-      bool entered = cur.next();
-      if (cur.live()) entered = cur.next() || entered;
-      if (entered && cur.live()) enter_item();
+      const int64_t key_row = (int64_t)key_row0 + key;
+      c += 2;
+      stage += 2;
+      if (stage >= kStages) stage -= kStages;
+      settle(false);
       e_next = entry_of();
-      dq_out(dst, use);
+      if constexpr (S::kDq == 1) {          // one dQ buffer for both groups: the other one is waiting for it
+        mbar_wait_warp(smem_u32(&bars.dq_done[wg]), use & 1, &abort_flag);
+        dq_out(dst_prev);
+      }
       ++use;
       if (flush) {
         // flush dK/dV of this item: keys 16w..16w+15 live in the lanes of quarter w, either half of the group takes half of
@@ -1486,17 +1494,23 @@ sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         const float f = lane < 16 ? 1.f : P.scale;
         float* const dstp = (lane < 16 ? P.dv : P.dk) + key_row * D + half * (D / 2);
 #pragma unroll 1
-        for (int c = 0; c < D / 2; c += 32) {
+        for (int cc = 0; cc < D / 2; cc += 32) {
           float tk[32];
-          tmem_ld32(tm_quarter + S::tAcc + half * (D / 2) + c, tk);
+          tmem_ld32(tm_quarter + S::tAcc + half * (D / 2) + cc, tk);
           tmem_ld_wait();
           if (key < P.Nk) {
 #pragma unroll
-            for (int x = 0; x < 8; ++x) red_add_v4(dstp + c + x * 4, tk[x * 4] * f, tk[x * 4 + 1] * f, tk[x * 4 + 2] * f, tk[x * 4 + 3] * f);
+            for (int x = 0; x < 8; ++x) red_add_v4(dstp + cc + x * 4, tk[x * 4] * f, tk[x * 4 + 1] * f, tk[x * 4 + 2] * f, tk[x * 4 + 3] * f);
           }
         }
         tc_fence_before_sync();
         mbar_arrive(smem_u32(&bars.acc_free));
+      }
+    }
+    if constexpr (S::kDq == 2) {
+      if (use > 0) {
+        mbar_wait_warp(smem_u32(&bars.tiles_free[wg]), (use - 1) & 1, &abort_flag);
+        dq_out(dst_prev);
       }
     }
   } else if (warp == kSoftmaxWarps) {
@@ -1557,7 +1571,7 @@ sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
       const uint32_t tDQ = tm + S::tDQ + (S::kDq == 2 ? grp * D : 0);
 #pragma unroll
       for (int k = 0; k < 4; ++k) mma_bf16_elect(tDQ, desc_advance(dDSt, k * 32), desc_advance(dKt, k * 2048), idDQ, k > 0);
-      mma_commit_elect(smem_u32(&bars.dq_done[grp]));
+      if (S::kDq == 1) mma_commit_elect(smem_u32(&bars.dq_done[grp]));
       // dK += dS^T Q
 #pragma unroll
       for (int k = 0; k < 8; ++k)
@@ -1602,42 +1616,58 @@ sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     constexpr int CH = D / 8, RPP = kLoaderThreads / CH, kPasses = kRows / RPP;   // pieces per row, rows per pass
     const int lt = tid - (kSoftmaxWarps + 3) * 32;   // 0..127
     const int sub = lt % CH, r0 = lt / CH;
+    // A thread's rows are RPP apart: with up to RPP heads per KV head all of the same head (at dim_head 128 and 16 heads the odd
+    // passes are eight heads on).  Row strides are 32-bit (see problem_bwd): one multiplication per row and tensor.
+    const int g0 = r0 & (G - 1), g1 = (r0 + RPP) & (G - 1);
+    const uint32_t q_sn = (uint32_t)P.q_sn, do_sn = (uint32_t)P.do_sn, off0 = sw128_offset(r0, sub % 8);
+    const __nv_bfloat16 *q_head[2] = {nullptr, nullptr}, *do_head[2] = {nullptr, nullptr};
+    const float *lse_head = nullptr, *delta_head = nullptr;
+    int list_of = -1;
     for (Cursor cur(P.items, nitems, first_item); cur.live(); cur.next()) {
-      const int bh = cur.item.x / P.nfb, b = bh / P.Hkv, h = bh - b * P.Hkv;
-      const __nv_bfloat16* qb = P.q + b * P.q_sb + sub * 8;
-      const __nv_bfloat16* dob = P.dout + b * P.do_sb + sub * 8;
+      if (cur.item.x != list_of) {
+        list_of = cur.item.x;
+        const int bh = list_of / P.nfb, b = bh / P.Hkv, h = bh - b * P.Hkv;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const int64_t hq = (int64_t)h * G + (k == 0 ? g0 : g1);
+          q_head[k] = P.q + b * P.q_sb + hq * P.q_sh + sub * 8;
+          do_head[k] = P.dout + b * P.do_sb + hq * P.do_sh + sub * 8;
+        }
+        const int64_t row0 = ((int64_t)b * P.Hq + (int64_t)h * G + (lt & (G - 1))) * P.N;
+        lse_head = P.lse + row0;
+        delta_head = P.delta + row0;
+      }
       const int stage = cur.n % kStages;
-      if (cur.n >= kStages) mbar_wait_warp(smem_u32(&bars.q_free[stage]), (uint32_t)(cur.n / kStages - 1) & 1, &abort_flag);
-      const uint32_t sQ = sQ0 + stage * S::kStageBytes + (sub / 8) * 16384, sDO = sQ + S::kTileQ;
       const uint32_t* chunk_entries = P.entries + cur.item.w + cur.c * QT;
+      // read the entries first: the copies below are compiler barriers, a load placed between them would be
+      // waited for eight times
+      uint32_t ev[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) ev[k] = __ldg(chunk_entries + ((r0 + k * RPP) >> g_shift));
+      const uint32_t es = __ldg(chunk_entries + (lt >> g_shift));
+      if (cur.n >= kStages) mbar_wait_warp(smem_u32(&bars.q_free[stage]), (uint32_t)(cur.n / kStages - 1) & 1, &abort_flag);
+      const uint32_t sQ = sQ0 + stage * S::kStageBytes + (sub / 8) * 16384 + off0, sDO = sQ + S::kTileQ;
 #pragma unroll
       for (int k0 = 0; k0 < kPasses; k0 += 8) {
-        // read the entries first: the copies below are compiler barriers, a load placed between them would be
-        // waited for eight times
-        uint32_t ev[8];
+        if (k0 > 0)
 #pragma unroll
-        for (int k = 0; k < 8; ++k) ev[k] = __ldg(chunk_entries + ((r0 + (k0 + k) * RPP) >> g_shift));
+          for (int k = 0; k < 8; ++k) ev[k] = __ldg(chunk_entries + ((r0 + (k0 + k) * RPP) >> g_shift));
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-          const int row = r0 + (k0 + k) * RPP;
-          const int g = row & ((1 << g_shift) - 1);
           const bool valid = ev[k] != kInvalidEntry;
-          const int64_t i = valid ? (int64_t)(ev[k] & 0xffffffu) : 0;
-          const int64_t hq = (int64_t)((h << g_shift) + g);
-          const uint32_t off = sw128_offset(row, sub % 8);
-          cp_async16(sQ + off, qb + hq * P.q_sh + i * P.q_sn, valid ? 16u : 0u);
-          cp_async16(sDO + off, dob + hq * P.do_sh + i * P.do_sn, valid ? 16u : 0u);
+          const uint32_t i = valid ? ev[k] & 0xffffffu : 0u, bytes = valid ? 16u : 0u;
+          const uint32_t off = (k0 + k) * RPP * 128;       // RPP is a multiple of 8: the swizzle of all its rows is that of r0
+          cp_async16(sQ + off, q_head[k & 1] + (uint64_t)i * q_sn, bytes);
+          cp_async16(sDO + off, do_head[k & 1] + (uint64_t)i * do_sn, bytes);
         }
       }
       {
         // the statistics of row lt
-        const uint32_t e = __ldg(chunk_entries + (lt >> g_shift));
-        const bool valid = e != kInvalidEntry;
-        const int64_t row = ((int64_t)b * P.Hq + (int64_t)((h << g_shift) + (lt & ((1 << g_shift) - 1)))) * P.N +
-                            (valid ? (int64_t)(e & 0xffffffu) : 0);
+        const bool valid = es != kInvalidEntry;
+        const uint32_t i = valid ? es & 0xffffffu : 0u, bytes = valid ? 4u : 0u;
         const uint32_t sMeta = sMeta0 + stage * S::kMetaBytes + lt * 4;
-        cp_async4(sMeta, P.lse + row, valid ? 4u : 0u);
-        cp_async4(sMeta + kRows * 4, P.delta + row, valid ? 4u : 0u);
+        cp_async4(sMeta, lse_head + i, bytes);
+        cp_async4(sMeta + kRows * 4, delta_head + i, bytes);
       }
       // the stage announces itself when this thread's copies have landed; the thread moves on at once
       cp_async_arrive_noinc(smem_u32(&bars.q_full[stage]));
@@ -2125,12 +2155,14 @@ static int run_bwd(const SelProblem& a, const SelPlan& p, uint8_t* ws, cudaStrea
   if (own_delta) sel_delta_kernel<D><<<row_blocks + kv_blocks, 256, 0, st>>>(P, delta, row_blocks, kv_pieces);
   else if (kv_pieces > 0) CUDA_TRY(cudaMemsetAsync(a.dk, 0, (size_t)kv_pieces * 16, st));
   if (a.slot_grads != nullptr) CUDA_TRY(cudaMemsetAsync(a.slot_grads, 0, (size_t)a.B * a.Hkv * a.N * a.nsel * sizeof(float), st));
-  CUDA_TRY(allow_shared_memory<sel_bwd_ws_kernel<D>>());
+  CUDA_TRY((allow_shared_memory<sel_bwd_ws_kernel<D, false>>()));
+  if (a.slot_grads != nullptr) CUDA_TRY((allow_shared_memory<sel_bwd_ws_kernel<D, true>>()));
   P.partial = reinterpret_cast<__nv_bfloat16*>(ws + p.off_partial);
   for (int s = 0; s < p.slices; ++s) {
     P.bh0 = s * p.pairs_per_slice;
     P.bh1 = P.bh0 + p.pairs_per_slice < a.B * a.Hkv ? P.bh0 + p.pairs_per_slice : a.B * a.Hkv;
-    sel_bwd_ws_kernel<D><<<num_sms(), ws::kThreads, ws::Shape<D>::kBytes, st>>>(tmK, tmV, P);
+    if (a.slot_grads != nullptr) sel_bwd_ws_kernel<D, true><<<num_sms(), ws::kThreads, ws::Shape<D>::kBytes, st>>>(tmK, tmV, P);
+    else sel_bwd_ws_kernel<D, false><<<num_sms(), ws::kThreads, ws::Shape<D>::kBytes, st>>>(tmK, tmV, P);
     const unsigned mblocks = (unsigned)(((int64_t)(P.bh1 - P.bh0) * p.G * a.N * (D / 8) + 255) / 256);
     const bool last = s == p.slices - 1;
     const unsigned grid = mblocks + (last ? (kv_blocks + 1) / 2 : 0);
@@ -2209,6 +2241,7 @@ static int problem_fwd(const SelProblem& x, cudaStream_t st) {
 }
 
 static int problem_bwd(const SelProblem& x, cudaStream_t st) {
+  if (x.q.stride_n >> 32 || x.dout.stride_n >> 32) return NSA_ERR_UNSUPPORTED;   // the gathers multiply in 32 bits
   const SelPlan p = make_plan(x, true);
   uint8_t* ws = nullptr;
   const int rc = check_ws(x, p, &ws);
