@@ -1237,7 +1237,10 @@ struct Shape {
   static constexpr int kKv = D == 64 ? 2 : 1;              // K / V buffers
   static constexpr int kDq = D == 64 ? 2 : 1;              // dQ buffers in tensor memory
   static constexpr uint32_t kTileQ = NC * 16384, kStageBytes = 2 * kTileQ, kTileK = NC * 8192, kKvBytes = 2 * kTileK;
-  static constexpr uint32_t kMetaBytes = 2 * kRows * 4;    // per stage: lse, delta of every row of the chunk
+  // Per stage: lse and delta of every row of the chunk; where there is room, also what the loaders know of the rows already:
+  // the (row, slot) id its dQ goes to, the visible columns, and for an item's last chunk the keys whose dK / dV are complete
+  static constexpr bool kRowMeta = D == 64;
+  static constexpr uint32_t kMetaBytes = kRowMeta ? 4 * kRows * 4 + 16 : 2 * kRows * 4;
   static constexpr uint32_t kBytes = kStages * kStageBytes + 2 * kPBytes + kKv * kKvBytes + kStages * kMetaBytes;
   static constexpr uint32_t tGroup = 128, tDP = 64, tAcc = 256, tDQ = tAcc + D;   // tensor-memory columns
 };
@@ -1302,7 +1305,7 @@ sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     abort_flag = 0;
     if (base & 1023u) abort_flag = 1;   // the tiles would be mis-swizzled: report instead of computing
     for (int i = 0; i < 3; ++i) {
-      mbar_init(smem_u32(&bars.q_full[i]), kLoaderThreads);
+      mbar_init(smem_u32(&bars.q_full[i]), (S::kRowMeta ? 2 : 1) * kLoaderThreads);
       mbar_init(smem_u32(&bars.q_free[i]), 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -1387,10 +1390,16 @@ sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
       // the two warps that share these rows have read what they staged before either writes P again
       asm volatile("bar.sync %0, 64;" ::"r"(1 + wg * 4 + (warp & 3)) : "memory");
     };
-    // The chunks of the group: every second one of the CTA.  Chunk c of `item`; the next item is requested when this one is entered.
+    // The chunks of the group: every second one of the CTA
+    int chunks = 0;
+    for (int t = first_item + lane * (int)gridDim.x; t < nitems; t += 32 * (int)gridDim.x) chunks += P.items[t].z;
+    chunks = (int)__reduce_add_sync(kFullMask, (unsigned)chunks);
     uint32_t use = 0, flushes = 0;
-    int it = first_item, c = wg, stage = wg % kStages, j = 0, key_row0 = 0, dst0 = 0;
-    int4 item = P.items[it], ahead = P.items[min(it + (int)gridDim.x, nitems - 1)];
+    int stage = wg % kStages;
+    // Without room for the rows' data beside the stage the groups look them up themselves: chunk c of `item`; the next item is
+    // requested when this one is entered
+    int it = first_item, c = wg, j = 0, key_row0 = 0, dst0 = 0;
+    int4 item = make_int4(0, 0, 0, 0), ahead = item;
     auto settle = [&](bool entered) {       // onto the item that holds chunk c
       while (it < nitems && c >= item.z) {
         c -= item.z;
@@ -1406,19 +1415,40 @@ sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
       dst0 = ((bh - P.bh0) * G + g) * P.N * P.ns;
     };
     auto entry_of = [&]() { return it < nitems ? __ldg(P.entries + item.w + c * QT + q_local) : kInvalidEntry; };
-    settle(true);
-    uint32_t e_next = entry_of();
+    uint32_t e_next = kInvalidEntry;
+    if constexpr (!S::kRowMeta) {
+      item = P.items[it];
+      ahead = P.items[min(it + (int)gridDim.x, nitems - 1)];
+      settle(true);
+      e_next = entry_of();
+    }
     int dst_prev = -1;
-    while (it < nitems) {
-      const RowInfo r = decode_row(e_next, j, P.rule);
+    for (int n = wg; n < chunks; n += 2) {
       const uint32_t sMeta = sMeta0 + stage * S::kMetaBytes + row * 4;
       mbar_wait_warp(smem_u32(&bars.s_full[wg]), use & 1, &abort_flag);
       tc_fence_after_sync();
       const float lse2 = __uint_as_float(lds_u32(sMeta)) * kLog2e;
       const float delta = __uint_as_float(lds_u32(sMeta + kRows * 4));
+      int dst, lo, lim, key_row, keys;      // first visible column, last one (-1: padding); key_row < 0: not an item's last chunk
+      if constexpr (S::kRowMeta) {
+        dst = (int)lds_u32(sMeta + 2 * kRows * 4);
+        const int cols = (int)lds_u32(sMeta + 3 * kRows * 4);
+        lo = cols & 0xff;
+        lim = cols >> 8;
+        const uint2 last = lds_v2(sMeta0 + stage * S::kMetaBytes + 4 * kRows * 4);
+        key_row = (int)last.x;
+        keys = (int)last.y;
+      } else {
+        const RowInfo r = decode_row(e_next, j, P.rule);
+        dst = r.valid ? dst0 + r.i * P.ns + r.slot : -1;
+        lo = r.lo;
+        lim = r.lim;
+        key_row = c == item.z - 1 ? key_row0 + j * kBlock : -1;
+        keys = P.Nk - j * kBlock;
+      }
       float slot_part = 0.f;
       // rows that see the whole block need no per-column test; only own-block (causal) and padding rows do
-      const bool all_full = __all_sync(kFullMask, r.lim == kBlock - 1 && r.lo == 0);
+      const bool all_full = __all_sync(kFullMask, lim == kBlock - 1 && lo == 0);
       const uint64_t scale2 = pack2(P.scale_log2, P.scale_log2), lse2n = pack2(-lse2, -lse2), delta2n = pack2(-delta, -delta);
 #pragma unroll 1
       for (int q = 0; q < 2; ++q) {         // 16 columns at a time: the body stays small enough for the instruction cache
@@ -1429,7 +1459,7 @@ sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
           tmem_ld16(tS + col, sv);
           tmem_ld16(tS + S::tDP + col, dv);
           tmem_ld_wait();
-          const int rem = r.lim - col, rlo = r.lo - col;   // columns rlo..rem of this group are visible
+          const int rem = lim - col, rlo = lo - col;       // columns rlo..rem of this group are visible
 #pragma unroll
           for (int x = 0; x < 8; ++x) {
             float p0, p1, d0, d1;
@@ -1462,27 +1492,28 @@ sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
       fence_proxy_async_smem();
       tc_fence_before_sync();
       mbar_arrive(smem_u32(&bars.p_full[wg]));
-      dst_prev = r.valid ? dst0 + r.i * P.ns + r.slot : -1;
+      dst_prev = dst;
       if constexpr (SLOTS) {   // two threads of a row, in different warps: two additions to a cleared slot
         for (int o = G / 2; o > 0; o >>= 1) slot_part += __shfl_xor_sync(kFullMask, slot_part, o);
-        const int bh = item.x / P.nfb;
-        if (r.valid && g == 0 && r.slot < P.nsel) atomicAdd(P.slot_grads + ((int64_t)bh * P.N + r.i) * P.nsel + r.slot, slot_part * P.scale);
+        if (dst >= 0 && g == 0) {           // dst = (row of the slice) ns + slot
+          const int part_row = dst / P.ns, slot = dst - part_row * P.ns, pair = part_row / P.N;   // (batch, query head) of the slice
+          const int64_t query = (int64_t)(P.bh0 + pair / G) * P.N + (part_row - pair * P.N);
+          if (slot < P.nsel) atomicAdd(P.slot_grads + query * P.nsel + slot, slot_part * P.scale);
+        }
       }
-      // on to the group's next chunk: its entry travels under what is left of this one
-      const bool flush = c == item.z - 1;
-      const int key = j * kBlock + (warp & 3) * 16 + (lane & 15);
-      const int64_t key_row = (int64_t)key_row0 + key;
-      c += 2;
       stage += 2;
       if (stage >= kStages) stage -= kStages;
-      settle(false);
-      e_next = entry_of();
+      if constexpr (!S::kRowMeta) {         // on to the group's next chunk: its entry travels under what is left of this one
+        c += 2;
+        settle(false);
+        e_next = entry_of();
+      }
       if constexpr (S::kDq == 1) {          // one dQ buffer for both groups: the other one is waiting for it
         mbar_wait_warp(smem_u32(&bars.dq_done[wg]), use & 1, &abort_flag);
         dq_out(dst_prev);
       }
       ++use;
-      if (flush) {
+      if (key_row >= 0) {
         // flush dK/dV of this item: keys 16w..16w+15 live in the lanes of quarter w, either half of the group takes half of
         // the columns.  "Accumulator complete" has one barrier per flushing group, counted by
         // that group: with one barrier for both, a group that reached its wait before the other group's item was complete
@@ -1492,13 +1523,14 @@ sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         tc_fence_after_sync();
         __syncwarp();
         const float f = lane < 16 ? 1.f : P.scale;
-        float* const dstp = (lane < 16 ? P.dv : P.dk) + key_row * D + half * (D / 2);
+        const int key = (warp & 3) * 16 + (lane & 15);
+        float* const dstp = (lane < 16 ? P.dv : P.dk) + ((int64_t)key_row + key) * D + half * (D / 2);
 #pragma unroll 1
         for (int cc = 0; cc < D / 2; cc += 32) {
           float tk[32];
           tmem_ld32(tm_quarter + S::tAcc + half * (D / 2) + cc, tk);
           tmem_ld_wait();
-          if (key < P.Nk) {
+          if (key < keys) {
 #pragma unroll
             for (int x = 0; x < 8; ++x) red_add_v4(dstp + cc + x * 4, tk[x * 4] * f, tk[x * 4 + 1] * f, tk[x * 4 + 2] * f, tk[x * 4 + 3] * f);
           }
@@ -1622,7 +1654,7 @@ sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     const uint32_t q_sn = (uint32_t)P.q_sn, do_sn = (uint32_t)P.do_sn, off0 = sw128_offset(r0, sub % 8);
     const __nv_bfloat16 *q_head[2] = {nullptr, nullptr}, *do_head[2] = {nullptr, nullptr};
     const float *lse_head = nullptr, *delta_head = nullptr;
-    int list_of = -1;
+    int list_of = -1, j = 0, key_row0 = 0, dst0 = 0;
     for (Cursor cur(P.items, nitems, first_item); cur.live(); cur.next()) {
       if (cur.item.x != list_of) {
         list_of = cur.item.x;
@@ -1633,6 +1665,9 @@ sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
           q_head[k] = P.q + b * P.q_sb + hq * P.q_sh + sub * 8;
           do_head[k] = P.dout + b * P.do_sb + hq * P.do_sh + sub * 8;
         }
+        j = list_of - bh * P.nfb;
+        key_row0 = bh * P.Nk + j * kBlock;   // 32 bits hold every row id (see `supported`)
+        dst0 = ((bh - P.bh0) * G + (lt & (G - 1))) * P.N * P.ns;
         const int64_t row0 = ((int64_t)b * P.Hq + (int64_t)h * G + (lt & (G - 1))) * P.N;
         lse_head = P.lse + row0;
         delta_head = P.delta + row0;
@@ -1668,6 +1703,17 @@ sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         const uint32_t sMeta = sMeta0 + stage * S::kMetaBytes + lt * 4;
         cp_async4(sMeta, lse_head + i, bytes);
         cp_async4(sMeta + kRows * 4, delta_head + i, bytes);
+        if constexpr (S::kRowMeta) {
+          const RowInfo r = decode_row(es, j, P.rule);
+          sts_u32(sMeta + 2 * kRows * 4, (uint32_t)(valid ? dst0 + r.i * P.ns + r.slot : -1));
+          sts_u32(sMeta + 3 * kRows * 4, (uint32_t)(r.lim * 256 + r.lo));
+          if (lt == 0) {
+            const uint32_t last = sMeta + 4 * kRows * 4;
+            sts_u32(last, (uint32_t)(cur.last() ? key_row0 : -1));
+            sts_u32(last + 4, (uint32_t)(P.Nk - j * kBlock));
+          }
+          mbar_arrive(smem_u32(&bars.q_full[stage]));   // these are stores: announced apart from the copies
+        }
       }
       // the stage announces itself when this thread's copies have landed; the thread moves on at once
       cp_async_arrive_noinc(smem_u32(&bars.q_full[stage]));
