@@ -294,6 +294,12 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// The largest of three
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 // Two fp32 operations per instruction, each rounded as the single one is
 __device__ __forceinline__ uint64_t pack2(float a, float b) {
   uint64_t r;

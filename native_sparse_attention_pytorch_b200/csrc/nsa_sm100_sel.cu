@@ -340,6 +340,34 @@ __device__ __forceinline__ RowInfo decode_row(uint32_t e, int j, const BlockRule
   return r;
 }
 
+// The largest of 32 values
+__device__ __forceinline__ float max32(const float (&s)[32]) {
+  float m[4] = {fmaxf(s[0], s[1]), fmaxf(s[2], s[3]), fmaxf(s[4], s[5]), fmaxf(s[6], s[7])};
+#pragma unroll
+  for (int x = 8; x < 32; x += 8)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) m[k] = max3(m[k], s[x + 2 * k], s[x + 2 * k + 1]);
+  return fmaxf(max3(m[0], m[1], m[2]), m[3]);
+}
+// s = 2^(s * scale2 - off) in place; the sum, in fp32 (four partial sums: values x with equal x % 4)
+__device__ __forceinline__ float exp_row32(float (&s)[32], float scale_log2, float off) {
+  const uint64_t scale2 = pack2(scale_log2, scale_log2), off2 = pack2(-off, -off);
+  uint64_t l0 = 0ull, l1 = 0ull;
+#pragma unroll
+  for (int x = 0; x < 32; x += 4) {
+    unpack2(fma2(pack2(s[x], s[x + 1]), scale2, off2), s[x], s[x + 1]);
+    unpack2(fma2(pack2(s[x + 2], s[x + 3]), scale2, off2), s[x + 2], s[x + 3]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) s[x + k] = ex2(s[x + k]);
+    l0 = add2(l0, pack2(s[x], s[x + 1]));
+    l1 = add2(l1, pack2(s[x + 2], s[x + 3]));
+  }
+  float a, b, c, d;
+  unpack2(l0, a, b);
+  unpack2(l1, c, d);
+  return (a + b) + (c + d);
+}
+
 // ---- forward -------------------------------------------------------------------------
 
 // Forward of the selected-block branch.  A CTA of 256 threads walks gather -> S -> softmax -> P V -> store chunk by
@@ -350,26 +378,27 @@ __device__ __forceinline__ RowInfo decode_row(uint32_t e, int j, const BlockRule
 // and more), plus 440 for the bulk store of the partial rows; the chunk takes 1900.  With the partial rows stored row by
 // row through the load / store units it took 2200: batch 4, 8192 positions, 32 / 4 heads of 64 1.10 -> 0.96 ms, 65536
 // positions, 64 / 8 heads of 128 9.1 -> 7.4 ms.
+// A thread's rows are RPP apart, with up to RPP heads per KV head all of the same head (at dim_head 128 every row of 16 heads:
+// RPP is 16): `head` is that head's row 0 at the thread's piece.  Row strides are 32-bit (see problem_fwd).
 template <int D>
-__device__ __forceinline__ void gather_tile_async2(uint32_t tile, const __nv_bfloat16* base, int64_t stride_h,
-                                                   int64_t stride_n, const uint32_t* entries, int g_shift, int h,
-                                                   int tid) {
-  constexpr int CH = D / 8;               // 16-byte pieces per row
-  constexpr int RPP = 2 * kRows / CH;     // rows covered by one pass of the 256 threads
-  const int sub = tid % CH, r0 = tid / CH;
-  uint32_t ev[kRows / RPP];
+struct GatherTile {
+  static constexpr int CH = D / 8;               // 16-byte pieces per row
+  static constexpr int RPP = 2 * kRows / CH;     // rows covered by one pass of the 256 threads
+  __device__ __forceinline__ static void issue(uint32_t tile, const __nv_bfloat16* head, uint32_t stride_n, const uint32_t* entries,
+                                               int g_shift, int tid) {
+    const int sub = tid % CH, r0 = tid / CH;
+    uint32_t ev[kRows / RPP];
 #pragma unroll
-  for (int it = 0; it < kRows / RPP; ++it) ev[it] = __ldg(entries + ((r0 + it * RPP) >> g_shift));
+    for (int it = 0; it < kRows / RPP; ++it) ev[it] = __ldg(entries + ((r0 + it * RPP) >> g_shift));
+    const uint32_t dst = tile + (sub / 8) * (kRows * 128) + sw128_offset(r0, sub % 8);   // (RPP is a multiple of 8)
 #pragma unroll
-  for (int it = 0; it < kRows / RPP; ++it) {
-    const int row = r0 + it * RPP;
-    const int g = row & ((1 << g_shift) - 1);
-    const bool valid = ev[it] != kInvalidEntry;
-    const int64_t i = valid ? (int64_t)(ev[it] & 0xffffffu) : 0;
-    cp_async16(tile + (sub / 8) * (kRows * 128) + sw128_offset(row, sub % 8),
-               base + (int64_t)((h << g_shift) + g) * stride_h + i * stride_n + sub * 8, valid ? 16u : 0u);
+    for (int it = 0; it < kRows / RPP; ++it) {
+      const bool valid = ev[it] != kInvalidEntry;
+      const uint32_t i = valid ? ev[it] & 0xffffffu : 0u;
+      cp_async16(dst + it * RPP * 128, head + (uint64_t)i * stride_n, valid ? 16u : 0u);
+    }
   }
-}
+};
 
 template <int D>
 __global__ void __launch_bounds__(2 * kRows, D == 64 ? 4 : 2)
@@ -428,11 +457,13 @@ sel_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
         tma_load_4d(sV + c * 8192, &tmV, bar_kv, c * 64, j * kBlock, h, b);
       }
     }
+    const __nv_bfloat16* const q_head =
+        P.q + b * P.q_sb + (int64_t)(h * G + (tid / GatherTile<D>::CH & (G - 1))) * P.q_sh + tid % GatherTile<D>::CH * 8;
     bool prefetched = false;
     for (int c = 0; c < item.z; ++c) {
       const uint32_t* chunk_entries = P.entries + item.w + c * QT;
       const uint32_t e = chunk_entries[q_local];
-      if (!prefetched) gather_tile_async2<D>(sQ, P.q + b * P.q_sb, P.q_sh, P.q_sn, chunk_entries, g_shift, h, tid);
+      if (!prefetched) GatherTile<D>::issue(sQ, q_head, (uint32_t)P.q_sn, chunk_entries, g_shift, tid);
       cp_async_commit();
       cp_async_wait<0>();
       fence_proxy_async_smem();
@@ -459,7 +490,7 @@ sel_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
       // softmax, second MMA and output run
       prefetched = c + 1 < item.z;
       if (prefetched)
-        gather_tile_async2<D>(sQ, P.q + b * P.q_sb, P.q_sh, P.q_sn, chunk_entries + QT, g_shift, h, tid);
+        GatherTile<D>::issue(sQ, q_head, (uint32_t)P.q_sn, chunk_entries + QT, g_shift, tid);
       __syncwarp();
       const RowInfo r = decode_row(e, j, P.rule);
       const int lim = r.lim - half * 32;   // last visible column of this thread's half (negative: none)
@@ -467,35 +498,31 @@ sel_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
       tmem_ld32(tm_lane + tS + half * 32, s);
       tmem_ld_wait();
       const bool all_full = __all_sync(kFullMask, lim >= 31);
-      float mm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      float m = -INFINITY;
       if (all_full) {
-#pragma unroll
-        for (int x = 0; x < 32; ++x) mm[x & 3] = fmaxf(mm[x & 3], s[x]);
+        m = max32(s);
       } else {
 #pragma unroll
-        for (int x = 0; x < 32; ++x) mm[x & 3] = x <= lim ? fmaxf(mm[x & 3], s[x]) : mm[x & 3];
+        for (int x = 0; x < 32; ++x) m = x <= lim ? fmaxf(m, s[x]) : m;
       }
-      float m = fmaxf(fmaxf(mm[0], mm[1]), fmaxf(mm[2], mm[3]));
       xmax[half][row] = m;
       if (tid == 0) bulk_wait_read();   // the staging tile's last store has left shared memory (written again behind the barriers)
       __syncthreads();
       m = fmaxf(m, xmax[half ^ 1][row]);
       const float m2 = r.valid ? m * P.scale_log2 : 0.f;
-      float ll[4] = {0.f, 0.f, 0.f, 0.f};
+      float l_half;          // the fp32 sum: the log-sum-exp stays exact although P is rounded to bf16 for the MMA
       if (all_full) {
-#pragma unroll
-        for (int x = 0; x < 32; ++x) {
-          s[x] = ex2(fmaf(s[x], P.scale_log2, -m2));
-          ll[x & 3] += s[x];   // the fp32 sum: the log-sum-exp stays exact although P is rounded to bf16 for the MMA
-        }
+        l_half = exp_row32(s, P.scale_log2, m2);
       } else {
+        float ll[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int x = 0; x < 32; ++x) {
           s[x] = x <= lim ? ex2(fmaf(s[x], P.scale_log2, -m2)) : 0.f;
           ll[x & 3] += s[x];
         }
+        l_half = (ll[0] + ll[1]) + (ll[2] + ll[3]);
       }
-      xsum[half][row] = (ll[0] + ll[1]) + (ll[2] + ll[3]);
+      xsum[half][row] = l_half;
       // P goes to the tensor cores through tensor memory, over the first half of this row's S columns (both threads
       // of the row have read their S columns: the exchange of the maxima lies in between)
       tmem_st_bf16_row32(tm_lane + tS + half * 16, s);
@@ -957,10 +984,7 @@ dense_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           for (int x = 0; x < 32; ++x)
             if (x < lo || x > lim) x0[x] = -INFINITY;
         }
-        float mm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-        for (int x = 0; x < 32; ++x) mm[x & 3] = fmaxf(mm[x & 3], x0[x]);
-        float m = fmaxf(fmaxf(mm[0], mm[1]), fmaxf(mm[2], mm[3]));
+        float m = max32(x0);
         // the row maximum over both halves; behind the barrier both have also read their S columns and written the ring
         xchg[u & 1][s][half][row] = m;
         pair_sync();
@@ -1016,14 +1040,7 @@ dense_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           tmem_st_wait();
         }
         // a masked logit is -inf and gives 0; a row that has seen nothing yet must not compute -inf - -inf
-        const float off = m_ref == -INFINITY ? 0.f : -m_ref;
-        float ll[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int x = 0; x < 32; ++x) {
-          x0[x] = ex2(fmaf(x0[x], P.scale_log2, off));
-          ll[x & 3] += x0[x];
-        }
-        l += (ll[0] + ll[1]) + (ll[2] + ll[3]);
+        l += exp_row32(x0, P.scale_log2, m_ref == -INFINITY ? 0.f : m_ref);
         // P through tensor memory, over the first 32 columns of the row's S; S(t+2), which is issued after PV(t) by the
         // same lane, overwrites them only after PV(t) has read them
         tmem_st_bf16_row32(tS + half * 16, x0);
@@ -2279,6 +2296,7 @@ static int check_ws(const SelProblem& x, const SelPlan& p, uint8_t** ws) {
 }
 
 static int problem_fwd(const SelProblem& x, cudaStream_t st) {
+  if (x.q.stride_n >> 32) return NSA_ERR_UNSUPPORTED;   // the gathers multiply in 32 bits
   const SelPlan p = make_plan(x, false);
   uint8_t* ws = nullptr;
   const int rc = check_ws(x, p, &ws);
