@@ -104,7 +104,7 @@ struct SelParams {
   const int4* items;
   const int* num_items;    // [0] items, [1] the tag the item kernel left
   const int* list_item;    // per list (and one more): its first item
-  const int* positions;    // kModeSel: [B*Hkv*N][ns], the entry of every (query, slot)
+  const int* positions;    // kModeSel: [B*Hkv*N][ns], the entry of every (query, slot), -1 where the query does not have it
   int bh0, bh1;            // backward: the (batch, KV head) pairs of this launch, whose partial results share the buffer
   const uint32_t* bits;    // [B*Hkv*N][words]: the slots a query has (kModeSel)
   int words;
@@ -301,6 +301,7 @@ __global__ void __launch_bounds__(kIndexQueries) sel_fill_kernel(const BlockRule
     int blk = 0;
     const bool valid = i < R.N && slot_block<MODE>(R, bh, i, s, &blk);
     const unsigned vm = __ballot_sync(kFullMask, valid);
+    if (MODE == kModeSel && !valid && i < R.N) positions[((int64_t)bh * R.N + i) * R.ns + s] = -1;
     if (valid) {
       const unsigned peers = __match_any_sync(vm, blk);
       const int leader = __ffs(peers) - 1;
@@ -582,67 +583,64 @@ sel_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
 
 // Merges the partial results of head g of the group (batch, KV head) bh at query i: acc[8] of a thread's 16-byte piece
 // (unnormalised), the reference maximum and the sum.  The D/8 threads of a row (neighbouring lanes) share the work on the
-// slots: each looks up the position and the statistics of every D/8-th one, and hands them on by shuffles; the rows' loads
-// are issued eight at a time with nothing depending on them in between, the kernel is a stream over the partial buffer.
-// The index's slot bits (one word per 32 slots of a query, shared by its heads) say which slots the query has.
+// slots: each looks up the position and the statistics of every D/8-th one, and hands them on by shuffles.  The kernel is a
+// stream over the partial buffer: the rows' loads go nine at a time (selected blocks and own block are 17 slots in the
+// layers here: two rounds), the first nine beside the statistics, as soon as the positions are there.
 template <int D>
 __device__ __forceinline__ void merge_row(const SelParams& P, int bh, int i, int g, int part, float (&acc)[8], float* M_out, float* L_out) {
-  constexpr int TPR = D / 8, PER = 32 / TPR;
+  constexpr int TPR = D / 8, PER = 32 / TPR, BATCH = 9;
   const unsigned mask = (TPR == 8 ? 0xffu : 0xffffu) << (threadIdx.x & 31 & ~(TPR - 1));
   const int ns = P.ns;
-  const int64_t query = (int64_t)bh * P.N + i;
-  const uint32_t* bits = P.bits + query * P.words;
-  const int* positions = P.positions + query * ns;
+  const int* positions = P.positions + ((int64_t)bh * P.N + i) * ns;
   float M = -INFINITY, L = 0.f;
 #pragma unroll
   for (int x = 0; x < 8; ++x) acc[x] = 0.f;
   for (int s0 = 0; s0 < ns; s0 += 32) {
-    const uint32_t has = bits[s0 >> 5] >> part;
     int pos[PER];
-    float w[PER], lsum = 0.f, m = -INFINITY;
-#pragma unroll
-    for (int k = 0; k < PER; ++k) pos[k] = has >> (k * TPR) & 1u ? positions[s0 + k * TPR + part] : -1;
     float2 st[PER];
 #pragma unroll
-    for (int k = 0; k < PER; ++k) {
-      st[k] = pos[k] >= 0 ? P.stats[(int64_t)pos[k] * P.G + g] : make_float2(-INFINITY, 0.f);
-      m = fmaxf(m, st[k].x);
-    }
+    for (int k = 0; k < PER; ++k) pos[k] = s0 + k * TPR + part < ns ? positions[s0 + k * TPR + part] : -1;
 #pragma unroll
-    for (int o = TPR / 2; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(mask, m, o));
-    if (m == -INFINITY) continue;          // (the same for all threads of the row)
-    const float top = fmaxf(M, m), keep = ex2(M - top);
+    for (int k = 0; k < PER; ++k) st[k] = pos[k] >= 0 ? P.stats[(int64_t)pos[k] * P.G + g] : make_float2(-INFINITY, 0.f);
+    float w[PER];
 #pragma unroll
-    for (int k = 0; k < PER; ++k) {
-      w[k] = ex2(st[k].x - top);
-      lsum = fmaf(w[k], st[k].y, lsum);
-    }
+    for (int b0 = 0; b0 < 32; b0 += BATCH) {
+      if (s0 + b0 >= ns) break;
+      uint4 v[BATCH];
 #pragma unroll
-    for (int o = TPR / 2; o > 0; o >>= 1) lsum += __shfl_xor_sync(mask, lsum, o);
-    L = fmaf(L, keep, lsum);
-    M = top;
+      for (int u = 0; u < BATCH; ++u) {
+        const int p = b0 + u < 32 ? __shfl_sync(mask, pos[(b0 + u) % 32 / TPR], (b0 + u) % TPR, TPR) : -1;
+        v[u] = p >= 0 ? *partial_piece<D>(P.partial, (int64_t)p * P.G + g, part) : make_uint4(0u, 0u, 0u, 0u);
+      }
+      if (b0 == 0) {
+        float m = -INFINITY, lsum = 0.f;
 #pragma unroll
-    for (int x = 0; x < 8; ++x) acc[x] *= keep;
+        for (int k = 0; k < PER; ++k) m = fmaxf(m, st[k].x);
 #pragma unroll
-    for (int k = 0; k < PER; ++k) {
+        for (int o = TPR / 2; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(mask, m, o));
+        if (m == -INFINITY) break;           // none of these slots (the same for all threads of the row)
+        const float top = fmaxf(M, m), keep = ex2(M - top);
 #pragma unroll
-      for (int u0 = 0; u0 < TPR; u0 += 8) {
-        if (s0 + k * TPR + u0 >= ns) break;
-        uint4 v[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int p = __shfl_sync(mask, pos[k], u0 + u, TPR);
-          v[u] = p >= 0 ? *partial_piece<D>(P.partial, (int64_t)p * P.G + g, part) : make_uint4(0u, 0u, 0u, 0u);
+        for (int k = 0; k < PER; ++k) {
+          w[k] = ex2(st[k].x - top);
+          lsum = fmaf(w[k], st[k].y, lsum);
         }
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const float wu = __shfl_sync(mask, w[k], u0 + u, TPR);
-          const uint32_t q[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+        for (int o = TPR / 2; o > 0; o >>= 1) lsum += __shfl_xor_sync(mask, lsum, o);
+        L = fmaf(L, keep, lsum);
+        M = top;
 #pragma unroll
-          for (int x = 0; x < 4; ++x) {
-            acc[2 * x] = fmaf(wu, __uint_as_float(q[x] << 16), acc[2 * x]);
-            acc[2 * x + 1] = fmaf(wu, __uint_as_float(q[x] & 0xffff0000u), acc[2 * x + 1]);
-          }
+        for (int x = 0; x < 8; ++x) acc[x] *= keep;
+      }
+#pragma unroll
+      for (int u = 0; u < BATCH; ++u) {
+        if (b0 + u >= 32) break;
+        const float wu = __shfl_sync(mask, w[(b0 + u) % 32 / TPR], (b0 + u) % TPR, TPR);
+        const uint32_t q[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          acc[2 * x] = fmaf(wu, __uint_as_float(q[x] << 16), acc[2 * x]);
+          acc[2 * x + 1] = fmaf(wu, __uint_as_float(q[x] & 0xffff0000u), acc[2 * x + 1]);
         }
       }
     }
@@ -651,11 +649,11 @@ __device__ __forceinline__ void merge_row(const SelParams& P, int bh, int i, int
   *L_out = L;
 }
 
-// One group of D/8 threads per row; the heads of a group, whose partial rows are neighbours, next to each other.  Four
-// blocks per SM (64 registers): 17 slots of 1 M rows of 64 take 520 us = 0.73 of the copy bandwidth; left to the compiler
-// (78 registers, three blocks) 600 us, at 40 registers the loads no longer stay in flight together, 583 us.
+// One group of D/8 threads per row; the heads of a group, whose partial rows are neighbours, next to each other.  Three
+// blocks per SM (80 registers, for nine rows in flight per thread): 17 slots of 1 M rows of 64 take 495 us = 0.78 of the
+// copy bandwidth, 7 slots of 48 k rows of 128 35 us; eight rows at a time behind the statistics, four blocks: 520 and 42 us.
 template <int D>
-__global__ void __launch_bounds__(256, 4) sel_merge_kernel(const SelParams P) {
+__global__ void __launch_bounds__(256, 3) sel_merge_kernel(const SelParams P) {
   constexpr int TPR = D / 8;
   const int64_t t = ((int64_t)blockIdx.x * 256 + threadIdx.x) / TPR;
   const int part = threadIdx.x % TPR;
@@ -681,7 +679,7 @@ __global__ void __launch_bounds__(256, 4) sel_merge_kernel(const SelParams P) {
 // branch's own output tensor is written where the caller wants it.  Thread groups walk the rows position-major
 // (b, i, head), so that the heads of one position land next to each other in the destinations' [B, N, features] rows.
 template <int D, bool MC>
-__global__ void __launch_bounds__(256, 4) sel_merge_combine_kernel(const SelParams P, const CombineParams Cp, const GatherTargets Gt) {
+__global__ void __launch_bounds__(256, 3) sel_merge_combine_kernel(const SelParams P, const CombineParams Cp, const GatherTargets Gt) {
   constexpr int TPR = D / 8;
   const int64_t t = ((int64_t)blockIdx.x * 256 + threadIdx.x) / TPR;
   const int part = threadIdx.x % TPR;
@@ -1770,19 +1768,20 @@ __global__ void __launch_bounds__(256) sel_dq_merge_kernel(const SelParams P, un
   const int h = hq / P.G;
   const int ns = P.ns;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  constexpr int BYTES = ws::kDqElem<D>, BATCH = BYTES == 2 ? 8 : 4, QUADS = BYTES / 2;
+  // Rows in flight: nine of 64 (17 slots in two rounds; 4 x 8192 positions, 32 heads 437 -> 395 us, eight before), but eight in the
+  // sliding branch (10 slots: 144 us, with nine 150, with ten 161), four of 128 in fp32 (44 us, with six 48)
+  constexpr int BYTES = ws::kDqElem<D>, BATCH = BYTES == 4 ? 4 : MODE == kModeSwa ? 8 : 9, QUADS = BYTES / 2;
   const uint8_t* prow = reinterpret_cast<const uint8_t*>(P.partial) + (part_row * ns * D + part * 8) * BYTES;
   // some slots at a time: first which of them the query has, then their loads together, then the sums
   const uint32_t* bits = P.bits + ((int64_t)(b * P.Hkv + h) * P.N + i) * P.words;
   for (int s0 = 0; s0 < ns; s0 += BATCH) {
-    const uint32_t has = MODE == kModeSel ? bits[s0 >> 5] >> (s0 & 31) : 0u;
     bool ok[BATCH];
     uint4 v[BATCH][QUADS];
 #pragma unroll
     for (int u = 0; u < BATCH; ++u) {
       int blk_;
-      ok[u] = MODE == kModeSel ? (has >> u & 1u) != 0
-                               : s0 + u < ns && slot_block<MODE>(P.rule, b * P.Hkv + h, i, s0 + u, &blk_);
+      ok[u] = s0 + u < ns && (MODE == kModeSel ? (bits[(s0 + u) >> 5] >> ((s0 + u) & 31) & 1u) != 0
+                                               : slot_block<MODE>(P.rule, b * P.Hkv + h, i, s0 + u, &blk_));
     }
 #pragma unroll
     for (int u = 0; u < BATCH; ++u)
