@@ -493,7 +493,7 @@ static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor>
     return kept.narrow(0, off, n * (int64_t)c10::elementSize(t)).view(t).view(sizes);
   };
 
-  // fp32 accumulators, cleared together: dk, dv; dck, dcv; (counters); then the small gradients that end up in the layer's type.  An
+  // fp32 accumulators, cleared together (beside the combine's backward): dk, dv; dck, dcv; (counters); then the small gradients that end up in the layer's type.  An
   // fp32 layer returns the small ones as they are: there they have memory of their own, a gradient that a program keeps
   // must not keep the scratch of dk and dv with it.
   const int64_t pos = hkv * c.cbs * d, mems = hkv * c.num_mem * d, hid = w.k1.size(0);
@@ -507,8 +507,6 @@ static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor>
   float* const dk = ptr<float>(acc);
   float* const dck = dk + 2 * k_elems;
   float* const small = apart ? ptr<float>(rounded) : dk + a_small;
-  if (cudaMemsetAsync(dk, 0, acc.numel() * 4, st) != cudaSuccess || (apart && cudaMemsetAsync(small, 0, s_end * 4, st) != cudaSuccess))
-    throw Error("clearing the gradient accumulators failed");
 
   // output projection and gated combine
   dout = dout.reshape({BN, L.dim}).contiguous();
@@ -538,6 +536,8 @@ static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor>
     for (int s = 0; s < 3; ++s) p.d_o[s] = d_outs[s].data_ptr();
     p.delta = reinterpret_cast<float*>(tmp.at(t_delta));
     p.d_logits = d_logits.data_ptr();
+    p.clear[0] = dk; p.clear_pieces[0] = acc.numel() / 4;
+    if (apart) { p.clear[1] = small; p.clear_pieces[1] = s_end / 4; }
     check(nsa::launch_combine(p, L.dt, true, st));
     d_merged = Tensor();
   }
@@ -654,16 +654,18 @@ static std::vector<OptTensor> layer_backward(Tensor dout, std::vector<OptTensor>
     p.run(st);
   }
   dhk = dhv = Tensor();
-  check(nsa::launch_pos_grad(L.shape, dkw.data_ptr(), dvw.data_ptr(), small + s_pos, L.dt, st));
 
   // qkv, gates, norm
   const Tensor d_qkv = at::empty({BN, L.F}, x.options());
   qg.dk = dk; qg.dv = dk + k_elems; qg.dkw = dkw.data_ptr(); qg.dvw = dvw.data_ptr(); qg.inv_freq = ptr<float>(inv_freq); qg.out = d_qkv.data_ptr();
-  check(nsa::launch_qkv_grad(L.shape, qg, L.dt, st));
+  {
+    nsa::GateSums sums = {};
+    sums.x = d_logits.data_ptr(); sums.out = small + s_gate; sums.rows = BN; sums.cols = (int)(3 * H);
+    sums.partial = reinterpret_cast<float*>(tmp.at(t_gates)); sums.arrived = reinterpret_cast<unsigned*>(dk + a_counters);
+    check(nsa::launch_layer_tail(L.shape, qg, sums, small + s_pos, L.dt, st));
+  }
   for (Tensor& t : dqs) t = Tensor();
   dkw = dvw = Tensor();
-  check(nsa::launch_gate_sums(d_logits.data_ptr(), small + s_gate, BN, (int)(3 * H), reinterpret_cast<float*>(tmp.at(t_gates)),
-                              reinterpret_cast<unsigned*>(dk + a_counters), L.dt, st));
   Tensor dxn;
   {
     Products p(type, L.status);

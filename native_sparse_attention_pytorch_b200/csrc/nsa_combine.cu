@@ -131,10 +131,19 @@ __global__ void __launch_bounds__(128) combine_bwd_kernel(const CombineParams P)
   }
 }
 
-// The same with 16-byte accesses: TPR threads share a (batch, head, position) row, 32 / TPR rows per warp.
+// The same with 16-byte accesses: TPR threads share a (batch, head, position) row, 32 / TPR rows per warp.  The blocks behind
+// those of the rows clear what the caller wants cleared before its next launches.
 template <typename T, int TPR>
-__global__ void __launch_bounds__(256) combine_bwd_vec_kernel(const CombineParams P) {
+__global__ void __launch_bounds__(256) combine_bwd_vec_kernel(const CombineParams P, unsigned row_blocks) {
   constexpr int V = 16 / (int)sizeof(T);
+  if (blockIdx.x >= row_blocks) {
+    const int64_t step = (int64_t)(gridDim.x - row_blocks) * 256;
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      for (int64_t e = (int64_t)(blockIdx.x - row_blocks) * 256 + threadIdx.x; e < P.clear_pieces[k]; e += step)
+        reinterpret_cast<float4*>(P.clear[k])[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+    return;
+  }
   const int64_t tasks = (int64_t)P.batch * P.q_heads * P.seq;
   const int64_t task = ((int64_t)blockIdx.x * 256 + threadIdx.x) / TPR;
   const int part = threadIdx.x % TPR;
@@ -195,14 +204,16 @@ static bool launch_combine_bwd_vec(const CombineParams& P, cudaStream_t stream) 
   const int tpr = P.d / V;
   const int64_t threads = (int64_t)P.batch * P.q_heads * P.seq * tpr;
   const int64_t blocks = (threads + 255) / 256;
-  if (blocks > 0x7fffffffLL) return false;
-  const unsigned grid = (unsigned)blocks;
+  const int64_t pieces = P.clear_pieces[0] > P.clear_pieces[1] ? P.clear_pieces[0] : P.clear_pieces[1];
+  const int64_t clearing = (pieces + 255) / 256 < 148 * 4 ? (pieces + 255) / 256 : 148 * 4;
+  if (blocks + clearing > 0x7fffffffLL) return false;
+  const unsigned rows = (unsigned)blocks, grid = (unsigned)(blocks + clearing);
   switch (tpr) {
-    case 2: combine_bwd_vec_kernel<T, 2><<<grid, 256, 0, stream>>>(P); return true;
-    case 4: combine_bwd_vec_kernel<T, 4><<<grid, 256, 0, stream>>>(P); return true;
-    case 8: combine_bwd_vec_kernel<T, 8><<<grid, 256, 0, stream>>>(P); return true;
-    case 16: combine_bwd_vec_kernel<T, 16><<<grid, 256, 0, stream>>>(P); return true;
-    case 32: combine_bwd_vec_kernel<T, 32><<<grid, 256, 0, stream>>>(P); return true;
+    case 2: combine_bwd_vec_kernel<T, 2><<<grid, 256, 0, stream>>>(P, rows); return true;
+    case 4: combine_bwd_vec_kernel<T, 4><<<grid, 256, 0, stream>>>(P, rows); return true;
+    case 8: combine_bwd_vec_kernel<T, 8><<<grid, 256, 0, stream>>>(P, rows); return true;
+    case 16: combine_bwd_vec_kernel<T, 16><<<grid, 256, 0, stream>>>(P, rows); return true;
+    case 32: combine_bwd_vec_kernel<T, 32><<<grid, 256, 0, stream>>>(P, rows); return true;
     default: return false;
   }
 }
@@ -219,6 +230,9 @@ int launch_combine(const CombineParams& P, int dtype, bool backward, cudaStream_
   } else if (dtype == NSA_F32 ? launch_combine_bwd_vec<float>(P, stream) : launch_combine_bwd_vec<__nv_bfloat16>(P, stream)) {
     // 16-byte accesses served it
   } else {
+    for (int k = 0; k < 2; ++k)
+      if (P.clear_pieces[k] > 0 && cudaMemsetAsync(P.clear[k], 0, (size_t)P.clear_pieces[k] * 16, stream) != cudaSuccess)
+        return fail((int)cudaGetLastError(), "clearing the gradient accumulators failed");
     const int64_t blocks = (rows + 3) / 4;
     if (blocks > 0x7fffffffLL) return fail(NSA_ERR_SHAPE, "too many rows for one launch");
     if (dtype == NSA_F32) combine_bwd_kernel<float><<<(unsigned)blocks, 128, 0, stream>>>(P);

@@ -63,6 +63,8 @@ struct CombineParams {
   void* d_logits;          // backward, with `logits`: [batch, seq, 3 q_heads] in the tensors' type, instead of d_gates
   int logits;              // `gates` holds logits: the gate is their sigmoid, rounded as a tensor of it would be
   int batch, q_heads, seq, d;
+  float* clear[2];         // backward, optional: fp32 buffers of `clear_pieces` sixteen-byte pieces to zero in the same launch
+  int64_t clear_pieces[2];
 };
 
 constexpr int kMaxGather = NSA_MAX_GATHER;
@@ -178,6 +180,16 @@ struct QkvGrad {
   void* out;                         // [B, N, (Hq + 2 Hkv) d]
 };
 
+// Column sums of the gates' gradient (see nsa_layer.cu)
+struct GateSums {
+  const void* x;                     // [rows, cols]
+  float* out;
+  int64_t rows;
+  int cols;
+  float* partial;                    // gate_sums_partial(cols) floats
+  unsigned* arrived;                 // gate_sums_counters(cols), zero
+};
+
 // Gradient through the differentiable top-k (see nsa_topk_grad.cu)
 struct TopkGrad {
   const float* importance;           // [B, Hs, N, ncb], as the forward left it
@@ -231,9 +243,7 @@ int launch_split_mem(const LayerShape& L, const float* grad, void* dc, float* dm
 int launch_relu_sums(const ColumnSums& P, int dtype, cudaStream_t stream);
 int64_t gate_sums_partial(int cols);    // floats
 int gate_sums_counters(int cols);       // zero before the call
-int launch_gate_sums(const void* x, float* out, int64_t rows, int cols, float* partial, unsigned* arrived, int dtype, cudaStream_t stream);
-int launch_qkv_grad(const LayerShape& L, const QkvGrad& P, int dtype, cudaStream_t stream);
-int launch_pos_grad(const LayerShape& L, const void* dkw, const void* dvw, float* dpos, int dtype, cudaStream_t stream);
+int launch_layer_tail(const LayerShape& L, const QkvGrad& P, const GateSums& S, float* dpos, int dtype, cudaStream_t stream);
 bool gemm_serves(const GemmGroup& G, int dtype);   // fp32: sums of up to 35840 products (70 steps of 64 on each of 8 CTAs)
 int launch_gemm(GemmGroup& G, int dtype, cudaStream_t stream);
 int launch_topk_grad(const TopkGrad& P, int dtype, cudaStream_t stream);

@@ -196,7 +196,7 @@ int launch_split_mem(const LayerShape& L, const float* grad, void* dc, float* dm
 
 // ---- column sums (the bias of the first compress layer) behind the ReLU whose output is `act`: x = act > 0 ? x : 0 in
 // place.  A block owns 32 sixteen-byte columns and a slice of the rows; sets side by side in blockIdx.z.  The slices meet in
-// float atomics, as those of split_mem_kernel and pos_grad_kernel do: the last bits of these sums differ from run to run,
+// float atomics, as those of split_mem_kernel and pos_grad do: the last bits of these sums differ from run to run,
 // like those of dk and dv behind them (fp32 reductions of the attention kernels).
 template <typename T>
 __global__ void __launch_bounds__(256) relu_sums_kernel(const ColumnSums P) {
@@ -260,18 +260,22 @@ int launch_relu_sums(const ColumnSums& P, int dtype, cudaStream_t stream) {
 // `arrived`: one counter per 256 columns, zero.
 constexpr int kGateSlices = 64;
 template <typename T, int VEC>
-__global__ void __launch_bounds__(256) gate_sums_kernel(const T* x, float* out, int64_t rows, int cols, float* partial, unsigned* arrived) {
+__device__ __forceinline__ void gate_sums(const GateSums& P, int group, int slice, int slices) {
   __shared__ float fold[256 * VEC];
   __shared__ bool last;
-  const int c0 = blockIdx.x * 256, width = min(256, cols - c0), units = width / VEC;
+  const T* x = (const T*)P.x;
+  float *out = P.out, *partial = P.partial;
+  const int64_t rows = P.rows;
+  const int cols = P.cols;
+  const int c0 = group * 256, width = min(256, cols - c0), units = width / VEC;
   const int tid = threadIdx.x, u = tid % units, r0 = tid / units, step = 256 / units;
   float sum[VEC];
 #pragma unroll
   for (int i = 0; i < VEC; ++i) sum[i] = 0.f;
   if (r0 < step) {
-    const int64_t per = (rows + gridDim.y - 1) / gridDim.y, end = min(rows, (blockIdx.y + 1) * per);
+    const int64_t per = (rows + slices - 1) / slices, end = min(rows, (slice + 1) * per);
 #pragma unroll 4
-    for (int64_t r = blockIdx.y * per + r0; r < end; r += step) {
+    for (int64_t r = slice * per + r0; r < end; r += step) {
       const T* at = x + r * cols + c0 + u * VEC;
       if constexpr (VEC == 1) {
         sum[0] += Elem<T>::to_float(*at);
@@ -289,11 +293,11 @@ __global__ void __launch_bounds__(256) gate_sums_kernel(const T* x, float* out, 
   if (tid < width) {
     float s = 0.f;
     for (int k = 0; k < step; ++k) s += fold[k * width + tid];
-    partial[(int64_t)blockIdx.y * cols + c0 + tid] = s;
+    partial[(int64_t)slice * cols + c0 + tid] = s;
   }
   __threadfence();
   __syncthreads();
-  if (tid == 0) last = atomicAdd(arrived + blockIdx.x, 1u) == gridDim.y - 1;
+  if (tid == 0) last = atomicAdd(P.arrived + group, 1u) == slices - 1;
   __syncthreads();
   if (!last) return;
   __threadfence();
@@ -301,7 +305,7 @@ __global__ void __launch_bounds__(256) gate_sums_kernel(const T* x, float* out, 
   float s = 0.f;
   if (g < groups) {
 #pragma unroll 8
-    for (int y = g; y < (int)gridDim.y; y += groups) s += __ldcg(partial + (int64_t)y * cols + c0 + c);
+    for (int y = g; y < (int)slices; y += groups) s += __ldcg(partial + (int64_t)y * cols + c0 + c);
     fold[g * width + c] = s;
   }
   __syncthreads();
@@ -315,35 +319,17 @@ __global__ void __launch_bounds__(256) gate_sums_kernel(const T* x, float* out, 
 int64_t gate_sums_partial(int cols) { return (int64_t)kGateSlices * cols; }
 int gate_sums_counters(int cols) { return (cols + 255) / 256; }
 
-int launch_gate_sums(const void* x, float* out, int64_t rows, int cols, float* partial, unsigned* arrived, int dtype, cudaStream_t stream) {
-  if (rows == 0 || cols == 0) return NSA_OK;
-  const int V = dtype == NSA_F32 ? 4 : 8;
-  const int64_t slices = (rows * cols + 2047) / 2048;
-  const dim3 grid((unsigned)gate_sums_counters(cols), (unsigned)(slices < kGateSlices ? slices : kGateSlices));
-  const bool vec = cols % V == 0 && aligned16(x);
-  if (dtype == NSA_F32) {
-    if (vec) gate_sums_kernel<float, 4><<<grid, 256, 0, stream>>>((const float*)x, out, rows, cols, partial, arrived);
-    else gate_sums_kernel<float, 1><<<grid, 256, 0, stream>>>((const float*)x, out, rows, cols, partial, arrived);
-  } else {
-    if (vec) gate_sums_kernel<__nv_bfloat16, 8><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)x, out, rows, cols, partial, arrived);
-    else gate_sums_kernel<__nv_bfloat16, 1><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)x, out, rows, cols, partial, arrived);
-  }
-  count_launches(1);
-  const cudaError_t err = cudaGetLastError();
-  return err == cudaSuccess ? NSA_OK : fail((int)err, cudaGetErrorString(err));
-}
-
 // ---- gradient of the qkv projection's output, [B, N, (Hq + 2 Hkv) d]: per query head the gradient of the un-rotated
 // query (compressed branch) plus the two rotated ones turned back; per key head the rotated key's gradient turned back
 // plus what arrives through the windows that hold the token; per value head the same without the rotation.  Sums in
 // fp32, one rounding.
 template <typename T>
-__global__ void __launch_bounds__(256) qkv_grad_kernel(const LayerShape L, const QkvGrad P) {
+__device__ __forceinline__ void qkv_grad(const LayerShape& L, const QkvGrad& P, int block) {
   constexpr int V = Vec<T>::V;
   extern __shared__ float angles[];
   const int vpr = L.d / V, F = (L.heads + 2 * L.kv_heads) * L.d;
   const int tiles = (L.seq + kTileN - 1) / kTileN;
-  const int b = blockIdx.x / tiles, n0 = (blockIdx.x - b * tiles) * kTileN;
+  const int b = block / tiles, n0 = (block - b * tiles) * kTileN;
   float *co = angles, *si = angles + kTileN * (L.d / 2);
   fill_angles(L, P.inv_freq, n0, co, si);
   __syncthreads();
@@ -380,49 +366,74 @@ __global__ void __launch_bounds__(256) qkv_grad_kernel(const LayerShape L, const
   }
 }
 
-int launch_qkv_grad(const LayerShape& L, const QkvGrad& P, int dtype, cudaStream_t stream) {
-  const int64_t grid = (int64_t)L.batch * ((L.seq + kTileN - 1) / kTileN);
-  if (grid == 0) return NSA_OK;
-  if (grid > 0x7fffffff) return fail(NSA_ERR_SHAPE, "layer: too many positions for one launch");
-  const size_t smem = (size_t)kTileN * L.d * sizeof(float);
-  if (dtype == NSA_F32) qkv_grad_kernel<float><<<(unsigned)grid, 256, smem, stream>>>(L, P);
-  else qkv_grad_kernel<__nv_bfloat16><<<(unsigned)grid, 256, smem, stream>>>(L, P);
-  count_launches(1);
-  const cudaError_t err = cudaGetLastError();
-  return err == cudaSuccess ? NSA_OK : fail((int)err, cudaGetErrorString(err));
-}
-
 // ---- gradients of the intra-block positions: sums over batch and windows of the window gradients, keys and values side
 // by side (blockIdx.z); a thread owns a 16-byte piece of the window and a slice of the (batch, window) pairs
 template <typename T>
-__global__ void __launch_bounds__(128) pos_grad_kernel(const LayerShape L, const T* dkw, const T* dvw, float* dpos, int slot_groups) {
+__device__ __forceinline__ void pos_grad(const LayerShape& L, const T* dkw, const T* dvw, float* dpos, int group, int slot_groups, int slice, int slices,
+                                         int val) {
   constexpr int V = Vec<T>::V;
   const int slots = L.cbs * L.d / V;
-  const int h = blockIdx.x / slot_groups, slot = (blockIdx.x % slot_groups) * 128 + threadIdx.x;
+  const int h = group / slot_groups, slot = (group % slot_groups) * 256 + threadIdx.x;
   if (slot >= slots) return;
   const int64_t pairs = (int64_t)L.batch * L.ncb, window = (int64_t)slots * V;
-  const int64_t per = (pairs + gridDim.y - 1) / gridDim.y, k0 = blockIdx.y * per, k1 = k0 + per < pairs ? k0 + per : pairs;
-  const T* base = (blockIdx.z ? dvw : dkw) + (int64_t)slot * V;
+  const int64_t per = (pairs + slices - 1) / slices, k0 = slice * per, k1 = k0 + per < pairs ? k0 + per : pairs;
+  const T* base = (val ? dvw : dkw) + (int64_t)slot * V;
   Vec<T> sum;
   sum.zero();
 #pragma unroll 4
   for (int64_t k = k0; k < k1; ++k) sum.add(base + (((k / L.ncb) * L.kv_heads + h) * L.ncb + k % L.ncb) * window);
-  float* dst = dpos + ((int64_t)blockIdx.z * L.kv_heads + h) * window + (int64_t)slot * V;
+  float* dst = dpos + ((int64_t)val * L.kv_heads + h) * window + (int64_t)slot * V;
 #pragma unroll
   for (int i = 0; i < V; ++i) atomicAdd(dst + i, sum.x[i]);
 }
 
-int launch_pos_grad(const LayerShape& L, const void* dkw, const void* dvw, float* dpos, int dtype, cudaStream_t stream) {
+// The three passes behind the window gradients, which do not depend on one another, in one launch: first the blocks of
+// qkv_grad, then those of the positions, then those of the gates.
+struct TailGrid {
+  int qkv, pos_groups, slot_groups, pos_slices, gate_groups, gate_slices;
+};
+template <typename T, int VEC>
+__global__ void __launch_bounds__(256, 5) layer_tail_kernel(const LayerShape L, const QkvGrad P, const GateSums S, float* dpos, const TailGrid g) {
+  int block = blockIdx.x;
+  if (block < g.qkv) {
+    qkv_grad<T>(L, P, block);
+    return;
+  }
+  block -= g.qkv;
+  if (block < 2 * g.pos_groups * g.pos_slices) {
+    const int group = block % g.pos_groups, rest = block / g.pos_groups;
+    pos_grad<T>(L, (const T*)P.dkw, (const T*)P.dvw, dpos, group, g.slot_groups, rest % g.pos_slices, g.pos_slices, rest / g.pos_slices);
+    return;
+  }
+  block -= 2 * g.pos_groups * g.pos_slices;
+  gate_sums<T, VEC>(S, block % g.gate_groups, block / g.gate_groups, g.gate_slices);
+}
+
+int launch_layer_tail(const LayerShape& L, const QkvGrad& P, const GateSums& S, float* dpos, int dtype, cudaStream_t stream) {
   const int V = dtype == NSA_F32 ? 4 : 8;
-  const int64_t pairs = (int64_t)L.batch * L.ncb;
-  if (pairs == 0) return NSA_OK;
-  const int slot_groups = (L.cbs * L.d / V + 127) / 128;
-  const int64_t ctas = (int64_t)L.kv_heads * slot_groups * 2;
-  int64_t slices = (148 * 4 + ctas - 1) / ctas;                   // about four blocks per SM: every slice ends in atomics
+  const int64_t qkv = (int64_t)L.batch * ((L.seq + kTileN - 1) / kTileN), pairs = (int64_t)L.batch * L.ncb;
+  TailGrid g = {};
+  g.slot_groups = (L.cbs * L.d / V + 255) / 256;
+  g.pos_groups = L.kv_heads * g.slot_groups;
+  int64_t slices = (148 * 2 + 2 * (int64_t)g.pos_groups - 1) / (2 * (int64_t)g.pos_groups);   // about two blocks per SM: every slice ends in atomics
   slices = slices < (pairs + 7) / 8 ? slices : (pairs + 7) / 8;
-  const dim3 grid((unsigned)(L.kv_heads * slot_groups), (unsigned)slices, 2);
-  if (dtype == NSA_F32) pos_grad_kernel<float><<<grid, 128, 0, stream>>>(L, (const float*)dkw, (const float*)dvw, dpos, slot_groups);
-  else pos_grad_kernel<__nv_bfloat16><<<grid, 128, 0, stream>>>(L, (const __nv_bfloat16*)dkw, (const __nv_bfloat16*)dvw, dpos, slot_groups);
+  g.pos_slices = pairs > 0 ? (int)slices : 0;
+  const int64_t parts = (S.rows * S.cols + 2047) / 2048;
+  g.gate_groups = gate_sums_counters(S.cols);
+  g.gate_slices = S.rows > 0 && S.cols > 0 ? (int)(parts < kGateSlices ? parts : kGateSlices) : 0;
+  const int64_t grid = qkv + 2 * (int64_t)g.pos_groups * g.pos_slices + (int64_t)g.gate_groups * g.gate_slices;
+  if (grid == 0) return NSA_OK;
+  if (grid > 0x7fffffff) return fail(NSA_ERR_SHAPE, "layer: too many positions for one launch");
+  g.qkv = (int)qkv;
+  const size_t smem = (size_t)kTileN * L.d * sizeof(float);
+  const bool vec = S.cols % V == 0 && aligned16(S.x);
+  if (dtype == NSA_F32) {
+    if (vec) layer_tail_kernel<float, 4><<<(unsigned)grid, 256, smem, stream>>>(L, P, S, dpos, g);
+    else layer_tail_kernel<float, 1><<<(unsigned)grid, 256, smem, stream>>>(L, P, S, dpos, g);
+  } else {
+    if (vec) layer_tail_kernel<__nv_bfloat16, 8><<<(unsigned)grid, 256, smem, stream>>>(L, P, S, dpos, g);
+    else layer_tail_kernel<__nv_bfloat16, 1><<<(unsigned)grid, 256, smem, stream>>>(L, P, S, dpos, g);
+  }
   count_launches(1);
   const cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? NSA_OK : fail((int)err, cudaGetErrorString(err));
