@@ -347,6 +347,18 @@ __device__ __forceinline__ uint4 lds_v4(uint32_t addr) {
   return v;
 }
 
+// A piece that is read once, zeros where `ok` is false: nothing is fetched then and nothing branches, so that several which stand
+// together are issued together.
+__device__ __forceinline__ uint4 ldg_stream_if(bool ok, const void* p) {
+  uint4 v;
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\t"
+      "mov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
+      "@q ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
+      : "=&r"(v.x), "=&r"(v.y), "=&r"(v.z), "=&r"(v.w) : "l"(p), "r"((uint32_t)ok));
+  return v;
+}
+
 // Bulk (TMA) copy from this CTA's shared memory to global memory; size is a multiple of 16 bytes and both addresses are
 // 16-byte aligned.  Whoever wrote the shared memory must have run fence_proxy_async_smem() first.
 __device__ __forceinline__ void bulk_store(void* gdst, uint32_t ssrc, uint32_t bytes) {

@@ -696,10 +696,11 @@ __device__ __forceinline__ void merge_row(const SelParams& P, int bh, int i, int
 template <int D>
 __global__ void __launch_bounds__(256, 3) sel_merge_kernel(const SelParams P) {
   constexpr int TPR = D / 8;
-  const int64_t t = ((int64_t)blockIdx.x * 256 + threadIdx.x) / TPR;
+  const uint32_t t = blockIdx.x * (256 / TPR) + threadIdx.x / TPR;     // 32 bits hold every row id (see `supported`)
   const int part = threadIdx.x % TPR;
-  if (t >= (int64_t)P.B * P.Hq * P.N || foreign_index(P)) return;
-  const int g = (int)(t % P.G), i = (int)((t / P.G) % P.N), bh = (int)(t / ((int64_t)P.G * P.N));
+  if (t >= (uint32_t)P.B * P.Hq * P.N || foreign_index(P)) return;
+  const uint32_t g_shift = 31 - __clz(P.G), query = t >> g_shift;
+  const int g = (int)(t & (P.G - 1)), bh = (int)(query / (uint32_t)P.N), i = (int)query - bh * P.N;
   const int b = bh / P.Hkv, hq = (bh - b * P.Hkv) * P.G + g;
   float acc[8], M, L;
   merge_row<D>(P, bh, i, g, part, acc, &M, &L);
@@ -722,16 +723,14 @@ __global__ void __launch_bounds__(256, 3) sel_merge_kernel(const SelParams P) {
 template <int D, bool MC>
 __global__ void __launch_bounds__(256, 3) sel_merge_combine_kernel(const SelParams P, const CombineParams Cp, const GatherTargets Gt) {
   constexpr int TPR = D / 8;
-  const int64_t t = ((int64_t)blockIdx.x * 256 + threadIdx.x) / TPR;
+  const uint32_t t = blockIdx.x * (256 / TPR) + threadIdx.x / TPR;     // 32 bits hold every row id (see `supported`)
   const int part = threadIdx.x % TPR;
-  const int64_t nrows = (int64_t)P.B * P.Hq * P.N;
-  if (t < nrows && !foreign_index(P)) {
-    const int hq = (int)(t % P.Hq);
-    const int i = (int)((t / P.Hq) % P.N);
-    const int b = (int)(t / ((int64_t)P.N * P.Hq));
+  if (t < (uint32_t)P.B * P.Hq * P.N && !foreign_index(P)) {
+    const uint32_t token = t / (uint32_t)P.Hq;
+    const int hq = (int)(t - token * P.Hq), b = (int)(token / (uint32_t)P.N), i = (int)token - b * P.N, g_shift = 31 - __clz(P.G);
     const int64_t row = ((int64_t)b * P.Hq + hq) * P.N + i;
     float acc[8], M, Lsum;
-    merge_row<D>(P, b * P.Hkv + hq / P.G, i, hq % P.G, part, acc, &M, &Lsum);
+    merge_row<D>(P, b * P.Hkv + (hq >> g_shift), i, hq & (P.G - 1), part, acc, &M, &Lsum);
     const float inv = Lsum > 0.f ? 1.f / Lsum : 0.f;
     if (part == 0 && P.lse != nullptr) P.lse[row] = Lsum > 0.f ? (M + log2f(Lsum)) * kLn2 : -INFINITY;
     // combine: gates in the order compressed, selected, sliding
@@ -831,12 +830,14 @@ template <int G>
 __device__ __forceinline__ uint32_t imp_offset(int r, int c) {
   return (uint32_t)((r * 64) ^ (((r / G) & 1) << 6)) + ((uint32_t)(c ^ ((r >> 1) & 3)) << 4);
 }
-// The sum of G values in the order of a butterfly over neighbouring lanes
+// The sums of G pairs of values, each in the order of a butterfly over neighbouring lanes
 template <int G>
-__device__ __forceinline__ float tree_sum(const float* a) {
+__device__ __forceinline__ uint64_t tree_sum(const uint64_t* a) {
   if constexpr (G == 1) return a[0];
-  else return tree_sum<G / 2>(a) + tree_sum<G / 2>(a + G / 2);
+  else return add2(tree_sum<G / 2>(a), tree_sum<G / 2>(a + G / 2));
 }
+// A word of two bf16 as two fp32 values
+__device__ __forceinline__ uint64_t widen2(uint32_t w) { return pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
 }  // namespace dense
 
 template <int D, int MODE, int GI, bool POOL = false>   // GI: 0 = no importance output, else the heads per KV head
@@ -955,13 +956,16 @@ dense_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           constexpr int OWN = 32 / (IMP ? GI : 1);
           constexpr float inv_g = 1.f / (float)(IMP ? GI : 1);
           float mean[OWN];
+          const uint64_t logit_scale = pack2(P.scale, P.scale);
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
             uint32_t w[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               const uint32_t r = pack_bf16(x0[c * 8 + 2 * k], x0[c * 8 + 2 * k + 1]);   // (one value at a time would convert at a quarter of the rate)
-              w[k] = pack_bf16(__uint_as_float(r << 16) * P.scale, __uint_as_float(r & 0xffff0000u) * P.scale);
+              float a, b2;
+              unpack2(mul2(widen2(r), logit_scale), a, b2);
+              w[k] = pack_bf16(a, b2);
             }
             if constexpr (GI == 1) {
 #pragma unroll
@@ -995,11 +999,11 @@ dense_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 }
               }
 #pragma unroll
-              for (int c = 0; c < PIECE; ++c) {
-                float a[GI];
+              for (int c = 0; c < PIECE / 2; ++c) {
+                uint64_t a[GI];
 #pragma unroll
-                for (int k = 0; k < GI; ++k) a[k] = __uint_as_float(c & 1 ? w[k][c / 2] & 0xffff0000u : w[k][c / 2] << 16);
-                mean[p * PIECE + c] = tree_sum<GI>(a);
+                for (int k = 0; k < GI; ++k) a[k] = widen2(w[k][c]);
+                unpack2(tree_sum<GI>(a), mean[p * PIECE + 2 * c], mean[p * PIECE + 2 * c + 1]);
               }
             }
           }
@@ -1232,14 +1236,12 @@ __global__ void __launch_bounds__(256) sel_delta_kernel(const SelParams P, float
       reinterpret_cast<float4*>(P.dk)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
     return;
   }
-  const int64_t row = ((int64_t)blockIdx.x * 256 + threadIdx.x) / TPR;
+  const uint32_t row = blockIdx.x * (256 / TPR) + threadIdx.x / TPR, nrows = (uint32_t)P.B * P.Hq * P.N;   // (see `supported`)
   const int part = threadIdx.x % TPR;
-  const int64_t nrows = (int64_t)P.B * P.Hq * P.N;
   float acc = 0.f;
   if (row < nrows) {
-    const int i = (int)(row % P.N);
-    const int hq = (int)((row / P.N) % P.Hq);
-    const int b = (int)(row / ((int64_t)P.N * P.Hq));
+    const uint32_t head = row / (uint32_t)P.N;
+    const int i = (int)(row - head * P.N), b = (int)(head / (uint32_t)P.Hq), hq = (int)head - b * P.Hq;
     const uint4 o = *reinterpret_cast<const uint4*>(P.out + b * P.o_sb + (int64_t)hq * P.o_sh + (int64_t)i * P.o_sn + part * 8);
     const uint4 g = *reinterpret_cast<const uint4*>(P.dout + b * P.do_sb + (int64_t)hq * P.do_sh + (int64_t)i * P.do_sn + part * 8);
     const uint32_t ou[4] = {o.x, o.y, o.z, o.w}, gu[4] = {g.x, g.y, g.z, g.w};
@@ -1788,7 +1790,7 @@ sel_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 // sums the dQ partials of every (batch, query head, query) into the fp32 dq row: D/8 threads per row.  The blocks behind
 // those of the rows round dk and dv, which the kernel before has completed, to bf16 (`round` pieces of 8 from P.dk on).
 template <int D, int MODE>
-__global__ void __launch_bounds__(256) sel_dq_merge_kernel(const SelParams P, unsigned row_blocks, int64_t round) {
+__global__ void __launch_bounds__(256, 6) sel_dq_merge_kernel(const SelParams P, unsigned row_blocks, int64_t round) {
   constexpr int TPR = D / 8;
   if (blockIdx.x >= row_blocks) {
     const int64_t step = (int64_t)(gridDim.x - row_blocks) * 256;
@@ -1798,37 +1800,40 @@ __global__ void __launch_bounds__(256) sel_dq_merge_kernel(const SelParams P, un
     }
     return;
   }
-  const int64_t part_row = ((int64_t)blockIdx.x * 256 + threadIdx.x) / TPR;   // row of the slice
+  const uint32_t slice_row = blockIdx.x * (256 / TPR) + threadIdx.x / TPR;   // 32 bits hold every row id (see `supported`)
   const int part = threadIdx.x % TPR;
-  const int64_t first = (int64_t)P.bh0 * P.G * P.N, nrows = (int64_t)(P.bh1 - P.bh0) * P.G * P.N;
-  if (part_row >= nrows) return;
-  const int64_t row = first + part_row;
-  const int i = (int)(row % P.N);
-  const int hq = (int)((row / P.N) % P.Hq);
-  const int b = (int)(row / ((int64_t)P.N * P.Hq));
-  const int h = hq / P.G;
+  if (slice_row >= (uint32_t)(P.bh1 - P.bh0) * P.G * P.N) return;
+  const uint32_t row = (uint32_t)P.bh0 * P.G * P.N + slice_row, head = row / (uint32_t)P.N;
+  const int i = (int)(row - head * P.N), b = (int)(head / (uint32_t)P.Hq), hq = (int)head - b * P.Hq;
+  const int h = hq >> (31 - __clz(P.G));
+  const int64_t part_row = slice_row;
   const int ns = P.ns;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  // Rows in flight: nine of 64 (17 slots in two rounds; 4 x 8192 positions, 32 heads 437 -> 395 us, eight before), but eight in the
-  // sliding branch (10 slots: 144 us, with nine 150, with ten 161), four of 128 in fp32 (44 us, with six 48)
+  // Rows in flight: nine of 64 (17 slots in two rounds), but eight in the sliding branch (10 slots: with nine 4 % slower, with ten
+  // 12 %), four of 128 in fp32 (with six 9 % slower).  Bound by the partials' bytes: 4 x 8192 positions, 32 heads 437 -> 360 us
+  // (97 % of the copy bandwidth), 2 x 1536 x 8 heads of 128 45 -> 32 us.  The bound of six blocks an SM is what keeps the loads of a
+  // batch together: without one the compiler stops at 32 registers and fetches them in turns (445 us; with four blocks 356 us, but
+  // the sliding branch 125 us instead of 118 us and the compressed one 163 us instead of 148 us).
   constexpr int BYTES = ws::kDqElem<D>, BATCH = BYTES == 4 ? 4 : MODE == kModeSwa ? 8 : 9, QUADS = BYTES / 2;
   const uint8_t* prow = reinterpret_cast<const uint8_t*>(P.partial) + (part_row * ns * D + part * 8) * BYTES;
   // some slots at a time: first which of them the query has, then their loads together, then the sums
   const uint32_t* bits = P.bits + ((int64_t)(b * P.Hkv + h) * P.N + i) * P.words;
   for (int s0 = 0; s0 < ns; s0 += BATCH) {
+    const int word = s0 >> 5;              // (bits behind the last slot are zero)
+    const uint32_t has = MODE == kModeSel ? __funnelshift_r(bits[word], word + 1 < P.words ? bits[word + 1] : 0u, s0 & 31) : 0u;
     bool ok[BATCH];
     uint4 v[BATCH][QUADS];
 #pragma unroll
     for (int u = 0; u < BATCH; ++u) {
       int blk_;
-      ok[u] = s0 + u < ns && (MODE == kModeSel ? (bits[(s0 + u) >> 5] >> ((s0 + u) & 31) & 1u) != 0
-                                               : slot_block<MODE>(P.rule, b * P.Hkv + h, i, s0 + u, &blk_));
+      ok[u] = MODE == kModeSel ? (has >> u & 1u) != 0
+                               : s0 + u < ns && slot_block<MODE>(P.rule, b * P.Hkv + h, i, s0 + u, &blk_);
     }
 #pragma unroll
     for (int u = 0; u < BATCH; ++u)
 #pragma unroll
       for (int w = 0; w < QUADS; ++w)
-        v[u][w] = ok[u] ? reinterpret_cast<const uint4*>(prow + (int64_t)(s0 + u) * (D * BYTES))[w] : make_uint4(0u, 0u, 0u, 0u);
+        v[u][w] = ldg_stream_if(ok[u], prow + (int64_t)(s0 + u) * (D * BYTES) + w * 16);
 #pragma unroll
     for (int u = 0; u < BATCH; ++u)
 #pragma unroll
@@ -1853,7 +1858,7 @@ __global__ void __launch_bounds__(256) sel_dq_merge_kernel(const SelParams P, un
     *reinterpret_cast<uint4*>(P.dq_lp + b * P.dq_sb + hq * P.dq_sh + i * P.dq_sn + part * 8) = o;
     return;
   }
-  float4* dst = reinterpret_cast<float4*>(P.dq + row * D + part * 8);
+  float4* dst = reinterpret_cast<float4*>(P.dq + (int64_t)row * D + part * 8);
   dst[0] = make_float4(acc[0] * P.scale, acc[1] * P.scale, acc[2] * P.scale, acc[3] * P.scale);
   dst[1] = make_float4(acc[4] * P.scale, acc[5] * P.scale, acc[6] * P.scale, acc[7] * P.scale);
 }
