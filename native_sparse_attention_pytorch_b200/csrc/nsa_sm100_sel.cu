@@ -625,11 +625,11 @@ sel_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
 // Merges the partial results of head g of the group (batch, KV head) bh at query i: acc[8] of a thread's 16-byte piece
 // (unnormalised), the reference maximum and the sum.  The D/8 threads of a row (neighbouring lanes) share the work on the
 // slots: each looks up the position and the statistics of every D/8-th one, and hands them on by shuffles.  The kernel is a
-// stream over the partial buffer: the rows' loads go nine at a time (selected blocks and own block are 17 slots in the
-// layers here: two rounds), the first nine beside the statistics, as soon as the positions are there.
+// stream over the partial buffer: the rows' loads go six at a time (selected blocks and own block are 17 slots in the
+// layers here: three rounds), the first six beside the statistics, as soon as the positions are there.
 template <int D>
 __device__ __forceinline__ void merge_row(const SelParams& P, int bh, int i, int g, int part, float (&acc)[8], float* M_out, float* L_out) {
-  constexpr int TPR = D / 8, PER = 32 / TPR, BATCH = 9;
+  constexpr int TPR = D / 8, PER = 32 / TPR, BATCH = 6;
   const unsigned mask = (TPR == 8 ? 0xffu : 0xffffu) << (threadIdx.x & 31 & ~(TPR - 1));
   const int ns = P.ns;
   const int* positions = P.positions + ((int64_t)bh * P.N + i) * ns;
@@ -651,7 +651,7 @@ __device__ __forceinline__ void merge_row(const SelParams& P, int bh, int i, int
 #pragma unroll
       for (int u = 0; u < BATCH; ++u) {
         const int p = b0 + u < 32 ? __shfl_sync(mask, pos[(b0 + u) % 32 / TPR], (b0 + u) % TPR, TPR) : -1;
-        v[u] = p >= 0 ? *partial_piece<D>(P.partial, (int64_t)p * P.G + g, part) : make_uint4(0u, 0u, 0u, 0u);
+        v[u] = ldg_stream_if(p >= 0, partial_piece<D>(P.partial, (int64_t)p * P.G + g, part));
       }
       if (b0 == 0) {
         float m = -INFINITY, lsum = 0.f;
@@ -690,11 +690,14 @@ __device__ __forceinline__ void merge_row(const SelParams& P, int bh, int i, int
   *L_out = L;
 }
 
-// One group of D/8 threads per row; the heads of a group, whose partial rows are neighbours, next to each other.  Three
-// blocks per SM (80 registers, for nine rows in flight per thread): 17 slots of 1 M rows of 64 take 495 us = 0.78 of the
-// copy bandwidth, 7 slots of 48 k rows of 128 35 us; eight rows at a time behind the statistics, four blocks: 520 and 42 us.
+// One group of D/8 threads per row; the heads of a group, whose partial rows are neighbours, next to each other.  Bound by
+// the partial buffer's bytes: 17 slots of 1 M rows of 64 take 421 us = 0.94 of the copy bandwidth (478 us with branches
+// around the loads and nine rows at a time, 520 us with eight behind the statistics), 7 slots of 48 k rows of 128 27 us (42).
+// Four blocks per SM (64 registers) with six rows in flight per thread; measured beside them, at 64 and (with the combine,
+// 65536 x 64 heads) 128 features: three blocks and nine rows 456 us and 4.89 ms, two and seventeen 542 and 5.86, four and nine
+// 460 and 4.57, five and six 482 and 4.75, five and four 545 and 4.54, six and four 554 and 5.26; four and six 421 and 4.39.
 template <int D>
-__global__ void __launch_bounds__(256, 3) sel_merge_kernel(const SelParams P) {
+__global__ void __launch_bounds__(256, 4) sel_merge_kernel(const SelParams P) {
   constexpr int TPR = D / 8;
   const uint32_t t = blockIdx.x * (256 / TPR) + threadIdx.x / TPR;     // 32 bits hold every row id (see `supported`)
   const int part = threadIdx.x % TPR;
@@ -721,7 +724,7 @@ __global__ void __launch_bounds__(256, 3) sel_merge_kernel(const SelParams P) {
 // branch's own output tensor is written where the caller wants it.  Thread groups walk the rows position-major
 // (b, i, head), so that the heads of one position land next to each other in the destinations' [B, N, features] rows.
 template <int D, bool MC>
-__global__ void __launch_bounds__(256, 3) sel_merge_combine_kernel(const SelParams P, const CombineParams Cp, const GatherTargets Gt) {
+__global__ void __launch_bounds__(256, 4) sel_merge_combine_kernel(const SelParams P, const CombineParams Cp, const GatherTargets Gt) {
   constexpr int TPR = D / 8;
   const uint32_t t = blockIdx.x * (256 / TPR) + threadIdx.x / TPR;     // 32 bits hold every row id (see `supported`)
   const int part = threadIdx.x % TPR;
