@@ -2,8 +2,8 @@
 //
 // Run module by module, a training step of the layer is nine autograd functions, some 140 launches and 3 ms of host
 // time whatever the size; most of the launches are small conversions, additions and copies between layouts.  Here the
-// layer is about 50 launches: the GEMMs (library), the attention kernels, and one pass for everything that happens
-// between two of them (nsa_layer.cu).
+// layer is 35 to 50 launches: the GEMMs (library in the forward, which decides ReLU units and blocks; in the backward
+// nsa_gemm.cu where it is faster), the attention kernels, and one pass for everything between two of them (nsa_layer.cu).
 
 #include <ATen/Context.h>
 #include <ATen/cuda/CUDAContext.h>

@@ -2,6 +2,8 @@
 //
 // One warp serves one (batch, head group, query) task and all query heads of
 // the group, so every fetched key/value row is shared by the group (GQA).
+// In the compressed and the sliding branch, where neighbours see nearly the
+// same keys, the queries of a block also share staged tiles of 32 keys.
 // The keys of a task are runs of consecutive positions:
 //   selected branch  : one run per visible slot + the own-block run
 //   compressed branch: the memory slots and the visible compressed blocks

@@ -154,8 +154,8 @@ __device__ __forceinline__ int item_count(const SelParams& P) {
 
 // ---- index pre-pass --------------------------------------------------------------
 //
-// Four short integer kernels, 28 us at batch 4, 8192 tokens, 16 slots (72 us as a [query block x key block] matrix of
-// counts with a scan over it): clear the list totals, count, lay the lists out, fill them.  A block owns 128 queries
+// Four short integer kernels, 69 us at batch 4, 8192 tokens, 4 KV heads, 16 slots, most of it the latency of the look-ups
+// (a [query block x key block] matrix of counts with a scan over it takes more than twice as long): clear the list totals, count, lay the lists out, fill them.  A block owns 128 queries
 // of one (batch, KV head); it counts in shared memory and touches a list's total and cursor once, so the order of the
 // query blocks inside a list is whatever order the blocks arrive in.  Nothing downstream depends on it: every
 // (row, slot) partial is computed from its own row alone, and dk / dv are sums of fp32 reductions in any case.
@@ -417,9 +417,10 @@ __device__ __forceinline__ float exp_row32(float (&s)[32], float scale_log2, flo
 // block's 64 columns each; they exchange maximum and sum through shared memory), which halves the serial work per thread.
 // What bounds it: the gather of the Q rows, 18 bytes per clock and SM out of the L2 (900 cycles for the 16 KB of a chunk
 // at dim_head 64, measured with nothing else running, whatever the number of copying warps; as TMA boxes or gathers 1900
-// and more), plus 440 for the bulk store of the partial rows; the chunk takes 1900.  With the partial rows stored row by
-// row through the load / store units it took 2200: batch 4, 8192 positions, 32 / 4 heads of 64 1.10 -> 0.96 ms, 65536
-// positions, 64 / 8 heads of 128 9.1 -> 7.4 ms.
+// and more), plus 440 for the bulk store of the partial rows; the chunk takes 1700.  Batch 4, 8192 positions, 32 / 4 heads of
+// 64: 1.10 ms with the partial rows stored row by row through the load / store units, 0.96 with bulk stores, 0.90 with waits
+// of whole warps (a lane that polls takes a quarter of the issue slots), 0.85 with two values per instruction, three-way
+// maxima and gathers of one multiplication per row; 65536 positions, 64 / 8 heads of 128 9.1, 7.8 and now 7.0 ms.
 // A thread's rows are RPP apart, with up to RPP heads per KV head all of the same head (at dim_head 128 every row of 16 heads:
 // RPP is 16): `head` is that head's row 0 at the thread's piece.  Row strides are 32-bit (see problem_fwd).
 template <int D>
@@ -691,10 +692,10 @@ __device__ __forceinline__ void merge_row(const SelParams& P, int bh, int i, int
 }
 
 // One group of D/8 threads per row; the heads of a group, whose partial rows are neighbours, next to each other.  Bound by
-// the partial buffer's bytes: 17 slots of 1 M rows of 64 take 421 us = 0.94 of the copy bandwidth (478 us with branches
+// the partial buffer's bytes: 17 slots of 1 M rows of 64 take 414-421 us = 0.89 of the copy bandwidth (478 us with branches
 // around the loads and nine rows at a time, 520 us with eight behind the statistics), 7 slots of 48 k rows of 128 27 us (42).
 // Four blocks per SM (64 registers) with six rows in flight per thread; measured beside them, at 64 and (with the combine,
-// 65536 x 64 heads) 128 features: three blocks and nine rows 456 us and 4.89 ms, two and seventeen 542 and 5.86, four and nine
+// 65536 positions, 64 heads) 128 features: three blocks and nine rows 456 us and 4.89 ms, two and seventeen 542 and 5.86, four and nine
 // 460 and 4.57, five and six 482 and 4.75, five and four 545 and 4.54, six and four 554 and 5.26; four and six 421 and 4.39.
 template <int D>
 __global__ void __launch_bounds__(256, 4) sel_merge_kernel(const SelParams P) {
@@ -796,8 +797,8 @@ __global__ void __launch_bounds__(256, 4) sel_merge_combine_kernel(const SelPara
 // of it waits inside the softmax warps.  Sharing K / V matters: tile loads run at 29 bytes per clock and SM, 1100 cycles
 // for the 32 KB of a key block at dim_head 128.  One issuing warp per stream, because an issuing warp needs some 100
 // cycles per MMA next to the softmax warps: one for both streams took 15 % longer.
-// 65536 positions, 64 / 8 heads of 128: compressed 11.5 -> 7.6 ms, sliding (window 512) 2.6 -> 1.8 ms; 2 x 16384, 16 / 4
-// heads of 64: 419 -> 309 us and 290 -> 180 us (before: two CTAs per SM that walked the stages one after the other).
+// 65536 positions, 64 / 8 heads of 128: compressed 11.5 -> 7.8 ms, sliding (window 512) 2.6 -> 1.6 ms; 2 x 16384, 16 / 4
+// heads of 64: 419 -> 289 us and 290 -> 160 us (before: two CTAs per SM that walked the stages one after the other).
 //   * The accumulator is rescaled lazily: a row keeps its reference maximum until a block exceeds it by more than 2^8;
 //     only then is the O row read from tensor memory, scaled and written back (P stays below 2^8, exact in bf16's
 //     range, and the sum is fp32).
@@ -1267,7 +1268,8 @@ __global__ void __launch_bounds__(256) sel_delta_kernel(const SelParams P, float
 //   warps 0-7, 8-15  two softmax groups; chunk n (counted per CTA) belongs to group n % 2.  Two threads share a row (32
 //                    of the block's 64 columns each): they read S and dP from tensor memory, write P and dS (bf16) for
 //                    the second set of MMAs and then store the dQ row as a partial result (summed by
-//                    sel_dq_merge_kernel).  The group of an item's last chunk flushes its dK / dV with fp32 reductions.
+//                    sel_dq_merge_kernel): at dim_head 128 at once, at 64, where either group has a dQ of its own in tensor
+//                    memory, under the arithmetic of the group's next chunk.  The group of an item's last chunk flushes its dK / dV with fp32 reductions.
 //   warp 16, 17      issue the tcgen05.mma: S / dP, which run a chunk ahead, and dV, dQ, dK.  Two of them, because an MMA
 //                    is accepted when the one before it starts: the waits and addresses in between leave the tensor
 //                    cores idle unless another warp issues meanwhile.
@@ -1275,13 +1277,14 @@ __global__ void __launch_bounds__(256) sel_delta_kernel(const SelParams P, float
 //                    for the consumer: a gathering thread that did so would hold back the announcements the consumer is
 //                    waiting for.
 //   warps 19-22      gather the Q and dO rows with 16-byte cp.async into a ring of stages; a stage announces itself
-//                    (cp.async.mbarrier.arrive) when the copies have landed, the threads never wait for data.
-// What bounds it: the chain of a group's chunk (wait for S, 2500 cycles of arithmetic, dV and dQ, 1500 of dQ read-out) with
-// two groups in flight; the gathers alone (32 KB per chunk at 18 bytes per clock and SM, the rate of scattered 128-byte
-// rows out of the L2) would take 1800 cycles per chunk, the MMAs 1100.  Batch 1, 3001 positions, 16 / 2 heads of 128: 253 us
-// -> 134 + 27 us for the dQ merge (before: a walk over chunks behind block-wide barriers, dq in fp32 reductions); batch 4,
-// 8192 positions, 32 / 4 heads of 64: 1.70 -> 1.75 ms; layer step with 2 x 16384, 16 / 4 heads of 64: 1.92 ms for its three
-// branches, as before.
+//                    (cp.async.mbarrier.arrive) when the copies have landed, the threads never wait for data.  At dim_head 64
+//                    they leave what they know of the rows (dQ destination, visible columns) beside the stage.
+// What bounds it: issue slots and the chain of a group's chunk (wait for S, arithmetic, dV and dQ, dQ read-out) with two
+// groups in flight; the gathers alone (32 KB per chunk at 18 bytes per clock and SM, the rate of scattered 128-byte rows out
+// of the L2) would take 1800 cycles per chunk, the MMAs 1100.  Batch 4, 8192 positions, 32 / 4 heads of 64: 1.76 ms with one
+// lane polling each barrier, 1.62 with waits of whole warps, 1.54 with dQ under the next chunk and two values per
+// instruction, 1.43 with the row data from the loaders (four stages and one K / V buffer 1.48, S released before the
+// arithmetic the same, row ids and pointers in registers 1.54).  Batch 1, 3001 positions, 16 / 2 heads of 128: 113 -> 104 us.
 // Tensor memory (512 columns): S and dP of either group (64 columns each); dV and dK share D columns, dV in lanes 0-15 and
 // dK in lanes 16-31 of every quarter (a 64-row accumulator occupies half of the lanes); dQ: D columns, one buffer per
 // group at dim_head 64, one for both at 128.
@@ -1814,7 +1817,7 @@ __global__ void __launch_bounds__(256, 6) sel_dq_merge_kernel(const SelParams P,
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   // Rows in flight: nine of 64 (17 slots in two rounds), but eight in the sliding branch (10 slots: with nine 4 % slower, with ten
   // 12 %), four of 128 in fp32 (with six 9 % slower).  Bound by the partials' bytes: 4 x 8192 positions, 32 heads 437 -> 360 us
-  // (97 % of the copy bandwidth), 2 x 1536 x 8 heads of 128 45 -> 32 us.  The bound of six blocks an SM is what keeps the loads of a
+  // (0.95 of the copy bandwidth), 3001 positions, 16 heads of 128 45 -> 32 us.  The bound of six blocks an SM is what keeps the loads of a
   // batch together: without one the compiler stops at 32 registers and fetches them in turns (445 us; with four blocks 356 us, but
   // the sliding branch 125 us instead of 118 us and the compressed one 163 us instead of 148 us).
   constexpr int BYTES = ws::kDqElem<D>, BATCH = BYTES == 4 ? 4 : MODE == kModeSwa ? 8 : 9, QUADS = BYTES / 2;
@@ -2344,7 +2347,7 @@ static int check_ws(const SelProblem& x, const SelPlan& p, uint8_t** ws) {
 }
 
 static int problem_fwd(const SelProblem& x, cudaStream_t st) {
-  if (x.q.stride_n >> 32) return NSA_ERR_UNSUPPORTED;   // the gathers multiply in 32 bits
+  if (x.N > 1 && x.q.stride_n >> 32) return NSA_ERR_UNSUPPORTED;   // the gathers multiply in 32 bits
   const SelPlan p = make_plan(x, false);
   uint8_t* ws = nullptr;
   const int rc = check_ws(x, p, &ws);
@@ -2353,7 +2356,7 @@ static int problem_fwd(const SelProblem& x, cudaStream_t st) {
 }
 
 static int problem_bwd(const SelProblem& x, cudaStream_t st) {
-  if (x.q.stride_n >> 32 || x.dout.stride_n >> 32) return NSA_ERR_UNSUPPORTED;   // the gathers multiply in 32 bits
+  if (x.N > 1 && (x.q.stride_n >> 32 || x.dout.stride_n >> 32)) return NSA_ERR_UNSUPPORTED;   // the gathers multiply in 32 bits
   const SelPlan p = make_plan(x, true);
   uint8_t* ws = nullptr;
   const int rc = check_ws(x, p, &ws);
