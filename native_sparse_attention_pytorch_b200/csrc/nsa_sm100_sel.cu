@@ -1279,8 +1279,8 @@ __global__ void __launch_bounds__(256) sel_delta_kernel(const SelParams P, float
 //   warps 19-22      gather the Q and dO rows with 16-byte cp.async into a ring of stages; a stage announces itself
 //                    (cp.async.mbarrier.arrive) when the copies have landed, the threads never wait for data.  At dim_head 64
 //                    they leave what they know of the rows (dQ destination, visible columns) beside the stage.
-// What bounds it: issue slots and the chain of a group's chunk (wait for S, arithmetic, dV and dQ, dQ read-out) with two
-// groups in flight; the gathers alone (32 KB per chunk at 18 bytes per clock and SM, the rate of scattered 128-byte rows out
+// What bounds it: the chain of a group's chunk (wait for S, arithmetic, dV and dQ, dQ read-out) with two groups in flight
+// (issue slots 42 % busy, tensor pipe 29 %); the gathers alone (32 KB per chunk at 18 bytes per clock and SM, the rate of scattered 128-byte rows out
 // of the L2) would take 1800 cycles per chunk, the MMAs 1100.  Batch 4, 8192 positions, 32 / 4 heads of 64: 1.76 ms with one
 // lane polling each barrier, 1.62 with waits of whole warps, 1.54 with dQ under the next chunk and two values per
 // instruction, 1.43 with the row data from the loaders (four stages and one K / V buffer 1.48, S released before the
