@@ -378,7 +378,10 @@ __device__ __forceinline__ RowInfo decode_row(uint32_t e, int j, const BlockRule
   } else {
     r.lim = min(kBlock - 1, R.num_mem + r.i / R.stride - 1 - j * kBlock);
   }
-  if (!r.valid) r.lim = -1;
+  if (!r.valid) {
+    r.lo = 0;      // (the index of a padding entry would put it past the eight bits the backward keeps it in)
+    r.lim = -1;
+  }
   return r;
 }
 
