@@ -10,12 +10,15 @@
 // tensor cores reach with six products.
 //
 // A CTA computes a tile of 128 x BN.  Eight (fp32: sixteen) warps bring the operands in K steps of 64 into a ring of stages: bf16 by
-// cp.async, fp32 through registers (the next step's loads stand before the split of the present one; 16-byte pieces, whole
-// memory rows per warp: with 32 bytes per thread every load took twice the wavefronts, 3744 x 2048 x 2048 520 -> 473 us).  Another warp issues
+// cp.async, fp32 through registers (an operand's loads for the next step stand behind the split of the present one; 16-byte
+// pieces, whole memory rows per warp: with 32 bytes per thread every load takes twice the wavefronts).  Another warp issues
 // the products.  What bounds it: operands out of the L2, 24 (fp32 48 to 64) KB per step and tile.
-// Accuracy in fp32: tensor cores do not round their sums to nearest, so long sums lose bits in one direction.  The leading
-// products of a slice of K therefore have an accumulator of their own, the five small ones another, and the epilogue adds
-// them in fp32.
+// Accuracy in fp32: tensor cores cut their sums instead of rounding them, so a sum of one sign loses about 2^-25 of itself with
+// every product added to it.  An accumulator therefore takes the leading products of one K step (four), the loading threads add
+// step after step in fp32 while the next ones run, and the small products of all steps have an accumulator of their own.
+// Relative 2-norm of the error against 64 bits, operands in [0, 1), 2048 x 2048: K 512 8.6e-8 (library 3.1e-7), K 2048 1.1e-7
+// (6.0e-7), K 15000 9.1e-8 (1.7e-6); 1024 x 512 with K 15000, which the library splits, 9.1e-8 (9.9e-8).  With a third of K per
+// accumulator, added at the end, it was 2.2e-7, 1.2e-6 and 1.0e-6, and tiles of 128 columns took 15 % less time.
 #include <string.h>
 
 #include <type_traits>
@@ -40,8 +43,8 @@ struct Shape {
   static constexpr uint32_t kPlaneA = kBM * 128, kPlaneB = BN * 128;              // one bf16 term of an operand tile
   static constexpr uint32_t kStage = kTerms * (kPlaneA + kPlaneB);
   static constexpr uint32_t kBytes = kStages * kStage + 1024;
-  static constexpr int kSlices = sizeof(T) == 4 ? 512 / BN - 1 : 1;               // accumulators for the leading products
-  static constexpr uint32_t kCols = sizeof(T) == 4 ? 512 : BN;
+  // Tensor memory: bf16 one accumulator; fp32 three for the leading products of a step, in turn, and one for the small products
+  static constexpr uint32_t tSmall = 3 * BN, kCols = (sizeof(T) == 4 ? 4 : 1) * BN;
 };
 
 // x = h + m + l, each term rounded to bf16; the remainders are exact.  Where h is not finite (x is not, or rounds to infinity)
@@ -164,12 +167,6 @@ struct Bars {
   uint64_t full[4], empty[4], done;
 };
 
-// The accumulator that takes the leading products of a step
-template <typename T, int BN>
-__device__ __forceinline__ int slice_of(int step, int steps) {
-  constexpr int N = Shape<T, BN>::kSlices;
-  return N == 1 ? 0 : step * N / steps;
-}
 __device__ __forceinline__ void tmem_ld_cols(uint32_t at, float (&v)[32]) { tmem_ld32(at, v); }
 __device__ __forceinline__ void tmem_ld_cols(uint32_t at, float (&v)[16]) { tmem_ld16(at, v); }
 }  // namespace gemm
@@ -218,6 +215,23 @@ __global__ void __launch_bounds__((gemm::Shape<T, BN>::kThreads), sizeof(T) == 4
   tc_fence_after_sync();
   const uint32_t tm = tmem_slot;
 
+  // The sum of this CTA's steps: a loading thread has a row and kOwn columns of the tile.  fp32: the leading products of a step
+  const int own_row = (warp & 3) * 32 + lane, own_col = (warp >> 2) * kOwn;
+  const uint32_t tm_own = tm + ((uint32_t)((warp & 3) * 32) << 16) + own_col;
+  float v[kOwn];
+#pragma unroll
+  for (int x = 0; x < kOwn; ++x) v[x] = 0.f;
+  auto fold = [&](int step) {
+#pragma unroll
+    for (int c = 0; c < kOwn; c += 8) {
+      float t[8];
+      tmem_ld8(tm_own + step % 3 * BN + c, t);
+      tmem_ld_wait();
+#pragma unroll
+      for (int x = 0; x < 8; ++x) v[c + x] += t[x];
+    }
+  };
+
   if (tid < kLoaders) {
     // ------------------------------------------------------------------ operands
     auto operand = [&](bool second, int seg) {
@@ -248,28 +262,27 @@ __global__ void __launch_bounds__((gemm::Shape<T, BN>::kThreads), sizeof(T) == 4
     };
     if constexpr (F32) {
       __nv_bfloat162 odd = __floats2bfloat162_rn(0.f, 0.f);
-      float4 a[2][decltype(A)::N], b[2][decltype(B)::N];
+      float4 a[decltype(A)::N], b[decltype(B)::N];
       if (steps > 0) {
-        fetch(A, a[0]);
-        fetch(B, b[0]);
+        fetch(A, a);
+        fetch(B, b);
       }
-      for (int step0 = 0; step0 < steps; step0 += 2) {
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int step = step0 + u;
-          if (step < steps) {
-            if (step + 1 < steps) {
-              advance();
-              fetch(A, a[u ^ 1]);
-              fetch(B, b[u ^ 1]);
-            }
-            wait_free(step);
-            const uint32_t at = base + (step % kStages) * S::kStage;   // (the places depend on the layout only, not on the part)
-            put(A, at, a[u], odd);
-            put(B, at + 3 * S::kPlaneA, b[u], odd);
-            fence_proxy_async_smem();
-            mbar_arrive(smem_u32(&bars.full[step % kStages]));
-          }
+      for (int step = 0; step < steps; ++step) {
+        wait_free(step);
+        const uint32_t at = base + (step % kStages) * S::kStage;   // (the places depend on the layout only, not on the part)
+        put(A, at, a, odd);
+        if (step + 1 < steps) {
+          advance();
+          fetch(A, a);
+        }
+        put(B, at + 3 * S::kPlaneA, b, odd);
+        if (step + 1 < steps) fetch(B, b);
+        fence_proxy_async_smem();
+        mbar_arrive(smem_u32(&bars.full[step % kStages]));
+        if (step >= 2) {        // (wait_free)
+          tc_fence_after_sync();
+          fold(step - 2);
+          tc_fence_before_sync();
         }
       }
       if (__hisnan(odd.x) || __hisnan(odd.y)) odd_input = 1;
@@ -295,7 +308,6 @@ __global__ void __launch_bounds__((gemm::Shape<T, BN>::kThreads), sizeof(T) == 4
     // ------------------------------------------------------------------ products
     const uint32_t idesc = instr_desc_bf16(kBM, BN, a_mn, b_mn);
     const uint32_t step_a = a_mn ? 2048 : 32, step_b = b_mn ? 2048 : 32;
-    int slice = -1;
     for (int step = 0; step < steps; ++step) {
       const int stage = step % kStages;
       mbar_wait_bounded(smem_u32(&bars.full[stage]), (uint32_t)(step / kStages) & 1, &abort_flag);
@@ -303,15 +315,12 @@ __global__ void __launch_bounds__((gemm::Shape<T, BN>::kThreads), sizeof(T) == 4
       tc_fence_after_sync();
       const uint32_t at = base + stage * S::kStage;
       const uint64_t dA = smem_desc_sw128(at, 8192), dB = smem_desc_sw128(at + S::kTerms * S::kPlaneA, 8192);
-      const int now = slice_of<T, BN>(step, steps);
-      const bool fresh = now != slice;
-      slice = now;
+      const uint32_t tL = tm + (F32 ? step % 3 * BN : 0), tR = tm + S::tSmall;
 #pragma unroll
       for (int k = 0; k < kBK / 16; ++k) {
         const uint64_t ak = desc_advance(dA, k * step_a), bk = desc_advance(dB, k * step_b);
-        mma_bf16_elect(tm + slice * BN, ak, bk, idesc, !fresh || k > 0);
+        mma_bf16_elect(tL, ak, bk, idesc, (!F32 && step > 0) || k > 0);
         if constexpr (F32) {
-          const uint32_t tR = tm + S::kSlices * BN;
           const uint64_t a1 = desc_advance(ak, S::kPlaneA), a2 = desc_advance(ak, 2 * S::kPlaneA);
           const uint64_t b1 = desc_advance(bk, S::kPlaneB), b2 = desc_advance(bk, 2 * S::kPlaneB);
           mma_bf16_elect(tR, ak, b2, idesc, step > 0 || k > 0);
@@ -365,30 +374,15 @@ __global__ void __launch_bounds__((gemm::Shape<T, BN>::kThreads), sizeof(T) == 4
     }
   };
 
-  // The sum of this CTA's steps: a thread has a row and kOwn columns
-  const int own_row = (warp & 3) * 32 + lane, own_col = (warp >> 2) * kOwn;
-  float v[kOwn];
   if (tid < kLoaders) {
-    const uint32_t tm_lane = tm + ((uint32_t)((warp & 3) * 32) << 16) + own_col;
-#pragma unroll
-    for (int x = 0; x < kOwn; ++x) v[x] = 0.f;
+    if (F32)
+      for (int step = max(steps - 2, 0); step < steps; ++step) fold(step);
     if (steps > 0) {
-      tmem_ld_cols(tm_lane + (F32 ? S::kSlices * BN : 0), v);
+      float t[kOwn];
+      tmem_ld_cols(tm_own + (F32 ? S::tSmall : 0), t);
       tmem_ld_wait();
-      if constexpr (F32) {
-        int seen = -1;
-#pragma unroll 1
-        for (int step = 0; step < steps; ++step) {
-          const int slice = slice_of<T, BN>(step, steps);
-          if (slice == seen) continue;
-          seen = slice;
-          float t[kOwn];
-          tmem_ld_cols(tm_lane + slice * BN, t);
-          tmem_ld_wait();
 #pragma unroll
-          for (int x = 0; x < kOwn; ++x) v[x] += t[x];
-        }
-      }
+      for (int x = 0; x < kOwn; ++x) v[x] += t[x];
     }
     const int row = m0 + own_row, col = n0 + own_col;
     if (F32 && odd_input != 0 && row < task.m) {
@@ -469,10 +463,8 @@ __global__ void __launch_bounds__((gemm::Shape<T, BN>::kThreads), sizeof(T) == 4
 
 static int64_t steps_of(const GemmTask& t) { return ((int64_t)t.k[0] + gemm::kBK - 1) / gemm::kBK + ((int64_t)t.k[1] + gemm::kBK - 1) / gemm::kBK; }
 static int64_t tiles_of(const GemmTask& t, int cols) { return (int64_t)((t.m + gemm::kBM - 1) / gemm::kBM) * ((t.n + cols - 1) / cols); }
-// K steps that fp32 accumulators can take.  Up to ten steps (640 products) per accumulator of the leading products the result
-// is nearer to the exact one than fp32 steps are (relative 2-norm, normal operands: K 2048 6.5e-7 against the library's 8.1e-7
-// with three accumulators, 2.7e-7 with seven; K 512 1.7e-7 against 4.1e-7); twice as many and it is not (K 4096 1.4e-6 against
-// 1.1e-6).  Longer sums are split over the CTAs of a cluster.
+// K steps that a CTA adds up in fp32.  Longer sums are split over the CTAs of a cluster: the roundings of a sum of n steps come to
+// some 2^-25 sqrt(n / 3) of it, which stays below what the last bit of the leading products loses.
 static int most_steps(int cols) { return cols == 64 ? 70 : 32; }
 
 // How a group of products is cut: columns of a tile, CTAs per cluster, and the K steps from which on a task's tiles are shared by a cluster
@@ -480,9 +472,9 @@ struct GemmCut {
   int cols, split, from;
   int of(const GemmTask& t) const { return t.sums == nullptr && steps_of(t) >= from ? split : 1; }
 };
-// The cut with the shortest estimate (against the best of all cuts, measured for 22 groups of 62 to 15000 rows: within 10 % for all but two,
-// which take 1.2 times as long): the K steps of the longest CTA, or the steps per SM, whichever is more; a step with 128
-// columns costs 1.6 of one with 64, and CTAs that share a tile meet for the price of some two steps.
+// The cut with the shortest estimate (against the best of all cuts, measured for 24 groups of 62 to 15000 rows in fp32: 3 % longer on
+// average, 12 % at most): the K steps of the longest CTA, or the steps per SM, whichever is more; a step with 128 columns costs
+// 1.95 of one with 64, and a CTA that shares a tile spends some three steps (bf16: two, and two more per launch) on every other one.
 static GemmCut gemm_cut(const GemmGroup& G, int dtype) {
   const bool f32 = dtype == NSA_F32;
   GemmCut best = {64, 1, 1 << 30};
@@ -499,10 +491,10 @@ static GemmCut gemm_cut(const GemmGroup& G, int dtype) {
         for (int t = 0; t < G.tasks; ++t) {
           const int64_t per = (steps_of(G.task[t]) + cut.of(G.task[t]) - 1) / cut.of(G.task[t]);
           longest = per > longest && tiles_of(G.task[t], cols) > 0 ? per : longest;
-          total += tiles_of(G.task[t], cols) * (steps_of(G.task[t]) + (cut.of(G.task[t]) > 1 ? 2 * split : 0));
+          total += tiles_of(G.task[t], cols) * (steps_of(G.task[t]) + (cut.of(G.task[t]) > 1 ? (f32 ? 3 : 2) * split : 0));
           fits = fits && (!f32 || per <= most_steps(cols));
         }
-        const double per_sm = (double)total / 148., estimate = (per_sm > longest ? per_sm : longest + .5 * per_sm) * (cols == 64 ? 1. : 1.6) + (split > 1 ? 2. : 0.);
+        const double per_sm = (double)total / 148., estimate = (per_sm > longest ? per_sm : longest + .5 * per_sm) * (cols == 64 ? 1. : 1.95) + (split > 1 && !f32 ? 2. : 0.);
         if (G.split == 0 && !fits) continue;
         if (least < 0. || estimate < least) {
           least = estimate;
