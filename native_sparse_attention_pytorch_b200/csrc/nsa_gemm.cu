@@ -47,8 +47,9 @@ struct Shape {
   static constexpr uint32_t tSmall = 3 * BN, kCols = (sizeof(T) == 4 ? 4 : 1) * BN;
 };
 
-// x = h + m + l, each term rounded to bf16; the remainders are exact.  Where h is not finite (x is not, or rounds to infinity)
-// the last term is NaN, and stays in `odd`: the terms would give NaN for an infinite product.
+// x = h + m + l, each term rounded to bf16; the remainders are exact.  Infinities and NaN are in h as they are, and m and l are
+// NaN: the leading products are then what fp32 gives, the small ones are left out (see the epilogue).  A finite x that rounds to
+// an infinite h (above 3.39e38) has an infinite m, which stays in `odd`.
 __device__ __forceinline__ void split3(const float4& x, uint2& h, uint2& m, uint2& l, __nv_bfloat162& odd) {
   auto pair = [&](float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
     hi = pack_bf16(a, b);
@@ -58,7 +59,7 @@ __device__ __forceinline__ void split3(const float4& x, uint2& h, uint2& m, uint
     a -= __uint_as_float(mid << 16);
     b -= __uint_as_float(mid & 0xffff0000u);
     lo = pack_bf16(a, b);
-    odd = __hfma2(*reinterpret_cast<const __nv_bfloat162*>(&lo), __floats2bfloat162_rn(0.f, 0.f), odd);
+    odd = __hmax2(odd, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&mid)));      // (keeps the number beside a NaN)
   };
   pair(x.x, x.y, h.x, m.x, l.x);
   pair(x.z, x.w, h.y, m.y, l.y);
@@ -285,7 +286,7 @@ __global__ void __launch_bounds__((gemm::Shape<T, BN>::kThreads), sizeof(T) == 4
           tc_fence_before_sync();
         }
       }
-      if (__hisnan(odd.x) || __hisnan(odd.y)) odd_input = 1;
+      if (__hisinf(odd.x) || __hisinf(odd.y)) odd_input = 1;
     } else {
       constexpr int kAhead = kStages - 1;
       for (int step = 0; step < steps + kAhead; ++step) {
@@ -382,11 +383,14 @@ __global__ void __launch_bounds__((gemm::Shape<T, BN>::kThreads), sizeof(T) == 4
       tmem_ld_cols(tm_own + (F32 ? S::tSmall : 0), t);
       tmem_ld_wait();
 #pragma unroll
-      for (int x = 0; x < kOwn; ++x) v[x] += t[x];
+      for (int x = 0; x < kOwn; ++x)
+        if (isfinite(v[x])) v[x] += t[x];    // else an operand is not finite and its small terms are NaN; the leading ones are
+                                             // fp32's, but for infinity times a number below 2^-134, which is zero in bf16: NaN
     }
     const int row = m0 + own_row, col = n0 + own_col;
     if (F32 && odd_input != 0 && row < task.m) {
-      // an operand of the tile is infinite, NaN or next to overflow: in fp32 steps, as IEEE has it
+      // a finite operand of the tile has no bf16 term next to it: in fp32 steps, as IEEE has it.  Many times as long as the
+      // products above, so not for infinities and NaN, which a step with an overflow is full of.
 #pragma unroll 1
       for (int x = 0; x < kOwn; ++x) {
         float s = 0.f;
