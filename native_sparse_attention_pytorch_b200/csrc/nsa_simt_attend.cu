@@ -3,7 +3,8 @@
 // One warp serves one (batch, head group, query) task and all query heads of
 // the group, so every fetched key/value row is shared by the group (GQA).
 // In the compressed and the sliding branch, where neighbours see nearly the
-// same keys, the queries of a block also share staged tiles of 32 keys.
+// same keys, the queries of a block also share staged tiles of 32 keys, unless
+// they see few (see shares_tiles).
 // The keys of a task are runs of consecutive positions:
 //   selected branch  : one run per visible slot + the own-block run
 //   compressed branch: the memory slots and the visible compressed blocks
@@ -56,18 +57,40 @@ __device__ __forceinline__ void dot_rows(float (&s)[GT], const float* rows, cons
   }
 }
 
-// The runs of one task of the selected branch.  get(r) yields [start, end) in key-row units: slot s is run s, the own block is
-// run nsel; `uniform`: the query sees no key at all (all logits equal, no gradient to q and k).
+// The keys of query i in the compressed and the sliding branch: rows first .. first + total - 1 (compressed: the memory slots, then the visible blocks)
+template <int BR>
+struct KeyRange {
+  int first, total;
+  __device__ __forceinline__ KeyRange(const AttnParams& P, int i) {
+    if (BR == BR_CMP) {
+      first = 0;
+      total = P.num_mem + (P.causal ? min(P.ncb, i / P.stride) : P.ncb);
+    } else {
+      first = max(0, i - P.window);
+      total = (P.causal ? i + 1 : min(P.seq, i + P.window + 1)) - first;
+    }
+  }
+};
+
+// The runs of one task.  get(r) yields [start, end) in key-row units.  Selected branch: slot s is run s, the own block is run nsel;
+// `uniform`: the query sees no key at all (all logits equal, no gradient to q and k).  The other two: one run.
 struct Run {
   int start, end;
   int slot;  // slot index, or -1
 };
 
+template <int BR>
 struct TaskRuns {
   int count;
   bool uniform;
   int total_keys; // number of keys when uniform
   __device__ __forceinline__ void init(const AttnParams& P, int b, int grp, int i) {
+    if (BR != BR_SEL) {
+      count = 1;
+      uniform = false;
+      total_keys = 0;
+      return;
+    }
     count = P.nsel + (P.diag != NSA_DIAG_NONE ? 1 : 0);
     bool any = P.diag != NSA_DIAG_NONE;
     const int nfb = (P.seq + P.block - 1) / P.block;
@@ -85,7 +108,11 @@ struct TaskRuns {
   __device__ __forceinline__ Run get(const AttnParams& P, int b, int grp, int i, int r) const {
     Run run;
     run.slot = -1;
-    if (r < P.nsel) {
+    if (BR != BR_SEL) {
+      const KeyRange<BR> keys(P, i);
+      run.start = keys.first;
+      run.end = keys.first + keys.total;
+    } else if (r < P.nsel) {
       const int nfb = (P.seq + P.block - 1) / P.block;
       const int64_t base = (((int64_t)b * P.groups + grp) * P.seq + i) * P.nsel;
       const int64_t blk = P.idx[base + r];
@@ -102,8 +129,8 @@ struct TaskRuns {
   }
 };
 
-template <typename T, int GT>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32) attend_sel_fwd_kernel(const AttnParams P) {
+template <typename T, int GT, int BR>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32) attend_query_fwd_kernel(const AttnParams P) {
   extern __shared__ __align__(16) float smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t task = (int64_t)blockIdx.x * kWarpsPerBlock + warp;
@@ -131,7 +158,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) attend_sel_fwd_kernel(con
     acc[g][0][0] = acc[g][0][1] = acc[g][1][0] = acc[g][1][1] = 0.f;
   }
 
-  TaskRuns runs;
+  TaskRuns<BR> runs;
   runs.init(P, b, grp, i);
   for (int r = 0; r < runs.count; ++r) {
     const Run run = runs.get(P, b, grp, i, r);
@@ -194,8 +221,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) attend_sel_fwd_kernel(con
   }
 }
 
-template <typename T, int GT>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32) attend_sel_bwd_kernel(const AttnParams P) {
+template <typename T, int GT, int BR>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32) attend_query_bwd_kernel(const AttnParams P) {
   extern __shared__ __align__(16) float smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t task = (int64_t)blockIdx.x * kWarpsPerBlock + warp;
@@ -240,7 +267,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) attend_sel_bwd_kernel(con
     dq[g][0][0] = dq[g][0][1] = dq[g][1][0] = dq[g][1][1] = 0.f;
   }
 
-  TaskRuns runs;
+  TaskRuns<BR> runs;
   runs.init(P, b, grp, i);
   const float p_uniform = runs.total_keys > 0 ? 1.f / (float)runs.total_keys : 0.f;
   for (int r = 0; r < runs.count; ++r) {
@@ -310,7 +337,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) attend_sel_bwd_kernel(con
         }
       }
     }
-    if (P.slot_grads != nullptr && run.slot >= 0) {
+    if (BR == BR_SEL && P.slot_grads != nullptr && run.slot >= 0) {
       const float total = warp_sum(slot_part);
       if (lane == 0)
         P.slot_grads[(((int64_t)b * P.groups + grp) * P.seq + i) * P.nsel + run.slot] = total;
@@ -338,24 +365,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) attend_sel_bwd_kernel(con
 // them once: one reduction per key and block instead of one per key and query.
 // Bound: instruction issue.  4 x 512 positions, 8 / 4 heads of 64 in fp32, forward and backward in us, against a warp per
 // query that fetches its keys alone: sliding window of 32
-// 37 + 85 -> 31 + 52, 64 compressed blocks 50 + 96 -> 33 + 49; 4 x 1024, 8 heads, 512 compressed blocks 826 + 1691 -> 423 + 610.  A
-// window of 2, where a block shares little, takes longer on its own (4 x 1024, 8 heads: 32 + 51 -> 39 + 67), a tenth of what a
-// layer of such sizes gains in its compressed branch.
-//
-// The keys of query i: rows first .. first + total - 1 (compressed: the memory slots, then the visible blocks)
-template <int BR>
-struct KeyRange {
-  int first, total;
-  __device__ __forceinline__ KeyRange(const AttnParams& P, int i) {
-    if (BR == BR_CMP) {
-      first = 0;
-      total = P.num_mem + (P.causal ? min(P.ncb, i / P.stride) : P.ncb);
-    } else {
-      first = max(0, i - P.window);
-      total = (P.causal ? i + 1 : min(P.seq, i + P.window + 1)) - first;
-    }
-  }
-};
+// 37 + 85 -> 31 + 52, 64 compressed blocks 50 + 96 -> 33 + 49; 4 x 1024, 8 heads, 512 compressed blocks 826 + 1691 -> 423 + 610.
 // Rows of a tile lie 16 bytes further apart than they are long: neighbours fall on other banks.
 template <typename T>
 __host__ __device__ __forceinline__ int tile_pitch(int d) { return d * (int)sizeof(T) + 16; }
@@ -686,19 +696,42 @@ static int launch_with(const AttnParams& P, int64_t blocks, int threads, int64_t
   return err == cudaSuccess ? NSA_OK : fail((int)err, cudaGetErrorString(err));
 }
 
+// Whether the queries of a block share tiles, or a warp fetches the keys of its query alone (the selected branch always): by the
+// most keys that a query sees, because a query of few shares little and a tile costs its staging whatever is seen of it, by the
+// heads that share a fetched row anyway, and in the backward by dim_head (fewer queries in a block of 32 rows, and larger ones).
+// Measured, the time alone over that with tiles (fp32 and bf16, 1 x 256 to 2 x 4096 positions).  Forward: up to four heads per KV head
+// 0.8 to 0.96 with 3 to 9 keys, 1.0 to 1.2 with 11, 1.4 to 2 with 65; eight heads 0.8 to 1.0 up to 15 keys, 0.95 to 1.14 with 21;
+// sixteen 0.96 to 1.1 from 11 on, but 0.85 to 1.0 where the blocks do not fill the GPU.  Backward: 0.75 to 0.9 with 3 keys, 0.9 to 1.0
+// with 9 (sixteen heads 0.9 to 1.35), 1.0 to 1.3 with 11, 1.6 to 2 with 65; heads of 128, eight of them 0.85 to 1.0 up to 15 keys, 1.04
+// to 1.2 with 21; sixteen 0.7 to 0.9 with 9 to 21, 1.0 to 1.2 with 25, with few blocks 0.95 to 1.2 with 11.  Compressed backward: 0.7 to 1.0
+// with two keys, 1.0 to 1.3 with three; sixteen heads of 128 in many blocks 0.8 to 1.0 with five to nine; forward 1.0 to 2, but for
+// 10 us against 13 with a single block and eight heads or more.
+template <int BR>
+static bool shares_tiles(const AttnParams& P, int heads, bool backward) {
+  if (BR == BR_SEL) return false;
+  const bool wide = P.d > 64, fills = (int64_t)P.batch * P.groups * P.seq >= 8 * 148;   // (blocks of eight queries, SMs)
+  if (BR == BR_CMP) return !backward || P.num_mem + P.ncb >= (wide && heads > 8 && fills ? 12 : 3);
+  const int64_t keys = (int64_t)P.window * (P.causal ? 1 : 2) + 1;
+  if (!backward) return heads > 8 ? fills && keys >= 11 : keys >= (heads > 4 ? 20 : 11);
+  if (wide && heads > 4) return keys >= (heads <= 8 ? 20 : fills ? 24 : 11);
+  return keys >= (heads > 8 ? 9 : 11);
+}
+
 template <typename T, int GT, int BR>
 static int launch_one(const AttnParams& P, bool backward, cudaStream_t stream) {
-  if constexpr (BR == BR_SEL) {
+  if (!shares_tiles<BR>(P, GT, backward)) {
     const int64_t ntasks = (int64_t)P.batch * P.groups * P.seq, blocks = (ntasks + kWarpsPerBlock - 1) / kWarpsPerBlock;
     const int64_t smem = (int64_t)kWarpsPerBlock * GT * P.d * sizeof(float) * (backward ? 2 : 1);
-    return backward ? launch_with<attend_sel_bwd_kernel<T, GT>>(P, blocks, kWarpsPerBlock * 32, smem, stream)
-                    : launch_with<attend_sel_fwd_kernel<T, GT>>(P, blocks, kWarpsPerBlock * 32, smem, stream);
-  } else {
+    if (backward) return launch_with<attend_query_bwd_kernel<T, GT, BR>>(P, blocks, kWarpsPerBlock * 32, smem, stream);
+    if constexpr (BR != BR_CMP) return launch_with<attend_query_fwd_kernel<T, GT, BR>>(P, blocks, kWarpsPerBlock * 32, smem, stream);
+  }
+  if constexpr (BR != BR_SEL) {
     const int queries = backward ? DenseBwd<T, GT>::QB : DenseFwd<T, GT>::QB;
     const int64_t blocks = (int64_t)P.batch * P.groups * ((P.seq + queries - 1) / queries);
     return backward ? launch_with<attend_dense_bwd_kernel<T, GT, BR>>(P, blocks, queries * 32, DenseBwd<T, GT>::smem(P.d), stream)
                     : launch_with<attend_dense_fwd_kernel<T, GT, BR>>(P, blocks, queries * 32, DenseFwd<T, GT>::smem(P.d), stream);
   }
+  return NSA_OK;   // (not reached)
 }
 
 template <typename T, int BR>
