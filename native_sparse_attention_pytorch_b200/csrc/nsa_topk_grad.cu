@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(256) topk_logits_kernel(const TopkGrad P) {
 template <typename T>
 __global__ void __launch_bounds__(256) topk_products_kernel(const TopkGrad P, int dq_tiles, int dck_slices) {
   constexpr int TILE = 64, KB = 16;
-  __shared__ float a_s[KB][TILE + 4], b_s[KB][TILE + 4];
+  __shared__ __align__(16) float a_s[KB][TILE + 4], b_s[KB][TILE + 4];   // (read as float4)
   const int tid = threadIdx.x, ty = tid / 16, tx = tid % 16, d0 = blockIdx.y * TILE;
   const int sel_per_kv = P.sel_heads / P.kv_heads, per_sel = P.heads / P.sel_heads, F = (P.heads + 2 * P.kv_heads) * P.d;
   const int kv = P.num_mem + P.ncb, row_tiles = (P.seq + TILE - 1) / TILE, col_tiles = (P.ncb + TILE - 1) / TILE;
