@@ -10,6 +10,8 @@ from util import assert_close_bf16, assert_close_f32
 pytestmark = pytest.mark.gpu
 
 
+# Both sides run the decoding kernel, in the layer's one call and between the layer's modules: what is compared here is what the two
+# forms of a step hand it.  Its picks are compared with picks computed apart in test_gpu_decode_picks.py.
 # (cache length, selected blocks of 64, equal scores everywhere, dtype): 1, 2, 32, 33, 65 and 102 columns
 @pytest.mark.parametrize('n, nsel, equal, dtype', [(66, 4, False, torch.float32), (130, 2, False, torch.bfloat16),
                                                    (2050, 16, False, torch.float32), (2114, 16, True, torch.float32),

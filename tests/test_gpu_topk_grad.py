@@ -37,5 +37,6 @@ def test_gradient_through_the_topk(b, n, heads, kv_heads, d, options):
     assert_close_f32(out, want, 'out')
     assert_close_f32(dx, want_dx, 'd input')
     for name, ref in want_grads.items():
+        assert (ref is None) == (grads[name] is None), name
         if ref is not None and grads[name] is not None:
             assert_close_f32(grads[name], ref, name)
