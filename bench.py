@@ -486,12 +486,13 @@ def kernel_rows(breakdown, w, mask, f_fwd, f_bwd, tensor_peak):
     b, n, hq, hkv, d = w['batch'], w['seq'], w['q_heads'], w['kv_heads'], w['dim_head']
     slots = int(mask.sum().item()) * (hq // hkv) + b * hq * n          # (row, slot) pairs incl. the own block
     part = slots * (d * 2)                                            # bf16 partial rows
-    rows_bytes = b * hq * n * d * 2
+    rows_bytes, kv = b * hq * n * d * 2, 2 * b * hkv * n * d           # bytes of q, values of dk and dv
     work = {   # kernel name prefix -> (bound, algorithmic FLOPs or bytes per launch)
         'sel_fwd_kernel': ('tensor', f_fwd), 'sel_bwd_ws_kernel': ('tensor', f_bwd),
-        'sel_merge_kernel': ('hbm', part + slots * 8 + rows_bytes), 'sel_dq_merge_kernel': ('hbm', part + rows_bytes),
-        'sel_delta_kernel': ('hbm', 2 * rows_bytes + b * hq * n * 4),
-        'attend_fwd_kernel': ('tensor', f_fwd), 'attend_bwd_kernel': ('tensor', f_bwd),
+        # the last two also round and clear the fp32 accumulators of dk and dv
+        'sel_merge_kernel': ('hbm', part + slots * 8 + rows_bytes), 'sel_dq_merge_kernel': ('hbm', part + rows_bytes + kv * (4 + 2)),
+        'sel_delta_kernel': ('hbm', 2 * rows_bytes + b * hq * n * 4 + kv * 4),
+        'attend_query_fwd_kernel': ('tensor', f_fwd), 'attend_query_bwd_kernel': ('tensor', f_bwd),
     }
     out = []
     for name, (per_step, us) in sorted(breakdown.items(), key=lambda kv: -kv[1][0] * kv[1][1]):
