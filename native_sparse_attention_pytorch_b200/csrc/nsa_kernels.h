@@ -244,7 +244,9 @@ int launch_relu_sums(const ColumnSums& P, int dtype, cudaStream_t stream);
 int64_t gate_sums_partial(int cols);    // floats
 int gate_sums_counters(int cols);       // zero before the call
 int launch_layer_tail(const LayerShape& L, const QkvGrad& P, const GateSums& S, float* dpos, int dtype, cudaStream_t stream);
-bool gemm_serves(const GemmGroup& G, int dtype);   // fp32: sums of up to 35840 products (70 steps of 64 on each of 8 CTAs)
+// fp32: sums of up to 35840 products (70 steps of 64 on each of 8 CTAs), of up to 4480 in a task with column sums (one CTA); a task
+// beyond that is not served, nor is any other of its group
+bool gemm_serves(const GemmGroup& G, int dtype);
 int launch_gemm(GemmGroup& G, int dtype, cudaStream_t stream);
 int launch_topk_grad(const TopkGrad& P, int dtype, cudaStream_t stream);
 int launch_round(const float* src, void* dst, int64_t n, cudaStream_t stream);

@@ -2,7 +2,7 @@
 // between the layouts of the projections and those of the branches, one pass each.  Bound: HBM at training sizes, launch
 // count at small ones.  As separate tensor operations these were some 60 of the 140 launches of a training step.
 // Measured for the whole step with csrc/host/layer.cpp (forward + backward): dim 512, 8 heads of 64, 2 x 31 fp32 2.77 ->
-// 0.46 ms; dim 256, 4 / 2 heads, 1 x 1024 bf16 3.20 -> 0.58 ms; dim 1024, 16 / 4 heads, 2 x 16384 bf16 6.49 -> 4.90 ms.
+// 0.47 ms; dim 256, 4 / 2 heads, 1 x 1024 bf16 3.20 -> 0.60 ms; dim 1024, 16 / 4 heads, 2 x 16384 bf16 6.49 -> 4.90 ms.
 
 #include "nsa_common.cuh"
 #include "nsa_kernels.h"

@@ -363,8 +363,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) attend_query_bwd_kernel(c
 // walks the union of their keys in tiles of 32 that it stages once, whole rows per access.  In the backward the warps leave P
 // and dS of a tile in shared memory; then every warp sums dk and dv of its share of the tile's keys over all rows and adds
 // them once: one reduction per key and block instead of one per key and query.
-// Bound: instruction issue.  4 x 512 positions, 8 / 4 heads of 64 in fp32, forward and backward in us, against a warp per
-// query that fetches its keys alone: sliding window of 32
+// Bound: issue slots and shared memory are busy half of the time each (51 to 55 and 41 to 45 % in the forward, 45 to 48 and 53 to 55 % in the
+// backward), a third of the warps is resident and waits for the one or the other.  4 x 512 positions, 8 / 4 heads of 64 in fp32,
+// forward and backward in us, against a warp per query that fetches its keys alone: sliding window of 32
 // 37 + 85 -> 31 + 52, 64 compressed blocks 50 + 96 -> 33 + 49; 4 x 1024, 8 heads, 512 compressed blocks 826 + 1691 -> 423 + 610.
 // Rows of a tile lie 16 bytes further apart than they are long: neighbours fall on other banks.
 template <typename T>

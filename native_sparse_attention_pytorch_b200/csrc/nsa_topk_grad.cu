@@ -1,10 +1,10 @@
 // Gradient through the differentiable top-k: d(value of a pick) back through the softmax with the sink, the mean over a
 // block's compressed columns and the mean over the heads to the logits, and from there to queries and compressed keys.
 //
-// Two launches.  As tensor operations with two library products these were 38 launches and 300 us of host time, 100 us on
-// the GPU for 4 x 512 positions of 8 / 4 heads with 64 compressed columns; now 37 us, and the whole
-// step 1286 -> 1154 us.
-// Bound: launch count at such sizes, then the CUDA cores (4 d ncb operations per row in fp32).
+// Two launches, 37 us for 4 x 512 positions of 8 / 4 heads with 64 compressed columns; as tensor operations with two library products
+// 38 launches, 100 us on the GPU and 300 us on the host.
+// Bound there: latency of the loads in the products (256 blocks, issue slots 16 % busy); with more rows the CUDA cores (4 d ncb
+// operations per row in fp32).
 #include "nsa_common.cuh"
 #include "nsa_kernels.h"
 
